@@ -6,7 +6,7 @@
 //   * the token tiles (expert, first entry, entry count <= block_m) the grouped GEMMs iterate over;
 //   * the plan words: tile count, K-split factors for both GEMMs, entry count.
 // It first waits (bounded) for every source rank's dispatch flag of this forward, so the receive
-// buffer is complete when it is read, and clears the split-K arrival counters.
+// buffer is complete when it is read, and clears the counters that the GEMMs of this forward use.
 //
 // The stable expert-major order is a counting sort: every warp owns a contiguous range of the flat
 // (row, slot) index space, counts its keys per expert, a scan over (expert, warp) turns the counts
@@ -54,6 +54,23 @@ __device__ __forceinline__ int block_exclusive_scan(int v, int* warp_sums, int& 
   return res;
 }
 
+// Row pitch of the per-warp histograms, in words: odd, so that the prefix over the warps (lane = source warp, one
+// expert at a time) reads 32 different banks.  With the pitch equal to L, 288 experts put all 32 lanes on one bank:
+// 9 rounds x 32 warps x 64 serialised accesses, about 10 us of the kernel.
+__host__ __device__ __forceinline__ int hist_pitch(int L) { return L | 1; }
+
+// Clears what the two GEMMs of this forward will count on: the finished quarters of the token tiles in use, and,
+// for a GEMM whose units are cut along K, the arrival counters of those units.  (The counters are zero again after
+// every complete forward; a forward that gave up part-way leaves some set, which is why they are cleared at all.)
+// Only the words in use: clearing the arrays whole was 100 KB to 400 KB of stores by one CTA at 288 experts.
+__device__ __forceinline__ void clear_counters(const mf_meta_args& a, int n_tiles, int cut1, int cut2) {
+  for (int i = threadIdx.x; i < min(n_tiles, a.n_tile_done); i += kMetaThreads) a.counters1[a.n_counters1 + i] = 0;
+  if (cut1 != 1)
+    for (int i = threadIdx.x; i < min(n_tiles * a.m_blocks1 * 8, a.n_counters1); i += kMetaThreads) a.counters1[i] = 0;
+  if (cut2 != 1)
+    for (int i = threadIdx.x; i < min(n_tiles * a.m_blocks2 * 8, a.n_counters2); i += kMetaThreads) a.counters2[i] = 0;
+}
+
 // Pick the K split S in {1,2,4,8}.  Cost model in units of one K block of streaming: a unit costs its
 // K blocks plus a fixed overhead (pipeline fill, epilogue, and for S > 1 the partial-sum round trip);
 // the kernel takes ceil(units * S / SMs) rounds of such units.  Ties go to the smaller S.
@@ -89,9 +106,9 @@ __device__ __forceinline__ int choose_cut(const mf_meta_args& a, int units, int 
 
 __global__ void __launch_bounds__(kMetaThreads) expert_meta_kernel(const mf_meta_args a) {
   extern __shared__ int sm[];
-  const int L = a.L, K = a.K;
-  int* hist = sm;                       // [kMetaWarps][L]
-  int* cnt = hist + kMetaWarps * L;     // [L]
+  const int L = a.L, K = a.K, P = hist_pitch(a.L);
+  int* hist = sm;                       // [kMetaWarps][P]
+  int* cnt = hist + kMetaWarps * P;     // [L]
   int* offs = cnt + L;                  // [L]
   int* warp_sums = offs + L;            // [33]
 
@@ -99,7 +116,7 @@ __global__ void __launch_bounds__(kMetaThreads) expert_meta_kernel(const mf_meta
   unsigned long long* trace = (a.trace != nullptr && tid == 0) ? a.trace : nullptr;
   if (trace) trace[0] = global_timer_ns();
   grid_dep_launch();
-  for (int i = tid; i < kMetaWarps * L; i += kMetaThreads) hist[i] = 0;
+  for (int i = tid; i < kMetaWarps * P; i += kMetaThreads) hist[i] = 0;
   grid_dep_wait_cta();  // the dispatch kernel of this forward has completed (epoch, local rows)
   if (trace) trace[1] = global_timer_ns();
   const unsigned epoch = a.epoch ? *a.epoch : 0u;
@@ -109,10 +126,8 @@ __global__ void __launch_bounds__(kMetaThreads) expert_meta_kernel(const mf_meta
     if (!wait_flag_ge(a.flags + tid, epoch * (unsigned)(a.rows / a.R), a.wait_ns))
       report_status(a.status, kDispatchFlagTimeout, tid, 0, epoch);
   }
-  for (int i = tid; i < a.n_counters1; i += kMetaThreads) a.counters1[i] = 0;
-  for (int i = tid; i < a.n_counters2; i += kMetaThreads) a.counters2[i] = 0;
   __syncthreads();
-  if (trace) trace[2] = global_timer_ns();  // flags seen, counters cleared
+  if (trace) trace[2] = global_timer_ns();  // flags seen
 
   const int N = a.rows * K;
   int per = (N + kMetaWarps - 1) / kMetaWarps;
@@ -120,7 +135,7 @@ __global__ void __launch_bounds__(kMetaThreads) expert_meta_kernel(const mf_meta
   const int begin = min(N, warp * per), end = min(N, (warp + 1) * per);
   const uint8_t* recv = static_cast<const uint8_t*>(a.recv);
   const size_t meta_off = (size_t)a.H * 2;
-  int* my_hist = hist + warp * L;
+  int* my_hist = hist + warp * P;
 
   // Keys of a batch of kMetaBatch warp-wide steps are loaded together (independent loads in flight at
   // once) before the dependent match/count steps: the received rows are cold in cache when this kernel
@@ -163,8 +178,8 @@ __global__ void __launch_bounds__(kMetaThreads) expert_meta_kernel(const mf_meta
   for (int e = tid; e < L; e += kMetaThreads) {
     int run = 0;
     for (int w = 0; w < kMetaWarps; ++w) {
-      const int c = hist[w * L + e];
-      hist[w * L + e] = run;
+      const int c = hist[w * P + e];
+      hist[w * P + e] = run;
       run += c;
     }
     cnt[e] = run;
@@ -225,13 +240,14 @@ __global__ void __launch_bounds__(kMetaThreads) expert_meta_kernel(const mf_meta
       cols = 0;  // fixed slots of the kernel's n_max columns
     }
     a.plan[MF_PLAN_N_TILES] = nt;
-    a.plan[MF_PLAN_SPLIT1] = choose_cut(a, nt * a.m_blocks1, a.k_blocks1, slots1, 4, wide_cols);
-    a.plan[MF_PLAN_SPLIT2] = choose_cut(a, nt * a.m_blocks2, a.k_blocks2, slots2, 8, wide_cols);
+    warp_sums[36] = a.plan[MF_PLAN_SPLIT1] = choose_cut(a, nt * a.m_blocks1, a.k_blocks1, slots1, 4, wide_cols);
+    warp_sums[37] = a.plan[MF_PLAN_SPLIT2] = choose_cut(a, nt * a.m_blocks2, a.k_blocks2, slots2, 8, wide_cols);
     a.plan[MF_PLAN_N_ENTRIES] = n_entries;
     a.plan[MF_PLAN_SLOT_COLS] = cols;
     a.plan[MF_PLAN_VALID_ROWS] = warp_sums[35];
   }
   __syncthreads();
+  clear_counters(a, min(n_tiles, a.max_tiles), warp_sums[36], warp_sums[37]);
   if (trace) trace[4] = global_timer_ns();  // offsets, tiles and plan written
 
   // sweep 2: place the entries
@@ -276,9 +292,9 @@ __global__ void __launch_bounds__(kMetaThreads) expert_meta_kernel(const mf_meta
 // ---------------------------------------------------------------------------------------------------
 __global__ void __launch_bounds__(kMetaThreads) expert_meta_small_kernel(const mf_meta_args a) {
   extern __shared__ int sm[];
-  const int L = a.L, K = a.K;
-  int* hist = sm;                       // [kMetaWarps][L]
-  int* cnt = hist + kMetaWarps * L;     // [L]
+  const int L = a.L, K = a.K, P = hist_pitch(a.L);
+  int* hist = sm;                       // [kMetaWarps][P]
+  int* cnt = hist + kMetaWarps * P;     // [L]
   int* offs = cnt + L;                  // [L]
   int* warp_sums = offs + L;            // [40]
 
@@ -286,15 +302,16 @@ __global__ void __launch_bounds__(kMetaThreads) expert_meta_small_kernel(const m
   unsigned long long* trace = (a.trace != nullptr && tid == 0) ? a.trace : nullptr;
   if (trace) trace[0] = global_timer_ns();
   if (!a.late_launch) grid_dep_launch();
-  for (int i = tid; i < kMetaWarps * L; i += kMetaThreads) hist[i] = 0;
-  if (tid == 0) warp_sums[34] = warp_sums[35] = 0;
   const int N = a.rows * K;
   int per = (N + kMetaWarps - 1) / kMetaWarps;
   per = (per + 31) & ~31;               // <= 32 * kMetaBatch by the launcher's choice of this kernel
+  const int n_warps = (N + per - 1) / per;  // warps that hold slot words (one at a single token)
+  for (int i = tid; i < n_warps * P; i += kMetaThreads) hist[i] = 0;
+  if (tid == 0) warp_sums[34] = warp_sums[35] = 0;
   const int begin = min(N, warp * per), end = min(N, (warp + 1) * per);
   const uint8_t* recv = static_cast<const uint8_t*>(a.recv);
   const size_t meta_off = (size_t)a.H * 2;
-  int* my_hist = hist + warp * L;
+  int* my_hist = hist + warp * P;
   {
     // While the dispatch kernel runs: touch every page this kernel reads or writes after the wait.
     if (tid == 0) {
@@ -315,8 +332,7 @@ __global__ void __launch_bounds__(kMetaThreads) expert_meta_small_kernel(const m
       touch(a.entry_slot + i);
       touch(a.entry_w + i);
     }
-    if (tid < a.n_counters1) touch(a.counters1 + tid);
-    if (tid < a.n_counters2) touch(a.counters2 + tid);
+    if (tid == 0) touch(a.counters1 + a.n_counters1);
   }
   grid_dep_wait_cta();  // the dispatch kernel of this forward has completed (epoch, local rows)
   if (trace) trace[1] = global_timer_ns();
@@ -347,10 +363,7 @@ __global__ void __launch_bounds__(kMetaThreads) expert_meta_small_kernel(const m
       }
     }
   }
-  // the split-K arrival counters are cleared while those loads are in flight
-  for (int i = tid; i < a.n_counters1; i += kMetaThreads) a.counters1[i] = 0;
-  for (int i = tid; i < a.n_counters2; i += kMetaThreads) a.counters2[i] = 0;
-  if (trace) trace[6] = global_timer_ns();  // counter stores issued
+  if (trace) trace[6] = global_timer_ns();  // loads issued
 
   // warp histogram; pre[b] = entries of the same expert earlier in this warp's range
   const unsigned lt_mask = (1u << lane) - 1u;
@@ -391,14 +404,14 @@ __global__ void __launch_bounds__(kMetaThreads) expert_meta_small_kernel(const m
 
   // per expert: exclusive prefix over the warps (lane = source warp), total count
   for (int e = warp; e < L; e += kMetaWarps) {
-    const int c = hist[lane * L + e];
+    const int c = lane < n_warps ? hist[lane * P + e] : 0;
     int incl = c;
 #pragma unroll
     for (int off = 1; off < 32; off <<= 1) {
       const int o = __shfl_up_sync(0xffffffffu, incl, off);
       if (lane >= off) incl += o;
     }
-    hist[lane * L + e] = incl - c;
+    if (lane < n_warps) hist[lane * P + e] = incl - c;
     if (lane == 31) cnt[e] = incl;
   }
   if (!k_pow2) {
@@ -454,8 +467,8 @@ __global__ void __launch_bounds__(kMetaThreads) expert_meta_small_kernel(const m
       cols = 0;
     }
     a.plan[MF_PLAN_N_TILES] = nt;
-    a.plan[MF_PLAN_SPLIT1] = choose_cut(a, nt * a.m_blocks1, a.k_blocks1, slots1, 4, wide_cols);
-    a.plan[MF_PLAN_SPLIT2] = choose_cut(a, nt * a.m_blocks2, a.k_blocks2, slots2, 8, wide_cols);
+    warp_sums[36] = a.plan[MF_PLAN_SPLIT1] = choose_cut(a, nt * a.m_blocks1, a.k_blocks1, slots1, 4, wide_cols);
+    warp_sums[37] = a.plan[MF_PLAN_SPLIT2] = choose_cut(a, nt * a.m_blocks2, a.k_blocks2, slots2, 8, wide_cols);
     a.plan[MF_PLAN_N_ENTRIES] = n_entries;
     a.plan[MF_PLAN_SLOT_COLS] = cols;
     a.plan[MF_PLAN_VALID_ROWS] = warp_sums[35];
@@ -484,6 +497,8 @@ __global__ void __launch_bounds__(kMetaThreads) expert_meta_small_kernel(const m
       a.inv[i] = pos;
     }
   }
+  __syncthreads();  // the cuts are in warp_sums
+  clear_counters(a, min(n_tiles, a.max_tiles), warp_sums[36], warp_sums[37]);
   if (trace) trace[5] = global_timer_ns();  // entries placed
 }
 
@@ -549,13 +564,13 @@ __device__ __forceinline__ void meta_histogram(const mf_meta_args& a, MetaRange 
 
 __global__ void __launch_bounds__(kMetaThreads) expert_meta_count_kernel(const mf_meta_args a) {
   extern __shared__ int sm[];
-  const int L = a.L, K = a.K;
-  int* hist = sm;                    // [kMetaWarps][L]
-  int* warp_sums = hist + kMetaWarps * L;
+  const int L = a.L, K = a.K, P = hist_pitch(a.L);
+  int* hist = sm;                    // [kMetaWarps][P]
+  int* warp_sums = hist + kMetaWarps * P;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int cta = blockIdx.x, n_ctas = gridDim.x;
   grid_dep_launch();
-  for (int i = tid; i < kMetaWarps * L; i += kMetaThreads) hist[i] = 0;
+  for (int i = tid; i < kMetaWarps * P; i += kMetaThreads) hist[i] = 0;
   if (tid == 0) warp_sums[0] = 0;
   grid_dep_wait_cta();  // the dispatch kernel of this forward has completed (epoch, local rows)
   const unsigned epoch = a.epoch ? *a.epoch : 0u;
@@ -563,16 +578,14 @@ __global__ void __launch_bounds__(kMetaThreads) expert_meta_count_kernel(const m
     if (!wait_flag_ge(a.flags + tid, epoch * (unsigned)(a.rows / a.R), a.wait_ns))
       report_status(a.status, kDispatchFlagTimeout, tid, cta, epoch);
   }
-  for (int i = cta * kMetaThreads + tid; i < a.n_counters1; i += n_ctas * kMetaThreads) a.counters1[i] = 0;
-  for (int i = cta * kMetaThreads + tid; i < a.n_counters2; i += n_ctas * kMetaThreads) a.counters2[i] = 0;
   __syncthreads();
 
   const int N = a.rows * K;
-  meta_histogram(a, meta_range(N, n_ctas, cta, warp), lane, hist + warp * L);
+  meta_histogram(a, meta_range(N, n_ctas, cta, warp), lane, hist + warp * P);
   __syncthreads();
   for (int e = tid; e < L; e += kMetaThreads) {
     int total = 0;
-    for (int w = 0; w < kMetaWarps; ++w) total += hist[w * L + e];
+    for (int w = 0; w < kMetaWarps; ++w) total += hist[w * P + e];
     a.cta_hist[(size_t)cta * L + e] = total;
   }
   // slots per received row, and the number of rows with at least one
@@ -594,30 +607,30 @@ __global__ void __launch_bounds__(kMetaThreads) expert_meta_count_kernel(const m
 
 __global__ void __launch_bounds__(kMetaThreads) expert_meta_place_kernel(const mf_meta_args a) {
   extern __shared__ int sm[];
-  const int L = a.L, K = a.K;
-  int* hist = sm;                       // [kMetaWarps][L]
-  int* cnt = hist + kMetaWarps * L;     // [L] entries of the expert over all CTAs
+  const int L = a.L, K = a.K, P = hist_pitch(a.L);
+  int* hist = sm;                       // [kMetaWarps][P]
+  int* cnt = hist + kMetaWarps * P;     // [L] entries of the expert over all CTAs
   int* offs = cnt + L;                  // [L] first position of this CTA's entries of the expert
   int* warp_sums = offs + L;            // [40]
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int cta = blockIdx.x, n_ctas = gridDim.x;
   grid_dep_launch();
-  for (int i = tid; i < kMetaWarps * L; i += kMetaThreads) hist[i] = 0;
+  for (int i = tid; i < kMetaWarps * P; i += kMetaThreads) hist[i] = 0;
   if (tid == 0) warp_sums[34] = 0;
   grid_dep_wait_cta();  // the count launch has completed (and with it the dispatch kernel)
   __syncthreads();
 
   const int N = a.rows * K;
   const MetaRange range = meta_range(N, n_ctas, cta, warp);
-  int* my_hist = hist + warp * L;
+  int* my_hist = hist + warp * P;
   meta_histogram(a, range, lane, my_hist);
   __syncthreads();
 
   for (int e = tid; e < L; e += kMetaThreads) {
     int run = 0;
     for (int w = 0; w < kMetaWarps; ++w) {
-      const int c = hist[w * L + e];
-      hist[w * L + e] = run;
+      const int c = hist[w * P + e];
+      hist[w * P + e] = run;
       run += c;
     }
     int before = 0, total = 0;
@@ -666,12 +679,16 @@ __global__ void __launch_bounds__(kMetaThreads) expert_meta_place_kernel(const m
       cols = 0;
     }
     a.plan[MF_PLAN_N_TILES] = nt;
-    a.plan[MF_PLAN_SPLIT1] = choose_cut(a, nt * a.m_blocks1, a.k_blocks1, slots1, 4, wide_cols);
-    a.plan[MF_PLAN_SPLIT2] = choose_cut(a, nt * a.m_blocks2, a.k_blocks2, slots2, 8, wide_cols);
+    warp_sums[36] = a.plan[MF_PLAN_SPLIT1] = choose_cut(a, nt * a.m_blocks1, a.k_blocks1, slots1, 4, wide_cols);
+    warp_sums[37] = a.plan[MF_PLAN_SPLIT2] = choose_cut(a, nt * a.m_blocks2, a.k_blocks2, slots2, 8, wide_cols);
     a.plan[MF_PLAN_N_ENTRIES] = n_entries;
     a.plan[MF_PLAN_SLOT_COLS] = cols;
     a.plan[MF_PLAN_VALID_ROWS] = a.acc[0];
     a.acc[0] = 0;  // ready for the next forward (its count launch runs after this one)
+  }
+  if (cta == 0) {
+    __syncthreads();
+    clear_counters(a, min(n_tiles, a.max_tiles), warp_sums[36], warp_sums[37]);
   }
 
   for (int i0 = range.begin; i0 < range.end; i0 += 32 * kMetaBatch) {
@@ -708,7 +725,7 @@ extern "C" int mf_plan_split(int units, int k_blocks, int n_sms, int max_slots, 
 
 extern "C" int mf_expert_meta(const mf_meta_args* a, mf_stream_t stream) {
   if (!a || a->L < 1 || a->L > mf::kMetaThreads || a->R > mf::kMetaThreads || a->block_m < 1) return -1;
-  const size_t smem = ((size_t)mf::kMetaWarps * a->L + 2 * (size_t)a->L + 40) * sizeof(int);
+  const size_t smem = ((size_t)mf::kMetaWarps * mf::hist_pitch(a->L) + 2 * (size_t)a->L + 40) * sizeof(int);
   static size_t configured_all[64] = {};  // per device: the attribute belongs to (function, device)
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) dev = 0;

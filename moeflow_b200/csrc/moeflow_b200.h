@@ -83,7 +83,7 @@ typedef struct {
   // activations stored; the down kernel, given the same array as tile_wait, fetches a tile's activations as
   // soon as the count reaches tile_wait_target (= 4 * the gate/up GEMM's m_blocks) instead of waiting for the
   // whole gate/up grid, so SMs that the gate/up GEMM has left go straight on with down-projection units.
-  // The array must be zero before the gate/up kernel starts (mf_expert_meta clears it with the counters).
+  // The array must be zero before the gate/up kernel starts (mf_expert_meta clears it).
   int* tile_done;
   const int* tile_wait;
   int tile_wait_target;
@@ -188,8 +188,8 @@ typedef struct {
   int* tile_s;
   int* tile_n;
   int* plan;                 // MF_PLAN_WORDS
-  int* counters1;            // split-K counters to clear
-  int n_counters1;
+  int* counters1;            // arrival counters of cut gate/up units, then n_tile_done words that count tiles
+  int n_counters1;           // arrival counters (the tile words follow them)
   int* counters2;
   int n_counters2;
   int block_m;               // tokens per tile (= n_max of the GEMMs)
@@ -213,6 +213,7 @@ typedef struct {
   unsigned long long* trace; // optional [8] globaltimer stamps of CTA 0 (profiling aid), or NULL
   int late_launch;           // 1: the kernels that follow may only start when this one exits (no early launch)
   int plain_launch;          // 1: launched without programmatic serialization (starts when its predecessor has completed)
+  int n_tile_done;           // words at counters1 + n_counters1: finished gate/up quarters per token tile (cleared per tile in use)
 } mf_meta_args;
 int mf_expert_meta(const mf_meta_args* args, mf_stream_t stream);
 // The K-split rule of the metadata kernels, callable on the host (no device needed): the split in {1,2,4,8}

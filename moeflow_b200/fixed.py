@@ -431,7 +431,7 @@ class FixedEPLayer:
         if self.block_m not in (32, 64, 128, 256):
             raise ValueError("block_m must be 32, 64, 128 or 256")
         self.n_sms = int(self.gemm_kwargs.get("n_sms", sm_count(dev.index if dev.index is not None else 0)))
-        self.max_tiles = (N + self.block_m - 1) // self.block_m + L
+        self.max_tiles = N // self.block_m + min(L, N)  # every tile holds an entry, and full ones hold block_m
         self.out = torch.zeros(Cc, H, dtype=torch.bfloat16, device=dev)
         self.hit = torch.zeros(Cc, R, dtype=torch.uint8, device=dev)
         self._route_w = torch.zeros(Cc, K, dtype=torch.float32, device=dev)
@@ -455,7 +455,7 @@ class FixedEPLayer:
         # arrival counters of cut units: one per (unit, 32-row quarter) and, in the fp8 kernels with 128-column
         # tiles, per column group (two)
         n_cnt1 = self.max_tiles * mb1 * 8
-        # the tail of the first counter array (cleared with it by the metadata kernel) counts, per token tile, the
+        # the tail of the first counter array (cleared by the metadata kernel) counts, per token tile, the
         # gate/up quarters whose activations are final: the down GEMM starts a tile as soon as it is complete
         self._counters1 = torch.zeros(n_cnt1 + self.max_tiles, **i32)
         self._tile_done = self._counters1[n_cnt1:]
@@ -480,11 +480,11 @@ class FixedEPLayer:
             raise ValueError(f"unknown scoring function {cfg.scoring_func!r}")
         self._a_meta = S.MetaArgs(
             recv=self._recv_store.data_ptr(), pitch=self.pitch * 2, H=H, K=K, L=L, rows=R * Cc, R=R,
-            flags=self._disp_flags.data_ptr(), epoch=self._epoch.data_ptr(), offsets=self.offsets.data_ptr(),
+            flags=self._disp_flags.data_ptr() if R > 1 else None, epoch=self._epoch.data_ptr(), offsets=self.offsets.data_ptr(),
             entry_row=self.entry_row.data_ptr(), entry_slot=self.entry_slot.data_ptr(), entry_w=self.entry_w.data_ptr(),
             inv=self.inv.data_ptr(), tile_e=self.tile_e.data_ptr(), tile_s=self.tile_s.data_ptr(),
             tile_n=self.tile_n.data_ptr(), plan=self.plan.data_ptr(), counters1=self._counters1.data_ptr(),
-            n_counters1=self._counters1.numel(), counters2=self._counters2.data_ptr(),
+            n_counters1=n_cnt1, n_tile_done=self.max_tiles, counters2=self._counters2.data_ptr(),
             n_counters2=self._counters2.numel(), block_m=self.block_m, max_tiles=self.max_tiles, m_blocks1=mb1,
             k_blocks1=H // 64, m_blocks2=mb2, k_blocks2=I // 64, n_sms=self.n_sms,
             max_split_slots=self.max_split_slots, status=self.status.data_ptr(), wait_ns=self.wait_ns,
@@ -595,7 +595,7 @@ class FixedEPLayer:
         self._scratch_out = None
         self._a_combine = S.CombineArgs(
             ret=self.ret_recv.data_ptr(), hit=self.hit.data_ptr(), out=self.out.data_ptr(),
-            flags=self._ret_flags.data_ptr(), epoch=self._push_epoch.data_ptr(), R=R, C=Cc, H=H, rank=self.rank,
+            flags=self._ret_flags.data_ptr() if R > 1 else None, epoch=self._push_epoch.data_ptr(), R=R, C=Cc, H=H, rank=self.rank,
             ring=int(self.combine_mode == "bf16_ring"), status=self.status.data_ptr(), wait_ns=self.wait_ns,
         )
         self._tmap13 = self._tmap2 = None

@@ -159,6 +159,7 @@ class MetaArgs(C.Structure):
         ("trace", C.c_void_p),
         ("late_launch", C.c_int),
         ("plain_launch", C.c_int),
+        ("n_tile_done", C.c_int),
     ]
 
 
