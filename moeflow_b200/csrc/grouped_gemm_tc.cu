@@ -831,15 +831,15 @@ static int check_args(const mf_gemm_args* a, int n_max, int grid) {
 
 extern "C" {
 
-int mf_make_tile_tmap(void* out_tmap, const void* base, long long rows, long long k_elems, int elem_bytes,
-                      int box_rows) {
+int mf_make_pitched_tmap(void* out_tmap, const void* base, long long rows, long long k_elems, int elem_bytes,
+                         long long pitch_bytes, int box_rows) {
   auto fn = mf::get_encode_fn();
   if (!fn) return -10;
-  if ((reinterpret_cast<uintptr_t>(base) & 15) != 0 || ((k_elems * elem_bytes) & 15) != 0) return -11;
+  if ((reinterpret_cast<uintptr_t>(base) & 15) != 0 || (pitch_bytes & 15) != 0 || pitch_bytes < k_elems * elem_bytes) return -11;
   if (box_rows < 1 || box_rows > 256 || rows < 1) return -13;
   CUtensorMap tm;
   cuuint64_t dims[2] = {(cuuint64_t)k_elems, (cuuint64_t)rows};
-  cuuint64_t strides[1] = {(cuuint64_t)(k_elems * elem_bytes)};
+  cuuint64_t strides[1] = {(cuuint64_t)pitch_bytes};
   cuuint32_t box[2] = {(cuuint32_t)(128 / elem_bytes), (cuuint32_t)box_rows};
   cuuint32_t estr[2] = {1, 1};
   CUtensorMapDataType dt = elem_bytes == 2 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_UINT8;
@@ -848,6 +848,11 @@ int mf_make_tile_tmap(void* out_tmap, const void* base, long long rows, long lon
   if (r != CUDA_SUCCESS) return -12 - (int)r * 100;
   memcpy(out_tmap, &tm, sizeof(tm));
   return 0;
+}
+
+int mf_make_tile_tmap(void* out_tmap, const void* base, long long rows, long long k_elems, int elem_bytes,
+                      int box_rows) {
+  return mf_make_pitched_tmap(out_tmap, base, rows, k_elems, elem_bytes, k_elems * elem_bytes, box_rows);
 }
 
 int mf_make_weight_tmap(void* out_tmap, const void* w, long long rows, long long k_elems, int elem_bytes) {

@@ -99,6 +99,33 @@ int mf_make_tile_tmap(void* out_tmap, const void* base, long long rows, long lon
                       int box_rows);
 int mf_make_weight_tmap(void* out_tmap, const void* w, long long rows, long long k_elems, int elem_bytes);
 
+// The same for rows `pitch_bytes` apart (a multiple of 16).  Boxes may reach past the last row: those rows read zero.
+int mf_make_pitched_tmap(void* out_tmap, const void* base, long long rows, long long k_elems, int elem_bytes,
+                         long long pitch_bytes, int box_rows);
+
+// ---- dense projections of a decode step ------------------------------------------------------------------
+// out[t, r] = x[t, :] . W[r, :], bf16 operands, fp32 sums; any number of tokens, tiles of 64.  gate_up: W holds the
+// gate rows and, up_row_offset further, the up rows; out is silu(min(gate, limit)) * clamp(up, +-limit).
+// tmap_w: mf_make_tile_tmap over W with boxes of 128 rows (64 for gate_up).  n_sms sizes the cut along K.
+typedef struct {
+  const void* x;             // [T, 64 * k_blocks] bf16, rows x_pitch bytes apart, 16-byte aligned
+  long long x_pitch;
+  int T;
+  int k_blocks;              // K / 64
+  int row_blocks;            // weight rows / 128; gate_up: outputs / 64
+  int up_row_offset;
+  void* out;                 // bf16 (fp32 with out_fp32) [T, out_pitch]
+  long long out_pitch;       // elements
+  int out_fp32;
+  int out_cols;              // > 0: only output columns below this are stored (weight rows padded to a block)
+  float limit;               // SwiGLU clamp (<= 0: none)
+  const void* residual;      // optional bf16 [T, residual_pitch]: added to the rounded product, rounded again
+  long long residual_pitch;  // elements
+  unsigned long long* status;
+  unsigned long long wait_ns;
+} mf_skinny_args;
+int mf_skinny_gemm(const void* tmap_w, const mf_skinny_args* args, int gate_up, int n_sms, mf_stream_t stream);
+
 int mf_gemm_gate_up(const void* tmap, const mf_gemm_args* args, int n_max, int grid, mf_stream_t stream);
 int mf_gemm_down(const void* tmap, const mf_gemm_args* args, int n_max, int grid, mf_stream_t stream);
 int mf_gemm_smem_bytes(int gate_up, int n_max);

@@ -3,9 +3,8 @@
 Components (all inference-only, bf16, one process per GPU, attention TP=1 with data-parallel tokens,
 DP = EP = world):
 
-``SharedExpert``   the always-on SwiGLU MLP, run through the same tcgen05 grouped GEMM kernels as the
-                   routed experts with a static one-expert plan;
-``MoEBlock``       RMSNorm (sm_100a kernel) -> router logits (``RouterLogits``: the tcgen05 grouped kernel, fp32 output) ->
+``SharedExpert``   the always-on SwiGLU MLP, on the tcgen05 kernel for dense projections of a decode step;
+``MoEBlock``       RMSNorm (sm_100a kernel) -> router logits (``RouterLogits``: the same dense kernel, fp32 output) ->
                    routed experts (``FixedEPLayer``: fused route+dispatch, expert GEMMs, return push,
                    combine) + shared expert -> residual;
 ``Attention``      grouped-query attention over a static KV cache for single-token decode steps, with
@@ -21,7 +20,6 @@ shape can be measured and tested without that engine.
 
 from __future__ import annotations
 
-import ctypes as C
 import math
 from dataclasses import dataclass
 
@@ -60,100 +58,44 @@ class SharedExpert:
         self.cuda = w13.is_cuda and w13.dtype == torch.bfloat16 and self.hidden % 128 == 0 and self.inter % 128 == 0
         if not self.cuda:
             return
-        from ..ops import _lib
-        from ..ops.grouped_gemm import plan_from_offsets
-        from ..ops.kernels import make_weight_tmap, sm_count
+        from ..ops.dense import DenseProjection
 
         dev = w13.device
-        self._lib = _lib
-        self.n_sms = sm_count(dev.index or 0)
-        n_tiles = (capacity + block_m - 1) // block_m
-
-        # One expert has few weight blocks (12 and 32 at the GLM shape): the stream-K cut (plan word 0) lays the
-        # K steps of all units end to end and gives every SM the same share of the weight stream.
-        self.tp = plan_from_offsets([0, capacity], block_m, dev, split1=0, split2=0)
         self.act = torch.zeros(capacity, self.inter, dtype=torch.bfloat16, device=dev)
         self.out = torch.zeros(capacity, self.hidden, dtype=torch.bfloat16, device=dev)
         self.status = torch.zeros(1, dtype=torch.int64, device=dev)
-        self._x = torch.zeros(capacity, self.hidden, dtype=torch.bfloat16, device=dev)
-        self._tm13 = make_weight_tmap(self.w13.view(1, 2 * self.inter, self.hidden))
-        self._tm2 = make_weight_tmap(self.w2.view(1, self.hidden, self.inter))
-        slots = 2 * self.n_sms  # stream-K: two partial tiles per CTA
-        self._scratch = torch.zeros(slots * 2 * block_m * 128, dtype=torch.float32, device=dev)
-        self._counters = torch.zeros(self.tp.n_tiles * max(self.inter, self.hidden) // 128 * 4, dtype=torch.int32, device=dev)
-        common = dict(tile_e=self.tp.tile_e.data_ptr(), tile_s=self.tp.tile_s.data_ptr(), tile_n=self.tp.tile_n.data_ptr(),
-                      plan=self.tp.plan.data_ptr(), partial=self._scratch.data_ptr(), counters=self._counters.data_ptr(),
-                      max_split_slots=slots, status=self.status.data_ptr(), wait_ns=2_000_000_000,
-                      partial_floats=self._scratch.numel(), n_counters=self._counters.numel(),
-                      max_tiles=self.tp.tile_e.numel())
-        self._a1 = _lib.GemmArgs(b_base=self._x.data_ptr(), b_pitch=self.hidden * 2, b_index=None, split_word=_lib.PLAN_SPLIT1,
-                                 m_blocks=self.inter // 128, k_blocks=self.hidden // 64, rows_per_expert=2 * self.inter,
-                                 up_row_offset=self.inter, out=self.act.data_ptr(), out_pitch=self.inter, row_scale=None,
-                                 limit=float(limit) if limit is not None else 0.0, round_h=0, **common)
-        self._a2 = _lib.GemmArgs(b_base=self.act.data_ptr(), b_pitch=self.inter * 2, b_index=None, split_word=_lib.PLAN_SPLIT2,
-                                 m_blocks=self.hidden // 128, k_blocks=self.inter // 64, rows_per_expert=self.hidden,
-                                 up_row_offset=0, out=self.out.data_ptr(), out_pitch=self.hidden, row_scale=None, limit=0.0,
-                                 round_h=0, **common)
+        self._gate_up = DenseProjection(self.w13, gate_up=True, limit=limit, status=self.status)
+        self._down = DenseProjection(self.w2, status=self.status)
 
     def __call__(self, x: torch.Tensor) -> torch.Tensor:
         t = x.shape[0]
         if not self.cuda:
             h = swiglu_clamp(x @ self.w13.transpose(0, 1), self.limit)
             return h @ self.w2.transpose(0, 1)
-        self._x[:t].copy_(x)
-        lib, s = self._lib.lib(), self._lib.stream_ptr()
-        self._lib.check(lib.mf_gemm_gate_up(self._tm13, C.byref(self._a1), self.block_m, self.n_sms, s), "shared gate/up")
-        self._lib.check(lib.mf_gemm_down(self._tm2, C.byref(self._a2), self.block_m, self.n_sms, s), "shared down")
-        return self.out[:t]
+        return self._down(self._gate_up(x, self.act), self.out)
 
 
 class RouterLogits:
-    """Router logits ``h . gate_w^T`` as fp32 ``[T, E]`` on the grouped down-projection kernel (tcgen05, bf16
-    operands, fp32 accumulation and fp32 output): the gate matrix is one "expert" whose rows are padded to a
-    multiple of 128, K is split so that the few weight blocks spread over several SMs, and only the E real
-    columns are stored.  With it the MoE block issues no library GEMM."""
+    """Router logits ``h . gate_w^T`` as fp32 ``[T, E]`` on the dense projection kernel (tcgen05, bf16 operands, fp32
+    accumulation and fp32 output): the gate matrix's rows are padded to a multiple of 128 and only the E real columns
+    are stored.  With it the MoE block issues no library GEMM."""
 
     def __init__(self, gate_w: torch.Tensor, capacity: int, block_m: int = 64):
-        from ..ops import _lib
-        from ..ops.grouped_gemm import plan_from_offsets
-        from ..ops.kernels import make_weight_tmap, sm_count
+        from ..ops.dense import DenseProjection
 
         E, H = gate_w.shape
         dev = gate_w.device
         if H % 64:
             raise ValueError("hidden size must be a multiple of 64")
-        self._lib, self.E, self.H, self.C, self.block_m = _lib, E, H, capacity, block_m
-        rows = (E + 127) // 128 * 128
-        self.w = torch.zeros(1, rows, H, dtype=torch.bfloat16, device=dev)
-        self.w[0, :E] = gate_w.to(torch.bfloat16)
-        self.n_sms = sm_count(dev.index or 0)
-        k_blocks = H // 64
-        split = max(s for s in (1, 2, 4, 8) if k_blocks % s == 0 and k_blocks // s >= 2 or s == 1)
-        self.tp = plan_from_offsets([0, capacity], block_m, dev, split2=split)
-        m_blocks = rows // 128
-        slots = self.tp.n_tiles * m_blocks * split
-        self._x = torch.zeros(max(capacity, block_m), H, dtype=torch.bfloat16, device=dev)
+        self.E, self.H, self.C, self.block_m = E, H, capacity, block_m
+        self.w = torch.zeros((E + 127) // 128 * 128, H, dtype=torch.bfloat16, device=dev)
+        self.w[:E] = gate_w.to(torch.bfloat16)
         self.logits = torch.zeros(capacity, E, dtype=torch.float32, device=dev)
         self.status = torch.zeros(1, dtype=torch.int64, device=dev)
-        self._scratch = torch.zeros(max(1, slots) * block_m * 128, dtype=torch.float32, device=dev)
-        self._counters = torch.zeros(self.tp.n_tiles * m_blocks * 8, dtype=torch.int32, device=dev)
-        self._tmap = make_weight_tmap(self.w)
-        self._args = _lib.GemmArgs(
-            b_base=self._x.data_ptr(), b_pitch=H * 2, b_index=None, tile_e=self.tp.tile_e.data_ptr(),
-            tile_s=self.tp.tile_s.data_ptr(), tile_n=self.tp.tile_n.data_ptr(), plan=self.tp.plan.data_ptr(),
-            split_word=_lib.PLAN_SPLIT2, m_blocks=m_blocks, k_blocks=k_blocks, rows_per_expert=rows, up_row_offset=0,
-            out=self.logits.data_ptr(), out_pitch=E, row_scale=None, partial=self._scratch.data_ptr(),
-            counters=self._counters.data_ptr(), max_split_slots=slots, limit=0.0, round_h=0, status=self.status.data_ptr(),
-            wait_ns=2_000_000_000, partial_floats=self._scratch.numel(), n_counters=self._counters.numel(),
-            max_tiles=self.tp.tile_e.numel(), out_fp32=1, out_cols=E,
-        )
+        self._project = DenseProjection(self.w, out_cols=E, status=self.status)
 
     def __call__(self, h: torch.Tensor) -> torch.Tensor:
-        t = h.shape[0]
-        self._x[:t].copy_(h)
-        self._lib.check(self._lib.lib().mf_gemm_down(self._tmap, C.byref(self._args), self.block_m, self.n_sms,
-                                                     self._lib.stream_ptr()), "router logits")
-        return self.logits[:t]
+        return self._project(h, self.logits)
 
 
 class MoEBlock:

@@ -82,6 +82,26 @@ class GemmArgs(C.Structure):
     ]
 
 
+class SkinnyArgs(C.Structure):
+    _fields_ = [
+        ("x", C.c_void_p),
+        ("x_pitch", C.c_longlong),
+        ("T", C.c_int),
+        ("k_blocks", C.c_int),
+        ("row_blocks", C.c_int),
+        ("up_row_offset", C.c_int),
+        ("out", C.c_void_p),
+        ("out_pitch", C.c_longlong),
+        ("out_fp32", C.c_int),
+        ("out_cols", C.c_int),
+        ("limit", C.c_float),
+        ("residual", C.c_void_p),
+        ("residual_pitch", C.c_longlong),
+        ("status", C.c_void_p),
+        ("wait_ns", C.c_ulonglong),
+    ]
+
+
 class DispatchArgs(C.Structure):
     _fields_ = [
         ("x", C.c_void_p),
@@ -228,6 +248,8 @@ def lib() -> C.CDLL:
     sigs = {
         "mf_make_weight_tmap": [P, P, LL, LL, I],
         "mf_make_tile_tmap": [P, P, LL, LL, I, I],
+        "mf_make_pitched_tmap": [P, P, LL, LL, I, LL, I],
+        "mf_skinny_gemm": [P, C.POINTER(SkinnyArgs), I, I, P],
         "mf_gemm_gate_up": [P, C.POINTER(GemmArgs), I, I, P],
         "mf_gemm_down": [P, C.POINTER(GemmArgs), I, I, P],
         "mf_gemm_smem_bytes": [I, I],
