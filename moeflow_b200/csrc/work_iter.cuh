@@ -2,12 +2,19 @@
 //
 // A unit is (token tile, 128-row weight block); it needs k_blocks K steps.  The plan word of a GEMM says how
 // the units are cut along K:
-//   * K split S in {1, 2, 4, 8}: every unit is cut into S equal segments, dealt to the CTAs round-robin;
-//   * stream-K (plan word 0): the units' K steps are laid end to end and every CTA takes one contiguous share
-//     of that line, so all CTAs stream the same number of weight bytes whatever the unit count; a unit that
+//   * K split S in {1, 2, 4, 8}: every unit is cut into S equal segments, handed out one by one;
+//   * stream-K (plan word 0): the units' K steps are laid end to end and every CTA takes one contiguous
+//     share of that line, so all CTAs stream the same number of weight bytes whatever the unit count; a unit that
 //     straddles CTA boundaries is cut there.
-// Every warp role of a CTA builds its own iterator from the same plan words and walks the same sequence of
-// segments, so the roles stay in step without talking to each other.
+// With a counter (mf_gemm_args.sched) the segments of a K split go to whichever CTA asks next.  SMs do not get equal
+// shares of the memory rate: with a fixed round-robin the fastest CTA of a weight-streaming GEMM was done a third
+// before the slowest, and the down GEMM's CTAs that took the free SMs had a fixed share as well (8 tokens on 288 e4m3
+// experts: the last 40 % of the bytes ran at two thirds of the rate).  Without a counter segments are dealt
+// round-robin.  A segment's result does not depend on who computes it.
+//
+// Only the weight producer warp decides what comes next; it also fetches the tile's words.  It publishes each segment
+// in a small ring in shared memory, about one segment ahead, and the other roles read it there: no global loads and no
+// index arithmetic in them between two units.
 #pragma once
 
 #include "common.cuh"
@@ -17,15 +24,14 @@ namespace mf {
 
 // One piece of work of a CTA: `nkb` K steps of unit (tt, mb) starting at K block kb0.
 struct Seg {
-  int unit, tt, mb;
+  int unit, tt, mb;          // unit < 0: no more work
   int e, row_start, n_rows;  // the token tile: expert, first entry, entries
   int kb0, nkb;
   int nseg, seg;             // segments of this unit and this one's index in K order (nseg == 1: whole unit)
   int c_first;               // stream-K: CTA that holds segment 0 of the unit
+  int pad;
 };
 
-// Enumerates the segments of CTA `cta`.  Every warp role builds its own iterator from the same plan words
-// and therefore walks the same sequence.
 struct WorkIter {
   const mf_gemm_args* a;
   int n_max, m_blocks, KB, split, stream;
@@ -33,8 +39,7 @@ struct WorkIter {
   int cta, G;        // this CTA, CTAs that take part
   long long W;       // stream-K: units * KB
   long long w, w1;   // stream-K: cursor and end of this CTA's share
-  int u;             // K split: next (unit, split) index
-  bool bad_tile;     // a tile wider than the kernel's token tile was met (and skipped)
+  int u;             // K split: this CTA's next (unit, split) index
 
   __device__ __forceinline__ long long share_begin(int c) const { return (long long)c * W / G; }
   // CTA holding K step x of the line (the largest c with share_begin(c) <= x)
@@ -51,7 +56,6 @@ struct WorkIter {
     cta = cta_;
     W = (long long)units * KB;
     G = stream ? (int)(W < (long long)grid ? W : (long long)grid) : grid;
-    bad_tile = false;
     u = cta;
     w = w1 = 0;
     if (stream && cta < G) {
@@ -60,38 +64,49 @@ struct WorkIter {
     }
   }
 
-  __device__ __forceinline__ bool next(Seg& s) {
-    while (true) {
-      if (stream) {
-        if (w >= w1) return false;
-        s.unit = (int)(w / KB);
-        s.kb0 = (int)(w - (long long)s.unit * KB);
-        const long long left = w1 - w;
-        s.nkb = (KB - s.kb0) < left ? (KB - s.kb0) : (int)left;
-        w += s.nkb;
-        const long long x0 = (long long)s.unit * KB;
-        s.c_first = cta_of(x0);
-        s.nseg = cta_of(x0 + KB - 1) - s.c_first + 1;
-        s.seg = cta - s.c_first;
-      } else {
-        if (u >= units * split) return false;
-        const int ks = u % split;
-        s.unit = u / split;
-        u += G;
-        s.nkb = KB / split;
-        s.kb0 = ks * s.nkb;
-        s.nseg = split;
-        s.seg = ks;
-        s.c_first = 0;
-      }
-      s.tt = s.unit / m_blocks;
-      s.mb = s.unit - s.tt * m_blocks;
-      s.e = __ldcg(a->tile_e + s.tt);
-      s.row_start = __ldcg(a->tile_s + s.tt);
-      s.n_rows = __ldcg(a->tile_n + s.tt);
-      if ((unsigned)s.n_rows <= (unsigned)n_max) return true;
-      bad_tile = true;  // a plan built for wider tiles than this kernel: skip the segment, every role alike
+  // The segment at the cursor, its tile words still in flight (nothing here waits for the three loads).
+  __device__ __forceinline__ bool locate(Seg& s) {
+    if (stream) {
+      if (w >= w1) return false;
+      s.unit = (int)(w / KB);
+      s.kb0 = (int)(w - (long long)s.unit * KB);
+      const long long left = w1 - w;
+      s.nkb = (KB - s.kb0) < left ? (KB - s.kb0) : (int)left;
+      w += s.nkb;
+      const long long x0 = (long long)s.unit * KB;
+      s.c_first = cta_of(x0);
+      s.nseg = cta_of(x0 + KB - 1) - s.c_first + 1;
+      s.seg = cta - s.c_first;
+    } else {
+      if (u >= units * split) return false;
+      const int ks = u % split;
+      s.unit = u / split;
+      s.nkb = KB / split;
+      s.kb0 = ks * s.nkb;
+      s.nseg = split;
+      s.seg = ks;
+      s.c_first = 0;
     }
+    s.tt = s.unit / m_blocks;
+    s.mb = s.unit - s.tt * m_blocks;
+    s.e = __ldcg(a->tile_e + s.tt);
+    s.row_start = __ldcg(a->tile_s + s.tt);
+    s.n_rows = __ldcg(a->tile_n + s.tt);
+    return true;
+  }
+  // Moves the cursor of a K split (stream-K moves in locate).  The counter's answer may still be in flight on return.
+  __device__ __forceinline__ void step() {
+    if (stream) return;
+    if (a->sched != nullptr) {
+      int t = 0;
+      if (lane_id() == 0) t = atomicAdd(a->sched, 1);
+      u = t;
+    } else {
+      u += G;
+    }
+  }
+  __device__ __forceinline__ void stepped() {  // ... and is here now
+    if (!stream && a->sched != nullptr) u = G + __shfl_sync(0xffffffffu, u, 0);
   }
 
   // Partial-sum slot of segment `sg` of the unit of `s`.  K split: slots are (unit, segment).  Stream-K: every
@@ -105,6 +120,116 @@ struct WorkIter {
   __device__ __forceinline__ long long slots_needed() const {
     if (stream) return 2ll * G;
     return split > 1 ? (long long)units * split : 0;
+  }
+};
+
+// The ring of published segments.
+constexpr int kSegRing = 4;
+struct SegRing {
+  Seg slot[kSegRing];
+  uint64_t full[kSegRing], empty[kSegRing];
+  __device__ __forceinline__ void init(int consumers) {
+    for (int i = 0; i < kSegRing; ++i) {
+      mbar_init(&full[i], 1);
+      mbar_init(&empty[i], consumers);
+    }
+  }
+};
+
+// Consumer side (one per warp, the whole warp calls).
+struct SegReader {
+  SegRing* ring;
+  volatile int* abort_flag;
+  unsigned long long wait_ns;
+  int i = 0;
+  uint32_t phase = 0;
+  __device__ __forceinline__ SegReader(SegRing* r, volatile int* abort, unsigned long long ns)
+      : ring(r), abort_flag(abort), wait_ns(ns) {}
+  // The next segment; false at the end of the work, or with `ok` cleared when the wait ran out.
+  __device__ __forceinline__ bool next(Seg& s, bool& ok) {
+    ok = __all_sync(0xffffffffu, mbar_wait_bounded(&ring->full[i], phase, abort_flag, wait_ns));
+    if (!ok) return false;
+    const int4* p = reinterpret_cast<const int4*>(&ring->slot[i]);
+    const int4 x = p[0], y = p[1], z = p[2];
+    s.unit = x.x;
+    s.tt = x.y;
+    s.mb = x.z;
+    s.e = x.w;
+    s.row_start = y.x;
+    s.n_rows = y.y;
+    s.kb0 = y.z;
+    s.nkb = y.w;
+    s.nseg = z.x;
+    s.seg = z.y;
+    s.c_first = z.z;
+    __syncwarp();
+    if (lane_id() == 0) mbar_arrive(&ring->empty[i]);
+    if (++i == kSegRing) {
+      i = 0;
+      phase ^= 1u;
+    }
+    return s.unit >= 0;
+  }
+};
+
+// Producer side (the weight producer warp, the whole warp calls).  The segment behind the current one is prepared in
+// three steps spread over the current one's first K blocks: ask the counter, fetch the tile's words, publish.
+struct SegFeed {
+  WorkIter it;
+  SegRing* ring;
+  volatile int* abort_flag;
+  unsigned long long wait_ns;
+  Seg nx;
+  int i = 0, stage = 0;
+  uint32_t phase = 0;
+  bool have = false, bad_tile = false, ok = true;
+  __device__ __forceinline__ SegFeed(const WorkIter& w, SegRing* r, volatile int* abort, unsigned long long ns)
+      : it(w), ring(r), abort_flag(abort), wait_ns(ns) {}
+
+  __device__ __forceinline__ void publish() {
+    ok = ok && __all_sync(0xffffffffu, mbar_wait_bounded(&ring->empty[i], phase ^ 1u, abort_flag, wait_ns));
+    if (ok && lane_id() == 0) {
+      int4* p = reinterpret_cast<int4*>(&ring->slot[i]);
+      p[0] = make_int4(have ? nx.unit : -1, nx.tt, nx.mb, nx.e);
+      p[1] = make_int4(nx.row_start, nx.n_rows, nx.kb0, nx.nkb);
+      p[2] = make_int4(nx.nseg, nx.seg, nx.c_first, 0);
+      mbar_arrive(&ring->full[i]);
+    }
+    __syncwarp();
+    if (++i == kSegRing) {
+      i = 0;
+      phase ^= 1u;
+    }
+  }
+  // One of the three steps; after the third the next segment is in `nx` (have == false: there is none).
+  __device__ __forceinline__ void advance() {
+    if (stage == 0) {
+      it.step();
+    } else if (stage == 1) {
+      it.stepped();
+      have = it.locate(nx);
+    } else if (stage == 2) {
+      // a plan built for wider tiles than this kernel: such segments are skipped (and reported)
+      while (have && (unsigned)nx.n_rows > (unsigned)it.n_max) {
+        bad_tile = true;
+        it.step();
+        it.stepped();
+        have = it.locate(nx);
+      }
+      publish();
+    }
+    if (stage < 3) ++stage;
+  }
+  __device__ __forceinline__ bool first(Seg& s) {
+    have = it.locate(nx);
+    stage = 2;
+    return next(s);
+  }
+  __device__ __forceinline__ bool next(Seg& s) {
+    while (stage < 3) advance();
+    s = nx;
+    stage = 0;
+    return have && ok;
   }
 };
 
