@@ -18,6 +18,7 @@
 // (moeflow/kernels/grouped_gemm.py:83-98).
 #include "common.cuh"
 #include "moeflow_b200.h"
+#include "quant.cuh"
 
 namespace mf {
 
@@ -243,6 +244,7 @@ __global__ void __launch_bounds__(kMetaThreads) expert_meta_kernel(const mf_meta
     warp_sums[36] = a.plan[MF_PLAN_SPLIT1] = choose_cut(a, nt * a.m_blocks1, a.k_blocks1, slots1, 4, wide_cols);
     warp_sums[37] = a.plan[MF_PLAN_SPLIT2] = choose_cut(a, nt * a.m_blocks2, a.k_blocks2, slots2, 8, wide_cols);
     a.plan[MF_PLAN_N_ENTRIES] = n_entries;
+    a.plan[MF_PLAN_NEXT1] = a.plan[MF_PLAN_NEXT2] = 0;
     a.plan[MF_PLAN_SLOT_COLS] = cols;
     a.plan[MF_PLAN_VALID_ROWS] = warp_sums[35];
   }
@@ -290,8 +292,35 @@ __global__ void __launch_bounds__(kMetaThreads) expert_meta_kernel(const mf_meta
 // the warps runs as warp scans (one expert per warp at a time) instead of one thread per expert.
 // Identical output to expert_meta_kernel; about a quarter of its latency.
 // ---------------------------------------------------------------------------------------------------
+// Received rows -> e4m3 (layers with block-scaled experts), by the CTAs behind the first one: the two jobs read the same
+// rows and neither needs the other, so the quantiser costs no launch and no time of its own.
+__device__ __forceinline__ void quantise_received_rows(const mf_meta_args& a) {
+  grid_dep_wait_cta();
+  if (a.flags != nullptr && threadIdx.x < a.R) {
+    const unsigned epoch = a.epoch ? __ldcg(a.epoch) : 0u;
+    if (!wait_flag_ge(a.flags + threadIdx.x, epoch * (unsigned)(a.rows / a.R), a.wait_ns))
+      report_status(a.status, kDispatchFlagTimeout, threadIdx.x, blockIdx.x, epoch);
+  }
+  __syncthreads();
+  const int chunks = a.H / 8, groups = a.H / 128;  // chunks: a multiple of 16, so a group's threads work on one row
+  const long long total = (long long)a.rows * chunks;
+  const uint8_t* recv = static_cast<const uint8_t*>(a.recv);
+  const size_t valid_off = (size_t)a.H * 2 + (size_t)8 * a.K;
+  for (long long i = (long long)(blockIdx.x - 1) * kMetaThreads + threadIdx.x; i < total; i += (long long)(gridDim.x - 1) * kMetaThreads) {
+    const int row = (int)(i / chunks), c = (int)(i - (long long)row * chunks);
+    const uint8_t* src = recv + (size_t)row * a.pitch;
+    if (__ldcg(reinterpret_cast<const int*>(src + valid_off)) == 0) continue;
+    quant_chunk(src, c, a.xq + (size_t)row * a.H, a.xs + (size_t)row * groups);
+  }
+}
+
 __global__ void __launch_bounds__(kMetaThreads) expert_meta_small_kernel(const mf_meta_args a) {
   extern __shared__ int sm[];
+  if (blockIdx.x > 0) {
+    if (!a.late_launch) grid_dep_launch();
+    quantise_received_rows(a);
+    return;
+  }
   const int L = a.L, K = a.K, P = hist_pitch(a.L);
   int* hist = sm;                       // [kMetaWarps][P]
   int* cnt = hist + kMetaWarps * P;     // [L]
@@ -470,6 +499,7 @@ __global__ void __launch_bounds__(kMetaThreads) expert_meta_small_kernel(const m
     warp_sums[36] = a.plan[MF_PLAN_SPLIT1] = choose_cut(a, nt * a.m_blocks1, a.k_blocks1, slots1, 4, wide_cols);
     warp_sums[37] = a.plan[MF_PLAN_SPLIT2] = choose_cut(a, nt * a.m_blocks2, a.k_blocks2, slots2, 8, wide_cols);
     a.plan[MF_PLAN_N_ENTRIES] = n_entries;
+    a.plan[MF_PLAN_NEXT1] = a.plan[MF_PLAN_NEXT2] = 0;
     a.plan[MF_PLAN_SLOT_COLS] = cols;
     a.plan[MF_PLAN_VALID_ROWS] = warp_sums[35];
   }
@@ -682,6 +712,7 @@ __global__ void __launch_bounds__(kMetaThreads) expert_meta_place_kernel(const m
     warp_sums[36] = a.plan[MF_PLAN_SPLIT1] = choose_cut(a, nt * a.m_blocks1, a.k_blocks1, slots1, 4, wide_cols);
     warp_sums[37] = a.plan[MF_PLAN_SPLIT2] = choose_cut(a, nt * a.m_blocks2, a.k_blocks2, slots2, 8, wide_cols);
     a.plan[MF_PLAN_N_ENTRIES] = n_entries;
+    a.plan[MF_PLAN_NEXT1] = a.plan[MF_PLAN_NEXT2] = 0;
     a.plan[MF_PLAN_SLOT_COLS] = cols;
     a.plan[MF_PLAN_VALID_ROWS] = a.acc[0];
     a.acc[0] = 0;  // ready for the next forward (its count launch runs after this one)
@@ -745,6 +776,7 @@ extern "C" int mf_expert_meta(const mf_meta_args* a, mf_stream_t stream) {
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   if (a->n_ctas > 1) {
     if (!a->cta_hist || !a->acc || a->n_ctas > 1024) return -2;
+    if (a->xq != nullptr) return -4;  // only the one-pass kernel quantises
     cudaError_t e = mf::launch_kernel(mf::expert_meta_count_kernel, dim3(a->n_ctas), dim3(mf::kMetaThreads), smem, s,
                                       !a->plain_launch, *a);
     if (e != cudaSuccess) return (int)e;
@@ -753,7 +785,16 @@ extern "C" int mf_expert_meta(const mf_meta_args* a, mf_stream_t stream) {
   }
   // one CTA: the register-resident one-pass kernel when every warp's range fits one batch of steps
   const long long n_words = (long long)a->rows * a->K;
-  if (n_words <= (long long)mf::kMetaThreads * mf::kMetaBatch)
-    return (int)mf::launch_kernel(mf::expert_meta_small_kernel, dim3(1), dim3(mf::kMetaThreads), smem, s, !a->plain_launch, *a);
+  if (n_words <= (long long)mf::kMetaThreads * mf::kMetaBatch) {
+    int quant_ctas = 0;
+    if (a->xq != nullptr) {
+      if (!a->xs || a->H % 128 != 0) return -3;
+      const long long ctas = ((long long)a->rows * (a->H / 8) + mf::kMetaThreads - 1) / mf::kMetaThreads;
+      quant_ctas = (int)(ctas < a->n_sms - 1 ? ctas : a->n_sms > 1 ? a->n_sms - 1 : 1);
+    }
+    return (int)mf::launch_kernel(mf::expert_meta_small_kernel, dim3(1 + quant_ctas), dim3(mf::kMetaThreads), smem, s,
+                                  !a->plain_launch, *a);
+  }
+  if (a->xq != nullptr) return -4;  // only the one-pass kernel quantises
   return (int)mf::launch_kernel(mf::expert_meta_kernel, dim3(1), dim3(mf::kMetaThreads), smem, s, !a->plain_launch, *a);
 }

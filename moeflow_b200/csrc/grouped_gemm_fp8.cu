@@ -11,32 +11,42 @@
 //
 // The weight block of a unit (128 rows) is exactly one scale-block row, and one K block of 128 bytes is
 // one TMA box row and one scale-block column, so a unit needs one weight scale per K block (two for
-// gate/up) and one activation scale per token and K block; the epilogue warps preload them into
-// shared memory per unit.  Tensor-memory accumulators are double-buffered per K block so that the
-// promotion of block kb overlaps the MMAs of block kb+1.
+// gate/up) and one activation scale per token and K block.  Tensor-memory accumulators are buffered per K block so
+// that the promotion of block kb overlaps the MMAs of the blocks behind it.
+//
+// A unit is half as long as in bf16 (32 K blocks of 32 KB: 23 us at an SM's share of the memory rate), so what a
+// unit costs besides its stream weighs twice as much, and everything that sat between two units is off the promotion
+// warps' path:
+//   * units are handed out by a counter, and every role finds its next one ready in shared memory (work_iter.cuh);
+//   * one warp fills the scale tables, a unit ahead, and reports finished token tiles for the promotion warps (a
+//     device-scope fence under load takes about as long as three K blocks);
+//   * the gate/up epilogue quantises the activations itself (q_out): its 128 weight rows are exactly one 128-wide
+//     group of the activation row, so a token's scale is a maximum over the unit's four warps.  The bf16 activations
+//     are never stored, and the down GEMM starts a token tile as soon as the tile's units have reported (tile_done),
+//     as in the bf16 kernels, instead of waiting for the gate/up grid and for a quantiser launch behind it.
 //
 // Everything else (swap-AB, persistent CTAs, device-side plan, split-K with ordered fix-up, bounded
-// waits, warp roles) is as in grouped_gemm_tc.cu.  Output is bf16: SwiGLU activations for gate/up,
-// routing-weighted rows for the down projection.
+// waits) is as in grouped_gemm_tc.cu.
 //
 // The reference has no FP8 kernel of its own: it dequantises to bf16 (moeflow/weights.py:23-27) or calls
 // the serving engine's fused experts and moe_kernel_quantize_input (moeflow/integrations/vllm_pf.py:97).
 #include <cuda.h>
-#include <cuda_fp8.h>
 
 #include <cstring>
 
 #include "common.cuh"
 #include "moeflow_b200.h"
+#include "quant.cuh"
 #include "work_iter.cuh"
 
 namespace mf {
 
 constexpr int kF8BlockM = 128;
 constexpr int kF8TileA = 128 * 128;
-constexpr int kF8Gather = 64;
-constexpr int kF8Tables = 2;  // scale tables: the unit being promoted and the prefetched next one
-constexpr int kF8MaxKb = 32;  // K <= 4096 (one unit never spans more K blocks than this)
+constexpr int kF8Gather = 32;  // one warp gathers, the other one fills the tables: 12 warps keep 168 registers each
+constexpr int kF8Tables = 2;   // scale tables: the unit being promoted and the prefetched next one
+constexpr int kF8MaxKb = 32;   // K <= 4096 (one unit never spans more K blocks than this)
+constexpr int kF8Stage = 1024;  // per promotion warp: 16 token columns x 32 outputs of the epilogue, transposed
 
 template <bool kGateUp, int N_MAX>
 struct F8Cfg {
@@ -45,20 +55,23 @@ struct F8Cfg {
   static constexpr int kStageB = N_MAX * 128;
   static constexpr int kStageBytes = kStageA + kStageB;
   // Promotion warps: one group of four warps (one per tensor-memory lane quarter) takes N_MAX / kGroups token
-  // columns: 32 columns per group for tiles of up to 64 rows (a K block's promotion is then one tensor-memory
-  // round trip per warp), 64 for 128-row tiles (a thread keeps at most 2 x 64 running sums in registers).
+  // columns: 32 columns per group for tiles of up to 64 rows, 64 for 128-row tiles.
   static constexpr int kGroups = N_MAX > 32 ? 2 : 1;
   static constexpr int kCols = N_MAX / kGroups;
-  static constexpr int kThreads = 128 + 128 * kGroups;
+  static constexpr int kPromo = 4 * kGroups;             // promotion warps: 4 .. 4 + kPromo - 1
+  static constexpr int kThreads = 128 + 32 * kPromo;
   static constexpr int kTableFloats = N_MAX * kF8MaxKb + 2 * kF8MaxKb;  // x scales [kb][n], weight scales [2][kb]
   static constexpr int kTableBytes = kF8Tables * kTableFloats * 4;
-  static constexpr int kStages = (222 * 1024 - kTableBytes) / kStageBytes > 8 ? 8 : (222 * 1024 - kTableBytes) / kStageBytes;
+  static constexpr int kBarrierBytes = 1024;             // barriers and the segment ring
+  static constexpr int kExtra = kPromo * kF8Stage + kBarrierBytes;
+  static constexpr int kFree = 227 * 1024 - 1024 /*alignment*/ - kTableBytes - kExtra;
+  static constexpr int kStages = kFree / kStageBytes > 8 ? 8 : kFree / kStageBytes;
   static constexpr int kTmpCols = kATiles * N_MAX;
   // One tensor-memory accumulator per K block in flight: the MMA -> promotion -> MMA round trip is about a
   // microsecond, so two stages cannot keep up with the weight stream; use all 512 columns (at most 8 stages).
   static constexpr int kTmpStages = 512 / kTmpCols > 8 ? 8 : 512 / kTmpCols;
   static constexpr int kTmemCols = kTmpStages * kTmpCols;
-  static constexpr int kSmemBytes = kStages * kStageBytes + kTableBytes + 1024 + 512;
+  static constexpr int kSmemBytes = kStages * kStageBytes + kTableBytes + kExtra + 1024;
 };
 
 struct F8Pipe {
@@ -72,6 +85,35 @@ struct F8Pipe {
   }
 };
 
+// Two fp32 values in one 64-bit register: the promotion works on pairs of token columns (one instruction for two
+// multiply-adds, each rounded like fmaf).
+using f32x2 = unsigned long long;
+__device__ __forceinline__ f32x2 pack2(float lo, float hi) {
+  f32x2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+  return r;
+}
+__device__ __forceinline__ f32x2 pack2(uint32_t lo, uint32_t hi) {
+  f32x2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "r"(lo), "r"(hi));
+  return r;
+}
+__device__ __forceinline__ float2 unpack2(f32x2 v) {
+  float2 r;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+  return r;
+}
+__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
+  f32x2 r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
+  f32x2 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+
 template <bool kGateUp, int N_MAX>
 __global__ void __launch_bounds__(F8Cfg<kGateUp, N_MAX>::kThreads, 1)
 grouped_gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_b,
@@ -80,22 +122,29 @@ grouped_gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid
   constexpr int STAGES = Cfg::kStages;
   constexpr int GROUPS = Cfg::kGroups;
   constexpr int COLS = Cfg::kCols;
-  constexpr int PROMO_WARPS = 4 * GROUPS;
+  constexpr int PROMO_WARPS = Cfg::kPromo;
+  static_assert(STAGES >= 2 && Cfg::kSmemBytes <= 227 * 1024, "shared memory");
+  static_assert((int)sizeof(SegRing) + (2 * STAGES + 2 * Cfg::kTmpStages + 2 * kF8Tables + GROUPS + 2) * 8 + 8 + 4 * GROUPS <=
+                    Cfg::kBarrierBytes, "barriers");
 
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint8_t* sA = smem;
   uint8_t* sB = smem + STAGES * Cfg::kStageA;
   float* sTable = reinterpret_cast<float*>(smem + STAGES * Cfg::kStageBytes);  // [kF8Tables][kTableFloats]
-  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + STAGES * Cfg::kStageBytes + Cfg::kTableBytes);
-  uint64_t* full_bar = bars;
-  uint64_t* empty_bar = bars + STAGES;
-  uint64_t* tmp_full = bars + 2 * STAGES;
+  uint8_t* sStage = smem + STAGES * Cfg::kStageBytes + Cfg::kTableBytes;       // [PROMO_WARPS][kF8Stage]
+  SegRing* ring = reinterpret_cast<SegRing*>(sStage + PROMO_WARPS * kF8Stage);
+  uint64_t* full_bar = reinterpret_cast<uint64_t*>(ring + 1);
+  uint64_t* empty_bar = full_bar + STAGES;
+  uint64_t* tmp_full = empty_bar + STAGES;
   uint64_t* tmp_empty = tmp_full + Cfg::kTmpStages;
   uint64_t* tbl_bar = tmp_empty + Cfg::kTmpStages;  // [kF8Tables] table filled
   uint64_t* tbl_free = tbl_bar + kF8Tables;         // [kF8Tables] table no longer read
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tbl_free + kF8Tables);
+  uint64_t* grp_bar = tbl_free + kF8Tables;         // [GROUPS] the group's four warps met (epilogue)
+  uint64_t* epi_bar = grp_bar + GROUPS;             // [2] a unit's outputs are stored (all promotion warps)
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(epi_bar + 2);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+  volatile int* grp_last = abort_flag + 1;          // [GROUPS] a cut unit's arrival count, seen by the group's first warp
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const bool b_tma = a.b_tmap != nullptr;  // token tiles by TMA (contiguous rows) instead of the 16-byte gather
@@ -109,9 +158,12 @@ grouped_gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid
       mbar_init(&tmp_empty[s], PROMO_WARPS);
     }
     for (int s = 0; s < kF8Tables; ++s) {
-      mbar_init(&tbl_bar[s], PROMO_WARPS);
+      mbar_init(&tbl_bar[s], 1);
       mbar_init(&tbl_free[s], PROMO_WARPS);
     }
+    for (int s = 0; s < GROUPS; ++s) mbar_init(&grp_bar[s], 4);
+    for (int s = 0; s < 2; ++s) mbar_init(&epi_bar[s], PROMO_WARPS);
+    ring->init(3 + PROMO_WARPS);  // UMMA, token producer, table warp, promotion warps
     *abort_flag = 0;
     fence_mbar_init();
     tma_prefetch_desc(&tmap_w);
@@ -126,12 +178,24 @@ grouped_gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid
   tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_slot;
 
-  grid_dep_wait_cta();
-  grid_dep_launch();
+  if (tid < 6) {
+    // while the predecessor runs: touch the pages read right after the wait (see touch() in common.cuh)
+    const void* p = tid == 0 ? (const void*)a.plan : tid == 1 ? (const void*)a.tile_e : tid == 2 ? (const void*)a.tile_s
+                  : tid == 3 ? (const void*)a.tile_n : tid == 4 ? (const void*)a.b_index : (const void*)a.tile_wait;
+    touch(p);
+  }
+  // As in the bf16 kernels: the gate/up GEMM waits for the plan and only then lets the next kernel start, so the
+  // down GEMM finds the plan complete; with tile-level hand-over nothing in it waits for the gate/up grid as a whole.
+  if (kGateUp || a.tile_wait == nullptr) {
+    grid_dep_wait_cta();
+    grid_dep_launch();
+  } else {
+    grid_dep_launch();
+  }
 
-  int n_tiles = a.plan[MF_PLAN_N_TILES];
-  const int cut = a.plan[a.split_word];  // 0 = stream-K, else the K split
-  int slot_cols = a.plan[MF_PLAN_SLOT_COLS];
+  int n_tiles = __ldcg(a.plan + MF_PLAN_N_TILES);
+  const int cut = __ldcg(a.plan + a.split_word);  // 0 = stream-K, else the K split
+  int slot_cols = __ldcg(a.plan + MF_PLAN_SLOT_COLS);
   if (slot_cols <= 0 || slot_cols > N_MAX) slot_cols = N_MAX;
   const long long slot_floats = (long long)Cfg::kATiles * slot_cols * kF8BlockM;
   const unsigned long long wait_ns = a.wait_ns;
@@ -150,14 +214,26 @@ grouped_gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid
       work.init(a, N_MAX, 0, 1, blockIdx.x, gridDim.x);
     }
   }
+  auto tile_ready = [&](int tt) -> bool {  // bounded; one lane asks
+    bool got = true;
+    if (lane == 0) got = wait_count_ge_gpu(a.tile_wait + tt, a.tile_wait_target, wait_ns);
+    got = __all_sync(0xffffffffu, got);
+    if (!got && lane == 0) {
+      *abort_flag = 1;
+      report_status(a.status, kGemmFullTimeout, 6, blockIdx.x, 0);
+    }
+    return got;
+  };
+  SegReader reader(ring, abort_flag, wait_ns);
 
   if (warp == 0) {
-    // ---------------------------------------------------------------- weight TMA producer
+    // ---------------------------------------------------------------- weight TMA producer, hands out the segments
     F8Pipe st;
     bool ok = true;
-    WorkIter it = work;
+    SegFeed feed(work, ring, abort_flag, wait_ns);
     Seg sg;
-    while (ok && it.next(sg)) {
+    bool have = feed.first(sg);
+    while (ok && have) {
       const int row0 = sg.e * a.rows_per_expert + sg.mb * kF8BlockM;
       for (int j = 0; j < sg.nkb; ++j) {
         const int kb = sg.kb0 + j;
@@ -174,8 +250,11 @@ grouped_gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid
         }
         __syncwarp();
         st.advance(STAGES);
+        feed.advance();
       }
+      if (ok) have = feed.next(sg);
     }
+    if (feed.bad_tile && lane == 0) report_status(a.status, kBadArgument, 7, blockIdx.x, 0);
     if (!ok) {
       const unsigned long long t0 = global_timer_ns();
       while (global_timer_ns() - t0 < 100000ull) __nanosleep(1000);
@@ -184,9 +263,8 @@ grouped_gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid
     // ---------------------------------------------------------------- UMMA issuer (one K block per tmp stage)
     F8Pipe st, tmp;
     bool ok = true;
-    WorkIter it = work;
     Seg sg;
-    while (ok && it.next(sg)) {
+    while (ok && reader.next(sg, ok)) {
       uint32_t n_tile = (uint32_t)((sg.n_rows + 15) & ~15);
       if (n_tile < 16) n_tile = 16;
       const uint32_t idesc = umma_idesc(0, 0, kF8BlockM, n_tile);  // e4m3 x e4m3 -> fp32
@@ -221,55 +299,70 @@ grouped_gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid
         tmp.advance(Cfg::kTmpStages);
       }
     }
-  } else if (warp < 4 && b_tma) {
+  } else if (warp == 2 && b_tma) {
     // ---------------------------------------------------------------- token-operand producer (TMA)
-    if (warp == 2) {
-      F8Pipe st;
-      bool ok = true;
-      WorkIter it = work;
-      Seg sg;
-      while (ok && it.next(sg)) {
-        for (int j = 0; j < sg.nkb; ++j) {
-          const int kb = sg.kb0 + j;
-          ok = __all_sync(0xffffffffu, mbar_wait_bounded(&empty_bar[st.stage], st.phase ^ 1u, abort_flag, wait_ns));
-          if (!ok) {
-            if (lane == 0) report_status(a.status, kGemmEmptyTimeout, 2, blockIdx.x, 0);
-            break;
-          }
-          if (lane == 0) {
-            mbar_arrive_expect_tx(&full_bar[st.stage], Cfg::kStageB);
-            tma_load_2d(sB + st.stage * Cfg::kStageB, &tmap_b, &full_bar[st.stage], kb * 128, sg.row_start);
-          }
-          __syncwarp();
-          st.advance(STAGES);
-        }
-      }
-      if (!ok) {
-        const unsigned long long t0 = global_timer_ns();
-        while (global_timer_ns() - t0 < 100000ull) __nanosleep(1000);
-      }
-    }
-  } else if (warp < 4) {
-    // ---------------------------------------------------------------- token-operand producers (e4m3 rows)
-    const int gt = tid - 64, r_in = gt >> 3, chunk = gt & 7;
-    const uint32_t sw_off = (uint32_t)((chunk ^ r_in) << 4);
     F8Pipe st;
     bool ok = true;
-    WorkIter it = work;
     Seg sg;
-    while (ok && it.next(sg)) {
-      const int n_rows = sg.n_rows, row_start = sg.row_start;
+    int ready_tile = -1;
+    while (ok && reader.next(sg, ok)) {
+      if (a.tile_wait != nullptr && sg.tt != ready_tile) {
+        ok = tile_ready(sg.tt);
+        if (!ok) break;
+        if (lane == 0) fence_proxy_async_all();  // the TMA reads below come after the acquire
+        ready_tile = sg.tt;
+      }
+      for (int j = 0; j < sg.nkb; ++j) {
+        const int kb = sg.kb0 + j;
+        ok = __all_sync(0xffffffffu, mbar_wait_bounded(&empty_bar[st.stage], st.phase ^ 1u, abort_flag, wait_ns));
+        if (!ok) {
+          if (lane == 0) report_status(a.status, kGemmEmptyTimeout, 2, blockIdx.x, 0);
+          break;
+        }
+        if (lane == 0) {
+          mbar_arrive_expect_tx(&full_bar[st.stage], Cfg::kStageB);
+          tma_load_2d(sB + st.stage * Cfg::kStageB, &tmap_b, &full_bar[st.stage], kb * 128, sg.row_start);
+        }
+        __syncwarp();
+        st.advance(STAGES);
+      }
+    }
+    if (!ok) {
+      const unsigned long long t0 = global_timer_ns();
+      while (global_timer_ns() - t0 < 100000ull) __nanosleep(1000);
+    }
+  } else if (warp == 2) {
+    // ---------------------------------------------------------------- token-operand producer (gathered e4m3 rows)
+    const int r_in = lane >> 3, chunk = lane & 7;  // rows r_in, r_in + 4, ...: two swizzle phases
+    const uint32_t sw_off[2] = {(uint32_t)((chunk ^ r_in) << 4), (uint32_t)((chunk ^ (r_in + 4)) << 4)};
+    F8Pipe st;
+    bool ok = true;
+    Seg sg, nx;
+    int ready_tile = -1;
+    int idx[N_MAX / 4];  // source rows of the segment at hand, fetched during the previous one
+    auto row_indices = [&](const Seg& s_) {
+#pragma unroll
+      for (int i = 0; i < N_MAX / 4; ++i) {
+        const int n = r_in + 4 * i;
+        if (n < s_.n_rows) idx[i] = a.b_index ? __ldcg(a.b_index + s_.row_start + n) : s_.row_start + n;
+      }
+    };
+    bool have = reader.next(sg, ok), more = false;
+    if (have) row_indices(sg);
+    while (ok && have) {
+      if (a.tile_wait != nullptr && sg.tt != ready_tile) {
+        ok = tile_ready(sg.tt);
+        if (!ok) break;
+        ready_tile = sg.tt;
+      }
+      const int n_rows = sg.n_rows;
       int n_tile = (n_rows + 15) & ~15;
       if (n_tile < 16) n_tile = 16;
-      const uint8_t* rp[N_MAX / 8];
+      const uint8_t* rp[N_MAX / 4];
 #pragma unroll
-      for (int i = 0; i < N_MAX / 8; ++i) {
-        const int n = r_in + 8 * i;
-        rp[i] = nullptr;
-        if (n < n_rows) {
-          const long long idx = a.b_index ? (long long)a.b_index[row_start + n] : (long long)(row_start + n);
-          rp[i] = static_cast<const uint8_t*>(a.b_base) + idx * a.b_pitch + chunk * 16;
-        }
+      for (int i = 0; i < N_MAX / 4; ++i) {
+        const int n = r_in + 4 * i;
+        rp[i] = n < n_rows ? static_cast<const uint8_t*>(a.b_base) + (long long)idx[i] * a.b_pitch + chunk * 16 : nullptr;
       }
       for (int j = 0; j < sg.nkb; ++j) {
         const int kb = sg.kb0 + j;
@@ -280,18 +373,110 @@ grouped_gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid
         }
         const uint32_t b_stage = smem_u32(sB + st.stage * Cfg::kStageB);
 #pragma unroll
-        for (int i = 0; i < N_MAX / 8; ++i) {
-          const int n = r_in + 8 * i;
+        for (int i = 0; i < N_MAX / 4; ++i) {
+          const int n = r_in + 4 * i;
           if (n < n_tile) {
             const bool live = rp[i] != nullptr;
-            cp_async_16(b_stage + n * 128 + sw_off, live ? (const void*)(rp[i] + (long long)kb * 128) : a.b_base, live ? 16u : 0u);
+            cp_async_16(b_stage + n * 128 + sw_off[i & 1], live ? (const void*)(rp[i] + (long long)kb * 128) : a.b_base, live ? 16u : 0u);
           }
         }
         cp_async_mbar_arrive_noinc(&full_bar[st.stage]);
         st.advance(STAGES);
+        // the producer warp publishes the next segment during the third K block of this one
+        if (j == (sg.nkb < 4 ? sg.nkb - 1 : 3)) {
+          more = reader.next(nx, ok);
+          if (more) row_indices(nx);
+          if (!ok) break;
+        }
       }
+      sg = nx;
+      have = more;
     }
     asm volatile("cp.async.wait_all;" ::: "memory");
+  } else if (warp == 3) {
+    // ---------------------------------------------------------------- scale tables (a unit ahead), finished tiles
+    // Table: x scales [j][n] and weight scales [t][j] of a segment, j = kb - kb0.  A lane takes whole token rows: all of a
+    // row's scales are requested before the first one is stored.
+    // Finished tiles: two units behind, the outputs of a whole gate/up unit are fenced and counted for the down GEMM.
+    const int row_blocks = a.rows_per_expert / kF8BlockM;
+    const bool vec = (a.b_scale_pitch & 3) == 0 && (reinterpret_cast<uintptr_t>(a.b_scale) & 15) == 0;
+    const bool report = kGateUp && a.tile_done != nullptr;
+    bool ok = true;
+    Seg sg;
+    int n_it = 0, ready_tile = -1;
+    int done_tile[2] = {-1, -1};  // tiles of the last two units, if this warp has to report them
+    auto report_unit = [&](int k) -> bool {  // unit k of this CTA
+      const bool got = __all_sync(0xffffffffu, mbar_wait_bounded(&epi_bar[k & 1], (uint32_t)(k >> 1) & 1u, abort_flag, wait_ns));
+      const int tt = k & 1 ? done_tile[1] : done_tile[0];
+      if (got && lane == 0 && tt >= 0) {
+        __threadfence();  // the promotion warps' stores (ordered before by the barrier) are visible device-wide
+        atomicAdd(a.tile_done + tt, PROMO_WARPS);
+      }
+      return got;
+    };
+    while (ok && reader.next(sg, ok)) {
+      const int buf = n_it % kF8Tables;
+      float* t = sTable + buf * Cfg::kTableFloats;
+      float wv[kGateUp ? 2 : 1];
+#pragma unroll
+      for (int q = 0; q < (kGateUp ? 2 : 1); ++q) {
+        const int rb = (q == 0 ? 0 : a.up_row_offset / kF8BlockM) + sg.mb;
+        wv[q] = lane < sg.nkb ? __ldcg(a.w_scale + ((long long)sg.e * row_blocks + rb) * a.k_blocks + sg.kb0 + lane) : 0.f;
+      }
+      if (a.tile_wait != nullptr && sg.tt != ready_tile) {
+        ok = tile_ready(sg.tt);
+        if (!ok) break;
+        ready_tile = sg.tt;
+      }
+      if (n_it >= kF8Tables) {
+        ok = __all_sync(0xffffffffu, mbar_wait_bounded(&tbl_free[buf], (uint32_t)(n_it / kF8Tables - 1) & 1u, abort_flag, wait_ns));
+        if (!ok) {
+          if (lane == 0) report_status(a.status, kGemmAccTimeout, 6, blockIdx.x, 0);
+          break;
+        }
+      }
+      int n_tile = (sg.n_rows + 15) & ~15;
+      if (n_tile < 16) n_tile = 16;
+      for (int n = lane; n < n_tile; n += 32) {
+        const bool live = n < sg.n_rows;
+        long long idx = 0;
+        if (live) idx = a.b_index ? (long long)__ldcg(a.b_index + sg.row_start + n) : (long long)(sg.row_start + n);
+        const float* src = a.b_scale + idx * a.b_scale_pitch + sg.kb0;
+        float v[kF8MaxKb];
+        if (vec && ((sg.kb0 | sg.nkb) & 3) == 0) {
+#pragma unroll
+          for (int j = 0; j < kF8MaxKb; j += 4) {
+            float4 f = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (live && j < sg.nkb) f = __ldcg(reinterpret_cast<const float4*>(src + j));
+            v[j] = f.x;
+            v[j + 1] = f.y;
+            v[j + 2] = f.z;
+            v[j + 3] = f.w;
+          }
+        } else {
+#pragma unroll
+          for (int j = 0; j < kF8MaxKb; ++j) v[j] = (live && j < sg.nkb) ? __ldcg(src + j) : 0.f;
+        }
+#pragma unroll
+        for (int j = 0; j < kF8MaxKb; ++j)
+          if (j < sg.nkb) t[j * N_MAX + n] = v[j];
+      }
+#pragma unroll
+      for (int q = 0; q < (kGateUp ? 2 : 1); ++q) t[N_MAX * kF8MaxKb + q * kF8MaxKb + lane] = wv[q];
+      if (report) {
+        // before the table is handed over: with it the promotion warps may come back to the same barrier
+        if (n_it >= 2) ok = report_unit(n_it - 2);
+        if (!ok) break;
+        const int tt = sg.nseg == 1 ? sg.tt : -1;
+        if (n_it & 1) done_tile[1] = tt;
+        else done_tile[0] = tt;
+      }
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&tbl_bar[buf]);
+      ++n_it;
+    }
+    if (report)
+      for (int k = n_it < 2 ? 0 : n_it - 2; ok && k < n_it; ++k) ok = report_unit(k);
   } else {
     // ---------------------------------------------------------------- promotion + epilogue
     const int pw = warp - 4;                 // 0 .. PROMO_WARPS-1
@@ -299,275 +484,293 @@ grouped_gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid
     const int grp = pw >> 2;                 // column group
     const int col0 = grp * COLS;
     const int row = wq * 32 + lane;
+    const uint32_t lane_base = tmem_base + ((uint32_t)(wq * 32) << 16) + col0;
+    uint8_t* stage = sStage + pw * kF8Stage;
     F8Pipe tmp;
     bool ok = true;
-    const int row_blocks = a.rows_per_expert / kF8BlockM;
-    // Scale table of one segment into buffer `buf`: x scales [j][n] and weight scales [t][j], j = kb - kb0.
-    // Every promotion warp fills its share (token columns n = pw, pw + PROMO_WARPS, ... in blocks of 32 lanes)
-    // and arrives once on the buffer's barrier.
-    auto load_table = [&](const Seg& s_, int buf) {
-      int n_tile_ = (s_.n_rows + 15) & ~15;
-      if (n_tile_ < 16) n_tile_ = 16;
-      float* t = sTable + buf * Cfg::kTableFloats;
-      for (int n0 = pw * 32; n0 < n_tile_; n0 += PROMO_WARPS * 32) {
-        const int n = n0 + lane;
-        if (n < n_tile_) {
-          const bool live = n < s_.n_rows;
-          long long idx = 0;
-          if (live) idx = a.b_index ? (long long)a.b_index[s_.row_start + n] : (long long)(s_.row_start + n);
-          // all of the row's scales are requested before the first one is stored: one memory round trip per
-          // token instead of one per K block (a dependent load-store loop here cost as much as the unit's
-          // whole weight stream)
-          const float* src = a.b_scale + idx * a.b_scale_pitch + s_.kb0;
-          float v[kF8MaxKb];
-#pragma unroll
-          for (int j = 0; j < kF8MaxKb; ++j) v[j] = (live && j < s_.nkb) ? __ldcg(src + j) : 0.f;
-#pragma unroll
-          for (int j = 0; j < kF8MaxKb; ++j)
-            if (j < s_.nkb) t[j * N_MAX + n] = v[j];
-        }
-      }
-      if (pw < (kGateUp ? 2 : 1)) {
-        const int rb = (pw == 0 ? 0 : a.up_row_offset / kF8BlockM) + s_.mb;
-        const float* ws = a.w_scale + ((long long)s_.e * row_blocks + rb) * a.k_blocks + s_.kb0;
-        for (int j = lane; j < s_.nkb; j += 32) t[N_MAX * kF8MaxKb + pw * kF8MaxKb + j] = ws[j];
-      }
+    uint32_t grp_phase = 0;
+    // The four warps of this column group meet (bounded, so not a named barrier).
+    auto group_sync = [&]() -> bool {
       __syncwarp();
-      if (lane == 0) mbar_arrive(&tbl_bar[buf]);
+      if (lane == 0) mbar_arrive(&grp_bar[grp]);
+      const bool k = __all_sync(0xffffffffu, mbar_wait_bounded(&grp_bar[grp], grp_phase, abort_flag, wait_ns));
+      grp_phase ^= 1u;
+      if (!k && lane == 0) report_status(a.status, kGemmAccTimeout, 7, blockIdx.x, 0);
+      return k;
     };
-    WorkIter it = work;    // the segment being promoted
-    WorkIter ahead = work; // one segment ahead, for the table prefetch
-    Seg sg, nx;
-    bool have_next = ahead.next(nx);
-    if (have_next) load_table(nx, 0);
+    Seg sg;
     int n_it = 0;  // index of this CTA's segment
-    while (ok && it.next(sg)) {
+    while (ok && reader.next(sg, ok)) {
       const int mb = sg.mb, n_rows = sg.n_rows, row_start = sg.row_start;
       int n_tile = (n_rows + 15) & ~15;
       if (n_tile < 16) n_tile = 16;
       const int buf = n_it % kF8Tables;
       const float* tbl = sTable + buf * Cfg::kTableFloats;
       const float* tblW = tbl + N_MAX * kF8MaxKb;
+      f32x2 acc_g[COLS / 2], acc_u[kGateUp ? COLS / 2 : 1];
+#pragma unroll
+      for (int i = 0; i < COLS / 2; ++i) acc_g[i] = 0ull;
+      if (kGateUp) {
+#pragma unroll
+        for (int i = 0; i < COLS / 2; ++i) acc_u[i] = 0ull;
+      }
+      float row_scale[COLS / 32];  // routing weights of this group's columns, requested ahead of the K loop
+      if (!kGateUp && a.row_scale != nullptr) {
+#pragma unroll
+        for (int i = 0; i < COLS / 32; ++i) {
+          const int n = col0 + 32 * i + lane;
+          row_scale[i] = n < n_rows ? __ldcg(a.row_scale + row_start + n) : 1.f;
+        }
+      }
       ok = __all_sync(0xffffffffu, mbar_wait_bounded(&tbl_bar[buf], (uint32_t)(n_it / kF8Tables) & 1u, abort_flag, wait_ns));
       if (!ok) {
         if (lane == 0) report_status(a.status, kGemmAccTimeout, 4, blockIdx.x, 0);
         break;
       }
-      // Prefetch the next segment's table into the other buffer, once every warp has stopped reading what
-      // that buffer held (the table of the previous segment).
-      have_next = ahead.next(nx);
-      if (have_next) {
-        const int nb = (n_it + 1) % kF8Tables;
-        if (n_it >= 1) {
-          ok = __all_sync(0xffffffffu, mbar_wait_bounded(&tbl_free[nb], (uint32_t)((n_it - 1) / kF8Tables) & 1u, abort_flag, wait_ns));
-          if (!ok) {
-            if (lane == 0) report_status(a.status, kGemmAccTimeout, 6, blockIdx.x, 0);
-            break;
-          }
-        }
-        load_table(nx, nb);
-      }
 
-      float acc_g[COLS], acc_u[kGateUp ? COLS : 1];
-#pragma unroll
-      for (int i = 0; i < COLS; ++i) acc_g[i] = 0.f;
-      if (kGateUp) {
-#pragma unroll
-        for (int i = 0; i < COLS; ++i) acc_u[i] = 0.f;
-      }
-
-      for (int j = 0; j < sg.nkb; ++j) {
-        if (!kGateUp && COLS == 32 && Cfg::kTmpStages >= 2 && j + 1 < sg.nkb) {
-          // Down projection, 32-column groups: two K blocks per round trip.  A K block is only 16 KB of weights
-          // here, so the fixed cost of a promotion step (barrier, tensor-memory load, fence, arrival) has to be
-          // shared between two of them to keep up with the weight stream.
-          F8Pipe nxt = tmp;
-          nxt.advance(Cfg::kTmpStages);
-          ok = __all_sync(0xffffffffu, mbar_wait_bounded(&tmp_full[tmp.stage], tmp.phase, abort_flag, wait_ns));
-          if (ok) ok = __all_sync(0xffffffffu, mbar_wait_bounded(&tmp_full[nxt.stage], nxt.phase, abort_flag, wait_ns));
-          if (!ok) {
-            if (lane == 0) report_status(a.status, kGemmAccTimeout, 3, blockIdx.x, 0);
-            break;
-          }
-          tc_fence_after_sync();
-          if (col0 < n_tile) {
-            const uint32_t lane_base = tmem_base + ((uint32_t)(wq * 32) << 16) + col0;
-            uint32_t r0[32], r1[32];
-            tmem_ld_32(lane_base + tmp.stage * Cfg::kTmpCols, r0);
-            tmem_ld_32(lane_base + nxt.stage * Cfg::kTmpCols, r1);
-            tmem_ld_wait();
-            const float w0 = tblW[j], w1 = tblW[j + 1];
-            const float4* x0 = reinterpret_cast<const float4*>(tbl + j * N_MAX + col0);
-            const float4* x1 = reinterpret_cast<const float4*>(tbl + (j + 1) * N_MAX + col0);
-#pragma unroll
-            for (int q = 0; q < 8; ++q) {
-              const float4 a0 = x0[q], a1 = x1[q];
-              acc_g[4 * q] = fmaf(__uint_as_float(r0[4 * q]), w0 * a0.x, acc_g[4 * q]);
-              acc_g[4 * q + 1] = fmaf(__uint_as_float(r0[4 * q + 1]), w0 * a0.y, acc_g[4 * q + 1]);
-              acc_g[4 * q + 2] = fmaf(__uint_as_float(r0[4 * q + 2]), w0 * a0.z, acc_g[4 * q + 2]);
-              acc_g[4 * q + 3] = fmaf(__uint_as_float(r0[4 * q + 3]), w0 * a0.w, acc_g[4 * q + 3]);
-              acc_g[4 * q] = fmaf(__uint_as_float(r1[4 * q]), w1 * a1.x, acc_g[4 * q]);
-              acc_g[4 * q + 1] = fmaf(__uint_as_float(r1[4 * q + 1]), w1 * a1.y, acc_g[4 * q + 1]);
-              acc_g[4 * q + 2] = fmaf(__uint_as_float(r1[4 * q + 2]), w1 * a1.z, acc_g[4 * q + 2]);
-              acc_g[4 * q + 3] = fmaf(__uint_as_float(r1[4 * q + 3]), w1 * a1.w, acc_g[4 * q + 3]);
-            }
-          }
-          tc_fence_before_sync();
-          __syncwarp();
-          if (lane == 0) {
-            mbar_arrive(&tmp_empty[tmp.stage]);
-            mbar_arrive(&tmp_empty[nxt.stage]);
-          }
-          tmp.advance(Cfg::kTmpStages);
-          tmp.advance(Cfg::kTmpStages);
-          ++j;
-          continue;
-        }
-        ok = __all_sync(0xffffffffu, mbar_wait_bounded(&tmp_full[tmp.stage], tmp.phase, abort_flag, wait_ns));
+      // Down projection: two K blocks per trip (a K block is only 16 KB of weights there), gate/up: one.
+      constexpr int kTrip = kGateUp ? 1 : 2;
+      for (int j = 0; j < sg.nkb; j += kTrip) {
+        const int nb = kTrip == 2 && j + 1 < sg.nkb ? 2 : 1;
+        F8Pipe nxt = tmp;
+        nxt.advance(Cfg::kTmpStages);
+        ok = mbar_wait_bounded(&tmp_full[tmp.stage], tmp.phase, abort_flag, wait_ns);
+        if (ok && nb == 2) ok = mbar_wait_bounded(&tmp_full[nxt.stage], nxt.phase, abort_flag, wait_ns);
+        ok = __all_sync(0xffffffffu, ok);
         if (!ok) {
           if (lane == 0) report_status(a.status, kGemmAccTimeout, 3, blockIdx.x, 0);
           break;
         }
         tc_fence_after_sync();
-        const uint32_t taddr = tmem_base + ((uint32_t)(wq * 32) << 16) + tmp.stage * Cfg::kTmpCols + col0;
-        const float wsg = tblW[j];
-        const float wsu = kGateUp ? tblW[kF8MaxKb + j] : 0.f;
-        const float4* xs4 = reinterpret_cast<const float4*>(tbl + j * N_MAX + col0);
-        // Thirty-two token columns per tensor-memory round trip (the load latency, not the arithmetic, bounds a
-        // K block's promotion); with 32-column groups the gate and the up values travel together.
-        constexpr bool kBoth = kGateUp && COLS == 32;
+        const uint32_t t0 = lane_base + tmp.stage * Cfg::kTmpCols, t1 = lane_base + nxt.stage * Cfg::kTmpCols;
+        const f32x2 w0 = pack2(tblW[j], tblW[j]);
+        const f32x2 w1 = kGateUp ? pack2(tblW[kF8MaxKb + j], tblW[kF8MaxKb + j])
+                                 : (nb == 2 ? pack2(tblW[j + 1], tblW[j + 1]) : 0ull);
+        const ulonglong2* x0 = reinterpret_cast<const ulonglong2*>(tbl + j * N_MAX + col0);
+        const ulonglong2* x1 = reinterpret_cast<const ulonglong2*>(tbl + (j + 1) * N_MAX + col0);
+        // 16 token columns at a time, as many as the tile has; first and second accumulator (gate and up, or two K
+        // blocks) travel together.
 #pragma unroll
-        for (int c0 = 0; c0 < COLS; c0 += 32) {
+        for (int c0 = 0; c0 < COLS; c0 += 16) {
           if (col0 + c0 < n_tile) {
-            uint32_t g[32], u2[kBoth ? 32 : 1];
-            tmem_ld_32(taddr + c0, g);
-            if (kBoth) tmem_ld_32(taddr + N_MAX + c0, reinterpret_cast<uint32_t(&)[32]>(u2));
+            uint32_t p[16], q[16];
+            tmem_ld_16(t0 + c0, p);
+            if (kGateUp) tmem_ld_16(t0 + N_MAX + c0, q);
+            else if (nb == 2) tmem_ld_16(t1 + c0, q);
             tmem_ld_wait();
 #pragma unroll
-            for (int q = 0; q < 8; ++q) {
-              const float4 xs = xs4[c0 / 4 + q];
-              acc_g[c0 + 4 * q] = fmaf(__uint_as_float(g[4 * q]), wsg * xs.x, acc_g[c0 + 4 * q]);
-              acc_g[c0 + 4 * q + 1] = fmaf(__uint_as_float(g[4 * q + 1]), wsg * xs.y, acc_g[c0 + 4 * q + 1]);
-              acc_g[c0 + 4 * q + 2] = fmaf(__uint_as_float(g[4 * q + 2]), wsg * xs.z, acc_g[c0 + 4 * q + 2]);
-              acc_g[c0 + 4 * q + 3] = fmaf(__uint_as_float(g[4 * q + 3]), wsg * xs.w, acc_g[c0 + 4 * q + 3]);
-            }
-            if (kGateUp) {
-              if (!kBoth) {
-                tmem_ld_32(taddr + N_MAX + c0, g);
-                tmem_ld_wait();
+            for (int i = 0; i < 4; ++i) {
+              const ulonglong2 xs = x0[c0 / 4 + i];
+              f32x2* ag = acc_g + c0 / 2 + 2 * i;
+              ag[0] = fma2(pack2(p[4 * i], p[4 * i + 1]), mul2(w0, xs.x), ag[0]);
+              ag[1] = fma2(pack2(p[4 * i + 2], p[4 * i + 3]), mul2(w0, xs.y), ag[1]);
+              if (kGateUp) {
+                f32x2* au = acc_u + c0 / 2 + 2 * i;
+                au[0] = fma2(pack2(q[4 * i], q[4 * i + 1]), mul2(w1, xs.x), au[0]);
+                au[1] = fma2(pack2(q[4 * i + 2], q[4 * i + 3]), mul2(w1, xs.y), au[1]);
               }
+            }
+            if (!kGateUp && nb == 2) {
 #pragma unroll
-              for (int q = 0; q < 8; ++q) {
-                const float4 xs = xs4[c0 / 4 + q];
-                const uint32_t* r = kBoth ? u2 : g;
-                acc_u[c0 + 4 * q] = fmaf(__uint_as_float(r[4 * q]), wsu * xs.x, acc_u[c0 + 4 * q]);
-                acc_u[c0 + 4 * q + 1] = fmaf(__uint_as_float(r[4 * q + 1]), wsu * xs.y, acc_u[c0 + 4 * q + 1]);
-                acc_u[c0 + 4 * q + 2] = fmaf(__uint_as_float(r[4 * q + 2]), wsu * xs.z, acc_u[c0 + 4 * q + 2]);
-                acc_u[c0 + 4 * q + 3] = fmaf(__uint_as_float(r[4 * q + 3]), wsu * xs.w, acc_u[c0 + 4 * q + 3]);
+              for (int i = 0; i < 4; ++i) {
+                const ulonglong2 xs = x1[c0 / 4 + i];
+                f32x2* ag = acc_g + c0 / 2 + 2 * i;
+                ag[0] = fma2(pack2(q[4 * i], q[4 * i + 1]), mul2(w1, xs.x), ag[0]);
+                ag[1] = fma2(pack2(q[4 * i + 2], q[4 * i + 3]), mul2(w1, xs.y), ag[1]);
               }
             }
           }
         }
         tc_fence_before_sync();
         __syncwarp();
-        if (lane == 0) mbar_arrive(&tmp_empty[tmp.stage]);
+        if (lane == 0) {
+          mbar_arrive(&tmp_empty[tmp.stage]);
+          if (nb == 2) mbar_arrive(&tmp_empty[nxt.stage]);
+        }
         tmp.advance(Cfg::kTmpStages);
+        if (nb == 2) tmp.advance(Cfg::kTmpStages);
       }
       if (!ok) break;
       __syncwarp();
       if (lane == 0) mbar_arrive(&tbl_free[buf]);  // this warp is done with the segment's table
 
-      __nv_bfloat16* out = static_cast<__nv_bfloat16*>(a.out);
-      const long long out_col = (long long)mb * kF8BlockM + row;
-      if (sg.nseg == 1) {
-        // 16 columns at a time: their arithmetic first (independent chains overlap), then their stores
-        __nv_bfloat16* p = out + (long long)(row_start + col0) * a.out_pitch + out_col;
-        const bool all = col0 + COLS <= n_rows;
-#pragma unroll
-        for (int c0 = 0; c0 < COLS; c0 += 16) {
-          if (kGateUp) {
-            if (a.round_h) {
-#pragma unroll
-              for (int c = c0; c < c0 + 16; ++c) {
-                acc_g[c] = bf16_round(acc_g[c]);
-                acc_u[c] = bf16_round(acc_u[c]);
-              }
-            }
-#pragma unroll
-            for (int c = c0; c < c0 + 16; ++c) acc_g[c] = swiglu_clamped(acc_g[c], acc_u[c], a.limit);
-          } else if (a.row_scale) {
-#pragma unroll
-            for (int c = c0; c < c0 + 16; ++c)
-              acc_g[c] *= col0 + c < n_rows ? __ldcg(a.row_scale + row_start + col0 + c) : 1.f;
-          }
-#pragma unroll
-          for (int c = c0; c < c0 + 16; ++c)
-            if (all || col0 + c < n_rows) p[(long long)c * a.out_pitch] = __float2bfloat16_rn(acc_g[c]);
-        }
-      } else {
-        float* mine = a.partial + (long long)it.slot_of(sg, sg.seg) * slot_floats;
+      bool finish = true;
+      if (sg.nseg > 1) {
+        // The unit is cut along K: park the sums; the group that arrives last adds the segments in K order.
+        float* mine = a.partial + (long long)work.slot_of(sg, sg.seg) * slot_floats;
 #pragma unroll
         for (int c = 0; c < COLS; ++c) {
           const int n = col0 + c;
           if (n < n_rows) {
-            __stcg(&mine[(long long)n * kF8BlockM + row], acc_g[c]);
-            if (kGateUp) __stcg(&mine[(long long)(slot_cols + n) * kF8BlockM + row], acc_u[c]);
+            const float2 g = unpack2(acc_g[c / 2]);
+            __stcg(&mine[(long long)n * kF8BlockM + row], c & 1 ? g.y : g.x);
+            if (kGateUp) {
+              const float2 u = unpack2(acc_u[c / 2]);
+              __stcg(&mine[(long long)(slot_cols + n) * kF8BlockM + row], c & 1 ? u.y : u.x);
+            }
           }
         }
         __threadfence();
-        __syncwarp();
-        int* counter = a.counters + ((long long)sg.unit * 4 + wq) * GROUPS + grp;
-        int old = 0;
-        if (lane == 0) old = atomicAdd(counter, 1);
-        old = __shfl_sync(0xffffffffu, old, 0);
-        if (old == sg.nseg - 1) {
+        ok = group_sync();
+        if (!ok) break;
+        int* counter = a.counters + (long long)sg.unit * 4 * GROUPS + grp;
+        if (wq == 0 && lane == 0) grp_last[grp] = atomicAdd(counter, 1);
+        ok = group_sync();
+        if (!ok) break;
+        finish = grp_last[grp] == sg.nseg - 1;
+        if (finish) {
           __threadfence();
-          constexpr int kFix = 8;
-          const int n_end = n_rows < col0 + COLS ? n_rows : col0 + COLS;
-          for (int n0 = col0; n0 < n_end; n0 += kFix) {
-            float v[kFix], w[kFix];
+          if (wq == 0 && lane == 0) *counter = 0;
 #pragma unroll
-            for (int jx = 0; jx < kFix; ++jx) v[jx] = w[jx] = 0.f;
-            for (int s_ = 0; s_ < sg.nseg; ++s_) {
-              const float* p = a.partial + (long long)it.slot_of(sg, s_) * slot_floats;
-              float pv[kFix], pw_[kFix];
+          for (int i = 0; i < COLS / 2; ++i) acc_g[i] = 0ull;
+          if (kGateUp) {
 #pragma unroll
-              for (int jx = 0; jx < kFix; ++jx) {
-                const int n = n0 + jx;
-                pv[jx] = n < n_end ? __ldcg(&p[(long long)n * kF8BlockM + row]) : 0.f;
-                pw_[jx] = (kGateUp && n < n_end) ? __ldcg(&p[(long long)(slot_cols + n) * kF8BlockM + row]) : 0.f;
-              }
+            for (int i = 0; i < COLS / 2; ++i) acc_u[i] = 0ull;
+          }
+          const f32x2 one = pack2(1.f, 1.f);
+          for (int s_ = 0; s_ < sg.nseg; ++s_) {
+            const float* p = a.partial + (long long)work.slot_of(sg, s_) * slot_floats + row;
 #pragma unroll
-              for (int jx = 0; jx < kFix; ++jx) {
-                v[jx] += pv[jx];
-                w[jx] += pw_[jx];
-              }
-            }
+            for (int c0 = 0; c0 < COLS; c0 += 16) {
+              if (col0 + c0 < n_rows) {
+                float v[16], w[kGateUp ? 16 : 1];
 #pragma unroll
-            for (int jx = 0; jx < kFix; ++jx) {
-              const int n = n0 + jx;
-              if (n < n_end) {
-                float r = v[jx];
-                if (kGateUp) {
-                  float u = w[jx];
-                  if (a.round_h) {
-                    r = bf16_round(r);
-                    u = bf16_round(u);
-                  }
-                  r = swiglu_clamped(r, u, a.limit);
-                } else if (a.row_scale) {
-                  r *= a.row_scale[row_start + n];
+                for (int c = 0; c < 16; ++c) {
+                  const int n = col0 + c0 + c;
+                  v[c] = n < n_rows ? __ldcg(&p[(long long)n * kF8BlockM]) : 0.f;
+                  if (kGateUp) w[c] = n < n_rows ? __ldcg(&p[(long long)(slot_cols + n) * kF8BlockM]) : 0.f;
                 }
-                out[(long long)(row_start + n) * a.out_pitch + out_col] = __float2bfloat16_rn(r);
+#pragma unroll
+                for (int c = 0; c < 16; c += 2) {
+                  acc_g[(c0 + c) / 2] = fma2(pack2(v[c], v[c + 1]), one, acc_g[(c0 + c) / 2]);
+                  if (kGateUp) acc_u[(c0 + c) / 2] = fma2(pack2(w[c], w[c + 1]), one, acc_u[(c0 + c) / 2]);
+                }
               }
             }
           }
-          if (lane == 0) *counter = 0;
         }
+      }
+
+      if (finish) {
+        const bool quantise = kGateUp && a.q_out != nullptr;
+        unsigned peak[COLS / 32];  // quantise: lane l keeps the maximum of columns l (and l + 32) over this warp's rows
+        // values of 16 columns at a time; gate/up: after the activation
+        auto values = [&](int c0, float (&v)[16]) {
+#pragma unroll
+          for (int c = 0; c < 16; c += 2) {
+            float2 g = unpack2(acc_g[(c0 + c) / 2]);
+            if (kGateUp) {
+              float2 u = unpack2(acc_u[(c0 + c) / 2]);
+              if (a.round_h) {
+                g.x = bf16_round(g.x);
+                g.y = bf16_round(g.y);
+                u.x = bf16_round(u.x);
+                u.y = bf16_round(u.y);
+              }
+              g.x = swiglu_clamped(g.x, u.x, a.limit);
+              g.y = swiglu_clamped(g.y, u.y, a.limit);
+            }
+            v[c] = g.x;
+            v[c + 1] = g.y;
+          }
+        };
+        if (!quantise) {
+          __nv_bfloat16* st = reinterpret_cast<__nv_bfloat16*>(stage);
+          __nv_bfloat16* out = static_cast<__nv_bfloat16*>(a.out) + (long long)row_start * a.out_pitch + (long long)mb * kF8BlockM +
+                               wq * 32 + (lane & 3) * 8;
+#pragma unroll
+          for (int c0 = 0; c0 < COLS; c0 += 16) {
+            if (col0 + c0 < n_rows) {
+              float v[16];
+              values(c0, v);
+              if (!kGateUp && a.row_scale != nullptr) {
+#pragma unroll
+                for (int c = 0; c < 16; ++c) v[c] *= __shfl_sync(0xffffffffu, row_scale[c0 / 32], (c0 + c) & 31);
+              }
+              __syncwarp();
+#pragma unroll
+              for (int c = 0; c < 16; ++c) st[c * 32 + lane] = __float2bfloat16_rn(v[c]);
+              __syncwarp();
+#pragma unroll
+              for (int h = 0; h < 2; ++h) {
+                const int n = col0 + c0 + 8 * h + (lane >> 2);
+                const uint4 x = reinterpret_cast<const uint4*>(stage)[32 * h + lane];
+                if (n < n_rows) *reinterpret_cast<uint4*>(out + (long long)n * a.out_pitch) = x;
+              }
+            }
+          }
+        } else {
+          // 1. activations rounded to bf16 (what the quantiser is defined on), kept in the accumulators; column maxima
+#pragma unroll
+          for (int i = 0; i < COLS / 32; ++i) peak[i] = 0u;
+#pragma unroll
+          for (int c0 = 0; c0 < COLS; c0 += 16) {
+            if (col0 + c0 < n_rows) {
+              float v[16];
+              values(c0, v);
+#pragma unroll
+              for (int c = 0; c < 16; ++c) {
+                v[c] = bf16_round(v[c]);
+                const unsigned m = __reduce_max_sync(0xffffffffu, __float_as_uint(fabsf(v[c])));
+                if (lane == ((c0 + c) & 31)) peak[c0 / 32] = m;
+              }
+#pragma unroll
+              for (int c = 0; c < 16; c += 2) acc_g[(c0 + c) / 2] = pack2(v[c], v[c + 1]);
+            }
+          }
+          // 2. a token's group is the unit's 128 rows: maximum over the group's four warps, exchanged through the upper
+          //    half of their staging buffers, which the e4m3 bytes below leave free
+          auto maxima = [&](int q) { return reinterpret_cast<float*>(sStage + (grp * 4 + q) * kF8Stage + 512); };
+#pragma unroll
+          for (int i = 0; i < COLS / 32; ++i) maxima(wq)[32 * i + lane] = __uint_as_float(peak[i]);
+          ok = group_sync();
+          if (!ok) break;
+          float inv[COLS / 32];
+#pragma unroll
+          for (int i = 0; i < COLS / 32; ++i) {
+            const int at = 32 * i + lane;
+            const float scale = group_scale(fmaxf(fmaxf(maxima(0)[at], maxima(1)[at]), fmaxf(maxima(2)[at], maxima(3)[at])));
+            inv[i] = 1.f / scale;
+            const int n = col0 + at;
+            if (wq == 0 && n < n_rows) a.q_scale[(long long)(row_start + n) * a.q_scale_pitch + mb] = scale;
+          }
+          // A warp that runs ahead writes its next maxima a unit later; with more K blocks than accumulator stages
+          // that unit needed the slowest warp's arrivals, otherwise they meet again here.
+          if (sg.nseg > 1 || a.k_blocks <= 2 * Cfg::kTmpStages) {
+            ok = group_sync();
+            if (!ok) break;
+          }
+          // 3. e4m3 bytes, transposed through shared memory: 16 bytes per lane
+          uint8_t* out = static_cast<uint8_t*>(a.q_out) + (long long)row_start * a.q_pitch + (long long)mb * kF8BlockM + wq * 32 +
+                         (lane & 1) * 16;
+#pragma unroll
+          for (int c0 = 0; c0 < COLS; c0 += 16) {
+            if (col0 + c0 < n_rows) {
+              __syncwarp();
+#pragma unroll
+              for (int c = 0; c < 16; ++c) {
+                const float2 v = unpack2(acc_g[(c0 + c) / 2]);
+                stage[c * 32 + lane] = to_e4m3(c & 1 ? v.y : v.x, __shfl_sync(0xffffffffu, inv[c0 / 32], (c0 + c) & 31));
+              }
+              __syncwarp();
+              const int n = col0 + c0 + (lane >> 1);
+              const uint4 x = reinterpret_cast<const uint4*>(stage)[lane];
+              if (n < n_rows) *reinterpret_cast<uint4*>(out + (long long)n * a.q_pitch) = x;
+            }
+          }
+        }
+        if (kGateUp && a.tile_done != nullptr && sg.nseg > 1) {  // only the group that finished a cut unit knows
+          __threadfence();  // every lane's stores are visible device-wide before the count
+          __syncwarp();
+          if (lane == 0) atomicAdd(a.tile_done + sg.tt, 1);
+        }
+      }
+      if (kGateUp && a.tile_done != nullptr) {  // warp 3 reports whole units
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&epi_bar[n_it & 1]);
       }
       ++n_it;
     }
-    if (it.bad_tile && pw == 0 && lane == 0) report_status(a.status, kBadArgument, 7, blockIdx.x, 0);
   }
 
   __syncwarp();
@@ -599,38 +802,10 @@ quant_rows_kernel(const uint8_t* x, long long x_pitch, const int* row_index, int
   if (valid_off >= 0 && __ldcg(reinterpret_cast<const int*>(row + valid_off)) == 0) return;
   const int chunks = hidden / 8;
   const int groups = hidden / 128;
-  for (int c = threadIdx.x; c < chunks; c += blockDim.x) {
-    const uint4 v = __ldcg(reinterpret_cast<const uint4*>(row) + c);
-    const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&v);
-    float f[8];
-    float amax = 0.f;
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const float2 t = __bfloat1622float2(h[i]);
-      f[2 * i] = t.x;
-      f[2 * i + 1] = t.y;
-      amax = fmaxf(amax, fmaxf(fabsf(t.x), fabsf(t.y)));
-    }
-    // 16 consecutive threads hold one 128-wide group (chunks is a multiple of 16, so a group is either
-    // fully active or fully idle in the last sweep)
-    const unsigned active = __activemask();
-#pragma unroll
-    for (int off = 8; off > 0; off >>= 1) amax = fmaxf(amax, __shfl_xor_sync(active, amax, off));
-    const float scale = fmaxf(amax, 1e-10f) / 448.f;
-    const float inv = 1.f / scale;
-    uint2 packed;
-    uint8_t* pb = reinterpret_cast<uint8_t*>(&packed);
-#pragma unroll
-    for (int i = 0; i < 8; ++i)
-      pb[i] = (uint8_t)__nv_cvt_float_to_fp8(f[i] * inv, __NV_SATFINITE, __NV_E4M3);
-    reinterpret_cast<uint2*>(q + (long long)r * hidden)[c] = packed;
-    if ((c & 15) == 0) scales[(long long)r * groups + (c >> 4)] = scale;
-  }
+  // (chunks is a multiple of 16, so a group is either fully active or fully idle in the last sweep)
+  for (int c = threadIdx.x; c < chunks; c += blockDim.x)
+    quant_chunk(row, c, q + (long long)r * hidden, scales + (long long)r * groups);
 }
-
-typedef CUresult (*F8EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
-                                    const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
-                                    CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
 
 template <bool kGateUp, int N_MAX>
 static int launch_f8(const void* tmap, const mf_gemm_args* args, int grid, cudaStream_t stream) {
@@ -658,6 +833,9 @@ static int check_f8(const mf_gemm_args* a, int n_max, int grid) {
   if (a->m_blocks < 1 || a->k_blocks < 1 || a->k_blocks > kF8MaxKb) return -3;
   if ((a->b_pitch & 15) != 0 || (reinterpret_cast<uintptr_t>(a->b_base) & 15) != 0) return -4;
   if (!a->w_scale || !a->b_scale) return -5;
+  if (a->q_out ? (!a->q_scale || (a->q_pitch & 15) != 0 || (reinterpret_cast<uintptr_t>(a->q_out) & 15) != 0)
+               : (!a->out || (a->out_pitch & 7) != 0 || (reinterpret_cast<uintptr_t>(a->out) & 15) != 0))
+    return -7;  // 16-byte stores
   return 0;
 }
 

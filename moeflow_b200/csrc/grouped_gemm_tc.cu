@@ -16,15 +16,15 @@
 // the units are cut along K come from a device-side plan (see expert_meta.cu), so nothing is read back
 // to the host.  Two cuts exist:
 //   * K split S in {1, 2, 4, 8} (plan word = S): every unit is cut into S equal segments, segments are
-//     dealt to the CTAs round-robin;
+//     handed to the CTAs one by one (work_iter.cuh);
 //   * stream-K (plan word = 0): the units' K steps are laid end to end and every CTA takes one contiguous
 //     share of that line, so all CTAs stream the same number of weight bytes whatever the unit count
 //     (no partly filled last round); a unit that straddles CTA boundaries is cut there.
 // A segment that is not a whole unit stores its fp32 partial sums; the last segment to arrive (per
 // 32-row quarter) adds the segments in K order, so the result does not depend on arrival order.
 //
-// Warp roles (256 threads, one CTA per SM, persistent over units blockIdx.x, +gridDim.x, ...):
-//   warp 0      TMA producer for the weight tiles (lane 0 issues)
+// Warp roles (256 threads, one CTA per SM, persistent):
+//   warp 0      TMA producer for the weight tiles (lane 0 issues); hands the segments out to the other roles
 //   warp 1      UMMA issuer (lane 0 issues); owns the tensor-memory allocation
 //   warps 2-3   token-operand producers: gather rows by index with cp.async into the swizzled tile
 //   warps 4-7   epilogue: tcgen05.ld -> registers -> activation / scale -> global
@@ -258,7 +258,8 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint8_t* sA = smem;                                 // STAGES x kStageA
   uint8_t* sB = smem + STAGES * Cfg::kStageA;         // STAGES x kStageB
-  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + STAGES * Cfg::kStageBytes);
+  SegRing* ring = reinterpret_cast<SegRing*>(smem + STAGES * Cfg::kStageBytes);
+  uint64_t* bars = reinterpret_cast<uint64_t*>(ring + 1);
   uint64_t* full_bar = bars;                          // [STAGES]
   uint64_t* empty_bar = bars + STAGES;                // [STAGES]
   uint64_t* acc_full = bars + 2 * STAGES;             // [kMaxAccStages]
@@ -268,6 +269,8 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
   int* ret_desc = reinterpret_cast<int*>(ret_empty + 4 * kRetDepth);  // [4][kRetDepth][4]: n_rows, row_start, mb
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(ret_desc + 4 * kRetDepth * 4);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+  static_assert(sizeof(SegRing) + (2 * STAGES + 2 * kMaxAccStages + 8 * kRetDepth) * 8 + 4 * kRetDepth * 16 + 8 <= 1024,
+                "barriers, segment ring and return queue");
   uint8_t* out_stage = smem + STAGES * Cfg::kStageBytes + 1024;  // [4 epilogue warps][kOutStageBytes]
   // The fused return path runs on four extra warps (the kernel is then launched with 384 threads).
   constexpr bool with_return = kReturn;  // the down GEMM with four extra warps for the fused return path
@@ -309,6 +312,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
       mbar_init(&ret_full[s], 1);
       mbar_init(&ret_empty[s], 1);
     }
+    ring->init(1 + (b_tma ? 1 : 2) + 4 * kGroups);  // UMMA, token producers, epilogue
     *abort_flag = 0;
     fence_mbar_init();
     tma_prefetch_desc(&tmap_w);
@@ -382,13 +386,15 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
     }
   }
 
+  SegReader reader(ring, abort_flag, wait_ns);
   if (warp == 0) {
     // ------------------------------------------------------------------ weight TMA producer
     PipeState st;
     bool ok = true;
-    WorkIter it = work;
+    SegFeed feed(work, ring, abort_flag, wait_ns);
     Seg sg;
-    while (ok && it.next(sg)) {
+    bool have = feed.first(sg);
+    while (ok && have) {
       const int row0 = sg.e * a.rows_per_expert + sg.mb * (a.two_blocks ? 2 * kBlockM : kBlockM);
       for (int j = 0; j < sg.nkb; ++j) {
         const int kb = sg.kb0 + j;
@@ -407,8 +413,11 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
         }
         __syncwarp();
         st.advance(STAGES);
+        feed.advance();
       }
+      if (ok) have = feed.next(sg);
     }
+    if (feed.bad_tile && lane == 0) report_status(a.status, kBadArgument, 7, blockIdx.x, 0);
     if (!ok) {
       // Give copies that are still in flight a moment to land before the CTA goes away.
       const unsigned long long t0 = global_timer_ns();
@@ -418,9 +427,8 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
     // ------------------------------------------------------------------ UMMA issuer
     PipeState st, acc;
     bool ok = true;
-    WorkIter it = work;
     Seg sg;
-    while (ok && it.next(sg)) {
+    while (ok && reader.next(sg, ok)) {
       const uint32_t n_tile = (uint32_t)((sg.n_rows + 15) & ~15);
       const uint32_t idesc = umma_idesc(1, 1, kBlockM, n_tile < 16 ? 16 : n_tile);
       ok = mbar_wait_bounded(&acc_empty[acc.stage], acc.phase ^ 1u, abort_flag, wait_ns);
@@ -466,10 +474,9 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
     if (warp == 2) {
       PipeState st;
       bool ok = true;
-      WorkIter it = work;
       Seg sg;
       int ready_tile = -1;
-      while (ok && it.next(sg)) {
+      while (ok && reader.next(sg, ok)) {
         if (a.tile_wait != nullptr && sg.tt != ready_tile) {
           // the tile's activations are final once every gate/up unit of the tile has reported its four quarters
           bool got = true;
@@ -519,10 +526,19 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
     const uint32_t sw_off = (uint32_t)((chunk ^ r_in) << 4);
     PipeState st;
     bool ok = true;
-    WorkIter it = work;
-    Seg sg;
+    Seg sg, nx;
     int ready_tile = -1;
-    while (ok && it.next(sg)) {
+    int idx[N_MAX / 8];  // source rows of the segment at hand, fetched during the previous one
+    auto row_indices = [&](const Seg& s_) {
+#pragma unroll
+      for (int i = 0; i < N_MAX / 8; ++i) {
+        const int n = r_in + 8 * i;
+        if (n < s_.n_rows) idx[i] = a.b_index ? __ldcg(a.b_index + s_.row_start + n) : s_.row_start + n;
+      }
+    };
+    bool have = reader.next(sg, ok), more = false;
+    if (have) row_indices(sg);
+    while (ok && have) {
       if (a.tile_wait != nullptr && sg.tt != ready_tile) {
         bool got = wait_count_ge_gpu(a.tile_wait + sg.tt, a.tile_wait_target, wait_ns);
         ok = __all_sync(0xffffffffu, got);
@@ -542,11 +558,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
 #pragma unroll
       for (int i = 0; i < N_MAX / 8; ++i) {
         const int n = r_in + 8 * i;
-        rp[i] = nullptr;
-        if (n < n_rows) {
-          const long long idx = a.b_index ? (long long)a.b_index[sg.row_start + n] : (long long)(sg.row_start + n);
-          rp[i] = static_cast<const uint8_t*>(a.b_base) + idx * a.b_pitch + chunk * 16;
-        }
+        rp[i] = n < n_rows ? static_cast<const uint8_t*>(a.b_base) + (long long)idx[i] * a.b_pitch + chunk * 16 : nullptr;
       }
       for (int j = 0; j < sg.nkb; ++j) {
         const int kb = sg.kb0 + j;
@@ -568,7 +580,15 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
         }
         cp_async_mbar_arrive_noinc(&full_bar[st.stage]);
         st.advance(STAGES);
+        // the producer warp publishes the next segment during the third K block of this one
+        if (j == (sg.nkb < 4 ? sg.nkb - 1 : 3)) {
+          more = reader.next(nx, ok);
+          if (more) row_indices(nx);
+          if (!ok) break;
+        }
       }
+      sg = nx;
+      have = more;
     }
     // Drain this thread's cp.async operations before the CTA may exit.
     asm volatile("cp.async.wait_all;" ::: "memory");
@@ -599,9 +619,8 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
       rq.advance(kRetDepth);
       return true;
     };
-    WorkIter it = work;
     Seg sg;
-    while (ok && it.next(sg)) {
+    while (ok && reader.next(sg, ok)) {
       const int mb = sg.mb;
       const int n_rows = sg.n_rows;
       const int row_start = sg.row_start;
@@ -666,7 +685,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
       } else {
         // The unit is cut along K: park the fp32 partial sums, then the last quarter-warp to arrive adds
         // the segments in K order.
-        float* mine = a.partial + (long long)it.slot_of(sg, sg.seg) * slot_floats;
+        float* mine = a.partial + (long long)work.slot_of(sg, sg.seg) * slot_floats;
         for (int c0 = c_begin; c0 < c_end; c0 += 16) {
           uint32_t g[16], up[16];
           tmem_ld_16(taddr + c0, g);
@@ -701,7 +720,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
 #pragma unroll
             for (int j = 0; j < kFix; ++j) v[j] = w[j] = 0.f;
             for (int s = 0; s < sg.nseg; ++s) {
-              const float* p = a.partial + (long long)it.slot_of(sg, s) * slot_floats;
+              const float* p = a.partial + (long long)work.slot_of(sg, s) * slot_floats;
               float pv[kFix], pw[kFix];
 #pragma unroll
               for (int j = 0; j < kFix; ++j) {
@@ -739,7 +758,6 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
         }
       }
     }
-    if (it.bad_tile && warp == 4 && lane == 0) report_status(a.status, kBadArgument, 7, blockIdx.x, 0);
     if (with_return) enqueue_return(-1, 0, 0);  // tell the return warp that nothing more will come
   } else {
     // ------------------------------------------------------------------ return warps (fused owner reduce + push)

@@ -19,6 +19,8 @@ enum {
   MF_PLAN_N_ENTRIES = 3,  // valid (row, slot) entries = offsets[L]
   MF_PLAN_SLOT_COLS = 4,  // token columns per split-K partial slot (multiple of 16; 0 = the kernel's n_max)
   MF_PLAN_VALID_ROWS = 5, // received rows with at least one hit on this rank
+  MF_PLAN_NEXT1 = 6,      // segments handed out so far by the gate/up GEMM (zeroed by mf_expert_meta; mf_gemm_args.sched)
+  MF_PLAN_NEXT2 = 7,      // ... by the down GEMM
   MF_PLAN_WORDS = 8
 };
 
@@ -90,6 +92,15 @@ typedef struct {
   // mf_gemm_down only: 1 = a unit is two adjacent 128-row weight blocks (m_blocks counts pairs, up_row_offset
   // must be 128): the token tile is shared by both, which halves its L2 traffic per output column.
   int two_blocks;
+  // mf_gemm_gate_up_fp8 only, optional (q_out != NULL): the activations leave as e4m3 with one fp32 scale per row and
+  // 128-wide group (the definition of mf_quant_rows_1x128, on the bf16-rounded values) and `out` is not written.
+  void* q_out;               // [entries, q_pitch bytes]
+  long long q_pitch;
+  float* q_scale;            // [entries, q_scale_pitch]
+  long long q_scale_pitch;   // floats
+  // Optional: a device counter, zero when the kernel starts.  Segments of a K split then go to the CTA that asks next
+  // instead of round-robin (work_iter.cuh).
+  int* sched;
 } mf_gemm_args;
 
 // Encode a 2-D tiled tensor map (K innermost) for a weight matrix [rows, k_elems]; box = 128 bytes x
@@ -241,6 +252,10 @@ typedef struct {
   int late_launch;           // 1: the kernels that follow may only start when this one exits (no early launch)
   int plain_launch;          // 1: launched without programmatic serialization (starts when its predecessor has completed)
   int n_tile_done;           // words at counters1 + n_counters1: finished gate/up quarters per token tile (cleared per tile in use)
+  // Optional (one CTA of metadata, at most 8192 slot words): the launch also quantises the valid received rows, like
+  // mf_quant_rows_1x128, on CTAs of its own.
+  uint8_t* xq;               // [rows, H] e4m3
+  float* xs;                 // [rows, H / 128]
 } mf_meta_args;
 int mf_expert_meta(const mf_meta_args* args, mf_stream_t stream);
 // The K-split rule of the metadata kernels, callable on the host (no device needed): the split in {1,2,4,8}

@@ -529,6 +529,9 @@ class FixedEPLayer:
             n_counters=self._counters2.numel(), **common,
         )
         self._a_gemm2.partial = self._partial[partial_floats:].data_ptr()
+        # units go to the CTA that asks next (the metadata kernel zeroes the counters)
+        self._a_gemm1.sched = self.plan[S.PLAN_NEXT1 :].data_ptr()
+        self._a_gemm2.sched = self.plan[S.PLAN_NEXT2 :].data_ptr()
         # Long prefill (256-row tiles): a down-projection unit covers two adjacent weight blocks, so a token tile is
         # fetched from L2 once per 256 output columns (gemm_kwargs down_two_blocks overrides).
         self.down_two_blocks = bool(self.gemm_kwargs.get("down_two_blocks", self.block_m >= 256)) and H % 256 == 0
@@ -615,7 +618,7 @@ class FixedEPLayer:
         if w13_local.dtype != torch.bfloat16 or w2_local.dtype != torch.bfloat16:
             raise ValueError("cuda backend takes bf16 weights")
         self.w13, self.w2 = w13_local.contiguous(), w2_local.contiguous()
-        self._fp8 = self._expand = None
+        self._bind_bf16()
         self._tmap13 = make_weight_tmap(self.w13)
         self._tmap2 = make_weight_tmap(self.w2)
 
@@ -702,6 +705,9 @@ class FixedEPLayer:
                                 up_row_offset=I, out=self.act.data_ptr(), out_pitch=I, row_scale=None, counters=g1.counters,
                                 n_counters=g1.n_counters, w_scale=None, b_scale=f["xs"].data_ptr(), b_scale_pitch=H // 128,
                                 **common)
+        # The gate/up kernel quantises its activations itself; the bf16 ones are not stored.
+        a1 = f["a1"]
+        a1.q_out, a1.q_pitch, a1.q_scale, a1.q_scale_pitch = f["aq"].data_ptr(), I, f["as"].data_ptr(), I // 128
         f["a2"] = _lib.GemmArgs(b_base=f["aq"].data_ptr(), b_pitch=I, b_index=None, split_word=_lib.PLAN_SPLIT2,
                                 m_blocks=H // 128, k_blocks=I // 128, rows_per_expert=H, up_row_offset=0,
                                 out=self.y.data_ptr(), out_pitch=H, row_scale=self.entry_w.data_ptr(), counters=g2.counters,
@@ -712,6 +718,13 @@ class FixedEPLayer:
 
             f["tm_aq"] = make_tile_tmap(f["aq"], self.block_m)  # the down GEMM reads its e4m3 token tiles by TMA
             f["a2"].b_tmap = C.addressof(f["tm_aq"])
+        a1.sched, f["a2"].sched = g1.sched, g2.sched
+        if self.tile_handover:  # one count per promotion warp of the gate/up kernel and weight block
+            a1.tile_done = self._tile_done.data_ptr()
+            f["a2"].tile_wait = self._tile_done.data_ptr()
+            f["a2"].tile_wait_target = (4 if self.block_m <= 32 else 8) * (I // 128)
+        # up to 8192 slot words the metadata launch quantises the received rows as well
+        f["in_meta"] = self.meta_ctas == 1 and rows * self.K <= 8192
         self._fp8_shared = f
         return f
 
@@ -719,7 +732,8 @@ class FixedEPLayer:
         """Point this (possibly shared) buffer set at one MoE layer's e4m3 weights; no copies."""
         if pack.get("expand"):
             e = self._expanded_weights()
-            self._fp8, self._expand = None, pack
+            self._bind_bf16()
+            self._expand = pack
             self.w13, self.w2, self._tmap13, self._tmap2 = e["w13"], e["w2"], e["tm13"], e["tm2"]
             return
         self._expand = None
@@ -727,6 +741,8 @@ class FixedEPLayer:
         f["a1"].w_scale, f["a2"].w_scale = pack["s13"].data_ptr(), pack["s2"].data_ptr()
         f["tm13"], f["tm2"], f["pack"] = pack["tm13"], pack["tm2"], pack
         self._fp8 = f
+        if f["in_meta"]:
+            self._a_meta.xq, self._a_meta.xs = f["xq"].data_ptr(), f["xs"].data_ptr()
         self.w13, self.w2 = pack["w13"], pack["w2"]
         self._tmap13, self._tmap2 = pack["tm13"], pack["tm2"]
 
@@ -746,8 +762,12 @@ class FixedEPLayer:
         if tmap13 is None or tmap2 is None:
             self.set_weights(w13_local, w2_local)
             return
-        self._fp8 = self._expand = None
+        self._bind_bf16()
         self.w13, self.w2, self._tmap13, self._tmap2 = w13_local, w2_local, tmap13, tmap2
+
+    def _bind_bf16(self) -> None:
+        self._fp8 = self._expand = None
+        self._a_meta.xq = self._a_meta.xs = None
 
     def _cuda_dispatch(self, x, weights, ids, num_valid, logits=None, bias=None) -> torch.Tensor:
         from .ops import _lib
@@ -799,15 +819,13 @@ class FixedEPLayer:
             return
         if self._fp8 is not None:
             f, lib = self._fp8, self._lib
-            valid_off = self.H * 2 + 2 * self.K * 4  # byte offset of a received row's valid flag
-            _lib.check(lib.mf_quant_rows_1x128(self._recv_store.data_ptr(), self.pitch * 2, None, self.world * self.C, self.H,
-                                               f["xq"].data_ptr(), f["xs"].data_ptr(), valid_off, None, s), "quantise rows")
+            if not f["in_meta"]:
+                valid_off = self.H * 2 + 2 * self.K * 4  # byte offset of a received row's valid flag
+                _lib.check(lib.mf_quant_rows_1x128(self._recv_store.data_ptr(), self.pitch * 2, None, self.world * self.C, self.H,
+                                                   f["xq"].data_ptr(), f["xs"].data_ptr(), valid_off, None, s), "quantise rows")
             _lib.check(lib.mf_gemm_gate_up_fp8(f["tm13"], C.byref(f["a1"]), self.block_m, self.n_sms, s), "fp8 gate/up gemm")
             if stop_after == "GEMM1":
                 return
-            entries = self.plan[_lib.PLAN_N_ENTRIES :]
-            _lib.check(lib.mf_quant_rows_1x128(self.act.data_ptr(), self.I * 2, None, self.n_entries, self.I, f["aq"].data_ptr(),
-                                               f["as"].data_ptr(), -1, entries.data_ptr(), s), "quantise activations")
             _lib.check(lib.mf_gemm_down_fp8(f["tm2"], C.byref(f["a2"]), self.block_m, self.n_sms, s), "fp8 down gemm")
             if stop_after == "GEMM2":
                 return

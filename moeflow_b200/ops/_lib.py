@@ -13,7 +13,8 @@ from pathlib import Path
 
 LIB_PATH = Path(__file__).resolve().parent.parent / "_lib" / "libmoeflow_b200.so"
 
-PLAN_N_TILES, PLAN_SPLIT1, PLAN_SPLIT2, PLAN_N_ENTRIES, PLAN_SLOT_COLS, PLAN_VALID_ROWS, PLAN_WORDS = 0, 1, 2, 3, 4, 5, 8
+PLAN_N_TILES, PLAN_SPLIT1, PLAN_SPLIT2, PLAN_N_ENTRIES, PLAN_SLOT_COLS, PLAN_VALID_ROWS = 0, 1, 2, 3, 4, 5
+PLAN_NEXT1, PLAN_NEXT2, PLAN_WORDS = 6, 7, 8
 
 STATUS_NAMES = {
     0: "ok",
@@ -79,6 +80,11 @@ class GemmArgs(C.Structure):
         ("tile_wait", C.c_void_p),
         ("tile_wait_target", C.c_int),
         ("two_blocks", C.c_int),
+        ("q_out", C.c_void_p),
+        ("q_pitch", C.c_longlong),
+        ("q_scale", C.c_void_p),
+        ("q_scale_pitch", C.c_longlong),
+        ("sched", C.c_void_p),
     ]
 
 
@@ -180,6 +186,8 @@ class MetaArgs(C.Structure):
         ("late_launch", C.c_int),
         ("plain_launch", C.c_int),
         ("n_tile_done", C.c_int),
+        ("xq", C.c_void_p),
+        ("xs", C.c_void_p),
     ]
 
 
