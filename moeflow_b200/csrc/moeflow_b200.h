@@ -292,6 +292,7 @@ typedef struct {
   unsigned long long* status;
   unsigned long long wait_ns;
   unsigned long long* trace; // optional [8] globaltimer stamps of CTA 0 (profiling aid), or NULL
+  int rows;                  // > 0: only these first rows of `out` are written (a caller's buffer shorter than C)
 } mf_combine_args;
 int mf_combine(const mf_combine_args* args, mf_stream_t stream);
 
@@ -316,6 +317,12 @@ int mf_quant_rows_1x128(const void* x, long long x_pitch, const int* row_index, 
 // b_base rows are e4m3 bytes, k_blocks = K / 128, the tensor map is built with elem_bytes = 1; n_max 32 or 64).
 int mf_gemm_gate_up_fp8(const void* tmap, const mf_gemm_args* args, int n_max, int grid, mf_stream_t stream);
 int mf_gemm_down_fp8(const void* tmap, const mf_gemm_args* args, int n_max, int grid, mf_stream_t stream);
+
+// ---- captured forwards ------------------------------------------------------------------------------------
+// mf_capture_last_node: the kernel node that the capture on `stream` added last.  mf_graph_set_args: replaces the single
+// by-value argument struct of such a node in the executable graph made from that capture.
+int mf_capture_last_node(mf_stream_t stream, void** node_out);
+int mf_graph_set_args(void* graph_exec, void* node, const void* args);
 
 // ---- peer-memory runtime ------------------------------------------------------------------------------------
 int mf_peer_alloc(void** ptr, unsigned long long bytes);

@@ -119,6 +119,7 @@ __global__ void __launch_bounds__(kThreads) combine_kernel(const mf_combine_args
   // the values are read after the wait), so that the read below does not go to DRAM.
   unsigned long long* trace = (a.trace != nullptr && blockIdx.x == 0 && tid == 0) ? a.trace : nullptr;
   if (trace) trace[0] = global_timer_ns();
+  if (a.rows > 0 && t >= a.rows) return;
   if (tid == 0) asm volatile("prefetch.global.L2 [%0];" ::"l"(a.hit + (size_t)t * a.R));
   // touch the pages read after the wait: flags, push count, this token's row in every owner's return block
   if (tid < a.R) {

@@ -52,22 +52,48 @@ __device__ __forceinline__ void route_token_warp(const float* __restrict__ lg, c
                                                  float* score, float* biased, const RouteParams& p, int lane,
                                                  float& out_w, int& out_id) {
   const int E = p.E;
+  if (E <= 32 * kRouteRegs) {
+    // All of the lane's logits and biases are requested before the first one is used: they are usually cold, and a
+    // loop that computes on each as it comes pays the DRAM latency once per unrolled round.
+    float l[kRouteRegs], b[kRouteRegs];
+#pragma unroll
+    for (int j = 0; j < kRouteRegs; ++j) {
+      const int e = lane + 32 * j;
+      if (e < E) {
+        l[j] = lg[e];
+        b[j] = bias ? bias[e] : 0.f;
+      }
+    }
+#pragma unroll
+    for (int j = 0; j < kRouteRegs; ++j) {
+      const int e = lane + 32 * j;
+      if (e < E) {
+        score[e] = l[j];
+        biased[e] = b[j];
+      }
+    }
+  } else {
+    for (int e = lane; e < E; e += 32) {
+      score[e] = lg[e];
+      biased[e] = bias ? bias[e] : 0.f;
+    }
+  }
   if (p.sigmoid) {
-    for (int e = lane; e < E; e += 32) score[e] = 1.f / (1.f + expf(-lg[e]));
+    for (int e = lane; e < E; e += 32) score[e] = 1.f / (1.f + expf(-score[e]));
   } else {
     float m = -CUDART_INF_F;
-    for (int e = lane; e < E; e += 32) m = fmaxf(m, lg[e]);
+    for (int e = lane; e < E; e += 32) m = fmaxf(m, score[e]);
     for (int off = 16; off > 0; off >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, off));
     float s = 0.f;
     for (int e = lane; e < E; e += 32) {
-      const float x = expf(lg[e] - m);
+      const float x = expf(score[e] - m);
       score[e] = x;
       s += x;
     }
     for (int off = 16; off > 0; off >>= 1) s += __shfl_xor_sync(0xffffffffu, s, off);
     for (int e = lane; e < E; e += 32) score[e] = score[e] / s;
   }
-  for (int e = lane; e < E; e += 32) biased[e] = bias ? score[e] + bias[e] : score[e];
+  for (int e = lane; e < E; e += 32) biased[e] = bias ? score[e] + biased[e] : score[e];
   __syncwarp();
 
   if (p.n_group > 1) {

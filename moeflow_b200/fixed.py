@@ -596,6 +596,7 @@ class FixedEPLayer:
             push_epoch=self._push_epoch.data_ptr(),
         )
         self._scratch_out = None
+        self._node_log: dict | None = None  # during a capture: graph nodes of the dispatch and combine kernels
         self._a_combine = S.CombineArgs(
             ret=self.ret_recv.data_ptr(), hit=self.hit.data_ptr(), out=self.out.data_ptr(),
             flags=self._ret_flags.data_ptr() if R > 1 else None, epoch=self._push_epoch.data_ptr(), R=R, C=Cc, H=H, rank=self.rank,
@@ -794,6 +795,8 @@ class FixedEPLayer:
         a.T = x.shape[0]
         self._keep = [x, weights, ids, num_valid, logits, bias]
         _lib.check(self._lib.mf_dispatch_push(C.byref(a), _lib.stream_ptr()), "dispatch_push")
+        if self._node_log is not None:
+            self._node_log["dispatch"] = _lib.last_captured_node()
         return self.hit
 
     def _cuda_meta(self) -> None:
@@ -862,6 +865,8 @@ class FixedEPLayer:
         from .ops import _lib
 
         _lib.check(self._lib.mf_combine(C.byref(self._a_combine), _lib.stream_ptr()), "combine")
+        if self._node_log is not None:
+            self._node_log["combine"] = _lib.last_captured_node()
         return self.out
 
     def check_status(self) -> dict:

@@ -1,26 +1,36 @@
 """Serving-side wrapper of one routed MoE layer: static buffers + one CUDA graph.
 
-``GraphedMoELayer`` is the call a user makes on the hot path.  It owns device-side input buffers of
-the layer's capacity, captures ``FixedEPLayer.forward`` once, and then every call is: copy this step's
-hidden states and router logits in (host pinned memory or device tensors), replay the graph, and
-hand back the output rows.  Nothing is allocated and nothing is read back to the host by the layer
-itself, so the call can sit inside a larger captured decode step as well.
+``GraphedMoELayer`` is the call a user makes on the hot path.  It captures ``FixedEPLayer.forward`` once, and then
+every call is a replay on this step's hidden states and router logits.  Nothing is allocated and nothing is read back
+to the host by the layer itself, so the call can sit inside a larger captured decode step as well.
 
 Two ways to feed it:
 
-* ``layer(x, logits, out)``: two tensors (pinned host or device), two copies and a fill of the row count.
-* ``layer.step(block, out)``: ``block = layer.new_pinned_inputs()`` is one pinned host block laid out exactly
-  like the device-side input block — hidden rows, logits, row count — which the caller fills in place
-  (``block.x``, ``block.logits``, ``block.set_rows(t)``).  A step is then a single host-to-device copy, the
-  replay, and one device-to-host copy of the output rows: three stream operations instead of five.
+* ``layer(x, logits, out)``: two tensors (pinned host or device);
+* ``layer.step(block, out)``: ``block = layer.new_pinned_inputs()`` is one pinned host block laid out like the
+  device-side input block — hidden rows, logits, row count — which the caller fills in place (``block.x``,
+  ``block.logits``, ``block.set_rows(t)``) and does not touch again before the step is done.
+
+On the cuda backend the captured graph has no buffers of its own in the way: its first kernel reads the caller's
+device tensors and its last one writes the caller's output rows (device, or pinned host memory at decode sizes), by
+updating the two kernel nodes' arguments when pointers or row count change.  Other inputs (host memory, other dtypes or
+strides) are copied into the static buffers ``.x`` / ``.logits`` / ``.num_valid`` first, which is also what ``load`` and
+``replay`` work on.  The small copies and the gap in front of the graph were 13 us of a device-fed call.  A pinned input
+block is still one copy: read by the first kernel itself over PCIe, 24 rows took 43 us, the copy engine needs 9.
 """
 
 from __future__ import annotations
+
+import ctypes as C
+from collections import deque
 
 import torch
 import torch.distributed as dist
 
 from ..fixed import FixedEPLayer
+
+#: Up to this many rows of pinned output are written by the combine kernel itself; beyond it the copy engine moves them.
+MAX_HOST_ROWS = 128
 
 
 class PinnedInputs:
@@ -50,6 +60,9 @@ class GraphedMoELayer:
         self.x, self.logits, self.num_valid = self._views(self._block)
         self.num_valid.fill_(layer.C)
         self.graph: torch.cuda.CUDAGraph | None = None
+        self._nodes: dict | None = None  # kernel nodes whose arguments follow the caller's buffers
+        self._bound = None               # what they point at: (x, logits, rows, out), or None for the static buffers
+        self._host_refs: deque = deque(maxlen=8)  # pinned outputs that recent replays may still be writing
         self._warmup = warmup
         # route+dispatch, meta (two launches in its multi-CTA form), gate/up, down(+reduce+push), combine
         self.kernels_per_step = (5 if getattr(layer, "fuse_return", False) else 6) + (
@@ -82,12 +95,60 @@ class GraphedMoELayer:
         torch.cuda.synchronize()
         if dist.is_available() and dist.is_initialized():
             dist.barrier(group=self.layer.group)
-        graph = torch.cuda.CUDAGraph()
-        with torch.cuda.graph(graph):
-            self.out = self._forward()
-        self.graph = graph
+        native = self.layer.backend == "cuda"
+        graph = torch.cuda.CUDAGraph(keep_graph=native)
+        nodes = {} if native else None
+        self.layer._node_log = nodes
+        try:
+            with torch.cuda.graph(graph):
+                self.out = self._forward()
+        finally:
+            self.layer._node_log = None
+        if native:
+            from ..ops import _lib
+
+            graph.instantiate()
+            a, c = _lib.DispatchArgs(), _lib.CombineArgs()
+            C.memmove(C.byref(a), C.byref(self.layer._a_dispatch), C.sizeof(a))
+            C.memmove(C.byref(c), C.byref(self.layer._a_combine), C.sizeof(c))
+            self._dispatch_args, self._combine_args, self._set_args = a, c, _lib.lib().mf_graph_set_args
+            self._exec, self._raw = graph.raw_cuda_graph_exec(), graph.raw_cuda_graph()
+        self.graph, self._nodes, self._bound = graph, nodes, None
         torch.cuda.synchronize()
         return self
+
+    def _bind(self, key) -> None:
+        """Point the captured forward at ``key = (x, logits, rows, out)`` (addresses; ``out`` None: the layer's own
+        buffer), or back at the static buffers (``key`` None)."""
+        if key == self._bound:
+            return
+        from ..ops import _lib
+
+        a, c = self._dispatch_args, self._combine_args
+        layer = self.layer
+        if key is None:
+            a.x, a.logits, a.T, a.num_valid = self.x.data_ptr(), self.logits.data_ptr(), layer.C, self.num_valid.data_ptr()
+            out, rows = None, 0
+        else:
+            a.x, a.logits, a.T, out = key
+            a.num_valid, rows = None, key[2]
+        was = None if self._bound is None else self._bound[3]
+        _lib.check(self._set_args(self._exec, self._nodes["dispatch"], C.addressof(a)), "graph update")
+        if out != was or out is not None:
+            c.out, c.rows = (layer.out.data_ptr(), 0) if out is None else (out, rows)
+            _lib.check(self._set_args(self._exec, self._nodes["combine"], C.addressof(c)), "graph update")
+        self._bound = key
+
+    def _readable(self, x: torch.Tensor, logits: torch.Tensor) -> bool:
+        """Can the captured kernels read these tensors where they are?"""
+        cfg, dev = self.layer.cfg, self.x.device
+        return (x.device == dev and logits.device == dev and x.dtype == torch.bfloat16 and logits.dtype == torch.float32
+                and x.dim() == 2 and x.shape[1] == cfg.hidden_size and logits.shape == (x.shape[0], cfg.n_routed_experts)
+                and x.is_contiguous() and logits.is_contiguous() and x.data_ptr() % 16 == 0 and 0 < x.shape[0] <= self.layer.C)
+
+    def _writable(self, out: torch.Tensor | None, rows: int, shape_ok) -> bool:
+        return (out is not None and out.dtype == torch.bfloat16 and out.is_contiguous() and out.data_ptr() % 16 == 0
+                and shape_ok and (out.device == self.x.device or (out.device.type == "cpu" and rows <= MAX_HOST_ROWS and out.is_pinned())))
 
     def load(self, x: torch.Tensor, logits: torch.Tensor) -> int:
         """Copy one step's inputs (``[T, H]``, ``[T, E]``; host-pinned or device) into the static buffers."""
@@ -102,29 +163,52 @@ class GraphedMoELayer:
     def replay(self) -> torch.Tensor:
         if self.graph is None:
             self.capture()
+        if self._nodes is not None:
+            self._bind(None)
         self.graph.replay()
         return self.out
 
     def __call__(self, x: torch.Tensor, logits: torch.Tensor, out: torch.Tensor | None = None) -> torch.Tensor:
         """One step.  With ``out`` (e.g. a pinned host tensor ``[T, H]``) the rows are copied there."""
-        t = self.load(x, logits)
-        res = self.replay()[:t]
+        if self.graph is None:
+            self.capture()
+        t = x.shape[0]
+        if self._nodes is not None and self._readable(x, logits):
+            if out is not None and out.is_cuda and self._writable(out, t, tuple(out.shape) == tuple(x.shape)):
+                self._bind((x.data_ptr(), logits.data_ptr(), t, out.data_ptr()))
+                self.graph.replay()
+                return out
+            self._bind((x.data_ptr(), logits.data_ptr(), t, None))
+            self.graph.replay()
+            res = self.out[:t]
+        else:
+            t = self.load(x, logits)
+            res = self.replay()[:t]
         if out is not None:
             out.copy_(res, non_blocking=True)
             return out
         return res
 
     def step(self, inputs: PinnedInputs, out: torch.Tensor | None = None) -> torch.Tensor:
-        """One step from a pinned input block: one host-to-device copy, the replay, one copy of the rows out."""
-        if inputs.rows > self.layer.C:
-            raise ValueError(f"{inputs.rows} tokens exceed capacity {self.layer.C}")
+        """One step from a pinned input block; with ``out`` (``[>= T, H]``, pinned host or device) the rows go there."""
+        t = inputs.rows
+        if t > self.layer.C:
+            raise ValueError(f"{t} tokens exceed capacity {self.layer.C}")
+        if self.graph is None:
+            self.capture()
         self._block.copy_(inputs.raw, non_blocking=True)
-        res = self.replay()[: inputs.rows]
+        if (self._nodes is not None and t > 0 and
+                self._writable(out, t, out is not None and out.dim() == 2 and out.shape[0] >= t and out.shape[1] == self.layer.H)):
+            self._bind((self.x.data_ptr(), self.logits.data_ptr(), t, out.data_ptr()))
+            self._host_refs.append(out)
+            self.graph.replay()
+            return out
+        res = self.replay()[:t]
         if out is not None:
-            out[: inputs.rows].copy_(res, non_blocking=True)
+            out[:t].copy_(res, non_blocking=True)
             return out
         return res
 
     def close(self) -> None:
         """Drop the graph (do this before destroying the process group)."""
-        self.graph = None
+        self.graph = self._nodes = self._bound = None

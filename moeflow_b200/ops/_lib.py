@@ -227,6 +227,7 @@ class CombineArgs(C.Structure):
         ("status", C.c_void_p),
         ("wait_ns", C.c_ulonglong),
         ("trace", C.c_void_p),
+        ("rows", C.c_int),
     ]
 
 
@@ -274,6 +275,8 @@ def lib() -> C.CDLL:
         "mf_owner_reduce_push": [C.POINTER(ReducePushArgs), P],
         "mf_combine": [C.POINTER(CombineArgs), P],
         "mf_expert_prepare": [P, LL, I, I, I, I, I, P, P, P, P, P],
+        "mf_capture_last_node": [P, C.POINTER(P)],
+        "mf_graph_set_args": [P, P, P],
         "mf_peer_alloc": [C.POINTER(P), ULL],
         "mf_peer_free": [P],
         "mf_peer_export": [P, P],
@@ -311,6 +314,13 @@ def stream_ptr() -> int:
     import torch
 
     return torch.cuda.current_stream().cuda_stream
+
+
+def last_captured_node() -> int:
+    """Handle of the kernel node that the capture on the current stream added last."""
+    node = C.c_void_p()
+    check(lib().mf_capture_last_node(stream_ptr(), C.byref(node)), "captured node")
+    return node.value
 
 
 def decode_status(word: int) -> dict:

@@ -1,0 +1,80 @@
+"""``GraphedMoELayer`` replays on the caller's own buffers: device tensors, pinned blocks, changing pointers and row
+counts, and back to the static buffers.  Every call must give exactly what an eager forward gives."""
+
+import pytest
+import torch
+
+from moeflow_b200 import MoEConfig
+from moeflow_b200.testing import make_bias, make_hidden, make_logits, make_weights
+
+pytestmark = pytest.mark.gpu
+
+CFG = MoEConfig(hidden_size=512, moe_intermediate_size=256, n_routed_experts=16, top_k=4)
+
+
+def _make(capacity):
+    from moeflow_b200.fixed import FixedEPLayer
+    from moeflow_b200.models.routed_moe import GraphedMoELayer
+
+    w13, w2 = make_weights(CFG, 0, device="cuda")
+    bias = make_bias(CFG, 1, device="cuda")
+    eager = FixedEPLayer(CFG, 0, 1, w13, w2, capacity=capacity, backend="cuda", wait_ns=50_000_000)
+    graphed = GraphedMoELayer(FixedEPLayer(CFG, 0, 1, w13, w2, capacity=capacity, backend="cuda", wait_ns=50_000_000), bias).capture()
+
+    def reference(x, logits):
+        return eager.forward(x, logits, bias)[: x.shape[0]].clone()
+
+    return graphed, reference
+
+
+def _inputs(tokens, seed):
+    return make_hidden(tokens, CFG, seed, device="cuda"), make_logits(tokens, CFG, seed + 50, device="cuda")
+
+
+@pytest.mark.parametrize("capacity", [1, 16, 130])
+def test_device_tensors_and_static_buffers_alternate(capacity):
+    graphed, reference = _make(capacity)
+    sizes = sorted({1, (capacity + 1) // 2, capacity})
+    for seed, t in enumerate(sizes + sizes[::-1]):
+        x, lg = _inputs(t, seed)
+        want = reference(x, lg)
+        assert torch.equal(graphed(x, lg), want)
+        into = torch.full((t, CFG.hidden_size), 7.0, dtype=torch.bfloat16, device="cuda")
+        assert graphed(x, lg, into) is into and torch.equal(into, want)
+        # strided rows and wider dtypes take the copying path
+        assert torch.equal(graphed(x.float().bfloat16().repeat_interleave(2, 0)[::2], lg), want)
+        pinned = torch.zeros(t, CFG.hidden_size, dtype=torch.bfloat16).pin_memory()
+        graphed(x.cpu().pin_memory(), lg.cpu().pin_memory(), pinned)
+        torch.cuda.synchronize()
+        assert torch.equal(pinned, want.cpu())
+        graphed.load(x, lg)
+        assert torch.equal(graphed.replay()[:t], want) and not graphed.replay()[t:].any()
+    assert graphed.layer.check_status()["code"] == 0
+    with pytest.raises(ValueError):
+        graphed(*_inputs(capacity + 1, 0))
+    graphed.close()
+
+
+@pytest.mark.parametrize("capacity", [1, 32, 300])
+def test_pinned_blocks(capacity):
+    """300 rows are above the direct limit and take the copy engine's way."""
+    graphed, reference = _make(capacity)
+    blocks = [graphed.new_pinned_inputs() for _ in range(2)]
+    for seed, t in enumerate([capacity, 1, (capacity + 1) // 2, capacity]):
+        x, lg = _inputs(t, seed)
+        want = reference(x, lg).cpu()
+        block = blocks[seed % 2]
+        block.x[:t].copy_(x)
+        block.logits[:t].copy_(lg)
+        block.set_rows(t)
+        out = torch.full((capacity, CFG.hidden_size), 7.0, dtype=torch.bfloat16).pin_memory()
+        graphed.step(block, out)
+        torch.cuda.synchronize()
+        assert torch.equal(out[:t], want) and (out[t:] == 7.0).all()  # rows past the batch stay the caller's
+        assert torch.equal(graphed.step(block).cpu(), want)
+        plain = torch.zeros(t, CFG.hidden_size, dtype=torch.bfloat16)  # pageable memory: copied
+        graphed.step(block, plain)
+        torch.cuda.synchronize()
+        assert torch.equal(plain, want)
+    assert graphed.layer.check_status()["code"] == 0
+    graphed.close()
