@@ -17,7 +17,9 @@
 // Replaces the reference's pack kernel plus its dispatch all_to_all_single
 // (moeflow/kernels/dispatch_pack.py:10-95, moeflow/fixed.py:95-125,234).
 #include "common.cuh"
+#include "expert_meta.cuh"
 #include "moeflow_b200.h"
+#include "quant.cuh"
 #include "router.cuh"
 
 namespace mf {
@@ -149,7 +151,130 @@ __global__ void __launch_bounds__(kDispatchThreads) dispatch_push_kernel(const m
   }
 }
 
+// The only rank is this GPU, decode sizes: dispatch and metadata in one launch.  There is no peer to wait for, so the CTA
+// that stores its row last goes on with the one-pass metadata build (expert_meta.cuh) on the rows it finds in L2: no
+// second launch, no flags, no cold start of another kernel behind a weight stream that has swept its code and pages out
+// of the caches.  The rows of e4m3 layers are quantised by the CTAs that hold them in registers.  512 threads: one
+// 16-byte chunk of a 4096-wide row each, and eight slot words each in the metadata pass.
+// 1 token on 288 experts, cold caches: 24.5 us for the two kernels, see the case table of the design notes.
+constexpr int kLocalThreads = 512;
+
+__global__ void __launch_bounds__(kLocalThreads) dispatch_local_kernel(const mf_dispatch_args a, const mf_meta_args m) {
+  extern __shared__ int s_dyn[];  // metadata pass, then the router's scores
+  __shared__ int s_id[kMaxTopK];
+  __shared__ float s_w[kMaxTopK];
+  __shared__ int s_last;
+  const int t = blockIdx.x, tid = threadIdx.x;
+  unsigned long long* trace = (a.trace != nullptr && blockIdx.x == 0 && tid == 0) ? a.trace : nullptr;
+  if (trace) trace[0] = global_timer_ns();
+  grid_dep_launch();
+  uint8_t* row = const_cast<uint8_t*>(static_cast<const uint8_t*>(m.recv)) + (size_t)t * a.pitch;
+  const bool has_token = t < a.T;
+  const uint4* xr = reinterpret_cast<const uint4*>(static_cast<const __nv_bfloat16*>(a.x) + (size_t)t * a.H);
+  const int chunks = a.H / 8;
+  uint4 xv[2];  // H <= 8192
+  if (has_token) {
+#pragma unroll
+    for (int i = 0; i < 2; ++i)
+      if (tid + i * kLocalThreads < chunks) xv[i] = xr[tid + i * kLocalThreads];
+  }
+  const bool live = has_token && (a.num_valid == nullptr || t < *a.num_valid);
+  if (tid < 32) {
+    float w = 0.f;
+    int id = -1;
+    if (a.logits != nullptr) {
+      if (has_token) {
+        float* score = reinterpret_cast<float*>(s_dyn + meta_smem_words(m.L, kLocalThreads));
+        const RouteParams p{a.E, a.K, a.n_group, a.topk_group, a.sigmoid, a.renorm, a.scale};
+        route_token_warp(a.logits + (size_t)t * a.E, a.bias, score, score + a.E, p, tid, w, id);
+        if (tid < a.K) {
+          a.route_w[(size_t)t * a.K + tid] = w;
+          a.route_ids[(size_t)t * a.K + tid] = id;
+        }
+      }
+    } else if (has_token && tid < a.K) {
+      id = a.ids[(size_t)t * a.K + tid];
+      w = a.weights[(size_t)t * a.K + tid];
+    }
+    if (tid < a.K) {
+      s_id[tid] = id;
+      s_w[tid] = w;
+    }
+  } else {
+    // in the shadow of the routing warp: the pages that the metadata pass stores to, and its histogram
+    if (tid < 48) {
+      const void* p = tid == 32 ? (const void*)m.plan : tid == 33 ? (const void*)m.offsets : tid == 34 ? (const void*)m.tile_e
+                    : tid == 35 ? (const void*)m.tile_s : tid == 36 ? (const void*)m.tile_n : tid == 37 ? (const void*)m.row_hits
+                    : tid == 38 ? (const void*)m.inv : tid == 39 ? (const void*)m.entry_row : tid == 40 ? (const void*)m.entry_slot
+                    : tid == 41 ? (const void*)m.entry_w : tid == 42 ? (const void*)(m.counters1 + m.n_counters1)
+                    : tid == 43 ? (const void*)(row + (size_t)a.H * 2) : tid == 44 ? (const void*)a.epoch
+                    : tid == 45 ? (const void*)a.done_counter : tid == 46 ? (const void*)(a.hit + t) : nullptr;
+      touch(p);
+    }
+  }
+  meta_begin<kLocalThreads>(m, s_dyn);
+  __syncthreads();
+  if (trace) trace[1] = global_timer_ns();  // routed, hidden row loaded
+  int present = 0;
+  if (live)
+    for (int k = 0; k < a.K; ++k) present |= (s_id[k] >= 0 && s_id[k] < a.L) ? 1 : 0;
+  if (has_token && (present || !a.skip_payload)) {
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      const int c = tid + i * kLocalThreads;
+      if (c < chunks) {
+        reinterpret_cast<uint4*>(row)[c] = xv[i];
+        if (m.xq != nullptr && present) quant_chunk(xv[i], c, m.xq + (size_t)t * a.H, m.xs + (size_t)t * (a.H / 128));
+      }
+    }
+  }
+  int* meta = reinterpret_cast<int*>(row + (size_t)a.H * 2);
+  if (tid < a.K) {
+    const bool on = present && s_id[tid] >= 0 && s_id[tid] < a.L;
+    meta[tid] = on ? s_id[tid] : -1;
+    meta[a.K + tid] = on ? __float_as_int(s_w[tid]) : 0;
+  } else if (tid == a.K) {
+    meta[2 * a.K] = present;
+    a.hit[t] = (unsigned char)present;
+  }
+  __syncthreads();
+  if (trace) trace[2] = global_timer_ns();  // row stored
+  if (tid == 0) {
+    __threadfence();  // cumulative: the whole CTA's stores, ordered by the barrier
+    const unsigned done = atomicAdd(a.done_counter, 1u);
+    s_last = done == gridDim.x - 1;
+    if (s_last) {
+      *a.done_counter = 0u;
+      *a.epoch += 1u;
+    }
+  }
+  __syncthreads();
+  if (!s_last) return;
+  if (tid == 0) __threadfence();  // every other CTA's row comes before what follows
+  __syncthreads();
+  meta_one_pass<kLocalThreads>(m, s_dyn, (m.trace != nullptr && tid == 0) ? m.trace : nullptr);
+}
+
 }  // namespace mf
+
+extern "C" int mf_dispatch_local(const mf_dispatch_args* a, const mf_meta_args* m, mf_stream_t stream) {
+  using namespace mf;
+  if (!a || !m || a->C < 1 || a->T > a->C || a->K < 1 || a->K > kMaxTopK || a->R != 1 || m->R != 1 || a->H % 8 != 0 || a->H > 8192 ||
+      (a->pitch & 15) != 0 || a->pitch < (long long)a->H * 2 + (2 * a->K + 1) * 4 || m->pitch != a->pitch || m->rows != a->C ||
+      m->K != a->K || m->L != a->L || m->block_m < 1)
+    return -1;
+  if (m->L < 1 || m->L > kLocalThreads || (long long)a->C * a->K > kLocalThreads * kMetaBatch) return -2;
+  if (m->xq != nullptr && (!m->xs || a->H % 128 != 0)) return -3;
+  size_t smem = (size_t)meta_smem_words(m->L, kLocalThreads) * sizeof(int);
+  if (a->logits != nullptr) {
+    if (a->E < a->K || a->E != a->L || a->n_group < 1 || a->n_group > 32 || a->E % a->n_group != 0 || !a->route_w || !a->route_ids)
+      return -4;
+    smem += 2 * (size_t)a->E * sizeof(float);
+  }
+  if (smem > 48 * 1024) return -5;  // L = E <= 512: at most 41 KB
+  dispatch_local_kernel<<<a->C, kLocalThreads, smem, static_cast<cudaStream_t>(stream)>>>(*a, *m);
+  return (int)cudaGetLastError();
+}
 
 extern "C" int mf_dispatch_push(const mf_dispatch_args* a, mf_stream_t stream) {
   const int threads = (a && a->C >= 1024 && a->H / 8 <= 128 * 4 && a->R <= 32) ? 128 : 256;

@@ -17,6 +17,7 @@
 // sort/scatter_add/cumsum chain in moeflow/fixed.py:179-186 and build_tile_schedule
 // (moeflow/kernels/grouped_gemm.py:83-98).
 #include "common.cuh"
+#include "expert_meta.cuh"
 #include "moeflow_b200.h"
 #include "quant.cuh"
 
@@ -24,86 +25,6 @@ namespace mf {
 
 constexpr int kMetaThreads = 1024;
 constexpr int kMetaWarps = kMetaThreads / 32;
-constexpr int kMetaBatch = 8;  // warp-wide steps whose loads are issued together
-
-// Exclusive scan of one int per thread over the whole block; `total` gets the sum.
-__device__ __forceinline__ int block_exclusive_scan(int v, int* warp_sums, int& total) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  int incl = v;
-#pragma unroll
-  for (int off = 1; off < 32; off <<= 1) {
-    const int o = __shfl_up_sync(0xffffffffu, incl, off);
-    if (lane >= off) incl += o;
-  }
-  if (lane == 31) warp_sums[warp] = incl;
-  __syncthreads();
-  if (warp == 0) {
-    int w = lane < kMetaWarps ? warp_sums[lane] : 0;
-    int wi = w;
-#pragma unroll
-    for (int off = 1; off < 32; off <<= 1) {
-      const int o = __shfl_up_sync(0xffffffffu, wi, off);
-      if (lane >= off) wi += o;
-    }
-    warp_sums[lane] = wi - w;            // exclusive prefix of the warp sums
-    if (lane == 31) warp_sums[32] = wi;  // grand total
-  }
-  __syncthreads();
-  const int res = warp_sums[warp] + incl - v;
-  total = warp_sums[32];
-  __syncthreads();
-  return res;
-}
-
-// Row pitch of the per-warp histograms, in words: odd, so that the prefix over the warps (lane = source warp, one
-// expert at a time) reads 32 different banks.  With the pitch equal to L, 288 experts put all 32 lanes on one bank:
-// 9 rounds x 32 warps x 64 serialised accesses, about 10 us of the kernel.
-__host__ __device__ __forceinline__ int hist_pitch(int L) { return L | 1; }
-
-// Clears what the two GEMMs of this forward will count on: the finished quarters of the token tiles in use, and,
-// for a GEMM whose units are cut along K, the arrival counters of those units.  (The counters are zero again after
-// every complete forward; a forward that gave up part-way leaves some set, which is why they are cleared at all.)
-// Only the words in use: clearing the arrays whole was 100 KB to 400 KB of stores by one CTA at 288 experts.
-__device__ __forceinline__ void clear_counters(const mf_meta_args& a, int n_tiles, int cut1, int cut2) {
-  for (int i = threadIdx.x; i < min(n_tiles, a.n_tile_done); i += kMetaThreads) a.counters1[a.n_counters1 + i] = 0;
-  if (cut1 != 1)
-    for (int i = threadIdx.x; i < min(n_tiles * a.m_blocks1 * 8, a.n_counters1); i += kMetaThreads) a.counters1[i] = 0;
-  if (cut2 != 1)
-    for (int i = threadIdx.x; i < min(n_tiles * a.m_blocks2 * 8, a.n_counters2); i += kMetaThreads) a.counters2[i] = 0;
-}
-
-// Pick the K split S in {1,2,4,8}.  Cost model in units of one K block of streaming: a unit costs its
-// K blocks plus a fixed overhead (pipeline fill, epilogue, and for S > 1 the partial-sum round trip);
-// the kernel takes ceil(units * S / SMs) rounds of such units.  Ties go to the smaller S.
-__host__ __device__ __forceinline__ int choose_split(int units, int k_blocks, int n_sms, int max_slots,
-                                                     int overhead_kb, int cols) {
-  if (units <= 0) return 1;
-  int best = 1;
-  long long best_cost = (long long)((units + n_sms - 1) / n_sms) * (k_blocks + overhead_kb);
-  // the partial-sum round trip of a split unit grows with the tile's token columns (measured: splitting
-  // 64-column tiles in two cost more than the idle SMs of an uneven last round)
-  const int wide = cols > 16 ? (cols - 16) / 8 : 0;
-  for (int s = 2; s <= 8; s <<= 1) {
-    if (k_blocks % s != 0 || k_blocks / s < 2) break;
-    if ((long long)units * s > max_slots) break;
-    const long long rounds = ((long long)units * s + n_sms - 1) / n_sms;
-    const long long cost = rounds * (k_blocks / s + overhead_kb + 1 + wide);
-    if (cost < best_cost) {
-      best_cost = cost;
-      best = s;
-    }
-  }
-  return best;
-}
-
-// The K cut of one GEMM: stream-K (0) when asked for, the units do not fill many rounds of the persistent CTAs
-// (below 8 units per CTA an uneven last round costs more than the partial tiles of the cut units) and the
-// scratch holds the two partial tiles a CTA may need; else the K split of choose_split.
-__device__ __forceinline__ int choose_cut(const mf_meta_args& a, int units, int k_blocks, int slots, int overhead_kb,
-                                          int cols) {
-  if (a.stream_k && units > 0 && units < 8 * a.n_sms && units % a.n_sms != 0 && slots >= 2 * a.n_sms) return 0;
-  return choose_split(units, k_blocks, a.n_sms, slots, overhead_kb, cols);
-}
 
 __global__ void __launch_bounds__(kMetaThreads) expert_meta_kernel(const mf_meta_args a) {
   extern __shared__ int sm[];
@@ -190,9 +111,9 @@ __global__ void __launch_bounds__(kMetaThreads) expert_meta_kernel(const mf_meta
   // scans over experts (L <= 1024: one expert per thread): entry offsets and tile bases
   const int my_cnt = tid < L ? cnt[tid] : 0;
   int n_entries, n_tiles;
-  const int my_off = block_exclusive_scan(my_cnt, warp_sums, n_entries);
+  const int my_off = block_exclusive_scan<kMetaThreads>(my_cnt, warp_sums, n_entries);
   const int my_nt = (my_cnt + a.block_m - 1) / a.block_m;
-  const int my_tb = block_exclusive_scan(my_nt, warp_sums, n_tiles);
+  const int my_tb = block_exclusive_scan<kMetaThreads>(my_nt, warp_sums, n_tiles);
   if (tid < L) {
     offs[tid] = my_off;
     a.offsets[tid] = my_off;
@@ -249,7 +170,7 @@ __global__ void __launch_bounds__(kMetaThreads) expert_meta_kernel(const mf_meta
     a.plan[MF_PLAN_VALID_ROWS] = warp_sums[35];
   }
   __syncthreads();
-  clear_counters(a, min(n_tiles, a.max_tiles), warp_sums[36], warp_sums[37]);
+  clear_counters<kMetaThreads>(a, min(n_tiles, a.max_tiles), warp_sums[36], warp_sums[37]);
   if (trace) trace[4] = global_timer_ns();  // offsets, tiles and plan written
 
   // sweep 2: place the entries
@@ -283,15 +204,6 @@ __global__ void __launch_bounds__(kMetaThreads) expert_meta_kernel(const mf_meta
 }
 
 
-// ---------------------------------------------------------------------------------------------------
-// Decode sizes (rows * K <= kMetaThreads * kMetaBatch = 8192 slot words): the same layout in one pass.
-// Every thread keeps its (at most kMetaBatch) keys and weight bits in registers: the received rows are
-// read once, with all loads of a thread in flight together; the position of an entry inside its warp's
-// range is recorded while the warp histogram is built, so that after the scans the placement is pure
-// arithmetic and stores (no second sweep over the rows, no second round of matching).  The prefix over
-// the warps runs as warp scans (one expert per warp at a time) instead of one thread per expert.
-// Identical output to expert_meta_kernel; about a quarter of its latency.
-// ---------------------------------------------------------------------------------------------------
 // Received rows -> e4m3 (layers with block-scaled experts), by the CTAs behind the first one: the two jobs read the same
 // rows and neither needs the other, so the quantiser costs no launch and no time of its own.
 __device__ __forceinline__ void quantise_received_rows(const mf_meta_args& a) {
@@ -321,27 +233,16 @@ __global__ void __launch_bounds__(kMetaThreads) expert_meta_small_kernel(const m
     quantise_received_rows(a);
     return;
   }
-  const int L = a.L, K = a.K, P = hist_pitch(a.L);
-  int* hist = sm;                       // [kMetaWarps][P]
-  int* cnt = hist + kMetaWarps * P;     // [L]
-  int* offs = cnt + L;                  // [L]
-  int* warp_sums = offs + L;            // [40]
-
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   unsigned long long* trace = (a.trace != nullptr && tid == 0) ? a.trace : nullptr;
   if (trace) trace[0] = global_timer_ns();
   if (!a.late_launch) grid_dep_launch();
-  const int N = a.rows * K;
-  int per = (N + kMetaWarps - 1) / kMetaWarps;
-  per = (per + 31) & ~31;               // <= 32 * kMetaBatch by the launcher's choice of this kernel
-  const int n_warps = (N + per - 1) / per;  // warps that hold slot words (one at a single token)
-  for (int i = tid; i < n_warps * P; i += kMetaThreads) hist[i] = 0;
-  if (tid == 0) warp_sums[34] = warp_sums[35] = 0;
-  const int begin = min(N, warp * per), end = min(N, (warp + 1) * per);
-  const uint8_t* recv = static_cast<const uint8_t*>(a.recv);
-  const size_t meta_off = (size_t)a.H * 2;
-  int* my_hist = hist + warp * P;
+  meta_begin<kMetaThreads>(a, sm);
   {
+    const MetaSpan span(a, kMetaWarps);
+    const int K = a.K, begin = min(span.N, warp * span.per), end = min(span.N, (warp + 1) * span.per);
+    const uint8_t* recv = static_cast<const uint8_t*>(a.recv);
+    const size_t meta_off = (size_t)a.H * 2;
     // While the dispatch kernel runs: touch every page this kernel reads or writes after the wait.
     if (tid == 0) {
       touch(a.epoch);
@@ -373,163 +274,7 @@ __global__ void __launch_bounds__(kMetaThreads) expert_meta_small_kernel(const m
   __syncthreads();
   if (trace) trace[2] = global_timer_ns();  // flags seen
 
-  // the only reads of the received rows: id, valid flag and weight bits of every slot word of this thread
-  int key[kMetaBatch], wbits[kMetaBatch], pre[kMetaBatch];
-#pragma unroll
-  for (int b = 0; b < kMetaBatch; ++b) {
-    const int i = begin + b * 32 + lane;
-    key[b] = -1;
-    wbits[b] = 0;
-    if (i < end) {
-      const int row = i / K, slot = i - row * K;
-      const int* meta = reinterpret_cast<const int*>(recv + (size_t)row * a.pitch + meta_off);
-      const int id = __ldcg(meta + slot);
-      const int valid = __ldcg(meta + 2 * K);
-      const int wb = __ldcg(meta + K + slot);
-      if (valid != 0 && id >= 0 && id < L) {
-        key[b] = id;
-        wbits[b] = wb;
-      }
-    }
-  }
-  if (trace) trace[6] = global_timer_ns();  // loads issued
-
-  // warp histogram; pre[b] = entries of the same expert earlier in this warp's range
-  const unsigned lt_mask = (1u << lane) - 1u;
-  int rows_hit = 0;
-  const bool k_pow2 = (K & (K - 1)) == 0 && K <= 32;
-#pragma unroll
-  for (int b = 0; b < kMetaBatch; ++b) {
-    if (begin + b * 32 < end) {  // warp-uniform
-      const unsigned same = __match_any_sync(0xffffffffu, key[b]);
-      int before = 0;
-      if (key[b] >= 0) before = my_hist[key[b]];
-      pre[b] = before + __popc(same & lt_mask);
-      __syncwarp();
-      if (key[b] >= 0 && lane == __ffs(same) - 1) my_hist[key[b]] = before + __popc(same);
-      __syncwarp();
-      if (k_pow2) {
-        // a received row is K consecutive slot words of one warp step: its hit count is a ballot away
-        const unsigned live = __ballot_sync(0xffffffffu, key[b] >= 0);
-        const int g0 = lane & ~(K - 1);
-        const unsigned gmask = (K == 32 ? 0xffffffffu : ((1u << K) - 1u)) << g0;
-        const int hits = __popc(live & gmask);
-        const int i = begin + b * 32 + lane;
-        if (lane == g0 && i < end) {
-          if (a.row_hits != nullptr) a.row_hits[i / K] = hits;
-          rows_hit += hits > 0 ? 1 : 0;
-        }
-      }
-    }
-  }
-  if (k_pow2) {
-#pragma unroll
-    for (int off = 16; off > 0; off >>= 1) rows_hit += __shfl_xor_sync(0xffffffffu, rows_hit, off);
-    if (lane == 0 && rows_hit) atomicAdd(&warp_sums[35], rows_hit);
-  }
-  if (trace) trace[7] = global_timer_ns();  // this warp's histogram done (its loads have landed)
-  __syncthreads();
-  if (trace) trace[3] = global_timer_ns();  // histogram done
-
-  // per expert: exclusive prefix over the warps (lane = source warp), total count
-  for (int e = warp; e < L; e += kMetaWarps) {
-    const int c = lane < n_warps ? hist[lane * P + e] : 0;
-    int incl = c;
-#pragma unroll
-    for (int off = 1; off < 32; off <<= 1) {
-      const int o = __shfl_up_sync(0xffffffffu, incl, off);
-      if (lane >= off) incl += o;
-    }
-    if (lane < n_warps) hist[lane * P + e] = incl - c;
-    if (lane == 31) cnt[e] = incl;
-  }
-  if (!k_pow2) {
-    // general K: rows do not line up with warp steps; count their hits from the rows (cache hits by now)
-    int mine = 0;
-    for (int r = tid; r < a.rows; r += kMetaThreads) {
-      const int* meta = reinterpret_cast<const int*>(recv + (size_t)r * a.pitch + meta_off);
-      int hits = 0;
-      if (__ldcg(meta + 2 * K) != 0)
-        for (int k = 0; k < K; ++k) {
-          const int id = __ldcg(meta + k);
-          hits += (id >= 0 && id < L) ? 1 : 0;
-        }
-      if (a.row_hits != nullptr) a.row_hits[r] = hits;
-      mine += hits > 0 ? 1 : 0;
-    }
-    if (mine) atomicAdd(&warp_sums[35], mine);
-  }
-  __syncthreads();
-
-  // scans over experts (L <= 1024: one expert per thread): entry offsets and tile bases
-  const int my_cnt = tid < L ? cnt[tid] : 0;
-  int n_entries, n_tiles;
-  const int my_off = block_exclusive_scan(my_cnt, warp_sums, n_entries);
-  const int my_nt = (my_cnt + a.block_m - 1) / a.block_m;
-  const int my_tb = block_exclusive_scan(my_nt, warp_sums, n_tiles);
-  if (tid < L) {
-    offs[tid] = my_off;
-    a.offsets[tid] = my_off;
-    for (int j = 0; j < my_nt; ++j) {
-      const int idx = my_tb + j;
-      if (idx < a.max_tiles) {
-        a.tile_e[idx] = tid;
-        a.tile_s[idx] = my_off + j * a.block_m;
-        a.tile_n[idx] = min(a.block_m, my_cnt - j * a.block_m);
-      }
-    }
-    if (my_cnt > 0) atomicMax(&warp_sums[34], min(my_cnt, a.block_m));
-  }
-  __syncthreads();
-  if (tid == kMetaThreads - 1) {
-    // the plan words, by a thread of the last warp (its range of slot words is the shortest, often empty)
-    a.offsets[L] = n_entries;
-    const int nt = min(n_tiles, a.max_tiles);
-    int cols = (warp_sums[34] + 15) & ~15;
-    if (cols < 16) cols = 16;
-    const int wide_cols = cols;
-    int slots1 = a.max_split_slots, slots2 = a.max_split_slots;
-    if (a.partial_floats > 0) {
-      slots1 = (int)min((long long)0x7fffffff, a.partial_floats / (2ll * cols * 128));
-      slots2 = (int)min((long long)0x7fffffff, a.partial_floats / (1ll * cols * 128));
-    } else {
-      cols = 0;
-    }
-    a.plan[MF_PLAN_N_TILES] = nt;
-    warp_sums[36] = a.plan[MF_PLAN_SPLIT1] = choose_cut(a, nt * a.m_blocks1, a.k_blocks1, slots1, 4, wide_cols);
-    warp_sums[37] = a.plan[MF_PLAN_SPLIT2] = choose_cut(a, nt * a.m_blocks2, a.k_blocks2, slots2, 8, wide_cols);
-    a.plan[MF_PLAN_N_ENTRIES] = n_entries;
-    a.plan[MF_PLAN_NEXT1] = a.plan[MF_PLAN_NEXT2] = 0;
-    a.plan[MF_PLAN_SLOT_COLS] = cols;
-    a.plan[MF_PLAN_VALID_ROWS] = warp_sums[35];
-  }
-  if (trace) trace[4] = global_timer_ns();  // offsets and tiles written
-
-  // placement: arithmetic and stores only
-#pragma unroll
-  for (int b = 0; b < kMetaBatch; ++b) {
-    const int i = begin + b * 32 + lane;
-    if (i < end) {
-      int pos = -1;
-      if (key[b] >= 0) {
-        pos = offs[key[b]] + my_hist[key[b]] + pre[b];
-        // pos < N always holds for a consistent buffer; the guard keeps a racing writer (a peer that runs ahead
-        // in a truncated stage-timing run) from causing a stray store
-        if (pos < N) {
-          const int row = i / K;
-          a.entry_row[pos] = row;
-          a.entry_slot[pos] = i - row * K;
-          a.entry_w[pos] = __int_as_float(wbits[b]);
-        } else {
-          pos = -1;
-        }
-      }
-      a.inv[i] = pos;
-    }
-  }
-  __syncthreads();  // the cuts are in warp_sums
-  clear_counters(a, min(n_tiles, a.max_tiles), warp_sums[36], warp_sums[37]);
-  if (trace) trace[5] = global_timer_ns();  // entries placed
+  meta_one_pass<kMetaThreads>(a, sm, trace);
 }
 
 
@@ -676,9 +421,9 @@ __global__ void __launch_bounds__(kMetaThreads) expert_meta_place_kernel(const m
 
   const int my_cnt = tid < L ? cnt[tid] : 0;
   int n_entries, n_tiles;
-  const int my_off = block_exclusive_scan(my_cnt, warp_sums, n_entries);
+  const int my_off = block_exclusive_scan<kMetaThreads>(my_cnt, warp_sums, n_entries);
   const int my_nt = (my_cnt + a.block_m - 1) / a.block_m;
-  const int my_tb = block_exclusive_scan(my_nt, warp_sums, n_tiles);
+  const int my_tb = block_exclusive_scan<kMetaThreads>(my_nt, warp_sums, n_tiles);
   if (tid < L) {
     offs[tid] += my_off;
     if (cta == 0) {
@@ -719,7 +464,7 @@ __global__ void __launch_bounds__(kMetaThreads) expert_meta_place_kernel(const m
   }
   if (cta == 0) {
     __syncthreads();
-    clear_counters(a, min(n_tiles, a.max_tiles), warp_sums[36], warp_sums[37]);
+    clear_counters<kMetaThreads>(a, min(n_tiles, a.max_tiles), warp_sums[36], warp_sums[37]);
   }
 
   for (int i0 = range.begin; i0 < range.end; i0 += 32 * kMetaBatch) {
@@ -756,7 +501,7 @@ extern "C" int mf_plan_split(int units, int k_blocks, int n_sms, int max_slots, 
 
 extern "C" int mf_expert_meta(const mf_meta_args* a, mf_stream_t stream) {
   if (!a || a->L < 1 || a->L > mf::kMetaThreads || a->R > mf::kMetaThreads || a->block_m < 1) return -1;
-  const size_t smem = ((size_t)mf::kMetaWarps * mf::hist_pitch(a->L) + 2 * (size_t)a->L + 40) * sizeof(int);
+  const size_t smem = (size_t)mf::meta_smem_words(a->L, mf::kMetaThreads) * sizeof(int);
   static size_t configured_all[64] = {};  // per device: the attribute belongs to (function, device)
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) dev = 0;

@@ -29,15 +29,14 @@ int mf_capture_last_node(mf_stream_t stream, void** node_out) {
   return 0;
 }
 
-// Replaces the single by-value argument of a kernel node (same kernel, same launch shape) in an executable graph.
-// The graph that the node belongs to must still exist.
-int mf_graph_set_args(void* graph_exec, void* node, const void* args) {
+// Replaces the by-value arguments of a kernel node (one pointer per argument; same kernel, same launch shape) in an
+// executable graph.  The graph that the node belongs to must still exist.
+int mf_graph_set_args(void* graph_exec, void* node, void** args) {
   if (!graph_exec || !node || !args) return -1;
   cudaKernelNodeParams p = {};
   cudaError_t e = cudaGraphKernelNodeGetParams(static_cast<cudaGraphNode_t>(node), &p);
   if (e != cudaSuccess) return (int)e;
-  void* list[1] = {const_cast<void*>(args)};
-  p.kernelParams = list;
+  p.kernelParams = args;
   p.extra = nullptr;
   return (int)cudaGraphExecKernelNodeSetParams(static_cast<cudaGraphExec_t>(graph_exec), static_cast<cudaGraphNode_t>(node), &p);
 }

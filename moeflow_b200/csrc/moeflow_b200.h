@@ -258,6 +258,8 @@ typedef struct {
   float* xs;                 // [rows, H / 128]
 } mf_meta_args;
 int mf_expert_meta(const mf_meta_args* args, mf_stream_t stream);
+// Dispatch and metadata in one launch: the only rank is this GPU (R = 1), at most 512 experts and 4096 slot words.
+int mf_dispatch_local(const mf_dispatch_args* args, const mf_meta_args* meta, mf_stream_t stream);
 // The K-split rule of the metadata kernels, callable on the host (no device needed): the split in {1,2,4,8}
 // for `units` (token tile, 128-row block) work items of `k_blocks` K blocks on `n_sms` persistent CTAs, given
 // `max_slots` partial-sum slots, the fixed per-unit overhead in K-block units (4 for gate/up, 8 for down) and
@@ -278,6 +280,10 @@ typedef struct {
   int valid_word;            // index of the valid flag among a row's int32 metadata words (2 * top_k)
   unsigned* push_epoch;      // local count of return pushes; the last CTA adds one (the combine's expectation)
   unsigned long long* trace; // optional [8] globaltimer stamps of CTA 0 (profiling aid), or NULL
+  // Optional (R = 1): the layer's output [C, H] bf16.  With a single rank the merge over ranks is the identity, so the
+  // reduced row is stored there as well (zeros for rows without a hit) and no arrival is sent: no combine launch follows.
+  void* out;
+  int rows;                  // > 0: only these first rows of `out` are written
 } mf_reduce_push_args;
 int mf_owner_reduce_push(const mf_reduce_push_args* args, mf_stream_t stream);
 
@@ -319,10 +325,10 @@ int mf_gemm_gate_up_fp8(const void* tmap, const mf_gemm_args* args, int n_max, i
 int mf_gemm_down_fp8(const void* tmap, const mf_gemm_args* args, int n_max, int grid, mf_stream_t stream);
 
 // ---- captured forwards ------------------------------------------------------------------------------------
-// mf_capture_last_node: the kernel node that the capture on `stream` added last.  mf_graph_set_args: replaces the single
-// by-value argument struct of such a node in the executable graph made from that capture.
+// mf_capture_last_node: the kernel node that the capture on `stream` added last.  mf_graph_set_args: replaces the
+// by-value argument structs of such a node in the executable graph made from that capture.
 int mf_capture_last_node(mf_stream_t stream, void** node_out);
-int mf_graph_set_args(void* graph_exec, void* node, const void* args);
+int mf_graph_set_args(void* graph_exec, void* node, void** args);
 
 // ---- peer-memory runtime ------------------------------------------------------------------------------------
 int mf_peer_alloc(void** ptr, unsigned long long bytes);

@@ -14,9 +14,8 @@ __device__ __forceinline__ uint8_t to_e4m3(float x, float inv_scale) {
   return (uint8_t)__nv_cvt_float_to_fp8(x * inv_scale, __NV_SATFINITE, __NV_E4M3);
 }
 
-// 16-byte chunk c of one row (8 values).  16 consecutive threads hold a group: all of them must call this together.
-__device__ __forceinline__ void quant_chunk(const uint8_t* row, int c, uint8_t* q_row, float* scale_row) {
-  const uint4 v = __ldcg(reinterpret_cast<const uint4*>(row) + c);
+// Chunk c of one row (`v`: its 8 bf16 values).  16 consecutive threads hold a group: all of them must call this together.
+__device__ __forceinline__ void quant_chunk(const uint4& v, int c, uint8_t* q_row, float* scale_row) {
   const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&v);
   float f[8];
   float amax = 0.f;
@@ -38,6 +37,9 @@ __device__ __forceinline__ void quant_chunk(const uint8_t* row, int c, uint8_t* 
   for (int i = 0; i < 8; ++i) pb[i] = to_e4m3(f[i], inv);
   reinterpret_cast<uint2*>(q_row)[c] = packed;
   if ((c & 15) == 0) scale_row[c >> 4] = scale;
+}
+__device__ __forceinline__ void quant_chunk(const uint8_t* row, int c, uint8_t* q_row, float* scale_row) {
+  quant_chunk(__ldcg(reinterpret_cast<const uint4*>(row) + c), c, q_row, scale_row);
 }
 
 }  // namespace mf

@@ -70,6 +70,7 @@ __global__ void __launch_bounds__(kRowThreads) owner_reduce_push_kernel(const mf
     const uint4* y = static_cast<const uint4*>(a.y);
     uint4* dst = reinterpret_cast<uint4*>(reinterpret_cast<uint8_t*>(a.peer_ret[s]) +
                                           ((size_t)a.rank * a.C + t) * a.H * 2);
+    uint4* out = a.out != nullptr && (a.rows <= 0 || t < a.rows) ? static_cast<uint4*>(a.out) + (size_t)t * chunks : nullptr;
     for (int c = tid; c < chunks; c += kRowThreads) {
       float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
       // Issue the loads of up to 8 slots together (they are independent), then add in slot order.
@@ -86,8 +87,17 @@ __global__ void __launch_bounds__(kRowThreads) owner_reduce_push_kernel(const mf
           if (p >= 0) acc_bf16x8(acc, v[j]);
         }
       }
-      dst[c] = pack_bf16x8(acc);
+      const uint4 packed = pack_bf16x8(acc);
+      dst[c] = packed;
+      if (out != nullptr) out[c] = packed;
     }
+  } else if (a.out != nullptr && (a.rows <= 0 || t < a.rows)) {
+    uint4* out = static_cast<uint4*>(a.out) + (size_t)t * (a.H / 8);
+    for (int c = tid; c < a.H / 8; c += kRowThreads) out[c] = make_uint4(0u, 0u, 0u, 0u);
+  }
+  if (a.out != nullptr) {
+    if (trace) trace[2] = global_timer_ns();  // row stored
+    return;
   }
   // The barrier orders every thread's stores before thread 0's fence, which is cumulative: one system
   // fence per CTA instead of one per thread; then this row's arrival at its source rank.
@@ -187,6 +197,7 @@ extern "C" {
 
 int mf_owner_reduce_push(const mf_reduce_push_args* a, mf_stream_t stream) {
   if (!a || a->K > 32 || a->H % 8 != 0 || a->R < 1 || a->C < 1) return -1;
+  if (a->out != nullptr && a->R != 1) return -2;
   return (int)mf::launch_kernel(mf::owner_reduce_push_kernel, dim3(a->R * a->C), dim3(mf::kRowThreads), 0,
                                 static_cast<cudaStream_t>(stream), true, *a);
 }

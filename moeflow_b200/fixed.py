@@ -347,6 +347,9 @@ class FixedEPLayer:
         hit = self.stage_dispatch_pack(x, weights, ids, num_valid)
         if self.backend == "torch":
             self._exchange(self._recv_store, self._send_store)
+        if self.backend == "cuda" and self.fuse_combine and expert_fn is None and prepare_fn is None and combine_fn is None:
+            self._cuda_experts(to_output=True)
+            return self.out[:T]
         partials = self.stage_experts(expert_fn, prepare_fn=prepare_fn, direct_output=direct_expert_output)
         if self.backend == "torch":
             self._exchange(self.ret_recv, self.ret_send if partials is None else partials)
@@ -381,6 +384,9 @@ class FixedEPLayer:
         if stop_after in CUDA_SUBSTAGES:
             self._cuda_experts(stop_after)
             return self.plan
+        if self.backend == "cuda" and self.fuse_combine and stop_after in (None, "COMBINE"):
+            self._cuda_experts(to_output=True)
+            return self.out
         self.stage_experts()
         if stop_after == "EXPERT":
             return self.ret_recv if self.backend == "cuda" else self.ret_send
@@ -595,8 +601,16 @@ class FixedEPLayer:
             done_counter=self._done[2:].data_ptr(), R=R, C=Cc, H=H, K=1, rank=self.rank, valid_word=2 * K,
             push_epoch=self._push_epoch.data_ptr(),
         )
-        self._scratch_out = None
-        self._node_log: dict | None = None  # during a capture: graph nodes of the dispatch and combine kernels
+        # A single rank has no peer to wait for: at decode sizes the dispatch kernel's last CTA builds the metadata, and
+        # a whole forward ends with the owner reduce, which then writes the output (the merge over one rank is the
+        # identity).  An explicit meta_ctas keeps the two launches apart.
+        self.fuse_meta = R == 1 and self.meta_ctas == 1 and n_words <= 4096 and L <= 512 and H <= 8192 and "meta_ctas" not in self.gemm_kwargs
+        self.fuse_combine = R == 1 and not self.fuse_return
+        self._meta_done = False
+        self._a_reduce_out = S.ReducePushArgs.from_buffer_copy(self._a_reduce)
+        self._a_reduce_out.out = self.out.data_ptr()
+        # during a capture: graph nodes and arguments of the first and the last kernel of the forward
+        self._node_log: dict | None = None
         self._a_combine = S.CombineArgs(
             ret=self.ret_recv.data_ptr(), hit=self.hit.data_ptr(), out=self.out.data_ptr(),
             flags=self._ret_flags.data_ptr() if R > 1 else None, epoch=self._push_epoch.data_ptr(), R=R, C=Cc, H=H, rank=self.rank,
@@ -794,17 +808,25 @@ class FixedEPLayer:
         a.num_valid = None if num_valid is None else num_valid.data_ptr()
         a.T = x.shape[0]
         self._keep = [x, weights, ids, num_valid, logits, bias]
-        _lib.check(self._lib.mf_dispatch_push(C.byref(a), _lib.stream_ptr()), "dispatch_push")
+        if self.fuse_meta:
+            _lib.check(self._lib.mf_dispatch_local(C.byref(a), C.byref(self._a_meta), _lib.stream_ptr()), "dispatch")
+            self._meta_done = True
+        else:
+            _lib.check(self._lib.mf_dispatch_push(C.byref(a), _lib.stream_ptr()), "dispatch_push")
         if self._node_log is not None:
-            self._node_log["dispatch"] = _lib.last_captured_node()
+            self._node_log["first"] = (_lib.last_captured_node(), [a, self._a_meta] if self.fuse_meta else [a])
         return self.hit
 
     def _cuda_meta(self) -> None:
         from .ops import _lib
 
+        if self._meta_done:  # built by the dispatch launch
+            self._meta_done = False
+            return
         _lib.check(self._lib.mf_expert_meta(C.byref(self._a_meta), _lib.stream_ptr()), "expert_meta")
 
-    def _cuda_experts(self, stop_after: str | None = None) -> None:
+    def _cuda_experts(self, stop_after: str | None = None, to_output: bool = False) -> None:
+        """``to_output`` (one rank): the owner reduce writes the layer's output, no combine follows."""
         from .ops import _lib
 
         if self._tmap13 is None:
@@ -832,7 +854,7 @@ class FixedEPLayer:
             _lib.check(lib.mf_gemm_down_fp8(f["tm2"], C.byref(f["a2"]), self.block_m, self.n_sms, s), "fp8 down gemm")
             if stop_after == "GEMM2":
                 return
-            _lib.check(lib.mf_owner_reduce_push(C.byref(self._a_reduce), s), "owner_reduce_push")
+            self._cuda_reduce(to_output)
             return
         if self.permute_rows:
             _lib.check(self._lib.mf_permute_rows(self._recv_store.data_ptr(), self.pitch * 2, self.entry_row.data_ptr(),
@@ -844,7 +866,15 @@ class FixedEPLayer:
         _lib.check(self._lib.mf_gemm_down(self._tmap2, C.byref(self._a_gemm2), self.block_m, self.n_sms, s), "down gemm")
         if stop_after == "GEMM2" or self.fuse_return:
             return
-        _lib.check(self._lib.mf_owner_reduce_push(C.byref(self._a_reduce), s), "owner_reduce_push")
+        self._cuda_reduce(to_output)
+
+    def _cuda_reduce(self, to_output: bool) -> None:
+        from .ops import _lib
+
+        a = self._a_reduce_out if to_output else self._a_reduce
+        _lib.check(self._lib.mf_owner_reduce_push(C.byref(a), _lib.stream_ptr()), "owner_reduce_push")
+        if to_output and self._node_log is not None:
+            self._node_log["last"] = (_lib.last_captured_node(), [a])
 
     def _cuda_push_partials(self, partials: torch.Tensor) -> None:
         """Return path for externally computed partial rows ``[RC, H]``: peer stores + return flags."""
@@ -866,7 +896,7 @@ class FixedEPLayer:
 
         _lib.check(self._lib.mf_combine(C.byref(self._a_combine), _lib.stream_ptr()), "combine")
         if self._node_log is not None:
-            self._node_log["combine"] = _lib.last_captured_node()
+            self._node_log["last"] = (_lib.last_captured_node(), [self._a_combine])
         return self.out
 
     def check_status(self) -> dict:

@@ -64,9 +64,20 @@ class GraphedMoELayer:
         self._bound = None               # what they point at: (x, logits, rows, out), or None for the static buffers
         self._host_refs: deque = deque(maxlen=8)  # pinned outputs that recent replays may still be writing
         self._warmup = warmup
-        # route+dispatch, meta (two launches in its multi-CTA form), gate/up, down(+reduce+push), combine
-        self.kernels_per_step = (5 if getattr(layer, "fuse_return", False) else 6) + (
-            1 if getattr(layer, "meta_ctas", 1) > 1 else 0) + (1 if getattr(layer, "permute_rows", False) else 0)
+
+    @property
+    def kernels_per_step(self) -> int:
+        ly = self.layer
+        fp8 = getattr(ly, "_fp8", None)
+        front = 1 if getattr(ly, "fuse_meta", False) else 3 if getattr(ly, "meta_ctas", 1) > 1 else 2  # dispatch, metadata
+        if fp8 is not None and not fp8["in_meta"]:
+            front += 1  # quantiser of the received rows
+        if getattr(ly, "_expand", None) is not None:
+            front += 2
+        if getattr(ly, "permute_rows", False) and fp8 is None:
+            front += 1
+        tail = 1 if getattr(ly, "fuse_return", False) or getattr(ly, "fuse_combine", False) else 2
+        return front + 2 + tail
 
     def _views(self, block: torch.Tensor):
         cfg, C = self.layer.cfg, self.layer.C
@@ -108,11 +119,10 @@ class GraphedMoELayer:
             from ..ops import _lib
 
             graph.instantiate()
-            a, c = _lib.DispatchArgs(), _lib.CombineArgs()
-            C.memmove(C.byref(a), C.byref(self.layer._a_dispatch), C.sizeof(a))
-            C.memmove(C.byref(c), C.byref(self.layer._a_combine), C.sizeof(c))
-            self._dispatch_args, self._combine_args, self._set_args = a, c, _lib.lib().mf_graph_set_args
-            self._exec, self._raw = graph.raw_cuda_graph_exec(), graph.raw_cuda_graph()
+            for name, (node, args) in nodes.items():
+                own = [type(a).from_buffer_copy(a) for a in args]
+                nodes[name] = (node, own[0], (C.c_void_p * len(own))(*(C.addressof(a) for a in own)), own)
+            self._set_args, self._exec = _lib.lib().mf_graph_set_args, graph.raw_cuda_graph_exec()
         self.graph, self._nodes, self._bound = graph, nodes, None
         torch.cuda.synchronize()
         return self
@@ -124,7 +134,8 @@ class GraphedMoELayer:
             return
         from ..ops import _lib
 
-        a, c = self._dispatch_args, self._combine_args
+        first, a, first_list, _ = self._nodes["first"]
+        last, c, last_list, _ = self._nodes["last"]
         layer = self.layer
         if key is None:
             a.x, a.logits, a.T, a.num_valid = self.x.data_ptr(), self.logits.data_ptr(), layer.C, self.num_valid.data_ptr()
@@ -133,10 +144,10 @@ class GraphedMoELayer:
             a.x, a.logits, a.T, out = key
             a.num_valid, rows = None, key[2]
         was = None if self._bound is None else self._bound[3]
-        _lib.check(self._set_args(self._exec, self._nodes["dispatch"], C.addressof(a)), "graph update")
+        _lib.check(self._set_args(self._exec, first, first_list), "graph update")
         if out != was or out is not None:
             c.out, c.rows = (layer.out.data_ptr(), 0) if out is None else (out, rows)
-            _lib.check(self._set_args(self._exec, self._nodes["combine"], C.addressof(c)), "graph update")
+            _lib.check(self._set_args(self._exec, last, last_list), "graph update")
         self._bound = key
 
     def _readable(self, x: torch.Tensor, logits: torch.Tensor) -> bool:

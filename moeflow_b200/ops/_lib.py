@@ -209,6 +209,8 @@ class ReducePushArgs(C.Structure):
         ("valid_word", C.c_int),
         ("push_epoch", C.c_void_p),
         ("trace", C.c_void_p),
+        ("out", C.c_void_p),
+        ("rows", C.c_int),
     ]
 
 
@@ -269,6 +271,7 @@ def lib() -> C.CDLL:
         "mf_router_topk": [P, P, P, P, I, I, I, I, I, I, I, F, P],
         "mf_rmsnorm": [P, P, P, I, I, F, P],
         "mf_dispatch_push": [C.POINTER(DispatchArgs), P],
+        "mf_dispatch_local": [C.POINTER(DispatchArgs), C.POINTER(MetaArgs), P],
         "mf_expert_meta": [C.POINTER(MetaArgs), P],
         "mf_plan_split": [I, I, I, I, I, I],
         "mf_permute_rows": [P, LL, P, P, P, I, I, I, P],
@@ -276,7 +279,7 @@ def lib() -> C.CDLL:
         "mf_combine": [C.POINTER(CombineArgs), P],
         "mf_expert_prepare": [P, LL, I, I, I, I, I, P, P, P, P, P],
         "mf_capture_last_node": [P, C.POINTER(P)],
-        "mf_graph_set_args": [P, P, P],
+        "mf_graph_set_args": [P, P, C.POINTER(P)],
         "mf_peer_alloc": [C.POINTER(P), ULL],
         "mf_peer_free": [P],
         "mf_peer_export": [P, P],
