@@ -231,6 +231,7 @@ grouped_gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid
     F8Pipe st;
     bool ok = true;
     SegFeed feed(work, ring, abort_flag, wait_ns);
+    const uint64_t policy = N_MAX <= 64 ? l2_evict_first() : l2_evict_normal();  // as in grouped_gemm_tc.cu
     Seg sg;
     bool have = feed.first(sg);
     while (ok && have) {
@@ -245,8 +246,8 @@ grouped_gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid
         if (lane == 0) {
           mbar_arrive_expect_tx(&full_bar[st.stage], Cfg::kStageA);
           uint8_t* dst = sA + st.stage * Cfg::kStageA;
-          tma_load_2d(dst, &tmap_w, &full_bar[st.stage], kb * 128, row0);
-          if (kGateUp) tma_load_2d(dst + kF8TileA, &tmap_w, &full_bar[st.stage], kb * 128, row0 + a.up_row_offset);
+          tma_load_2d(dst, &tmap_w, &full_bar[st.stage], kb * 128, row0, policy);
+          if (kGateUp) tma_load_2d(dst + kF8TileA, &tmap_w, &full_bar[st.stage], kb * 128, row0 + a.up_row_offset, policy);
         }
         __syncwarp();
         st.advance(STAGES);

@@ -392,6 +392,8 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
     PipeState st;
     bool ok = true;
     SegFeed feed(work, ring, abort_flag, wait_ns);
+    // Tiles of up to 64 rows are decode: an expert has one tile and its weights are read once per forward.
+    const uint64_t policy = N_MAX <= 64 ? l2_evict_first() : l2_evict_normal();
     Seg sg;
     bool have = feed.first(sg);
     while (ok && have) {
@@ -408,8 +410,8 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
           mbar_arrive_expect_tx(&full_bar[st.stage], Cfg::kStageA);
           uint8_t* dst = sA + st.stage * Cfg::kStageA;
           if (trace && trace[2] == 0) trace[2] = global_timer_ns();  // see the note at MF_STAMP_ONCE
-          tma_load_2d(dst, &tmap_w, &full_bar[st.stage], kb * 64, row0);
-          if (kGateUp) tma_load_2d(dst + kTileBytesA, &tmap_w, &full_bar[st.stage], kb * 64, row0 + a.up_row_offset);
+          tma_load_2d(dst, &tmap_w, &full_bar[st.stage], kb * 64, row0, policy);
+          if (kGateUp) tma_load_2d(dst + kTileBytesA, &tmap_w, &full_bar[st.stage], kb * 64, row0 + a.up_row_offset, policy);
         }
         __syncwarp();
         st.advance(STAGES);

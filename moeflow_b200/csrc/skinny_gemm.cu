@@ -96,14 +96,15 @@ skinny_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
 
   if (warp == 0) {
     if (lane == 0) {
+      const uint64_t policy = l2_evict_first();
       auto load_w = [&](int stage, int kb) {
         mbar_arrive_expect_tx(&full_bar[stage], kSkTileA);
         uint8_t* dst = smem + stage * kSkStage;
         if (kGateUp) {  // two boxes of 64 rows: one accumulator holds gate and up of the same 64 outputs
-          tma_load_2d(dst, &tmap_w, &full_bar[stage], kb * 64, unit * 64);
-          tma_load_2d(dst + kSkTileA / 2, &tmap_w, &full_bar[stage], kb * 64, unit * 64 + a.up_row_offset);
+          tma_load_2d(dst, &tmap_w, &full_bar[stage], kb * 64, unit * 64, policy);
+          tma_load_2d(dst + kSkTileA / 2, &tmap_w, &full_bar[stage], kb * 64, unit * 64 + a.up_row_offset, policy);
         } else {
-          tma_load_2d(dst, &tmap_w, &full_bar[stage], kb * 64, unit * kSkM);
+          tma_load_2d(dst, &tmap_w, &full_bar[stage], kb * 64, unit * kSkM, policy);
         }
       };
       auto load_x = [&](int stage, int kb) {
