@@ -132,6 +132,8 @@ typedef struct {
   float limit;               // SwiGLU clamp (<= 0: none)
   const void* residual;      // optional bf16 [T, residual_pitch]: added to the rounded product, rounded again
   long long residual_pitch;  // elements
+  const void* residual2;     // optional, with residual: added to it first, that sum rounded to bf16
+  long long residual2_pitch;
   unsigned long long* status;
   unsigned long long wait_ns;
 } mf_skinny_args;
@@ -180,6 +182,14 @@ int mf_gemm_down_static_scratch(const void* tmap, const mf_gemm_args* args, int 
 int mf_router_topk(const float* logits, const float* bias, float* weights, int* ids, int tokens, int experts,
                    int top_k, int n_group, int topk_group, int sigmoid, int renorm, float scale,
                    mf_stream_t stream);
+// sum = x + add (rounded to bf16), out = rmsnorm(sum).
+int mf_add_rmsnorm(const void* x, const void* add, const void* gamma, void* sum, void* out, int rows, int hidden, float eps,
+                   mf_stream_t stream);
+// Row *pos of the caches [B, kv_heads, S, head_dim] (bf16) from the keys and values of this step, each [B, kv_heads *
+// head_dim] with rows pitch elements apart; a position outside the cache stores nothing.  head_dim and pitch: multiples of
+// 8; all pointers 16-byte aligned.
+int mf_kv_append(const void* k, const void* v, long long pitch, void* k_cache, void* v_cache, const long long* pos, int B,
+                 int kv_heads, int S, int head_dim, mf_stream_t stream);
 int mf_rmsnorm(const void* x, const void* gamma, void* out, int rows, int hidden, float eps, mf_stream_t stream);
 
 // ---- dispatch (pack + peer stores + flags) ----------------------------------------------------------

@@ -31,20 +31,39 @@ router_topk_kernel(const float* __restrict__ logits, const float* __restrict__ b
   }
 }
 
-// out[r, :] = x[r, :] * rsqrt(mean(x[r, :]^2) + eps) * gamma, bf16 in/out, fp32 math.
+// out[r, :] = v * rsqrt(mean(v^2) + eps) * gamma with v = x[r, :], or (kAdd) v = sum[r, :] = bf16(x + add); fp32 math.
+// One row is 8 KB: a few microseconds of launch, first loads and one block reduction.  Launched with programmatic
+// serialization, so the launch and the block's start run under the predecessor; the addition of the attention output is
+// one launch (2.5 us in a decode layer) less as part of this kernel.
+template <bool kAdd>
 __global__ void __launch_bounds__(256)
-rmsnorm_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ gamma,
-               __nv_bfloat16* __restrict__ out, int hidden, float eps) {
+rmsnorm_kernel(const __nv_bfloat16* x, const __nv_bfloat16* add, const __nv_bfloat16* gamma, __nv_bfloat16* sum,
+               __nv_bfloat16* out, int hidden, float eps) {
   __shared__ float red[8];
-  const int r = blockIdx.x;
-  const uint4* xr = reinterpret_cast<const uint4*>(x + (size_t)r * hidden);
+  // Resident while its predecessor still runs: no read-only loads, and none ahead of the wait.
+  grid_dep_launch();
+  grid_dep_wait_cta();
+  const size_t row = (size_t)blockIdx.x * hidden;
+  const uint4* xr = reinterpret_cast<const uint4*>(x + row);
+  const uint4* ar = reinterpret_cast<const uint4*>(kAdd ? add + row : nullptr);
   const uint4* gr = reinterpret_cast<const uint4*>(gamma);
-  uint4* orow = reinterpret_cast<uint4*>(out + (size_t)r * hidden);
+  uint4* srow = reinterpret_cast<uint4*>(kAdd ? sum + row : nullptr);
+  uint4* orow = reinterpret_cast<uint4*>(out + row);
   const int chunks = hidden / 8;
   float ss = 0.f;
   for (int c = threadIdx.x; c < chunks; c += blockDim.x) {
-    const uint4 v = xr[c];
-    const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&v);
+    uint4 v = __ldcg(xr + c);
+    __nv_bfloat162* h = reinterpret_cast<__nv_bfloat162*>(&v);
+    if (kAdd) {
+      const uint4 w = __ldcg(ar + c);
+      const __nv_bfloat162* d = reinterpret_cast<const __nv_bfloat162*>(&w);
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const float2 f = __bfloat1622float2(h[i]), e = __bfloat1622float2(d[i]);
+        h[i] = __floats2bfloat162_rn(f.x + e.x, f.y + e.y);
+      }
+      srow[c] = v;
+    }
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
       const float2 f = __bfloat1622float2(h[i]);
@@ -58,8 +77,8 @@ rmsnorm_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restr
   for (int i = 0; i < (int)(blockDim.x >> 5); ++i) tot += red[i];
   const float inv = rsqrtf(tot / (float)hidden + eps);
   for (int c = threadIdx.x; c < chunks; c += blockDim.x) {
-    const uint4 v = xr[c];
-    const uint4 g = gr[c];
+    const uint4 v = kAdd ? srow[c] : __ldcg(xr + c);  // the sum: this thread's own store
+    const uint4 g = __ldcg(gr + c);
     const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&v);
     const __nv_bfloat162* gh = reinterpret_cast<const __nv_bfloat162*>(&g);
     uint4 o;
@@ -73,6 +92,23 @@ rmsnorm_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restr
     }
     orow[c] = o;
   }
+}
+
+// This step's keys and values into their caches, 16 bytes per thread.  Two generic scatters with an expanded index took
+// 4.4-5.9 us each in a decode layer (4 to 64 sequences), nearly all of it launch and indexing.
+__global__ void __launch_bounds__(256)
+kv_append_kernel(const uint4* k, const uint4* v, long long pitch, uint4* k_cache, uint4* v_cache, const long long* pos, int n,
+                 int kv_heads, int S, int chunks) {
+  grid_dep_launch();
+  grid_dep_wait_cta();
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;  // (sequence, kv head, chunk)
+  const long long at = __ldcg(pos);
+  if (i >= n || at < 0 || at >= S) return;
+  const int c = i % chunks, pair = i / chunks;
+  const int b = pair / kv_heads, h = pair - b * kv_heads;
+  const long long from = b * pitch + (long long)h * chunks + c, to = ((long long)pair * S + at) * chunks + c;
+  k_cache[to] = __ldcg(k + from);
+  v_cache[to] = __ldcg(v + from);
 }
 
 }  // namespace mf
@@ -96,10 +132,35 @@ int mf_router_topk(const float* logits, const float* bias, float* weights, int* 
 int mf_rmsnorm(const void* x, const void* gamma, void* out, int rows, int hidden, float eps, mf_stream_t stream) {
   if (rows == 0) return 0;
   if (hidden % 8 != 0) return -1;
-  mf::rmsnorm_kernel<<<rows, 256, 0, static_cast<cudaStream_t>(stream)>>>(
-      static_cast<const __nv_bfloat16*>(x), static_cast<const __nv_bfloat16*>(gamma),
-      static_cast<__nv_bfloat16*>(out), hidden, eps);
-  return (int)cudaGetLastError();
+  return (int)mf::launch_kernel(mf::rmsnorm_kernel<false>, dim3(rows), dim3(256), 0, static_cast<cudaStream_t>(stream), true,
+                                static_cast<const __nv_bfloat16*>(x), static_cast<const __nv_bfloat16*>(nullptr),
+                                static_cast<const __nv_bfloat16*>(gamma), static_cast<__nv_bfloat16*>(nullptr),
+                                static_cast<__nv_bfloat16*>(out), hidden, eps);
+}
+
+int mf_add_rmsnorm(const void* x, const void* add, const void* gamma, void* sum, void* out, int rows, int hidden, float eps,
+                   mf_stream_t stream) {
+  if (rows == 0) return 0;
+  if (hidden % 8 != 0 || !add || !sum) return -1;
+  return (int)mf::launch_kernel(mf::rmsnorm_kernel<true>, dim3(rows), dim3(256), 0, static_cast<cudaStream_t>(stream), true,
+                                static_cast<const __nv_bfloat16*>(x), static_cast<const __nv_bfloat16*>(add),
+                                static_cast<const __nv_bfloat16*>(gamma), static_cast<__nv_bfloat16*>(sum),
+                                static_cast<__nv_bfloat16*>(out), hidden, eps);
+}
+
+int mf_kv_append(const void* k, const void* v, long long pitch, void* k_cache, void* v_cache, const long long* pos, int B,
+                 int kv_heads, int S, int head_dim, mf_stream_t stream) {
+  if (B < 0 || kv_heads < 1 || S < 1 || head_dim < 8 || head_dim % 8 != 0 || pitch % 8 != 0 ||
+      (long long)B * kv_heads * (head_dim / 8) > 0x7fffffffLL)
+    return -1;
+  const uintptr_t all = reinterpret_cast<uintptr_t>(k) | reinterpret_cast<uintptr_t>(v) | reinterpret_cast<uintptr_t>(k_cache) |
+                        reinterpret_cast<uintptr_t>(v_cache);
+  if ((all & 15) != 0 || !k || !v || !k_cache || !v_cache || !pos) return -2;
+  const int chunks = head_dim / 8, n = B * kv_heads * chunks;
+  if (n == 0) return 0;
+  return (int)mf::launch_kernel(mf::kv_append_kernel, dim3((n + 255) / 256), dim3(256), 0, static_cast<cudaStream_t>(stream), true,
+                                static_cast<const uint4*>(k), static_cast<const uint4*>(v), pitch / 8, static_cast<uint4*>(k_cache),
+                                static_cast<uint4*>(v_cache), pos, n, kv_heads, S, chunks);
 }
 
 }  // extern "C"

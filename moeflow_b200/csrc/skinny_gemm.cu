@@ -52,6 +52,10 @@ __device__ __forceinline__ float ld_cluster_f32(uint32_t addr) {
   return v;
 }
 
+__device__ __forceinline__ float ldcg_bf16(const void* base, long long i) {
+  return __bfloat162float(__ushort_as_bfloat16(__ldcg(static_cast<const unsigned short*>(base) + i)));
+}
+
 template <bool kGateUp>
 __global__ void __launch_bounds__(kSkThreads)
 skinny_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_x,
@@ -202,9 +206,11 @@ skinny_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
         static_cast<float*>(a.out)[at] = o[h];
       } else {
         float v = bf16_round(o[h]);
-        if (a.residual != nullptr)
-          v += __bfloat162float(__ushort_as_bfloat16(__ldcg(static_cast<const unsigned short*>(a.residual) +
-                                                            (long long)(t0 + c) * a.residual_pitch + col)));
+        if (a.residual != nullptr) {
+          float add = ldcg_bf16(a.residual, (long long)(t0 + c) * a.residual_pitch + col);
+          if (a.residual2 != nullptr) add = bf16_round(add + ldcg_bf16(a.residual2, (long long)(t0 + c) * a.residual2_pitch + col));
+          v += add;
+        }
         static_cast<__nv_bfloat16*>(a.out)[at] = __float2bfloat16_rn(v);
       }
     }

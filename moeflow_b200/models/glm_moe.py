@@ -68,11 +68,15 @@ class SharedExpert:
         self._down = DenseProjection(self.w2, status=self.status)
 
     def __call__(self, x: torch.Tensor) -> torch.Tensor:
-        t = x.shape[0]
         if not self.cuda:
             h = swiglu_clamp(x @ self.w13.transpose(0, 1), self.limit)
             return h @ self.w2.transpose(0, 1)
         return self._down(self._gate_up(x, self.act), self.out)
+
+    def add_to(self, x: torch.Tensor, first: torch.Tensor, second: torch.Tensor, out: torch.Tensor) -> torch.Tensor:
+        """``out = (first + second) + self(x)``, rounded to bf16 after every addition; the down projection adds (two
+        element-wise launches less per layer).  cuda path only."""
+        return self._down(self._gate_up(x, self.act), out, first, second)
 
 
 class RouterLogits:
@@ -106,17 +110,28 @@ class MoEBlock:
         self.cfg, self.routed, self.gate_w, self.bias, self.norm_w, self.shared, self.eps = cfg, routed, gate_w, bias, norm_w, shared, eps
         self.router = router
 
-    def __call__(self, x: torch.Tensor, num_valid: torch.Tensor | None = None) -> torch.Tensor:
-        h = _rmsnorm(x, self.norm_w, self.eps)
+    def __call__(self, x: torch.Tensor, num_valid: torch.Tensor | None = None, add: torch.Tensor | None = None,
+                 out: torch.Tensor | None = None) -> torch.Tensor:
+        """``add``: summand of ``x`` that is still missing (the attention output).  ``out`` (contiguous bf16 ``[T, H]``,
+        not ``x``) receives the result."""
+        if add is not None and x.is_cuda and x.dtype == torch.bfloat16:
+            from ..ops.kernels import add_rmsnorm
+
+            x, h = add_rmsnorm(x, add, self.norm_w, self.eps)
+        else:
+            x = x if add is None else x + add
+            h = _rmsnorm(x, self.norm_w, self.eps)
         if self.router is not None:
             logits = self.router(h)
         else:
             logits = torch.matmul(h.to(self.gate_w.dtype), self.gate_w.transpose(0, 1)).to(torch.float32)
         routed = self.routed.forward(h, logits, self.bias, num_valid)[: x.shape[0]]
-        out = x + routed
+        if self.shared is not None and self.shared.cuda and x.dtype == routed.dtype == torch.bfloat16:
+            return self.shared.add_to(h, x, routed, torch.empty_like(h) if out is None else out)
+        y = x + routed
         if self.shared is not None:
-            out = out + self.shared(h)
-        return out
+            y = y + self.shared(h)
+        return y if out is None else out.copy_(y)
 
 
 class Attention:
@@ -143,6 +158,10 @@ class Attention:
 
     def __call__(self, x: torch.Tensor, pos: torch.Tensor, mask: torch.Tensor) -> torch.Tensor:
         """``x [B, H]``; ``pos`` device int64 scalar (position being written); ``mask [1,1,1,max_seq]`` additive."""
+        return x + self.delta(x, pos, mask)
+
+    def delta(self, x: torch.Tensor, pos: torch.Tensor, mask: torch.Tensor) -> torch.Tensor:
+        """What the attention adds to ``x``."""
         a = self.acfg
         h = _rmsnorm(x, self.norm_w, 1e-6)
         qkv = h @ self.wqkv.transpose(0, 1)
@@ -150,11 +169,16 @@ class Attention:
         q = qkv[:, :q_out].view(self.batch, a.n_heads, 1, a.head_dim)
         k = qkv[:, q_out : q_out + kv_out].view(self.batch, a.n_kv_heads, 1, a.head_dim)
         v = qkv[:, q_out + kv_out :].view(self.batch, a.n_kv_heads, 1, a.head_dim)
-        idx = pos.view(1, 1, 1, 1).expand(self.batch, a.n_kv_heads, 1, a.head_dim)
-        self.k_cache.scatter_(2, idx, k)
-        self.v_cache.scatter_(2, idx, v)
+        if qkv.is_cuda and qkv.dtype == torch.bfloat16 and a.head_dim % 8 == 0:
+            from ..ops.kernels import kv_append
+
+            kv_append(qkv[:, q_out : q_out + kv_out], qkv[:, q_out + kv_out :], self.k_cache, self.v_cache, pos)
+        else:
+            idx = pos.view(1, 1, 1, 1).expand(self.batch, a.n_kv_heads, 1, a.head_dim)
+            self.k_cache.scatter_(2, idx, k)
+            self.v_cache.scatter_(2, idx, v)
         o = F.scaled_dot_product_attention(q, self.k_cache, self.v_cache, attn_mask=mask, enable_gqa=True)
-        return x + o.reshape(self.batch, q_out) @ self.wo.transpose(0, 1)
+        return o.reshape(self.batch, q_out) @ self.wo.transpose(0, 1)
 
 
 class DecodeModel:
@@ -239,17 +263,21 @@ class DecodeModel:
 
     def _forward(self) -> None:
         x = self.x
-        for layer in self.layers:
-            if layer["attn"] is not None:
-                x = layer["attn"](x, self.pos, self.mask)
+        for i, layer in enumerate(self.layers):
+            delta = layer["attn"].delta(x, self.pos, self.mask) if layer["attn"] is not None else None
             if layer["fp8"] is not None:
                 self.routed.bind_weights_fp8(layer["fp8"])
             else:
                 self.routed.bind_weights(layer["w13"], layer["w2"], *layer["maps"])
             block = MoEBlock(self.cfg, self.routed, layer["gate_w"], layer["bias"], layer["norm_w"], layer["shared"],
                              router=layer["router"])
-            x = block(x)
-        self.out.copy_(x)
+            x = block(x, add=delta, out=self.out if i == len(self.layers) - 1 else None)
+        if not self.layers:
+            self.out.copy_(x)
+
+    def _advance(self) -> None:
+        self.pos.add_(1)
+        self.mask.view(-1).index_fill_(0, self.pos.view(1), 0.0)
 
     def capture(self) -> "DecodeModel":
         import torch.distributed as dist
@@ -265,6 +293,7 @@ class DecodeModel:
         self.graph = torch.cuda.CUDAGraph()
         with torch.cuda.graph(self.graph):
             self._forward()
+            self._advance()
         torch.cuda.synchronize()
         return self
 
@@ -272,10 +301,9 @@ class DecodeModel:
         """One decode step for the whole batch; advances the position (mask and KV write index)."""
         if self.graph is None:
             self._forward()
+            self._advance()
         else:
             self.graph.replay()
-        self.pos.add_(1)
-        self.mask.view(-1).index_fill_(0, self.pos.view(1), 0.0)
         return self.out
 
     def close(self) -> None:

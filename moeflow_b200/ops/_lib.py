@@ -103,6 +103,8 @@ class SkinnyArgs(C.Structure):
         ("limit", C.c_float),
         ("residual", C.c_void_p),
         ("residual_pitch", C.c_longlong),
+        ("residual2", C.c_void_p),
+        ("residual2_pitch", C.c_longlong),
         ("status", C.c_void_p),
         ("wait_ns", C.c_ulonglong),
     ]
@@ -270,6 +272,8 @@ def lib() -> C.CDLL:
         "mf_dequant_block_fp8": [P, P, P, LL, I, P],
         "mf_router_topk": [P, P, P, P, I, I, I, I, I, I, I, F, P],
         "mf_rmsnorm": [P, P, P, I, I, F, P],
+        "mf_add_rmsnorm": [P, P, P, P, P, I, I, F, P],
+        "mf_kv_append": [P, P, LL, P, P, P, I, I, I, I, P],
         "mf_dispatch_push": [C.POINTER(DispatchArgs), P],
         "mf_dispatch_local": [C.POINTER(DispatchArgs), C.POINTER(MetaArgs), P],
         "mf_expert_meta": [C.POINTER(MetaArgs), P],

@@ -35,9 +35,10 @@ class DenseProjection:
                                      out_cols=out_cols, limit=float(limit) if limit is not None else 0.0,
                                      status=self.status.data_ptr(), wait_ns=wait_ns)
 
-    def __call__(self, x: torch.Tensor, out: torch.Tensor, residual: torch.Tensor | None = None) -> torch.Tensor:
-        """Writes ``out[: T]`` for ``x [T, K]`` (bf16 rows, any 16-byte pitch).  ``residual`` (bf16 ``[T, rows]``) is
-        added to the bf16 product."""
+    def __call__(self, x: torch.Tensor, out: torch.Tensor, residual: torch.Tensor | None = None,
+                 residual2: torch.Tensor | None = None) -> torch.Tensor:
+        """Writes ``out[: T]`` for ``x [T, K]`` (bf16 rows, any 16-byte pitch).  ``residual`` (bf16 ``[T, rows]``), or
+        the bf16 sum ``residual + residual2``, is added to the bf16 product."""
         t = x.shape[0]
         if x.shape[1] != self.k or out.shape[0] < t:
             raise ValueError("token rows do not fit this projection")
@@ -47,6 +48,7 @@ class DenseProjection:
         a.x, a.x_pitch, a.T = x.data_ptr(), x.stride(0) * 2, t
         a.out, a.out_pitch, a.out_fp32 = out.data_ptr(), out.stride(0), int(out.dtype == torch.float32)
         a.residual, a.residual_pitch = (residual.data_ptr(), residual.stride(0)) if residual is not None else (None, 0)
+        a.residual2, a.residual2_pitch = (residual2.data_ptr(), residual2.stride(0)) if residual2 is not None else (None, 0)
         _lib.check(self._lib.mf_skinny_gemm(self._tmap, C.byref(a), int(self.gate_up), self.n_sms, _lib.stream_ptr()),
                    "dense projection")
         return out[:t]

@@ -76,6 +76,43 @@ def rmsnorm(x: torch.Tensor, gamma: torch.Tensor, eps: float = 1e-6, out: torch.
     return out
 
 
+def add_rmsnorm(x: torch.Tensor, add: torch.Tensor, gamma: torch.Tensor, eps: float = 1e-6) -> tuple[torch.Tensor, torch.Tensor]:
+    """``(x + add, rmsnorm(x + add))`` in one launch; the sum is rounded to bf16 before it is normalised."""
+    for name, t in (("x", x), ("add", add), ("gamma", gamma)):
+        _need_cuda(t, name)
+        if t.dtype != torch.bfloat16:
+            raise ValueError("add_rmsnorm takes bf16 tensors")
+    hidden = x.shape[-1]
+    if add.shape != x.shape or gamma.numel() != hidden:
+        raise ValueError("x, add and gamma do not fit each other")
+    total, out = torch.empty_like(x), torch.empty_like(x)
+    _lib.check(
+        _lib.lib().mf_add_rmsnorm(x.data_ptr(), add.data_ptr(), gamma.data_ptr(), total.data_ptr(), out.data_ptr(),
+                                  x.numel() // hidden, hidden, float(eps), _lib.stream_ptr()),
+        "add_rmsnorm",
+    )
+    return total, out
+
+
+def kv_append(k: torch.Tensor, v: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor, pos: torch.Tensor) -> None:
+    """Stores ``k`` / ``v`` (``[B, kv * d]``, equal row strides) as row ``pos`` (device int64 scalar) of the contiguous
+    bf16 caches ``[B, kv, S, d]``."""
+    B, kv, S, d = k_cache.shape
+    for t in (k, v, k_cache, v_cache):
+        if t.dtype != torch.bfloat16 or not t.is_cuda:
+            raise ValueError("bf16 CUDA tensors expected")
+    if (tuple(k.shape) != (B, kv * d) or v.shape != k.shape or v_cache.shape != k_cache.shape or k.stride(1) != 1 or v.stride() != k.stride()
+            or not k_cache.is_contiguous() or not v_cache.is_contiguous()):
+        raise ValueError("keys, values and caches do not fit each other")
+    if pos.dtype != torch.int64 or pos.numel() != 1 or not pos.is_cuda:
+        raise ValueError("pos must be a device int64 scalar")
+    _lib.check(
+        _lib.lib().mf_kv_append(k.data_ptr(), v.data_ptr(), k.stride(0), k_cache.data_ptr(), v_cache.data_ptr(), pos.data_ptr(),
+                                B, kv, S, d, _lib.stream_ptr()),
+        "kv append",
+    )
+
+
 def make_tile_tmap(x: torch.Tensor, box_rows: int) -> C.Array:
     """128-byte TMA descriptor over a contiguous ``x [rows, K]`` with boxes of ``box_rows`` rows x 128 bytes.
 

@@ -20,6 +20,7 @@ MIRRORS = {
     "mf_meta_args": _lib.MetaArgs,
     "mf_reduce_push_args": _lib.ReducePushArgs,
     "mf_combine_args": _lib.CombineArgs,
+    "mf_skinny_args": _lib.SkinnyArgs,
 }
 
 

@@ -1,0 +1,47 @@
+"""The small kernels of a decode layer, bitwise against the torch operations they stand for."""
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("rows,hidden", [(1, 8), (3, 512), (64, 4096), (5, 4104)])
+def test_add_rmsnorm(rows, hidden):
+    from moeflow_b200.ops.kernels import add_rmsnorm, rmsnorm
+
+    g = torch.Generator().manual_seed(rows)
+    x, add = (torch.randn(rows, hidden, generator=g).bfloat16().cuda() for _ in range(2))
+    gamma = torch.randn(hidden, generator=g).bfloat16().cuda()
+    total, normed = add_rmsnorm(x, add, gamma, 1e-6)
+    assert torch.equal(total, x + add)
+    assert torch.equal(normed, rmsnorm(x + add, gamma, 1e-6))
+
+
+@pytest.mark.parametrize("B,kv,S,d", [(1, 1, 1, 8), (4, 4, 37, 128), (65, 2, 9, 64)])
+def test_kv_append(B, kv, S, d):
+    from moeflow_b200.ops.kernels import kv_append
+
+    g = torch.Generator().manual_seed(B)
+    qkv = torch.randn(B, 3 * kv * d, generator=g).bfloat16().cuda()
+    k, v = qkv[:, kv * d : 2 * kv * d], qkv[:, 2 * kv * d :]
+    kc, vc = (torch.randn(B, kv, S, d, generator=g).bfloat16().cuda() for _ in range(2))
+    for pos in {0, S // 2, S - 1, S, -1}:
+        kw, vw = kc.clone(), vc.clone()
+        if 0 <= pos < S:
+            kw[:, :, pos], vw[:, :, pos] = k.view(B, kv, d), v.view(B, kv, d)
+        kv_append(k, v, kc, vc, torch.tensor(pos, device="cuda"))
+        assert torch.equal(kc, kw) and torch.equal(vc, vw)
+
+
+@pytest.mark.parametrize("tokens", [1, 64, 65])
+def test_two_residuals(tokens):
+    from moeflow_b200.ops.dense import DenseProjection
+
+    g = torch.Generator().manual_seed(tokens)
+    x = torch.randn(tokens, 192, generator=g).bfloat16().cuda()
+    w = torch.randn(256, 192, generator=g).bfloat16().cuda()
+    a, b = (torch.randn(tokens, 256, generator=g).bfloat16().cuda() for _ in range(2))
+    project = DenseProjection(w)
+    plain = project(x, torch.empty(tokens, 256, dtype=torch.bfloat16, device="cuda"))
+    assert torch.equal(project(x, torch.empty_like(a), a, b), (a + b) + plain)
