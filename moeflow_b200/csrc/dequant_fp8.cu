@@ -17,34 +17,54 @@
 
 namespace mf {
 
-__global__ void __launch_bounds__(256) dequant_block_fp8_kernel(const uint8_t* w8, const float* scale, __nv_bfloat16* out,
-                                                                long long rows, int K) {
+// A CTA expands 16 rows of one 128-row block, 8 values (8 bytes in, 16 out) per thread and step: whole sectors both ways,
+// eight loads in flight, and addresses that only grow (the rows are contiguous), so that the pass is bound by memory.
+// With 16 values per step and a 64-bit division for the row in each it was bound by its instructions: 36 experts of
+// 3 x 4096 x 1536 (0.68 GB in, 1.36 GB out) took 430 us, 4.7 TB/s.
+constexpr int kDqThreads = 256;
+constexpr int kDqRows = 16;
+constexpr int kDqBatch = 8;
+
+__device__ __forceinline__ uint4 expand_8(uint2 q, float s) {
+  const uint32_t words[2] = {q.x, q.y};
+  uint32_t o[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const __nv_fp8x2_storage_t pair = (__nv_fp8x2_storage_t)((words[i >> 1] >> (16 * (i & 1))) & 0xffffu);
+    const __half2_raw hr = __nv_cvt_fp8x2_to_halfraw2(pair, __NV_E4M3);
+    const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&hr));
+    const __nv_bfloat162 b = __floats2bfloat162_rn(f.x * s, f.y * s);
+    o[i] = *reinterpret_cast<const uint32_t*>(&b);
+  }
+  return make_uint4(o[0], o[1], o[2], o[3]);
+}
+
+__global__ void __launch_bounds__(kDqThreads) dequant_block_fp8_kernel(const uint8_t* w8, const float* scale, __nv_bfloat16* out, int K) {
   grid_dep_wait_cta();
   grid_dep_launch();
-  const int chunks_per_row = K / 16;  // 16 e4m3 values per thread and step
-  const int k_blocks = K / 128;
-  const long long total = rows * chunks_per_row;
-  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
-    const long long r = i / chunks_per_row;
-    const int c = (int)(i - r * chunks_per_row);
-    const uint4 q = __ldcs(reinterpret_cast<const uint4*>(w8 + r * K) + c);  // streamed once
-    const float s = __ldg(scale + (r >> 7) * k_blocks + (c >> 3));
-    const uint32_t words[4] = {q.x, q.y, q.z, q.w};
-    uint32_t o[8];
+  const int cpr = K / 8;                                  // steps of 8 values per row
+  const int n = kDqRows * cpr;
+  const size_t at = (size_t)blockIdx.x * n;               // rows are contiguous
+  const uint2* src = reinterpret_cast<const uint2*>(w8) + at;
+  uint4* dst = reinterpret_cast<uint4*>(out) + at;
+  const float* sc = scale + (size_t)(blockIdx.x / (128 / kDqRows)) * (K / 128);
+  const int wrap = kDqThreads % cpr;
+  int c = threadIdx.x % cpr;
+  for (int i = threadIdx.x; i < n; i += kDqThreads * kDqBatch) {
+    uint2 q[kDqBatch];
+    float s[kDqBatch];
 #pragma unroll
-    for (int w = 0; w < 4; ++w) {
-#pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        const __nv_fp8x2_storage_t pair = (__nv_fp8x2_storage_t)((words[w] >> (16 * h)) & 0xffffu);
-        const __half2_raw hr = __nv_cvt_fp8x2_to_halfraw2(pair, __NV_E4M3);
-        const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&hr));
-        const __nv_bfloat162 b = __floats2bfloat162_rn(f.x * s, f.y * s);
-        o[2 * w + h] = *reinterpret_cast<const uint32_t*>(&b);
+    for (int j = 0; j < kDqBatch; ++j) {
+      if (i + j * kDqThreads < n) {
+        q[j] = __ldcs(src + i + j * kDqThreads);  // streamed once
+        s[j] = __ldg(sc + (c >> 4));
       }
+      c += wrap;
+      if (c >= cpr) c -= cpr;
     }
-    uint4* dst = reinterpret_cast<uint4*>(out + r * K + (long long)c * 16);
-    dst[0] = make_uint4(o[0], o[1], o[2], o[3]);
-    dst[1] = make_uint4(o[4], o[5], o[6], o[7]);
+#pragma unroll
+    for (int j = 0; j < kDqBatch; ++j)
+      if (i + j * kDqThreads < n) dst[i + j * kDqThreads] = expand_8(q[j], s[j]);
   }
 }
 
@@ -57,10 +77,8 @@ extern "C" int mf_dequant_block_fp8(const void* w8, const float* scale, void* ou
   if (w8 == nullptr || scale == nullptr || out_bf16 == nullptr) return -1;
   if (rows <= 0 || K <= 0 || rows % 128 != 0 || K % 128 != 0) return -2;
   if ((reinterpret_cast<uintptr_t>(w8) | reinterpret_cast<uintptr_t>(out_bf16)) & 15) return -3;
-  const long long total = rows * (K / 16);
-  long long blocks = (total + 255) / 256;
-  if (blocks > 148 * 16) blocks = 148 * 16;
-  return (int)mf::launch_kernel(mf::dequant_block_fp8_kernel, dim3((unsigned)blocks), dim3(256), 0,
+  if (rows / mf::kDqRows > 0x7fffffffLL) return -2;
+  return (int)mf::launch_kernel(mf::dequant_block_fp8_kernel, dim3((unsigned)(rows / mf::kDqRows)), dim3(mf::kDqThreads), 0,
                                 static_cast<cudaStream_t>(stream), true, static_cast<const uint8_t*>(w8), scale,
-                                static_cast<__nv_bfloat16*>(out_bf16), rows, K);
+                                static_cast<__nv_bfloat16*>(out_bf16), K);
 }
