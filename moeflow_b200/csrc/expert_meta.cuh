@@ -39,9 +39,8 @@ __device__ __forceinline__ int block_exclusive_scan(int v, int* warp_sums, int& 
   return res;
 }
 
-// Row pitch of the per-warp histograms, in words: odd, so that the prefix over the warps (lane = source warp, one
-// expert at a time) reads 32 different banks.  With the pitch equal to L, 288 experts put all 32 lanes on one bank:
-// 9 rounds x 32 warps x 64 serialised accesses, about 10 us of the kernel.
+// Row pitch of the per-warp histograms, in words: odd, so that one expert's counts in the rows of different warps lie on
+// different banks.
 __host__ __device__ __forceinline__ int hist_pitch(int L) { return L | 1; }
 
 // Clears what the two GEMMs of this forward will count on: the finished quarters of the token tiles in use, and,
@@ -90,13 +89,33 @@ __device__ __forceinline__ int choose_cut(const mf_meta_args& a, int units, int 
   return choose_split(units, k_blocks, a.n_sms, slots, overhead_kb, cols);
 }
 
+// The same choice by the four lanes of a group (lane & 3 = log2 of the split it weighs; the whole warp calls): the splits
+// are weighed side by side and in 32-bit divisions, where one thread went through them one after the other, in the tail
+// of the pass that the GEMMs wait for.  units * 8 fits 32 bits (at most 8192 tiles).
+__device__ __forceinline__ int choose_cut_lanes(const mf_meta_args& a, int units, int k_blocks, int slots, int overhead_kb,
+                                                int cols, int log_s) {
+  const int s = 1 << log_s;
+  const int wide = cols > 16 ? (cols - 16) / 8 : 0;
+  const int rounds = (int)((unsigned)(units * s + a.n_sms - 1) / (unsigned)a.n_sms);
+  const bool can = s == 1 || ((k_blocks & (s - 1)) == 0 && (k_blocks >> log_s) >= 2 && (long long)units * s <= slots);
+  const long long cost = (long long)rounds * ((k_blocks >> log_s) + overhead_kb + (s == 1 ? 0 : 1 + wide));
+  long long key = can ? cost * 4 + log_s : 0x7fffffffffffffffll;  // ties go to the smaller split
+#pragma unroll
+  for (int off = 1; off < 4; off <<= 1) {
+    const long long o = __shfl_xor_sync(0xffffffffu, key, off);
+    key = o < key ? o : key;
+  }
+  if (units <= 0) return 1;
+  if (a.stream_k && units < 8 * a.n_sms && units % a.n_sms != 0 && slots >= 2 * a.n_sms) return 0;
+  return 1 << (int)(key & 3);
+}
+
 // ---------------------------------------------------------------------------------------------------
 // Decode sizes (rows * K <= kMetaThreads * kMetaBatch = 8192 slot words): the same layout in one pass.
 // Every thread keeps its (at most kMetaBatch) keys and weight bits in registers: the received rows are
 // read once, with all loads of a thread in flight together; the position of an entry inside its warp's
 // range is recorded while the warp histogram is built, so that after the scans the placement is pure
-// arithmetic and stores (no second sweep over the rows, no second round of matching).  The prefix over
-// the warps runs as warp scans (one expert per warp at a time) instead of one thread per expert.
+// arithmetic and stores (no second sweep over the rows, no second round of matching).
 // Identical output to expert_meta_kernel; about a quarter of its latency.
 // ---------------------------------------------------------------------------------------------------
 // Shared memory: meta_smem_words(L, kThreads) ints at `sm`.  meta_begin clears the histogram (any time before the pass, with a
@@ -194,17 +213,22 @@ __device__ __forceinline__ void meta_one_pass(const mf_meta_args& a, int* sm, un
   __syncthreads();
   if (trace) trace[3] = global_timer_ns();  // histogram done
 
-  // per expert: exclusive prefix over the warps (lane = source warp), total count
-  for (int e = warp; e < L; e += kWarps) {
-    const int c = lane < n_warps ? hist[lane * P + e] : 0;
-    int incl = c;
+  // Per expert (one thread each): exclusive prefix over the warps and total count.  The counts of 16 warps are loaded
+  // together; a warp scan per expert instead was 18 dependent rounds per warp at 288 experts.
+  for (int e = tid; e < L; e += kThreads) {
+    int run = 0;
+#pragma unroll 1
+    for (int w0 = 0; w0 < n_warps; w0 += 16) {
+      int c[16];
 #pragma unroll
-    for (int off = 1; off < 32; off <<= 1) {
-      const int o = __shfl_up_sync(0xffffffffu, incl, off);
-      if (lane >= off) incl += o;
+      for (int w = 0; w < 16; ++w) c[w] = w0 + w < n_warps ? hist[(w0 + w) * P + e] : 0;
+#pragma unroll
+      for (int w = 0; w < 16; ++w) {
+        if (w0 + w < n_warps) hist[(w0 + w) * P + e] = run;
+        run += c[w];
+      }
     }
-    if (lane < n_warps) hist[lane * P + e] = incl - c;
-    if (lane == 31) cnt[e] = incl;
+    cnt[e] = run;
   }
   if (!k_pow2) {
     // general K: rows do not line up with warp steps; count their hits from the rows (cache hits by now)
@@ -224,12 +248,14 @@ __device__ __forceinline__ void meta_one_pass(const mf_meta_args& a, int* sm, un
   }
   __syncthreads();
 
-  // scans over experts (L <= 1024: one expert per thread): entry offsets and tile bases
+  // scan over experts (L <= kThreads: one expert per thread): entry offsets and tile bases.  Both sums stay below 8193
+  // (kThreads * kMetaBatch slot words), so one scan carries them in the halves of a word.
   const int my_cnt = tid < L ? cnt[tid] : 0;
-  int n_entries, n_tiles;
-  const int my_off = block_exclusive_scan<kThreads>(my_cnt, warp_sums, n_entries);
   const int my_nt = (my_cnt + a.block_m - 1) / a.block_m;
-  const int my_tb = block_exclusive_scan<kThreads>(my_nt, warp_sums, n_tiles);
+  int total;
+  const int base = block_exclusive_scan<kThreads>(my_cnt | (my_nt << 16), warp_sums, total);
+  const int n_entries = total & 0xffff, n_tiles = total >> 16;
+  const int my_off = base & 0xffff, my_tb = base >> 16;
   if (tid < L) {
     offs[tid] = my_off;
     a.offsets[tid] = my_off;
@@ -244,27 +270,29 @@ __device__ __forceinline__ void meta_one_pass(const mf_meta_args& a, int* sm, un
     if (my_cnt > 0) atomicMax(&warp_sums[34], min(my_cnt, a.block_m));
   }
   __syncthreads();
-  if (tid == kThreads - 1) {
-    // the plan words, by a thread of the last warp (its range of slot words is the shortest, often empty)
-    a.offsets[L] = n_entries;
+  if (warp == kWarps - 1) {
+    // the plan words, by the last warp (its range of slot words is the shortest, often empty): lanes 0-3 weigh the
+    // splits 1, 2, 4, 8 of the gate/up GEMM, lanes 4-7 those of the down GEMM
     const int nt = min(n_tiles, a.max_tiles);
     int cols = (warp_sums[34] + 15) & ~15;
     if (cols < 16) cols = 16;
-    const int wide_cols = cols;
-    int slots1 = a.max_split_slots, slots2 = a.max_split_slots;
-    if (a.partial_floats > 0) {
-      slots1 = (int)min((long long)0x7fffffff, a.partial_floats / (2ll * cols * 128));
-      slots2 = (int)min((long long)0x7fffffff, a.partial_floats / (1ll * cols * 128));
-    } else {
-      cols = 0;
+    const bool second = (lane & 4) != 0;
+    int slots = a.max_split_slots;
+    if (a.partial_floats > 0)  // partial tiles of 256 * cols floats (gate and up), 128 * cols for the down GEMM
+      slots = (int)((unsigned)min((long long)0x7fffffff, a.partial_floats >> (second ? 7 : 8)) / (unsigned)cols);
+    const int cut = choose_cut_lanes(a, nt * (second ? a.m_blocks2 : a.m_blocks1), second ? a.k_blocks2 : a.k_blocks1, slots,
+                                     second ? 8 : 4, cols, lane & 3);
+    if (lane == 0) {
+      warp_sums[36] = a.plan[MF_PLAN_SPLIT1] = cut;
+      a.offsets[L] = n_entries;
+      a.plan[MF_PLAN_N_TILES] = nt;
+      a.plan[MF_PLAN_N_ENTRIES] = n_entries;
+      a.plan[MF_PLAN_NEXT1] = a.plan[MF_PLAN_NEXT2] = 0;
+      a.plan[MF_PLAN_SLOT_COLS] = a.partial_floats > 0 ? cols : 0;
+      a.plan[MF_PLAN_VALID_ROWS] = warp_sums[35];
+    } else if (lane == 4) {
+      warp_sums[37] = a.plan[MF_PLAN_SPLIT2] = cut;
     }
-    a.plan[MF_PLAN_N_TILES] = nt;
-    warp_sums[36] = a.plan[MF_PLAN_SPLIT1] = choose_cut(a, nt * a.m_blocks1, a.k_blocks1, slots1, 4, wide_cols);
-    warp_sums[37] = a.plan[MF_PLAN_SPLIT2] = choose_cut(a, nt * a.m_blocks2, a.k_blocks2, slots2, 8, wide_cols);
-    a.plan[MF_PLAN_N_ENTRIES] = n_entries;
-    a.plan[MF_PLAN_NEXT1] = a.plan[MF_PLAN_NEXT2] = 0;
-    a.plan[MF_PLAN_SLOT_COLS] = cols;
-    a.plan[MF_PLAN_VALID_ROWS] = warp_sums[35];
   }
   if (trace) trace[4] = global_timer_ns();  // offsets and tiles written
 

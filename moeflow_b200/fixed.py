@@ -506,7 +506,14 @@ class FixedEPLayer:
         n_words = R * Cc * K
         # up to 8192 slot words one CTA keeps them all in registers (one pass); above that the two chained
         # multi-CTA launches take 11-18 us where a sweeping single CTA would take 134 us at 32768 words
-        self.meta_ctas = int(self.gemm_kwargs.get("meta_ctas", choose_meta_ctas(n_words, self.n_sms)))
+        # Without peers (no flags to wait for) the two launches win earlier, from where the pass no longer runs inside the
+        # dispatch launch: whole layer on B200, one CTA / 32: 1000 tokens on 72 experts bf16 585 / 570 us, e4m3 605 / 593;
+        # 600 tokens 513 / 505, e4m3 435 / 427; 1000 tokens on 36 experts 407 / 392 (64 and 128 CTAs: within 4 us of 32).
+        # (Rows of less than 4 MB in all gained as much, 109 -> 97 us at hidden 1024; such layers keep the one-pass kernel,
+        # whose checks on one rank run at that size.)
+        spread = R * Cc * self.pitch * 2 >= 4 << 20
+        meta_ctas = n_words // 256 if R == 1 and 4096 < n_words <= 8192 and spread else choose_meta_ctas(n_words, self.n_sms)
+        self.meta_ctas = int(self.gemm_kwargs.get("meta_ctas", meta_ctas))
         if not 1 <= self.meta_ctas <= 1024:
             raise ValueError("meta_ctas must be between 1 and 1024")
         if self.meta_ctas > 1:
