@@ -46,7 +46,7 @@ constexpr int kTileBytesA = 128 * 128;  // 128 rows x 128 bytes
 constexpr int kThreads = 256;
 constexpr int kThreadsWithReturn = 384;  // + 4 return warps (fused owner reduce + return push)
 // Epilogue warp groups.  Tiles of 256 token columns fill all 512 tensor-memory columns with one accumulator stage
-// (two accumulators of 256 columns), so their epilogue is not hidden behind the next unit's main loop: two groups of
+// (two accumulators of 256 columns) when they hold more than 128 rows, so their epilogue is not hidden behind the next unit's main loop: two groups of
 // four warps then take half of the token columns each.  The variant with return warps keeps one group.
 template <int N_MAX, bool kReturn>
 constexpr int kEpiGroups = (N_MAX >= 256 && !kReturn) ? 2 : 1;
@@ -66,10 +66,14 @@ struct GemmCfg {
   // barriers): the bytes in flight per SM, not the tensor pipe, bound these weight-streaming kernels.
   static constexpr int kStages = (216 * 1024) / kStageBytes > 10 ? 10 : (216 * 1024) / kStageBytes;
   static constexpr int kAccCols = kATiles * N_MAX;
-  // Two accumulator stages (the epilogue of unit i overlaps the main loop of unit i + 1) wherever the 512
-  // tensor-memory columns allow it; the gate/up GEMM with 256-row token tiles needs all 512 for one stage.
-  static constexpr int kAccStages = 2 * kAccCols <= 512 ? 2 : 1;
-  static constexpr int kTmemCols = kAccStages * kAccCols;  // power of two for N_MAX in {32, 64, 128, 256}
+  // Two accumulator stages: the epilogue of unit i overlaps the main loop of unit i + 1.  With two accumulators of 256
+  // columns a wide unit (more than 128 token columns) needs all 512 tensor-memory columns and takes both stages; a narrow
+  // one takes one, its accumulators 128 columns apart.  Tiles are narrow more often than not where 256-row tiles begin (80
+  // expected rows per expert).
+  static constexpr int kAccStages = 2;
+  static constexpr bool kWide = kAccStages * kAccCols > 512;
+  static constexpr int kStageCols = kWide ? 256 : kAccCols;
+  static constexpr int kTmemCols = kAccStages * kStageCols;  // power of two for N_MAX in {32, 64, 128, 256}
   static constexpr int kSmemBytes = kStages * kStageBytes + 1024 /*alignment slack*/ + 1024 /*barriers, return queue*/ +
                                     (N_MAX >= 256 ? 8 : 4) * kOutStageBytes /*one transposing store buffer per epilogue warp*/;
 };
@@ -433,14 +437,19 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
     while (ok && reader.next(sg, ok)) {
       const uint32_t n_tile = (uint32_t)((sg.n_rows + 15) & ~15);
       const uint32_t idesc = umma_idesc(1, 1, kBlockM, n_tile < 16 ? 16 : n_tile);
+      const bool wide = Cfg::kWide && n_tile > 128;
+      PipeState acc2 = acc;  // a wide unit's second stage
+      acc2.advance(Cfg::kAccStages);
       ok = mbar_wait_bounded(&acc_empty[acc.stage], acc.phase ^ 1u, abort_flag, wait_ns);
+      if (wide && ok) ok = mbar_wait_bounded(&acc_empty[acc2.stage], acc2.phase ^ 1u, abort_flag, wait_ns);
       ok = __all_sync(0xffffffffu, ok);
       if (!ok) {
         if (lane == 0) report_status(a.status, kGemmAccTimeout, 1, blockIdx.x, 0);
         break;
       }
       tc_fence_after_sync();
-      const uint32_t d0 = tmem_base + acc.stage * Cfg::kAccCols;
+      const uint32_t d0 = tmem_base + (wide ? 0 : acc.stage * Cfg::kStageCols);
+      const uint32_t d1 = d0 + (Cfg::kWide && !wide ? 128 : N_MAX);
       for (int j = 0; j < sg.nkb; ++j) {
         ok = mbar_wait_bounded(&full_bar[st.stage], st.phase, abort_flag, wait_ns);
         ok = __all_sync(0xffffffffu, ok);
@@ -459,7 +468,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
             const uint64_t bdesc = umma_desc_sw128(b_addr + k * 32);
             const uint32_t accum = (j > 0 || k > 0) ? 1u : 0u;
             umma_f16(d0, umma_desc_sw128(a_addr + k * 32), bdesc, idesc, accum);
-            if (kGateUp) umma_f16(d0 + N_MAX, umma_desc_sw128(a_addr + kTileBytesA + k * 32), bdesc, idesc, accum);
+            if (kGateUp) umma_f16(d1, umma_desc_sw128(a_addr + kTileBytesA + k * 32), bdesc, idesc, accum);
           }
           umma_commit(&empty_bar[st.stage]);
         }
@@ -467,9 +476,13 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
         st.advance(STAGES);
       }
       if (!ok) break;
-      if (lane == 0) umma_commit(&acc_full[acc.stage]);
+      if (lane == 0) {
+        umma_commit(&acc_full[acc.stage]);
+        if (wide) umma_commit(&acc_full[acc2.stage]);
+      }
       __syncwarp();
       acc.advance(Cfg::kAccStages);
+      if (wide) acc.advance(Cfg::kAccStages);
     }
   } else if (warp < 4 && b_tma) {
     // ------------------------------------------------------------------ token-operand producer (TMA)
@@ -478,6 +491,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
       bool ok = true;
       Seg sg;
       int ready_tile = -1;
+      const int box_rows = a.b_box_rows > 0 ? a.b_box_rows : N_MAX;
       while (ok && reader.next(sg, ok)) {
         if (a.tile_wait != nullptr && sg.tt != ready_tile) {
           // the tile's activations are final once every gate/up unit of the tile has reported its four quarters
@@ -496,6 +510,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
           }
           ready_tile = sg.tt;
         }
+        const int n_box = max(1, (sg.n_rows + box_rows - 1) / box_rows);
         for (int j = 0; j < sg.nkb; ++j) {
           const int kb = sg.kb0 + j;
           ok = mbar_wait_bounded(&empty_bar[st.stage], st.phase ^ 1u, abort_flag, wait_ns);
@@ -505,11 +520,13 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
             break;
           }
           if (lane == 0) {
-            // the box is N_MAX rows whatever the tile's row count: rows past the tile (the next expert's
-            // entries, or zero fill past the end of the buffer) land in smem rows the MMA does not read
-            // or in accumulator columns the epilogue skips
-            mbar_arrive_expect_tx(&full_bar[st.stage], Cfg::kStageB);
-            tma_load_2d(sB + st.stage * Cfg::kStageB, &tmap_b, &full_bar[st.stage], kb * 64, sg.row_start);
+            // as many boxes as hold the tile's rows: rows past the tile (the next expert's entries, or zero fill
+            // past the end of the buffer) land in smem rows the MMA does not read or in accumulator columns the
+            // epilogue skips
+            mbar_arrive_expect_tx(&full_bar[st.stage], n_box * box_rows * 128);
+            for (int i = 0; i < n_box; ++i)
+              tma_load_2d(sB + st.stage * Cfg::kStageB + i * box_rows * 128, &tmap_b, &full_bar[st.stage], kb * 64,
+                          sg.row_start + i * box_rows);
           }
           __syncwarp();
           st.advance(STAGES);
@@ -628,7 +645,11 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
       const int row_start = sg.row_start;
       int n_tile = (n_rows + 15) & ~15;
       if (n_tile < 16) n_tile = 16;
+      const bool wide = Cfg::kWide && n_tile > 128;
+      PipeState acc2 = acc;
+      acc2.advance(Cfg::kAccStages);
       ok = mbar_wait_bounded(&acc_full[acc.stage], acc.phase, abort_flag, wait_ns);
+      if (wide && ok) ok = mbar_wait_bounded(&acc_full[acc2.stage], acc2.phase, abort_flag, wait_ns);
       ok = __all_sync(0xffffffffu, ok);
       if (warp == 4 && lane == 0) MF_STAMP_ONCE(4);
       if (!ok) {
@@ -636,7 +657,8 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
         break;
       }
       tc_fence_after_sync();
-      const uint32_t taddr = tmem_base + ((uint32_t)(wq * 32) << 16) + acc.stage * Cfg::kAccCols;
+      const uint32_t taddr = tmem_base + ((uint32_t)(wq * 32) << 16) + (wide ? 0 : acc.stage * Cfg::kStageCols);
+      const uint32_t tup = taddr + (Cfg::kWide && !wide ? 128 : N_MAX);
       const long long out_col = (long long)mb * (a.two_blocks ? 2 * kBlockM : kBlockM) + row;
       const bool col_ok = a.out_cols <= 0 || out_col < a.out_cols;  // weight rows padded up to a block are not stored
 
@@ -659,7 +681,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
         for (int c0 = c_begin; c0 < c_end; c0 += 16) {
           uint32_t g[16], up[16];
           tmem_ld_16(taddr + c0, g);
-          if (kGateUp) tmem_ld_16(taddr + N_MAX + c0, up);
+          if (kGateUp) tmem_ld_16(tup + c0, up);
           const float s_cur = s_next;
           s_next = scale_of(c0 + 16);
           tmem_ld_wait();
@@ -677,7 +699,10 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
         if (warp == 4 && lane == 0) MF_STAMP_ONCE(10);
         tc_fence_before_sync();
         __syncwarp();
-        if (lane == 0) mbar_arrive(&acc_empty[acc.stage]);
+        if (lane == 0) {
+          mbar_arrive(&acc_empty[acc.stage]);
+          if (wide) mbar_arrive(&acc_empty[acc2.stage]);
+        }
         if (a.tile_done != nullptr) {
           __threadfence();  // every lane's stores are visible device-wide before the count
           __syncwarp();
@@ -691,7 +716,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
         for (int c0 = c_begin; c0 < c_end; c0 += 16) {
           uint32_t g[16], up[16];
           tmem_ld_16(taddr + c0, g);
-          if (kGateUp) tmem_ld_16(taddr + N_MAX + c0, up);
+          if (kGateUp) tmem_ld_16(tup + c0, up);
           tmem_ld_wait();
 #pragma unroll
           for (int j = 0; j < 16; ++j) {
@@ -704,7 +729,10 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
         }
         tc_fence_before_sync();
         __syncwarp();
-        if (lane == 0) mbar_arrive(&acc_empty[acc.stage]);
+        if (lane == 0) {
+          mbar_arrive(&acc_empty[acc.stage]);
+          if (wide) mbar_arrive(&acc_empty[acc2.stage]);
+        }
         __threadfence();
         __syncwarp();
         int old = 0;
@@ -751,6 +779,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
         }
       }
       acc.advance(Cfg::kAccStages);
+      if (wide) acc.advance(Cfg::kAccStages);
       if (trace && warp == 4 && lane == 0) {
         const unsigned long long now = global_timer_ns();
         trace[5] = now;
@@ -842,6 +871,7 @@ static int check_args(const mf_gemm_args* a, int n_max, int grid) {
   if (n_max != 32 && n_max != 64 && n_max != 128 && n_max != 256) return -2;
   if (a->m_blocks < 1 || a->k_blocks < 1) return -3;
   if ((a->b_pitch & 15) != 0 || (reinterpret_cast<uintptr_t>(a->b_base) & 15) != 0) return -4;
+  if (a->b_box_rows < 0 || (a->b_box_rows > 0 && (a->b_box_rows % 16 != 0 || n_max % a->b_box_rows != 0))) return -8;
   if (a->b_tmap != nullptr && a->b_index != nullptr) return -5;  // TMA token tiles need contiguous rows
   if (a->ret_peer != nullptr && (a->out_fp32 || a->out_cols > 0)) return -6;  // the fused return path reads bf16 rows of full width
   return 0;

@@ -69,9 +69,9 @@ typedef struct {
   const int* inv;            // [rows * top_k] (row, slot) -> entry, -1 = none
   int ret_rank, ret_R, ret_C, ret_K;
   // Optional: host pointer to a 128-byte tensor map over the token operand viewed as [rows, K] with a box of
-  // n_max rows x 128 bytes (mf_make_tile_tmap).  When set, b_index must be NULL (entry n reads row
-  // b_base + n * b_pitch): token tiles are then fetched by TMA, one bulk copy per pipeline stage, instead of
-  // being gathered 16 bytes at a time.  Rows past a tile's end are fetched too and ignored.
+  // b_box_rows (0: n_max) rows x 128 bytes (mf_make_tile_tmap).  When set, b_index must be NULL (entry n reads row
+  // b_base + n * b_pitch): token tiles are then fetched by TMA, as many boxes per pipeline stage as the
+  // tile's rows need, instead of being gathered 16 bytes at a time.  Rows past a tile's end are fetched too and ignored.
   const void* b_tmap;
   // Capacities the kernel checks the plan against before it stores anything (0 = not checked).  A plan whose
   // tile count or K cut needs more than this is refused on the device: status word kBadArgument, no store.
@@ -101,6 +101,7 @@ typedef struct {
   // Optional: a device counter, zero when the kernel starts.  Segments of a K split then go to the CTA that asks next
   // instead of round-robin (work_iter.cuh).
   int* sched;
+  int b_box_rows;            // bf16 kernels: rows of a box of b_tmap, 0 = n_max; a divisor of n_max and a multiple of 16
 } mf_gemm_args;
 
 // Encode a 2-D tiled tensor map (K innermost) for a weight matrix [rows, k_elems]; box = 128 bytes x

@@ -566,8 +566,10 @@ class FixedEPLayer:
         if bool(self.gemm_kwargs.get("b_tma", True)):
             from .ops.kernels import make_tile_tmap
 
-            self._tmap_act = make_tile_tmap(self.act, self.block_m)
-            self._a_gemm2.b_tmap = C.addressof(self._tmap_act)
+            # boxes of up to 64 rows: a tile fetches what it holds in steps of 64, not block_m rows whatever it holds
+            box = min(self.block_m, 64)
+            self._tmap_act = make_tile_tmap(self.act, box)
+            self._a_gemm2.b_tmap, self._a_gemm2.b_box_rows = C.addressof(self._tmap_act), box
         # Opt-in (gemm_kwargs permute_rows=True): copy the received hidden rows into expert-major order first,
         # so that the gate/up GEMM reads token tiles by TMA too instead of gathering them by entry index.
         # Default: on with 256-row tiles, where 64 gather threads would have to place 32 chunks each per stage.
@@ -576,8 +578,10 @@ class FixedEPLayer:
             from .ops.kernels import make_tile_tmap
 
             self._xg = torch.zeros(max(N, self.block_m), H, dtype=torch.bfloat16, device=dev)
-            self._tmap_xg = make_tile_tmap(self._xg, self.block_m)
+            box = min(self.block_m, 64)
+            self._tmap_xg = make_tile_tmap(self._xg, box)
             g1 = self._a_gemm1
+            g1.b_box_rows = box
             g1.b_base, g1.b_pitch, g1.b_index = self._xg.data_ptr(), H * 2, None
             g1.b_tmap = C.addressof(self._tmap_xg)
         # Owner reduce + return push can run inside the down GEMM (gemm_kwargs fuse_return=True: four extra

@@ -85,6 +85,7 @@ class GemmArgs(C.Structure):
         ("q_scale", C.c_void_p),
         ("q_scale_pitch", C.c_longlong),
         ("sched", C.c_void_p),
+        ("b_box_rows", C.c_int),
     ]
 
 
