@@ -62,7 +62,10 @@ class GraphedMoELayer:
         self.graph: torch.cuda.CUDAGraph | None = None
         self._nodes: dict | None = None  # kernel nodes whose arguments follow the caller's buffers
         self._bound = None               # what they point at: (x, logits, rows, out), or None for the static buffers
-        self._host_refs: deque = deque(maxlen=8)  # pinned outputs that recent replays may still be writing
+        # pinned outputs that replays may still be writing: the latest one (with its stream), and earlier ones with an
+        # event behind their last replay
+        self._host_out: tuple | None = None
+        self._host_refs: deque = deque()
         self._warmup = warmup
 
     @property
@@ -161,6 +164,18 @@ class GraphedMoELayer:
         return (out is not None and out.dtype == torch.bfloat16 and out.is_contiguous() and out.data_ptr() % 16 == 0
                 and shape_ok and (out.device == self.x.device or (out.device.type == "cpu" and rows <= MAX_HOST_ROWS and out.is_pinned())))
 
+    def _hold(self, out: torch.Tensor | None) -> None:
+        """Keep a pinned output alive until the replays that write it are done (its allocator does not know of them)."""
+        refs, last = self._host_refs, self._host_out
+        now = None if out is None else torch.cuda.current_stream(self.x.device)
+        if last is not None and (last[0] is not out or last[1] != now):
+            done = torch.cuda.Event()
+            done.record(last[1])
+            refs.append((done, last[0]))
+        self._host_out = None if out is None else (out, now)
+        while refs and refs[0][0].query():
+            refs.popleft()
+
     def load(self, x: torch.Tensor, logits: torch.Tensor) -> int:
         """Copy one step's inputs (``[T, H]``, ``[T, E]``; host-pinned or device) into the static buffers."""
         t = x.shape[0]
@@ -184,7 +199,7 @@ class GraphedMoELayer:
         if self.graph is None:
             self.capture()
         t = x.shape[0]
-        if self._nodes is not None and self._readable(x, logits):
+        if self._nodes is not None and self._readable(x, logits) and not torch.cuda.is_current_stream_capturing():
             if out is not None and out.is_cuda and self._writable(out, t, tuple(out.shape) == tuple(x.shape)):
                 self._bind((x.data_ptr(), logits.data_ptr(), t, out.data_ptr()))
                 self.graph.replay()
@@ -208,10 +223,11 @@ class GraphedMoELayer:
         if self.graph is None:
             self.capture()
         self._block.copy_(inputs.raw, non_blocking=True)
-        if (self._nodes is not None and t > 0 and
+        if (self._nodes is not None and t > 0 and not torch.cuda.is_current_stream_capturing() and
                 self._writable(out, t, out is not None and out.dim() == 2 and out.shape[0] >= t and out.shape[1] == self.layer.H)):
             self._bind((self.x.data_ptr(), self.logits.data_ptr(), t, out.data_ptr()))
-            self._host_refs.append(out)
+            if not out.is_cuda:
+                self._hold(out)
             self.graph.replay()
             return out
         res = self.replay()[:t]
@@ -222,4 +238,9 @@ class GraphedMoELayer:
 
     def close(self) -> None:
         """Drop the graph (do this before destroying the process group)."""
+        if self._host_out is not None:
+            self._hold(None)
+        for done, _ in self._host_refs:
+            done.synchronize()
+        self._host_refs.clear()
         self.graph = self._nodes = self._bound = None

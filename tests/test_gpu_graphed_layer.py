@@ -78,3 +78,25 @@ def test_pinned_blocks(capacity):
         assert torch.equal(plain, want)
     assert graphed.layer.check_status()["code"] == 0
     graphed.close()
+
+
+def test_pinned_outputs_that_the_caller_drops():
+    """A new pinned output per step, the earlier ones dropped at once: each is held until its replay is done."""
+    graphed, reference = _make(16)
+    block, kept = graphed.new_pinned_inputs(), []
+    x, lg = _inputs(16, 3)
+    want = reference(x, lg).cpu()
+    block.x.copy_(x)
+    block.logits.copy_(lg)
+    block.set_rows(16)
+    torch.cuda.synchronize()
+    for i in range(40):
+        out = torch.zeros(16, CFG.hidden_size, dtype=torch.bfloat16).pin_memory()
+        graphed.step(block, out)
+        if i % 8 == 0:
+            kept.append(out)
+        del out
+    torch.cuda.synchronize()
+    assert all(torch.equal(o, want) for o in kept)
+    graphed.close()
+    assert not graphed._host_refs and graphed._host_out is None

@@ -1,0 +1,73 @@
+"""256-row token tiles that hold few rows next to full ones: units of up to 128 token columns take one accumulator stage,
+wider ones both, in any order.  Against the layer with 64-row tiles and float64 experts."""
+
+import pytest
+import torch
+
+from moeflow_b200 import MoEConfig
+from moeflow_b200.testing import make_hidden, make_weights
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("inter", [128, 384])
+@pytest.mark.parametrize("counts", [(1, 256, 16, 129, 128, 0, 257, 63), (128,) * 8, (129,) * 8, (300, 5, 300, 5, 64, 65, 192, 193)])
+def test_narrow_and_wide_units(counts, inter):
+    from moeflow_b200.fixed import FixedEPLayer
+
+    cfg = MoEConfig(hidden_size=512, moe_intermediate_size=inter, n_routed_experts=8, top_k=1)
+    w13, w2 = make_weights(cfg, 0, device="cuda")
+    t = sum(counts)
+    x = make_hidden(t, cfg, 1, device="cuda")
+    g = torch.Generator().manual_seed(2)
+    ids = torch.repeat_interleave(torch.arange(8), torch.tensor(counts))[torch.randperm(t, generator=g)].int()[:, None].cuda()
+    weights = torch.rand(t, 1, generator=g).cuda() + 0.5
+    outs = {}
+    for block_m in (64, 256):
+        layer = FixedEPLayer(cfg, 0, 1, w13, w2, capacity=t, backend="cuda", gemm_kwargs={"block_m": block_m}, wait_ns=100_000_000)
+        outs[block_m] = layer.forward_routed(x, weights, ids).clone()
+        assert torch.equal(layer.forward_routed(x, weights, ids), outs[block_m])
+        assert layer.check_status()["code"] == 0
+    exact = torch.empty(t, 512, dtype=torch.float64, device="cuda")
+    for e in range(8):
+        rows = ids[:, 0] == e
+        h = x[rows].double() @ w13[e].double().t()
+        gate, up = h[:, :inter], h[:, inter:]
+        if cfg.swiglu_limit is not None:
+            gate, up = gate.clamp(max=cfg.swiglu_limit), up.clamp(-cfg.swiglu_limit, cfg.swiglu_limit)
+        exact[rows] = weights[rows].double() * ((torch.nn.functional.silu(gate) * up) @ w2[e].double().t())
+    for out in outs.values():
+        # activations and result are rounded to bf16 once each (2**-9 of a value at most, averaged over a row)
+        err = (out.double() - exact).norm(dim=1) / exact.norm(dim=1)
+        assert float(err.max()) < 2 * 2.0**-8
+
+
+@pytest.mark.parametrize("K", [128, 384, 1536, 2048, 4096])
+def test_expansion_is_exact(K):
+    from moeflow_b200.ops.fp8 import expand_block_fp8
+
+    g = torch.Generator().manual_seed(K)
+    w = torch.randn(256, K, generator=g).to(torch.float8_e4m3fn).cuda()
+    s = torch.rand(2, K // 128, generator=g).cuda() + 0.1
+    want = (w.float() * s.repeat_interleave(128, 0).repeat_interleave(128, 1)).bfloat16()
+    assert torch.equal(expand_block_fp8(w, s), want)
+
+
+@pytest.mark.parametrize("tokens", [1, 3, 8, 100])
+@pytest.mark.parametrize("experts", [8, 36, 288])
+def test_k_splits_of_the_one_pass_metadata(tokens, experts):
+    """The splits weighed by four lanes are those of the host's cost model."""
+    from moeflow_b200.fixed import FixedEPLayer
+    from moeflow_b200.ops import _lib
+    from moeflow_b200.testing import make_logits
+
+    cfg = MoEConfig(hidden_size=512, moe_intermediate_size=256, n_routed_experts=experts, top_k=4)
+    w13, w2 = make_weights(cfg, 0, device="cuda")
+    layer = FixedEPLayer(cfg, 0, 1, w13, w2, capacity=tokens, backend="cuda")
+    layer.forward(make_hidden(tokens, cfg, 1, device="cuda"), make_logits(tokens, cfg, 2, device="cuda"), None, stop_after="META")
+    plan = layer.plan.tolist()
+    cols = max(16, (int(layer.tile_n[: plan[0]].max()) + 15) // 16 * 16)
+    floats = layer._a_meta.partial_floats
+    for word, m, k, per, over in ((1, 2, 8, 256, 4), (2, 4, 4, 128, 8)):
+        want = _lib.lib().mf_plan_split(plan[0] * m, k, layer.n_sms, floats // (per * cols), over, cols)
+        assert plan[word] == want
