@@ -188,7 +188,7 @@ class FixedEPLayer:
         if T > self.C:
             raise ValueError(f"{T} tokens exceed capacity {self.C}")
         if self.backend == "cuda":
-            return self._cuda_dispatch(x, weights, ids, num_valid)
+            return self._cuda_dispatch(x, weights, ids, num_valid)[0]
         R, K, H, L = self.world, self.K, self.H, self.L
         ids = ids.to(torch.int64)
         owner = torch.div(ids, L, rounding_mode="floor")  # [T, K]
@@ -216,7 +216,7 @@ class FixedEPLayer:
         if self.backend == "cuda":
             if x.shape[0] > self.C:
                 raise ValueError(f"{x.shape[0]} tokens exceed capacity {self.C}")
-            return self._cuda_dispatch(x, None, None, num_valid, logits=logits, bias=bias)
+            return self._cuda_dispatch(x, None, None, num_valid, logits=logits, bias=bias)[0]
         weights, ids = self.stage_route(logits, bias)
         return self.stage_dispatch_pack(x, weights, ids, num_valid)
 
@@ -242,13 +242,17 @@ class FixedEPLayer:
         ``direct_output`` the tensor ``expert_fn`` returns is itself used as the return buffer (no
         copy) after a strict shape/dtype/device/contiguity check, and is returned as ``[R, C, H]``.
         """
+        return self._experts(expert_fn, prepare_fn, direct_output)
+
+    def _experts(self, expert_fn=None, prepare_fn=None, direct_output=False, meta_done=False) -> torch.Tensor | None:
+        """``meta_done`` (cuda backend): the dispatch launch of this same forward has built the metadata."""
         R, Cc, H = self.world, self.C, self.H
         if direct_output and prepare_fn is None:
             raise ValueError("Direct expert output requires custom input preparation")
         if prepare_fn is not None:
             if expert_fn is None:
                 raise ValueError("Custom input preparation requires an external expert function")
-            if self.backend == "cuda":
+            if self.backend == "cuda" and not meta_done:
                 self._cuda_meta()  # waits for the dispatch flags of every source rank
             rows = self._recv_store.view(R * Cc, self.pitch)[:, : self.row_width]
             output = expert_fn(*prepare_fn(rows))
@@ -264,13 +268,13 @@ class FixedEPLayer:
             self._store_partials(output)
             return None
         if expert_fn is not None:
-            if self.backend == "cuda":
+            if self.backend == "cuda" and not meta_done:
                 self._cuda_meta()  # waits for the dispatch flags of every source rank
             x_rows, local, wts = self.received_routing()
             self._store_partials(expert_fn(x_rows, local, wts))
             return None
         if self.backend == "cuda":
-            self._cuda_experts()
+            self._cuda_experts(meta_done=meta_done)
             return None
         self._torch_experts()
         return None
@@ -344,13 +348,18 @@ class FixedEPLayer:
     ):
         """Pre-routed forward; ``combine_fn(ret_recv, hit)`` may replace the built-in combine."""
         T = x.shape[0]
-        hit = self.stage_dispatch_pack(x, weights, ids, num_valid)
-        if self.backend == "torch":
+        meta_done = False
+        if self.backend == "cuda":
+            if T > self.C:
+                raise ValueError(f"{T} tokens exceed capacity {self.C}")
+            hit, meta_done = self._cuda_dispatch(x, weights, ids, num_valid, whole=True)
+        else:
+            hit = self.stage_dispatch_pack(x, weights, ids, num_valid)
             self._exchange(self._recv_store, self._send_store)
         if self.backend == "cuda" and self.fuse_combine and expert_fn is None and prepare_fn is None and combine_fn is None:
-            self._cuda_experts(to_output=True)
+            self._cuda_experts(to_output=True, meta_done=meta_done)
             return self.out[:T]
-        partials = self.stage_experts(expert_fn, prepare_fn=prepare_fn, direct_output=direct_expert_output)
+        partials = self._experts(expert_fn, prepare_fn, direct_expert_output, meta_done)
         if self.backend == "torch":
             self._exchange(self.ret_recv, self.ret_send if partials is None else partials)
         elif partials is not None:
@@ -368,8 +377,13 @@ class FixedEPLayer:
         if stop_after is not None and stop_after not in STAGES:
             if not (self.backend == "cuda" and stop_after in CUDA_SUBSTAGES):
                 raise ValueError(f"stop_after must be one of {STAGES}")
+        meta_done = False
         if self.backend == "cuda" and stop_after != "ROUTER":
-            hit = self.stage_pack(x, logits, bias, num_valid)  # routing fused into the dispatch kernel
+            if x.shape[0] > self.C:
+                raise ValueError(f"{x.shape[0]} tokens exceed capacity {self.C}")
+            # routing fused into the dispatch kernel; a forward that ends before the metadata does not build them
+            hit, meta_done = self._cuda_dispatch(x, None, None, num_valid, logits=logits, bias=bias,
+                                                 whole=stop_after not in ("DISPATCH", "A2A_FORWARD"))
         else:
             weights, ids = self.stage_route(logits, bias)
             if stop_after == "ROUTER":
@@ -382,12 +396,12 @@ class FixedEPLayer:
         if stop_after == "A2A_FORWARD":
             return self.recv
         if stop_after in CUDA_SUBSTAGES:
-            self._cuda_experts(stop_after)
+            self._cuda_experts(stop_after, meta_done=meta_done)
             return self.plan
         if self.backend == "cuda" and self.fuse_combine and stop_after in (None, "COMBINE"):
-            self._cuda_experts(to_output=True)
+            self._cuda_experts(to_output=True, meta_done=meta_done)
             return self.out
-        self.stage_experts()
+        self._experts(meta_done=meta_done)
         if stop_after == "EXPERT":
             return self.ret_recv if self.backend == "cuda" else self.ret_send
         if self.backend == "torch":
@@ -614,10 +628,11 @@ class FixedEPLayer:
         )
         # A single rank has no peer to wait for: at decode sizes the dispatch kernel's last CTA builds the metadata, and
         # a whole forward ends with the owner reduce, which then writes the output (the merge over one rank is the
-        # identity).  An explicit meta_ctas keeps the two launches apart.
+        # identity).  Only a forward that goes on to the experts by itself does so: the stages called one by one stay
+        # two launches, since weights may be bound, rows rewritten or a graph capture begun between them.  An explicit
+        # meta_ctas keeps the two launches apart as well.
         self.fuse_meta = R == 1 and self.meta_ctas == 1 and n_words <= 4096 and L <= 512 and H <= 8192 and "meta_ctas" not in self.gemm_kwargs
         self.fuse_combine = R == 1 and not self.fuse_return
-        self._meta_done = False
         self._a_reduce_out = S.ReducePushArgs.from_buffer_copy(self._a_reduce)
         self._a_reduce_out.out = self.out.data_ptr()
         # during a capture: graph nodes and arguments of the first and the last kernel of the forward
@@ -795,7 +810,9 @@ class FixedEPLayer:
         self._fp8 = self._expand = None
         self._a_meta.xq = self._a_meta.xs = None
 
-    def _cuda_dispatch(self, x, weights, ids, num_valid, logits=None, bias=None) -> torch.Tensor:
+    def _cuda_dispatch(self, x, weights, ids, num_valid, logits=None, bias=None, whole: bool = False) -> tuple[torch.Tensor, bool]:
+        """``(hit, metadata built)``.  ``whole``: the caller goes on with this forward's experts, on the rows stored here
+        and the weights bound now, so the launch may build the metadata (and quantise the rows) as well."""
         from .ops import _lib
 
         if x.dtype != torch.bfloat16 or not x.is_contiguous():
@@ -819,25 +836,23 @@ class FixedEPLayer:
         a.num_valid = None if num_valid is None else num_valid.data_ptr()
         a.T = x.shape[0]
         self._keep = [x, weights, ids, num_valid, logits, bias]
-        if self.fuse_meta:
+        fused = whole and self.fuse_meta
+        if fused:
             _lib.check(self._lib.mf_dispatch_local(C.byref(a), C.byref(self._a_meta), _lib.stream_ptr()), "dispatch")
-            self._meta_done = True
         else:
             _lib.check(self._lib.mf_dispatch_push(C.byref(a), _lib.stream_ptr()), "dispatch_push")
         if self._node_log is not None:
-            self._node_log["first"] = (_lib.last_captured_node(), [a, self._a_meta] if self.fuse_meta else [a])
-        return self.hit
+            self._node_log["first"] = (_lib.last_captured_node(), [a, self._a_meta] if fused else [a])
+        return self.hit, fused
 
     def _cuda_meta(self) -> None:
         from .ops import _lib
 
-        if self._meta_done:  # built by the dispatch launch
-            self._meta_done = False
-            return
         _lib.check(self._lib.mf_expert_meta(C.byref(self._a_meta), _lib.stream_ptr()), "expert_meta")
 
-    def _cuda_experts(self, stop_after: str | None = None, to_output: bool = False) -> None:
-        """``to_output`` (one rank): the owner reduce writes the layer's output, no combine follows."""
+    def _cuda_experts(self, stop_after: str | None = None, to_output: bool = False, meta_done: bool = False) -> None:
+        """``to_output`` (one rank): the owner reduce writes the layer's output, no combine follows.  ``meta_done``: the
+        dispatch launch of this forward has built the metadata."""
         from .ops import _lib
 
         if self._tmap13 is None:
@@ -850,7 +865,8 @@ class FixedEPLayer:
                                                 self.L * 2 * self.I, self.H, s), "expand e4m3 gate/up weights")
             _lib.check(lib.mf_dequant_block_fp8(p["w2"].data_ptr(), p["s2"].data_ptr(), self.w2.data_ptr(),
                                                 self.L * self.H, self.I, s), "expand e4m3 down weights")
-        self._cuda_meta()
+        if not meta_done:
+            self._cuda_meta()
         if stop_after == "META":
             return
         if self._fp8 is not None:
