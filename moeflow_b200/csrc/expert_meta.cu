@@ -496,7 +496,11 @@ __global__ void __launch_bounds__(kMetaThreads) expert_meta_place_kernel(const m
 }  // namespace mf
 
 extern "C" int mf_plan_split(int units, int k_blocks, int n_sms, int max_slots, int overhead_kb, int cols) {
-  return mf::choose_split(units, k_blocks, n_sms, max_slots, overhead_kb, cols);
+  return mf_plan_split_steps(units, k_blocks, 1, n_sms, max_slots, overhead_kb, cols);
+}
+
+extern "C" int mf_plan_split_steps(int units, int k_blocks, int k_step, int n_sms, int max_slots, int overhead_kb, int cols) {
+  return mf::choose_split(units, k_blocks, k_step, n_sms, max_slots, overhead_kb, cols);
 }
 
 extern "C" int mf_expert_meta(const mf_meta_args* a, mf_stream_t stream) {

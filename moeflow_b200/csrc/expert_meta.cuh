@@ -56,29 +56,42 @@ __device__ __forceinline__ void clear_counters(const mf_meta_args& a, int n_tile
     for (int i = threadIdx.x; i < min(n_tiles * a.m_blocks2 * 8, a.n_counters2); i += kThreads) a.counters2[i] = 0;
 }
 
-// Pick the K split S in {1,2,4,8}.  Cost model in units of one K block of streaming: a unit costs its
+// Cost of the K split S = 2^log_s, or kNoSplit.  In units of one K block of 64 values of streaming: a unit costs its
 // K blocks plus a fixed overhead (pipeline fill, epilogue, and for S > 1 the partial-sum round trip);
-// the kernel takes ceil(units * S / SMs) rounds of such units.  Ties go to the smaller S.
-__host__ __device__ __forceinline__ int choose_split(int units, int k_blocks, int n_sms, int max_slots,
-                                                     int overhead_kb, int cols) {
-  if (units <= 0) return 1;
-  int best = 1;
-  long long best_cost = (long long)((units + n_sms - 1) / n_sms) * (k_blocks + overhead_kb);
+// the kernel takes ceil(units * S / SMs) rounds of such units.  K is cut between steps of k_step blocks: the e4m3 kernels
+// work on K blocks of 128 values (k_step 2) and refuse a split that does not divide those.  units * 8 fits 32 bits (16
+// million token tiles of 32 weight blocks).
+constexpr long long kNoSplit = 0x7fffffffffffffffll;
+__host__ __device__ __forceinline__ long long split_cost(int log_s, int units, int k_blocks, int k_step, int n_sms, int max_slots,
+                                                         int overhead_kb, int cols) {
+  const int s = 1 << log_s;
+  const int rounds = (int)(((unsigned)units * (unsigned)s + (unsigned)n_sms - 1u) / (unsigned)n_sms);
+  if (s == 1) return (long long)rounds * (k_blocks + overhead_kb);
+  if ((k_blocks & (s * k_step - 1)) != 0 || (k_blocks >> log_s) < 2 || (long long)units * s > max_slots) return kNoSplit;
   // the partial-sum round trip of a split unit grows with the tile's token columns (measured: splitting
   // 64-column tiles in two cost more than the idle SMs of an uneven last round)
   const int wide = cols > 16 ? (cols - 16) / 8 : 0;
-  for (int s = 2; s <= 8; s <<= 1) {
-    if (k_blocks % s != 0 || k_blocks / s < 2) break;
-    if ((long long)units * s > max_slots) break;
-    const long long rounds = ((long long)units * s + n_sms - 1) / n_sms;
-    const long long cost = rounds * (k_blocks / s + overhead_kb + 1 + wide);
+  return (long long)rounds * ((k_blocks >> log_s) + overhead_kb + 1 + wide);
+}
+
+// The cheapest of the splits 1, 2, 4, 8; ties go to the smaller one.
+__host__ __device__ __forceinline__ int choose_split(int units, int k_blocks, int k_step, int n_sms, int max_slots,
+                                                     int overhead_kb, int cols) {
+  if (units <= 0) return 1;
+  int best = 0;
+  long long best_cost = split_cost(0, units, k_blocks, k_step, n_sms, max_slots, overhead_kb, cols);
+  for (int log_s = 1; log_s < 4; ++log_s) {
+    const long long cost = split_cost(log_s, units, k_blocks, k_step, n_sms, max_slots, overhead_kb, cols);
     if (cost < best_cost) {
       best_cost = cost;
-      best = s;
+      best = log_s;
     }
   }
-  return best;
+  return 1 << best;
 }
+
+// K steps of the bound experts' kernels, in blocks of 64 values (1 unless the caller says 2).
+__device__ __forceinline__ int k_step_of(const mf_meta_args& a) { return a.k_step == 2 ? 2 : 1; }
 
 // The K cut of one GEMM: stream-K (0) when asked for, the units do not fill many rounds of the persistent CTAs
 // (below 8 units per CTA an uneven last round costs more than the partial tiles of the cut units) and the
@@ -86,20 +99,16 @@ __host__ __device__ __forceinline__ int choose_split(int units, int k_blocks, in
 __device__ __forceinline__ int choose_cut(const mf_meta_args& a, int units, int k_blocks, int slots, int overhead_kb,
                                           int cols) {
   if (a.stream_k && units > 0 && units < 8 * a.n_sms && units % a.n_sms != 0 && slots >= 2 * a.n_sms) return 0;
-  return choose_split(units, k_blocks, a.n_sms, slots, overhead_kb, cols);
+  return choose_split(units, k_blocks, k_step_of(a), a.n_sms, slots, overhead_kb, cols);
 }
 
 // The same choice by the four lanes of a group (lane & 3 = log2 of the split it weighs; the whole warp calls): the splits
-// are weighed side by side and in 32-bit divisions, where one thread went through them one after the other, in the tail
-// of the pass that the GEMMs wait for.  units * 8 fits 32 bits (at most 8192 tiles).
+// are weighed side by side, where one thread went through them one after the other, in the tail of the pass that the GEMMs
+// wait for.
 __device__ __forceinline__ int choose_cut_lanes(const mf_meta_args& a, int units, int k_blocks, int slots, int overhead_kb,
                                                 int cols, int log_s) {
-  const int s = 1 << log_s;
-  const int wide = cols > 16 ? (cols - 16) / 8 : 0;
-  const int rounds = (int)((unsigned)(units * s + a.n_sms - 1) / (unsigned)a.n_sms);
-  const bool can = s == 1 || ((k_blocks & (s - 1)) == 0 && (k_blocks >> log_s) >= 2 && (long long)units * s <= slots);
-  const long long cost = (long long)rounds * ((k_blocks >> log_s) + overhead_kb + (s == 1 ? 0 : 1 + wide));
-  long long key = can ? cost * 4 + log_s : 0x7fffffffffffffffll;  // ties go to the smaller split
+  const long long cost = split_cost(log_s, units, k_blocks, k_step_of(a), a.n_sms, slots, overhead_kb, cols);
+  long long key = cost != kNoSplit ? cost * 4 + log_s : kNoSplit;  // ties go to the smaller split
 #pragma unroll
   for (int off = 1; off < 4; off <<= 1) {
     const long long o = __shfl_xor_sync(0xffffffffu, key, off);

@@ -267,6 +267,7 @@ typedef struct {
   // mf_quant_rows_1x128, on CTAs of its own.
   uint8_t* xq;               // [rows, H] e4m3
   float* xs;                 // [rows, H / 128]
+  int k_step;                // K blocks of 64 values per K step of the GEMMs the plan is for: 2 for the e4m3 kernels, else 1
 } mf_meta_args;
 int mf_expert_meta(const mf_meta_args* args, mf_stream_t stream);
 // Dispatch and metadata in one launch: the only rank is this GPU (R = 1), at most 512 experts and 4096 slot words.
@@ -276,6 +277,8 @@ int mf_dispatch_local(const mf_dispatch_args* args, const mf_meta_args* meta, mf
 // `max_slots` partial-sum slots, the fixed per-unit overhead in K-block units (4 for gate/up, 8 for down) and
 // the tile's token columns `cols`.
 int mf_plan_split(int units, int k_blocks, int n_sms, int max_slots, int overhead_kb, int cols);
+// The same with K cut only between steps of k_step (1 or 2) blocks of 64 values (mf_meta_args.k_step).
+int mf_plan_split_steps(int units, int k_blocks, int k_step, int n_sms, int max_slots, int overhead_kb, int cols);
 
 // ---- owner reduce + return push, combine -------------------------------------------------------------
 typedef struct {

@@ -782,6 +782,7 @@ class FixedEPLayer:
         f["a1"].w_scale, f["a2"].w_scale = pack["s13"].data_ptr(), pack["s2"].data_ptr()
         f["tm13"], f["tm2"], f["pack"] = pack["tm13"], pack["tm2"], pack
         self._fp8 = f
+        self._a_meta.k_step = 2  # the e4m3 kernels' K blocks hold 128 values: no split between two halves of one
         if f["in_meta"]:
             self._a_meta.xq, self._a_meta.xs = f["xq"].data_ptr(), f["xs"].data_ptr()
         self.w13, self.w2 = pack["w13"], pack["w2"]
@@ -809,6 +810,7 @@ class FixedEPLayer:
     def _bind_bf16(self) -> None:
         self._fp8 = self._expand = None
         self._a_meta.xq = self._a_meta.xs = None
+        self._a_meta.k_step = 1
 
     def _cuda_dispatch(self, x, weights, ids, num_valid, logits=None, bias=None, whole: bool = False) -> tuple[torch.Tensor, bool]:
         """``(hit, metadata built)``.  ``whole``: the caller goes on with this forward's experts, on the rows stored here

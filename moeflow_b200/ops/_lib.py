@@ -191,6 +191,7 @@ class MetaArgs(C.Structure):
         ("n_tile_done", C.c_int),
         ("xq", C.c_void_p),
         ("xs", C.c_void_p),
+        ("k_step", C.c_int),
     ]
 
 
@@ -279,6 +280,7 @@ def lib() -> C.CDLL:
         "mf_dispatch_local": [C.POINTER(DispatchArgs), C.POINTER(MetaArgs), P],
         "mf_expert_meta": [C.POINTER(MetaArgs), P],
         "mf_plan_split": [I, I, I, I, I, I],
+        "mf_plan_split_steps": [I, I, I, I, I, I, I],
         "mf_permute_rows": [P, LL, P, P, P, I, I, I, P],
         "mf_owner_reduce_push": [C.POINTER(ReducePushArgs), P],
         "mf_combine": [C.POINTER(CombineArgs), P],

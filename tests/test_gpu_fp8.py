@@ -164,6 +164,36 @@ def test_layer_with_fp8_weights_matches_dequantised_oracle(world):
         assert outs[r][t:].abs().sum() == 0
 
 
+@pytest.mark.parametrize("hidden,inter,experts,tokens,top_k", [
+    (384, 128, 8, 3, 2), (2048, 1408, 4, 5, 2), (2048, 1536, 2, 1, 1), (640, 384, 3, 40, 1), (384, 128, 8, 700, 8)])
+def test_layers_with_an_odd_number_of_scale_blocks(hidden, inter, experts, tokens, top_k):
+    """Few units on many SMs: the K split has to divide the 128-wide blocks, in the dispatch launch's metadata pass, in
+    the one-pass launch of its own and (700 tokens of 8) in the two-launch form."""
+    from moeflow_b200 import MoEConfig
+    from moeflow_b200.fixed import FixedEPLayer
+    from moeflow_b200.reference import moe_reference
+    from moeflow_b200.testing import make_bias, make_hidden, make_logits, make_weights
+
+    cfg = MoEConfig(hidden_size=hidden, moe_intermediate_size=inter, n_routed_experts=experts, top_k=top_k)
+    w13, w2 = make_weights(cfg, 0, dtype=torch.float32)
+    packs = [(quant_block_fp8(w13[e]), quant_block_fp8(w2[e])) for e in range(experts)]
+    stack8 = lambda ts: torch.stack([t.view(torch.uint8) for t in ts]).view(torch.float8_e4m3fn).cuda()  # noqa: E731
+    bias = make_bias(cfg, 1, device="cuda")
+    x, logits = make_hidden(tokens, cfg, 2, device="cuda"), make_logits(tokens, cfg, 3, device="cuda")
+    ref = moe_reference(x.cpu(), logits.cpu(), bias.cpu(), torch.stack([dequant_block_fp8(*p[0]) for p in packs]),
+                        torch.stack([dequant_block_fp8(*p[1]) for p in packs]), cfg)
+    for kwargs in ({}, {"meta_ctas": 1}, {"meta_ctas": 3}):
+        layer = FixedEPLayer(cfg, 0, 1, None, None, capacity=tokens, backend="cuda", device="cuda",
+                             gemm_kwargs={"block_m": 64, **kwargs}, wait_ns=50_000_000)
+        layer.set_weights_fp8(stack8([p[0][0] for p in packs]), torch.stack([p[0][1] for p in packs]).cuda(),
+                              stack8([p[1][0] for p in packs]), torch.stack([p[1][1] for p in packs]).cuda())
+        out = layer.forward(x, logits, bias)
+        assert layer.check_status()["code"] == 0
+        assert (hidden // 128) % int(layer.plan[1]) == 0 and (inter // 128) % int(layer.plan[2]) == 0
+        # activations are e4m3 (3 mantissa bits) per 128-wide group, as in the test above
+        assert normwise_rel_err(out.cpu(), ref) < 0.06
+
+
 @pytest.mark.parametrize("shape", [(128, 128), (3, 256, 512), (2, 384, 1536)])
 def test_expand_block_fp8_equals_definition(shape):
     """e4m3 x block scale -> bf16 in one pass equals the PyTorch dequantisation rounded once to bf16."""

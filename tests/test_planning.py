@@ -65,3 +65,22 @@ def test_decode_sizes_split_k_to_fill_the_sms(plan_split):
 def test_split_always_divides_k_and_fits_the_slots(plan_split, units, k_blocks, cols):
     s = plan_split(units, k_blocks, 148, 1024, 4, cols)
     assert s in (1, 2, 4, 8) and k_blocks % s == 0 and (s == 1 or (k_blocks // s >= 2 and units * s <= 1024))
+
+
+def test_k_splits_of_e4m3_layers_divide_their_128_wide_blocks(plan_split):
+    """The e4m3 kernels refuse any other plan.  Where the plain rule's split divides them, it is the one taken."""
+    from moeflow_b200.ops import _lib
+
+    steps = _lib.lib().mf_plan_split_steps
+    refused = 0
+    for blocks in range(1, 33):  # K = 128 .. 4096
+        for units in (1, 2, 3, 8, 12, 22, 32, 96, 148, 149, 300, 432, 1024):
+            for overhead, cols in ((4, 16), (8, 16), (4, 64), (8, 128)):
+                plain, got = plan_split(units, 2 * blocks, 148, 4096, overhead, cols), steps(units, 2 * blocks, 2, 148, 4096, overhead, cols)
+                assert blocks % got == 0 and got <= plain
+                if blocks % plain == 0:
+                    assert got == plain
+                refused += blocks % plain != 0
+                assert steps(units, 2 * blocks, 1, 148, 4096, overhead, cols) == plain
+    assert refused > 0  # hidden 384 with intermediate 128, hidden 2048 with 1408 or (one tile) 1536
+    assert plan_split(3, 6, 148, 4096, 4, 16) == 2 and steps(3, 6, 2, 148, 4096, 4, 16) == 1
