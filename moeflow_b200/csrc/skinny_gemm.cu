@@ -242,6 +242,8 @@ extern "C" int mf_skinny_gemm(const void* tmap_w, const mf_skinny_args* a, int g
   if (a->T == 0) return 0;
   if (a->T < 0 || a->k_blocks < 1 || a->row_blocks < 1) return -2;
   if ((a->x_pitch & 15) != 0 || (reinterpret_cast<uintptr_t>(a->x) & 15) != 0) return -3;
+  if (a->residual2 != nullptr && a->residual == nullptr) return -4;
+  if (a->residual != nullptr && a->out_fp32) return -4;  // added in the bf16 epilogue only
   CUtensorMap tw, tx;
   memcpy(&tw, tmap_w, sizeof(tw));
   // The token rows may be any buffer of the caller's (no copy into a fixed one): rows past T read as zero.

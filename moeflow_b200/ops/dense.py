@@ -27,6 +27,7 @@ class DenseProjection:
         if k % 64 or self.outputs % block or w.dtype != torch.bfloat16:
             raise ValueError("bf16 weights with K a multiple of 64 and rows in whole blocks expected")
         self.w, self.k, self.gate_up = w.contiguous(), k, gate_up
+        self._width = min(out_cols, self.outputs) if out_cols > 0 else self.outputs  # columns that are stored
         self.status = status if status is not None else torch.zeros(1, dtype=torch.int64, device=w.device)
         self.n_sms = sm_count(w.device.index or 0)
         self._lib = _lib.lib()
@@ -35,17 +36,39 @@ class DenseProjection:
                                      out_cols=out_cols, limit=float(limit) if limit is not None else 0.0,
                                      status=self.status.data_ptr(), wait_ns=wait_ns)
 
+    def _check(self, name: str, t: torch.Tensor, rows: int, dtypes: tuple) -> None:
+        """The kernel takes raw pointers: what it indexes has to be there."""
+        if t.dtype not in dtypes or t.device != self.w.device:
+            raise ValueError(f"{name} must be {' or '.join(str(d) for d in dtypes)} on the weights' device")
+        if t.dim() != 2 or t.shape[0] < rows or t.shape[1] < self._width or (self._width > 1 and t.stride(1) != 1):
+            raise ValueError(f"{name} must hold {rows} rows of {self._width} adjacent values")
+
     def __call__(self, x: torch.Tensor, out: torch.Tensor, residual: torch.Tensor | None = None,
                  residual2: torch.Tensor | None = None) -> torch.Tensor:
-        """Writes ``out[: T]`` for ``x [T, K]`` (bf16 rows, any 16-byte pitch).  ``residual`` (bf16 ``[T, rows]``), or
-        the bf16 sum ``residual + residual2``, is added to the bf16 product."""
+        """Writes ``out[: T]`` for ``x [T, K]``: bf16 rows at any 16-byte pitch are read in place, other types, layouts and
+        devices are copied first.  ``residual`` (bf16 ``[T, rows]``), or the bf16 sum ``residual + residual2``, is added
+        to the bf16 product."""
         t = x.shape[0]
-        if x.shape[1] != self.k or out.shape[0] < t:
+        if x.dim() != 2 or x.shape[1] != self.k:
             raise ValueError("token rows do not fit this projection")
-        if x.dtype != torch.bfloat16 or x.stride(1) != 1 or x.stride(0) % 8 or x.data_ptr() % 16:
-            x = x.to(torch.bfloat16).contiguous()
+        self._check("out", out, t, (torch.bfloat16, torch.float32))
+        if out.shape[0] > 1 and out.stride(0) < self._width:
+            raise ValueError("the rows of out overlap")
+        if residual2 is not None and residual is None:
+            raise ValueError("residual2 is added to residual")
+        for name, r in (("residual", residual), ("residual2", residual2)):
+            if r is not None:
+                self._check(name, r, t, (torch.bfloat16,))
+        if residual is not None and out.dtype != torch.bfloat16:
+            raise ValueError("a residual is added to a bf16 product")
+        if t == 0:
+            return out[:0]
+        if x.device != self.w.device or x.dtype != torch.bfloat16:
+            x = x.to(self.w.device, torch.bfloat16)
+        if x.stride(1) != 1 or (t > 1 and (x.stride(0) < self.k or x.stride(0) % 8)) or x.data_ptr() % 16:
+            x = x.clone(memory_format=torch.contiguous_format)
         a = self._args
-        a.x, a.x_pitch, a.T = x.data_ptr(), x.stride(0) * 2, t
+        a.x, a.x_pitch, a.T = x.data_ptr(), (x.stride(0) if t > 1 else self.k) * 2, t
         a.out, a.out_pitch, a.out_fp32 = out.data_ptr(), out.stride(0), int(out.dtype == torch.float32)
         a.residual, a.residual_pitch = (residual.data_ptr(), residual.stride(0)) if residual is not None else (None, 0)
         a.residual2, a.residual2_pitch = (residual2.data_ptr(), residual2.stride(0)) if residual2 is not None else (None, 0)

@@ -68,3 +68,62 @@ def test_fp32_output_stores_only_the_real_columns(cols):
     exact = x.double() @ w[:cols].double().t()
     slack = (x.double().abs() @ w[:cols].double().abs().t()) * (512 * 2.0**-24)
     assert ((out.double() - exact).abs() <= slack).all() and not guard.any()
+
+
+@pytest.mark.parametrize("tokens", [1, 5])
+def test_token_rows_of_any_layout_type_and_device(tokens):
+    """What the kernel cannot read in place is copied: expanded, overlapping, odd or transposed rows, other types, host memory."""
+    from moeflow_b200.models.glm_moe import RouterLogits, SharedExpert
+
+    k, inter = 256, 128
+    g = torch.Generator().manual_seed(3)
+    base = torch.randn(4 * tokens * k, generator=g).bfloat16().cuda()
+    gate_w = torch.randn(48, k, generator=g).cuda()
+    shared = SharedExpert((torch.randn(2 * inter, k, generator=g) / 16).bfloat16().cuda(),
+                          (torch.randn(k, inter, generator=g) / 11).bfloat16().cuda(), 8, 10.0)
+    router = RouterLogits(gate_w, 8)
+    rows = {
+        "expanded": base[:k].expand(tokens, k),
+        "overlapping": base.as_strided((tokens, k), (8, 1)),
+        "odd pitch": base.as_strided((tokens, k), (k + 1, 1)),
+        "odd start": base.as_strided((tokens, k), (k, 1), 1),
+        "row stride 1": base.as_strided((1, k), (1, 1)).expand(tokens, k),
+        "transposed": base[: tokens * k].view(k, tokens).t(),
+        "fp32": base[: tokens * k].view(tokens, k).float(),
+        "host": base[: tokens * k].view(tokens, k).cpu(),
+        "empty": base[:0].view(0, k),
+    }
+    for name, x in rows.items():
+        plain = x.clone(memory_format=torch.contiguous_format).bfloat16().cuda()
+        first = router(x).clone()
+        assert torch.equal(first, router(plain)), name
+        first = shared(x).clone()
+        assert torch.equal(first, shared(plain)) and first.shape == (x.shape[0], k), name
+    assert int(shared.status.item()) == 0 and int(router.status.item()) == 0
+
+
+def test_operands_that_do_not_fit_are_refused():
+    from moeflow_b200.ops.dense import DenseProjection
+
+    x, w = _case(3, 256, 128)
+    project, bf16 = DenseProjection(w), dict(dtype=torch.bfloat16, device="cuda")
+    good, wide = torch.zeros(3, 256, **bf16), torch.zeros(3, 512, **bf16)
+    bad = [good.float(), good.cpu(), good[:2], good[:, :255], wide[:, ::2], good[0]]
+    for r in bad:
+        with pytest.raises(ValueError):
+            project(x, good, r)
+        with pytest.raises(ValueError):
+            project(x, good, good, r)
+    for out in [good.half(), *bad[1:], good[:1].expand(3, 256)]:
+        with pytest.raises(ValueError):
+            project(x, out)
+    with pytest.raises(ValueError):
+        project(x, good.float(), good)  # residuals belong to a bf16 product
+    with pytest.raises(ValueError):
+        project(x, good, None, good)
+    with pytest.raises(ValueError):
+        project(x[:, :64], good)
+    want = project(x, good.clone(), good)
+    assert torch.equal(project(x, wide[:, 256:], good[:1].expand(3, 256)), want)  # a strided out, an expanded residual
+    narrow = DenseProjection(w, out_cols=100)
+    assert torch.equal(narrow(x, torch.zeros(3, 100, **bf16)), want[:, :100])
