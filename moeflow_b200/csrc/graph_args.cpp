@@ -3,7 +3,8 @@
 // A serving step used to copy its inputs into the buffers the captured graph reads and its output out of the one it
 // writes: three or four small stream operations around the replay, about 3 us each plus the gap in front of the graph.
 // Instead the graph's first and last kernels are pointed at the caller's buffers (a host-side update of the executable
-// graph, only when the pointers or the row count have changed).
+// graph, only when the pointers or the row count have changed).  That is done on an executable graph of its own, launched
+// only behind such an update: the one that the owner of the capture replays keeps the arguments it was captured with.
 #include <cuda_runtime.h>
 
 #include "moeflow_b200.h"
@@ -27,6 +28,30 @@ int mf_capture_last_node(mf_stream_t stream, void** node_out) {
   if (type != cudaGraphNodeTypeKernel) return -3;
   *node_out = deps[0];
   return 0;
+}
+
+int mf_graph_instantiate(void* graph, mf_stream_t stream, void** exec_out) {
+  if (!graph || !exec_out) return -1;
+  cudaGraphExec_t exec = nullptr;
+  cudaError_t e = cudaGraphInstantiate(&exec, static_cast<cudaGraph_t>(graph), 0);
+  if (e != cudaSuccess) return (int)e;
+  e = cudaGraphUpload(exec, static_cast<cudaStream_t>(stream));  // not at the first launch
+  if (e != cudaSuccess) {
+    cudaGraphExecDestroy(exec);
+    return (int)e;
+  }
+  *exec_out = exec;
+  return 0;
+}
+
+int mf_graph_launch(void* graph_exec, mf_stream_t stream) {
+  if (!graph_exec) return -1;
+  return (int)cudaGraphLaunch(static_cast<cudaGraphExec_t>(graph_exec), static_cast<cudaStream_t>(stream));
+}
+
+int mf_graph_destroy(void* graph_exec) {
+  if (!graph_exec) return -1;
+  return (int)cudaGraphExecDestroy(static_cast<cudaGraphExec_t>(graph_exec));
 }
 
 // Replaces the by-value arguments of a kernel node (one pointer per argument; same kernel, same launch shape) in an

@@ -340,8 +340,12 @@ int mf_gemm_down_fp8(const void* tmap, const mf_gemm_args* args, int n_max, int 
 
 // ---- captured forwards ------------------------------------------------------------------------------------
 // mf_capture_last_node: the kernel node that the capture on `stream` added last.  mf_graph_set_args: replaces the
-// by-value argument structs of such a node in the executable graph made from that capture.
+// by-value argument structs of such a node in an executable graph made from that capture.  mf_graph_instantiate,
+// _launch, _destroy: such an executable graph beside the owner's.
 int mf_capture_last_node(mf_stream_t stream, void** node_out);
+int mf_graph_instantiate(void* graph, mf_stream_t stream, void** exec_out);
+int mf_graph_launch(void* graph_exec, mf_stream_t stream);
+int mf_graph_destroy(void* graph_exec);
 int mf_graph_set_args(void* graph_exec, void* node, void** args);
 
 // ---- peer-memory runtime ------------------------------------------------------------------------------------

@@ -2,7 +2,8 @@
 
 ``GraphedMoELayer`` is the call a user makes on the hot path.  It captures ``FixedEPLayer.forward`` once, and then
 every call is a replay on this step's hidden states and router logits.  Nothing is allocated and nothing is read back
-to the host by the layer itself, so the call can sit inside a larger captured decode step as well.
+to the host by the layer itself.  A replay cannot be captured: a larger captured decode step takes
+``FixedEPLayer.forward`` instead, and these calls raise while the current stream is capturing.
 
 Two ways to feed it:
 
@@ -17,11 +18,16 @@ updating the two kernel nodes' arguments when pointers or row count change.  Oth
 strides) are copied into the static buffers ``.x`` / ``.logits`` / ``.num_valid`` first, which is also what ``load`` and
 ``replay`` work on.  The small copies and the gap in front of the graph were 13 us of a device-fed call.  A pinned input
 block is still one copy: read by the first kernel itself over PCIe, 24 rows took 43 us, the copy engine needs 9.
+
+The calls on the caller's buffers launch an executable graph of their own.  ``.graph`` is the forward on the static
+buffers, whoever replays it and whatever was called before (it is instantiated by its first replay); ``.out`` holds the
+rows of ``replay`` and of the calls without ``out`` (a call with ``out`` may leave it as it was).
 """
 
 from __future__ import annotations
 
 import ctypes as C
+import weakref
 from collections import deque
 
 import torch
@@ -61,7 +67,8 @@ class GraphedMoELayer:
         self.num_valid.fill_(layer.C)
         self.graph: torch.cuda.CUDAGraph | None = None
         self._nodes: dict | None = None  # kernel nodes whose arguments follow the caller's buffers
-        self._bound = None               # what they point at: (x, logits, rows, out), or None for the static buffers
+        self._exec = None                # executable graph with those arguments; only _launch uses it
+        self._bound: dict = {}           # what its first and last node point at
         # pinned outputs that replays may still be writing: the latest one (with its stream), and earlier ones with an
         # event behind their last replay
         self._host_out: tuple | None = None
@@ -100,6 +107,7 @@ class GraphedMoELayer:
 
     def capture(self) -> "GraphedMoELayer":
         """Warm up on a side stream, then capture one forward.  Every rank must call this together."""
+        self._drop()
         side = torch.cuda.Stream(device=self.layer.device)
         side.wait_stream(torch.cuda.current_stream())
         with torch.cuda.stream(side):
@@ -121,37 +129,37 @@ class GraphedMoELayer:
         if native:
             from ..ops import _lib
 
-            graph.instantiate()
             for name, (node, args) in nodes.items():
                 own = [type(a).from_buffer_copy(a) for a in args]
                 nodes[name] = (node, own[0], (C.c_void_p * len(own))(*(C.addressof(a) for a in own)), own)
-            self._set_args, self._exec = _lib.lib().mf_graph_set_args, graph.raw_cuda_graph_exec()
-        self.graph, self._nodes, self._bound = graph, nodes, None
+            own_exec = C.c_void_p()
+            _lib.check(_lib.lib().mf_graph_instantiate(graph.raw_cuda_graph(), _lib.stream_ptr(), C.byref(own_exec)), "graph instantiation")
+            self._set_args, self._exec = _lib.lib().mf_graph_set_args, own_exec.value
+            self._drop_exec = weakref.finalize(self, _lib.lib().mf_graph_destroy, own_exec.value)
+            self._drop_exec.atexit = False  # the context goes first
+            self._own_out = (self.layer.out.data_ptr(), 0)
+            self._bound = {"last": self._own_out}  # as captured
+        self.graph, self._nodes = graph, nodes
         torch.cuda.synchronize()
         return self
 
-    def _bind(self, key) -> None:
-        """Point the captured forward at ``key = (x, logits, rows, out)`` (addresses; ``out`` None: the layer's own
-        buffer), or back at the static buffers (``key`` None)."""
-        if key == self._bound:
-            return
+    def _launch(self, x: int, logits: int, rows: int, out: int | None) -> None:
+        """Replay on the caller's buffers (addresses; ``out`` None: all rows of the layer's own buffer)."""
         from ..ops import _lib
 
-        first, a, first_list, _ = self._nodes["first"]
-        last, c, last_list, _ = self._nodes["last"]
-        layer = self.layer
-        if key is None:
-            a.x, a.logits, a.T, a.num_valid = self.x.data_ptr(), self.logits.data_ptr(), layer.C, self.num_valid.data_ptr()
-            out, rows = None, 0
-        else:
-            a.x, a.logits, a.T, out = key
-            a.num_valid, rows = None, key[2]
-        was = None if self._bound is None else self._bound[3]
-        _lib.check(self._set_args(self._exec, first, first_list), "graph update")
-        if out != was or out is not None:
-            c.out, c.rows = (layer.out.data_ptr(), 0) if out is None else (out, rows)
-            _lib.check(self._set_args(self._exec, last, last_list), "graph update")
-        self._bound = key
+        for name, key in (("first", (x, logits, rows)), ("last", self._own_out if out is None else (out, rows))):
+            if self._bound.get(name) == key:
+                continue
+            node, a, arg_list, _ = self._nodes[name]
+            if name == "first":
+                a.x, a.logits, a.T = key
+                a.num_valid = None
+            else:
+                a.out, a.rows = key
+            self._bound.pop(name, None)  # unknown if the update fails
+            _lib.check(self._set_args(self._exec, node, arg_list), "graph update")
+            self._bound[name] = key
+        _lib.check(_lib.lib().mf_graph_launch(self._exec, _lib.stream_ptr()), "graph launch")
 
     def _readable(self, x: torch.Tensor, logits: torch.Tensor) -> bool:
         """Can the captured kernels read these tensors where they are?"""
@@ -189,8 +197,6 @@ class GraphedMoELayer:
     def replay(self) -> torch.Tensor:
         if self.graph is None:
             self.capture()
-        if self._nodes is not None:
-            self._bind(None)
         self.graph.replay()
         return self.out
 
@@ -201,11 +207,9 @@ class GraphedMoELayer:
         t = x.shape[0]
         if self._nodes is not None and self._readable(x, logits) and not torch.cuda.is_current_stream_capturing():
             if out is not None and out.is_cuda and self._writable(out, t, tuple(out.shape) == tuple(x.shape)):
-                self._bind((x.data_ptr(), logits.data_ptr(), t, out.data_ptr()))
-                self.graph.replay()
+                self._launch(x.data_ptr(), logits.data_ptr(), t, out.data_ptr())
                 return out
-            self._bind((x.data_ptr(), logits.data_ptr(), t, None))
-            self.graph.replay()
+            self._launch(x.data_ptr(), logits.data_ptr(), t, None)
             res = self.out[:t]
         else:
             t = self.load(x, logits)
@@ -225,16 +229,21 @@ class GraphedMoELayer:
         self._block.copy_(inputs.raw, non_blocking=True)
         if (self._nodes is not None and t > 0 and not torch.cuda.is_current_stream_capturing() and
                 self._writable(out, t, out is not None and out.dim() == 2 and out.shape[0] >= t and out.shape[1] == self.layer.H)):
-            self._bind((self.x.data_ptr(), self.logits.data_ptr(), t, out.data_ptr()))
             if not out.is_cuda:
                 self._hold(out)
-            self.graph.replay()
+            self._launch(self.x.data_ptr(), self.logits.data_ptr(), t, out.data_ptr())
             return out
         res = self.replay()[:t]
         if out is not None:
             out[:t].copy_(res, non_blocking=True)
             return out
         return res
+
+    def _drop(self) -> None:
+        if self._exec is not None:
+            self._drop_exec()  # one still running is freed when it is done
+        self.graph = self._nodes = self._exec = None
+        self._bound = {}
 
     def close(self) -> None:
         """Drop the graph (do this before destroying the process group)."""
@@ -243,4 +252,4 @@ class GraphedMoELayer:
         for done, _ in self._host_refs:
             done.synchronize()
         self._host_refs.clear()
-        self.graph = self._nodes = self._bound = None
+        self._drop()

@@ -286,6 +286,9 @@ def lib() -> C.CDLL:
         "mf_combine": [C.POINTER(CombineArgs), P],
         "mf_expert_prepare": [P, LL, I, I, I, I, I, P, P, P, P, P],
         "mf_capture_last_node": [P, C.POINTER(P)],
+        "mf_graph_instantiate": [P, P, C.POINTER(P)],
+        "mf_graph_launch": [P, P],
+        "mf_graph_destroy": [P],
         "mf_graph_set_args": [P, P, C.POINTER(P)],
         "mf_peer_alloc": [C.POINTER(P), ULL],
         "mf_peer_free": [P],

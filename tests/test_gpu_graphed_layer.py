@@ -100,3 +100,38 @@ def test_pinned_outputs_that_the_caller_drops():
     assert all(torch.equal(o, want) for o in kept)
     graphed.close()
     assert not graphed._host_refs and graphed._host_out is None
+
+
+def test_the_graph_keeps_to_the_static_buffers():
+    """``.graph`` replayed by its holder after a call on the caller's buffers: static inputs in, ``.out`` out, and nothing is
+    written to what that call was given."""
+    graphed, reference = _make(16)
+    graph = graphed.graph
+    (x, lg), (x2, lg2) = _inputs(9, 1), _inputs(5, 2)
+    into = torch.empty(9, CFG.hidden_size, dtype=torch.bfloat16, device="cuda")
+    graphed(x, lg, into)
+    into.fill_(7.0)
+    graphed.load(x2, lg2)
+    graph.replay()
+    assert torch.equal(graphed.out[:5], reference(x2, lg2)) and (into == 7.0).all()
+    assert torch.equal(graphed(x, lg), reference(x, lg))
+    graph.replay()
+    assert torch.equal(graphed.out[:5], reference(x2, lg2))
+    graphed.capture()  # again: the earlier executable graph goes
+    assert torch.equal(graphed(x, lg, into), reference(x, lg))
+    graphed.close()
+
+
+def test_refused_inside_another_capture():
+    """A replay cannot be captured; the refusal leaves the layer as it was."""
+    graphed, reference = _make(16)
+    x, lg = _inputs(9, 1)
+    block = graphed.new_pinned_inputs()
+    block.set_rows(9)
+    out = torch.zeros(9, CFG.hidden_size, dtype=torch.bfloat16, device="cuda")
+    for call in (lambda: graphed(x, lg), lambda: graphed(x, lg, out), lambda: graphed.step(block, out), graphed.replay):
+        with pytest.raises(RuntimeError, match="captur"):
+            with torch.cuda.graph(torch.cuda.CUDAGraph()):
+                call()
+        assert torch.equal(graphed(x, lg, out), reference(x, lg))
+    graphed.close()
