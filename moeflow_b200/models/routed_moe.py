@@ -35,7 +35,18 @@ import torch.distributed as dist
 
 from ..fixed import FixedEPLayer
 
-#: Up to this many rows of pinned output are written by the combine kernel itself; beyond it the copy engine moves them.
+#: Pinned output of 8 to 128 rows is written by the forward's last kernel itself, anything else by the copy engine.  us per
+#: step on 72 bf16 experts, direct / copied:
+#:
+#:     rows                             1      2      4      8     16     24     32     64    128
+#:     queued, the same output     98/ 98 126/130 191/192 247/257 345/356 400/412 414/419 456/457 480/486
+#:     queued, new outputs         97/ 98 129/131 191/192 247/255 350/356 406/409 419/422 456/465 484/488
+#:     waited for, same output    111/101 140/138 205/203 261/263 360/362 414/416 424/427 460/468 488/496
+#:     waited for, new outputs    115/101 143/138 207/203 266/262 366/359 422/411 430/428 466/469 488/501
+#:
+#: Below 8 rows a step that is waited for loses what the pointer checks and the update of the graph's last node cost in front
+#: of the launch; from 8 rows on only a new output in every step that is waited for does, up to 32 rows.
+MIN_HOST_ROWS = 8
 MAX_HOST_ROWS = 128
 
 
@@ -170,7 +181,7 @@ class GraphedMoELayer:
 
     def _writable(self, out: torch.Tensor | None, rows: int, shape_ok) -> bool:
         return (out is not None and out.dtype == torch.bfloat16 and out.is_contiguous() and out.data_ptr() % 16 == 0
-                and shape_ok and (out.device == self.x.device or (out.device.type == "cpu" and rows <= MAX_HOST_ROWS and out.is_pinned())))
+                and shape_ok and (out.device == self.x.device or (out.device.type == "cpu" and MIN_HOST_ROWS <= rows <= MAX_HOST_ROWS and out.is_pinned())))
 
     def _hold(self, out: torch.Tensor | None) -> None:
         """Keep a pinned output alive until the replays that write it are done (its allocator does not know of them)."""
@@ -229,9 +240,9 @@ class GraphedMoELayer:
         self._block.copy_(inputs.raw, non_blocking=True)
         if (self._nodes is not None and t > 0 and not torch.cuda.is_current_stream_capturing() and
                 self._writable(out, t, out is not None and out.dim() == 2 and out.shape[0] >= t and out.shape[1] == self.layer.H)):
-            if not out.is_cuda:
-                self._hold(out)
             self._launch(self.x.data_ptr(), self.logits.data_ptr(), t, out.data_ptr())
+            if not out.is_cuda:
+                self._hold(out)  # behind the launch: with a new output its event takes about as long as that
             return out
         res = self.replay()[:t]
         if out is not None:

@@ -81,23 +81,26 @@ def test_pinned_blocks(capacity):
 
 
 def test_pinned_outputs_that_the_caller_drops():
-    """A new pinned output per step, the earlier ones dropped at once: each is held until its replay is done."""
+    """A pinned output dropped while its replay is still queued is held until that is done: pinned memory allocated in the
+    meantime is not the same."""
     graphed, reference = _make(16)
-    block, kept = graphed.new_pinned_inputs(), []
+    block = graphed.new_pinned_inputs()
     x, lg = _inputs(16, 3)
     want = reference(x, lg).cpu()
     block.x.copy_(x)
     block.logits.copy_(lg)
     block.set_rows(16)
-    torch.cuda.synchronize()
-    for i in range(40):
-        out = torch.zeros(16, CFG.hidden_size, dtype=torch.bfloat16).pin_memory()
-        graphed.step(block, out)
-        if i % 8 == 0:
-            kept.append(out)
-        del out
-    torch.cuda.synchronize()
-    assert all(torch.equal(o, want) for o in kept)
+    for _ in range(5):
+        torch.cuda.synchronize()
+        torch.cuda._sleep(50_000_000)
+        dropped = torch.zeros(16, CFG.hidden_size, dtype=torch.bfloat16).pin_memory()
+        graphed.step(block, dropped)
+        del dropped
+        later = [torch.full((16, CFG.hidden_size), 7.0, dtype=torch.bfloat16).pin_memory() for _ in range(3)]
+        kept = torch.zeros(16, CFG.hidden_size, dtype=torch.bfloat16).pin_memory()
+        graphed.step(block, kept)
+        torch.cuda.synchronize()
+        assert torch.equal(kept, want) and all((t == 7.0).all() for t in later)
     graphed.close()
     assert not graphed._host_refs and graphed._host_out is None
 
