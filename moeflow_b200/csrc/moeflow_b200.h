@@ -183,7 +183,8 @@ int mf_gemm_down_static_scratch(const void* tmap, const mf_gemm_args* args, int 
 int mf_router_topk(const float* logits, const float* bias, float* weights, int* ids, int tokens, int experts,
                    int top_k, int n_group, int topk_group, int sigmoid, int renorm, float scale,
                    mf_stream_t stream);
-// sum = x + add (rounded to bf16), out = rmsnorm(sum).
+// sum = x + add (rounded to bf16), out = rmsnorm(sum).  hidden: a multiple of 8; all pointers 16-byte aligned (as for
+// mf_rmsnorm).
 int mf_add_rmsnorm(const void* x, const void* add, const void* gamma, void* sum, void* out, int rows, int hidden, float eps,
                    mf_stream_t stream);
 // Row *pos of the caches [B, kv_heads, S, head_dim] (bf16) from the keys and values of this step, each [B, kv_heads *

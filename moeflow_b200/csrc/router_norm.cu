@@ -132,6 +132,7 @@ int mf_router_topk(const float* logits, const float* bias, float* weights, int* 
 int mf_rmsnorm(const void* x, const void* gamma, void* out, int rows, int hidden, float eps, mf_stream_t stream) {
   if (rows == 0) return 0;
   if (hidden % 8 != 0) return -1;
+  if ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(gamma) | reinterpret_cast<uintptr_t>(out)) & 15) return -2;
   return (int)mf::launch_kernel(mf::rmsnorm_kernel<false>, dim3(rows), dim3(256), 0, static_cast<cudaStream_t>(stream), true,
                                 static_cast<const __nv_bfloat16*>(x), static_cast<const __nv_bfloat16*>(nullptr),
                                 static_cast<const __nv_bfloat16*>(gamma), static_cast<__nv_bfloat16*>(nullptr),
@@ -142,6 +143,9 @@ int mf_add_rmsnorm(const void* x, const void* add, const void* gamma, void* sum,
                    mf_stream_t stream) {
   if (rows == 0) return 0;
   if (hidden % 8 != 0 || !add || !sum) return -1;
+  if ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(add) | reinterpret_cast<uintptr_t>(gamma) |
+       reinterpret_cast<uintptr_t>(sum) | reinterpret_cast<uintptr_t>(out)) & 15)
+    return -2;
   return (int)mf::launch_kernel(mf::rmsnorm_kernel<true>, dim3(rows), dim3(256), 0, static_cast<cudaStream_t>(stream), true,
                                 static_cast<const __nv_bfloat16*>(x), static_cast<const __nv_bfloat16*>(add),
                                 static_cast<const __nv_bfloat16*>(gamma), static_cast<__nv_bfloat16*>(sum),

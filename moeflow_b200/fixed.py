@@ -817,8 +817,10 @@ class FixedEPLayer:
         and the weights bound now, so the launch may build the metadata (and quantise the rows) as well."""
         from .ops import _lib
 
-        if x.dtype != torch.bfloat16 or not x.is_contiguous():
-            raise ValueError("x must be contiguous bf16")
+        if x.dtype != torch.bfloat16 or not x.is_contiguous() or x.data_ptr() % 16:
+            raise ValueError("x must be contiguous bf16, 16-byte aligned")
+        if not all(t is None or t.is_cuda for t in (x, weights, ids, num_valid, logits, bias)):
+            raise ValueError("the kernels read device tensors only")
         a = self._a_dispatch
         if logits is not None:
             if logits.dtype != torch.float32 or not logits.is_contiguous() or logits.shape[1] != self.cfg.n_routed_experts:

@@ -45,3 +45,27 @@ def test_two_residuals(tokens):
     project = DenseProjection(w)
     plain = project(x, torch.empty(tokens, 256, dtype=torch.bfloat16, device="cuda"))
     assert torch.equal(project(x, torch.empty_like(a), a, b), (a + b) + plain)
+
+
+def test_rows_off_the_16_byte_grid_and_host_tensors_are_refused():
+    """The kernels read 16 bytes at a time from raw device pointers."""
+    from conftest import SMALL_GPU
+    from moeflow_b200.fixed import FixedEPLayer
+    from moeflow_b200.ops.kernels import add_rmsnorm, rmsnorm
+    from moeflow_b200.testing import make_logits, make_weights
+
+    H = SMALL_GPU.hidden_size
+    off = torch.zeros(2 * H + 1, dtype=torch.bfloat16, device="cuda")[1:].view(2, H)
+    fine, gamma = torch.zeros(2, H, dtype=torch.bfloat16, device="cuda"), torch.ones(H, dtype=torch.bfloat16, device="cuda")
+    for call in (lambda: rmsnorm(off, gamma), lambda: rmsnorm(fine, off[0]), lambda: rmsnorm(fine, gamma, out=off),
+                 lambda: add_rmsnorm(off, fine, gamma), lambda: add_rmsnorm(fine, off, gamma), lambda: add_rmsnorm(fine, fine, off[0])):
+        with pytest.raises(RuntimeError):
+            call()
+    layer = FixedEPLayer(SMALL_GPU, 0, 1, *make_weights(SMALL_GPU, 0, device="cuda"), capacity=2, backend="cuda")
+    lg = make_logits(2, SMALL_GPU, 1, device="cuda")
+    bias = torch.zeros(SMALL_GPU.n_routed_experts)
+    for args in ((off, lg, None), (fine.cpu(), lg, None), (fine, lg.cpu(), None), (fine, lg, bias),
+                 (fine, lg, None, torch.tensor(1, dtype=torch.int32))):
+        with pytest.raises(ValueError):
+            layer.forward(*args)
+    assert not layer.forward(fine, lg, bias.cuda()).any() and layer.check_status()["code"] == 0
