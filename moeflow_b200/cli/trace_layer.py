@@ -6,9 +6,11 @@ Every kernel of the forward takes an optional trace buffer: the two grouped GEMM
 (entry, dependencies met, first weight tile requested, first operand stage complete, first accumulator
 complete, last epilogue done, exit, and for the first unit: epilogue done, first 16-column group loaded from
 tensor memory, first group stored, all groups stored), the transport kernels stamp CTA 0 (dispatch: entry, routed, rows stored,
-fenced, arrivals sent, last CTA done; metadata: entry, dispatch complete, flags seen, histogram, plan written,
-entries placed; reduce + push: entry, GEMM complete, row stored, fenced, -, last CTA done; combine: entry,
-predecessor complete, return flags seen, row written).  The layer is captured in a CUDA graph, replayed with a
+fenced, arrivals sent, last CTA done; metadata: entry, dispatch complete, flags seen, loads issued, warp 0's histogram, histogram,
+plan written, entries placed; reduce + push: entry, GEMM complete, row stored, fenced, -, last CTA done; combine: entry,
+predecessor complete, return flags seen, row written).  On one rank the dispatch launch builds the metadata at decode
+sizes (its last CTA then stamps the metadata phases) and the reduce writes the output: nothing is fenced or sent, and no
+combine is launched.  The layer is captured in a CUDA graph, replayed with a
 cold L2, and the stamps are printed in microseconds relative to the first one, so the gaps between kernels
 (launch chain, grid dependencies, fences) can be read directly.  One GPU; ``--experts`` sets the local expert
 count so that a rank's share of a larger EP group can be reproduced.
@@ -31,10 +33,23 @@ GEMM_EVENTS = ("entry", "deps met", "first weight tile", "first stage full", "fi
 SMALL_EVENTS = {
     "dispatch": ("entry", "routed", "rows stored", "fenced", "arrivals sent", "last CTA done"),
     "metadata": ("entry", "dispatch complete", "flags seen", "histogram", "plan written", "entries placed",
-                 "counters cleared", "warp 0 histogram"),
+                 "loads issued", "warp 0 histogram"),
     "reduce+push": ("entry", "GEMM complete", "row stored", "fenced", "-", "last CTA done"),
     "combine": ("entry", "predecessor complete", "flags seen", "row written"),
 }
+
+
+def attach_traces(layer: FixedEPLayer) -> dict[str, torch.Tensor]:
+    """Trace buffers for every kernel a forward of this layer may launch, by name."""
+    dev = layer.device
+    traces = {name: torch.zeros(8, dtype=torch.int64, device=dev) for name in SMALL_EVENTS}
+    traces.update({name: torch.zeros(layer.n_sms, 16, dtype=torch.int64, device=dev) for name in ("gate/up GEMM", "down GEMM")})
+    layer._a_gemm1.trace, layer._a_gemm2.trace = traces["gate/up GEMM"].data_ptr(), traces["down GEMM"].data_ptr()
+    layer._a_dispatch.trace, layer._a_meta.trace = traces["dispatch"].data_ptr(), traces["metadata"].data_ptr()
+    for args in (layer._a_reduce, layer._a_reduce_out):  # across ranks, and the one that writes the output
+        args.trace = traces["reduce+push"].data_ptr()
+    layer._a_combine.trace = traces["combine"].data_ptr()
+    return traces
 
 
 def main() -> None:
@@ -57,13 +72,7 @@ def main() -> None:
     bias = make_bias(cfg, 1, device=dev)
     extra = {k: int(v) for k, v in (kv.split("=") for kv in args.gemm_kwargs.split(",") if kv)}
     layer = FixedEPLayer(cfg, 0, 1, w13, w2, capacity=T, backend="cuda", gemm_kwargs={"fuse_return": bool(args.fuse_return), **extra})
-    n_sms = layer.n_sms
-    tr_g1 = torch.zeros(n_sms, 16, dtype=torch.int64, device=dev)
-    tr_g2 = torch.zeros_like(tr_g1)
-    small = {name: torch.zeros(8, dtype=torch.int64, device=dev) for name in SMALL_EVENTS}
-    layer._a_gemm1.trace, layer._a_gemm2.trace = tr_g1.data_ptr(), tr_g2.data_ptr()
-    layer._a_dispatch.trace, layer._a_meta.trace = small["dispatch"].data_ptr(), small["metadata"].data_ptr()
-    layer._a_reduce.trace, layer._a_combine.trace = small["reduce+push"].data_ptr(), small["combine"].data_ptr()
+    traces = attach_traces(layer)
     x = make_hidden(T, cfg, 3, device=dev)
     lg = make_logits(T, cfg, 4, device=dev)
     flush = L2Flush(device=dev)  # write pass, then a read pass: cold cache, no write-back pending
@@ -75,7 +84,7 @@ def main() -> None:
         layer.forward(x, lg, bias)
     for _ in range(args.reps):
         flush()
-        for t in (tr_g1, tr_g2, *small.values()):
+        for t in traces.values():
             t.zero_()
         torch.cuda.synchronize()
         s, e = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
@@ -86,17 +95,19 @@ def main() -> None:
     st = layer.check_status()
     print(f"tokens {T}, local experts {E}, plan {layer.plan.tolist()[:6]}, meta CTAs {layer.meta_ctas}, "
           f"status {st['name']}, event time {s.elapsed_time(e) * 1e3:.1f} us")
-    stamps = [t[t > 0] for t in (tr_g1, tr_g2, *small.values())]
+    stamps = [t[t > 0] for t in traces.values()]
     base = min(float(t.min()) for t in stamps if t.numel())
 
     def us(v) -> float:
         return (float(v) - base) / 1e3
 
     for name, events in SMALL_EVENTS.items():
-        t = small[name].cpu()
-        row = "  ".join(f"{ev} {us(t[i]):.2f}" for i, ev in enumerate(events) if ev != "-" and int(t[i]) > 0)
-        print(f"{name:12s} {row}")
-    for name, t in (("gate/up GEMM", tr_g1.cpu().double()), ("down GEMM", tr_g2.cpu().double())):
+        t = traces[name].cpu()
+        seen = sorted((int(t[i]), ev) for i, ev in enumerate(events) if ev != "-" and int(t[i]) > 0)
+        row = "  ".join(f"{ev} {us(at):.2f}" for at, ev in seen)
+        print(f"{name:12s} {row or 'not launched'}")
+    for name in ("gate/up GEMM", "down GEMM"):
+        t = traces[name].cpu().double()
         print(name)
         for i, ev in enumerate(GEMM_EVENTS):
             col = t[:, i]
