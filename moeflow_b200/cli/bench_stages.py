@@ -6,6 +6,11 @@
 For every capacity T the layer is captured up to each stage (``forward(stop_after=...)``); the time of a
 stage is the difference between consecutive prefixes (max over ranks, median over repetitions).  The
 padding cost of the fixed layout is the full-layer time with one valid row versus T valid rows.
+
+On one rank the prefixes are not nested launches: at decode sizes META (and every longer prefix) runs dispatch and metadata
+in one launch, so META is what that launch takes more than dispatch alone, and COMBINE is the difference between the
+owner reduce that writes the output and the one of the EXPERT prefix, which stores return rows (no merge follows it;
+the figure may be negative).
 Counterpart of ``scripts/bench_stages.py:30-93``.
 """
 
@@ -37,7 +42,8 @@ def _weights(cfg: MoEConfig, rank: int, world: int, dev):
 
 
 def main() -> None:
-    ap = argparse.ArgumentParser()
+    ap = argparse.ArgumentParser(description="Stage times as differences of CUDA-graph prefixes.  One rank: META and COMBINE "
+                                             "compare two forms of a launch (see the module's text).")
     ap.add_argument("--tokens", default="1,8,128")
     ap.add_argument("--dist", default="uniform")
     ap.add_argument("--reps", type=int, default=10)
