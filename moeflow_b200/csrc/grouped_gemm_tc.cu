@@ -172,19 +172,16 @@ __device__ __forceinline__ void return_finish(const mf_gemm_args& a, int complet
   }
 }
 
-// One output element: bf16 (one rounding of the fp32 value), or fp32 as it is when the caller asked for it
-// (router logits from the down-projection kernel).
 // Last step of the epilogue for C token columns of one weight row: the activation (gate/up), or the routing
 // weight (down), then the stores.  The arithmetic of all C columns comes first and has no branch that depends on
 // the column, so that the C dependency chains (exp, reciprocal) overlap: the epilogue warps are alone on their
 // scheduler and a column-by-column loop ran at one chain's latency (about 300 cycles per column).
 // v: first accumulator (gate, or the only one); w: second accumulator (up; with two_blocks the second weight block).
-// With a staging buffer (`stage`, 1 KB of shared memory owned by the calling warp; C == 16; 16-bit outputs, all
-// columns stored) the 16 x 32 block is transposed through it, and every lane stores 16 bytes (8 weight rows of one
+// With a staging buffer (`stage`, 1 KB of shared memory owned by the calling warp; C == 16) the 16 x 32 block is transposed through it, and every lane stores 16 bytes (8 weight rows of one
 // token): two store instructions per block instead of sixteen 64-byte ones.
 template <bool kTwoAcc, int C>
 __device__ __forceinline__ void finish_store(const mf_gemm_args& a, float (&v)[C], float (&w)[C], const float (&sc)[C],
-                                             int n0, int n_rows, int row_start, long long out_col, bool col_ok,
+                                             int n0, int n_rows, int row_start, long long out_col,
                                              uint8_t* stage = nullptr, int lane = 0) {
   if (kTwoAcc && !a.two_blocks) {
     if (a.round_h) {
@@ -204,7 +201,7 @@ __device__ __forceinline__ void finish_store(const mf_gemm_args& a, float (&v)[C
     }
   }
   const bool second = kTwoAcc && a.two_blocks;  // the other weight block's outputs, 128 columns further
-  if (C == 16 && stage != nullptr && !a.out_fp32 && a.out_cols <= 0 && (a.out_pitch & 7) == 0 &&
+  if (C == 16 && stage != nullptr && (a.out_pitch & 7) == 0 &&
       (reinterpret_cast<uintptr_t>(a.out) & 15) == 0) {  // 16-byte stores need rows that start on 16 bytes
     __nv_bfloat16* st = reinterpret_cast<__nv_bfloat16*>(stage);
     __nv_bfloat16* out = static_cast<__nv_bfloat16*>(a.out) + (long long)(row_start + n0) * a.out_pitch + (out_col - lane) +
@@ -228,24 +225,12 @@ __device__ __forceinline__ void finish_store(const mf_gemm_args& a, float (&v)[C
     return;
   }
   const bool all = n0 + C <= n_rows;
-  const long long first = (long long)(row_start + n0) * a.out_pitch + out_col;
-  if (a.out_fp32) {
-    float* p = static_cast<float*>(a.out) + first;
+  __nv_bfloat16* p = static_cast<__nv_bfloat16*>(a.out) + (long long)(row_start + n0) * a.out_pitch + out_col;
 #pragma unroll
-    for (int j = 0; j < C; ++j) {
-      if (all || n0 + j < n_rows) {
-        if (col_ok) p[(long long)j * a.out_pitch] = v[j];
-        if (second) p[(long long)j * a.out_pitch + kBlockM] = w[j];
-      }
-    }
-  } else {
-    __nv_bfloat16* p = static_cast<__nv_bfloat16*>(a.out) + first;
-#pragma unroll
-    for (int j = 0; j < C; ++j) {
-      if (all || n0 + j < n_rows) {
-        if (col_ok) p[(long long)j * a.out_pitch] = __float2bfloat16_rn(v[j]);
-        if (second) p[(long long)j * a.out_pitch + kBlockM] = __float2bfloat16_rn(w[j]);
-      }
+  for (int j = 0; j < C; ++j) {
+    if (all || n0 + j < n_rows) {
+      p[(long long)j * a.out_pitch] = __float2bfloat16_rn(v[j]);
+      if (second) p[(long long)j * a.out_pitch + kBlockM] = __float2bfloat16_rn(w[j]);
     }
   }
 }
@@ -660,7 +645,6 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
       const uint32_t taddr = tmem_base + ((uint32_t)(wq * 32) << 16) + (wide ? 0 : acc.stage * Cfg::kStageCols);
       const uint32_t tup = taddr + (Cfg::kWide && !wide ? 128 : N_MAX);
       const long long out_col = (long long)mb * (a.two_blocks ? 2 * kBlockM : kBlockM) + row;
-      const bool col_ok = a.out_cols <= 0 || out_col < a.out_cols;  // weight rows padded up to a block are not stored
 
       const bool scaled = a.row_scale != nullptr && (!kGateUp || a.two_blocks);
       // this warp group's share of the token columns (whole 16-column groups)
@@ -693,7 +677,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
             w[j] = kGateUp ? __uint_as_float(up[j]) : 0.f;
             sc[j] = scaled ? __shfl_sync(0xffffffffu, s_cur, j) : 1.f;
           }
-          finish_store<kGateUp, 16>(a, v, w, sc, c0, n_rows, row_start, out_col, col_ok, out_stage + (warp - 4) * kOutStageBytes, lane);
+          finish_store<kGateUp, 16>(a, v, w, sc, c0, n_rows, row_start, out_col, out_stage + (warp - 4) * kOutStageBytes, lane);
           if (warp == 4 && lane == 0) MF_STAMP_ONCE(9);
         }
         if (warp == 4 && lane == 0) MF_STAMP_ONCE(10);
@@ -767,7 +751,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
             float sc[kFix];
 #pragma unroll
             for (int j = 0; j < kFix; ++j) sc[j] = (scaled && n0 + j < n_rows) ? __ldcg(a.row_scale + row_start + n0 + j) : 1.f;
-            finish_store<kGateUp, kFix>(a, v, w, sc, n0, n_rows, row_start, out_col, col_ok);
+            finish_store<kGateUp, kFix>(a, v, w, sc, n0, n_rows, row_start, out_col);
           }
           if (lane == 0) a.counters[counter_ix] = 0;
           if (a.tile_done != nullptr) {
@@ -873,7 +857,6 @@ static int check_args(const mf_gemm_args* a, int n_max, int grid) {
   if ((a->b_pitch & 15) != 0 || (reinterpret_cast<uintptr_t>(a->b_base) & 15) != 0) return -4;
   if (a->b_box_rows < 0 || (a->b_box_rows > 0 && (a->b_box_rows % 16 != 0 || n_max % a->b_box_rows != 0))) return -8;
   if (a->b_tmap != nullptr && a->b_index != nullptr) return -5;  // TMA token tiles need contiguous rows
-  if (a->ret_peer != nullptr && (a->out_fp32 || a->out_cols > 0)) return -6;  // the fused return path reads bf16 rows of full width
   return 0;
 }
 
@@ -940,7 +923,7 @@ int mf_gemm_down(const void* tmap, const mf_gemm_args* args, int n_max, int grid
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   if (args->two_blocks) {
     // two adjacent weight blocks per unit: the kernel form with two operand tiles and two accumulators
-    if (args->ret_peer != nullptr || args->out_cols > 0 || args->up_row_offset != mf::kBlockM) return -7;
+    if (args->ret_peer != nullptr || args->up_row_offset != mf::kBlockM) return -7;
     if (n_max == 32) return mf::launch<true, 32>(tmap, args, grid, s);
     if (n_max == 64) return mf::launch<true, 64>(tmap, args, grid, s);
     if (n_max == 128) return mf::launch<true, 128>(tmap, args, grid, s);

@@ -78,8 +78,6 @@ typedef struct {
   long long partial_floats;  // floats in `partial`
   int n_counters;            // ints in `counters`
   int max_tiles;             // entries in tile_e / tile_s / tile_n
-  int out_fp32;              // bf16 kernels: 1 = `out` is fp32 [entries, out_pitch] (no rounding); not with ret_peer
-  int out_cols;              // bf16 kernels: > 0 = only output columns below this are stored (weight rows padded to 128)
   // Tile-level hand-over from the gate/up GEMM to the down GEMM (bf16 kernels, both optional).  The gate/up
   // kernel adds one to tile_done[tile] whenever a 32-row quarter of one of the tile's units has its final
   // activations stored; the down kernel, given the same array as tile_wait, fetches a tile's activations as

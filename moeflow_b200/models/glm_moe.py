@@ -50,10 +50,11 @@ def _rmsnorm(x: torch.Tensor, gamma: torch.Tensor, eps: float) -> torch.Tensor:
 
 
 class SharedExpert:
-    """Dense SwiGLU MLP ``w2 . swiglu(w13 . x)`` for up to ``capacity`` rows per call."""
+    """Dense SwiGLU MLP ``w2 . swiglu(w13 . x)`` for up to ``capacity`` rows per call.  ``block_m`` is accepted for older
+    call sites and selects nothing."""
 
     def __init__(self, w13: torch.Tensor, w2: torch.Tensor, capacity: int, limit: float | None, block_m: int = 64):
-        self.w13, self.w2, self.C, self.limit, self.block_m = w13.contiguous(), w2.contiguous(), capacity, limit, block_m
+        self.w13, self.w2, self.C, self.limit = w13.contiguous(), w2.contiguous(), capacity, limit
         self.inter, self.hidden = w2.shape[-1], w2.shape[-2]
         self.cuda = w13.is_cuda and w13.dtype == torch.bfloat16 and self.hidden % 128 == 0 and self.inter % 128 == 0
         if not self.cuda:
@@ -82,7 +83,7 @@ class SharedExpert:
 class RouterLogits:
     """Router logits ``h . gate_w^T`` as fp32 ``[T, E]`` on the dense projection kernel (tcgen05, bf16 operands, fp32
     accumulation and fp32 output): the gate matrix's rows are padded to a multiple of 128 and only the E real columns
-    are stored.  With it the MoE block issues no library GEMM."""
+    are stored.  With it the MoE block issues no library GEMM.  ``block_m`` as in ``SharedExpert``."""
 
     def __init__(self, gate_w: torch.Tensor, capacity: int, block_m: int = 64):
         from ..ops.dense import DenseProjection
@@ -91,7 +92,7 @@ class RouterLogits:
         dev = gate_w.device
         if H % 64:
             raise ValueError("hidden size must be a multiple of 64")
-        self.E, self.H, self.C, self.block_m = E, H, capacity, block_m
+        self.E, self.H, self.C = E, H, capacity
         self.w = torch.zeros((E + 127) // 128 * 128, H, dtype=torch.bfloat16, device=dev)
         self.w[:E] = gate_w.to(torch.bfloat16)
         self.logits = torch.zeros(capacity, E, dtype=torch.float32, device=dev)

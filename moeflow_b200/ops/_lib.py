@@ -74,8 +74,6 @@ class GemmArgs(C.Structure):
         ("partial_floats", C.c_longlong),
         ("n_counters", C.c_int),
         ("max_tiles", C.c_int),
-        ("out_fp32", C.c_int),
-        ("out_cols", C.c_int),
         ("tile_done", C.c_void_p),
         ("tile_wait", C.c_void_p),
         ("tile_wait_target", C.c_int),
