@@ -62,12 +62,12 @@ def test_fp32_output_stores_only_the_real_columns(cols):
     from moeflow_b200.ops.dense import DenseProjection
 
     x, w = _case(5, (cols + 127) // 128 * 128, 512, seed=2)
-    out = torch.zeros(5, cols, device="cuda")
-    guard = torch.zeros(64, device="cuda")
+    store = torch.full((6, cols + 160), 7.0, device="cuda")  # what a block of 128 columns would run over
+    out = store[:5, :cols]
     DenseProjection(w, out_cols=cols)(x, out)
     exact = x.double() @ w[:cols].double().t()
     slack = (x.double().abs() @ w[:cols].double().abs().t()) * (512 * 2.0**-24)
-    assert ((out.double() - exact).abs() <= slack).all() and not guard.any()
+    assert ((out.double() - exact).abs() <= slack).all() and (store[:5, cols:] == 7.0).all() and (store[5] == 7.0).all()
 
 
 @pytest.mark.parametrize("tokens", [1, 5])

@@ -41,8 +41,13 @@ def test_device_tensors_and_static_buffers_alternate(capacity):
         assert torch.equal(graphed(x, lg), want)
         into = torch.full((t, CFG.hidden_size), 7.0, dtype=torch.bfloat16, device="cuda")
         assert graphed(x, lg, into) is into and torch.equal(into, want)
-        # strided rows and wider dtypes take the copying path
-        assert torch.equal(graphed(x.float().bfloat16().repeat_interleave(2, 0)[::2], lg), want)
+        # strided rows, wider dtypes and rows off the 16-byte grid take the copying path
+        strided = torch.cat([x, x], dim=1)[:, : CFG.hidden_size]
+        off = torch.cat([x.new_zeros(1), x.flatten()])[1:].view_as(x)
+        for other in (strided, x.float(), off):
+            assert t == 1 or not graphed._readable(other, lg)
+            assert torch.equal(graphed(other, lg), want)
+        assert torch.equal(graphed(x, lg.double()), want) and torch.equal(graphed(x, torch.cat([lg, lg], dim=1)[:, : CFG.n_routed_experts]), want)
         pinned = torch.zeros(t, CFG.hidden_size, dtype=torch.bfloat16).pin_memory()
         graphed(x.cpu().pin_memory(), lg.cpu().pin_memory(), pinned)
         torch.cuda.synchronize()
