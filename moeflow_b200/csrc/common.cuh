@@ -232,7 +232,7 @@ __device__ __forceinline__ void tma_load_2d(void* smem_dst, const void* tmap, ui
       ::"r"(smem_u32(smem_dst)), "l"(reinterpret_cast<uint64_t>(tmap)), "r"(smem_u32(bar)), "r"(x), "r"(y), "l"(policy)
       : "memory");
 }
-// Policy for data that is read once: a weight stream of hundreds of MB otherwise sweeps everything else out of the L2,
+// Policy for a stream that is read once, or nearly so: a weight stream of hundreds of MB otherwise sweeps everything else out of the L2,
 // and every small kernel of the next forward starts with its instructions, tables and page-table entries in DRAM.
 __device__ __forceinline__ uint64_t l2_evict_first() {
   uint64_t p;

@@ -381,7 +381,11 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
     PipeState st;
     bool ok = true;
     SegFeed feed(work, ring, abort_flag, wait_ns);
-    // Tiles of up to 64 rows are decode: an expert has one tile and its weights are read once per forward.
+    // Tiles of up to 64 rows are decode: an expert usually has one tile, and its weights are then read once per forward.
+    // Skewed routing gives a hot expert several that read the same blocks, but they run close together and most blocks are
+    // still read once: evict-first / normal, us per layer, 1 token 81 / 96, 128 tokens 1325 / 1347 (bf16, 288 experts), 8
+    // tokens e4m3 220 / 241; zipf popularity: 100 tokens on 36 experts bf16 149 / 160, e4m3 113 / 126, 128 on 288 e4m3
+    // 116 / 129, 250 on 72 e4m3 (inter 2048) 223 / 230.
     const uint64_t policy = N_MAX <= 64 ? l2_evict_first() : l2_evict_normal();
     Seg sg;
     bool have = feed.first(sg);

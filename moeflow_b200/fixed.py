@@ -11,13 +11,16 @@ fp32 owner reduce, ascending-rank fp32 combine — with static shapes and no dev
 
 Two backends share this surface:
 
-``backend="cuda"`` (B200): five kernels per forward (six when the return push is not fused) and no library collective.  ``dispatch_push``
+``backend="cuda"`` (B200): six kernels per forward across ranks (seven where the metadata pass takes two launches, five when
+the return push is fused into the down GEMM), four on one rank at decode sizes, and no library collective.  ``dispatch_push``
 packs rows and stores them straight into the owners' ``recv`` buffers over peer memory, then publishes
 an epoch flag; ``expert_meta`` waits for the flags and builds expert offsets, the tile map and the
 K-split plan on the device; two tcgen05 grouped GEMMs (gate/up + SwiGLU, down + routing weight)
 stream the expert weights by TMA; ``owner_reduce_push`` sums each row's slots in order and stores the
 partial row straight into the source rank's ``ret_recv``; ``combine`` waits for the return flags and
-merges by ascending rank in fp32.
+merges by ascending rank in fp32.  On one rank dispatch and metadata share a launch at decode sizes, and the owner reduce
+writes the output.  e4m3 experts: the received rows are quantised in the metadata launch (or by a launch of their own), and
+layers with 256-row token tiles expand the experts to bf16 first.
 
 ``backend="torch"``: the same stages in plain PyTorch for any device and dtype, exchanging the static
 buffers with ``all_to_all_single`` (NCCL or gloo).  It is the CPU path and the twin the CUDA kernels are

@@ -190,7 +190,7 @@ class DecodeModel:
                  own_router_gemm: bool = True):
         """``fp8``: the routed experts are kept as block-scaled e4m3 (one fp32 scale per 128x128 block, quantised
         from the random bf16 weights) and run on the ``kind::f8f6f4`` grouped GEMMs.  ``own_router_gemm``: router
-        logits on the tcgen05 grouped kernel instead of a library matmul."""
+        logits on the tcgen05 dense projection kernel instead of a library matmul."""
         self.cfg, self.rank, self.world, self.batch, self.device = cfg, rank, world, batch, torch.device(device)
         self.acfg = acfg or AttentionConfig()
         dev, H, I, L = self.device, cfg.hidden_size, cfg.moe_intermediate_size, cfg.experts_per_rank(world)

@@ -1,7 +1,7 @@
 """Dense projections of a decode step on tcgen05 (``csrc/skinny_gemm.cu``): a weight matrix streamed past a few tokens.
 
-The reference leaves these to the serving engine; here they carry the shared expert, the router logits and the
-projections around attention of the decode model.
+The reference leaves these to the serving engine; here they carry the shared expert and the router logits of the decode
+model (the projections around its attention are library GEMMs).
 """
 
 from __future__ import annotations

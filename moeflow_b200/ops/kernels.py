@@ -116,8 +116,9 @@ def kv_append(k: torch.Tensor, v: torch.Tensor, k_cache: torch.Tensor, v_cache: 
 def make_tile_tmap(x: torch.Tensor, box_rows: int) -> C.Array:
     """128-byte TMA descriptor over a contiguous ``x [rows, K]`` with boxes of ``box_rows`` rows x 128 bytes.
 
-    Used for the token operand of the down GEMM (its rows are contiguous in expert-major order), with
-    ``box_rows`` equal to the kernel's token-tile width.  The buffer must outlive every launch that uses it.
+    Used for token operands whose rows are contiguous in expert-major order (boxes of up to 64 rows, as many as a tile holds;
+    the e4m3 kernels take boxes of a whole tile) and for the weights of dense projections.  The buffer must outlive every
+    launch that uses it.
     """
     _need_cuda(x, "token operand")
     if x.dim() != 2 or not x.is_contiguous():
