@@ -35,6 +35,8 @@ import torch.distributed as dist
 
 from ..fixed import FixedEPLayer
 
+_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)  # handle of a device's current stream
+
 #: Pinned output of 8 to 128 rows is written by the forward's last kernel itself, anything else by the copy engine.  us per
 #: step on 72 bf16 experts, direct / copied:
 #:
@@ -145,7 +147,8 @@ class GraphedMoELayer:
                 nodes[name] = (node, own[0], (C.c_void_p * len(own))(*(C.addressof(a) for a in own)), own)
             own_exec = C.c_void_p()
             _lib.check(_lib.lib().mf_graph_instantiate(graph.raw_cuda_graph(), _lib.stream_ptr(), C.byref(own_exec)), "graph instantiation")
-            self._set_args, self._exec = _lib.lib().mf_graph_set_args, own_exec.value
+            self._set_args, self._graph_launch, self._check = _lib.lib().mf_graph_set_args, _lib.lib().mf_graph_launch, _lib.check
+            self._exec, self._device_index = own_exec.value, self.x.device.index
             self._drop_exec = weakref.finalize(self, _lib.lib().mf_graph_destroy, own_exec.value)
             self._drop_exec.atexit = False  # the context goes first
             self._own_out = (self.layer.out.data_ptr(), 0)
@@ -156,21 +159,27 @@ class GraphedMoELayer:
 
     def _launch(self, x: int, logits: int, rows: int, out: int | None) -> None:
         """Replay on the caller's buffers (addresses; ``out`` None: all rows of the layer's own buffer)."""
-        from ..ops import _lib
+        first, last = (x, logits, rows), self._own_out if out is None else (out, rows)
+        if first != self._bound.get("first"):
+            self._update("first", first)
+        if last != self._bound.get("last"):
+            self._update("last", last)
+        # nothing else between here and the device: a call that is waited for pays for every line (4 us with the stream
+        # object and the module lookups)
+        code = self._graph_launch(self._exec, _raw_stream(self._device_index))
+        if code:
+            self._check(code, "graph launch")
 
-        for name, key in (("first", (x, logits, rows)), ("last", self._own_out if out is None else (out, rows))):
-            if self._bound.get(name) == key:
-                continue
-            node, a, arg_list, _ = self._nodes[name]
-            if name == "first":
-                a.x, a.logits, a.T = key
-                a.num_valid = None
-            else:
-                a.out, a.rows = key
-            self._bound.pop(name, None)  # unknown if the update fails
-            _lib.check(self._set_args(self._exec, node, arg_list), "graph update")
-            self._bound[name] = key
-        _lib.check(_lib.lib().mf_graph_launch(self._exec, _lib.stream_ptr()), "graph launch")
+    def _update(self, name: str, key: tuple) -> None:
+        node, a, arg_list, _ = self._nodes[name]
+        if name == "first":
+            a.x, a.logits, a.T = key
+            a.num_valid = None
+        else:
+            a.out, a.rows = key
+        self._bound.pop(name, None)  # unknown if the update fails
+        self._check(self._set_args(self._exec, node, arg_list), "graph update")
+        self._bound[name] = key
 
     def _readable(self, x: torch.Tensor, logits: torch.Tensor) -> bool:
         """Can the captured kernels read these tensors where they are?"""
@@ -211,6 +220,14 @@ class GraphedMoELayer:
         self.graph.replay()
         return self.out
 
+    def _replay_static(self, t: int) -> torch.Tensor:
+        """The first ``t`` rows of the static input buffers; on the calls' own executable graph, which is ready since the
+        capture."""
+        if self._nodes is None or t < 1 or torch.cuda.is_current_stream_capturing():
+            return self.replay()[:t]
+        self._launch(self.x.data_ptr(), self.logits.data_ptr(), t, None)
+        return self.out[:t]
+
     def __call__(self, x: torch.Tensor, logits: torch.Tensor, out: torch.Tensor | None = None) -> torch.Tensor:
         """One step.  With ``out`` (e.g. a pinned host tensor ``[T, H]``) the rows are copied there."""
         if self.graph is None:
@@ -224,7 +241,7 @@ class GraphedMoELayer:
             res = self.out[:t]
         else:
             t = self.load(x, logits)
-            res = self.replay()[:t]
+            res = self._replay_static(t)
         if out is not None:
             out.copy_(res, non_blocking=True)
             return out
@@ -244,7 +261,7 @@ class GraphedMoELayer:
             if not out.is_cuda:
                 self._hold(out)  # behind the launch: with a new output its event takes about as long as that
             return out
-        res = self.replay()[:t]
+        res = self._replay_static(t)
         if out is not None:
             out[:t].copy_(res, non_blocking=True)
             return out
