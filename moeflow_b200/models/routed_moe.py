@@ -37,18 +37,14 @@ from ..fixed import FixedEPLayer
 
 _raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)  # handle of a device's current stream
 
-#: Pinned output of 8 to 128 rows is written by the forward's last kernel itself, anything else by the copy engine.  us per
-#: step on 72 bf16 experts, direct / copied:
+#: Up to this many rows of pinned output are written by the forward's last kernel itself; beyond it the copy engine moves
+#: them (not measured there).  us per step on 72 bf16 experts, direct / copied, the two taken in turn call by call:
 #:
 #:     rows                             1      2      4      8     16     24     32     64    128
-#:     queued, the same output     98/ 98 126/130 191/192 247/257 345/356 400/412 414/419 456/457 480/486
-#:     queued, new outputs         97/ 98 129/131 191/192 247/255 350/356 406/409 419/422 456/465 484/488
-#:     waited for, same output    111/101 140/138 205/203 261/263 360/362 414/416 424/427 460/468 488/496
-#:     waited for, new outputs    115/101 143/138 207/203 266/262 366/359 422/411 430/428 466/469 488/501
-#:
-#: Below 8 rows a step that is waited for loses what the pointer checks and the update of the graph's last node cost in front
-#: of the launch; from 8 rows on only a new output in every step that is waited for does, up to 32 rows.
-MIN_HOST_ROWS = 8
+#:     queued, the same output     88/ 97 126/134 175/185 234/236 333/338 394/406 407/418 445/453 472/476
+#:     queued, new outputs         88/ 95 126/135 175/185 234/245 333/342 395/401 407/418 448/453 472/477
+#:     waited for, same output    102/111 134/140 182/188 236/241 342/346 402/407 421/429 457/460 496/502
+#:     waited for, new outputs    106/109 137/138 186/187 239/241 346/347 405/411 424/429 457/459 491/501
 MAX_HOST_ROWS = 128
 
 
@@ -190,7 +186,7 @@ class GraphedMoELayer:
 
     def _writable(self, out: torch.Tensor | None, rows: int, shape_ok) -> bool:
         return (out is not None and out.dtype == torch.bfloat16 and out.is_contiguous() and out.data_ptr() % 16 == 0
-                and shape_ok and (out.device == self.x.device or (out.device.type == "cpu" and MIN_HOST_ROWS <= rows <= MAX_HOST_ROWS and out.is_pinned())))
+                and shape_ok and (out.device == self.x.device or (out.device.type == "cpu" and rows <= MAX_HOST_ROWS and out.is_pinned())))
 
     def _hold(self, out: torch.Tensor | None) -> None:
         """Keep a pinned output alive until the replays that write it are done (its allocator does not know of them)."""
@@ -259,7 +255,7 @@ class GraphedMoELayer:
                 self._writable(out, t, out is not None and out.dim() == 2 and out.shape[0] >= t and out.shape[1] == self.layer.H)):
             self._launch(self.x.data_ptr(), self.logits.data_ptr(), t, out.data_ptr())
             if not out.is_cuda:
-                self._hold(out)  # behind the launch: with a new output its event takes about as long as that
+                self._hold(out)  # behind the launch: in front of it a new output cost a waited-for step 7 to 15 us more
             return out
         res = self._replay_static(t)
         if out is not None:
