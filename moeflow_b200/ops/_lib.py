@@ -324,7 +324,8 @@ def ptr(t) -> int | None:
 def stream_ptr() -> int:
     import torch
 
-    return torch.cuda.current_stream().cuda_stream
+    # the handle of torch.cuda.current_stream(), without its stream object
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
 
 
 def last_captured_node() -> int:

@@ -27,6 +27,7 @@ class DenseProjection:
         if k % 64 or self.outputs % block or w.dtype != torch.bfloat16:
             raise ValueError("bf16 weights with K a multiple of 64 and rows in whole blocks expected")
         self.w, self.k, self.gate_up = w.contiguous(), k, gate_up
+        self._device = w.device
         self._width = min(out_cols, self.outputs) if out_cols > 0 else self.outputs  # columns that are stored
         self.status = status if status is not None else torch.zeros(1, dtype=torch.int64, device=w.device)
         self.n_sms = sm_count(w.device.index or 0)
@@ -38,9 +39,9 @@ class DenseProjection:
 
     def _check(self, name: str, t: torch.Tensor, rows: int, dtypes: tuple) -> None:
         """The kernel takes raw pointers: what it indexes has to be there."""
-        if t.dtype not in dtypes or t.device != self.w.device:
+        if t.dtype not in dtypes or t.device != self._device:
             raise ValueError(f"{name} must be {' or '.join(str(d) for d in dtypes)} on the weights' device")
-        if t.dim() != 2 or t.shape[0] < rows or t.shape[1] < self._width or (self._width > 1 and t.stride(1) != 1):
+        if t.dim() != 2 or t.shape[0] < rows or t.shape[1] < self._width or (t.stride(1) != 1 and self._width > 1):
             raise ValueError(f"{name} must hold {rows} rows of {self._width} adjacent values")
 
     def __call__(self, x: torch.Tensor, out: torch.Tensor, residual: torch.Tensor | None = None,
@@ -63,8 +64,8 @@ class DenseProjection:
             raise ValueError("a residual is added to a bf16 product")
         if t == 0:
             return out[:0]
-        if x.device != self.w.device or x.dtype != torch.bfloat16:
-            x = x.to(self.w.device, torch.bfloat16)
+        if x.device != self._device or x.dtype != torch.bfloat16:
+            x = x.to(self._device, torch.bfloat16)
         if x.stride(1) != 1 or (t > 1 and (x.stride(0) < self.k or x.stride(0) % 8)) or x.data_ptr() % 16:
             x = x.clone(memory_format=torch.contiguous_format)
         a = self._args
