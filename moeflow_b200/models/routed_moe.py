@@ -19,9 +19,9 @@ strides) are copied into the static buffers ``.x`` / ``.logits`` / ``.num_valid`
 ``replay`` work on.  The small copies and the gap in front of the graph were 13 us of a device-fed call.  A pinned input
 block is still one copy: read by the first kernel itself over PCIe, 24 rows took 43 us, the copy engine needs 9.
 
-The calls on the caller's buffers launch an executable graph of their own.  ``.graph`` is the forward on the static
-buffers, whoever replays it and whatever was called before (it is instantiated by its first replay); ``.out`` holds the
-rows of ``replay`` and of the calls without ``out`` (a call with ``out`` may leave it as it was).
+All calls launch one executable graph of the layer's own.  ``.graph`` is the forward on the static buffers for a holder
+that replays it, whatever was called before (it is instantiated by its first replay); ``.out`` holds the rows
+of ``replay`` and of the calls without ``out`` (a call with ``out`` may leave it as it was).
 """
 
 from __future__ import annotations
@@ -148,14 +148,16 @@ class GraphedMoELayer:
             self._drop_exec = weakref.finalize(self, _lib.lib().mf_graph_destroy, own_exec.value)
             self._drop_exec.atexit = False  # the context goes first
             self._own_out = (self.layer.out.data_ptr(), 0)
-            self._bound = {"last": self._own_out}  # as captured
+            self._bound = {"first": (self.x.data_ptr(), self.logits.data_ptr(), self.layer.C, self.num_valid.data_ptr()),
+                           "last": self._own_out}  # as captured
         self.graph, self._nodes = graph, nodes
         torch.cuda.synchronize()
         return self
 
-    def _launch(self, x: int, logits: int, rows: int, out: int | None) -> None:
-        """Replay on the caller's buffers (addresses; ``out`` None: all rows of the layer's own buffer)."""
-        first, last = (x, logits, rows), self._own_out if out is None else (out, rows)
+    def _launch(self, x: int, logits: int, rows: int, out: int | None, num_valid: int | None = None) -> None:
+        """Replay on the caller's buffers (addresses; ``out`` None: all rows of the layer's own buffer; ``num_valid``: the
+        device word that says how many of ``rows`` are live, None: all)."""
+        first, last = (x, logits, rows, num_valid), self._own_out if out is None else (out, rows)
         if first != self._bound.get("first"):
             self._update("first", first)
         if last != self._bound.get("last"):
@@ -169,8 +171,7 @@ class GraphedMoELayer:
     def _update(self, name: str, key: tuple) -> None:
         node, a, arg_list, _ = self._nodes[name]
         if name == "first":
-            a.x, a.logits, a.T = key
-            a.num_valid = None
+            a.x, a.logits, a.T, a.num_valid = key
         else:
             a.out, a.rows = key
         self._bound.pop(name, None)  # unknown if the update fails
@@ -213,7 +214,10 @@ class GraphedMoELayer:
     def replay(self) -> torch.Tensor:
         if self.graph is None:
             self.capture()
-        self.graph.replay()
+        if self._nodes is None or torch.cuda.is_current_stream_capturing():
+            self.graph.replay()
+        else:  # one executable graph for all calls: replays on several streams follow one another
+            self._launch(self.x.data_ptr(), self.logits.data_ptr(), self.layer.C, None, self.num_valid.data_ptr())
         return self.out
 
     def _replay_static(self, t: int) -> torch.Tensor:

@@ -130,6 +130,28 @@ def test_the_graph_keeps_to_the_static_buffers():
     graphed.close()
 
 
+def test_calls_on_two_streams_follow_one_another():
+    """Nothing but the launch order separates them: they share the layer's buffers."""
+    graphed, reference = _make(64)
+    streams = [torch.cuda.Stream() for _ in range(2)]
+    cases = [_inputs(t, t) for t in (64, 7)]
+    want = [reference(*c) for c in cases]
+    graphed.load(*cases[1])
+    torch.cuda.synchronize()
+    for _ in range(20):
+        outs = [torch.zeros_like(w) for w in want]
+        torch.cuda.synchronize()
+        for c, out, stream in zip(cases, outs, streams):
+            with torch.cuda.stream(stream):
+                graphed(*c, out)
+        with torch.cuda.stream(streams[0]):
+            last = graphed.replay()
+        torch.cuda.synchronize()
+        assert all(torch.equal(out, w) for out, w in zip(outs, want)) and torch.equal(last[:7], want[1])
+    assert graphed.layer.check_status()["code"] == 0
+    graphed.close()
+
+
 def test_refused_inside_another_capture():
     """A replay cannot be captured; the refusal leaves the layer as it was."""
     graphed, reference = _make(16)
