@@ -157,7 +157,7 @@ __global__ void __launch_bounds__(kMetaThreads) expert_meta_kernel(const mf_meta
     int slots1 = a.max_split_slots, slots2 = a.max_split_slots;
     if (a.partial_floats > 0) {
       slots1 = (int)min((long long)0x7fffffff, a.partial_floats / (2ll * cols * 128));
-      slots2 = (int)min((long long)0x7fffffff, a.partial_floats / (1ll * cols * 128));
+      slots2 = (int)min((long long)0x7fffffff, a.partial_floats / ((a.pair2 ? 2ll : 1ll) * cols * 128));
     } else {
       cols = 0;  // fixed slots of the kernel's n_max columns
     }
@@ -449,7 +449,7 @@ __global__ void __launch_bounds__(kMetaThreads) expert_meta_place_kernel(const m
     int slots1 = a.max_split_slots, slots2 = a.max_split_slots;
     if (a.partial_floats > 0) {
       slots1 = (int)min((long long)0x7fffffff, a.partial_floats / (2ll * cols * 128));
-      slots2 = (int)min((long long)0x7fffffff, a.partial_floats / (1ll * cols * 128));
+      slots2 = (int)min((long long)0x7fffffff, a.partial_floats / ((a.pair2 ? 2ll : 1ll) * cols * 128));
     } else {
       cols = 0;
     }

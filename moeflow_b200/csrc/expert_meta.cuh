@@ -287,8 +287,8 @@ __device__ __forceinline__ void meta_one_pass(const mf_meta_args& a, int* sm, un
     if (cols < 16) cols = 16;
     const bool second = (lane & 4) != 0;
     int slots = a.max_split_slots;
-    if (a.partial_floats > 0)  // partial tiles of 256 * cols floats (gate and up), 128 * cols for the down GEMM
-      slots = (int)((unsigned)min((long long)0x7fffffff, a.partial_floats >> (second ? 7 : 8)) / (unsigned)cols);
+    if (a.partial_floats > 0)  // partial tiles of 256 * cols floats (two accumulators) or 128 * cols
+      slots = (int)((unsigned)min((long long)0x7fffffff, a.partial_floats >> (second && !a.pair2 ? 7 : 8)) / (unsigned)cols);
     const int cut = choose_cut_lanes(a, nt * (second ? a.m_blocks2 : a.m_blocks1), second ? a.k_blocks2 : a.k_blocks1, slots,
                                      second ? 8 : 4, cols, lane & 3);
     if (lane == 0) {

@@ -25,6 +25,8 @@
 //     are never stored, and the down GEMM starts a token tile as soon as the tile's units have reported (tile_done),
 //     as in the bf16 kernels, instead of waiting for the gate/up grid and for a quantiser launch behind it.
 //
+// Token tiles of 128 rows have a kernel of their own (grouped_gemm_fp8_wide.cu).
+//
 // Everything else (swap-AB, persistent CTAs, device-side plan, split-K with ordered fix-up, bounded
 // waits) is as in grouped_gemm_tc.cu.
 //
@@ -35,17 +37,15 @@
 #include <cstring>
 
 #include "common.cuh"
+#include "fp8_pipe.cuh"
 #include "moeflow_b200.h"
 #include "quant.cuh"
 #include "work_iter.cuh"
 
 namespace mf {
 
-constexpr int kF8BlockM = 128;
-constexpr int kF8TileA = 128 * 128;
 constexpr int kF8Gather = 32;  // one warp gathers, the other one fills the tables: 12 warps keep 168 registers each
 constexpr int kF8Tables = 2;   // scale tables: the unit being promoted and the prefetched next one
-constexpr int kF8MaxKb = 32;   // K <= 4096 (one unit never spans more K blocks than this)
 constexpr int kF8Stage = 1024;  // per promotion warp: 16 token columns x 32 outputs of the epilogue, transposed
 
 template <bool kGateUp, int N_MAX>
@@ -54,8 +54,7 @@ struct F8Cfg {
   static constexpr int kStageA = kATiles * kF8TileA;
   static constexpr int kStageB = N_MAX * 128;
   static constexpr int kStageBytes = kStageA + kStageB;
-  // Promotion warps: one group of four warps (one per tensor-memory lane quarter) takes N_MAX / kGroups token
-  // columns: 32 columns per group for tiles of up to 64 rows, 64 for 128-row tiles.
+  // Promotion warps: one group of four warps (one per tensor-memory lane quarter) per 32 token columns.
   static constexpr int kGroups = N_MAX > 32 ? 2 : 1;
   static constexpr int kCols = N_MAX / kGroups;
   static constexpr int kPromo = 4 * kGroups;             // promotion warps: 4 .. 4 + kPromo - 1
@@ -73,46 +72,6 @@ struct F8Cfg {
   static constexpr int kTmemCols = kTmpStages * kTmpCols;
   static constexpr int kSmemBytes = kStages * kStageBytes + kTableBytes + kExtra + 1024;
 };
-
-struct F8Pipe {
-  int stage = 0;
-  uint32_t phase = 0;
-  __device__ __forceinline__ void advance(int n) {
-    if (++stage == n) {
-      stage = 0;
-      phase ^= 1u;
-    }
-  }
-};
-
-// Two fp32 values in one 64-bit register: the promotion works on pairs of token columns (one instruction for two
-// multiply-adds, each rounded like fmaf).
-using f32x2 = unsigned long long;
-__device__ __forceinline__ f32x2 pack2(float lo, float hi) {
-  f32x2 r;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
-  return r;
-}
-__device__ __forceinline__ f32x2 pack2(uint32_t lo, uint32_t hi) {
-  f32x2 r;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "r"(lo), "r"(hi));
-  return r;
-}
-__device__ __forceinline__ float2 unpack2(f32x2 v) {
-  float2 r;
-  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
-  return r;
-}
-__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
-  f32x2 r;
-  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-  return r;
-}
-__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
-  f32x2 r;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-  return r;
-}
 
 template <bool kGateUp, int N_MAX>
 __global__ void __launch_bounds__(F8Cfg<kGateUp, N_MAX>::kThreads, 1)
@@ -598,7 +557,7 @@ grouped_gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid
       bool finish = true;
       if (sg.nseg > 1) {
         // The unit is cut along K: park the sums; the group that arrives last adds the segments in K order.
-        float* mine = a.partial + (long long)work.slot_of(sg, sg.seg) * slot_floats;
+        float* mine = a.partial + (long long)slot_of(sg, sg.seg) * slot_floats;
 #pragma unroll
         for (int c = 0; c < COLS; ++c) {
           const int n = col0 + c;
@@ -630,7 +589,7 @@ grouped_gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid
           }
           const f32x2 one = pack2(1.f, 1.f);
           for (int s_ = 0; s_ < sg.nseg; ++s_) {
-            const float* p = a.partial + (long long)work.slot_of(sg, s_) * slot_floats + row;
+            const float* p = a.partial + (long long)slot_of(sg, s_) * slot_floats + row;
 #pragma unroll
             for (int c0 = 0; c0 < COLS; c0 += 16) {
               if (col0 + c0 < n_rows) {
@@ -827,10 +786,15 @@ static int launch_f8(const void* tmap, const mf_gemm_args* args, int grid, cudaS
   return (int)launch_kernel(kern, dim3(grid), dim3(Cfg::kThreads), Cfg::kSmemBytes, stream, true, tm, tb, *args);
 }
 
+// 128-row tiles (grouped_gemm_fp8_wide.cu)
+int launch_fp8_wide(bool gate_up, const void* tmap, const mf_gemm_args* args, int grid, cudaStream_t stream);
+
 static int check_f8(const mf_gemm_args* a, int n_max, int grid) {
   if (!a || grid < 1) return -1;
   if (n_max != 32 && n_max != 64 && n_max != 128) return -2;
   if (a->b_tmap != nullptr && a->b_index != nullptr) return -6;  // TMA token tiles need contiguous rows
+  if (a->b_box_rows < 0 || (a->b_box_rows > 0 && (a->b_box_rows % 16 != 0 || n_max % a->b_box_rows != 0))) return -9;
+  if (n_max != 128 && a->b_box_rows > 0 && a->b_box_rows != n_max) return -8;
   if (a->m_blocks < 1 || a->k_blocks < 1 || a->k_blocks > kF8MaxKb) return -3;
   if ((a->b_pitch & 15) != 0 || (reinterpret_cast<uintptr_t>(a->b_base) & 15) != 0) return -4;
   if (!a->w_scale || !a->b_scale) return -5;
@@ -850,7 +814,7 @@ int mf_gemm_gate_up_fp8(const void* tmap, const mf_gemm_args* args, int n_max, i
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   if (n_max == 32) return mf::launch_f8<true, 32>(tmap, args, grid, s);
   if (n_max == 64) return mf::launch_f8<true, 64>(tmap, args, grid, s);
-  return mf::launch_f8<true, 128>(tmap, args, grid, s);
+  return mf::launch_fp8_wide(true, tmap, args, grid, s);
 }
 
 int mf_gemm_down_fp8(const void* tmap, const mf_gemm_args* args, int n_max, int grid, mf_stream_t stream) {
@@ -859,7 +823,8 @@ int mf_gemm_down_fp8(const void* tmap, const mf_gemm_args* args, int n_max, int 
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   if (n_max == 32) return mf::launch_f8<false, 32>(tmap, args, grid, s);
   if (n_max == 64) return mf::launch_f8<false, 64>(tmap, args, grid, s);
-  return mf::launch_f8<false, 128>(tmap, args, grid, s);
+  if (args->b_index != nullptr || (args->b_tmap == nullptr && args->b_rows < 1)) return -8;
+  return mf::launch_fp8_wide(false, tmap, args, grid, s);
 }
 
 int mf_quant_rows_1x128(const void* x, long long x_pitch, const int* row_index, int rows, int hidden, void* q,

@@ -700,7 +700,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
       } else {
         // The unit is cut along K: park the fp32 partial sums, then the last quarter-warp to arrive adds
         // the segments in K order.
-        float* mine = a.partial + (long long)work.slot_of(sg, sg.seg) * slot_floats;
+        float* mine = a.partial + (long long)slot_of(sg, sg.seg) * slot_floats;
         for (int c0 = c_begin; c0 < c_end; c0 += 16) {
           uint32_t g[16], up[16];
           tmem_ld_16(taddr + c0, g);
@@ -738,7 +738,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
 #pragma unroll
             for (int j = 0; j < kFix; ++j) v[j] = w[j] = 0.f;
             for (int s = 0; s < sg.nseg; ++s) {
-              const float* p = a.partial + (long long)work.slot_of(sg, s) * slot_floats;
+              const float* p = a.partial + (long long)slot_of(sg, s) * slot_floats;
               float pv[kFix], pw[kFix];
 #pragma unroll
               for (int j = 0; j < kFix; ++j) {

@@ -99,7 +99,8 @@ typedef struct {
   // Optional: a device counter, zero when the kernel starts.  Segments of a K split then go to the CTA that asks next
   // instead of round-robin (work_iter.cuh).
   int* sched;
-  int b_box_rows;            // bf16 kernels: rows of a box of b_tmap, 0 = n_max; a divisor of n_max and a multiple of 16
+  int b_box_rows;            // bf16 and 128-row e4m3 kernels: rows of a box of b_tmap, 0 = n_max; a divisor of n_max and a multiple of 16
+  long long b_rows;          // 128-row e4m3 down kernel without b_tmap: rows of b_base, for the map that the launch makes
 } mf_gemm_args;
 
 // Encode a 2-D tiled tensor map (K innermost) for a weight matrix [rows, k_elems]; box = 128 bytes x
@@ -247,7 +248,7 @@ typedef struct {
   int max_split_slots;       // unused when partial_floats > 0
   unsigned long long* status;
   unsigned long long wait_ns;
-  long long partial_floats;  // capacity of the split-K scratch in floats: bounds slots = floats / (tiles * cols * 128)
+  long long partial_floats;  // capacity of the split-K scratch in floats: bounds slots = floats / (accumulators of a unit * cols * 128)
   int* row_hits;             // optional [rows]: valid slots per received row (for the fused return path)
   // Multi-CTA variant (prefill sizes): with n_ctas > 1 the work is split over n_ctas CTAs in two chained
   // launches (count, then scan + place); cta_hist [n_ctas * L] and acc [2] are its scratch (acc zeroed once
@@ -267,6 +268,7 @@ typedef struct {
   uint8_t* xq;               // [rows, H] e4m3
   float* xs;                 // [rows, H / 128]
   int k_step;                // K blocks of 64 values per K step of the GEMMs the plan is for: 2 for the e4m3 kernels, else 1
+  int pair2;                 // 1: a unit of the down GEMM has two accumulators (m_blocks2 counts pairs of weight blocks)
 } mf_meta_args;
 int mf_expert_meta(const mf_meta_args* args, mf_stream_t stream);
 // Dispatch and metadata in one launch: the only rank is this GPU (R = 1), at most 512 experts and 4096 slot words.
@@ -333,7 +335,9 @@ int mf_permute_rows(const void* recv, long long pitch, const int* entry_row, con
 int mf_quant_rows_1x128(const void* x, long long x_pitch, const int* row_index, int rows, int hidden, void* q,
                         float* scales, long long valid_off, const int* n_rows_dev, mf_stream_t stream);
 // Block-scaled e4m3 variants of the grouped GEMMs (args->w_scale, b_scale, b_scale_pitch are required;
-// b_base rows are e4m3 bytes, k_blocks = K / 128, the tensor map is built with elem_bytes = 1; n_max 32 or 64).
+// b_base rows are e4m3 bytes, k_blocks = K / 128, the tensor map is built with elem_bytes = 1; n_max 32, 64 or 128).
+// With n_max = 128 a unit of the down GEMM covers two adjacent weight blocks whatever m_blocks says; that kernel reads
+// contiguous rows only (no b_index), through b_tmap or a map that the launch makes (b_rows).
 int mf_gemm_gate_up_fp8(const void* tmap, const mf_gemm_args* args, int n_max, int grid, mf_stream_t stream);
 int mf_gemm_down_fp8(const void* tmap, const mf_gemm_args* args, int n_max, int grid, mf_stream_t stream);
 

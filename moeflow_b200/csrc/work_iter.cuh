@@ -28,9 +28,16 @@ struct Seg {
   int e, row_start, n_rows;  // the token tile: expert, first entry, entries
   int kb0, nkb;
   int nseg, seg;             // segments of this unit and this one's index in K order (nseg == 1: whole unit)
-  int c_first;               // stream-K: CTA that holds segment 0 of the unit
-  int pad;
+  int c_first;               // stream-K: CTA that holds segment 0 of the unit; K split: -1
+  int late;                  // stream-K: 1 when that CTA's share begins before the unit
 };
+
+// Partial-sum slot of segment `sg` of the unit of `s`.  K split: slots are (unit, segment).  Stream-K: every CTA owns two
+// slots, one for the segment its share starts with and one for the segment it ends with.
+__device__ __forceinline__ int slot_of(const Seg& s, int sg) {
+  if (s.c_first < 0) return s.unit * s.nseg + sg;
+  return 2 * (s.c_first + sg) + (sg == 0 ? s.late : 0);
+}
 
 struct WorkIter {
   const mf_gemm_args* a;
@@ -77,6 +84,7 @@ struct WorkIter {
       s.c_first = cta_of(x0);
       s.nseg = cta_of(x0 + KB - 1) - s.c_first + 1;
       s.seg = cta - s.c_first;
+      s.late = share_begin(s.c_first) < x0 ? 1 : 0;
     } else {
       if (u >= units * split) return false;
       const int ks = u % split;
@@ -85,7 +93,8 @@ struct WorkIter {
       s.kb0 = ks * s.nkb;
       s.nseg = split;
       s.seg = ks;
-      s.c_first = 0;
+      s.c_first = -1;
+      s.late = 0;
     }
     s.tt = s.unit / m_blocks;
     s.mb = s.unit - s.tt * m_blocks;
@@ -109,13 +118,6 @@ struct WorkIter {
     if (!stream && a->sched != nullptr) u = G + __shfl_sync(0xffffffffu, u, 0);
   }
 
-  // Partial-sum slot of segment `sg` of the unit of `s`.  K split: slots are (unit, segment).  Stream-K: every
-  // CTA owns two slots, one for the segment its share starts with and one for the segment it ends with.
-  __device__ __forceinline__ int slot_of(const Seg& s, int sg) const {
-    if (!stream) return s.unit * split + sg;
-    const int c = s.c_first + sg;
-    return 2 * c + (share_begin(c) >= (long long)s.unit * KB ? 0 : 1);
-  }
   // Slots the plan needs (for the capacity check).
   __device__ __forceinline__ long long slots_needed() const {
     if (stream) return 2ll * G;
@@ -162,6 +164,7 @@ struct SegReader {
     s.nseg = z.x;
     s.seg = z.y;
     s.c_first = z.z;
+    s.late = z.w;
     __syncwarp();
     if (lane_id() == 0) mbar_arrive(&ring->empty[i]);
     if (++i == kSegRing) {
@@ -192,7 +195,7 @@ struct SegFeed {
       int4* p = reinterpret_cast<int4*>(&ring->slot[i]);
       p[0] = make_int4(have ? nx.unit : -1, nx.tt, nx.mb, nx.e);
       p[1] = make_int4(nx.row_start, nx.n_rows, nx.kb0, nx.nkb);
-      p[2] = make_int4(nx.nseg, nx.seg, nx.c_first, 0);
+      p[2] = make_int4(nx.nseg, nx.seg, nx.c_first, nx.late);
       mbar_arrive(&ring->full[i]);
     }
     __syncwarp();

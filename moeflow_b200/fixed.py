@@ -757,11 +757,13 @@ class FixedEPLayer:
                                 out=self.y.data_ptr(), out_pitch=H, row_scale=self.entry_w.data_ptr(), counters=g2.counters,
                                 n_counters=g2.n_counters, w_scale=None, b_scale=f["as"].data_ptr(), b_scale_pitch=I // 128,
                                 **common)
+        f["a2"].b_rows = max(N, self.block_m)
         if bool(self.gemm_kwargs.get("b_tma", True)):
             from .ops.kernels import make_tile_tmap
 
-            f["tm_aq"] = make_tile_tmap(f["aq"], self.block_m)  # the down GEMM reads its e4m3 token tiles by TMA
-            f["a2"].b_tmap = C.addressof(f["tm_aq"])
+            box = min(self.block_m, 64)  # as in the bf16 layers
+            f["tm_aq"] = make_tile_tmap(f["aq"], box)  # the down GEMM reads its e4m3 token tiles by TMA
+            f["a2"].b_tmap, f["a2"].b_box_rows = C.addressof(f["tm_aq"]), box
         a1.sched, f["a2"].sched = g1.sched, g2.sched
         if self.tile_handover:  # one count per promotion warp of the gate/up kernel and weight block
             a1.tile_done = self._tile_done.data_ptr()
@@ -786,6 +788,8 @@ class FixedEPLayer:
         f["tm13"], f["tm2"], f["pack"] = pack["tm13"], pack["tm2"], pack
         self._fp8 = f
         self._a_meta.k_step = 2  # the e4m3 kernels' K blocks hold 128 values: no split between two halves of one
+        if self.block_m == 128:  # their units of the down GEMM cover two weight blocks
+            self._a_meta.pair2, self._a_meta.m_blocks2 = 1, (self.H // 128 + 1) // 2
         if f["in_meta"]:
             self._a_meta.xq, self._a_meta.xs = f["xq"].data_ptr(), f["xs"].data_ptr()
         self.w13, self.w2 = pack["w13"], pack["w2"]
@@ -814,6 +818,7 @@ class FixedEPLayer:
         self._fp8 = self._expand = None
         self._a_meta.xq = self._a_meta.xs = None
         self._a_meta.k_step = 1
+        self._a_meta.pair2, self._a_meta.m_blocks2 = int(self.down_two_blocks), self._a_gemm2.m_blocks
 
     def _cuda_dispatch(self, x, weights, ids, num_valid, logits=None, bias=None, whole: bool = False) -> tuple[torch.Tensor, bool]:
         """``(hit, metadata built)``.  ``whole``: the caller goes on with this forward's experts, on the rows stored here

@@ -84,6 +84,7 @@ class GemmArgs(C.Structure):
         ("q_scale_pitch", C.c_longlong),
         ("sched", C.c_void_p),
         ("b_box_rows", C.c_int),
+        ("b_rows", C.c_longlong),
     ]
 
 
@@ -190,6 +191,7 @@ class MetaArgs(C.Structure):
         ("xq", C.c_void_p),
         ("xs", C.c_void_p),
         ("k_step", C.c_int),
+        ("pair2", C.c_int),
     ]
 
 

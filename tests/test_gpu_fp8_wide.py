@@ -1,0 +1,93 @@
+"""The 128-row e4m3 kernels: tile edges, an odd number of weight blocks, cut units, scale rows off the 16-byte grid."""
+
+import pytest
+import torch
+
+from moeflow_b200 import MoEConfig
+from moeflow_b200.testing import make_bias, make_hidden, make_logits, make_weights
+from moeflow_b200.tolerances import normwise_rel_err
+from moeflow_b200.weights import dequant_block_fp8, quant_block_fp8
+
+pytestmark = pytest.mark.gpu
+
+
+def _swiglu(h, limit):
+    gate, up = h.chunk(2, dim=-1)
+    gate, up = gate.clamp(max=limit), up.clamp(-limit, limit)
+    return torch.nn.functional.silu(gate) * up
+
+
+@pytest.mark.parametrize("counts", [[1], [3, 4, 5], [31, 0, 33], [127, 129], [256, 2]])
+@pytest.mark.parametrize("hidden,inter,split", [(256, 128, 1), (384, 128, 1), (640, 384, 1), (1024, 512, 2), (1024, 512, 4), (768, 384, 0)])
+def test_128_row_tiles_match_the_dequantised_definition(counts, hidden, inter, split):
+    from moeflow_b200.ops.fp8 import dequant_rows, down_proj_fp8, gate_up_swiglu_fp8, quant_rows_1x128
+    from moeflow_b200.ops.grouped_gemm import plan_from_offsets
+
+    gen = torch.Generator().manual_seed(hidden + sum(counts))
+    q13, s13, q2, s2 = [], [], [], []
+    for _ in counts:
+        a, b = quant_block_fp8(torch.randn(2 * inter, hidden, generator=gen) * (2.0 / hidden**0.5))
+        c, d = quant_block_fp8(torch.randn(hidden, inter, generator=gen) / inter**0.5)
+        q13.append(a.view(torch.uint8)), s13.append(b), q2.append(c.view(torch.uint8)), s2.append(d)
+    q13, q2 = (torch.stack(t).view(torch.float8_e4m3fn).cuda() for t in (q13, q2))
+    s13, s2 = torch.stack(s13).cuda(), torch.stack(s2).cuda()
+    n = sum(counts)
+    offsets = [sum(counts[:i]) for i in range(len(counts) + 1)]
+    x = torch.randn(n + 3, hidden, generator=gen).bfloat16().cuda()
+    idx = torch.randint(0, n + 3, (n,), generator=gen).int().cuda()
+    scale = (torch.rand(n, generator=gen) + 0.5).cuda()
+    tp = plan_from_offsets(offsets, 128, x.device)
+    status = torch.zeros(1, dtype=torch.int64, device="cuda")
+    kw = dict(split=split, status=status, wait_ns=50_000_000)
+    xq, xs = quant_rows_1x128(x)
+    padded = torch.zeros(n + 3, xs.shape[1] + 1, device="cuda")
+    padded[:, 1:] = xs
+    act = gate_up_swiglu_fp8(xq, xs, q13, s13, tp, row_index=idx, limit=10.0, **kw)
+    assert torch.equal(gate_up_swiglu_fp8(xq, padded[:, 1:], q13, s13, tp, row_index=idx, limit=10.0, **kw), act)
+    in_order = gate_up_swiglu_fp8(xq[idx.long()], xs[idx.long()], q13, s13, tp, limit=10.0, **kw)
+    assert torch.equal(in_order, act), "rows by index and contiguous rows differ"
+    aq, a_s = quant_rows_1x128(act.contiguous())
+    y = down_proj_fp8(aq, a_s, q2, s2, tp, row_scale=scale, **kw)
+    y_own_map = down_proj_fp8(aq, a_s, q2, s2, tp, row_scale=scale, b_tma=False, **kw)
+    assert int(status) == 0
+    assert torch.equal(y, y_own_map), "the caller's tensor map and the launch's own differ"
+    x_dq, a_dq = dequant_rows(xq, xs)[idx.long()], dequant_rows(aq, a_s)
+    for e, (lo, hi) in enumerate(zip(offsets[:-1], offsets[1:])):
+        if hi > lo:
+            # one bf16 rounding of every element (2**-9) on sums whose fp32 error is far below it
+            ref = _swiglu(x_dq[lo:hi] @ dequant_block_fp8(q13[e], s13[e]).t(), 10.0)
+            assert normwise_rel_err(act[lo:hi], ref) < 4 * 2.0**-8
+            ref = (a_dq[lo:hi] @ dequant_block_fp8(q2[e], s2[e]).t()) * scale[lo:hi, None]
+            assert normwise_rel_err(y[lo:hi], ref) < 4 * 2.0**-8
+
+
+@pytest.mark.parametrize("tokens,hidden,inter", [(1, 384, 256), (50, 640, 384), (300, 512, 256)])
+def test_layer_on_128_row_tiles_matches_64_row_tiles(tokens, hidden, inter):
+    """Whole layers: the plan counts pairs of weight blocks for the down GEMM, and every tile is handed over complete."""
+    from moeflow_b200.fixed import FixedEPLayer
+
+    cfg = MoEConfig(hidden_size=hidden, moe_intermediate_size=inter, n_routed_experts=4, top_k=2)
+    w13, w2 = make_weights(cfg, 0, dtype=torch.float32)
+    packs = [(*quant_block_fp8(w13[e]), *quant_block_fp8(w2[e])) for e in range(4)]
+    weights = [torch.stack([p[i].view(torch.uint8) if i in (0, 2) else p[i] for p in packs]).cuda() for i in range(4)]
+    weights = [w.view(torch.float8_e4m3fn) if w.dtype == torch.uint8 else w for w in weights]
+    bias = make_bias(cfg, 1, device="cuda")
+    x, logits = make_hidden(tokens, cfg, 2, device="cuda"), make_logits(tokens, cfg, 3, device="cuda")
+    outs = []
+    for block_m in (64, 128):
+        layer = FixedEPLayer(cfg, 0, 1, None, None, capacity=tokens + 3, backend="cuda", device="cuda",
+                             gemm_kwargs={"block_m": block_m}, wait_ns=50_000_000)
+        layer.set_weights_fp8(*weights)
+        for _ in range(2):
+            out = layer.forward(x, logits, bias).clone()
+        assert layer.check_status()["code"] == 0
+        outs.append(out)
+    # a K cut may move a bf16 activation by a step and with it the e4m3 code of some (2**-3 of the element): of 1 in 30
+    # codes at most, 2**-3 / sqrt(30) = 0.023 of the norm
+    assert normwise_rel_err(outs[1], outs[0]) < 0.023
+    # bound to bf16 experts afterwards, the layer's plan is that of the bf16 kernels again
+    layer.set_weights(torch.stack([dequant_block_fp8(p[0], p[1]) for p in packs]).bfloat16().cuda(),
+                      torch.stack([dequant_block_fp8(p[2], p[3]) for p in packs]).bfloat16().cuda())
+    out = layer.forward(x, logits, bias)
+    assert layer.check_status()["code"] == 0
+    assert normwise_rel_err(out, outs[0]) < 0.06  # e4m3 activations against bf16 ones
