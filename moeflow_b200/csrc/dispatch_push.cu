@@ -45,10 +45,14 @@ __global__ void __launch_bounds__(kDispatchThreads) dispatch_push_kernel(const m
     // First touches in parallel instead of one after the other (see touch() in common.cuh): every page this CTA
     // reads or writes, one lane each; warp 1 also touches this token's row in every destination's receive buffer.
     if (tid < 12) {
-      const void* warm[12] = {a.epoch, a.num_valid, a.logits ? (const void*)(a.logits + (size_t)min(t, a.T > 0 ? a.T - 1 : 0) * a.E) : nullptr,
-                              a.bias, a.x, a.peer_recv, a.peer_flag, a.hit + (size_t)t * a.R, a.route_w, a.route_ids,
-                              a.done_counter, a.weights};
-      touch(warm[tid]);
+      // (a chain of selects: an array of pointers would live in local memory)
+      const void* p = tid == 0 ? (const void*)a.epoch : tid == 1 ? (const void*)a.num_valid
+                    : tid == 2 ? (a.logits ? (const void*)(a.logits + (size_t)min(t, a.T > 0 ? a.T - 1 : 0) * a.E) : nullptr)
+                    : tid == 3 ? (const void*)a.bias : tid == 4 ? (const void*)a.x : tid == 5 ? (const void*)a.peer_recv
+                    : tid == 6 ? (const void*)a.peer_flag : tid == 7 ? (const void*)(a.hit + (size_t)t * a.R)
+                    : tid == 8 ? (const void*)a.route_w : tid == 9 ? (const void*)a.route_ids
+                    : tid == 10 ? (const void*)a.done_counter : (const void*)a.weights;
+      touch(p);
     } else if (tid >= 32 && tid < 32 + a.R && tid < 64) {
       const int d = tid - 32;
       touch(reinterpret_cast<const uint8_t*>(a.peer_recv[d]) + ((size_t)a.rank * a.C + t) * a.pitch);
@@ -156,10 +160,15 @@ __global__ void __launch_bounds__(kDispatchThreads) dispatch_push_kernel(const m
 // second launch, no flags, no cold start of another kernel behind a weight stream that has swept its code and pages out
 // of the caches.  The rows of e4m3 layers are quantised by the CTAs that hold them in registers.  512 threads: one
 // 16-byte chunk of a 4096-wide row each, and eight slot words each in the metadata pass.
-// 1 token on 288 experts: 24.5 us for the two kernels behind a cold cache, 17 us for this one.
+// The layout is there, from the kernel's start and between passes that stream weights: 1 token on 288 experts 9.0 us (13.1
+// with the router's scores in shared memory, the payload in front of the fence and the metadata pass unrolled throughout),
+// 128 tokens 13.4 (19.6).
 constexpr int kLocalThreads = 512;
 
-__global__ void __launch_bounds__(kLocalThreads) dispatch_local_kernel(const mf_dispatch_args a, const mf_meta_args m) {
+// kPerSm: CTAs an SM should hold.  With at most one token per SM the registers for one CTA are free and nothing spills; above
+// that two share an SM (500 tokens: 1 % of the layer).
+template <int kPerSm>
+__global__ void __launch_bounds__(kLocalThreads, kPerSm) dispatch_local_kernel(const mf_dispatch_args a, const mf_meta_args m) {
   extern __shared__ int s_dyn[];  // metadata pass, then the router's scores
   __shared__ int s_id[kMaxTopK];
   __shared__ float s_w[kMaxTopK];
@@ -218,6 +227,32 @@ __global__ void __launch_bounds__(kLocalThreads) dispatch_local_kernel(const mf_
   int present = 0;
   if (live)
     for (int k = 0; k < a.K; ++k) present |= (s_id[k] >= 0 && s_id[k] < a.L) ? 1 : 0;
+  if (tid < 32) {
+    // What the metadata pass reads goes first and is fenced by itself: the fence then waits for one warp's few words, while
+    // the other warps store (and quantise) the payload, which only has to be there when the grid is done.
+    int* meta = reinterpret_cast<int*>(row + (size_t)a.H * 2);
+    if (tid < a.K) {
+      const bool on = present && s_id[tid] >= 0 && s_id[tid] < a.L;
+      meta[tid] = on ? s_id[tid] : -1;
+      meta[a.K + tid] = on ? __float_as_int(s_w[tid]) : 0;
+    }
+    if (tid == 31) {
+      meta[2 * a.K] = present;
+      a.hit[t] = (unsigned char)present;
+    }
+    __syncwarp();
+    if (tid == 0) {
+      __threadfence();  // cumulative: the whole warp's stores, ordered by the barrier
+      const unsigned done = atomicAdd(a.done_counter, 1u);
+      __threadfence();  // in the last CTA: every other CTA's words come before what follows
+      s_last = done == gridDim.x - 1;
+      if (s_last) {
+        *a.done_counter = 0u;
+        *a.epoch += 1u;
+      }
+    }
+    __syncwarp();
+  }
   if (has_token && (present || !a.skip_payload)) {
 #pragma unroll
     for (int i = 0; i < 2; ++i) {
@@ -228,30 +263,9 @@ __global__ void __launch_bounds__(kLocalThreads) dispatch_local_kernel(const mf_
       }
     }
   }
-  int* meta = reinterpret_cast<int*>(row + (size_t)a.H * 2);
-  if (tid < a.K) {
-    const bool on = present && s_id[tid] >= 0 && s_id[tid] < a.L;
-    meta[tid] = on ? s_id[tid] : -1;
-    meta[a.K + tid] = on ? __float_as_int(s_w[tid]) : 0;
-  } else if (tid == a.K) {
-    meta[2 * a.K] = present;
-    a.hit[t] = (unsigned char)present;
-  }
   __syncthreads();
   if (trace) trace[2] = global_timer_ns();  // row stored
-  if (tid == 0) {
-    __threadfence();  // cumulative: the whole CTA's stores, ordered by the barrier
-    const unsigned done = atomicAdd(a.done_counter, 1u);
-    s_last = done == gridDim.x - 1;
-    if (s_last) {
-      *a.done_counter = 0u;
-      *a.epoch += 1u;
-    }
-  }
-  __syncthreads();
   if (!s_last) return;
-  if (tid == 0) __threadfence();  // every other CTA's row comes before what follows
-  __syncthreads();
   meta_one_pass<kLocalThreads>(m, s_dyn, (m.trace != nullptr && tid == 0) ? m.trace : nullptr);
 }
 
@@ -272,7 +286,10 @@ extern "C" int mf_dispatch_local(const mf_dispatch_args* a, const mf_meta_args* 
     smem += 2 * (size_t)a->E * sizeof(float);
   }
   if (smem > 48 * 1024) return -5;  // L = E <= 512: at most 41 KB
-  dispatch_local_kernel<<<a->C, kLocalThreads, smem, static_cast<cudaStream_t>(stream)>>>(*a, *m);
+  if (a->C <= m->n_sms)
+    dispatch_local_kernel<1><<<a->C, kLocalThreads, smem, static_cast<cudaStream_t>(stream)>>>(*a, *m);
+  else
+    dispatch_local_kernel<2><<<a->C, kLocalThreads, smem, static_cast<cudaStream_t>(stream)>>>(*a, *m);
   return (int)cudaGetLastError();
 }
 

@@ -49,10 +49,13 @@ __host__ __device__ __forceinline__ int hist_pitch(int L) { return L | 1; }
 // Only the words in use: clearing the arrays whole was 100 KB to 400 KB of stores by one CTA at 288 experts.
 template <int kThreads>
 __device__ __forceinline__ void clear_counters(const mf_meta_args& a, int n_tiles, int cut1, int cut2) {
+#pragma unroll 1
   for (int i = threadIdx.x; i < min(n_tiles, a.n_tile_done); i += kThreads) a.counters1[a.n_counters1 + i] = 0;
   if (cut1 != 1)
+#pragma unroll 1
     for (int i = threadIdx.x; i < min(n_tiles * a.m_blocks1 * 8, a.n_counters1); i += kThreads) a.counters1[i] = 0;
   if (cut2 != 1)
+#pragma unroll 1
     for (int i = threadIdx.x; i < min(n_tiles * a.m_blocks2 * 8, a.n_counters2); i += kThreads) a.counters2[i] = 0;
 }
 
@@ -144,6 +147,7 @@ template <int kThreads>
 __device__ __forceinline__ void meta_begin(const mf_meta_args& a, int* sm) {
   const int P = hist_pitch(a.L);
   const MetaSpan span(a, kThreads / 32);
+#pragma unroll 1
   for (int i = threadIdx.x; i < span.n_warps * P; i += kThreads) sm[i] = 0;
   if (threadIdx.x == 0) sm[kThreads / 32 * P + 2 * a.L + 34] = sm[kThreads / 32 * P + 2 * a.L + 35] = 0;
 }
@@ -164,23 +168,25 @@ __device__ __forceinline__ void meta_one_pass(const mf_meta_args& a, int* sm, un
   const size_t meta_off = (size_t)a.H * 2;
   int* my_hist = hist + warp * P;
 
-  // the only reads of the received rows: id, valid flag and weight bits of every slot word of this thread
-  int key[kMetaBatch], wbits[kMetaBatch], pre[kMetaBatch];
+  // The only reads of the received rows: id, valid flag and weight bits of every slot word of this thread, none of them
+  // used before all are requested.
+  // Every instruction of this pass runs once, so it costs what its fetch costs (about 4 cycles each): the loops over batches
+  // leave at the first empty one, and no loop is unrolled further than its usual count.  With all eight batches walked
+  // through and 64 registers (reloads from local memory on the way) the part behind the loads took 4.2 us for one token of
+  // 288 experts and 8.2 us for 128; it takes 1.8 and 4.0.
+  int key[kMetaBatch], wbits[kMetaBatch], pre[kMetaBatch], flag[kMetaBatch];
 #pragma unroll
   for (int b = 0; b < kMetaBatch; ++b) {
+    if (begin + b * 32 >= end) break;  // warp-uniform
     const int i = begin + b * 32 + lane;
     key[b] = -1;
-    wbits[b] = 0;
+    wbits[b] = flag[b] = 0;
     if (i < end) {
       const int row = i / K, slot = i - row * K;
       const int* meta = reinterpret_cast<const int*>(recv + (size_t)row * a.pitch + meta_off);
-      const int id = __ldcg(meta + slot);
-      const int valid = __ldcg(meta + 2 * K);
-      const int wb = __ldcg(meta + K + slot);
-      if (valid != 0 && id >= 0 && id < L) {
-        key[b] = id;
-        wbits[b] = wb;
-      }
+      key[b] = __ldcg(meta + slot);
+      flag[b] = __ldcg(meta + 2 * K);
+      wbits[b] = __ldcg(meta + K + slot);
     }
   }
   if (trace) trace[6] = global_timer_ns();  // loads issued
@@ -191,7 +197,9 @@ __device__ __forceinline__ void meta_one_pass(const mf_meta_args& a, int* sm, un
   const bool k_pow2 = (K & (K - 1)) == 0 && K <= 32;
 #pragma unroll
   for (int b = 0; b < kMetaBatch; ++b) {
-    if (begin + b * 32 < end) {  // warp-uniform
+    if (begin + b * 32 >= end) break;
+    {
+      if (flag[b] == 0 || key[b] < 0 || key[b] >= L) key[b] = -1;
       const unsigned same = __match_any_sync(0xffffffffu, key[b]);
       int before = 0;
       if (key[b] >= 0) before = my_hist[key[b]];
@@ -222,20 +230,20 @@ __device__ __forceinline__ void meta_one_pass(const mf_meta_args& a, int* sm, un
   __syncthreads();
   if (trace) trace[3] = global_timer_ns();  // histogram done
 
-  // Per expert (one thread each): exclusive prefix over the warps and total count.  The counts of 16 warps are loaded
+  // Per expert (one thread each): exclusive prefix over the warps and total count.  The counts of four warps are loaded
   // together; a warp scan per expert instead was 18 dependent rounds per warp at 288 experts.
+#pragma unroll 1
   for (int e = tid; e < L; e += kThreads) {
     int run = 0;
+    int* h = hist + e;
 #pragma unroll 1
-    for (int w0 = 0; w0 < n_warps; w0 += 16) {
-      int c[16];
-#pragma unroll
-      for (int w = 0; w < 16; ++w) c[w] = w0 + w < n_warps ? hist[(w0 + w) * P + e] : 0;
-#pragma unroll
-      for (int w = 0; w < 16; ++w) {
-        if (w0 + w < n_warps) hist[(w0 + w) * P + e] = run;
-        run += c[w];
-      }
+    for (int left = n_warps; left > 0; left -= 4, h += 4 * P) {
+      const int c0 = h[0], c1 = left > 1 ? h[P] : 0, c2 = left > 2 ? h[2 * P] : 0, c3 = left > 3 ? h[3 * P] : 0;
+      h[0] = run;
+      if (left > 1) h[P] = run + c0;
+      if (left > 2) h[2 * P] = run + c0 + c1;
+      if (left > 3) h[3 * P] = run + c0 + c1 + c2;
+      run += c0 + c1 + c2 + c3;
     }
     cnt[e] = run;
   }
@@ -268,6 +276,7 @@ __device__ __forceinline__ void meta_one_pass(const mf_meta_args& a, int* sm, un
   if (tid < L) {
     offs[tid] = my_off;
     a.offsets[tid] = my_off;
+#pragma unroll 1
     for (int j = 0; j < my_nt; ++j) {
       const int idx = my_tb + j;
       if (idx < a.max_tiles) {
@@ -308,6 +317,7 @@ __device__ __forceinline__ void meta_one_pass(const mf_meta_args& a, int* sm, un
   // placement: arithmetic and stores only
 #pragma unroll
   for (int b = 0; b < kMetaBatch; ++b) {
+    if (begin + b * 32 >= end) break;
     const int i = begin + b * 32 + lane;
     if (i < end) {
       int pos = -1;

@@ -52,7 +52,30 @@ __device__ __forceinline__ void route_token_warp(const float* __restrict__ lg, c
                                                  float* score, float* biased, const RouteParams& p, int lane,
                                                  float& out_w, int& out_id) {
   const int E = p.E;
-  if (E <= 32 * kRouteRegs) {
+  unsigned key[kRouteRegs] = {};  // E <= 512: order keys of the biased scores of experts lane, lane + 32, ...
+  const bool in_regs = E <= 32 * kRouteRegs;
+  // Sigmoid scores without groups never leave the registers, but for the score that a slot's weight is read from; the loops
+  // leave at the first batch of 32 that holds no expert.
+  const bool direct = in_regs && p.sigmoid && p.n_group <= 1;
+  if (direct) {
+    float l[kRouteRegs], b[kRouteRegs];
+#pragma unroll
+    for (int j = 0; j < kRouteRegs; ++j) {
+      if (32 * j >= E) break;
+      const int e = lane + 32 * j;
+      l[j] = e < E ? lg[e] : 0.f;
+      b[j] = bias && e < E ? bias[e] : 0.f;
+    }
+#pragma unroll
+    for (int j = 0; j < kRouteRegs; ++j) {
+      if (32 * j >= E) break;
+      const int e = lane + 32 * j;
+      const float v = 1.f / (1.f + expf(-l[j]));
+      if (e < E) score[e] = v;
+      key[j] = e < E ? float_order_key(bias ? v + b[j] : v) : 0u;  // padding never beats a real entry
+    }
+    __syncwarp();
+  } else if (in_regs) {
     // All of the lane's logits and biases are requested before the first one is used: they are usually cold, and a
     // loop that computes on each as it comes pays the DRAM latency once per unrolled round.
     float l[kRouteRegs], b[kRouteRegs];
@@ -78,7 +101,8 @@ __device__ __forceinline__ void route_token_warp(const float* __restrict__ lg, c
       biased[e] = bias ? bias[e] : 0.f;
     }
   }
-  if (p.sigmoid) {
+  if (direct) {
+  } else if (p.sigmoid) {
     for (int e = lane; e < E; e += 32) score[e] = 1.f / (1.f + expf(-score[e]));
   } else {
     float m = -CUDART_INF_F;
@@ -93,8 +117,10 @@ __device__ __forceinline__ void route_token_warp(const float* __restrict__ lg, c
     for (int off = 16; off > 0; off >>= 1) s += __shfl_xor_sync(0xffffffffu, s, off);
     for (int e = lane; e < E; e += 32) score[e] = score[e] / s;
   }
-  for (int e = lane; e < E; e += 32) biased[e] = bias ? score[e] + biased[e] : score[e];
-  __syncwarp();
+  if (!direct) {
+    for (int e = lane; e < E; e += 32) biased[e] = bias ? score[e] + biased[e] : score[e];
+    __syncwarp();
+  }
 
   if (p.n_group > 1) {
     // One lane per group (n_group <= 32): score the group, then rank the groups.
@@ -128,24 +154,28 @@ __device__ __forceinline__ void route_token_warp(const float* __restrict__ lg, c
   float wsum = 0.f;
   float my_w = 0.f;  // lane k keeps the weight of slot k (K <= 32)
   int my_id = 0;
-  if (E <= 32 * kRouteRegs) {
+  if (in_regs) {
     // Selection out of registers: lane l holds experts l, l + 32, ...; a round is a scan of the lane's own
-    // values, one warp-wide max over order-preserving integer keys and one warp-wide min over the ids that
+    // keys, one warp-wide max over them and one warp-wide min over the ids that
     // carry that maximum (ties go to the lower id), instead of ten dependent shuffles.
-    float v[kRouteRegs];
+    if (!direct) {
 #pragma unroll
-    for (int j = 0; j < kRouteRegs; ++j) {
-      const int e = lane + 32 * j;
-      v[j] = e < E ? biased[e] : -CUDART_INF_F;
+      for (int j = 0; j < kRouteRegs; ++j) {
+        if (32 * j >= E) break;
+        const int e = lane + 32 * j;
+        key[j] = e < E ? float_order_key(biased[e]) : 0u;
+      }
     }
+    const unsigned taken = float_order_key(-CUDART_INF_F);
+#pragma unroll 1
     for (int k = 0; k < p.K; ++k) {
       unsigned bk = 0u;
       int bj = 0;
 #pragma unroll
       for (int j = 0; j < kRouteRegs; ++j) {
-        const unsigned key = (lane + 32 * j < E) ? float_order_key(v[j]) : 0u;  // padding never beats a real entry
-        if (key > bk) {  // strictly greater: the lowest index (lowest id of this lane) keeps a tie
-          bk = key;
+        if (32 * j >= E) break;
+        if (key[j] > bk) {  // strictly greater: the lowest index (lowest id of this lane) keeps a tie
+          bk = key[j];
           bj = j;
         }
       }
@@ -158,9 +188,9 @@ __device__ __forceinline__ void route_token_warp(const float* __restrict__ lg, c
         my_w = w;
         my_id = id;
       }
+      const int out = lane == (id & 31) ? id >> 5 : -1;
 #pragma unroll
-      for (int j = 0; j < kRouteRegs; ++j)
-        if (lane == (id & 31) && j == (id >> 5)) v[j] = -CUDART_INF_F;
+      for (int j = 0; j < kRouteRegs; ++j) key[j] = out == j ? taken : key[j];
     }
   } else {
     for (int k = 0; k < p.K; ++k) {
