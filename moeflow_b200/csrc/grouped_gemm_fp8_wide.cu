@@ -12,9 +12,10 @@
 // Promotion works on 32 columns at a time, the next load under way while one is multiplied; its eight warps (a lane
 // quarter and half of the columns each) hold 128 sums and two loads in registers, which is why the other four warps
 // hand registers over to them.
-// 36 experts of 3 x 4096 x 1536, whole layer, against the 64-row kernel's form on 128-row tiles: 2000 tokens 951 / 619 us
-// (gate/up 528 / 345, down 305 / 180), 1000 tokens 522 / 368, 500 tokens 314 / 244.  What bounds it now: 48 KB from L2 per
-// K block (8.4 TB/s over all SMs in the down GEMM) next to 514 cycles of UMMA and about 400 of promotion.
+// 36 experts of 3 x 4096 x 1536, whole layer, against the 64-row kernel's form on 128-row tiles: 2000 tokens 951 / 542 us
+// (gate/up 528 / 285, down 305 / 160), 1000 tokens 522 / 326, 500 tokens 314 / 215.  What bounds it now: per K block 48 KB
+// through L2 (210 us of the gate/up GEMM at 2000 tokens with everything else taken out), the promotion, which only half
+// overlaps it, and 5 us of epilogue per gate/up unit.
 //
 // Warps: 0 weight TMA and segment hand-out, 1 UMMA, 2 token TMA (down: contiguous rows in boxes), 3 activation and weight
 // scales (four K blocks at a time, up to 16 ahead) and finished token tiles, 4-11 promotion and epilogue, 12-15 gather
@@ -39,7 +40,7 @@ constexpr int kFwGather = 128;                 // gather threads (gate/up)
 constexpr int kFwPromo = 8;                    // promotion warps: 4 .. 11
 constexpr int kFwStageW = 2 * kF8TileA;        // 256 weight rows x one K block
 constexpr int kFwStageX = kFwRows * 128;
-constexpr int kFwStages = 4;
+constexpr int kFwStages = 3;                   // (four: 4 % slower)
 constexpr int kFwTmp = 2;                      // tensor-memory accumulators of 256 columns
 constexpr int kFwScaleSlots = 4;               // scales of four K blocks each
 constexpr int kFwScaleFloats = 4 * kFwRows + 8;  // [4][128] activation scales, [2][4] weight scales
@@ -500,15 +501,16 @@ grouped_gemm_fp8_wide_kernel(const __grid_constant__ CUtensorMap tmap_w, const _
       }
       if (!ok) break;
 
+      // The unit is cut along K: park the sums, [half][column / 4][row][4]; the quarter that arrives last adds the segments
+      // in K order, straight into its outputs (sum_16).  Summed up in the registers of the K loop instead, these few lines
+      // made the compiler spill in that loop (layer at 2000 tokens: 585 us against 542).
+      const bool cut_unit = sg.nseg > 1;
       bool finish = true;
-      if (sg.nseg > 1) {
-        // The unit is cut along K: park the sums, [half][column / 4][row][4]; the quarter that arrives last adds the
-        // segments in K order.
-        auto slot_at = [&](int s_) {
-          return reinterpret_cast<float4*>(a.partial + (long long)slot_of(sg, s_) * 2 * slot_cols * kF8BlockM) +
-                 (long long)(16 * grp) * slot_cols + row;
-        };
-        const long long half = 32ll * slot_cols;
+      const int half = 32 * slot_cols;
+      auto slot_at = [&](int s_) {
+        return reinterpret_cast<float4*>(a.partial) + ((long long)slot_of(sg, s_) * 64 + 16 * grp) * slot_cols + row;
+      };
+      if (cut_unit) {
         if (row < n_rows) {
           float4* p = slot_at(sg.seg);
 #pragma unroll
@@ -530,49 +532,46 @@ grouped_gemm_fp8_wide_kernel(const __grid_constant__ CUtensorMap tmap_w, const _
         if (finish) {
           __threadfence();
           if (grp == 0 && lane == 0) *counter = 0;
+        }
+      }
+      // Columns 16 c .. of this warp's share of half h over all segments (finish only, cut units).
+      auto sum_16 = [&](int h, int c, float (&v)[16]) {
 #pragma unroll
-          for (int i = 0; i < 32; ++i) acc0[i] = acc1[i] = 0ull;
-          const f32x2 one = pack2(1.f, 1.f);
-          if (row < n_rows) {
-            for (int s_ = 0; s_ < sg.nseg; ++s_) {
-              const float4* p = slot_at(s_);
+        for (int i = 0; i < 16; ++i) v[i] = 0.f;
+#pragma unroll 1
+        for (int s_ = 0; s_ < sg.nseg; ++s_) {
+          float4 x[1][4];
 #pragma unroll
-              for (int h = 0; h < 2; ++h) {
-                float4 x[8], y[8];
+          for (int k = 0; k < 1; ++k) {
+            const float4* p = slot_at(min(s_ + k, sg.nseg - 1)) + h * half + (long long)(4 * c) * slot_cols;
 #pragma unroll
-                for (int i = 0; i < 8; ++i, p += slot_cols) {
-                  x[i] = __ldcg(p);
-                  y[i] = two ? __ldcg(p + half) : make_float4(0.f, 0.f, 0.f, 0.f);
-                }
+            for (int i = 0; i < 4; ++i, p += slot_cols)
+              x[k][i] = s_ + k < sg.nseg && row < n_rows ? __ldcg(p) : make_float4(0.f, 0.f, 0.f, 0.f);
+          }
 #pragma unroll
-                for (int i = 0; i < 8; ++i) {
-                  const int c = 16 * h + 2 * i;
-                  acc0[c] = fma2(pack2(x[i].x, x[i].y), one, acc0[c]);
-                  acc0[c + 1] = fma2(pack2(x[i].z, x[i].w), one, acc0[c + 1]);
-                  acc1[c] = fma2(pack2(y[i].x, y[i].y), one, acc1[c]);
-                  acc1[c + 1] = fma2(pack2(y[i].z, y[i].w), one, acc1[c + 1]);
-                }
-              }
+          for (int k = 0; k < 1; ++k) {
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+              v[4 * i] += x[k][i].x;
+              v[4 * i + 1] += x[k][i].y;
+              v[4 * i + 2] += x[k][i].z;
+              v[4 * i + 3] += x[k][i].w;
             }
           }
         }
-      }
+      };
 
       if (finish) {
-        // 32 outputs of every row of this quarter, 16 bytes per lane and four lanes per row
-        auto store_32 = [&](const f32x2* v, float scale, int col) {
+        auto pack_bf16 = [](float x, float y) {
+          const __nv_bfloat162 h = __floats2bfloat162_rn(x, y);
+          return *reinterpret_cast<const uint32_t*>(&h);
+        };
+        // 32 outputs (bf16 pairs) of every row of this quarter, 16 bytes per lane and four lanes per row
+        auto store_32 = [&](const uint32_t* o, int col) {
           __syncwarp();  // the previous block's reads are done
 #pragma unroll
-          for (int i = 0; i < 4; ++i) {
-            uint32_t o[4];
-#pragma unroll
-            for (int k = 0; k < 4; ++k) {
-              const float2 f = unpack2(v[4 * i + k]);
-              const __nv_bfloat162 h = __floats2bfloat162_rn(f.x * scale, f.y * scale);
-              o[k] = *reinterpret_cast<const uint32_t*>(&h);
-            }
-            *reinterpret_cast<uint4*>(stage + lane * kFwOutPitch + 16 * i) = make_uint4(o[0], o[1], o[2], o[3]);
-          }
+          for (int i = 0; i < 4; ++i)
+            *reinterpret_cast<uint4*>(stage + lane * kFwOutPitch + 16 * i) = make_uint4(o[4 * i], o[4 * i + 1], o[4 * i + 2], o[4 * i + 3]);
           __syncwarp();
           __nv_bfloat16* out = static_cast<__nv_bfloat16*>(a.out) + col + (lane & 3) * 8;
 #pragma unroll
@@ -583,38 +582,46 @@ grouped_gemm_fp8_wide_kernel(const __grid_constant__ CUtensorMap tmap_w, const _
           }
         };
         if (kGateUp) {
-          if (live) {
+          uint32_t act[32];  // bf16 pairs: this lane's 64 activations
+          auto activate = [&](float2 g, float2 u) {
+            if (a.round_h) {
+              g.x = bf16_round(g.x);
+              g.y = bf16_round(g.y);
+              u.x = bf16_round(u.x);
+              u.y = bf16_round(u.y);
+            }
+            return pack_bf16(swiglu_clamped(g.x, u.x, a.limit), swiglu_clamped(g.y, u.y, a.limit));
+          };
 #pragma unroll
-            for (int i = 0; i < 32; ++i) {
-              float2 g = unpack2(acc0[i]), u = unpack2(acc1[i]);
-              if (a.round_h) {
-                g.x = bf16_round(g.x);
-                g.y = bf16_round(g.y);
-                u.x = bf16_round(u.x);
-                u.y = bf16_round(u.y);
-              }
-              acc0[i] = pack2(swiglu_clamped(g.x, u.x, a.limit), swiglu_clamped(g.y, u.y, a.limit));
+          for (int i = 0; i < 32; ++i) act[i] = 0u;
+          if (live && !cut_unit) {
+#pragma unroll
+            for (int i = 0; i < 32; ++i) act[i] = activate(unpack2(acc0[i]), unpack2(acc1[i]));
+          } else if (live) {
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+              float g[16], u[16];
+              sum_16(0, c, g);
+              sum_16(1, c, u);
+#pragma unroll
+              for (int i = 0; i < 8; ++i)
+                act[8 * c + i] = activate(make_float2(g[2 * i], g[2 * i + 1]), make_float2(u[2 * i], u[2 * i + 1]));
             }
           }
           if (a.q_out == nullptr) {
             if (live) {
-              store_32(acc0, 1.f, sg.mb * kF8BlockM + 64 * grp);
-              store_32(acc0 + 16, 1.f, sg.mb * kF8BlockM + 64 * grp + 32);
+              store_32(act, sg.mb * kF8BlockM + 64 * grp);
+              store_32(act + 16, sg.mb * kF8BlockM + 64 * grp + 32);
             }
           } else {
             // The quantiser is defined on the bf16 activations; a group is the unit's 128 columns of one row, half of
             // them in this lane and half in the same lane of the quarter's other warp.  The maxima of two units in a row
             // lie in different words, so a warp that runs ahead does not touch what the other one still reads.
             float* maxima = sMax + (n_it & 1) * 2 * kFwRows;
+            auto value = [&](int i) { return __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&act[i])); };
             float peak = 0.f;
 #pragma unroll
-            for (int i = 0; i < 32; ++i) {
-              float2 v = unpack2(acc0[i]);
-              v.x = bf16_round(v.x);
-              v.y = bf16_round(v.y);
-              peak = fmaxf(peak, fmaxf(fabsf(v.x), fabsf(v.y)));
-              acc0[i] = pack2(v.x, v.y);
-            }
+            for (int i = 0; i < 32; ++i) peak = fmaxf(peak, fmaxf(fabsf(value(i).x), fabsf(value(i).y)));
             maxima[grp * kFwRows + row] = peak;
             ok = pair_sync();
             if (!ok) break;
@@ -628,22 +635,42 @@ grouped_gemm_fp8_wide_kernel(const __grid_constant__ CUtensorMap tmap_w, const _
               for (int i = 0; i < 4; ++i) {
                 uint32_t o[4];
 #pragma unroll
-                for (int k = 0; k < 4; ++k) {
-                  const float2 x = unpack2(acc0[8 * i + 2 * k]), y = unpack2(acc0[8 * i + 2 * k + 1]);
-                  o[k] = (uint32_t)to_e4m3(x.x, inv) | ((uint32_t)to_e4m3(x.y, inv) << 8) | ((uint32_t)to_e4m3(y.x, inv) << 16) |
-                         ((uint32_t)to_e4m3(y.y, inv) << 24);
-                }
+                for (int k = 0; k < 4; ++k)
+                  o[k] = (uint32_t)to_e4m3x2(value(8 * i + 2 * k), inv) | ((uint32_t)to_e4m3x2(value(8 * i + 2 * k + 1), inv) << 16);
                 out[i] = make_uint4(o[0], o[1], o[2], o[3]);
               }
             }
           }
         } else if (live) {
           const int col = sg.mb * 2 * kF8BlockM + 64 * grp;
-          store_32(acc0, row_scale, col);
-          store_32(acc0 + 16, row_scale, col + 32);
-          if (two) {
-            store_32(acc1, row_scale, col + kF8BlockM);
-            store_32(acc1 + 16, row_scale, col + kF8BlockM + 32);
+          if (!cut_unit) {
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {  // 32 columns of the first half, twice, then of the second
+              if (q < 2 || two) {
+                uint32_t o[16];
+#pragma unroll
+                for (int i = 0; i < 16; ++i) {
+                  const float2 f = unpack2(q < 2 ? acc0[16 * (q & 1) + i] : acc1[16 * (q & 1) + i]);
+                  o[i] = pack_bf16(f.x * row_scale, f.y * row_scale);
+                }
+                store_32(o, col + (q >> 1) * kF8BlockM + (q & 1) * 32);
+              }
+            }
+          } else {
+#pragma unroll 1
+            for (int q = 0; q < (two ? 8 : 4); ++q) {  // 16 columns, 32 bytes per lane
+              float v[16];
+              sum_16(q >> 2, q & 3, v);
+              uint32_t o[8];
+#pragma unroll
+              for (int i = 0; i < 8; ++i) o[i] = pack_bf16(v[2 * i] * row_scale, v[2 * i + 1] * row_scale);
+              if (row < n_rows) {
+                uint4* out = reinterpret_cast<uint4*>(static_cast<__nv_bfloat16*>(a.out) + (long long)(row_start + row) * a.out_pitch + col +
+                                                      (q >> 2) * kF8BlockM + (q & 3) * 16);
+                out[0] = make_uint4(o[0], o[1], o[2], o[3]);
+                out[1] = make_uint4(o[4], o[5], o[6], o[7]);
+              }
+            }
           }
         }
         if (kGateUp && a.tile_done != nullptr && sg.nseg > 1) {  // only the quarter that finished a cut unit knows

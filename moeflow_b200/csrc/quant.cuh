@@ -14,6 +14,10 @@ __device__ __forceinline__ uint8_t to_e4m3(float x, float inv_scale) {
   return (uint8_t)__nv_cvt_float_to_fp8(x * inv_scale, __NV_SATFINITE, __NV_E4M3);
 }
 
+__device__ __forceinline__ uint16_t to_e4m3x2(float2 v, float inv_scale) {  // v.x in the low byte
+  return (uint16_t)__nv_cvt_float2_to_fp8x2(make_float2(v.x * inv_scale, v.y * inv_scale), __NV_SATFINITE, __NV_E4M3);
+}
+
 // Chunk c of one row (`v`: its 8 bf16 values).  16 consecutive threads hold a group: all of them must call this together.
 __device__ __forceinline__ void quant_chunk(const uint4& v, int c, uint8_t* q_row, float* scale_row) {
   const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&v);

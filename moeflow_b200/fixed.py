@@ -972,14 +972,15 @@ def choose_block_m(capacity: int, top_k: int, local_experts: int, fp8: bool = Fa
     341 rows 1393 / 1155 (128 / 256).  A wider tile keeps an expert's rows in one tile (one pass over its weights)
     and, at 256 rows, halves the operand bytes per flop that a CTA pulls from L2.
 
-    ``fp8``: the layer will hold block-scaled e4m3 experts.  Their kernels take tiles of up to 128 rows (128 from 60
-    expected rows: 40 rows 167 / 197, 56 rows 194 / 202, 78 rows 262 / 215 (64 / 128, 36 experts), 57 rows 354 / 340, 67 rows
-    421 / 360 (72 experts)), and 256-row tiles mean expanding the experts to bf16 in every forward, which pays from about
-    512 expected rows per expert on.
+    ``fp8``: the layer will hold block-scaled e4m3 experts.  Their kernels take tiles of up to 128 rows, and 256-row tiles
+    mean expanding the experts to bf16 in every forward, which pays from about 512 expected rows per expert on.  64 / 128
+    rows: 144 experts of 2048, 44 rows 814 / 728, 55 rows 902 / 759; 72 experts, 28 rows 355 / 368 (zipf popularity 206 / 154),
+    40 rows 315 / 297, 50 rows 348 / 306; 36 experts, 28 rows (zipf) 104 / 106, 40 rows 167 / 174, 56 rows 194 / 180, 78 rows
+    262 / 215.  Layers with few experts have fewer units than CTAs want at 128 rows, so their line lies higher.
     """
     expected = (capacity * top_k) / max(local_experts, 1)
     if fp8:
-        return 256 if expected >= 512 else 128 if expected >= 60 else 64
+        return 256 if expected >= 512 else 128 if expected >= (36 if local_experts >= 64 else 60) else 64
     return 256 if expected >= 80 else 128 if expected >= 36 else 64
 
 
