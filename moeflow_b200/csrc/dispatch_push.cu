@@ -24,13 +24,11 @@
 
 namespace mf {
 
-// Threads per CTA: 256 at decode sizes (the hidden row is loaded and stored by many lanes at once); 128 from 1024
-// token positions on, where the kernel is bound by how many CTAs (one token each: a routing warp and its latency)
-// an SM holds at a time, and half-size CTAs double that number.
+// A CTA per token: the hidden row is loaded and stored by many lanes at once.
+constexpr int kDispatchThreads = 256;
 constexpr int kMaxTopK = 32;
 constexpr int kMaxRanks = 256;
 
-template <int kDispatchThreads>
 __global__ void __launch_bounds__(kDispatchThreads) dispatch_push_kernel(const mf_dispatch_args a) {
   __shared__ int s_id[kMaxTopK];
   __shared__ float s_w[kMaxTopK];
@@ -144,6 +142,95 @@ __global__ void __launch_bounds__(kDispatchThreads) dispatch_push_kernel(const m
     for (int d = tid; d < a.R; d += 32) red_add_relaxed_sys_u32(reinterpret_cast<unsigned*>(a.peer_flag[d]) + a.rank, 1u);
     if (tid == 0) {
       // the local epoch (read by this rank's later kernels after this grid has completed)
+      const unsigned done = atomicAdd(a.done_counter, 1u);
+      if (done == gridDim.x - 1) {
+        *a.done_counter = 0u;
+        *a.epoch = epoch_next;
+        if (a.trace) a.trace[5] = global_timer_ns();  // last CTA done
+      }
+    }
+    if (trace) trace[4] = global_timer_ns();  // arrivals sent
+  }
+}
+
+// The same for prefill sizes (from 1024 token positions, up to 32 ranks): a warp per token and four of them per CTA, with
+// nothing shared between them but the arrival.  With a CTA per token three of its four warps waited for the one that
+// routes, in 3.5 waves of CTAs at 8192 tokens; a quarter of the CTAs also means a quarter of the fences and arrivals.
+// Kernel at 8192 tokens 74 / 53 us, at 2000 21 / 14.
+constexpr int kManyWarps = 4;
+
+__global__ void __launch_bounds__(32 * kManyWarps) dispatch_push_many_kernel(const mf_dispatch_args a) {
+  extern __shared__ float s_many[];  // [kManyWarps][2 E] scores of the tokens being routed
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int t = blockIdx.x * kManyWarps + warp;
+  unsigned long long* trace = (a.trace != nullptr && blockIdx.x == 0 && threadIdx.x == 0) ? a.trace : nullptr;
+  if (trace) trace[0] = global_timer_ns();
+  grid_dep_launch();
+  const unsigned epoch_next = *a.epoch + 1u;
+  if (t < a.C) {
+    const bool has_token = t < a.T;
+    const bool live = has_token && (a.num_valid == nullptr || t < *a.num_valid);
+    // the first half of the row is under way while the token is routed
+    const int chunks = a.H / 8;  // 16-byte chunks
+    constexpr int kAhead = 8;
+    const uint4* xr = reinterpret_cast<const uint4*>(static_cast<const __nv_bfloat16*>(a.x) + (size_t)t * a.H);
+    uint4 xv[kAhead];
+    if (has_token) {
+#pragma unroll
+      for (int i = 0; i < kAhead; ++i)
+        if (lane + 32 * i < chunks) xv[i] = xr[lane + 32 * i];
+    }
+    float w = 0.f;
+    int id = -1;  // lane k (< K): slot k
+    if (has_token) {
+      if (a.logits != nullptr) {
+        float* score = s_many + (size_t)warp * 2 * a.E;
+        const RouteParams p{a.E, a.K, a.n_group, a.topk_group, a.sigmoid, a.renorm, a.scale};
+        route_token_warp(a.logits + (size_t)t * a.E, a.bias, score, score + a.E, p, lane, w, id);
+        if (lane < a.K) {
+          a.route_w[(size_t)t * a.K + lane] = w;
+          a.route_ids[(size_t)t * a.K + lane] = id;
+        }
+      } else if (lane < a.K) {
+        id = a.ids[(size_t)t * a.K + lane];
+        w = a.weights[(size_t)t * a.K + lane];
+      }
+    }
+    if (lane >= a.K) id = -1;
+    if (trace) trace[1] = global_timer_ns();  // routed
+    const int owner = id >= 0 ? id / a.L : -1;
+    for (int d = 0; d < a.R; ++d) {
+      const bool on = live && owner == d;
+      const int present = __any_sync(0xffffffffu, on) ? 1 : 0;
+      uint8_t* row = reinterpret_cast<uint8_t*>(a.peer_recv[d]) + ((size_t)a.rank * a.C + t) * a.pitch;
+      if (has_token && (present || !a.skip_payload)) {
+        uint4* dst = reinterpret_cast<uint4*>(row);
+#pragma unroll
+        for (int i = 0; i < kAhead; ++i)
+          if (lane + 32 * i < chunks) dst[lane + 32 * i] = xv[i];
+#pragma unroll 8
+        for (int c = lane + 32 * kAhead; c < chunks; c += 32) dst[c] = xr[c];
+      }
+      int* meta = reinterpret_cast<int*>(row + (size_t)a.H * 2);
+      if (lane < a.K) {
+        meta[lane] = on ? id - d * a.L : -1;
+        meta[a.K + lane] = on ? __float_as_int(w) : 0;
+      }
+      if (lane == 0) {
+        meta[2 * a.K] = present;
+        a.hit[(size_t)t * a.R + d] = (unsigned char)present;
+      }
+    }
+  }
+  __syncthreads();
+  if (trace) trace[2] = global_timer_ns();  // rows stored
+  if (warp == 0) {
+    fence_before_arrival(a.R);
+    if (trace) trace[3] = global_timer_ns();  // fenced
+    // one arrival per token position, as from a CTA per token
+    const unsigned rows = (unsigned)min(kManyWarps, a.C - (int)blockIdx.x * kManyWarps);
+    if (lane < a.R) red_add_relaxed_sys_u32(reinterpret_cast<unsigned*>(a.peer_flag[lane]) + a.rank, rows);
+    if (lane == 0) {
       const unsigned done = atomicAdd(a.done_counter, 1u);
       if (done == gridDim.x - 1) {
         *a.done_counter = 0u;
@@ -294,7 +381,7 @@ extern "C" int mf_dispatch_local(const mf_dispatch_args* a, const mf_meta_args* 
 }
 
 extern "C" int mf_dispatch_push(const mf_dispatch_args* a, mf_stream_t stream) {
-  const int threads = (a && a->C >= 1024 && a->H / 8 <= 128 * 4 && a->R <= 32) ? 128 : 256;
+  constexpr int threads = mf::kDispatchThreads;
   if (!a || a->C < 1 || a->T > a->C || a->K > mf::kMaxTopK || a->R > mf::kMaxRanks || a->H % 8 != 0 ||
       a->H / 8 > threads * 4 || (a->pitch & 15) != 0 || a->pitch < (long long)a->H * 2 + (2 * a->K + 1) * 4)
     return -1;
@@ -304,9 +391,11 @@ extern "C" int mf_dispatch_push(const mf_dispatch_args* a, mf_stream_t stream) {
     smem = 2 * (size_t)a->E * sizeof(float);
     if (smem > 40 * 1024) return -3;
   }
-  if (threads == 128)
-    mf::dispatch_push_kernel<128><<<a->C, 128, smem, static_cast<cudaStream_t>(stream)>>>(*a);
-  else
-    mf::dispatch_push_kernel<256><<<a->C, 256, smem, static_cast<cudaStream_t>(stream)>>>(*a);
+  if (a->C >= 1024 && a->R <= 32 && mf::kManyWarps * smem <= 40 * 1024) {
+    const int ctas = (a->C + mf::kManyWarps - 1) / mf::kManyWarps;
+    mf::dispatch_push_many_kernel<<<ctas, 32 * mf::kManyWarps, mf::kManyWarps * smem, static_cast<cudaStream_t>(stream)>>>(*a);
+  } else {
+    mf::dispatch_push_kernel<<<a->C, threads, smem, static_cast<cudaStream_t>(stream)>>>(*a);
+  }
   return (int)cudaGetLastError();
 }
