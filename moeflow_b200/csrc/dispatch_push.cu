@@ -153,10 +153,10 @@ __global__ void __launch_bounds__(kDispatchThreads) dispatch_push_kernel(const m
   }
 }
 
-// The same for prefill sizes (from 1024 token positions, up to 32 ranks): a warp per token and four of them per CTA, with
+// The same for prefill sizes (from 512 token positions, up to 32 ranks): a warp per token and four of them per CTA, with
 // nothing shared between them but the arrival.  With a CTA per token three of its four warps waited for the one that
 // routes, in 3.5 waves of CTAs at 8192 tokens; a quarter of the CTAs also means a quarter of the fences and arrivals.
-// Kernel at 8192 tokens 74 / 53 us, at 2000 21 / 14.
+// Kernel at 8192 tokens 74 / 53 us, at 2000 21 / 14, at 600 19 / 12.
 constexpr int kManyWarps = 4;
 
 __global__ void __launch_bounds__(32 * kManyWarps) dispatch_push_many_kernel(const mf_dispatch_args a) {
@@ -391,7 +391,7 @@ extern "C" int mf_dispatch_push(const mf_dispatch_args* a, mf_stream_t stream) {
     smem = 2 * (size_t)a->E * sizeof(float);
     if (smem > 40 * 1024) return -3;
   }
-  if (a->C >= 1024 && a->R <= 32 && mf::kManyWarps * smem <= 40 * 1024) {
+  if (a->C >= 512 && a->R <= 32 && mf::kManyWarps * smem <= 40 * 1024) {
     const int ctas = (a->C + mf::kManyWarps - 1) / mf::kManyWarps;
     mf::dispatch_push_many_kernel<<<ctas, 32 * mf::kManyWarps, mf::kManyWarps * smem, static_cast<cudaStream_t>(stream)>>>(*a);
   } else {

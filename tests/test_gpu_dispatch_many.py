@@ -12,7 +12,7 @@ pytestmark = pytest.mark.gpu
 
 @pytest.mark.parametrize("routed", [False, True])
 @pytest.mark.parametrize("world,capacity,tokens,valid,hidden,experts,top_k", [
-    (1, 1024, 1024, None, 512, 12, 4), (1, 1027, 1027, 1000, 256, 36, 8), (2, 1025, 900, None, 4096, 12, 3),
+    (1, 1024, 1024, None, 512, 12, 4), (2, 514, 500, None, 512, 12, 4), (1, 1027, 1027, 1000, 256, 36, 8), (2, 1025, 900, None, 4096, 12, 3),
     (3, 1026, 1026, 1, 384, 288, 8), (1, 1030, 1030, None, 6400, 600, 2)])
 def test_rows_stored_at_prefill_sizes(routed, world, capacity, tokens, valid, hidden, experts, top_k):
     from moeflow_b200.fixed import FixedEPLayer
