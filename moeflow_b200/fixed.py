@@ -511,7 +511,7 @@ class FixedEPLayer:
             n_counters2=self._counters2.numel(), block_m=self.block_m, max_tiles=self.max_tiles, m_blocks1=mb1,
             k_blocks1=H // 64, m_blocks2=mb2, k_blocks2=I // 64, n_sms=self.n_sms,
             max_split_slots=self.max_split_slots, status=self.status.data_ptr(), wait_ns=self.wait_ns,
-            partial_floats=partial_floats, stream_k=int(self.gemm_kwargs.get("stream_k", 0)),
+            partial_floats=partial_floats, split_min_kb=16, stream_k=int(self.gemm_kwargs.get("stream_k", 0)),
             # The metadata kernel is launched without programmatic serialization: started early, in the shadow of the
             # dispatch kernel, its phases after the wait ran three times slower (measured on B200: 18 us against
             # 8 us from dispatch end to plan), which cost more than the microsecond of launch latency it hid.  The
@@ -787,6 +787,7 @@ class FixedEPLayer:
         f["a1"].w_scale, f["a2"].w_scale = pack["s13"].data_ptr(), pack["s2"].data_ptr()
         f["tm13"], f["tm2"], f["pack"] = pack["tm13"], pack["tm2"], pack
         self._fp8 = f
+        self._a_meta.split_kb = 8  # split_cost in csrc/expert_meta.cuh has the figures
         self._a_meta.k_step = 2  # the e4m3 kernels' K blocks hold 128 values: no split between two halves of one
         if self.block_m == 128:  # their units of the down GEMM cover two weight blocks
             self._a_meta.pair2, self._a_meta.m_blocks2 = 1, (self.H // 128 + 1) // 2
@@ -817,7 +818,7 @@ class FixedEPLayer:
     def _bind_bf16(self) -> None:
         self._fp8 = self._expand = None
         self._a_meta.xq = self._a_meta.xs = None
-        self._a_meta.k_step = 1
+        self._a_meta.k_step = self._a_meta.split_kb = 1
         self._a_meta.pair2, self._a_meta.m_blocks2 = int(self.down_two_blocks), self._a_gemm2.m_blocks
 
     def _cuda_dispatch(self, x, weights, ids, num_valid, logits=None, bias=None, whole: bool = False) -> tuple[torch.Tensor, bool]:
