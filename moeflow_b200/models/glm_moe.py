@@ -67,14 +67,13 @@ class SharedExpert:
         self.status = torch.zeros(1, dtype=torch.int64, device=dev)
         self._gate_up = DenseProjection(self.w13, gate_up=True, limit=limit, status=self.status)
         self._down = DenseProjection(self.w2, status=self.status)
-        self._branch = torch.cuda.Stream(device=dev)  # used while a graph is captured, see begin()
 
-    def begin(self, x: torch.Tensor) -> None:
-        """The gate/up half of ``add_to(x, ..., begun=True)`` on a branch of the graph that is being captured: next to the
+    def begin(self, x: torch.Tensor, branch: torch.cuda.Stream) -> None:
+        """The gate/up half of ``add_to(x, ..., begun=branch)`` on a branch of the graph that is being captured: next to the
         router, the dispatch and the start of the routed experts, which leave most SMs idle, instead of behind the routed
-        experts (where it took 20 us of a decode layer)."""
-        self._branch.wait_stream(torch.cuda.current_stream())
-        with torch.cuda.stream(self._branch):
+        experts (12 us of a decode layer)."""
+        branch.wait_stream(torch.cuda.current_stream())
+        with torch.cuda.stream(branch):
             self._gate_up(x, self.act)
 
     def __call__(self, x: torch.Tensor) -> torch.Tensor:
@@ -84,11 +83,12 @@ class SharedExpert:
         return self._down(self._gate_up(x, self.act), self.out)
 
     def add_to(self, x: torch.Tensor, first: torch.Tensor, second: torch.Tensor, out: torch.Tensor,
-               begun: bool = False) -> torch.Tensor:
+               begun: torch.cuda.Stream | None = None) -> torch.Tensor:
         """``out = (first + second) + self(x)``, rounded to bf16 after every addition; the down projection adds (two
-        element-wise launches less per layer).  ``begun``: ``begin(x)`` has launched the first half.  cuda path only."""
-        if begun:
-            torch.cuda.current_stream().wait_stream(self._branch)
+        element-wise launches less per layer).  ``begun``: ``begin(x, begun)`` has launched the first half.  cuda path
+        only."""
+        if begun is not None:
+            torch.cuda.current_stream().wait_stream(begun)
             return self._down(self.act[: x.shape[0]], out, first, second)
         return self._down(self._gate_up(x, self.act), out, first, second)
 
@@ -120,9 +120,11 @@ class MoEBlock:
     """Pre-norm MoE block: ``x + routed(norm(x)) + shared(norm(x))``."""
 
     def __init__(self, cfg: MoEConfig, routed: FixedEPLayer, gate_w: torch.Tensor, bias: torch.Tensor | None,
-                 norm_w: torch.Tensor, shared: SharedExpert | None, eps: float = 1e-6, router: RouterLogits | None = None):
+                 norm_w: torch.Tensor, shared: SharedExpert | None, eps: float = 1e-6, router: RouterLogits | None = None,
+                 branch: torch.cuda.Stream | None = None):
+        """``branch``: a stream that captured calls may put the shared expert's first half on."""
         self.cfg, self.routed, self.gate_w, self.bias, self.norm_w, self.shared, self.eps = cfg, routed, gate_w, bias, norm_w, shared, eps
-        self.router = router
+        self.router, self.branch = router, branch
 
     def __call__(self, x: torch.Tensor, num_valid: torch.Tensor | None = None, add: torch.Tensor | None = None,
                  out: torch.Tensor | None = None) -> torch.Tensor:
@@ -137,15 +139,16 @@ class MoEBlock:
             h = _rmsnorm(x, self.norm_w, self.eps)
         fused = self.shared is not None and self.shared.cuda and x.dtype == torch.bfloat16
         # only in a graph, where a branch costs the host nothing per step
-        begun = fused and self.routed.backend == "cuda" and torch.cuda.is_current_stream_capturing()
-        if begun:
-            self.shared.begin(h)
+        capturing = fused and self.branch is not None and self.routed.backend == "cuda" and torch.cuda.is_current_stream_capturing()
+        begun = self.branch if capturing else None
+        if begun is not None:
+            self.shared.begin(h, begun)
         if self.router is not None:
             logits = self.router(h)
         else:
             logits = torch.matmul(h.to(self.gate_w.dtype), self.gate_w.transpose(0, 1)).to(torch.float32)
         routed = self.routed.forward(h, logits, self.bias, num_valid)[: x.shape[0]]
-        if begun or (fused and routed.dtype == torch.bfloat16):
+        if begun is not None or (fused and routed.dtype == torch.bfloat16):
             return self.shared.add_to(h, x, routed, torch.empty_like(h) if out is None else out, begun)
         y = x + routed
         if self.shared is not None:
@@ -271,6 +274,7 @@ class DecodeModel:
         self.pos = torch.zeros((), dtype=torch.int64, device=dev)
         self.mask = torch.full((1, 1, 1, self.acfg.max_seq), float("-inf"), dtype=torch.bfloat16, device=dev)
         self.graph: torch.cuda.CUDAGraph | None = None
+        self._side: torch.cuda.Stream | None = None  # warm-up before a capture, branches in it
 
     def prefill_standin(self, length: int) -> None:
         for i, layer in enumerate(self.layers):
@@ -289,7 +293,7 @@ class DecodeModel:
             else:
                 self.routed.bind_weights(layer["w13"], layer["w2"], *layer["maps"])
             block = MoEBlock(self.cfg, self.routed, layer["gate_w"], layer["bias"], layer["norm_w"], layer["shared"],
-                             router=layer["router"])
+                             router=layer["router"], branch=self._side)
             x = block(x, add=delta, out=self.out if i == len(self.layers) - 1 else None)
         if not self.layers:
             self.out.copy_(x)
@@ -301,7 +305,7 @@ class DecodeModel:
     def capture(self) -> "DecodeModel":
         import torch.distributed as dist
 
-        side = torch.cuda.Stream(device=self.device)
+        side = self._side = self._side or torch.cuda.Stream(device=self.device)
         side.wait_stream(torch.cuda.current_stream())
         with torch.cuda.stream(side):
             self._forward()

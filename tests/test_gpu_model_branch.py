@@ -23,7 +23,7 @@ def test_captured_block_equals_the_eager_one(tokens):
     shared = SharedExpert((torch.randn(512, 512, generator=gen) * 2 / 512**0.5).bfloat16().cuda(),
                           (torch.randn(512, 256, generator=gen) / 16).bfloat16().cuda(), tokens, cfg.swiglu_limit)
     block = MoEBlock(cfg, layer, gate, make_bias(cfg, 1, device="cuda"), torch.ones(512, dtype=torch.bfloat16, device="cuda"), shared,
-                     router=RouterLogits(gate, tokens))
+                     router=RouterLogits(gate, tokens), branch=torch.cuda.Stream())
     x = torch.zeros(tokens, 512, dtype=torch.bfloat16, device="cuda")
     out = torch.empty_like(x)
     block(x, out=out)
