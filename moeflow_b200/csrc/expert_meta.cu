@@ -510,12 +510,11 @@ extern "C" int mf_plan_split(int units, int k_blocks, int n_sms, int max_slots, 
 }
 
 extern "C" int mf_plan_split_steps(int units, int k_blocks, int k_step, int n_sms, int max_slots, int overhead_kb, int cols) {
-  return mf_plan_split_costs(units, k_blocks, k_step, n_sms, max_slots, overhead_kb, cols, 1, 0);
+  return mf_plan_split_costs(units, k_blocks, k_step, n_sms, max_slots, overhead_kb, cols, 1);
 }
 
-extern "C" int mf_plan_split_costs(int units, int k_blocks, int k_step, int n_sms, int max_slots, int overhead_kb, int cols, int split_kb,
-                                   int min_kb) {
-  return mf::choose_split(units, k_blocks, k_step, n_sms, max_slots, overhead_kb, cols, mf::SplitCosts{split_kb, min_kb});
+extern "C" int mf_plan_split_costs(int units, int k_blocks, int k_step, int n_sms, int max_slots, int overhead_kb, int cols, int split_kb) {
+  return mf::choose_split(units, k_blocks, k_step, n_sms, max_slots, overhead_kb, cols, split_kb);
 }
 
 extern "C" int mf_expert_meta(const mf_meta_args* a, mf_stream_t stream) {

@@ -64,34 +64,32 @@ __device__ __forceinline__ void clear_counters(const mf_meta_args& a, int n_tile
 // the kernel takes ceil(units * S / SMs) rounds of such units.  K is cut between steps of k_step blocks: the e4m3 kernels
 // work on K blocks of 128 values (k_step 2) and refuse a split that does not divide those.  units * 8 fits 32 bits (16
 // million token tiles of 32 weight blocks).
-// What a cut unit costs more (split_kb blocks) and from how many blocks on units are cut at all (min_kb) depends on the
-// kernels.  Measured, us per layer, split_kb 1 / 8: e4m3, 288 experts, 1 token 75 / 65, 4 tokens 142 / 123, 8 tokens 221 / 200
-// (their blocks are half as long, and the fix-up is exposed); bf16, 1 token 78 / 82, elsewhere the same.  Hidden 512 (8 blocks),
-// cut / whole: 1 token 28.3 / 26.9, 8 tokens 32.0 / 28.5: the round trip takes longer than what is left of the stream.
+// What a cut unit costs more (split_kb blocks) depends on the kernels.  Measured, us per layer, split_kb 1 / 8: e4m3, 288 experts, 1 token 75 / 65, 4 tokens 142 / 123, 8 tokens 221 / 200
+// (their blocks are half as long, and the fix-up is exposed); bf16, 1 token 78 / 82, elsewhere the same.  Units of fewer than 16
+// blocks are not cut (hidden 512, 8 blocks, cut / whole: 1 token 28.3 / 26.9, 8 tokens 32.0 / 28.5): the round trip takes longer
+// than what it saves of the stream.  One to three units on the whole chip are, as they always were.
 constexpr long long kNoSplit = 0x7fffffffffffffffll;
-struct SplitCosts {
-  int split_kb, min_kb;
-};
+constexpr int kMinCutBlocks = 16, kMinCutUnits = 4;
 __host__ __device__ __forceinline__ long long split_cost(int log_s, int units, int k_blocks, int k_step, int n_sms, int max_slots,
-                                                         int overhead_kb, int cols, SplitCosts c) {
+                                                         int overhead_kb, int cols, int split_kb) {
   const int s = 1 << log_s;
   const int rounds = (int)(((unsigned)units * (unsigned)s + (unsigned)n_sms - 1u) / (unsigned)n_sms);
   if (s == 1) return (long long)rounds * (k_blocks + overhead_kb);
-  if (k_blocks < c.min_kb || (k_blocks & (s * k_step - 1)) != 0 || (k_blocks >> log_s) < 2 || (long long)units * s > max_slots) return kNoSplit;
+  if ((k_blocks < kMinCutBlocks && units >= kMinCutUnits) || (k_blocks & (s * k_step - 1)) != 0 || (k_blocks >> log_s) < 2 || (long long)units * s > max_slots) return kNoSplit;
   // the partial-sum round trip of a split unit grows with the tile's token columns (measured: splitting
   // 64-column tiles in two cost more than the idle SMs of an uneven last round)
   const int wide = cols > 16 ? (cols - 16) / 8 : 0;
-  return (long long)rounds * ((k_blocks >> log_s) + overhead_kb + c.split_kb + wide);
+  return (long long)rounds * ((k_blocks >> log_s) + overhead_kb + split_kb + wide);
 }
 
 // The cheapest of the splits 1, 2, 4, 8; ties go to the smaller one.
 __host__ __device__ __forceinline__ int choose_split(int units, int k_blocks, int k_step, int n_sms, int max_slots,
-                                                     int overhead_kb, int cols, SplitCosts c) {
+                                                     int overhead_kb, int cols, int split_kb) {
   if (units <= 0) return 1;
   int best = 0;
-  long long best_cost = split_cost(0, units, k_blocks, k_step, n_sms, max_slots, overhead_kb, cols, c);
+  long long best_cost = split_cost(0, units, k_blocks, k_step, n_sms, max_slots, overhead_kb, cols, split_kb);
   for (int log_s = 1; log_s < 4; ++log_s) {
-    const long long cost = split_cost(log_s, units, k_blocks, k_step, n_sms, max_slots, overhead_kb, cols, c);
+    const long long cost = split_cost(log_s, units, k_blocks, k_step, n_sms, max_slots, overhead_kb, cols, split_kb);
     if (cost < best_cost) {
       best_cost = cost;
       best = log_s;
@@ -102,7 +100,7 @@ __host__ __device__ __forceinline__ int choose_split(int units, int k_blocks, in
 
 // K steps of the bound experts' kernels, in blocks of 64 values (1 unless the caller says 2).
 __device__ __forceinline__ int k_step_of(const mf_meta_args& a) { return a.k_step == 2 ? 2 : 1; }
-__device__ __forceinline__ SplitCosts split_costs_of(const mf_meta_args& a) { return SplitCosts{a.split_kb > 0 ? a.split_kb : 1, a.split_min_kb}; }
+__device__ __forceinline__ int split_kb_of(const mf_meta_args& a) { return a.split_kb > 0 ? a.split_kb : 1; }
 
 // The K cut of one GEMM: stream-K (0) when asked for, the units do not fill many rounds of the persistent CTAs
 // (below 8 units per CTA an uneven last round costs more than the partial tiles of the cut units) and the
@@ -110,7 +108,7 @@ __device__ __forceinline__ SplitCosts split_costs_of(const mf_meta_args& a) { re
 __device__ __forceinline__ int choose_cut(const mf_meta_args& a, int units, int k_blocks, int slots, int overhead_kb,
                                           int cols) {
   if (a.stream_k && units > 0 && units < 8 * a.n_sms && units % a.n_sms != 0 && slots >= 2 * a.n_sms) return 0;
-  return choose_split(units, k_blocks, k_step_of(a), a.n_sms, slots, overhead_kb, cols, split_costs_of(a));
+  return choose_split(units, k_blocks, k_step_of(a), a.n_sms, slots, overhead_kb, cols, split_kb_of(a));
 }
 
 // The same choice by the four lanes of a group (lane & 3 = log2 of the split it weighs; the whole warp calls): the splits
@@ -118,7 +116,7 @@ __device__ __forceinline__ int choose_cut(const mf_meta_args& a, int units, int 
 // wait for.
 __device__ __forceinline__ int choose_cut_lanes(const mf_meta_args& a, int units, int k_blocks, int slots, int overhead_kb,
                                                 int cols, int log_s) {
-  const long long cost = split_cost(log_s, units, k_blocks, k_step_of(a), a.n_sms, slots, overhead_kb, cols, split_costs_of(a));
+  const long long cost = split_cost(log_s, units, k_blocks, k_step_of(a), a.n_sms, slots, overhead_kb, cols, split_kb_of(a));
   long long key = cost != kNoSplit ? cost * 4 + log_s : kNoSplit;  // ties go to the smaller split
 #pragma unroll
   for (int off = 1; off < 4; off <<= 1) {

@@ -269,7 +269,6 @@ typedef struct {
   float* xs;                 // [rows, H / 128]
   int k_step;                // K blocks of 64 values per K step of the GEMMs the plan is for: 2 for the e4m3 kernels, else 1
   int split_kb;              // what a cut unit costs more than a whole one, in K blocks of 64 values of streaming (0: 1)
-  int split_min_kb;          // units of fewer K blocks are not cut
   int pair2;                 // 1: a unit of the down GEMM has two accumulators (m_blocks2 counts pairs of weight blocks)
 } mf_meta_args;
 int mf_expert_meta(const mf_meta_args* args, mf_stream_t stream);
@@ -282,9 +281,8 @@ int mf_dispatch_local(const mf_dispatch_args* args, const mf_meta_args* meta, mf
 int mf_plan_split(int units, int k_blocks, int n_sms, int max_slots, int overhead_kb, int cols);
 // The same with K cut only between steps of k_step (1 or 2) blocks of 64 values (mf_meta_args.k_step).
 int mf_plan_split_steps(int units, int k_blocks, int k_step, int n_sms, int max_slots, int overhead_kb, int cols);
-// The same with the cost of a cut unit and the shortest unit that is cut (mf_meta_args.split_kb, split_min_kb; 1 and 0 above).
-int mf_plan_split_costs(int units, int k_blocks, int k_step, int n_sms, int max_slots, int overhead_kb, int cols, int split_kb,
-                        int min_kb);
+// The same with the cost of a cut unit (mf_meta_args.split_kb; 1 above).
+int mf_plan_split_costs(int units, int k_blocks, int k_step, int n_sms, int max_slots, int overhead_kb, int cols, int split_kb);
 
 // ---- owner reduce + return push, combine -------------------------------------------------------------
 typedef struct {

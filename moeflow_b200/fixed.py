@@ -511,7 +511,7 @@ class FixedEPLayer:
             n_counters2=self._counters2.numel(), block_m=self.block_m, max_tiles=self.max_tiles, m_blocks1=mb1,
             k_blocks1=H // 64, m_blocks2=mb2, k_blocks2=I // 64, n_sms=self.n_sms,
             max_split_slots=self.max_split_slots, status=self.status.data_ptr(), wait_ns=self.wait_ns,
-            partial_floats=partial_floats, split_min_kb=16, stream_k=int(self.gemm_kwargs.get("stream_k", 0)),
+            partial_floats=partial_floats, stream_k=int(self.gemm_kwargs.get("stream_k", 0)),
             # The metadata kernel is launched without programmatic serialization: started early, in the shadow of the
             # dispatch kernel, its phases after the wait ran three times slower (measured on B200: 18 us against
             # 8 us from dispatch end to plan), which cost more than the microsecond of launch latency it hid.  The
@@ -696,9 +696,9 @@ class FixedEPLayer:
         pack = {"w13": w13_q.contiguous(), "w2": w2_q.contiguous(), "s13": w13_s.to(torch.float32).contiguous(),
                 "s2": w2_s.to(torch.float32).contiguous()}
         if self.block_m > 128:
-            # Long-prefill layers (256-row token tiles): the block-scaled kernels take tiles of up to 128 rows and are
-            # bound by their per-K-block promotion there, so every forward expands the bound experts into a bf16
-            # scratch (shared by all layers of this shape on the device) and runs the bf16 kernels on it.
+            # Long-prefill layers (256-row token tiles): the block-scaled kernels take tiles of up to 128 rows, so every
+            # forward expands the bound experts into a bf16 scratch (shared by all layers of this shape on the device) and
+            # runs the bf16 kernels on it; the activations are not quantised.
             pack["expand"] = True
             return pack
         pack["tm13"] = make_weight_tmap(pack["w13"].view(torch.uint8))
@@ -974,7 +974,9 @@ def choose_block_m(capacity: int, top_k: int, local_experts: int, fp8: bool = Fa
     and, at 256 rows, halves the operand bytes per flop that a CTA pulls from L2.
 
     ``fp8``: the layer will hold block-scaled e4m3 experts.  Their kernels take tiles of up to 128 rows, and 256-row tiles
-    mean expanding the experts to bf16 in every forward, which pays from about 512 expected rows per expert on.  64 / 128
+    mean expanding the experts to bf16 in every forward, from 512 expected rows per expert on.  (Below that line the e4m3
+    kernels are the faster ones, 600 against about 950 us at 450 rows.  Above it they would be too by now, but an expanded
+    layer keeps its activations in bf16, and its results would lose that precision.)  64 / 128
     rows: 144 experts of 2048, 44 rows 814 / 728, 55 rows 902 / 759; 72 experts, 28 rows 355 / 368 (zipf popularity 206 / 154),
     40 rows 315 / 297, 50 rows 348 / 306; 36 experts, 28 rows (zipf) 104 / 106, 40 rows 167 / 174, 56 rows 194 / 180, 78 rows
     262 / 215.  Layers with few experts have fewer units than CTAs want at 128 rows, so their line lies higher.

@@ -192,7 +192,6 @@ class MetaArgs(C.Structure):
         ("xs", C.c_void_p),
         ("k_step", C.c_int),
         ("split_kb", C.c_int),
-        ("split_min_kb", C.c_int),
         ("pair2", C.c_int),
     ]
 
@@ -283,7 +282,7 @@ def lib() -> C.CDLL:
         "mf_expert_meta": [C.POINTER(MetaArgs), P],
         "mf_plan_split": [I, I, I, I, I, I],
         "mf_plan_split_steps": [I, I, I, I, I, I, I],
-        "mf_plan_split_costs": [I, I, I, I, I, I, I, I, I],
+        "mf_plan_split_costs": [I, I, I, I, I, I, I, I],
         "mf_permute_rows": [P, LL, P, P, P, I, I, I, P],
         "mf_owner_reduce_push": [C.POINTER(ReducePushArgs), P],
         "mf_combine": [C.POINTER(CombineArgs), P],
