@@ -44,7 +44,12 @@
 
 namespace mf {
 
-constexpr int kF8Gather = 32;  // one warp gathers, the other one fills the tables: 12 warps keep 168 registers each
+// Gather threads: warp 2, or four warps of their own (12-15) in the gate/up GEMM of 64-row tiles, where one warp's 16 copy
+// instructions per K block (about 90 cycles each) took longer than the K block's promotion and its weights.  The promotion
+// warps then take the registers that the others give up.  Layer, us: 1 token on 288 experts 64.6 / 61.8, 250 on 72 351 / 346, 64
+// sequences of the decode model 262 / 256.  The split: 88 x 128 + 192 x 256 + 40 x 128 = 65536, what 512 threads start with.
+template <bool kGateUp, int N_MAX>
+constexpr bool kF8FourGather = kGateUp && N_MAX == 64;
 constexpr int kF8Tables = 2;   // scale tables: the unit being promoted and the prefetched next one
 constexpr int kF8Stage = 1024;  // per promotion warp: 16 token columns x 32 outputs of the epilogue, transposed
 
@@ -58,7 +63,9 @@ struct F8Cfg {
   static constexpr int kGroups = N_MAX > 32 ? 2 : 1;
   static constexpr int kCols = N_MAX / kGroups;
   static constexpr int kPromo = 4 * kGroups;             // promotion warps: 4 .. 4 + kPromo - 1
-  static constexpr int kThreads = 128 + 32 * kPromo;
+  static constexpr bool kFourGather = kF8FourGather<kGateUp, N_MAX>;
+  static constexpr int kGather = kFourGather ? 128 : 32;  // threads
+  static constexpr int kThreads = 128 + 32 * kPromo + (kFourGather ? 128 : 0);
   static constexpr int kTableFloats = N_MAX * kF8MaxKb + 2 * kF8MaxKb;  // x scales [kb][n], weight scales [2][kb]
   static constexpr int kTableBytes = kF8Tables * kTableFloats * 4;
   static constexpr int kBarrierBytes = 1024;             // barriers and the segment ring
@@ -109,7 +116,7 @@ grouped_gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid
   const bool b_tma = a.b_tmap != nullptr;  // token tiles by TMA (contiguous rows) instead of the 16-byte gather
   if (tid == 0) {
     for (int s = 0; s < STAGES; ++s) {
-      mbar_init(&full_bar[s], b_tma ? 2 : 1 + kF8Gather);
+      mbar_init(&full_bar[s], b_tma ? 2 : 1 + Cfg::kGather);
       mbar_init(&empty_bar[s], 1);
     }
     for (int s = 0; s < Cfg::kTmpStages; ++s) {
@@ -122,7 +129,7 @@ grouped_gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid
     }
     for (int s = 0; s < GROUPS; ++s) mbar_init(&grp_bar[s], 4);
     for (int s = 0; s < 2; ++s) mbar_init(&epi_bar[s], PROMO_WARPS);
-    ring->init(3 + PROMO_WARPS);  // UMMA, token producer, table warp, promotion warps
+    ring->init(2 + (b_tma ? 1 : Cfg::kGather / 32) + PROMO_WARPS);  // UMMA, table warp, token producers, promotion warps
     *abort_flag = 0;
     fence_mbar_init();
     tma_prefetch_desc(&tmap_w);
@@ -185,259 +192,305 @@ grouped_gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid
   };
   SegReader reader(ring, abort_flag, wait_ns);
 
-  if (warp == 0) {
-    // ---------------------------------------------------------------- weight TMA producer, hands out the segments
-    F8Pipe st;
-    bool ok = true;
-    SegFeed feed(work, ring, abort_flag, wait_ns);
-    const uint64_t policy = N_MAX <= 64 ? l2_evict_first() : l2_evict_normal();  // as in grouped_gemm_tc.cu
-    Seg sg;
-    bool have = feed.first(sg);
-    while (ok && have) {
-      const int row0 = sg.e * a.rows_per_expert + sg.mb * kF8BlockM;
-      for (int j = 0; j < sg.nkb; ++j) {
-        const int kb = sg.kb0 + j;
-        ok = __all_sync(0xffffffffu, mbar_wait_bounded(&empty_bar[st.stage], st.phase ^ 1u, abort_flag, wait_ns));
-        if (!ok) {
-          if (lane == 0) report_status(a.status, kGemmEmptyTimeout, 0, blockIdx.x, 0);
-          break;
-        }
-        if (lane == 0) {
-          mbar_arrive_expect_tx(&full_bar[st.stage], Cfg::kStageA);
-          uint8_t* dst = sA + st.stage * Cfg::kStageA;
-          tma_load_2d(dst, &tmap_w, &full_bar[st.stage], kb * 128, row0, policy);
-          if (kGateUp) tma_load_2d(dst + kF8TileA, &tmap_w, &full_bar[st.stage], kb * 128, row0 + a.up_row_offset, policy);
-        }
-        __syncwarp();
-        st.advance(STAGES);
-        feed.advance();
-      }
-      if (ok) have = feed.next(sg);
-    }
-    if (feed.bad_tile && lane == 0) report_status(a.status, kBadArgument, 7, blockIdx.x, 0);
-    if (!ok) {
-      const unsigned long long t0 = global_timer_ns();
-      while (global_timer_ns() - t0 < 100000ull) __nanosleep(1000);
-    }
-  } else if (warp == 1) {
-    // ---------------------------------------------------------------- UMMA issuer (one K block per tmp stage)
-    F8Pipe st, tmp;
-    bool ok = true;
-    Seg sg;
-    while (ok && reader.next(sg, ok)) {
-      uint32_t n_tile = (uint32_t)((sg.n_rows + 15) & ~15);
-      if (n_tile < 16) n_tile = 16;
-      const uint32_t idesc = umma_idesc(0, 0, kF8BlockM, n_tile);  // e4m3 x e4m3 -> fp32
-      for (int j = 0; j < sg.nkb; ++j) {
-        ok = __all_sync(0xffffffffu, mbar_wait_bounded(&tmp_empty[tmp.stage], tmp.phase ^ 1u, abort_flag, wait_ns));
-        if (!ok) {
-          if (lane == 0) report_status(a.status, kGemmAccTimeout, 1, blockIdx.x, 0);
-          break;
-        }
-        ok = __all_sync(0xffffffffu, mbar_wait_bounded(&full_bar[st.stage], st.phase, abort_flag, wait_ns));
-        if (!ok) {
-          if (lane == 0) report_status(a.status, kGemmFullTimeout, 1, blockIdx.x, 0);
-          break;
-        }
-        tc_fence_after_sync();
-        if (lane == 0) {
-          fence_proxy_async_smem();
-          const uint32_t d0 = tmem_base + tmp.stage * Cfg::kTmpCols;
-          const uint32_t a_addr = smem_u32(sA + st.stage * Cfg::kStageA);
-          const uint32_t b_addr = smem_u32(sB + st.stage * Cfg::kStageB);
-#pragma unroll
-          for (int k = 0; k < 4; ++k) {
-            const uint64_t bdesc = umma_desc_sw128(b_addr + k * 32);
-            umma_f8(d0, umma_desc_sw128(a_addr + k * 32), bdesc, idesc, k > 0 ? 1u : 0u);
-            if (kGateUp) umma_f8(d0 + N_MAX, umma_desc_sw128(a_addr + kF8TileA + k * 32), bdesc, idesc, k > 0 ? 1u : 0u);
+  // (The register split stands at the head of each warpgroup's branch: in front of a common join the compiler keeps everything
+  // behind it within the smallest share.)
+  if (warp < 4) {
+    if (Cfg::kFourGather) asm volatile("setmaxnreg.dec.sync.aligned.u32 88;");
+    if (warp == 0) {
+      // ---------------------------------------------------------------- weight TMA producer, hands out the segments
+      F8Pipe st;
+      bool ok = true;
+      SegFeed feed(work, ring, abort_flag, wait_ns);
+      const uint64_t policy = N_MAX <= 64 ? l2_evict_first() : l2_evict_normal();  // as in grouped_gemm_tc.cu
+      Seg sg;
+      bool have = feed.first(sg);
+      while (ok && have) {
+        const int row0 = sg.e * a.rows_per_expert + sg.mb * kF8BlockM;
+        for (int j = 0; j < sg.nkb; ++j) {
+          const int kb = sg.kb0 + j;
+          ok = __all_sync(0xffffffffu, mbar_wait_bounded(&empty_bar[st.stage], st.phase ^ 1u, abort_flag, wait_ns));
+          if (!ok) {
+            if (lane == 0) report_status(a.status, kGemmEmptyTimeout, 0, blockIdx.x, 0);
+            break;
           }
-          umma_commit(&empty_bar[st.stage]);
-          umma_commit(&tmp_full[tmp.stage]);
+          if (lane == 0) {
+            mbar_arrive_expect_tx(&full_bar[st.stage], Cfg::kStageA);
+            uint8_t* dst = sA + st.stage * Cfg::kStageA;
+            tma_load_2d(dst, &tmap_w, &full_bar[st.stage], kb * 128, row0, policy);
+            if (kGateUp) tma_load_2d(dst + kF8TileA, &tmap_w, &full_bar[st.stage], kb * 128, row0 + a.up_row_offset, policy);
+          }
+          __syncwarp();
+          st.advance(STAGES);
+          feed.advance();
         }
-        __syncwarp();
-        st.advance(STAGES);
-        tmp.advance(Cfg::kTmpStages);
+        if (ok) have = feed.next(sg);
       }
-    }
-  } else if (warp == 2 && b_tma) {
-    // ---------------------------------------------------------------- token-operand producer (TMA)
-    F8Pipe st;
-    bool ok = true;
-    Seg sg;
-    int ready_tile = -1;
-    while (ok && reader.next(sg, ok)) {
-      if (a.tile_wait != nullptr && sg.tt != ready_tile) {
-        ok = tile_ready(sg.tt);
-        if (!ok) break;
-        if (lane == 0) fence_proxy_async_all();  // the TMA reads below come after the acquire
-        ready_tile = sg.tt;
+      if (feed.bad_tile && lane == 0) report_status(a.status, kBadArgument, 7, blockIdx.x, 0);
+      if (!ok) {
+        const unsigned long long t0 = global_timer_ns();
+        while (global_timer_ns() - t0 < 100000ull) __nanosleep(1000);
       }
-      for (int j = 0; j < sg.nkb; ++j) {
-        const int kb = sg.kb0 + j;
-        ok = __all_sync(0xffffffffu, mbar_wait_bounded(&empty_bar[st.stage], st.phase ^ 1u, abort_flag, wait_ns));
-        if (!ok) {
-          if (lane == 0) report_status(a.status, kGemmEmptyTimeout, 2, blockIdx.x, 0);
-          break;
-        }
-        if (lane == 0) {
-          mbar_arrive_expect_tx(&full_bar[st.stage], Cfg::kStageB);
-          tma_load_2d(sB + st.stage * Cfg::kStageB, &tmap_b, &full_bar[st.stage], kb * 128, sg.row_start);
-        }
-        __syncwarp();
-        st.advance(STAGES);
-      }
-    }
-    if (!ok) {
-      const unsigned long long t0 = global_timer_ns();
-      while (global_timer_ns() - t0 < 100000ull) __nanosleep(1000);
-    }
-  } else if (warp == 2) {
-    // ---------------------------------------------------------------- token-operand producer (gathered e4m3 rows)
-    const int r_in = lane >> 3, chunk = lane & 7;  // rows r_in, r_in + 4, ...: two swizzle phases
-    const uint32_t sw_off[2] = {(uint32_t)((chunk ^ r_in) << 4), (uint32_t)((chunk ^ (r_in + 4)) << 4)};
-    F8Pipe st;
-    bool ok = true;
-    Seg sg, nx;
-    int ready_tile = -1;
-    int idx[N_MAX / 4];  // source rows of the segment at hand, fetched during the previous one
-    auto row_indices = [&](const Seg& s_) {
+    } else if (warp == 1) {
+      // ---------------------------------------------------------------- UMMA issuer (one K block per tmp stage)
+      F8Pipe st, tmp;
+      bool ok = true;
+      Seg sg;
+      while (ok && reader.next(sg, ok)) {
+        uint32_t n_tile = (uint32_t)((sg.n_rows + 15) & ~15);
+        if (n_tile < 16) n_tile = 16;
+        const uint32_t idesc = umma_idesc(0, 0, kF8BlockM, n_tile);  // e4m3 x e4m3 -> fp32
+        for (int j = 0; j < sg.nkb; ++j) {
+          ok = __all_sync(0xffffffffu, mbar_wait_bounded(&tmp_empty[tmp.stage], tmp.phase ^ 1u, abort_flag, wait_ns));
+          if (!ok) {
+            if (lane == 0) report_status(a.status, kGemmAccTimeout, 1, blockIdx.x, 0);
+            break;
+          }
+          ok = __all_sync(0xffffffffu, mbar_wait_bounded(&full_bar[st.stage], st.phase, abort_flag, wait_ns));
+          if (!ok) {
+            if (lane == 0) report_status(a.status, kGemmFullTimeout, 1, blockIdx.x, 0);
+            break;
+          }
+          tc_fence_after_sync();
+          if (lane == 0) {
+            fence_proxy_async_smem();
+            const uint32_t d0 = tmem_base + tmp.stage * Cfg::kTmpCols;
+            const uint32_t a_addr = smem_u32(sA + st.stage * Cfg::kStageA);
+            const uint32_t b_addr = smem_u32(sB + st.stage * Cfg::kStageB);
 #pragma unroll
-      for (int i = 0; i < N_MAX / 4; ++i) {
-        const int n = r_in + 4 * i;
-        if (n < s_.n_rows) idx[i] = a.b_index ? __ldcg(a.b_index + s_.row_start + n) : s_.row_start + n;
-      }
-    };
-    bool have = reader.next(sg, ok), more = false;
-    if (have) row_indices(sg);
-    while (ok && have) {
-      if (a.tile_wait != nullptr && sg.tt != ready_tile) {
-        ok = tile_ready(sg.tt);
-        if (!ok) break;
-        ready_tile = sg.tt;
-      }
-      const int n_rows = sg.n_rows;
-      int n_tile = (n_rows + 15) & ~15;
-      if (n_tile < 16) n_tile = 16;
-      const uint8_t* rp[N_MAX / 4];
-#pragma unroll
-      for (int i = 0; i < N_MAX / 4; ++i) {
-        const int n = r_in + 4 * i;
-        rp[i] = n < n_rows ? static_cast<const uint8_t*>(a.b_base) + (long long)idx[i] * a.b_pitch + chunk * 16 : nullptr;
-      }
-      for (int j = 0; j < sg.nkb; ++j) {
-        const int kb = sg.kb0 + j;
-        ok = __all_sync(0xffffffffu, mbar_wait_bounded(&empty_bar[st.stage], st.phase ^ 1u, abort_flag, wait_ns));
-        if (!ok) {
-          if (lane == 0) report_status(a.status, kGemmEmptyTimeout, 2, blockIdx.x, 0);
-          break;
+            for (int k = 0; k < 4; ++k) {
+              const uint64_t bdesc = umma_desc_sw128(b_addr + k * 32);
+              umma_f8(d0, umma_desc_sw128(a_addr + k * 32), bdesc, idesc, k > 0 ? 1u : 0u);
+              if (kGateUp) umma_f8(d0 + N_MAX, umma_desc_sw128(a_addr + kF8TileA + k * 32), bdesc, idesc, k > 0 ? 1u : 0u);
+            }
+            umma_commit(&empty_bar[st.stage]);
+            umma_commit(&tmp_full[tmp.stage]);
+          }
+          __syncwarp();
+          st.advance(STAGES);
+          tmp.advance(Cfg::kTmpStages);
         }
-        const uint32_t b_stage = smem_u32(sB + st.stage * Cfg::kStageB);
+      }
+    } else if (warp == 2 && b_tma) {
+      // ---------------------------------------------------------------- token-operand producer (TMA)
+      F8Pipe st;
+      bool ok = true;
+      Seg sg;
+      int ready_tile = -1;
+      while (ok && reader.next(sg, ok)) {
+        if (a.tile_wait != nullptr && sg.tt != ready_tile) {
+          ok = tile_ready(sg.tt);
+          if (!ok) break;
+          if (lane == 0) fence_proxy_async_all();  // the TMA reads below come after the acquire
+          ready_tile = sg.tt;
+        }
+        for (int j = 0; j < sg.nkb; ++j) {
+          const int kb = sg.kb0 + j;
+          ok = __all_sync(0xffffffffu, mbar_wait_bounded(&empty_bar[st.stage], st.phase ^ 1u, abort_flag, wait_ns));
+          if (!ok) {
+            if (lane == 0) report_status(a.status, kGemmEmptyTimeout, 2, blockIdx.x, 0);
+            break;
+          }
+          if (lane == 0) {
+            mbar_arrive_expect_tx(&full_bar[st.stage], Cfg::kStageB);
+            tma_load_2d(sB + st.stage * Cfg::kStageB, &tmap_b, &full_bar[st.stage], kb * 128, sg.row_start);
+          }
+          __syncwarp();
+          st.advance(STAGES);
+        }
+      }
+      if (!ok) {
+        const unsigned long long t0 = global_timer_ns();
+        while (global_timer_ns() - t0 < 100000ull) __nanosleep(1000);
+      }
+    } else if (warp == 2 && Cfg::kFourGather) {
+    } else if (warp == 2) {
+      // ---------------------------------------------------------------- token-operand producer (gathered e4m3 rows)
+      const int r_in = lane >> 3, chunk = lane & 7;  // rows r_in, r_in + 4, ...: two swizzle phases
+      const uint32_t sw_off[2] = {(uint32_t)((chunk ^ r_in) << 4), (uint32_t)((chunk ^ (r_in + 4)) << 4)};
+      F8Pipe st;
+      bool ok = true;
+      Seg sg, nx;
+      int ready_tile = -1;
+      int idx[N_MAX / 4];  // source rows of the segment at hand, fetched during the previous one
+      auto row_indices = [&](const Seg& s_) {
 #pragma unroll
         for (int i = 0; i < N_MAX / 4; ++i) {
           const int n = r_in + 4 * i;
-          if (n < n_tile) {
-            const bool live = rp[i] != nullptr;
-            cp_async_16(b_stage + n * 128 + sw_off[i & 1], live ? (const void*)(rp[i] + (long long)kb * 128) : a.b_base, live ? 16u : 0u);
+          if (n < s_.n_rows) idx[i] = a.b_index ? __ldcg(a.b_index + s_.row_start + n) : s_.row_start + n;
+        }
+      };
+      bool have = reader.next(sg, ok), more = false;
+      if (have) row_indices(sg);
+      while (ok && have) {
+        if (a.tile_wait != nullptr && sg.tt != ready_tile) {
+          ok = tile_ready(sg.tt);
+          if (!ok) break;
+          ready_tile = sg.tt;
+        }
+        const int n_rows = sg.n_rows;
+        int n_tile = (n_rows + 15) & ~15;
+        if (n_tile < 16) n_tile = 16;
+        const uint8_t* rp[N_MAX / 4];
+#pragma unroll
+        for (int i = 0; i < N_MAX / 4; ++i) {
+          const int n = r_in + 4 * i;
+          rp[i] = n < n_rows ? static_cast<const uint8_t*>(a.b_base) + (long long)idx[i] * a.b_pitch + chunk * 16 : nullptr;
+        }
+        for (int j = 0; j < sg.nkb; ++j) {
+          const int kb = sg.kb0 + j;
+          ok = __all_sync(0xffffffffu, mbar_wait_bounded(&empty_bar[st.stage], st.phase ^ 1u, abort_flag, wait_ns));
+          if (!ok) {
+            if (lane == 0) report_status(a.status, kGemmEmptyTimeout, 2, blockIdx.x, 0);
+            break;
+          }
+          const uint32_t b_stage = smem_u32(sB + st.stage * Cfg::kStageB);
+#pragma unroll
+          for (int i = 0; i < N_MAX / 4; ++i) {
+            const int n = r_in + 4 * i;
+            if (n < n_tile) {
+              const bool live = rp[i] != nullptr;
+              cp_async_16(b_stage + n * 128 + sw_off[i & 1], live ? (const void*)(rp[i] + (long long)kb * 128) : a.b_base, live ? 16u : 0u);
+            }
+          }
+          cp_async_mbar_arrive_noinc(&full_bar[st.stage]);
+          st.advance(STAGES);
+          // the producer warp publishes the next segment during the third K block of this one
+          if (j == (sg.nkb < 4 ? sg.nkb - 1 : 3)) {
+            more = reader.next(nx, ok);
+            if (more) row_indices(nx);
+            if (!ok) break;
           }
         }
-        cp_async_mbar_arrive_noinc(&full_bar[st.stage]);
-        st.advance(STAGES);
-        // the producer warp publishes the next segment during the third K block of this one
-        if (j == (sg.nkb < 4 ? sg.nkb - 1 : 3)) {
-          more = reader.next(nx, ok);
-          if (more) row_indices(nx);
-          if (!ok) break;
-        }
+        sg = nx;
+        have = more;
       }
-      sg = nx;
-      have = more;
+      asm volatile("cp.async.wait_all;" ::: "memory");
+    } else if (warp == 3) {
+      // ---------------------------------------------------------------- scale tables (a unit ahead), finished tiles
+      // Table: x scales [j][n] and weight scales [t][j] of a segment, j = kb - kb0.  A lane takes whole token rows: all of a
+      // row's scales are requested before the first one is stored.
+      // Finished tiles: two units behind, the outputs of a whole gate/up unit are fenced and counted for the down GEMM.
+      const int row_blocks = a.rows_per_expert / kF8BlockM;
+      const bool vec = (a.b_scale_pitch & 3) == 0 && (reinterpret_cast<uintptr_t>(a.b_scale) & 15) == 0;
+      const bool report = kGateUp && a.tile_done != nullptr;
+      bool ok = true;
+      Seg sg;
+      int n_it = 0, ready_tile = -1;
+      int done_tile[2] = {-1, -1};  // tiles of the last two units, if this warp has to report them
+      auto report_unit = [&](int k) -> bool {  // unit k of this CTA
+        const bool got = __all_sync(0xffffffffu, mbar_wait_bounded(&epi_bar[k & 1], (uint32_t)(k >> 1) & 1u, abort_flag, wait_ns));
+        const int tt = k & 1 ? done_tile[1] : done_tile[0];
+        if (got && lane == 0 && tt >= 0) {
+          __threadfence();  // the promotion warps' stores (ordered before by the barrier) are visible device-wide
+          atomicAdd(a.tile_done + tt, PROMO_WARPS);
+        }
+        return got;
+      };
+      while (ok && reader.next(sg, ok)) {
+        const int buf = n_it % kF8Tables;
+        float* t = sTable + buf * Cfg::kTableFloats;
+        float wv[kGateUp ? 2 : 1];
+#pragma unroll
+        for (int q = 0; q < (kGateUp ? 2 : 1); ++q) {
+          const int rb = (q == 0 ? 0 : a.up_row_offset / kF8BlockM) + sg.mb;
+          wv[q] = lane < sg.nkb ? __ldcg(a.w_scale + ((long long)sg.e * row_blocks + rb) * a.k_blocks + sg.kb0 + lane) : 0.f;
+        }
+        if (a.tile_wait != nullptr && sg.tt != ready_tile) {
+          ok = tile_ready(sg.tt);
+          if (!ok) break;
+          ready_tile = sg.tt;
+        }
+        if (n_it >= kF8Tables) {
+          ok = __all_sync(0xffffffffu, mbar_wait_bounded(&tbl_free[buf], (uint32_t)(n_it / kF8Tables - 1) & 1u, abort_flag, wait_ns));
+          if (!ok) {
+            if (lane == 0) report_status(a.status, kGemmAccTimeout, 6, blockIdx.x, 0);
+            break;
+          }
+        }
+        int n_tile = (sg.n_rows + 15) & ~15;
+        if (n_tile < 16) n_tile = 16;
+        for (int n = lane; n < n_tile; n += 32) {
+          const bool live = n < sg.n_rows;
+          long long idx = 0;
+          if (live) idx = a.b_index ? (long long)__ldcg(a.b_index + sg.row_start + n) : (long long)(sg.row_start + n);
+          const float* src = a.b_scale + idx * a.b_scale_pitch + sg.kb0;
+          float v[kF8MaxKb];
+          if (vec && ((sg.kb0 | sg.nkb) & 3) == 0) {
+#pragma unroll
+            for (int j = 0; j < kF8MaxKb; j += 4) {
+              float4 f = make_float4(0.f, 0.f, 0.f, 0.f);
+              if (live && j < sg.nkb) f = __ldcg(reinterpret_cast<const float4*>(src + j));
+              v[j] = f.x;
+              v[j + 1] = f.y;
+              v[j + 2] = f.z;
+              v[j + 3] = f.w;
+            }
+          } else {
+#pragma unroll
+            for (int j = 0; j < kF8MaxKb; ++j) v[j] = (live && j < sg.nkb) ? __ldcg(src + j) : 0.f;
+          }
+#pragma unroll
+          for (int j = 0; j < kF8MaxKb; ++j)
+            if (j < sg.nkb) t[j * N_MAX + n] = v[j];
+        }
+#pragma unroll
+        for (int q = 0; q < (kGateUp ? 2 : 1); ++q) t[N_MAX * kF8MaxKb + q * kF8MaxKb + lane] = wv[q];
+        if (report) {
+          // before the table is handed over: with it the promotion warps may come back to the same barrier
+          if (n_it >= 2) ok = report_unit(n_it - 2);
+          if (!ok) break;
+          const int tt = sg.nseg == 1 ? sg.tt : -1;
+          if (n_it & 1) done_tile[1] = tt;
+          else done_tile[0] = tt;
+        }
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&tbl_bar[buf]);
+        ++n_it;
+      }
+      if (report)
+        for (int k = n_it < 2 ? 0 : n_it - 2; ok && k < n_it; ++k) ok = report_unit(k);
     }
-    asm volatile("cp.async.wait_all;" ::: "memory");
-  } else if (warp == 3) {
-    // ---------------------------------------------------------------- scale tables (a unit ahead), finished tiles
-    // Table: x scales [j][n] and weight scales [t][j] of a segment, j = kb - kb0.  A lane takes whole token rows: all of a
-    // row's scales are requested before the first one is stored.
-    // Finished tiles: two units behind, the outputs of a whole gate/up unit are fenced and counted for the down GEMM.
-    const int row_blocks = a.rows_per_expert / kF8BlockM;
-    const bool vec = (a.b_scale_pitch & 3) == 0 && (reinterpret_cast<uintptr_t>(a.b_scale) & 15) == 0;
-    const bool report = kGateUp && a.tile_done != nullptr;
+  } else if (Cfg::kFourGather && warp >= 12) {
+    if (Cfg::kFourGather) asm volatile("setmaxnreg.dec.sync.aligned.u32 40;");
+    // ---------------------------------------------------------------- token-operand producers (gathered e4m3 rows, four warps)
+    const int gt = tid - 384;  // rows gt / 8, + 16, ...; 16-byte chunk gt & 7
+    const int r_in = gt >> 3, chunk = gt & 7;
+    const uint32_t sw_off = (uint32_t)(r_in * 128 + ((chunk ^ (r_in & 7)) << 4));
+    const int pitch16 = (int)(a.b_pitch >> 4);
+    F8Pipe st;
     bool ok = true;
     Seg sg;
-    int n_it = 0, ready_tile = -1;
-    int done_tile[2] = {-1, -1};  // tiles of the last two units, if this warp has to report them
-    auto report_unit = [&](int k) -> bool {  // unit k of this CTA
-      const bool got = __all_sync(0xffffffffu, mbar_wait_bounded(&epi_bar[k & 1], (uint32_t)(k >> 1) & 1u, abort_flag, wait_ns));
-      const int tt = k & 1 ? done_tile[1] : done_tile[0];
-      if (got && lane == 0 && tt >= 0) {
-        __threadfence();  // the promotion warps' stores (ordered before by the barrier) are visible device-wide
-        atomicAdd(a.tile_done + tt, PROMO_WARPS);
-      }
-      return got;
-    };
-    while (ok && reader.next(sg, ok)) {
-      const int buf = n_it % kF8Tables;
-      float* t = sTable + buf * Cfg::kTableFloats;
-      float wv[kGateUp ? 2 : 1];
-#pragma unroll
-      for (int q = 0; q < (kGateUp ? 2 : 1); ++q) {
-        const int rb = (q == 0 ? 0 : a.up_row_offset / kF8BlockM) + sg.mb;
-        wv[q] = lane < sg.nkb ? __ldcg(a.w_scale + ((long long)sg.e * row_blocks + rb) * a.k_blocks + sg.kb0 + lane) : 0.f;
-      }
+    int ready_tile = -1;
+    while (ok && !b_tma && reader.next(sg, ok)) {
       if (a.tile_wait != nullptr && sg.tt != ready_tile) {
         ok = tile_ready(sg.tt);
         if (!ok) break;
         ready_tile = sg.tt;
       }
-      if (n_it >= kF8Tables) {
-        ok = __all_sync(0xffffffffu, mbar_wait_bounded(&tbl_free[buf], (uint32_t)(n_it / kF8Tables - 1) & 1u, abort_flag, wait_ns));
+      int off[N_MAX / 16];  // in 16-byte chunks; rows behind the tile repeat its last one, and nobody looks at their sums
+#pragma unroll
+      for (int i = 0; i < N_MAX / 16; ++i) {
+        const int n = sg.row_start + min(r_in + 16 * i, sg.n_rows - 1);
+        off[i] = (a.b_index ? __ldcg(a.b_index + n) : n) * pitch16 + chunk;
+      }
+      for (int j = 0; j < sg.nkb; ++j) {
+        ok = __all_sync(0xffffffffu, mbar_wait_bounded(&empty_bar[st.stage], st.phase ^ 1u, abort_flag, wait_ns));
         if (!ok) {
-          if (lane == 0) report_status(a.status, kGemmAccTimeout, 6, blockIdx.x, 0);
+          if (lane == 0) report_status(a.status, kGemmEmptyTimeout, 2, blockIdx.x, 0);
           break;
         }
+        const uint32_t dst = smem_u32(sB + st.stage * Cfg::kStageB) + sw_off;
+        const uint4* src = static_cast<const uint4*>(a.b_base) + (sg.kb0 + j) * 8;
+#pragma unroll
+        for (int i = 0; i < N_MAX / 16; ++i)
+          if (16 * i < sg.n_rows) cp_async_16(dst + i * 2048, src + off[i], 16u);
+        cp_async_mbar_arrive_noinc(&full_bar[st.stage]);
+        st.advance(STAGES);
       }
-      int n_tile = (sg.n_rows + 15) & ~15;
-      if (n_tile < 16) n_tile = 16;
-      for (int n = lane; n < n_tile; n += 32) {
-        const bool live = n < sg.n_rows;
-        long long idx = 0;
-        if (live) idx = a.b_index ? (long long)__ldcg(a.b_index + sg.row_start + n) : (long long)(sg.row_start + n);
-        const float* src = a.b_scale + idx * a.b_scale_pitch + sg.kb0;
-        float v[kF8MaxKb];
-        if (vec && ((sg.kb0 | sg.nkb) & 3) == 0) {
-#pragma unroll
-          for (int j = 0; j < kF8MaxKb; j += 4) {
-            float4 f = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (live && j < sg.nkb) f = __ldcg(reinterpret_cast<const float4*>(src + j));
-            v[j] = f.x;
-            v[j + 1] = f.y;
-            v[j + 2] = f.z;
-            v[j + 3] = f.w;
-          }
-        } else {
-#pragma unroll
-          for (int j = 0; j < kF8MaxKb; ++j) v[j] = (live && j < sg.nkb) ? __ldcg(src + j) : 0.f;
-        }
-#pragma unroll
-        for (int j = 0; j < kF8MaxKb; ++j)
-          if (j < sg.nkb) t[j * N_MAX + n] = v[j];
-      }
-#pragma unroll
-      for (int q = 0; q < (kGateUp ? 2 : 1); ++q) t[N_MAX * kF8MaxKb + q * kF8MaxKb + lane] = wv[q];
-      if (report) {
-        // before the table is handed over: with it the promotion warps may come back to the same barrier
-        if (n_it >= 2) ok = report_unit(n_it - 2);
-        if (!ok) break;
-        const int tt = sg.nseg == 1 ? sg.tt : -1;
-        if (n_it & 1) done_tile[1] = tt;
-        else done_tile[0] = tt;
-      }
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&tbl_bar[buf]);
-      ++n_it;
     }
-    if (report)
-      for (int k = n_it < 2 ? 0 : n_it - 2; ok && k < n_it; ++k) ok = report_unit(k);
+    asm volatile("cp.async.wait_all;" ::: "memory");
   } else {
+    if (Cfg::kFourGather) asm volatile("setmaxnreg.inc.sync.aligned.u32 192;");
     // ---------------------------------------------------------------- promotion + epilogue
     const int pw = warp - 4;                 // 0 .. PROMO_WARPS-1
     const int wq = pw & 3;                   // tensor-memory lane quarter
