@@ -26,7 +26,8 @@
 // Warp roles (256 threads, one CTA per SM, persistent):
 //   warp 0      TMA producer for the weight tiles (lane 0 issues); hands the segments out to the other roles
 //   warp 1      UMMA issuer (lane 0 issues); owns the tensor-memory allocation
-//   warps 2-3   token-operand producers: gather rows by index with cp.async into the swizzled tile
+//   warps 2-3   token-operand producers: gather rows by index with cp.async into the swizzled tile (256-row tiles: warps
+//               12-15), or warp 2 alone fetches contiguous rows by TMA
 //   warps 4-7   epilogue: tcgen05.ld -> registers -> activation / scale -> global
 //
 // Replaces the reference's Triton grouped GEMM, unfused SwiGLU and expert-input gather
@@ -51,7 +52,13 @@ constexpr int kThreadsWithReturn = 384;  // + 4 return warps (fused owner reduce
 template <int N_MAX, bool kReturn>
 constexpr int kEpiGroups = (N_MAX >= 256 && !kReturn) ? 2 : 1;
 constexpr int kRetDepth = 4;            // queued unit descriptors per quarter
-constexpr int kGatherThreads = 64;
+// Gather threads: warps 2 and 3, or four warps of their own (12-15) where a 256-row tile has 2048 chunks of 16 bytes per K
+// step; the register split then takes from them and from the first four warps what the epilogue needs beyond 128
+// (72 x 128 + 168 x 256 + 104 x 128 = 65536, what 512 threads are launched with).
+template <bool kGateUp, int N_MAX, bool kReturn>
+constexpr bool kWideGather = kGateUp && N_MAX >= 256 && !kReturn;
+template <bool kGateUp, int N_MAX, bool kReturn>
+constexpr int kLaunchThreads = kReturn ? kThreadsWithReturn : kWideGather<kGateUp, N_MAX, kReturn> ? 512 : 128 + 128 * kEpiGroups<N_MAX, kReturn>;
 constexpr int kMaxAccStages = 2;
 constexpr int kOutStageBytes = 1024;   // 16 token columns x 32 weight rows of 16-bit outputs, per epilogue warp
 constexpr int kMaxDevices = 64;        // devices one process may drive (per-device launch configuration)
@@ -236,12 +243,14 @@ __device__ __forceinline__ void finish_store(const mf_gemm_args& a, float (&v)[C
 }
 
 template <bool kGateUp, int N_MAX, bool kReturn = false>
-__global__ void __launch_bounds__(kReturn ? kThreadsWithReturn : 128 + 128 * kEpiGroups<N_MAX, kReturn>, 1)
+__global__ void __launch_bounds__(kLaunchThreads<kGateUp, N_MAX, kReturn>, 1)
 grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_b,
                     const mf_gemm_args a) {
   using Cfg = GemmCfg<kGateUp, N_MAX>;
   constexpr int STAGES = Cfg::kStages;
   constexpr int kGroups = kEpiGroups<N_MAX, kReturn>;
+  constexpr bool kFourGather = kWideGather<kGateUp, N_MAX, kReturn>;
+  constexpr int kGatherThreads = kFourGather ? 128 : 64, kGatherStep = kGatherThreads / 8;
 
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -301,7 +310,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
       mbar_init(&ret_full[s], 1);
       mbar_init(&ret_empty[s], 1);
     }
-    ring->init(1 + (b_tma ? 1 : 2) + 4 * kGroups);  // UMMA, token producers, epilogue
+    ring->init(1 + (b_tma ? 1 : kGatherThreads / 32) + 4 * kGroups);  // UMMA, token producers, epilogue
     *abort_flag = 0;
     fence_mbar_init();
     tma_prefetch_desc(&tmap_w);
@@ -376,171 +385,20 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
   }
 
   SegReader reader(ring, abort_flag, wait_ns);
-  if (warp == 0) {
-    // ------------------------------------------------------------------ weight TMA producer
-    PipeState st;
-    bool ok = true;
-    SegFeed feed(work, ring, abort_flag, wait_ns);
-    // Tiles of up to 64 rows are decode: an expert usually has one tile, and its weights are then read once per forward.
-    // Skewed routing gives a hot expert several that read the same blocks, but they run close together and most blocks are
-    // still read once: evict-first / normal, us per layer, 1 token 81 / 96, 128 tokens 1325 / 1347 (bf16, 288 experts), 8
-    // tokens e4m3 220 / 241; zipf popularity: 100 tokens on 36 experts bf16 149 / 160, e4m3 113 / 126, 128 on 288 e4m3
-    // 116 / 129, 250 on 72 e4m3 (inter 2048) 223 / 230.
-    const uint64_t policy = N_MAX <= 64 ? l2_evict_first() : l2_evict_normal();
-    Seg sg;
-    bool have = feed.first(sg);
-    while (ok && have) {
-      const int row0 = sg.e * a.rows_per_expert + sg.mb * (a.two_blocks ? 2 * kBlockM : kBlockM);
-      for (int j = 0; j < sg.nkb; ++j) {
-        const int kb = sg.kb0 + j;
-        ok = mbar_wait_bounded(&empty_bar[st.stage], st.phase ^ 1u, abort_flag, wait_ns);
-        ok = __all_sync(0xffffffffu, ok);
-        if (!ok) {
-          if (lane == 0) report_status(a.status, kGemmEmptyTimeout, 0, blockIdx.x, 0);
-          break;
-        }
-        if (lane == 0) {
-          mbar_arrive_expect_tx(&full_bar[st.stage], Cfg::kStageA);
-          uint8_t* dst = sA + st.stage * Cfg::kStageA;
-          if (trace && trace[2] == 0) trace[2] = global_timer_ns();  // see the note at MF_STAMP_ONCE
-          tma_load_2d(dst, &tmap_w, &full_bar[st.stage], kb * 64, row0, policy);
-          if (kGateUp) tma_load_2d(dst + kTileBytesA, &tmap_w, &full_bar[st.stage], kb * 64, row0 + a.up_row_offset, policy);
-        }
-        __syncwarp();
-        st.advance(STAGES);
-        feed.advance();
-      }
-      if (ok) have = feed.next(sg);
-    }
-    if (feed.bad_tile && lane == 0) report_status(a.status, kBadArgument, 7, blockIdx.x, 0);
-    if (!ok) {
-      // Give copies that are still in flight a moment to land before the CTA goes away.
-      const unsigned long long t0 = global_timer_ns();
-      while (global_timer_ns() - t0 < 100000ull) __nanosleep(1000);
-    }
-  } else if (warp == 1) {
-    // ------------------------------------------------------------------ UMMA issuer
-    PipeState st, acc;
-    bool ok = true;
-    Seg sg;
-    while (ok && reader.next(sg, ok)) {
-      const uint32_t n_tile = (uint32_t)((sg.n_rows + 15) & ~15);
-      const uint32_t idesc = umma_idesc(1, 1, kBlockM, n_tile < 16 ? 16 : n_tile);
-      const bool wide = Cfg::kWide && n_tile > 128;
-      PipeState acc2 = acc;  // a wide unit's second stage
-      acc2.advance(Cfg::kAccStages);
-      ok = mbar_wait_bounded(&acc_empty[acc.stage], acc.phase ^ 1u, abort_flag, wait_ns);
-      if (wide && ok) ok = mbar_wait_bounded(&acc_empty[acc2.stage], acc2.phase ^ 1u, abort_flag, wait_ns);
-      ok = __all_sync(0xffffffffu, ok);
-      if (!ok) {
-        if (lane == 0) report_status(a.status, kGemmAccTimeout, 1, blockIdx.x, 0);
-        break;
-      }
-      tc_fence_after_sync();
-      const uint32_t d0 = tmem_base + (wide ? 0 : acc.stage * Cfg::kStageCols);
-      const uint32_t d1 = d0 + (Cfg::kWide && !wide ? 128 : N_MAX);
-      for (int j = 0; j < sg.nkb; ++j) {
-        ok = mbar_wait_bounded(&full_bar[st.stage], st.phase, abort_flag, wait_ns);
-        ok = __all_sync(0xffffffffu, ok);
-        if (trace && lane == 0 && trace[3] == 0) trace[3] = global_timer_ns();
-        if (!ok) {
-          if (lane == 0) report_status(a.status, kGemmFullTimeout, 1, blockIdx.x, 0);
-          break;
-        }
-        tc_fence_after_sync();
-        if (lane == 0) {
-          fence_proxy_async_smem();
-          const uint32_t a_addr = smem_u32(sA + st.stage * Cfg::kStageA);
-          const uint32_t b_addr = smem_u32(sB + st.stage * Cfg::kStageB);
-#pragma unroll
-          for (int k = 0; k < 4; ++k) {
-            const uint64_t bdesc = umma_desc_sw128(b_addr + k * 32);
-            const uint32_t accum = (j > 0 || k > 0) ? 1u : 0u;
-            umma_f16(d0, umma_desc_sw128(a_addr + k * 32), bdesc, idesc, accum);
-            if (kGateUp) umma_f16(d1, umma_desc_sw128(a_addr + kTileBytesA + k * 32), bdesc, idesc, accum);
-          }
-          umma_commit(&empty_bar[st.stage]);
-        }
-        __syncwarp();
-        st.advance(STAGES);
-      }
-      if (!ok) break;
-      if (lane == 0) {
-        umma_commit(&acc_full[acc.stage]);
-        if (wide) umma_commit(&acc_full[acc2.stage]);
-      }
-      __syncwarp();
-      acc.advance(Cfg::kAccStages);
-      if (wide) acc.advance(Cfg::kAccStages);
-    }
-  } else if (warp < 4 && b_tma) {
-    // ------------------------------------------------------------------ token-operand producer (TMA)
-    if (warp == 2) {
-      PipeState st;
-      bool ok = true;
-      Seg sg;
-      int ready_tile = -1;
-      const int box_rows = a.b_box_rows > 0 ? a.b_box_rows : N_MAX;
-      while (ok && reader.next(sg, ok)) {
-        if (a.tile_wait != nullptr && sg.tt != ready_tile) {
-          // the tile's activations are final once every gate/up unit of the tile has reported its four quarters
-          bool got = true;
-          if (lane == 0) {
-            got = wait_count_ge_gpu(a.tile_wait + sg.tt, a.tile_wait_target, wait_ns);
-            fence_proxy_async_all();  // the TMA reads below come after the acquire
-          }
-          ok = __all_sync(0xffffffffu, got);
-          if (!ok) {
-            if (lane == 0) {
-              *abort_flag = 1;
-              report_status(a.status, kGemmFullTimeout, 6, blockIdx.x, 0);
-            }
-            break;
-          }
-          ready_tile = sg.tt;
-        }
-        const int n_box = max(1, (sg.n_rows + box_rows - 1) / box_rows);
-        for (int j = 0; j < sg.nkb; ++j) {
-          const int kb = sg.kb0 + j;
-          ok = mbar_wait_bounded(&empty_bar[st.stage], st.phase ^ 1u, abort_flag, wait_ns);
-          ok = __all_sync(0xffffffffu, ok);
-          if (!ok) {
-            if (lane == 0) report_status(a.status, kGemmEmptyTimeout, 2, blockIdx.x, 0);
-            break;
-          }
-          if (lane == 0) {
-            // as many boxes as hold the tile's rows: rows past the tile (the next expert's entries, or zero fill
-            // past the end of the buffer) land in smem rows the MMA does not read or in accumulator columns the
-            // epilogue skips
-            mbar_arrive_expect_tx(&full_bar[st.stage], n_box * box_rows * 128);
-            for (int i = 0; i < n_box; ++i)
-              tma_load_2d(sB + st.stage * Cfg::kStageB + i * box_rows * 128, &tmap_b, &full_bar[st.stage], kb * 64,
-                          sg.row_start + i * box_rows);
-          }
-          __syncwarp();
-          st.advance(STAGES);
-        }
-      }
-      if (!ok) {
-        const unsigned long long t0 = global_timer_ns();
-        while (global_timer_ns() - t0 < 100000ull) __nanosleep(1000);
-      }
-    }
-  } else if (warp < 4) {
-    // ------------------------------------------------------------------ token-operand producers (gather)
-    const int gt = tid - 64;       // 0..63
-    const int r_in = gt >> 3;      // row inside an 8-row group == swizzle phase
+  // Token-operand producers that gather rows by index (gt: 0 .. kGatherThreads - 1).
+  auto gather_rows = [&](const int gt) {
+    const int r_in = gt >> 3;      // first row (its low three bits are the swizzle phase)
     const int chunk = gt & 7;      // 16-byte chunk inside the 128-byte row
-    const uint32_t sw_off = (uint32_t)((chunk ^ r_in) << 4);
+    const uint32_t sw_off = (uint32_t)((chunk ^ (r_in & 7)) << 4);
     PipeState st;
     bool ok = true;
     Seg sg, nx;
     int ready_tile = -1;
-    int idx[N_MAX / 8];  // source rows of the segment at hand, fetched during the previous one
+    int idx[N_MAX / kGatherStep];  // source rows of the segment at hand, fetched during the previous one
     auto row_indices = [&](const Seg& s_) {
 #pragma unroll
-      for (int i = 0; i < N_MAX / 8; ++i) {
-        const int n = r_in + 8 * i;
+      for (int i = 0; i < N_MAX / kGatherStep; ++i) {
+        const int n = r_in + kGatherStep * i;
         if (n < s_.n_rows) idx[i] = a.b_index ? __ldcg(a.b_index + s_.row_start + n) : s_.row_start + n;
       }
     };
@@ -562,10 +420,10 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
       const int n_rows = sg.n_rows;
       int n_tile = (n_rows + 15) & ~15;
       if (n_tile < 16) n_tile = 16;
-      const uint8_t* rp[N_MAX / 8];
+      const uint8_t* rp[N_MAX / kGatherStep];
 #pragma unroll
-      for (int i = 0; i < N_MAX / 8; ++i) {
-        const int n = r_in + 8 * i;
+      for (int i = 0; i < N_MAX / kGatherStep; ++i) {
+        const int n = r_in + kGatherStep * i;
         rp[i] = n < n_rows ? static_cast<const uint8_t*>(a.b_base) + (long long)idx[i] * a.b_pitch + chunk * 16 : nullptr;
       }
       for (int j = 0; j < sg.nkb; ++j) {
@@ -578,8 +436,8 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
         }
         const uint32_t b_stage = smem_u32(sB + st.stage * Cfg::kStageB);
 #pragma unroll
-        for (int i = 0; i < N_MAX / 8; ++i) {
-          const int n = r_in + 8 * i;
+        for (int i = 0; i < N_MAX / kGatherStep; ++i) {
+          const int n = r_in + kGatherStep * i;
           if (n < n_tile) {
             const bool live = rp[i] != nullptr;
             cp_async_16(b_stage + n * 128 + sw_off, live ? (const void*)(rp[i] + (long long)kb * 128) : a.b_base,
@@ -600,7 +458,169 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
     }
     // Drain this thread's cp.async operations before the CTA may exit.
     asm volatile("cp.async.wait_all;" ::: "memory");
+  };
+  // (The register split stands at the head of each warpgroup's branch: in front of a common join the compiler keeps everything
+  // behind it within the smallest share.)
+  if (warp < 4) {
+    if (kFourGather) asm volatile("setmaxnreg.dec.sync.aligned.u32 72;");
+    if (warp == 0) {
+      // ------------------------------------------------------------------ weight TMA producer
+      PipeState st;
+      bool ok = true;
+      SegFeed feed(work, ring, abort_flag, wait_ns);
+      // Tiles of up to 64 rows are decode: an expert usually has one tile, and its weights are then read once per forward.
+      // Skewed routing gives a hot expert several that read the same blocks, but they run close together and most blocks are
+      // still read once: evict-first / normal, us per layer, 1 token 81 / 96, 128 tokens 1325 / 1347 (bf16, 288 experts), 8
+      // tokens e4m3 220 / 241; zipf popularity: 100 tokens on 36 experts bf16 149 / 160, e4m3 113 / 126, 128 on 288 e4m3
+      // 116 / 129, 250 on 72 e4m3 (inter 2048) 223 / 230.
+      const uint64_t policy = N_MAX <= 64 ? l2_evict_first() : l2_evict_normal();
+      Seg sg;
+      bool have = feed.first(sg);
+      while (ok && have) {
+        const int row0 = sg.e * a.rows_per_expert + sg.mb * (a.two_blocks ? 2 * kBlockM : kBlockM);
+        for (int j = 0; j < sg.nkb; ++j) {
+          const int kb = sg.kb0 + j;
+          ok = mbar_wait_bounded(&empty_bar[st.stage], st.phase ^ 1u, abort_flag, wait_ns);
+          ok = __all_sync(0xffffffffu, ok);
+          if (!ok) {
+            if (lane == 0) report_status(a.status, kGemmEmptyTimeout, 0, blockIdx.x, 0);
+            break;
+          }
+          if (lane == 0) {
+            mbar_arrive_expect_tx(&full_bar[st.stage], Cfg::kStageA);
+            uint8_t* dst = sA + st.stage * Cfg::kStageA;
+            if (trace && trace[2] == 0) trace[2] = global_timer_ns();  // see the note at MF_STAMP_ONCE
+            tma_load_2d(dst, &tmap_w, &full_bar[st.stage], kb * 64, row0, policy);
+            if (kGateUp) tma_load_2d(dst + kTileBytesA, &tmap_w, &full_bar[st.stage], kb * 64, row0 + a.up_row_offset, policy);
+          }
+          __syncwarp();
+          st.advance(STAGES);
+          feed.advance();
+        }
+        if (ok) have = feed.next(sg);
+      }
+      if (feed.bad_tile && lane == 0) report_status(a.status, kBadArgument, 7, blockIdx.x, 0);
+      if (!ok) {
+        // Give copies that are still in flight a moment to land before the CTA goes away.
+        const unsigned long long t0 = global_timer_ns();
+        while (global_timer_ns() - t0 < 100000ull) __nanosleep(1000);
+      }
+    } else if (warp == 1) {
+      // ------------------------------------------------------------------ UMMA issuer
+      PipeState st, acc;
+      bool ok = true;
+      Seg sg;
+      while (ok && reader.next(sg, ok)) {
+        const uint32_t n_tile = (uint32_t)((sg.n_rows + 15) & ~15);
+        const uint32_t idesc = umma_idesc(1, 1, kBlockM, n_tile < 16 ? 16 : n_tile);
+        const bool wide = Cfg::kWide && n_tile > 128;
+        PipeState acc2 = acc;  // a wide unit's second stage
+        acc2.advance(Cfg::kAccStages);
+        ok = mbar_wait_bounded(&acc_empty[acc.stage], acc.phase ^ 1u, abort_flag, wait_ns);
+        if (wide && ok) ok = mbar_wait_bounded(&acc_empty[acc2.stage], acc2.phase ^ 1u, abort_flag, wait_ns);
+        ok = __all_sync(0xffffffffu, ok);
+        if (!ok) {
+          if (lane == 0) report_status(a.status, kGemmAccTimeout, 1, blockIdx.x, 0);
+          break;
+        }
+        tc_fence_after_sync();
+        const uint32_t d0 = tmem_base + (wide ? 0 : acc.stage * Cfg::kStageCols);
+        const uint32_t d1 = d0 + (Cfg::kWide && !wide ? 128 : N_MAX);
+        for (int j = 0; j < sg.nkb; ++j) {
+          ok = mbar_wait_bounded(&full_bar[st.stage], st.phase, abort_flag, wait_ns);
+          ok = __all_sync(0xffffffffu, ok);
+          if (trace && lane == 0 && trace[3] == 0) trace[3] = global_timer_ns();
+          if (!ok) {
+            if (lane == 0) report_status(a.status, kGemmFullTimeout, 1, blockIdx.x, 0);
+            break;
+          }
+          tc_fence_after_sync();
+          if (lane == 0) {
+            fence_proxy_async_smem();
+            const uint32_t a_addr = smem_u32(sA + st.stage * Cfg::kStageA);
+            const uint32_t b_addr = smem_u32(sB + st.stage * Cfg::kStageB);
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+              const uint64_t bdesc = umma_desc_sw128(b_addr + k * 32);
+              const uint32_t accum = (j > 0 || k > 0) ? 1u : 0u;
+              umma_f16(d0, umma_desc_sw128(a_addr + k * 32), bdesc, idesc, accum);
+              if (kGateUp) umma_f16(d1, umma_desc_sw128(a_addr + kTileBytesA + k * 32), bdesc, idesc, accum);
+            }
+            umma_commit(&empty_bar[st.stage]);
+          }
+          __syncwarp();
+          st.advance(STAGES);
+        }
+        if (!ok) break;
+        if (lane == 0) {
+          umma_commit(&acc_full[acc.stage]);
+          if (wide) umma_commit(&acc_full[acc2.stage]);
+        }
+        __syncwarp();
+        acc.advance(Cfg::kAccStages);
+        if (wide) acc.advance(Cfg::kAccStages);
+      }
+    } else if (b_tma) {
+      // ------------------------------------------------------------------ token-operand producer (TMA)
+      if (warp == 2) {
+        PipeState st;
+        bool ok = true;
+        Seg sg;
+        int ready_tile = -1;
+        const int box_rows = a.b_box_rows > 0 ? a.b_box_rows : N_MAX;
+        while (ok && reader.next(sg, ok)) {
+          if (a.tile_wait != nullptr && sg.tt != ready_tile) {
+            // the tile's activations are final once every gate/up unit of the tile has reported its four quarters
+            bool got = true;
+            if (lane == 0) {
+              got = wait_count_ge_gpu(a.tile_wait + sg.tt, a.tile_wait_target, wait_ns);
+              fence_proxy_async_all();  // the TMA reads below come after the acquire
+            }
+            ok = __all_sync(0xffffffffu, got);
+            if (!ok) {
+              if (lane == 0) {
+                *abort_flag = 1;
+                report_status(a.status, kGemmFullTimeout, 6, blockIdx.x, 0);
+              }
+              break;
+            }
+            ready_tile = sg.tt;
+          }
+          const int n_box = max(1, (sg.n_rows + box_rows - 1) / box_rows);
+          for (int j = 0; j < sg.nkb; ++j) {
+            const int kb = sg.kb0 + j;
+            ok = mbar_wait_bounded(&empty_bar[st.stage], st.phase ^ 1u, abort_flag, wait_ns);
+            ok = __all_sync(0xffffffffu, ok);
+            if (!ok) {
+              if (lane == 0) report_status(a.status, kGemmEmptyTimeout, 2, blockIdx.x, 0);
+              break;
+            }
+            if (lane == 0) {
+              // as many boxes as hold the tile's rows: rows past the tile (the next expert's entries, or zero fill
+              // past the end of the buffer) land in smem rows the MMA does not read or in accumulator columns the
+              // epilogue skips
+              mbar_arrive_expect_tx(&full_bar[st.stage], n_box * box_rows * 128);
+              for (int i = 0; i < n_box; ++i)
+                tma_load_2d(sB + st.stage * Cfg::kStageB + i * box_rows * 128, &tmap_b, &full_bar[st.stage], kb * 64,
+                            sg.row_start + i * box_rows);
+            }
+            __syncwarp();
+            st.advance(STAGES);
+          }
+        }
+        if (!ok) {
+          const unsigned long long t0 = global_timer_ns();
+          while (global_timer_ns() - t0 < 100000ull) __nanosleep(1000);
+        }
+      }
+    } else if (!kFourGather) {
+      gather_rows(tid - 64);
+    }
+  } else if (kFourGather && warp >= 12) {
+    if (kFourGather) asm volatile("setmaxnreg.dec.sync.aligned.u32 104;");
+    if (!b_tma) gather_rows(tid - 384);
   } else if (warp < 4 + 4 * kGroups) {
+    if (kFourGather) asm volatile("setmaxnreg.inc.sync.aligned.u32 168;");
     // ------------------------------------------------------------------ epilogue
     const int wq = warp & 3;                 // TMEM lane quarter this warp may read
     const int grp = (warp - 4) >> 2;         // column group (0 unless kGroups == 2)
@@ -850,7 +870,7 @@ static int launch(const void* tmap, const mf_gemm_args* args, int grid, cudaStre
   CUtensorMap tm, tb;
   memcpy(&tm, tmap, sizeof(tm));
   memcpy(&tb, args->b_tmap ? args->b_tmap : tmap, sizeof(tb));
-  const int threads = kReturn ? kThreadsWithReturn : 128 + 128 * kEpiGroups<N_MAX, kReturn>;
+  const int threads = kLaunchThreads<kGateUp, N_MAX, kReturn>;
   return (int)launch_kernel(kern, dim3(grid), dim3(threads), Cfg::kSmemBytes, stream, true, tm, tb, *args);
 }
 

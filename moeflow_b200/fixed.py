@@ -587,10 +587,12 @@ class FixedEPLayer:
             box = min(self.block_m, 64)
             self._tmap_act = make_tile_tmap(self.act, box)
             self._a_gemm2.b_tmap, self._a_gemm2.b_box_rows = C.addressof(self._tmap_act), box
-        # Opt-in (gemm_kwargs permute_rows=True): copy the received hidden rows into expert-major order first,
-        # so that the gate/up GEMM reads token tiles by TMA too instead of gathering them by entry index.
-        # Default: on with 256-row tiles, where 64 gather threads would have to place 32 chunks each per stage.
-        self.permute_rows = bool(self.gemm_kwargs.get("permute_rows", self.block_m >= 256))
+        # Received hidden rows copied into expert-major order first, so that the gate/up GEMM fetches its token tiles by TMA
+        # instead of gathering them by entry index (gemm_kwargs permute_rows overrides).  With four gather warps on 256-row
+        # tiles the copy does not pay: copied / gathered 1000 tokens 548 / 532 us (72 experts), 700 tokens 328 / 317 and 8192
+        # tokens (e4m3, expanded) 2645 / 2622 (36 experts), 130 tokens 105.8 / 104.3 (8 experts, 8.5 MB).  Copies of less than
+        # 8 MB are a few microseconds either way; those layers keep it, and its checks run at that size.
+        self.permute_rows = bool(self.gemm_kwargs.get("permute_rows", self.block_m >= 256 and N * H * 2 < 8 << 20))
         if self.permute_rows:
             from .ops.kernels import make_tile_tmap
 
