@@ -88,7 +88,7 @@ __device__ __forceinline__ void promote_32(f32x2* acc, const uint32_t (&p)[32], 
 template <bool kGateUp>
 __global__ void __launch_bounds__(kFwThreads<kGateUp>, 1)
 grouped_gemm_fp8_wide_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_x,
-                             const mf_gemm_args a) {
+                             const mf_gemm_args a, const int blocks) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint8_t* sW = smem;                                // [kFwStages][kFwStageW]
@@ -186,9 +186,9 @@ grouped_gemm_fp8_wide_kernel(const __grid_constant__ CUtensorMap tmap_w, const _
     }
     return got;
   };
-  // Weight blocks of a unit: gate and up, or two adjacent ones (an odd block count leaves one for the last unit).
+  // Weight blocks of a unit: gate and up, or two adjacent ones of the `blocks` (an odd count leaves one for the last unit).
   auto unit_row = [&](const Seg& s) { return kGateUp ? s.mb * kF8BlockM : s.mb * 2 * kF8BlockM; };
-  auto two_halves = [&](const Seg& s) { return kGateUp || s.mb * 2 * kF8BlockM + kF8BlockM < a.rows_per_expert; };
+  auto two_halves = [&](const Seg& s) { return kGateUp || s.mb * 2 + 1 < blocks; };
   const int second_half = kGateUp ? a.up_row_offset : kF8BlockM;
   SegReader reader(ring, abort_flag, wait_ns);
 
@@ -709,7 +709,8 @@ static int launch_wide(const void* tmap, const mf_gemm_args* args, int grid, cud
     if (dev >= 0 && dev < 64) configured[dev] = true;
   }
   mf_gemm_args a = *args;
-  if (!kGateUp) a.m_blocks = (a.rows_per_expert / kF8BlockM + 1) / 2;  // a unit covers two weight blocks
+  const int blocks = a.m_blocks;
+  if (!kGateUp) a.m_blocks = (blocks + 1) / 2;  // a unit covers two weight blocks
   CUtensorMap tm, tx;
   memcpy(&tm, tmap, sizeof(tm));
   memcpy(&tx, a.b_tmap && !kGateUp ? a.b_tmap : tmap, sizeof(tx));
@@ -719,7 +720,7 @@ static int launch_wide(const void* tmap, const mf_gemm_args* args, int grid, cud
     const int e = mf_make_pitched_tmap(&tx, a.b_base, a.b_rows, (long long)a.k_blocks * 128, 1, a.b_pitch, a.b_box_rows);
     if (e) return e;
   }
-  return (int)launch_kernel(kern, dim3(grid), dim3(kFwThreads<kGateUp>), kFwSmem, stream, true, tm, tx, a);
+  return (int)launch_kernel(kern, dim3(grid), dim3(kFwThreads<kGateUp>), kFwSmem, stream, true, tm, tx, a, blocks);
 }
 
 int launch_fp8_wide(bool gate_up, const void* tmap, const mf_gemm_args* args, int grid, cudaStream_t stream) {

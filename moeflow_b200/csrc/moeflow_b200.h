@@ -339,7 +339,7 @@ int mf_quant_rows_1x128(const void* x, long long x_pitch, const int* row_index, 
                         float* scales, long long valid_off, const int* n_rows_dev, mf_stream_t stream);
 // Block-scaled e4m3 variants of the grouped GEMMs (args->w_scale, b_scale, b_scale_pitch are required;
 // b_base rows are e4m3 bytes, k_blocks = K / 128, the tensor map is built with elem_bytes = 1; n_max 32, 64 or 128).
-// With n_max = 128 a unit of the down GEMM covers two adjacent weight blocks whatever m_blocks says; that kernel reads
+// With n_max = 128 a unit of the down GEMM covers two adjacent ones of the m_blocks weight blocks; that kernel reads
 // contiguous rows only (no b_index), through b_tmap or a map that the launch makes (b_rows).
 int mf_gemm_gate_up_fp8(const void* tmap, const mf_gemm_args* args, int n_max, int grid, mf_stream_t stream);
 int mf_gemm_down_fp8(const void* tmap, const mf_gemm_args* args, int n_max, int grid, mf_stream_t stream);

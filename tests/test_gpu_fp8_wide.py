@@ -61,6 +61,63 @@ def test_128_row_tiles_match_the_dequantised_definition(counts, hidden, inter, s
             assert normwise_rel_err(y[lo:hi], ref) < 4 * 2.0**-8
 
 
+class _EditedCalls:
+    """The native library with ``edit(args)`` run on the arguments of every grouped GEMM first."""
+
+    def __init__(self, real, edit):
+        self._real, self._edit = real, edit
+
+    def __getattr__(self, name):
+        fn = getattr(self._real, name)
+        if not name.startswith("mf_gemm_"):
+            return fn
+
+        def call(tmap, args, *rest):
+            self._edit(args._obj)
+            return fn(tmap, args, *rest)
+
+        return call
+
+
+@pytest.fixture
+def edit_calls(monkeypatch):
+    from moeflow_b200.ops import _lib
+
+    real = _lib.lib()
+    return lambda edit: monkeypatch.setattr(_lib, "lib", lambda: _EditedCalls(real, edit))
+
+
+def _down_problem(counts, hidden, inter, seed=0):
+    """``(codes, scales, w2 codes, w2 scales, plan)`` of a down projection on 128-row tiles."""
+    from moeflow_b200.ops.fp8 import quant_rows_1x128
+    from moeflow_b200.ops.grouped_gemm import plan_from_offsets
+
+    gen = torch.Generator().manual_seed(seed)
+    packs = [quant_block_fp8(torch.randn(hidden, inter, generator=gen) / inter**0.5) for _ in counts]
+    w2 = torch.stack([q.view(torch.uint8) for q, _ in packs]).view(torch.float8_e4m3fn).cuda()
+    s2 = torch.stack([s for _, s in packs]).cuda()
+    aq, a_s = quant_rows_1x128(torch.randn(sum(counts), inter, generator=gen).bfloat16().cuda())
+    offsets = [sum(counts[:i]) for i in range(len(counts) + 1)]
+    return aq, a_s, w2, s2, plan_from_offsets(offsets, 128, aq.device)
+
+
+@pytest.mark.parametrize("split", [0, 1, 2])
+@pytest.mark.parametrize("blocks", [1, 3, 4])
+def test_only_the_weight_blocks_asked_for_are_computed(edit_calls, blocks, split):
+    from moeflow_b200.ops.fp8 import down_proj_fp8
+
+    aq, a_s, w2, s2, tp = _down_problem([5, 140], 640, 256)
+    whole = down_proj_fp8(aq, a_s, w2, s2, tp, split=split)
+    edit_calls(lambda a: setattr(a, "m_blocks", blocks))
+    some = down_proj_fp8(aq, a_s, w2, s2, tp, split=split)
+    assert some[:, blocks * 128 :].abs().sum() == 0
+    if split:  # (stream-K cuts the shorter line of work elsewhere)
+        assert torch.equal(some[:, : blocks * 128], whole[:, : blocks * 128])
+    else:
+        # a cut moves the last bit of an fp32 sum: some elements round to the other bf16 neighbour, 2**-8 of themselves
+        assert normwise_rel_err(some[:, : blocks * 128], whole[:, : blocks * 128]) < 2.0**-8
+
+
 @pytest.mark.parametrize("tokens,hidden,inter", [(1, 384, 256), (50, 640, 384), (300, 512, 256)])
 def test_layer_on_128_row_tiles_matches_64_row_tiles(tokens, hidden, inter):
     """Whole layers: the plan counts pairs of weight blocks for the down GEMM, and every tile is handed over complete."""
