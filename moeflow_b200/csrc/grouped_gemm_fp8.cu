@@ -876,7 +876,6 @@ int mf_gemm_down_fp8(const void* tmap, const mf_gemm_args* args, int n_max, int 
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   if (n_max == 32) return mf::launch_f8<false, 32>(tmap, args, grid, s);
   if (n_max == 64) return mf::launch_f8<false, 64>(tmap, args, grid, s);
-  if (args->b_index != nullptr || (args->b_tmap == nullptr && args->b_rows < 1)) return -8;
   return mf::launch_fp8_wide(false, tmap, args, grid, s);
 }
 

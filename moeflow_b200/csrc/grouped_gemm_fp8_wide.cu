@@ -17,10 +17,11 @@
 // through L2 (210 us of the gate/up GEMM at 2000 tokens with everything else taken out), the promotion, which only half
 // overlaps it, and 5 us of epilogue per gate/up unit.
 //
-// Warps: 0 weight TMA and segment hand-out, 1 UMMA, 2 token TMA (down: contiguous rows in boxes), 3 activation and weight
+// Warps: 0 weight TMA and segment hand-out, 1 UMMA, 2 token TMA (b_tmap: contiguous rows in boxes), 3 activation and weight
 // scales (four K blocks at a time, up to 16 ahead) and finished token tiles, 4-11 promotion and epilogue, 12-15 gather
-// (gate/up: rows by index, 16 bytes per cp.async).  Rows by index through the tensor copy engine (tile::gather4, 32
-// instructions per K block) took 66 cycles an instruction and bound the whole kernel.
+// (without b_tmap: rows by index or one after the other, 16 bytes per cp.async).  The layers gather for gate/up and use
+// boxes for down.  Rows by index through the tensor copy engine (tile::gather4, 32 instructions per K block) took 66 cycles
+// an instruction and bound the whole kernel.
 #include <cuda.h>
 
 #include <cstring>
@@ -34,9 +35,9 @@
 namespace mf {
 
 constexpr int kFwRows = 128;                   // token rows of a tile
-template <bool kGateUp>
-constexpr int kFwThreads = kGateUp ? 512 : 384;
-constexpr int kFwGather = 128;                 // gather threads (gate/up)
+template <bool kGather>
+constexpr int kFwThreads = kGather ? 512 : 384;
+constexpr int kFwGather = 128;                 // gather threads
 constexpr int kFwPromo = 8;                    // promotion warps: 4 .. 11
 constexpr int kFwStageW = 2 * kF8TileA;        // 256 weight rows x one K block
 constexpr int kFwStageX = kFwRows * 128;
@@ -52,8 +53,8 @@ static_assert(kFwSmem <= 227 * 1024, "shared memory");
 // Registers: 384 threads are launched with 168 each (64512), 512 with 128 (65536); the promotion warps take what the
 // others give up.  72 x 128 + 216 x 256 = 64512; 72 x 128 + 200 x 256 + 40 x 128 = 65536.
 constexpr int kFwRegsFew = 72, kFwRegsGather = 40;
-template <bool kGateUp>
-constexpr int kFwRegsMany = kGateUp ? 200 : 216;
+template <bool kGather>
+constexpr int kFwRegsMany = kGather ? 200 : 216;
 
 // 32 lanes x 32 consecutive fp32 columns.
 __device__ __forceinline__ void tmem_ld_32(uint32_t taddr, uint32_t (&r)[32]) {
@@ -85,8 +86,8 @@ __device__ __forceinline__ void promote_32(f32x2* acc, const uint32_t (&p)[32], 
   for (int i = 0; i < 16; ++i) acc[i] = fma2(pack2(p[2 * i], p[2 * i + 1]), s, acc[i]);
 }
 
-template <bool kGateUp>
-__global__ void __launch_bounds__(kFwThreads<kGateUp>, 1)
+template <bool kGateUp, bool kGather>
+__global__ void __launch_bounds__(kFwThreads<kGather>, 1)
 grouped_gemm_fp8_wide_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_x,
                              const mf_gemm_args a, const int blocks) {
   extern __shared__ uint8_t smem_raw[];
@@ -113,7 +114,7 @@ grouped_gemm_fp8_wide_kernel(const __grid_constant__ CUtensorMap tmap_w, const _
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   if (tid == 0) {
     for (int s = 0; s < kFwStages; ++s) {
-      mbar_init(&full_bar[s], kGateUp ? 1 + kFwGather : 2);  // weights, token rows
+      mbar_init(&full_bar[s], kGather ? 1 + kFwGather : 2);  // weights, token rows
       mbar_init(&empty_bar[s], 1);
     }
     for (int s = 0; s < kFwTmp; ++s) {
@@ -126,11 +127,11 @@ grouped_gemm_fp8_wide_kernel(const __grid_constant__ CUtensorMap tmap_w, const _
     }
     for (int s = 0; s < 4; ++s) mbar_init(&pair_bar[s], 2);
     for (int s = 0; s < 2; ++s) mbar_init(&epi_bar[s], kFwPromo);
-    ring->init((kGateUp ? 2 + kFwGather / 32 : 3) + kFwPromo);  // UMMA, scale warp, token producers, promotion warps
+    ring->init((kGather ? 2 + kFwGather / 32 : 3) + kFwPromo);  // UMMA, scale warp, token producers, promotion warps
     *abort_flag = 0;
     fence_mbar_init();
     tma_prefetch_desc(&tmap_w);
-    if (!kGateUp) tma_prefetch_desc(&tmap_x);
+    if (!kGather) tma_prefetch_desc(&tmap_x);
   }
   if (warp == 1) {
     tmem_alloc(tmem_slot, 512);
@@ -248,7 +249,7 @@ grouped_gemm_fp8_wide_kernel(const __grid_constant__ CUtensorMap tmap_w, const _
           }
           tc_fence_after_sync();
           if (lane == 0) {
-            if (kGateUp) fence_proxy_async_smem();  // the gathered rows
+            if (kGather) fence_proxy_async_smem();  // the gathered rows
             const uint32_t d = tmem_base + tmp.stage * 256;
             const uint32_t x_addr = smem_u32(sX + st.stage * kFwStageX);
             const uint32_t w_addr = smem_u32(sW + st.stage * kFwStageW);
@@ -264,13 +265,13 @@ grouped_gemm_fp8_wide_kernel(const __grid_constant__ CUtensorMap tmap_w, const _
         }
       }
     } else if (warp == 2) {
-      // -------------------------------------------------------------- token rows in boxes (down)
+      // -------------------------------------------------------------- token rows in boxes
       F8Pipe st;
       bool ok = true;
       Seg sg;
       int ready_tile = -1;
       const int box_rows = a.b_box_rows > 0 ? a.b_box_rows : kFwRows;
-      while (!kGateUp && ok && reader.next(sg, ok)) {
+      while (!kGather && ok && reader.next(sg, ok)) {
         if (a.tile_wait != nullptr && sg.tt != ready_tile) {
           ok = tile_ready(sg.tt);
           if (!ok) break;
@@ -383,16 +384,22 @@ grouped_gemm_fp8_wide_kernel(const __grid_constant__ CUtensorMap tmap_w, const _
       if (report)
         for (int k = n_it < 2 ? 0 : n_it - 2; ok && k < n_it; ++k) ok = report_unit(k);
     }
-  } else if (kGateUp && warp >= 4 + kFwPromo) {
+  } else if (kGather && warp >= 4 + kFwPromo) {
     asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kFwRegsGather));
-    // ---------------------------------------------------------------- token rows by index
+    // ---------------------------------------------------------------- token rows, 16 bytes at a time
     const int gt = tid - 32 * (4 + kFwPromo);  // 0 .. 127: rows gt / 8, + 16, ...; 16-byte chunk gt & 7
     const int r_in = gt >> 3, chunk = gt & 7;
     const uint32_t sw_off = (uint32_t)(r_in * 128 + ((chunk ^ (r_in & 7)) << 4));
     F8Pipe st;
     bool ok = true;
     Seg sg;
+    int ready_tile = -1;
     while (ok && reader.next(sg, ok)) {
+      if (!kGateUp && a.tile_wait != nullptr && sg.tt != ready_tile) {
+        ok = tile_ready(sg.tt);
+        if (!ok) break;
+        ready_tile = sg.tt;
+      }
       int off[kFwRows / 16];  // in 16-byte chunks (rows behind the tile repeat its last one; nobody looks at them)
       const int pitch16 = (int)(a.b_pitch >> 4);
 #pragma unroll
@@ -417,7 +424,7 @@ grouped_gemm_fp8_wide_kernel(const __grid_constant__ CUtensorMap tmap_w, const _
     }
     asm volatile("cp.async.wait_all;" ::: "memory");
   } else {
-    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kFwRegsMany<kGateUp>));
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kFwRegsMany<kGather>));
     // ---------------------------------------------------------------- promotion + epilogue
     const int wq = warp & 3;           // tensor-memory lane quarter: token rows 32 wq ..
     const int grp = (warp - 4) >> 2;   // columns 64 grp .. of both halves
@@ -696,10 +703,10 @@ grouped_gemm_fp8_wide_kernel(const __grid_constant__ CUtensorMap tmap_w, const _
   }
 }
 
-template <bool kGateUp>
+template <bool kGateUp, bool kGather>
 static int launch_wide(const void* tmap, const mf_gemm_args* args, int grid, cudaStream_t stream) {
   static bool configured[64] = {};  // per device: the attribute belongs to (function, device)
-  auto kern = grouped_gemm_fp8_wide_kernel<kGateUp>;
+  auto kern = grouped_gemm_fp8_wide_kernel<kGateUp, kGather>;
   int dev = 0;
   cudaError_t de = cudaGetDevice(&dev);
   if (de != cudaSuccess) return (int)de;
@@ -713,18 +720,14 @@ static int launch_wide(const void* tmap, const mf_gemm_args* args, int grid, cud
   if (!kGateUp) a.m_blocks = (blocks + 1) / 2;  // a unit covers two weight blocks
   CUtensorMap tm, tx;
   memcpy(&tm, tmap, sizeof(tm));
-  memcpy(&tx, a.b_tmap && !kGateUp ? a.b_tmap : tmap, sizeof(tx));
-  if (!kGateUp && a.b_tmap == nullptr) {
-    a.b_box_rows = 64;  // boxes that the operand can fill
-    while (a.b_box_rows > a.b_rows) a.b_box_rows /= 2;
-    const int e = mf_make_pitched_tmap(&tx, a.b_base, a.b_rows, (long long)a.k_blocks * 128, 1, a.b_pitch, a.b_box_rows);
-    if (e) return e;
-  }
-  return (int)launch_kernel(kern, dim3(grid), dim3(kFwThreads<kGateUp>), kFwSmem, stream, true, tm, tx, a, blocks);
+  memcpy(&tx, kGather ? tmap : a.b_tmap, sizeof(tx));
+  return (int)launch_kernel(kern, dim3(grid), dim3(kFwThreads<kGather>), kFwSmem, stream, true, tm, tx, a, blocks);
 }
 
 int launch_fp8_wide(bool gate_up, const void* tmap, const mf_gemm_args* args, int grid, cudaStream_t stream) {
-  return gate_up ? launch_wide<true>(tmap, args, grid, stream) : launch_wide<false>(tmap, args, grid, stream);
+  if (args->b_tmap == nullptr)
+    return gate_up ? launch_wide<true, true>(tmap, args, grid, stream) : launch_wide<false, true>(tmap, args, grid, stream);
+  return gate_up ? launch_wide<true, false>(tmap, args, grid, stream) : launch_wide<false, false>(tmap, args, grid, stream);
 }
 
 }  // namespace mf

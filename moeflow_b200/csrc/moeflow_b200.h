@@ -100,7 +100,6 @@ typedef struct {
   // instead of round-robin (work_iter.cuh).
   int* sched;
   int b_box_rows;            // bf16 and 128-row e4m3 kernels: rows of a box of b_tmap, 0 = n_max; a divisor of n_max and a multiple of 16
-  long long b_rows;          // 128-row e4m3 down kernel without b_tmap: rows of b_base, for the map that the launch makes
 } mf_gemm_args;
 
 // Encode a 2-D tiled tensor map (K innermost) for a weight matrix [rows, k_elems]; box = 128 bytes x
@@ -339,8 +338,7 @@ int mf_quant_rows_1x128(const void* x, long long x_pitch, const int* row_index, 
                         float* scales, long long valid_off, const int* n_rows_dev, mf_stream_t stream);
 // Block-scaled e4m3 variants of the grouped GEMMs (args->w_scale, b_scale, b_scale_pitch are required;
 // b_base rows are e4m3 bytes, k_blocks = K / 128, the tensor map is built with elem_bytes = 1; n_max 32, 64 or 128).
-// With n_max = 128 a unit of the down GEMM covers two adjacent ones of the m_blocks weight blocks; that kernel reads
-// contiguous rows only (no b_index), through b_tmap or a map that the launch makes (b_rows).
+// With n_max = 128 a unit of the down GEMM covers two adjacent ones of the m_blocks weight blocks.
 int mf_gemm_gate_up_fp8(const void* tmap, const mf_gemm_args* args, int n_max, int grid, mf_stream_t stream);
 int mf_gemm_down_fp8(const void* tmap, const mf_gemm_args* args, int n_max, int grid, mf_stream_t stream);
 

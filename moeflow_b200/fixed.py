@@ -760,7 +760,6 @@ class FixedEPLayer:
                                 n_counters=g2.n_counters, w_scale=None, b_scale=f["as"].data_ptr(), b_scale_pitch=I // 128,
                                 **common)
         f["a2"].partial = g2.partial  # its own half, as in the bf16 layers
-        f["a2"].b_rows = max(N, self.block_m)
         if bool(self.gemm_kwargs.get("b_tma", True)):
             from .ops.kernels import make_tile_tmap
 

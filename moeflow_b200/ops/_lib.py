@@ -84,7 +84,6 @@ class GemmArgs(C.Structure):
         ("q_scale_pitch", C.c_longlong),
         ("sched", C.c_void_p),
         ("b_box_rows", C.c_int),
-        ("b_rows", C.c_longlong),
     ]
 
 

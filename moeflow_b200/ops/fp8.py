@@ -81,7 +81,7 @@ def _gemm_fp8(gate_up: bool, xq, xs, wq, ws, tp: TilePlan, out, row_index, row_s
         out=out.data_ptr(), out_pitch=out.shape[1], row_scale=_lib.ptr(row_scale), partial=partial.data_ptr(),
         counters=counters.data_ptr(), max_split_slots=slots, limit=float(limit) if limit is not None else 0.0, round_h=0,
         status=status.data_ptr(), wait_ns=wait_ns, w_scale=ws.data_ptr(), b_scale=xs.data_ptr(), b_scale_pitch=xs.stride(0),
-        partial_floats=partial.numel(), n_counters=counters.numel(), max_tiles=tp.tile_e.numel(), b_rows=xq.shape[0],
+        partial_floats=partial.numel(), n_counters=counters.numel(), max_tiles=tp.tile_e.numel(),
     )
     tmap_b = None
     if b_tma:

@@ -48,9 +48,9 @@ def test_128_row_tiles_match_the_dequantised_definition(counts, hidden, inter, s
     assert torch.equal(in_order, act), "rows by index and contiguous rows differ"
     aq, a_s = quant_rows_1x128(act.contiguous())
     y = down_proj_fp8(aq, a_s, q2, s2, tp, row_scale=scale, **kw)
-    y_own_map = down_proj_fp8(aq, a_s, q2, s2, tp, row_scale=scale, b_tma=False, **kw)
+    y_gathered = down_proj_fp8(aq, a_s, q2, s2, tp, row_scale=scale, b_tma=False, **kw)
     assert int(status) == 0
-    assert torch.equal(y, y_own_map), "the caller's tensor map and the launch's own differ"
+    assert torch.equal(y, y_gathered), "token tiles by TMA and by the gather differ"
     x_dq, a_dq = dequant_rows(xq, xs)[idx.long()], dequant_rows(aq, a_s)
     for e, (lo, hi) in enumerate(zip(offsets[:-1], offsets[1:])):
         if hi > lo:
@@ -116,6 +116,27 @@ def test_only_the_weight_blocks_asked_for_are_computed(edit_calls, blocks, split
     else:
         # a cut moves the last bit of an fp32 sum: some elements round to the other bf16 neighbour, 2**-8 of themselves
         assert normwise_rel_err(some[:, : blocks * 128], whole[:, : blocks * 128]) < 2.0**-8
+
+
+@pytest.mark.parametrize("split", [0, 1, 2])
+@pytest.mark.parametrize("counts", [[1], [7, 0, 20], [128, 129, 15]])
+def test_rows_by_index_and_by_tensor_map_in_both_gemms(edit_calls, counts, split):
+    """The down GEMM takes a row index and needs no tensor map; the gate/up GEMM reads a caller's map and not b_base."""
+    from moeflow_b200.ops.fp8 import _gemm_fp8, down_proj_fp8, gate_up_swiglu_fp8
+
+    n = sum(counts)
+    aq, a_s, w2, s2, tp = _down_problem(counts, 512, 256)
+    idx = torch.randperm(n, generator=torch.Generator().manual_seed(n)).int().cuda()
+    status = torch.zeros(1, dtype=torch.int64, device="cuda")
+    kw = dict(limit=None, split=split, status=status, wait_ns=50_000_000, grid=None)
+    by_index = _gemm_fp8(False, aq, a_s, w2, s2, tp, torch.zeros(n, 512, dtype=torch.bfloat16, device="cuda"), idx, None, **kw)
+    in_order = down_proj_fp8(aq[idx.long()], a_s[idx.long()], w2, s2, tp, split=split, status=status)
+    assert int(status) == 0 and in_order.abs().sum() > 0 and torch.equal(by_index, in_order)
+
+    gathered = gate_up_swiglu_fp8(aq, a_s, w2, s2, tp, limit=None, split=split, status=status)
+    edit_calls(lambda a: setattr(a, "b_base", None))
+    mapped = _gemm_fp8(True, aq, a_s, w2, s2, tp, torch.zeros(n, 256, dtype=torch.bfloat16, device="cuda"), None, None, b_tma=True, **kw)
+    assert int(status) == 0 and gathered.abs().sum() > 0 and torch.equal(mapped, gathered)
 
 
 @pytest.mark.parametrize("tokens,hidden,inter", [(1, 384, 256), (50, 640, 384), (300, 512, 256)])
