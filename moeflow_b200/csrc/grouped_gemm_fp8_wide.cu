@@ -164,14 +164,23 @@ grouped_gemm_fp8_wide_kernel(const __grid_constant__ CUtensorMap tmap_w, const _
   {
     const int n_tiles = __ldcg(a.plan + MF_PLAN_N_TILES);
     const int cut = __ldcg(a.plan + a.split_word);  // 0 = stream-K, else the K split
-    const long long slot_floats = 2ll * slot_cols * kF8BlockM;
-    work.init(a, kFwRows, n_tiles, cut, blockIdx.x, gridDim.x);
+    // Scratch in accumulators of one weight block, as much as the other tile heights need.  Stream-K on units of two blocks
+    // would need twice that: where it is not there, fewer CTAs take part.
+    const long long acc_floats = (long long)slot_cols * kF8BlockM, steps = (long long)n_tiles * blocks * a.k_blocks;
+    long long need = cut == 0 ? 2 * min(steps, (long long)gridDim.x) : cut > 1 ? (long long)n_tiles * blocks * cut : 0;
+    int ctas = gridDim.x;
+    if (!kGateUp && cut == 0) {
+      const long long there = a.partial_floats > 0 ? a.partial_floats / acc_floats : need;
+      ctas = (int)max(1ll, min(there / 4, (long long)ctas));
+    }
+    work.init(a, kFwRows, n_tiles, cut, blockIdx.x, ctas);
+    if (kGateUp) need = 2 * work.slots_needed();
     // the plan is checked against the buffers it indexes before anything is stored (same rule as the other kernels)
     bool bad = n_tiles < 0 || !(cut == 0 || cut == 1 || cut == 2 || cut == 4 || cut == 8) ||
                (cut > 1 && a.k_blocks % cut != 0);
     bad = bad || (a.max_tiles > 0 && n_tiles > a.max_tiles);
     bad = bad || (a.n_counters > 0 && (long long)n_tiles * a.m_blocks * 4 > (long long)a.n_counters);
-    bad = bad || (a.partial_floats > 0 && work.slots_needed() * slot_floats > a.partial_floats);
+    bad = bad || (a.partial_floats > 0 && need * acc_floats > a.partial_floats);
     if (bad) {
       if (tid == 0) report_status(a.status, kBadArgument, 6, blockIdx.x, 0);
       work.init(a, kFwRows, 0, 1, blockIdx.x, gridDim.x);
@@ -508,14 +517,16 @@ grouped_gemm_fp8_wide_kernel(const __grid_constant__ CUtensorMap tmap_w, const _
       }
       if (!ok) break;
 
-      // The unit is cut along K: park the sums, [half][column / 4][row][4]; the quarter that arrives last adds the segments
+      // The unit is cut along K: park the sums, [block][column / 4][row][4]; the quarter that arrives last adds the segments
       // in K order, straight into its outputs (sum_16).  Summed up in the registers of the K loop instead, these few lines
       // made the compiler spill in that loop (layer at 2000 tokens: 585 us against 542).
       const bool cut_unit = sg.nseg > 1;
       bool finish = true;
       const int half = 32 * slot_cols;
-      auto slot_at = [&](int s_) {
-        return reinterpret_cast<float4*>(a.partial) + ((long long)slot_of(sg, s_) * 64 + 16 * grp) * slot_cols + row;
+      auto slot_at = [&](int s_) {  // (a last unit of one block leaves no gap behind a segment of a K split)
+        const long long acc = kGateUp || sg.c_first >= 0 ? 2ll * slot_of(sg, s_)
+                                                         : (long long)(sg.tt * blocks + 2 * sg.mb) * sg.nseg + (two ? 2 : 1) * s_;
+        return reinterpret_cast<float4*>(a.partial) + (acc * 32 + 16 * grp) * slot_cols + row;
       };
       if (cut_unit) {
         if (row < n_rows) {

@@ -139,6 +139,36 @@ def test_rows_by_index_and_by_tensor_map_in_both_gemms(edit_calls, counts, split
     assert int(status) == 0 and gathered.abs().sum() > 0 and torch.equal(mapped, gathered)
 
 
+@pytest.mark.parametrize("split,grid", [(0, 1), (0, 3), (0, 8), (0, 148), (2, 148), (4, 5)])
+@pytest.mark.parametrize("hidden", [128, 384, 640, 1024])
+def test_cut_down_units_stay_inside_the_scratch_of_one_block_units(edit_calls, hidden, split, grid):
+    """A unit of two weight blocks needs no more scratch than two of one: as many accumulators of 128 x 128 sums as units of
+    one block have segments (stream-K: two per CTA that has a K step)."""
+    from moeflow_b200.ops.fp8 import dequant_rows, down_proj_fp8
+
+    aq, a_s, w2, s2, tp = _down_problem([30, 128, 131], hidden, 512)
+    units = tp.n_tiles * (hidden // 128)
+    accumulators = 2 * min(units * 4, grid) if split == 0 else units * split
+    floats = accumulators * 128 * 128
+    scratch = torch.full((floats + 4096,), 77.0, device="cuda")
+    status = torch.zeros(1, dtype=torch.int64, device="cuda")
+    checked = [floats]
+
+    def shrink(a):
+        a.partial, a.partial_floats = scratch.data_ptr(), checked[0]
+
+    edit_calls(shrink)
+    ref = dequant_rows(aq, a_s)
+    ref = torch.cat([r @ dequant_block_fp8(w2[e], s2[e]).t() for e, r in enumerate(ref.split([30, 128, 131]))])
+    for checked[0] in (floats, 0):  # 0: the kernel is not told how much there is
+        y = down_proj_fp8(aq, a_s, w2, s2, tp, split=split, status=status, grid=grid, wait_ns=50_000_000)
+        assert int(status) == 0 and (scratch[floats:] == 77).all()
+        assert normwise_rel_err(y, ref) < 4 * 2.0**-8  # one bf16 rounding of sums whose fp32 error is far below it
+    checked[0] = floats - 1  # refused on the device, nothing stored
+    y = down_proj_fp8(aq, a_s, w2, s2, tp, split=split, status=status, grid=grid, wait_ns=50_000_000)
+    assert int(status) != 0 and y.abs().sum() == 0
+
+
 @pytest.mark.parametrize("tokens,hidden,inter", [(1, 384, 256), (50, 640, 384), (300, 512, 256)])
 def test_layer_on_128_row_tiles_matches_64_row_tiles(tokens, hidden, inter):
     """Whole layers: the plan counts pairs of weight blocks for the down GEMM, and every tile is handed over complete."""
