@@ -80,6 +80,22 @@ __device__ __forceinline__ void tmem_ld_wait_32(uint32_t (&r)[32]) {
                     "+r"(r[24]), "+r"(r[25]), "+r"(r[26]), "+r"(r[27]), "+r"(r[28]), "+r"(r[29]), "+r"(r[30]), "+r"(r[31]));
 }
 
+// Four partial sums, in scratch at any address of a float.
+__device__ __forceinline__ void park_4(float* p, float4 v) {
+  if ((reinterpret_cast<uintptr_t>(p) & 15) == 0) {
+    __stcg(reinterpret_cast<float4*>(p), v);
+  } else {
+    __stcg(p, v.x);
+    __stcg(p + 1, v.y);
+    __stcg(p + 2, v.z);
+    __stcg(p + 3, v.w);
+  }
+}
+__device__ __forceinline__ float4 parked_4(const float* p) {
+  if ((reinterpret_cast<uintptr_t>(p) & 15) == 0) return __ldcg(reinterpret_cast<const float4*>(p));
+  return make_float4(__ldcg(p), __ldcg(p + 1), __ldcg(p + 2), __ldcg(p + 3));
+}
+
 // acc[0..31] += s * p[0..31], both halves of s holding the same scale
 __device__ __forceinline__ void promote_32(f32x2* acc, const uint32_t (&p)[32], f32x2 s) {
 #pragma unroll
@@ -522,21 +538,21 @@ grouped_gemm_fp8_wide_kernel(const __grid_constant__ CUtensorMap tmap_w, const _
       // made the compiler spill in that loop (layer at 2000 tokens: 585 us against 542).
       const bool cut_unit = sg.nseg > 1;
       bool finish = true;
-      const int half = 32 * slot_cols;
+      const int half = kF8BlockM * slot_cols;
       auto slot_at = [&](int s_) {  // (a last unit of one block leaves no gap behind a segment of a K split)
         const long long acc = kGateUp || sg.c_first >= 0 ? 2ll * slot_of(sg, s_)
                                                          : (long long)(sg.tt * blocks + 2 * sg.mb) * sg.nseg + (two ? 2 : 1) * s_;
-        return reinterpret_cast<float4*>(a.partial) + (acc * 32 + 16 * grp) * slot_cols + row;
+        return a.partial + ((acc * 32 + 16 * grp) * slot_cols + row) * 4;
       };
       if (cut_unit) {
         if (row < n_rows) {
-          float4* p = slot_at(sg.seg);
+          float* p = slot_at(sg.seg);
 #pragma unroll
-          for (int i = 0; i < 16; ++i, p += slot_cols) {
+          for (int i = 0; i < 16; ++i, p += 4 * slot_cols) {
             const float2 x = unpack2(acc0[2 * i]), y = unpack2(acc0[2 * i + 1]);
-            __stcg(p, make_float4(x.x, x.y, y.x, y.y));
+            park_4(p, make_float4(x.x, x.y, y.x, y.y));
             const float2 z = unpack2(acc1[2 * i]), w = unpack2(acc1[2 * i + 1]);
-            if (two) __stcg(p + half, make_float4(z.x, z.y, w.x, w.y));
+            if (two) park_4(p + half, make_float4(z.x, z.y, w.x, w.y));
           }
         }
         __threadfence();
@@ -561,10 +577,10 @@ grouped_gemm_fp8_wide_kernel(const __grid_constant__ CUtensorMap tmap_w, const _
           float4 x[1][4];
 #pragma unroll
           for (int k = 0; k < 1; ++k) {
-            const float4* p = slot_at(min(s_ + k, sg.nseg - 1)) + h * half + (long long)(4 * c) * slot_cols;
+            const float* p = slot_at(min(s_ + k, sg.nseg - 1)) + h * half + 16 * c * slot_cols;
 #pragma unroll
-            for (int i = 0; i < 4; ++i, p += slot_cols)
-              x[k][i] = s_ + k < sg.nseg && row < n_rows ? __ldcg(p) : make_float4(0.f, 0.f, 0.f, 0.f);
+            for (int i = 0; i < 4; ++i, p += 4 * slot_cols)
+              x[k][i] = s_ + k < sg.nseg && row < n_rows ? parked_4(p) : make_float4(0.f, 0.f, 0.f, 0.f);
           }
 #pragma unroll
           for (int k = 0; k < 1; ++k) {

@@ -140,17 +140,17 @@ def test_rows_by_index_and_by_tensor_map_in_both_gemms(edit_calls, counts, split
 
 
 @pytest.mark.parametrize("split,grid", [(0, 1), (0, 3), (0, 8), (0, 148), (2, 148), (4, 5)])
-@pytest.mark.parametrize("hidden", [128, 384, 640, 1024])
-def test_cut_down_units_stay_inside_the_scratch_of_one_block_units(edit_calls, hidden, split, grid):
+@pytest.mark.parametrize("hidden,shift", [(128, 0), (384, 0), (640, 0), (1024, 0), (384, 1), (384, 2)])
+def test_cut_down_units_stay_inside_the_scratch_of_one_block_units(edit_calls, hidden, shift, split, grid):
     """A unit of two weight blocks needs no more scratch than two of one: as many accumulators of 128 x 128 sums as units of
-    one block have segments (stream-K: two per CTA that has a K step)."""
+    one block have segments (stream-K: two per CTA that has a K step).  ``shift``: floats from a 16-byte boundary."""
     from moeflow_b200.ops.fp8 import dequant_rows, down_proj_fp8
 
     aq, a_s, w2, s2, tp = _down_problem([30, 128, 131], hidden, 512)
     units = tp.n_tiles * (hidden // 128)
     accumulators = 2 * min(units * 4, grid) if split == 0 else units * split
     floats = accumulators * 128 * 128
-    scratch = torch.full((floats + 4096,), 77.0, device="cuda")
+    scratch = torch.full((shift + floats + 4096,), 77.0, device="cuda")[shift:]
     status = torch.zeros(1, dtype=torch.int64, device="cuda")
     checked = [floats]
 
