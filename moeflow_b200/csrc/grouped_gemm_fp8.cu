@@ -470,6 +470,7 @@ grouped_gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid
       int off[N_MAX / 16];  // in 16-byte chunks; rows behind the tile repeat its last one, and nobody looks at their sums
 #pragma unroll
       for (int i = 0; i < N_MAX / 16; ++i) {
+        if (16 * i >= sg.n_rows) break;  // (a tile without rows has no last one)
         const int n = sg.row_start + min(r_in + 16 * i, sg.n_rows - 1);
         off[i] = (a.b_index ? __ldcg(a.b_index + n) : n) * pitch16 + chunk;
       }

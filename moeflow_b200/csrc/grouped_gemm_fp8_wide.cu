@@ -354,6 +354,7 @@ grouped_gemm_fp8_wide_kernel(const __grid_constant__ CUtensorMap tmap_w, const _
         const float* src[4];  // this lane's rows: lane, lane + 32, ...
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
+          if (32 * i >= sg.n_rows) break;  // (a tile without rows has no last one)
           const int n = sg.row_start + min(lane + 32 * i, sg.n_rows - 1);
           src[i] = a.b_scale + (a.b_index ? (long long)__ldcg(a.b_index + n) : (long long)n) * a.b_scale_pitch + sg.kb0;
         }
@@ -429,6 +430,7 @@ grouped_gemm_fp8_wide_kernel(const __grid_constant__ CUtensorMap tmap_w, const _
       const int pitch16 = (int)(a.b_pitch >> 4);
 #pragma unroll
       for (int i = 0; i < kFwRows / 16; ++i) {
+        if (16 * i >= sg.n_rows) break;  // (a tile without rows has no last one)
         const int n = sg.row_start + min(r_in + 16 * i, sg.n_rows - 1);
         off[i] = (a.b_index ? __ldcg(a.b_index + n) : n) * pitch16 + chunk;
       }

@@ -169,6 +169,36 @@ def test_cut_down_units_stay_inside_the_scratch_of_one_block_units(edit_calls, h
     assert int(status) != 0 and y.abs().sum() == 0
 
 
+@pytest.mark.parametrize("block_m", [32, 64, 128])
+@pytest.mark.parametrize("split", [1, 2])
+def test_tiles_without_rows_are_passed_over(block_m, split):
+    """In front of the first row and behind the last one: such a tile has no last row that could be read in place of one."""
+    import dataclasses
+
+    from moeflow_b200.ops import _lib
+    from moeflow_b200.ops.fp8 import _gemm_fp8, down_proj_fp8
+    from moeflow_b200.ops.grouped_gemm import plan_from_offsets
+
+    aq, a_s, w2, s2, _ = _down_problem([5, 70], 512, 256)
+    tp = plan_from_offsets([0, 5, 75], block_m, aq.device)
+    i32 = dict(dtype=torch.int32, device="cuda")
+    more = dataclasses.replace(
+        tp, n_tiles=tp.n_tiles + 2, plan=tp.plan.clone(),
+        **{k: torch.cat([torch.tensor([first], **i32), getattr(tp, k), torch.tensor([last], **i32)])
+           for k, first, last in (("tile_e", 0, 1), ("tile_s", 0, 75), ("tile_n", 0, 0))})
+    more.plan[_lib.PLAN_N_TILES] = more.n_tiles
+    idx = torch.randperm(75, generator=torch.Generator().manual_seed(1)).int().cuda()
+    status = torch.zeros(1, dtype=torch.int64, device="cuda")
+    outs = []
+    for plan in (tp, more):
+        act = torch.zeros(75, 256, dtype=torch.bfloat16, device="cuda")
+        _gemm_fp8(True, aq, a_s, w2, s2, plan, act, idx, None, None, split, status, 50_000_000, None)
+        outs.append([act, *(down_proj_fp8(aq, a_s, w2, s2, plan, split=split, status=status, b_tma=b_tma) for b_tma in (True, False))])
+    assert int(status) == 0
+    for a, b in zip(*outs):
+        assert a.abs().sum() > 0 and torch.equal(a, b)
+
+
 @pytest.mark.parametrize("tokens,hidden,inter", [(1, 384, 256), (50, 640, 384), (300, 512, 256)])
 def test_layer_on_128_row_tiles_matches_64_row_tiles(tokens, hidden, inter):
     """Whole layers: the plan counts pairs of weight blocks for the down GEMM, and every tile is handed over complete."""
