@@ -1,4 +1,5 @@
-// What the two forms of the block-scaled e4m3 GEMM share: a pipeline position and arithmetic on pairs of fp32 values.
+// What the two forms of the block-scaled e4m3 GEMM share: a pipeline position, arithmetic on pairs of fp32 values, and where a
+// gathered row's bytes are.
 #pragma once
 
 #include "common.cuh"
@@ -47,6 +48,14 @@ __device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
   f32x2 r;
   asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
   return r;
+}
+
+// Address of 16-byte chunk `first` + row * pitch (addresses in chunks).  One multiply-add per use: as plain arithmetic the
+// compiler keeps the 64-bit products of all rows, which a gather warp has no registers for.
+__device__ __forceinline__ const void* row_chunk(uint64_t first, int row, int pitch) {
+  uint64_t at;
+  asm("mad.wide.s32 %0, %1, %2, %3;" : "=l"(at) : "r"(row), "r"(pitch), "l"(first));
+  return reinterpret_cast<const void*>(at << 4);
 }
 
 }  // namespace mf

@@ -467,12 +467,12 @@ grouped_gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid
         if (!ok) break;
         ready_tile = sg.tt;
       }
-      int off[N_MAX / 16];  // in 16-byte chunks; rows behind the tile repeat its last one, and nobody looks at their sums
+      int src_row[N_MAX / 16];  // rows behind the tile repeat its last one, and nobody looks at their sums
 #pragma unroll
       for (int i = 0; i < N_MAX / 16; ++i) {
         if (16 * i >= sg.n_rows) break;  // (a tile without rows has no last one)
         const int n = sg.row_start + min(r_in + 16 * i, sg.n_rows - 1);
-        off[i] = (a.b_index ? __ldcg(a.b_index + n) : n) * pitch16 + chunk;
+        src_row[i] = a.b_index ? __ldcg(a.b_index + n) : n;
       }
       for (int j = 0; j < sg.nkb; ++j) {
         ok = __all_sync(0xffffffffu, mbar_wait_bounded(&empty_bar[st.stage], st.phase ^ 1u, abort_flag, wait_ns));
@@ -481,10 +481,10 @@ grouped_gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid
           break;
         }
         const uint32_t dst = smem_u32(sB + st.stage * Cfg::kStageB) + sw_off;
-        const uint4* src = static_cast<const uint4*>(a.b_base) + (sg.kb0 + j) * 8;
+        const uint64_t src = (reinterpret_cast<uint64_t>(a.b_base) >> 4) + (sg.kb0 + j) * 8 + chunk;
 #pragma unroll
         for (int i = 0; i < N_MAX / 16; ++i)
-          if (16 * i < sg.n_rows) cp_async_16(dst + i * 2048, src + off[i], 16u);
+          if (16 * i < sg.n_rows) cp_async_16(dst + i * 2048, row_chunk(src, src_row[i], pitch16), 16u);
         cp_async_mbar_arrive_noinc(&full_bar[st.stage]);
         st.advance(STAGES);
       }

@@ -199,6 +199,26 @@ def test_tiles_without_rows_are_passed_over(block_m, split):
         assert a.abs().sum() > 0 and torch.equal(a, b)
 
 
+@pytest.mark.parametrize("block_m", [64, 128])
+def test_gathered_rows_32_gib_apart(block_m):
+    """Row 4 lies 2**31 chunks of 16 bytes behind row 0."""
+    from moeflow_b200.ops.fp8 import _gemm_fp8
+    from moeflow_b200.ops.grouped_gemm import plan_from_offsets
+
+    if torch.cuda.mem_get_info()[0] < 36 << 30:
+        pytest.skip("needs 36 GiB of device memory")
+    aq, a_s, w2, s2, _ = _down_problem([5], 512, 256)
+    tp = plan_from_offsets([0, 5], block_m, aq.device)
+    far = torch.empty((32 << 30) + 256, dtype=torch.uint8, device="cuda").as_strided((5, 256), (8 << 30, 1))
+    far.copy_(aq.view(torch.uint8))
+    far = far.view(torch.float8_e4m3fn)
+    idx = torch.tensor([4, 1, 0, 3, 2], dtype=torch.int32, device="cuda")
+    for gate_up, cols in ((True, 256), (False, 512)):
+        near, away = (_gemm_fp8(gate_up, x, a_s, w2, s2, tp, torch.zeros(5, cols, dtype=torch.bfloat16, device="cuda"), idx, None,
+                                None, 1, None, 50_000_000, None) for x in (aq, far))
+        assert near.abs().sum() > 0 and torch.equal(near, away)
+
+
 @pytest.mark.parametrize("tokens,hidden,inter", [(1, 384, 256), (50, 640, 384), (300, 512, 256)])
 def test_layer_on_128_row_tiles_matches_64_row_tiles(tokens, hidden, inter):
     """Whole layers: the plan counts pairs of weight blocks for the down GEMM, and every tile is handed over complete."""
