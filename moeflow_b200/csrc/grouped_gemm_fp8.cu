@@ -847,8 +847,7 @@ static int check_f8(const mf_gemm_args* a, int n_max, int grid) {
   if (!a || grid < 1) return -1;
   if (n_max != 32 && n_max != 64 && n_max != 128) return -2;
   if (a->b_tmap != nullptr && a->b_index != nullptr) return -6;  // TMA token tiles need contiguous rows
-  if (a->b_box_rows < 0 || (a->b_box_rows > 0 && (a->b_box_rows % 16 != 0 || n_max % a->b_box_rows != 0))) return -9;
-  if (n_max != 128 && a->b_box_rows > 0 && a->b_box_rows != n_max) return -8;
+  if (n_max == 128 && (a->b_box_rows < 0 || (a->b_box_rows > 0 && (a->b_box_rows % 16 != 0 || n_max % a->b_box_rows != 0)))) return -9;
   if (a->m_blocks < 1 || a->k_blocks < 1 || a->k_blocks > kF8MaxKb) return -3;
   if ((a->b_pitch & 15) != 0 || (reinterpret_cast<uintptr_t>(a->b_base) & 15) != 0) return -4;
   if (!a->w_scale || !a->b_scale) return -5;

@@ -99,7 +99,8 @@ typedef struct {
   // Optional: a device counter, zero when the kernel starts.  Segments of a K split then go to the CTA that asks next
   // instead of round-robin (work_iter.cuh).
   int* sched;
-  int b_box_rows;            // bf16 and 128-row e4m3 kernels: rows of a box of b_tmap, 0 = n_max; a divisor of n_max and a multiple of 16
+  int b_box_rows;            // bf16 and 128-row e4m3 kernels: rows of a box of b_tmap, 0 = n_max; a divisor of n_max and a multiple of 16.
+                             // The e4m3 kernels of 32- and 64-row tiles take boxes of n_max rows and do not look at it
 } mf_gemm_args;
 
 // Encode a 2-D tiled tensor map (K innermost) for a weight matrix [rows, k_elems]; box = 128 bytes x

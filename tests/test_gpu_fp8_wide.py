@@ -199,6 +199,19 @@ def test_tiles_without_rows_are_passed_over(block_m, split):
         assert a.abs().sum() > 0 and torch.equal(a, b)
 
 
+@pytest.mark.parametrize("block_m,box_rows", [(32, 16), (32, 48), (64, 32), (64, 128)])
+def test_box_rows_mean_nothing_to_tiles_of_up_to_64_rows(edit_calls, block_m, box_rows):
+    """Their boxes hold a whole tile, whatever the field says."""
+    from moeflow_b200.ops.fp8 import down_proj_fp8
+    from moeflow_b200.ops.grouped_gemm import plan_from_offsets
+
+    aq, a_s, w2, s2, _ = _down_problem([5, 70], 512, 256)
+    tp = plan_from_offsets([0, 5, 75], block_m, aq.device)
+    y = down_proj_fp8(aq, a_s, w2, s2, tp)
+    edit_calls(lambda a: setattr(a, "b_box_rows", box_rows))
+    assert y.abs().sum() > 0 and torch.equal(down_proj_fp8(aq, a_s, w2, s2, tp), y)
+
+
 @pytest.mark.parametrize("block_m", [64, 128])
 def test_gathered_rows_32_gib_apart(block_m):
     """Row 4 lies 2**31 chunks of 16 bytes behind row 0."""
