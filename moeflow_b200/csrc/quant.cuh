@@ -18,7 +18,7 @@ __device__ __forceinline__ uint16_t to_e4m3x2(float2 v, float inv_scale) {  // v
   return (uint16_t)__nv_cvt_float2_to_fp8x2(make_float2(v.x * inv_scale, v.y * inv_scale), __NV_SATFINITE, __NV_E4M3);
 }
 
-// Chunk c of one row (`v`: its 8 bf16 values).  16 consecutive threads hold a group: all of them must call this together.
+// Chunk c of one row (`v`: its 8 bf16 values).  Half a warp holds a group (threads 16 n ..): all of it calls this.
 __device__ __forceinline__ void quant_chunk(const uint4& v, int c, uint8_t* q_row, float* scale_row) {
   const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&v);
   float f[8];
@@ -30,9 +30,9 @@ __device__ __forceinline__ void quant_chunk(const uint4& v, int c, uint8_t* q_ro
     f[2 * i + 1] = t.y;
     amax = fmaxf(amax, fmaxf(fabsf(t.x), fabsf(t.y)));
   }
-  const unsigned active = __activemask();
+  const unsigned group = 0xffffu << (lane_id() & 16);  // named, not taken from where the compiler lets the warp meet
 #pragma unroll
-  for (int off = 8; off > 0; off >>= 1) amax = fmaxf(amax, __shfl_xor_sync(active, amax, off));
+  for (int off = 8; off > 0; off >>= 1) amax = fmaxf(amax, __shfl_xor_sync(group, amax, off));
   const float scale = group_scale(amax);
   const float inv = 1.f / scale;
   uint2 packed;
