@@ -201,7 +201,7 @@ grouped_gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid
       F8Pipe st;
       bool ok = true;
       SegFeed feed(work, ring, abort_flag, wait_ns);
-      const uint64_t policy = N_MAX <= 64 ? l2_evict_first() : l2_evict_normal();  // as in grouped_gemm_tc.cu
+      const uint64_t policy = l2_evict_first();  // as in grouped_gemm_tc.cu at these tile heights
       Seg sg;
       bool have = feed.first(sg);
       while (ok && have) {

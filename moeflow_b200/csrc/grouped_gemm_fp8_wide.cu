@@ -576,23 +576,16 @@ grouped_gemm_fp8_wide_kernel(const __grid_constant__ CUtensorMap tmap_w, const _
         for (int i = 0; i < 16; ++i) v[i] = 0.f;
 #pragma unroll 1
         for (int s_ = 0; s_ < sg.nseg; ++s_) {
-          float4 x[1][4];
+          const float* p = slot_at(s_) + h * half + 16 * c * slot_cols;
+          float4 x[4];
 #pragma unroll
-          for (int k = 0; k < 1; ++k) {
-            const float* p = slot_at(min(s_ + k, sg.nseg - 1)) + h * half + 16 * c * slot_cols;
+          for (int i = 0; i < 4; ++i, p += 4 * slot_cols) x[i] = row < n_rows ? parked_4(p) : make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
-            for (int i = 0; i < 4; ++i, p += 4 * slot_cols)
-              x[k][i] = s_ + k < sg.nseg && row < n_rows ? parked_4(p) : make_float4(0.f, 0.f, 0.f, 0.f);
-          }
-#pragma unroll
-          for (int k = 0; k < 1; ++k) {
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-              v[4 * i] += x[k][i].x;
-              v[4 * i + 1] += x[k][i].y;
-              v[4 * i + 2] += x[k][i].z;
-              v[4 * i + 3] += x[k][i].w;
-            }
+          for (int i = 0; i < 4; ++i) {
+            v[4 * i] += x[i].x;
+            v[4 * i + 1] += x[i].y;
+            v[4 * i + 2] += x[i].z;
+            v[4 * i + 3] += x[i].w;
           }
         }
       };
