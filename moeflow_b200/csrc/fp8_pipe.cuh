@@ -1,5 +1,5 @@
-// What the two forms of the block-scaled e4m3 GEMM share: a pipeline position, arithmetic on pairs of fp32 values, and where a
-// gathered row's bytes are.
+// What the two forms of the block-scaled e4m3 GEMM share: a pipeline position, arithmetic on pairs of fp32 values, and the
+// gather of a tile's rows by four warps.
 #pragma once
 
 #include "common.cuh"
@@ -50,12 +50,26 @@ __device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
   return r;
 }
 
-// Address of 16-byte chunk `first` + row * pitch (addresses in chunks).  One multiply-add per use: as plain arithmetic the
-// compiler keeps the 64-bit products of all rows, which a gather warp has no registers for.
-__device__ __forceinline__ const void* row_chunk(uint64_t first, int row, int pitch) {
+// first + row * pitch in one multiply-add per use: as plain arithmetic the compiler keeps the 64-bit products of all rows, which
+// a gather warp has no registers for.
+__device__ __forceinline__ uint64_t row_at(uint64_t first, int row, int pitch) {
   uint64_t at;
   asm("mad.wide.s32 %0, %1, %2, %3;" : "=l"(at) : "r"(row), "r"(pitch), "l"(first));
-  return reinterpret_cast<const void*>(at << 4);
+  return at;
+}
+// 16 bytes of every 16th row of a tile of n_rows into rows of 128 bytes.  `first`: address of those bytes in row 0.  Rows
+// 2 GiB apart and more are addressed in units of 16 bytes, two instructions more for each.
+template <int kRows>
+__device__ __forceinline__ void gather_chunks(uint32_t dst, uint64_t first, const int (&row)[kRows], long long pitch, int n_rows) {
+  if (pitch <= 0x7fffffffll) {
+#pragma unroll
+    for (int i = 0; i < kRows; ++i)
+      if (16 * i < n_rows) cp_async_16(dst + i * 2048, reinterpret_cast<const void*>(row_at(first, row[i], (int)pitch)), 16u);
+  } else {
+#pragma unroll
+    for (int i = 0; i < kRows; ++i)
+      if (16 * i < n_rows) cp_async_16(dst + i * 2048, reinterpret_cast<const void*>(row_at(first >> 4, row[i], (int)(pitch >> 4)) << 4), 16u);
+  }
 }
 
 }  // namespace mf

@@ -456,7 +456,6 @@ grouped_gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid
     const int gt = tid - 384;  // rows gt / 8, + 16, ...; 16-byte chunk gt & 7
     const int r_in = gt >> 3, chunk = gt & 7;
     const uint32_t sw_off = (uint32_t)(r_in * 128 + ((chunk ^ (r_in & 7)) << 4));
-    const int pitch16 = (int)(a.b_pitch >> 4);
     F8Pipe st;
     bool ok = true;
     Seg sg;
@@ -468,11 +467,12 @@ grouped_gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid
         ready_tile = sg.tt;
       }
       int src_row[N_MAX / 16];  // rows behind the tile repeat its last one, and nobody looks at their sums
+      if (sg.n_rows > 0) {  // (a tile without rows has no last one)
 #pragma unroll
-      for (int i = 0; i < N_MAX / 16; ++i) {
-        if (16 * i >= sg.n_rows) break;  // (a tile without rows has no last one)
-        const int n = sg.row_start + min(r_in + 16 * i, sg.n_rows - 1);
-        src_row[i] = a.b_index ? __ldcg(a.b_index + n) : n;
+        for (int i = 0; i < N_MAX / 16; ++i) {
+          const int n = sg.row_start + min(r_in + 16 * i, sg.n_rows - 1);
+          src_row[i] = a.b_index ? __ldcg(a.b_index + n) : n;
+        }
       }
       for (int j = 0; j < sg.nkb; ++j) {
         ok = __all_sync(0xffffffffu, mbar_wait_bounded(&empty_bar[st.stage], st.phase ^ 1u, abort_flag, wait_ns));
@@ -481,10 +481,7 @@ grouped_gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid
           break;
         }
         const uint32_t dst = smem_u32(sB + st.stage * Cfg::kStageB) + sw_off;
-        const uint64_t src = (reinterpret_cast<uint64_t>(a.b_base) >> 4) + (sg.kb0 + j) * 8 + chunk;
-#pragma unroll
-        for (int i = 0; i < N_MAX / 16; ++i)
-          if (16 * i < sg.n_rows) cp_async_16(dst + i * 2048, row_chunk(src, src_row[i], pitch16), 16u);
+        gather_chunks(dst, reinterpret_cast<uint64_t>(a.b_base) + (sg.kb0 + j) * 128 + chunk * 16, src_row, a.b_pitch, sg.n_rows);
         cp_async_mbar_arrive_noinc(&full_bar[st.stage]);
         st.advance(STAGES);
       }

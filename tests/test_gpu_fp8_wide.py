@@ -212,24 +212,27 @@ def test_box_rows_mean_nothing_to_tiles_of_up_to_64_rows(edit_calls, block_m, bo
     assert y.abs().sum() > 0 and torch.equal(down_proj_fp8(aq, a_s, w2, s2, tp), y)
 
 
+@pytest.mark.parametrize("rows,apart", [(5, 8 << 30), (34, 1 << 30)])
 @pytest.mark.parametrize("block_m", [64, 128])
-def test_gathered_rows_32_gib_apart(block_m):
-    """Row 4 lies 2**31 chunks of 16 bytes behind row 0."""
+def test_gathered_rows_over_more_than_32_gib(block_m, rows, apart):
+    """The last row lies 2**31 chunks of 16 bytes behind the first, or more."""
     from moeflow_b200.ops.fp8 import _gemm_fp8
     from moeflow_b200.ops.grouped_gemm import plan_from_offsets
 
-    if torch.cuda.mem_get_info()[0] < 36 << 30:
-        pytest.skip("needs 36 GiB of device memory")
-    aq, a_s, w2, s2, _ = _down_problem([5], 512, 256)
-    tp = plan_from_offsets([0, 5], block_m, aq.device)
-    far = torch.empty((32 << 30) + 256, dtype=torch.uint8, device="cuda").as_strided((5, 256), (8 << 30, 1))
+    if torch.cuda.mem_get_info()[0] < 38 << 30:
+        pytest.skip("needs 38 GiB of device memory")
+    aq, a_s, w2, s2, _ = _down_problem([rows], 512, 256)
+    tp = plan_from_offsets([0, rows], block_m, aq.device)
+    far = torch.empty((rows - 1) * apart + 256, dtype=torch.uint8, device="cuda").as_strided((rows, 256), (apart, 1))
     far.copy_(aq.view(torch.uint8))
     far = far.view(torch.float8_e4m3fn)
-    idx = torch.tensor([4, 1, 0, 3, 2], dtype=torch.int32, device="cuda")
+    idx = torch.randperm(rows, generator=torch.Generator().manual_seed(2)).int().cuda()
     for gate_up, cols in ((True, 256), (False, 512)):
-        near, away = (_gemm_fp8(gate_up, x, a_s, w2, s2, tp, torch.zeros(5, cols, dtype=torch.bfloat16, device="cuda"), idx, None,
+        near, away = (_gemm_fp8(gate_up, x, a_s, w2, s2, tp, torch.zeros(rows, cols, dtype=torch.bfloat16, device="cuda"), idx, None,
                                 None, 1, None, 50_000_000, None) for x in (aq, far))
         assert near.abs().sum() > 0 and torch.equal(near, away)
+    del far
+    torch.cuda.empty_cache()
 
 
 @pytest.mark.parametrize("tokens,hidden,inter", [(1, 384, 256), (50, 640, 384), (300, 512, 256)])
