@@ -156,7 +156,9 @@ __global__ void __launch_bounds__(kDispatchThreads) dispatch_push_kernel(const m
 // The same for prefill sizes (from 512 token positions, up to 32 ranks): a warp per token and four of them per CTA, with
 // nothing shared between them but the arrival.  With a CTA per token three of its four warps waited for the one that
 // routes, in 3.5 waves of CTAs at 8192 tokens; a quarter of the CTAs also means a quarter of the fences and arrivals.
-// Kernel at 8192 tokens 74 / 53 us, at 2000 21 / 14, at 600 19 / 12.
+// Kernel at 8192 tokens 74 / 53 us, at 2000 21 / 14, at 700 18.5 / 10.3, at 512 10.4 / 8.4.  Below, 256 to 511 tokens, it is
+// 10.4 / 8.3 as well, but the layer takes the same (185 / 181, 206 / 206, 235 / 238 us with 36 e4m3 experts), and one rank
+// uses the local dispatch there (top-8: up to 512 tokens).
 constexpr int kManyWarps = 4;
 
 __global__ void __launch_bounds__(32 * kManyWarps) dispatch_push_many_kernel(const mf_dispatch_args a) {

@@ -64,10 +64,17 @@ __device__ __forceinline__ void clear_counters(const mf_meta_args& a, int n_tile
 // the kernel takes ceil(units * S / SMs) rounds of such units.  K is cut between steps of k_step blocks: the e4m3 kernels
 // work on K blocks of 128 values (k_step 2) and refuse a split that does not divide those.  units * 8 fits 32 bits (16
 // million token tiles of 32 weight blocks).
-// What a cut unit costs more (split_kb blocks) depends on the kernels.  Measured, us per layer, split_kb 1 / 8: e4m3, 288 experts, 1 token 75 / 65, 4 tokens 142 / 123, 8 tokens 221 / 200
-// (their blocks are half as long, and the fix-up is exposed); bf16, 1 token 78 / 82, elsewhere the same.  Units of fewer than 16
-// blocks are not cut (hidden 512, 8 blocks, cut / whole: 1 token 28.3 / 26.9, 8 tokens 32.0 / 28.5): the round trip takes longer
-// than what it saves of the stream.  One to three units on the whole chip are, as they always were.
+// What a cut unit costs more (split_kb blocks of streaming) depends on the kernels: 1 for bf16, 8 for e4m3, whose K blocks are
+// half as long and whose fix-up is exposed.  us per layer, graph replay, split_kb 1 / 8:
+//   e4m3, 64-row tiles: 288 experts, 1 token 72.5 / 63.5, 4 tokens 133 / 119, 8 tokens 216 / 187; 72 experts, 16 tokens 227 / 196;
+//   e4m3, 128-row tiles: 8 experts, 80 rows 163 / 87; 4 experts, 200 rows 82 / 70; 72 experts, 400 tokens 335 / 312; 36 experts,
+//   8 to 1000 tokens, and 144 experts, 800 tokens: not cut with either, the same within 1 %;
+//   bf16: 288 experts, 1 token 78 / 82, elsewhere the same.
+// Units of fewer than kMinCutBlocks blocks are not cut where there are kMinCutUnits of them: the round trip takes longer than what
+// it saves of the stream.  bf16, us per layer, cut / whole: 4 blocks (8 experts) 1 token 24.8 / 22.6, 8 tokens 28.1 / 24.6;
+// 8 blocks (32 experts) 27.0 / 26.3, 29.4 / 27.2; 12 blocks (16 experts) 29.5 / 29.9, 34.0 / 31.3; 14 blocks, 4 tokens 33.2 / 32.7.
+// With one to three units nearly the whole chip is idle, and a cut pays from 8 blocks on: 4 blocks 25.1 / 24.5, 8 blocks 26.1 / 26.6,
+// 12 blocks 25.3 / 26.7, 14 blocks 26.9 / 28.4.
 constexpr long long kNoSplit = 0x7fffffffffffffffll;
 constexpr int kMinCutBlocks = 16, kMinCutUnits = 4;
 __host__ __device__ __forceinline__ long long split_cost(int log_s, int units, int k_blocks, int k_step, int n_sms, int max_slots,
@@ -75,7 +82,8 @@ __host__ __device__ __forceinline__ long long split_cost(int log_s, int units, i
   const int s = 1 << log_s;
   const int rounds = (int)(((unsigned)units * (unsigned)s + (unsigned)n_sms - 1u) / (unsigned)n_sms);
   if (s == 1) return (long long)rounds * (k_blocks + overhead_kb);
-  if ((k_blocks < kMinCutBlocks && units >= kMinCutUnits) || (k_blocks & (s * k_step - 1)) != 0 || (k_blocks >> log_s) < 2 || (long long)units * s > max_slots) return kNoSplit;
+  if (k_blocks < kMinCutBlocks && units >= kMinCutUnits) return kNoSplit;
+  if ((k_blocks & (s * k_step - 1)) != 0 || (k_blocks >> log_s) < 2 || (long long)units * s > max_slots) return kNoSplit;
   // the partial-sum round trip of a split unit grows with the tile's token columns (measured: splitting
   // 64-column tiles in two cost more than the idle SMs of an uneven last round)
   const int wide = cols > 16 ? (cols - 16) / 8 : 0;

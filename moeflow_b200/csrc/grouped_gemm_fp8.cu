@@ -46,8 +46,9 @@ namespace mf {
 
 // Gather threads: warp 2, or four warps of their own (12-15) in the gate/up GEMM of 64-row tiles, where one warp's 16 copy
 // instructions per K block (about 90 cycles each) took longer than the K block's promotion and its weights.  The promotion
-// warps then take the registers that the others give up.  Layer, us: 1 token on 288 experts 64.6 / 61.8, 250 on 72 351 / 346, 64
-// sequences of the decode model 262 / 256.  The split: 88 x 128 + 192 x 256 + 40 x 128 = 65536, what 512 threads start with.
+// warps then take the registers that the others give up.  Layer, us: 1 token on 288 experts 64.6 / 61.8; 250 on 72 and 64 sequences
+// of the decode model 1 to 2 % less in one run, which is what runs differ by there.  The split: 88 x 128 + 192 x 256 + 40 x 128 =
+// 65536, what 512 threads start with.
 template <bool kGateUp, int N_MAX>
 constexpr bool kF8FourGather = kGateUp && N_MAX == 64;
 constexpr int kF8Tables = 2;   // scale tables: the unit being promoted and the prefetched next one

@@ -12,8 +12,8 @@
 // Promotion works on 32 columns at a time, the next load under way while one is multiplied; its eight warps (a lane
 // quarter and half of the columns each) hold 128 sums and two loads in registers, which is why the other four warps
 // hand registers over to them.
-// 36 experts of 3 x 4096 x 1536, whole layer, against the 64-row kernel's form on 128-row tiles: 2000 tokens 951 / 542 us
-// (gate/up 528 / 285, down 305 / 160), 1000 tokens 522 / 326, 500 tokens 314 / 215.  What bounds it now: per K block 48 KB
+// 36 experts of 3 x 4096 x 1536, whole layer, against the 64-row kernel's form on 128-row tiles, forwards on three weight sets
+// in turn: 2000 tokens 917 / 581 us, 1000 tokens 524 / 353, 500 tokens 317 / 222.  What bounds it now: per K block 48 KB
 // through L2 (210 us of the gate/up GEMM at 2000 tokens with everything else taken out), the promotion, which only half
 // overlaps it, and 5 us of epilogue per gate/up unit.
 //
@@ -538,7 +538,7 @@ grouped_gemm_fp8_wide_kernel(const __grid_constant__ CUtensorMap tmap_w, const _
 
       // The unit is cut along K: park the sums, [block][column / 4][row][4]; the quarter that arrives last adds the segments
       // in K order, straight into its outputs (sum_16).  Summed up in the registers of the K loop instead, these few lines
-      // made the compiler spill in that loop (layer at 2000 tokens: 585 us against 542).
+      // made the compiler spill in that loop (layer at 2000 tokens: 8 % slower).
       const bool cut_unit = sg.nseg > 1;
       bool finish = true;
       const int half = kF8BlockM * slot_cols;

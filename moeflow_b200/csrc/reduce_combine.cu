@@ -41,8 +41,8 @@ __device__ __forceinline__ uint4 pack_bf16x8(const float (&acc)[8]) {
 }
 
 // kThreads: kRowThreads, or 512 where a row has more 16-byte chunks than that and there are only a few hundred rows: one round
-// trip to L2 behind the down GEMM instead of two.  Layer, 256 / 512 threads: 128 rows 103.5 / 101.0 us, 256 rows 355 / 351.5;
-// a thousand rows and more fill the SMs either way.
+// trip to L2 behind the down GEMM instead of two.  Layer (36 bf16 experts), 256 / 512 threads: 64 rows 248.2 / 247.5 us, 128 rows
+// 255.2 / 254.0, 256 rows 287 / 272; above, no gain that lasts: 300 rows 287 / 283, 400 rows 322 / 320, 512 rows 368 / 376.
 template <int kThreads>
 __global__ void __launch_bounds__(kThreads) owner_reduce_push_kernel(const mf_reduce_push_args a) {
   __shared__ int s_pos[32];
