@@ -282,34 +282,86 @@ __device__ __forceinline__ void tc_fence_before_sync() {
 __device__ __forceinline__ void tc_fence_after_sync() {
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 }
-// D[tmem] (+)= A[smem desc] * B[smem desc]^T, bf16/f16 inputs, fp32 accumulate.  One thread issues.
-__device__ __forceinline__ void umma_f16(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
-                                         uint32_t accumulate) {
+// One K block of 128 bytes: D[tmem] (+)= A[smem desc] * B[smem desc]^T in four instructions of 32 bytes of K each (16 values of
+// bf16 / f16, 32 of 8-bit floats), fp32 accumulate; with kTwo the same for a second accumulator and A tile.  `accumulate` 0: the
+// first instruction overwrites.  The whole warp calls, with the same operands in every lane, and one elected lane issues
+// (elect.sync names the same lane every time, so commits track these).  Issued one by one under `if (lane == 0)` an
+// instruction cost its warp about 100 cycles: the operands live in uniform registers, and behind a test of the lane number the
+// compiler has to move each of them there again.  K blocks of 16 KB of e4m3 weights were bound by that (128 tokens on 288
+// experts, down GEMM 273 / 205 us; 8 tokens 77 / 59), and of 32 KB by a little (gate/up 117 / 111 at 8 tokens).
+#define MF_UMMA_BLOCK(KIND)                                                                  \
+  asm volatile(                                                                              \
+      "{\n\t"                                                                                \
+      ".reg .pred one, more, first;\n\t"                                                     \
+      ".reg .b64 a1, a2, a3, b1, b2, b3;\n\t"                                                \
+      "elect.sync _|one, 0xffffffff;\n\t"                                                    \
+      "setp.ne.b32 first, %4, 0;\n\t"                                                        \
+      "setp.eq.b32 more, 0, 0;\n\t"                                                          \
+      "add.u64 a1, %1, 2;\n\tadd.u64 a2, %1, 4;\n\tadd.u64 a3, %1, 6;\n\t"                   \
+      "add.u64 b1, %2, 2;\n\tadd.u64 b2, %2, 4;\n\tadd.u64 b3, %2, 6;\n\t"                   \
+      "@one tcgen05.mma.cta_group::1.kind::" KIND " [%0], %1, %2, %3, first;\n\t"            \
+      "@one tcgen05.mma.cta_group::1.kind::" KIND " [%0], a1, b1, %3, more;\n\t"             \
+      "@one tcgen05.mma.cta_group::1.kind::" KIND " [%0], a2, b2, %3, more;\n\t"             \
+      "@one tcgen05.mma.cta_group::1.kind::" KIND " [%0], a3, b3, %3, more;\n\t"             \
+      "}" ::"r"(d), "l"(a), "l"(b), "r"(idesc), "r"(accumulate)                              \
+      : "memory")
+#define MF_UMMA_BLOCK_TWO(KIND)                                                              \
+  asm volatile(                                                                              \
+      "{\n\t"                                                                                \
+      ".reg .pred one, more, first;\n\t"                                                     \
+      ".reg .b64 a1, a2, a3, b1, b2, b3, c1, c2, c3;\n\t"                                    \
+      "elect.sync _|one, 0xffffffff;\n\t"                                                    \
+      "setp.ne.b32 first, %4, 0;\n\t"                                                        \
+      "setp.eq.b32 more, 0, 0;\n\t"                                                          \
+      "add.u64 a1, %1, 2;\n\tadd.u64 a2, %1, 4;\n\tadd.u64 a3, %1, 6;\n\t"                   \
+      "add.u64 b1, %2, 2;\n\tadd.u64 b2, %2, 4;\n\tadd.u64 b3, %2, 6;\n\t"                   \
+      "add.u64 c1, %6, 2;\n\tadd.u64 c2, %6, 4;\n\tadd.u64 c3, %6, 6;\n\t"                   \
+      "@one tcgen05.mma.cta_group::1.kind::" KIND " [%0], %1, %2, %3, first;\n\t"            \
+      "@one tcgen05.mma.cta_group::1.kind::" KIND " [%5], %6, %2, %3, first;\n\t"            \
+      "@one tcgen05.mma.cta_group::1.kind::" KIND " [%0], a1, b1, %3, more;\n\t"             \
+      "@one tcgen05.mma.cta_group::1.kind::" KIND " [%5], c1, b1, %3, more;\n\t"             \
+      "@one tcgen05.mma.cta_group::1.kind::" KIND " [%0], a2, b2, %3, more;\n\t"             \
+      "@one tcgen05.mma.cta_group::1.kind::" KIND " [%5], c2, b2, %3, more;\n\t"             \
+      "@one tcgen05.mma.cta_group::1.kind::" KIND " [%0], a3, b3, %3, more;\n\t"             \
+      "@one tcgen05.mma.cta_group::1.kind::" KIND " [%5], c3, b3, %3, more;\n\t"             \
+      "}" ::"r"(d), "l"(a), "l"(b), "r"(idesc), "r"(accumulate), "r"(d2), "l"(a2nd)          \
+      : "memory")
+// bf16 / f16 (kind::f16) or 8-bit floats (kind::f8f6f4); the types stand in idesc.
+template <bool kF8>
+__device__ __forceinline__ void umma_block(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t accumulate) {
+  if (kF8) MF_UMMA_BLOCK("f8f6f4");
+  else MF_UMMA_BLOCK("f16");
+}
+template <bool kF8>
+__device__ __forceinline__ void umma_block(uint32_t d, uint32_t d2, uint64_t a, uint64_t a2nd, uint64_t b, uint32_t idesc,
+                                           uint32_t accumulate) {
+  if (kF8) MF_UMMA_BLOCK_TWO("f8f6f4");
+  else MF_UMMA_BLOCK_TWO("f16");
+}
+#undef MF_UMMA_BLOCK
+#undef MF_UMMA_BLOCK_TWO
+// True in one lane of the warp, always the same (the whole warp calls).  For code that one lane runs, in place of a test of the lane
+// number: see umma_block.
+__device__ __forceinline__ bool elect_one() {
+  uint32_t r;
   asm volatile(
       "{\n\t"
-      ".reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t"
-      "}" ::"r"(d_tmem),
-      "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
-      : "memory");
+      ".reg .pred one;\n\t"
+      "elect.sync _|one, 0xffffffff;\n\t"
+      "selp.u32 %0, 1, 0, one;\n\t"
+      "}"
+      : "=r"(r)::"memory");
+  return r != 0;
 }
-// Same, 8-bit float inputs (e4m3/e5m2 selected in idesc), K = 32 per instruction.
-__device__ __forceinline__ void umma_f8(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
-                                        uint32_t accumulate) {
-  asm volatile(
-      "{\n\t"
-      ".reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f8f6f4 [%0], %1, %2, %3, p;\n\t"
-      "}" ::"r"(d_tmem),
-      "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
-// The mbarrier gets one arrival when every tcgen05 operation issued so far by this thread is done.
+// The mbarrier gets one arrival when every tcgen05 operation that the elected lane has issued so far is done (whole warp calls).
 __device__ __forceinline__ void umma_commit(uint64_t* bar) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar))
-               : "memory");
+  asm volatile(
+      "{\n\t"
+      ".reg .pred one;\n\t"
+      "elect.sync _|one, 0xffffffff;\n\t"
+      "@one tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t"
+      "}" ::"r"(smem_u32(bar))
+      : "memory");
 }
 // 32 lanes x 16 consecutive fp32 columns: thread i of the warp gets lane (base_lane + i).
 __device__ __forceinline__ void tmem_ld_16(uint32_t taddr, uint32_t (&r)[16]) {

@@ -214,7 +214,7 @@ grouped_gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid
             if (lane == 0) report_status(a.status, kGemmEmptyTimeout, 0, blockIdx.x, 0);
             break;
           }
-          if (lane == 0) {
+          if (elect_one()) {
             mbar_arrive_expect_tx(&full_bar[st.stage], Cfg::kStageA);
             uint8_t* dst = sA + st.stage * Cfg::kStageA;
             tma_load_2d(dst, &tmap_w, &full_bar[st.stage], kb * 128, row0, policy);
@@ -252,21 +252,14 @@ grouped_gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid
             break;
           }
           tc_fence_after_sync();
-          if (lane == 0) {
-            fence_proxy_async_smem();
-            const uint32_t d0 = tmem_base + tmp.stage * Cfg::kTmpCols;
-            const uint32_t a_addr = smem_u32(sA + st.stage * Cfg::kStageA);
-            const uint32_t b_addr = smem_u32(sB + st.stage * Cfg::kStageB);
-#pragma unroll
-            for (int k = 0; k < 4; ++k) {
-              const uint64_t bdesc = umma_desc_sw128(b_addr + k * 32);
-              umma_f8(d0, umma_desc_sw128(a_addr + k * 32), bdesc, idesc, k > 0 ? 1u : 0u);
-              if (kGateUp) umma_f8(d0 + N_MAX, umma_desc_sw128(a_addr + kF8TileA + k * 32), bdesc, idesc, k > 0 ? 1u : 0u);
-            }
-            umma_commit(&empty_bar[st.stage]);
-            umma_commit(&tmp_full[tmp.stage]);
-          }
-          __syncwarp();
+          if (!b_tma) fence_proxy_async_smem();  // the gathered rows
+          const uint32_t d0 = tmem_base + tmp.stage * Cfg::kTmpCols;
+          const uint64_t a_desc = umma_desc_sw128(smem_u32(sA + st.stage * Cfg::kStageA));
+          const uint64_t b_desc = umma_desc_sw128(smem_u32(sB + st.stage * Cfg::kStageB));
+          if (kGateUp) umma_block<true>(d0, d0 + N_MAX, a_desc, a_desc + (kF8TileA >> 4), b_desc, idesc, 0u);
+          else umma_block<true>(d0, a_desc, b_desc, idesc, 0u);
+          umma_commit(&empty_bar[st.stage]);
+          umma_commit(&tmp_full[tmp.stage]);
           st.advance(STAGES);
           tmp.advance(Cfg::kTmpStages);
         }
@@ -281,7 +274,8 @@ grouped_gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid
         if (a.tile_wait != nullptr && sg.tt != ready_tile) {
           ok = tile_ready(sg.tt);
           if (!ok) break;
-          if (lane == 0) fence_proxy_async_all();  // the TMA reads below come after the acquire
+          __syncwarp();
+          fence_proxy_async_all();  // the TMA reads below, by whichever lane, come after the acquire
           ready_tile = sg.tt;
         }
         for (int j = 0; j < sg.nkb; ++j) {
@@ -291,7 +285,7 @@ grouped_gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid
             if (lane == 0) report_status(a.status, kGemmEmptyTimeout, 2, blockIdx.x, 0);
             break;
           }
-          if (lane == 0) {
+          if (elect_one()) {
             mbar_arrive_expect_tx(&full_bar[st.stage], Cfg::kStageB);
             tma_load_2d(sB + st.stage * Cfg::kStageB, &tmap_b, &full_bar[st.stage], kb * 128, sg.row_start);
           }

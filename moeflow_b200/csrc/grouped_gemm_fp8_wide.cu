@@ -240,7 +240,7 @@ grouped_gemm_fp8_wide_kernel(const __grid_constant__ CUtensorMap tmap_w, const _
             if (lane == 0) report_status(a.status, kGemmEmptyTimeout, 0, blockIdx.x, 0);
             break;
           }
-          if (lane == 0) {
+          if (elect_one()) {
             mbar_arrive_expect_tx(&full_bar[st.stage], two ? 2 * kF8TileA : kF8TileA);
             uint8_t* dst = sW + st.stage * kFwStageW;
             tma_load_2d(dst, &tmap_w, &full_bar[st.stage], kb * 128, row0);
@@ -276,18 +276,11 @@ grouped_gemm_fp8_wide_kernel(const __grid_constant__ CUtensorMap tmap_w, const _
             break;
           }
           tc_fence_after_sync();
-          if (lane == 0) {
-            if (kGather) fence_proxy_async_smem();  // the gathered rows
-            const uint32_t d = tmem_base + tmp.stage * 256;
-            const uint32_t x_addr = smem_u32(sX + st.stage * kFwStageX);
-            const uint32_t w_addr = smem_u32(sW + st.stage * kFwStageW);
-#pragma unroll
-            for (int k = 0; k < 4; ++k)
-              umma_f8(d, umma_desc_sw128(x_addr + k * 32), umma_desc_sw128(w_addr + k * 32), idesc, k > 0 ? 1u : 0u);
-            umma_commit(&empty_bar[st.stage]);
-            umma_commit(&tmp_full[tmp.stage]);
-          }
-          __syncwarp();
+          if (kGather) fence_proxy_async_smem();  // the gathered rows
+          umma_block<true>(tmem_base + tmp.stage * 256, umma_desc_sw128(smem_u32(sX + st.stage * kFwStageX)),
+                           umma_desc_sw128(smem_u32(sW + st.stage * kFwStageW)), idesc, 0u);
+          umma_commit(&empty_bar[st.stage]);
+          umma_commit(&tmp_full[tmp.stage]);
           st.advance(kFwStages);
           tmp.advance(kFwTmp);
         }
@@ -303,7 +296,8 @@ grouped_gemm_fp8_wide_kernel(const __grid_constant__ CUtensorMap tmap_w, const _
         if (a.tile_wait != nullptr && sg.tt != ready_tile) {
           ok = tile_ready(sg.tt);
           if (!ok) break;
-          if (lane == 0) fence_proxy_async_all();  // the TMA reads below come after the acquire
+          __syncwarp();
+          fence_proxy_async_all();  // the TMA reads below, by whichever lane, come after the acquire
           ready_tile = sg.tt;
         }
         const int n_box = (sg.n_rows + box_rows - 1) / box_rows;
@@ -314,7 +308,7 @@ grouped_gemm_fp8_wide_kernel(const __grid_constant__ CUtensorMap tmap_w, const _
             if (lane == 0) report_status(a.status, kGemmEmptyTimeout, 2, blockIdx.x, 0);
             break;
           }
-          if (lane == 0) {
+          if (elect_one()) {
             // rows behind the tile (the next one's, or zero fill) end up in accumulator rows that are not looked at
             uint8_t* dst = sX + st.stage * kFwStageX;
             mbar_arrive_expect_tx(&full_bar[st.stage], n_box * box_rows * 128);

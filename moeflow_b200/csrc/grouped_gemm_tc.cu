@@ -486,7 +486,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
             if (lane == 0) report_status(a.status, kGemmEmptyTimeout, 0, blockIdx.x, 0);
             break;
           }
-          if (lane == 0) {
+          if (elect_one()) {
             mbar_arrive_expect_tx(&full_bar[st.stage], Cfg::kStageA);
             uint8_t* dst = sA + st.stage * Cfg::kStageA;
             if (trace && trace[2] == 0) trace[2] = global_timer_ns();  // see the note at MF_STAMP_ONCE
@@ -535,28 +535,17 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
             break;
           }
           tc_fence_after_sync();
-          if (lane == 0) {
-            fence_proxy_async_smem();
-            const uint32_t a_addr = smem_u32(sA + st.stage * Cfg::kStageA);
-            const uint32_t b_addr = smem_u32(sB + st.stage * Cfg::kStageB);
-#pragma unroll
-            for (int k = 0; k < 4; ++k) {
-              const uint64_t bdesc = umma_desc_sw128(b_addr + k * 32);
-              const uint32_t accum = (j > 0 || k > 0) ? 1u : 0u;
-              umma_f16(d0, umma_desc_sw128(a_addr + k * 32), bdesc, idesc, accum);
-              if (kGateUp) umma_f16(d1, umma_desc_sw128(a_addr + kTileBytesA + k * 32), bdesc, idesc, accum);
-            }
-            umma_commit(&empty_bar[st.stage]);
-          }
-          __syncwarp();
+          if (!b_tma) fence_proxy_async_smem();  // the gathered rows
+          const uint64_t a_desc = umma_desc_sw128(smem_u32(sA + st.stage * Cfg::kStageA));
+          const uint64_t b_desc = umma_desc_sw128(smem_u32(sB + st.stage * Cfg::kStageB));
+          if (kGateUp) umma_block<false>(d0, d1, a_desc, a_desc + (kTileBytesA >> 4), b_desc, idesc, j > 0 ? 1u : 0u);
+          else umma_block<false>(d0, a_desc, b_desc, idesc, j > 0 ? 1u : 0u);
+          umma_commit(&empty_bar[st.stage]);
           st.advance(STAGES);
         }
         if (!ok) break;
-        if (lane == 0) {
-          umma_commit(&acc_full[acc.stage]);
-          if (wide) umma_commit(&acc_full[acc2.stage]);
-        }
-        __syncwarp();
+        umma_commit(&acc_full[acc.stage]);
+        if (wide) umma_commit(&acc_full[acc2.stage]);
         acc.advance(Cfg::kAccStages);
         if (wide) acc.advance(Cfg::kAccStages);
       }
@@ -572,11 +561,10 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
           if (a.tile_wait != nullptr && sg.tt != ready_tile) {
             // the tile's activations are final once every gate/up unit of the tile has reported its four quarters
             bool got = true;
-            if (lane == 0) {
-              got = wait_count_ge_gpu(a.tile_wait + sg.tt, a.tile_wait_target, wait_ns);
-              fence_proxy_async_all();  // the TMA reads below come after the acquire
-            }
+            if (lane == 0) got = wait_count_ge_gpu(a.tile_wait + sg.tt, a.tile_wait_target, wait_ns);
             ok = __all_sync(0xffffffffu, got);
+            __syncwarp();
+            fence_proxy_async_all();  // the TMA reads below, by whichever lane, come after the acquire
             if (!ok) {
               if (lane == 0) {
                 *abort_flag = 1;
@@ -595,7 +583,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
               if (lane == 0) report_status(a.status, kGemmEmptyTimeout, 2, blockIdx.x, 0);
               break;
             }
-            if (lane == 0) {
+            if (elect_one()) {
               // as many boxes as hold the tile's rows: rows past the tile (the next expert's entries, or zero fill
               // past the end of the buffer) land in smem rows the MMA does not read or in accumulator columns the
               // epilogue skips

@@ -137,26 +137,21 @@ skinny_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
     }
     __syncwarp();
   } else if (warp == 1) {
-    if (lane == 0) {
-      const uint32_t idesc = umma_idesc(1, 1, kSkM, (uint32_t)n_tile);
-      bool ok = true;
-      for (int j = 0; j < nkb; ++j) {
-        const int stage = j % kSkStages;
-        ok = mbar_wait_bounded(&full_bar[stage], (uint32_t)(j / kSkStages) & 1u, abort_flag, a.wait_ns);
-        if (!ok) {
-          report_status(a.status, kGemmFullTimeout, 8, blockIdx.x, 0);
-          break;
-        }
-        tc_fence_after_sync();
-        const uint32_t a_addr = smem_u32(smem + stage * kSkStage), b_addr = a_addr + kSkTileA;
-#pragma unroll
-        for (int k = 0; k < 4; ++k)
-          umma_f16(tmem_base, umma_desc_sw128(a_addr + k * 32), umma_desc_sw128(b_addr + k * 32), idesc, (j > 0 || k > 0) ? 1u : 0u);
-        umma_commit(&empty_bar[stage]);
+    const uint32_t idesc = umma_idesc(1, 1, kSkM, (uint32_t)n_tile);
+    bool ok = true;
+    for (int j = 0; j < nkb; ++j) {
+      const int stage = j % kSkStages;
+      ok = __all_sync(0xffffffffu, mbar_wait_bounded(&full_bar[stage], (uint32_t)(j / kSkStages) & 1u, abort_flag, a.wait_ns));
+      if (!ok) {
+        if (lane == 0) report_status(a.status, kGemmFullTimeout, 8, blockIdx.x, 0);
+        break;
       }
-      if (ok) umma_commit(acc_bar);
+      tc_fence_after_sync();
+      const uint32_t a_addr = smem_u32(smem + stage * kSkStage);
+      umma_block<false>(tmem_base, umma_desc_sw128(a_addr), umma_desc_sw128(a_addr + kSkTileA), idesc, j > 0 ? 1u : 0u);
+      umma_commit(&empty_bar[stage]);
     }
-    __syncwarp();
+    if (ok) umma_commit(acc_bar);
   } else {
     // tensor memory -> this CTA's partial tile [column][row] (a warp writes 32 consecutive words: no bank conflicts).
     // The accumulator is complete, so every stage has been read and no copy is in flight.
