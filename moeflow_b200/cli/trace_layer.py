@@ -9,7 +9,8 @@ tensor memory, first group stored, all groups stored), the transport kernels sta
 fenced, arrivals sent, last CTA done; metadata: entry, dispatch complete, flags seen, loads issued, warp 0's histogram, histogram,
 plan written, entries placed; reduce + push: entry, GEMM complete, row stored, fenced, -, last CTA done; combine: entry,
 predecessor complete, return flags seen, row written).  On one rank the dispatch launch builds the metadata at decode
-sizes (its last CTA then stamps the metadata phases) and the reduce writes the output: nothing is fenced or sent, and no
+sizes (its last CTA then stamps the metadata phases; with up to 16 token positions that CTA stamps "rows stored" as well, when
+it has the slot words of all rows) and the reduce writes the output: nothing is fenced or sent, and no
 combine is launched.  The layer is captured in a CUDA graph, replayed with a
 cold L2, and the stamps are printed in microseconds relative to the first one, so the gaps between kernels
 (launch chain, grid dependencies, fences) can be read directly.  One GPU; ``--experts`` sets the local expert

@@ -252,17 +252,70 @@ __global__ void __launch_bounds__(32 * kManyWarps) dispatch_push_many_kernel(con
 // The layout is there, from the kernel's start and between passes that stream weights: 1 token on 288 experts 9.0 us (13.1
 // with the router's scores in shared memory, the payload in front of the fence and the metadata pass unrolled throughout),
 // 128 tokens 13.4 (19.6).
+//
+// Up to kLocalThreads / 32 token positions one more CTA, the bookkeeper, routes all of them for itself, a warp each, and
+// builds the layout from shared memory: nothing of it goes through L2 (slot words, fence, arrival and the loads behind it took
+// 2.3 us), and the tokens' own CTAs only store their rows.  Layout after 7.0 instead of 9.2 us at 1 token on 288 experts, 4.6
+// instead of 6.7 on 32; calls, us: 1 token 69.2 / 67.2 (32 experts of hidden 512, 8 tokens: 26.4 / 23.2), 8 tokens e4m3
+// 169.9 / 167.4, decode model of 4 sequences 217 / 211.  Above, a warp would route several tokens one after the other, 1 us each.
 constexpr int kLocalThreads = 512;
+constexpr int kLocalWarps = kLocalThreads / 32;
+constexpr int kKeeperSmem = 112 * 1024;
+
+__device__ __forceinline__ void bookkeeper(const mf_dispatch_args& a, const mf_meta_args& m, int* s_dyn) {
+  __shared__ int s_key[kLocalWarps * kMaxTopK], s_bits[kLocalWarps * kMaxTopK];
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, t = warp;
+  unsigned long long* trace = (m.trace != nullptr && tid == 0) ? m.trace : nullptr;
+  grid_dep_launch();
+  if (warp == kLocalWarps - 1 && lane < 12) {
+    // the pages that the metadata pass stores to
+    const void* p = lane == 0 ? (const void*)m.plan : lane == 1 ? (const void*)m.offsets : lane == 2 ? (const void*)m.tile_e
+                  : lane == 3 ? (const void*)m.tile_s : lane == 4 ? (const void*)m.tile_n : lane == 5 ? (const void*)m.row_hits
+                  : lane == 6 ? (const void*)m.inv : lane == 7 ? (const void*)m.entry_row : lane == 8 ? (const void*)m.entry_slot
+                  : lane == 9 ? (const void*)m.entry_w : lane == 10 ? (const void*)(m.counters1 + m.n_counters1) : (const void*)a.epoch;
+    touch(p);
+  }
+  if (t < a.C) {
+    const bool has_token = t < a.T;
+    float w = 0.f;
+    int id = -1;  // lane k (< K): slot k
+    if (has_token) {
+      if (a.logits != nullptr) {
+        float* score = reinterpret_cast<float*>(s_dyn + meta_smem_words(m.L, kLocalThreads)) + (size_t)warp * 2 * a.E;
+        const RouteParams p{a.E, a.K, a.n_group, a.topk_group, a.sigmoid, a.renorm, a.scale};
+        route_token_warp(a.logits + (size_t)t * a.E, a.bias, score, score + a.E, p, lane, w, id);
+      } else if (lane < a.K) {
+        id = a.ids[(size_t)t * a.K + lane];
+        w = a.weights[(size_t)t * a.K + lane];
+      }
+    }
+    const bool on = has_token && (a.num_valid == nullptr || t < *a.num_valid) && id >= 0 && id < a.L;
+    if (lane < a.K) {
+      s_key[t * a.K + lane] = on ? id : -1;
+      s_bits[t * a.K + lane] = on ? __float_as_int(w) : 0;
+    }
+  }
+  meta_begin<kLocalThreads>(m, s_dyn);
+  __syncthreads();
+  if (a.trace != nullptr && tid == 0) a.trace[2] = global_timer_ns();  // the slot words stand in shared memory
+  if (tid == 0) *a.epoch += 1u;
+  meta_one_pass<kLocalThreads>(m, SharedSlots{s_key, s_bits, a.K}, s_dyn, trace);
+}
 
 // kPerSm: CTAs an SM should hold.  With at most one token per SM the registers for one CTA are free and nothing spills; above
 // that two share an SM (500 tokens: 1 % of the layer).
-template <int kPerSm>
+// kKeeper: the last CTA is the bookkeeper (kernels of their own: with both forms in one the larger sizes lost 0.7 %).
+template <int kPerSm, bool kKeeper>
 __global__ void __launch_bounds__(kLocalThreads, kPerSm) dispatch_local_kernel(const mf_dispatch_args a, const mf_meta_args m) {
   extern __shared__ int s_dyn[];  // metadata pass, then the router's scores
   __shared__ int s_id[kMaxTopK];
   __shared__ float s_w[kMaxTopK];
   __shared__ int s_last;
   const int t = blockIdx.x, tid = threadIdx.x;
+  if (kKeeper && t == a.C) {
+    bookkeeper(a, m, s_dyn);
+    return;
+  }
   unsigned long long* trace = (a.trace != nullptr && blockIdx.x == 0 && tid == 0) ? a.trace : nullptr;
   if (trace) trace[0] = global_timer_ns();
   grid_dep_launch();
@@ -300,7 +353,7 @@ __global__ void __launch_bounds__(kLocalThreads, kPerSm) dispatch_local_kernel(c
     }
   } else {
     // in the shadow of the routing warp: the pages that the metadata pass stores to, and its histogram
-    if (tid < 48) {
+    if (tid < 48 && (!kKeeper || tid == 43 || tid == 46)) {
       const void* p = tid == 32 ? (const void*)m.plan : tid == 33 ? (const void*)m.offsets : tid == 34 ? (const void*)m.tile_e
                     : tid == 35 ? (const void*)m.tile_s : tid == 36 ? (const void*)m.tile_n : tid == 37 ? (const void*)m.row_hits
                     : tid == 38 ? (const void*)m.inv : tid == 39 ? (const void*)m.entry_row : tid == 40 ? (const void*)m.entry_slot
@@ -310,7 +363,7 @@ __global__ void __launch_bounds__(kLocalThreads, kPerSm) dispatch_local_kernel(c
       touch(p);
     }
   }
-  meta_begin<kLocalThreads>(m, s_dyn);
+  if (!kKeeper) meta_begin<kLocalThreads>(m, s_dyn);
   __syncthreads();
   if (trace) trace[1] = global_timer_ns();  // routed, hidden row loaded
   int present = 0;
@@ -330,7 +383,7 @@ __global__ void __launch_bounds__(kLocalThreads, kPerSm) dispatch_local_kernel(c
       a.hit[t] = (unsigned char)present;
     }
     __syncwarp();
-    if (tid == 0) {
+    if (tid == 0 && !kKeeper) {
       __threadfence();  // cumulative: the whole warp's stores, ordered by the barrier
       const unsigned done = atomicAdd(a.done_counter, 1u);
       __threadfence();  // in the last CTA: every other CTA's words come before what follows
@@ -352,10 +405,11 @@ __global__ void __launch_bounds__(kLocalThreads, kPerSm) dispatch_local_kernel(c
       }
     }
   }
+  if (kKeeper) return;
   __syncthreads();
   if (trace) trace[2] = global_timer_ns();  // row stored
   if (!s_last) return;
-  meta_one_pass<kLocalThreads>(m, s_dyn, (m.trace != nullptr && tid == 0) ? m.trace : nullptr);
+  meta_one_pass<kLocalThreads>(m, RowSlots(m), s_dyn, (m.trace != nullptr && tid == 0) ? m.trace : nullptr);
 }
 
 }  // namespace mf
@@ -369,16 +423,31 @@ extern "C" int mf_dispatch_local(const mf_dispatch_args* a, const mf_meta_args* 
   if (m->L < 1 || m->L > kLocalThreads || (long long)a->C * a->K > kLocalThreads * kMetaBatch) return -2;
   if (m->xq != nullptr && (!m->xs || a->H % 128 != 0)) return -3;
   size_t smem = (size_t)meta_smem_words(m->L, kLocalThreads) * sizeof(int);
+  const bool keeper = a->C <= kLocalWarps;
   if (a->logits != nullptr) {
     if (a->E < a->K || a->E != a->L || a->n_group < 1 || a->n_group > 32 || a->E % a->n_group != 0 || !a->route_w || !a->route_ids)
       return -4;
-    smem += 2 * (size_t)a->E * sizeof(float);
+    smem += 2 * (size_t)a->E * sizeof(float) * (keeper ? a->C : 1);
   }
-  if (smem > 48 * 1024) return -5;  // L = E <= 512: at most 41 KB
-  if (a->C <= m->n_sms)
-    dispatch_local_kernel<1><<<a->C, kLocalThreads, smem, static_cast<cudaStream_t>(stream)>>>(*a, *m);
-  else
-    dispatch_local_kernel<2><<<a->C, kLocalThreads, smem, static_cast<cudaStream_t>(stream)>>>(*a, *m);
+  // L = E <= 512: at most 41 KB, with a bookkeeper 102 KB
+  if (smem > (keeper ? kKeeperSmem : 48 * 1024)) return -5;
+  const cudaStream_t st = static_cast<cudaStream_t>(stream);
+  if (keeper) {
+    static bool configured[64] = {};  // per device: the attribute belongs to (function, device)
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return (int)e;
+    if (dev < 0 || dev >= 64 || !configured[dev]) {
+      e = cudaFuncSetAttribute(dispatch_local_kernel<1, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kKeeperSmem);
+      if (e != cudaSuccess) return (int)e;
+      if (dev >= 0 && dev < 64) configured[dev] = true;
+    }
+    dispatch_local_kernel<1, true><<<a->C + 1, kLocalThreads, smem, st>>>(*a, *m);
+  } else if (a->C <= m->n_sms) {
+    dispatch_local_kernel<1, false><<<a->C, kLocalThreads, smem, st>>>(*a, *m);
+  } else {
+    dispatch_local_kernel<2, false><<<a->C, kLocalThreads, smem, st>>>(*a, *m);
+  }
   return (int)cudaGetLastError();
 }
 

@@ -274,7 +274,7 @@ __global__ void __launch_bounds__(kMetaThreads) expert_meta_small_kernel(const m
   __syncthreads();
   if (trace) trace[2] = global_timer_ns();  // flags seen
 
-  meta_one_pass<kMetaThreads>(a, sm, trace);
+  meta_one_pass<kMetaThreads>(a, RowSlots(a), sm, trace);
 }
 
 

@@ -166,8 +166,34 @@ __device__ __forceinline__ void meta_begin(const mf_meta_args& a, int* sm) {
   if (threadIdx.x == 0) sm[kThreads / 32 * P + 2 * a.L + 34] = sm[kThreads / 32 * P + 2 * a.L + 35] = 0;
 }
 
-template <int kThreads>
-__device__ __forceinline__ void meta_one_pass(const mf_meta_args& a, int* sm, unsigned long long* trace) {
+// Slot words of the received rows.  `valid`: the row's flag, 0 for a row without an entry here.
+struct RowSlots {
+  const uint8_t* recv;
+  long long pitch;
+  size_t meta_off;
+  int K;
+  __device__ __forceinline__ explicit RowSlots(const mf_meta_args& a)
+      : recv(static_cast<const uint8_t*>(a.recv)), pitch(a.pitch), meta_off((size_t)a.H * 2), K(a.K) {}
+  __device__ __forceinline__ void get(int row, int slot, int& id, int& valid, int& wbits) const {
+    const int* meta = reinterpret_cast<const int*>(recv + (size_t)row * pitch + meta_off);
+    id = __ldcg(meta + slot);
+    valid = __ldcg(meta + 2 * K);
+    wbits = __ldcg(meta + K + slot);
+  }
+};
+// The same words, [row][K] each, in shared memory.
+struct SharedSlots {
+  const int *id, *wbits;
+  int K;
+  __device__ __forceinline__ void get(int row, int slot, int& id_, int& valid, int& wbits_) const {
+    id_ = id[row * K + slot];
+    valid = 1;
+    wbits_ = wbits[row * K + slot];
+  }
+};
+
+template <int kThreads, typename Slots>
+__device__ __forceinline__ void meta_one_pass(const mf_meta_args& a, const Slots& slots, int* sm, unsigned long long* trace) {
   constexpr int kWarps = kThreads / 32;
   const int L = a.L, K = a.K, P = hist_pitch(a.L);
   int* hist = sm;                       // [kWarps][P]
@@ -178,11 +204,9 @@ __device__ __forceinline__ void meta_one_pass(const mf_meta_args& a, int* sm, un
   const MetaSpan span(a, kWarps);
   const int N = span.N, n_warps = span.n_warps;
   const int begin = min(N, warp * span.per), end = min(N, (warp + 1) * span.per);
-  const uint8_t* recv = static_cast<const uint8_t*>(a.recv);
-  const size_t meta_off = (size_t)a.H * 2;
   int* my_hist = hist + warp * P;
 
-  // The only reads of the received rows: id, valid flag and weight bits of every slot word of this thread, none of them
+  // The only reads of the slot words: id, valid flag and weight bits of every slot word of this thread, none of them
   // used before all are requested.
   // Every instruction of this pass runs once, so it costs what its fetch costs (about 4 cycles each): the loops over batches
   // leave at the first empty one, and no loop is unrolled further than its usual count.  With all eight batches walked
@@ -196,11 +220,8 @@ __device__ __forceinline__ void meta_one_pass(const mf_meta_args& a, int* sm, un
     key[b] = -1;
     wbits[b] = flag[b] = 0;
     if (i < end) {
-      const int row = i / K, slot = i - row * K;
-      const int* meta = reinterpret_cast<const int*>(recv + (size_t)row * a.pitch + meta_off);
-      key[b] = __ldcg(meta + slot);
-      flag[b] = __ldcg(meta + 2 * K);
-      wbits[b] = __ldcg(meta + K + slot);
+      const int row = i / K;
+      slots.get(row, i - row * K, key[b], flag[b], wbits[b]);
     }
   }
   if (trace) trace[6] = global_timer_ns();  // loads issued
@@ -265,13 +286,12 @@ __device__ __forceinline__ void meta_one_pass(const mf_meta_args& a, int* sm, un
     // general K: rows do not line up with warp steps; count their hits from the rows (cache hits by now)
     int mine = 0;
     for (int r = tid; r < a.rows; r += kThreads) {
-      const int* meta = reinterpret_cast<const int*>(recv + (size_t)r * a.pitch + meta_off);
       int hits = 0;
-      if (__ldcg(meta + 2 * K) != 0)
-        for (int k = 0; k < K; ++k) {
-          const int id = __ldcg(meta + k);
-          hits += (id >= 0 && id < L) ? 1 : 0;
-        }
+      for (int k = 0; k < K; ++k) {
+        int id, valid, wb;
+        slots.get(r, k, id, valid, wb);
+        hits += (valid != 0 && id >= 0 && id < L) ? 1 : 0;
+      }
       if (a.row_hits != nullptr) a.row_hits[r] = hits;
       mine += hits > 0 ? 1 : 0;
     }
@@ -309,10 +329,10 @@ __device__ __forceinline__ void meta_one_pass(const mf_meta_args& a, int* sm, un
     int cols = (warp_sums[34] + 15) & ~15;
     if (cols < 16) cols = 16;
     const bool second = (lane & 4) != 0;
-    int slots = a.max_split_slots;
+    int room = a.max_split_slots;
     if (a.partial_floats > 0)  // partial tiles of 256 * cols floats (two accumulators) or 128 * cols
-      slots = (int)((unsigned)min((long long)0x7fffffff, a.partial_floats >> (second && !a.pair2 ? 7 : 8)) / (unsigned)cols);
-    const int cut = choose_cut_lanes(a, nt * (second ? a.m_blocks2 : a.m_blocks1), second ? a.k_blocks2 : a.k_blocks1, slots,
+      room = (int)((unsigned)min((long long)0x7fffffff, a.partial_floats >> (second && !a.pair2 ? 7 : 8)) / (unsigned)cols);
+    const int cut = choose_cut_lanes(a, nt * (second ? a.m_blocks2 : a.m_blocks1), second ? a.k_blocks2 : a.k_blocks1, room,
                                      second ? 8 : 4, cols, lane & 3);
     if (lane == 0) {
       warp_sums[36] = a.plan[MF_PLAN_SPLIT1] = cut;
