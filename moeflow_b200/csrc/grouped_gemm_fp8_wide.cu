@@ -9,9 +9,13 @@
 //     its own and its scales as broadcasts from shared memory;
 //   * one instruction of 128 x 256 x 32 reads 12 KB of shared memory in the time in which two of 128 x 128 x 32 read 16;
 //   * the epilogue's quantisation group (128 activations of a token) lies in two threads instead of 128.
-// Promotion works on 32 columns at a time, the next load under way while one is multiplied; its eight warps (a lane
+// Promotion works on 16 columns at a time, the next load under way while one is multiplied; its eight warps (a lane
 // quarter and half of the columns each) hold 128 sums and two loads in registers, which is why the other four warps
-// hand registers over to them.
+// hand registers over to them.  Loads of 32 columns leave no registers for anything else, and what the compiler then moves
+// about in the K loop costs more than the waits saved; single multiply-adds, not pairs: the same rate (128 a clock), and no
+// even register numbers to keep to.  Kernels alone, 2000 tokens on 36 experts, us, gate/up and down: 32 columns in pairs 309 /
+// 173, 16 in pairs 320 / 153, 32 single 297 / 161, 16 single 297 / 156.  Of the 297, with parts left out: epilogue 37,
+// multiply-adds 61, the rest (operands through L2, tensor-memory loads) 199.
 // 36 experts of 3 x 4096 x 1536, whole layer, against the 64-row kernel's form on 128-row tiles, forwards on three weight sets
 // in turn: 2000 tokens 917 / 581 us, 1000 tokens 524 / 353, 500 tokens 317 / 222.  What bounds it now: per K block 48 KB
 // through L2 (210 us of the gate/up GEMM at 2000 tokens with everything else taken out), the promotion, which only half
@@ -56,28 +60,13 @@ constexpr int kFwRegsFew = 72, kFwRegsGather = 40;
 template <bool kGather>
 constexpr int kFwRegsMany = kGather ? 200 : 216;
 
-// 32 lanes x 32 consecutive fp32 columns.
-__device__ __forceinline__ void tmem_ld_32(uint32_t taddr, uint32_t (&r)[32]) {
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
-      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
-      "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
-      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
-        "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]), "=r"(r[17]),
-        "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]), "=r"(r[25]), "=r"(r[26]),
-        "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
-      : "r"(taddr)
-      : "memory");
-}
 // Waits for the loads so far.  The loaded values pass through, so that nothing that uses them is moved ahead of the wait.
-__device__ __forceinline__ void tmem_ld_wait_32(uint32_t (&r)[32]) {
+__device__ __forceinline__ void tmem_ld_wait_16(uint32_t (&r)[16]) {
   asm volatile("tcgen05.wait::ld.sync.aligned;"
                : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]), "+r"(r[7]), "+r"(r[8]),
                  "+r"(r[9]), "+r"(r[10]), "+r"(r[11]), "+r"(r[12]), "+r"(r[13]), "+r"(r[14]), "+r"(r[15])
                :
                : "memory");
-  asm volatile("" : "+r"(r[16]), "+r"(r[17]), "+r"(r[18]), "+r"(r[19]), "+r"(r[20]), "+r"(r[21]), "+r"(r[22]), "+r"(r[23]),
-                    "+r"(r[24]), "+r"(r[25]), "+r"(r[26]), "+r"(r[27]), "+r"(r[28]), "+r"(r[29]), "+r"(r[30]), "+r"(r[31]));
 }
 
 // Four partial sums, 16 bytes at a time or (scratch off the 16-byte grid) float by float.  A template, not a test of the address:
@@ -99,10 +88,10 @@ __device__ __forceinline__ float4 parked_4(const float* p) {
   return make_float4(__ldcg(p), __ldcg(p + 1), __ldcg(p + 2), __ldcg(p + 3));
 }
 
-// acc[0..31] += s * p[0..31], both halves of s holding the same scale
-__device__ __forceinline__ void promote_32(f32x2* acc, const uint32_t (&p)[32], f32x2 s) {
+// acc[0..15] += s * p[0..15]
+__device__ __forceinline__ void promote_16(float* acc, const uint32_t (&p)[16], float s) {
 #pragma unroll
-  for (int i = 0; i < 16; ++i) acc[i] = fma2(pack2(p[2 * i], p[2 * i + 1]), s, acc[i]);
+  for (int i = 0; i < 16; ++i) acc[i] = fmaf(__uint_as_float(p[i]), s, acc[i]);
 }
 
 template <bool kGateUp, bool kGather, bool kAligned>
@@ -471,9 +460,9 @@ grouped_gemm_fp8_wide_kernel(const __grid_constant__ CUtensorMap tmap_w, const _
       const int n_rows = sg.n_rows, row_start = sg.row_start;
       const bool live = wq * 32 < n_rows;  // warp-uniform: this quarter holds rows
       const bool two = two_halves(sg);
-      f32x2 acc0[32], acc1[32];  // 64 columns of each half (gate and up, or the two blocks)
+      float acc0[64], acc1[64];  // 64 columns of each half (gate and up, or the two blocks)
 #pragma unroll
-      for (int i = 0; i < 32; ++i) acc0[i] = acc1[i] = 0ull;
+      for (int i = 0; i < 64; ++i) acc0[i] = acc1[i] = 0.f;
       float row_scale = 1.f;  // routing weight of this lane's row, requested ahead of the K loop
       if (!kGateUp && a.row_scale != nullptr && row < n_rows) row_scale = __ldcg(a.row_scale + row_start + row);
 
@@ -490,32 +479,39 @@ grouped_gemm_fp8_wide_kernel(const __grid_constant__ CUtensorMap tmap_w, const _
         if (live) {
           const float* t = sScale + sc.stage * kFwScaleFloats;
           const uint32_t d = lane_base + tmp.stage * 256;
-          uint32_t p[32], q[32];
-          tmem_ld_32(d, p);
           const float xs = t[sub * kFwRows + row];
           const float s0 = t[4 * kFwRows + sub] * xs, s1 = t[4 * kFwRows + 4 + sub] * xs;
-          const f32x2 v0 = pack2(s0, s0), v1 = pack2(s1, s1);
-          tmem_ld_wait_32(p);
+          uint32_t p[16], q[16];
+          auto release = [&]() {  // everything is in registers
+            tc_fence_before_sync();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&tmp_empty[tmp.stage]);
+          };
+          tmem_ld_16(d, p);
+          tmem_ld_wait_16(p);
           if (two) {
-            tmem_ld_32(d + 128, q);
-            promote_32(acc0, p, v0);
-            tmem_ld_wait_32(q);
-            tmem_ld_32(d + 32, p);
-            promote_32(acc1, q, v1);
-            tmem_ld_wait_32(p);
-            tmem_ld_32(d + 160, q);
-            promote_32(acc0 + 16, p, v0);
-            tmem_ld_wait_32(q);
+#pragma unroll
+            for (int c = 0; c < 64; c += 16) {
+              tmem_ld_16(d + 128 + c, q);
+              promote_16(acc0 + c, p, s0);
+              tmem_ld_wait_16(q);
+              if (c < 48) tmem_ld_16(d + c + 16, p);
+              else release();
+              promote_16(acc1 + c, q, s1);
+              if (c < 48) tmem_ld_wait_16(p);
+            }
           } else {
-            tmem_ld_32(d + 32, q);
-            promote_32(acc0, p, v0);
-            tmem_ld_wait_32(q);
+#pragma unroll
+            for (int c = 0; c < 64; c += 32) {
+              tmem_ld_16(d + c + 16, q);
+              promote_16(acc0 + c, p, s0);
+              tmem_ld_wait_16(q);
+              if (c < 32) tmem_ld_16(d + c + 32, p);
+              else release();
+              promote_16(acc0 + c + 16, q, s0);
+              if (c < 32) tmem_ld_wait_16(p);
+            }
           }
-          tc_fence_before_sync();
-          __syncwarp();
-          if (lane == 0) mbar_arrive(&tmp_empty[tmp.stage]);  // everything is in registers
-          if (two) promote_32(acc1 + 16, q, v1);
-          else promote_32(acc0 + 16, q, v0);
         } else {
           tc_fence_before_sync();
           __syncwarp();
@@ -546,10 +542,8 @@ grouped_gemm_fp8_wide_kernel(const __grid_constant__ CUtensorMap tmap_w, const _
           float* p = slot_at(sg.seg);
 #pragma unroll
           for (int i = 0; i < 16; ++i, p += 4 * slot_cols) {
-            const float2 x = unpack2(acc0[2 * i]), y = unpack2(acc0[2 * i + 1]);
-            park_4<kAligned>(p, make_float4(x.x, x.y, y.x, y.y));
-            const float2 z = unpack2(acc1[2 * i]), w = unpack2(acc1[2 * i + 1]);
-            if (two) park_4<kAligned>(p + half, make_float4(z.x, z.y, w.x, w.y));
+            park_4<kAligned>(p, make_float4(acc0[4 * i], acc0[4 * i + 1], acc0[4 * i + 2], acc0[4 * i + 3]));
+            if (two) park_4<kAligned>(p + half, make_float4(acc1[4 * i], acc1[4 * i + 1], acc1[4 * i + 2], acc1[4 * i + 3]));
           }
         }
         __threadfence();
@@ -620,7 +614,7 @@ grouped_gemm_fp8_wide_kernel(const __grid_constant__ CUtensorMap tmap_w, const _
           for (int i = 0; i < 32; ++i) act[i] = 0u;
           if (live && !cut_unit) {
 #pragma unroll
-            for (int i = 0; i < 32; ++i) act[i] = activate(unpack2(acc0[i]), unpack2(acc1[i]));
+            for (int i = 0; i < 32; ++i) act[i] = activate(make_float2(acc0[2 * i], acc0[2 * i + 1]), make_float2(acc1[2 * i], acc1[2 * i + 1]));
           } else if (live) {
 #pragma unroll
             for (int c = 0; c < 4; ++c) {
@@ -674,8 +668,8 @@ grouped_gemm_fp8_wide_kernel(const __grid_constant__ CUtensorMap tmap_w, const _
                 uint32_t o[16];
 #pragma unroll
                 for (int i = 0; i < 16; ++i) {
-                  const float2 f = unpack2(q < 2 ? acc0[16 * (q & 1) + i] : acc1[16 * (q & 1) + i]);
-                  o[i] = pack_bf16(f.x * row_scale, f.y * row_scale);
+                  const float* f = (q < 2 ? acc0 : acc1) + 32 * (q & 1) + 2 * i;
+                  o[i] = pack_bf16(f[0] * row_scale, f[1] * row_scale);
                 }
                 store_32(o, col + (q >> 1) * kF8BlockM + (q & 1) * 32);
               }
