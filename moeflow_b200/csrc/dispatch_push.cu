@@ -257,7 +257,8 @@ __global__ void __launch_bounds__(32 * kManyWarps) dispatch_push_many_kernel(con
 // builds the layout from shared memory: nothing of it goes through L2 (slot words, fence, arrival and the loads behind it took
 // 2.3 us), and the tokens' own CTAs only store their rows.  Layout after 7.0 instead of 9.2 us at 1 token on 288 experts, 4.6
 // instead of 6.7 on 32; calls, us: 1 token 69.2 / 67.2 (32 experts of hidden 512, 8 tokens: 26.4 / 23.2), 8 tokens e4m3
-// 169.9 / 167.4, decode model of 4 sequences 217 / 211.  Above, a warp would route several tokens one after the other, 1 us each.
+// 169.9 / 167.4, decode model of 4 sequences 217 / 211.  Above, a warp would route several tokens one after the other: with
+// two, 32 tokens on 36 experts (e4m3) 123.9 / 125.2, 20 on 288 325.7 / 328.4.
 constexpr int kLocalThreads = 512;
 constexpr int kLocalWarps = kLocalThreads / 32;
 constexpr int kKeeperSmem = 112 * 1024;

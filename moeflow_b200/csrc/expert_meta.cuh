@@ -66,15 +66,17 @@ __device__ __forceinline__ void clear_counters(const mf_meta_args& a, int n_tile
 // million token tiles of 32 weight blocks).
 // What a cut unit costs more (split_kb blocks of streaming) depends on the kernels: 1 for bf16, 8 for e4m3, whose K blocks are
 // half as long and whose fix-up is exposed.  us per layer, graph replay, split_kb 1 / 8:
-//   e4m3, 64-row tiles: 288 experts, 1 token 72.5 / 63.5, 4 tokens 133 / 119, 8 tokens 216 / 187; 72 experts, 16 tokens 227 / 196;
-//   e4m3, 128-row tiles: 8 experts, 80 rows 163 / 87; 4 experts, 200 rows 82 / 70; 72 experts, 400 tokens 335 / 312; 36 experts,
+//   e4m3, 64-row tiles: 288 experts, 1 token 62.0 / 57.6, 4 tokens 113 / 104, 8 tokens 174 / 166; 72 experts, 16 tokens 181 / 172;
+//   e4m3, 128-row tiles: 8 experts, 10 rows 147 / 79; 4 experts, 50 rows 73.5 / 58.9; 72 experts, 40 and 400 tokens, 36 experts,
 //   8 to 1000 tokens, and 144 experts, 800 tokens: not cut with either, the same within 1 %;
-//   bf16: 288 experts, 1 token 78 / 82, elsewhere the same.
+//   bf16: 288 experts, 1 token 67.3 / 69.9, 4 tokens 169 / 172; 72 experts, 16 tokens 306 / 309; 36 experts, 4 tokens the same.
 // Units of fewer than kMinCutBlocks blocks are not cut where there are kMinCutUnits of them: the round trip takes longer than what
-// it saves of the stream.  bf16, us per layer, cut / whole: 4 blocks (8 experts) 1 token 24.8 / 22.6, 8 tokens 28.1 / 24.6;
-// 8 blocks (32 experts) 27.0 / 26.3, 29.4 / 27.2; 12 blocks (16 experts) 29.5 / 29.9, 34.0 / 31.3; 14 blocks, 4 tokens 33.2 / 32.7.
-// With one to three units nearly the whole chip is idle, and a cut pays from 8 blocks on: 4 blocks 25.1 / 24.5, 8 blocks 26.1 / 26.6,
-// 12 blocks 25.3 / 26.7, 14 blocks 26.9 / 28.4.
+// it saves of the stream.  bf16, us per layer, cut / whole: 4 blocks (8 experts) 1 token 22.6 / 20.2, 8 tokens 24.3 / 20.4;
+// 8 blocks (32 experts) 24.5 / 22.4, 24.6 / 22.8; 12 blocks (16 experts) 26.8 / 24.7, 27.9 / 25.8; 14 blocks, 4 tokens 28.2 / 26.9.
+// With one to three units nearly the whole chip is idle, and a cut pays from 12 blocks on: 12 blocks 22.2 / 22.7, 14 blocks
+// 23.4 / 23.6; 8 blocks 22.6 / 21.2, 22.6 / 21.5 and 21.8 / 20.9, 4 blocks 22.1 / 20.2.  (The line is not drawn there for so few
+// units: before the GEMMs' instruction issue got cheaper a cut paid from 8 blocks on, and layers of one to three weight blocks
+// are what the checks of cut units are made of.)
 constexpr long long kNoSplit = 0x7fffffffffffffffll;
 constexpr int kMinCutBlocks = 16, kMinCutUnits = 4;
 __host__ __device__ __forceinline__ long long split_cost(int log_s, int units, int k_blocks, int k_step, int n_sms, int max_slots,

@@ -972,18 +972,19 @@ def choose_block_m(capacity: int, top_k: int, local_experts: int, fp8: bool = Fa
     """Token rows per GEMM tile from the expected rows per expert under even routing (``R * C * K`` entries over
     ``R * L`` experts): 64 for decode, 128 from 36 expected rows, 256 from 80.
 
-    Measured on 72 local experts (whole layer, us, narrower / wider tile): 28 rows 468 / 480, 43 rows 514 / 495,
-    57 rows 557 / 505, 85 rows 705 / 583 (64 / 128); 85 rows 588 / 568, 114 rows 663 / 591, 171 rows 854 / 700,
-    341 rows 1393 / 1155 (128 / 256).  A wider tile keeps an expert's rows in one tile (one pass over its weights)
+    Measured on 72 local experts (whole layer, two weight sets in turn, us, narrower / wider tile): 28 rows 446 / 463, 43 rows
+    498 / 475, 57 rows 545 / 521, 85 rows 683 / 557 (64 / 128); 85 rows 585 / 548, 114 rows 676 / 613, 171 rows 873 / 763
+    (128 / 256).  A wider tile keeps an expert's rows in one tile (one pass over its weights)
     and, at 256 rows, halves the operand bytes per flop that a CTA pulls from L2.
 
     ``fp8``: the layer will hold block-scaled e4m3 experts.  Their kernels take tiles of up to 128 rows, and 256-row tiles
     mean expanding the experts to bf16 in every forward, from 512 expected rows per expert on.  (Below that line the e4m3
     kernels are the faster ones, 600 against about 950 us at 450 rows.  Above it they would be too by now, but an expanded
-    layer keeps its activations in bf16, and its results would lose that precision.)  64 / 128
-    rows: 144 experts of 2048, 44 rows 814 / 728, 55 rows 902 / 759; 72 experts, 28 rows 355 / 368 (zipf popularity 206 / 154),
-    40 rows 315 / 297, 50 rows 348 / 306; 36 experts, 28 rows (zipf) 104 / 106, 40 rows 167 / 174, 56 rows 194 / 180, 78 rows
-    262 / 215.  Layers with few experts have fewer units than CTAs want at 128 rows, so their line lies higher.
+    layer keeps its activations in bf16, and its results would lose that precision.)  64 / 128 rows, two weight sets in turn:
+    72 experts, 28 rows 253 / 303 (zipf popularity 154 / 126), 40 rows 303 / 315, 50 rows 338 / 319; 144 experts of 2048, 44 rows
+    853 / 829; 36 experts, 28 rows (zipf) 97 / 105, 40 rows 150 / 171, 56 rows 176 / 176, 78 rows 233 / 193.  Between 36 and 45
+    rows even popularity loses 4 % on the wider tile and skewed popularity gains 18 %: the line stays at 36.  Layers with few
+    experts have fewer units than CTAs want at 128 rows, so their line lies higher.
     """
     expected = (capacity * top_k) / max(local_experts, 1)
     if fp8:
