@@ -157,13 +157,12 @@ class MoEBlock:
 
 
 class Attention:
-    """Single-token GQA decode step over a static KV cache ``[B, n_kv, max_seq, d]`` (library SDPA and projections; the
-    output projection of few sequences on the dense projection kernel)."""
+    """Single-token GQA decode step over a static KV cache ``[B, n_kv, max_seq, d]`` (library SDPA and projections).
 
-    #: Sequences below which the output projection runs on the dense kernel.  One after the other in a graph, cold weights,
-    #: library / own, us: output (4096 x 4096) 1 sequence 13.7 / 10.2, 4 12.5 / 10.4, 16 10.8 / 10.9, 64 10.9 / 13.3; queries, keys
-    #: and values (5120 x 4096) 11.6 / 16.2, 12.0 / 16.4, 13.1 / 17.1, 12.1 / 22.9.
-    OWN_OUTPUT_BELOW = 16
+    The library's projections at these sizes, one after the other in a graph, cold weights, library / dense projection kernel, us:
+    output (4096 x 4096) 1 sequence 13.7 / 10.2, 4 12.5 / 10.4, 16 10.8 / 10.9, 64 10.9 / 13.3; queries, keys and values (5120 x 4096)
+    11.6 / 16.2, 12.0 / 16.4, 13.1 / 17.1, 12.1 / 22.9.  The dense kernel keeps a tensor map of its weights, though, and these may be
+    exchanged, or changed through a view, between uncaptured steps."""
 
     def __init__(self, hidden: int, acfg: AttentionConfig, batch: int, device, seed: int):
         self.acfg, self.hidden, self.batch = acfg, hidden, batch
@@ -177,21 +176,6 @@ class Attention:
         self.norm_w = torch.ones(hidden, dtype=torch.bfloat16, device=device)
         self.k_cache = torch.zeros(batch, acfg.n_kv_heads, acfg.max_seq, acfg.head_dim, dtype=torch.bfloat16, device=device)
         self.v_cache = torch.zeros_like(self.k_cache)
-        self._own_wo = None  # the weights that the dense projection below was made for
-        self._o = None
-
-    def _output(self, o: torch.Tensor) -> torch.Tensor:
-        w = self.wo
-        if self._own_wo is not w:
-            self._own_wo, self._o = w, None
-            if (w.is_cuda and self.batch < self.OWN_OUTPUT_BELOW and w.dtype == torch.bfloat16 and w.shape[0] % 128 == 0
-                    and w.shape[1] % 64 == 0):
-                from ..ops.dense import DenseProjection
-
-                self._o = DenseProjection(w)
-        if self._o is None or o.dtype != torch.bfloat16:
-            return o @ w.transpose(0, 1)
-        return self._o(o, torch.empty(o.shape[0], w.shape[0], dtype=o.dtype, device=o.device))
 
     def fill_cache(self, length: int, seed: int) -> None:
         """Stand-in for a prefill: random keys/values for the first ``length`` positions."""
@@ -221,7 +205,7 @@ class Attention:
             self.k_cache.scatter_(2, idx, k)
             self.v_cache.scatter_(2, idx, v)
         o = F.scaled_dot_product_attention(q, self.k_cache, self.v_cache, attn_mask=mask, enable_gqa=True)
-        return self._output(o.reshape(self.batch, q_out))
+        return o.reshape(self.batch, q_out) @ self.wo.transpose(0, 1)
 
 
 class DecodeModel:
