@@ -517,8 +517,18 @@ grouped_gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid
       if (n_tile < 16) n_tile = 16;
       const int buf = n_it % kF8Tables;
       const bool alone = Cfg::kTurns && n_tile <= COLS;  // this group has the unit to itself, or nothing to do with it
-      const uint32_t share = alone ? 2u : 1u;            // arrivals: for both groups
+      const uint32_t share = alone ? 2u : 1u;            // arrivals on accumulators and outputs: for both groups
       if (alone && grp != (n_it & 1)) {
+        // The scale table is passed on by both groups all the same: tbl_free never completes a phase that one of them has not
+        // looked at, so it is at most one phase ahead of anybody, and its parity says which.  (With the other group arriving for
+        // both it got two ahead while this one was in its epilogue, where the next units' K blocks fit the accumulators.)  The
+        // wait keeps the arrival out of the phase of the table's last unit.
+        ok = __all_sync(0xffffffffu, mbar_wait_bounded(&tbl_bar[buf], (uint32_t)(n_it / kF8Tables) & 1u, abort_flag, wait_ns));
+        if (!ok) {
+          if (lane == 0) report_status(a.status, kGemmAccTimeout, 4, blockIdx.x, 0);
+          break;
+        }
+        if (lane == 0) mbar_arrive(&tbl_free[buf]);
         const int at = tmp.stage + sg.nkb;
         tmp.stage = at % Cfg::kTmpStages;
         tmp.phase ^= (uint32_t)(at / Cfg::kTmpStages) & 1u;
@@ -527,8 +537,7 @@ grouped_gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid
         continue;
       }
       if (Cfg::kTurns && skipped) {
-        // The parities of the accumulators mean what they say only when the other group has read all of its unit.  (Units are
-        // skipped one at a time, so the table barriers never run two phases ahead of a group.)
+        // The parities of the accumulators mean what they say only when the other group has read all of its unit.
         skipped = false;
         ok = __all_sync(0xffffffffu, mbar_wait_bounded(&tbl_free[(n_it - 1) % kF8Tables], (uint32_t)((n_it - 1) / kF8Tables) & 1u,
                                                        abort_flag, wait_ns));
@@ -626,7 +635,7 @@ grouped_gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid
       }
       if (!ok) break;
       __syncwarp();
-      if (lane == 0) mbar_arrive(&tbl_free[buf], share);  // this warp is done with the segment's table
+      if (lane == 0) mbar_arrive(&tbl_free[buf]);  // this warp is done with the segment's table
 
       bool finish = true;
       if (sg.nseg > 1) {
