@@ -109,7 +109,7 @@ def measure(args, info, cfg, factory, concurrency: int) -> dict:
         end.synchronize()
         samples.append(max_over_ranks(start.elapsed_time(end) / n))
         done += n
-    status = model.routed.check_status()
+    status = model.check_status()
     tpot = summarize(samples)
     result = {"concurrency": concurrency, "tpot_ms": tpot.to_dict(), "tokens_per_second": concurrency / (tpot.median / 1e3),
               "batch_per_rank": batch, "status": status, "finite": bool(torch.isfinite(model.out.float()).all())}

@@ -345,5 +345,17 @@ class DecodeModel:
             self.graph.replay()
         return self.out
 
+    def check_status(self) -> dict:
+        """The first status word that is set, of the routed experts and of every layer's router and shared expert: a wait that ran
+        out leaves wrong values in the residual stream (device-to-host; call it between steps)."""
+        from ..ops import _lib
+
+        found = self.routed.check_status()
+        for layer in self.layers:
+            for part in (layer["router"], layer["shared"]):
+                if found["code"] == 0 and getattr(part, "status", None) is not None:
+                    found = _lib.decode_status(int(part.status.item()))
+        return found
+
     def close(self) -> None:
         self.graph = None
