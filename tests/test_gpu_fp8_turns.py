@@ -58,3 +58,49 @@ def test_layer_bits_do_not_depend_on_who_promotes(tokens):
         outs += [layer.forward(x, logits, bias)[:tokens].clone() for _ in range(3)]
         assert layer.check_status()["code"] == 0 and layer.plan[1:3].tolist() == [1, 1]
     assert all(torch.equal(o, outs[0]) for o in outs)
+
+
+@pytest.mark.parametrize("hidden,inter", [(1152, 128), (4096, 384)])
+@pytest.mark.parametrize("n_sms", [1, 2, 5])
+def test_quantised_activations_of_long_whole_units(hidden, inter, n_sms):
+    """Units of 9 and 32 K blocks, narrow and wide ones, many per CTA: a group's warps meet once per epilogue and write the next
+    maxima a unit (of the other group's, when narrow) later.  Bytes, scales and output against the stand-alone kernels."""
+    from moeflow_b200.fixed import FixedEPLayer
+    from moeflow_b200.ops.fp8 import dequant_rows, down_proj_fp8, gate_up_swiglu_fp8, quant_rows_1x128
+    from moeflow_b200.ops.grouped_gemm import plan_from_offsets
+
+    tokens, counts = 64, ([1, 40, 16, 7], [33, 15, 2, 14], [20, 32, 3, 9])  # rows per expert of each slot
+    cfg = MoEConfig(hidden_size=hidden, moe_intermediate_size=inter, n_routed_experts=12, top_k=3)
+    gen = torch.Generator().manual_seed(hidden)
+    ids = torch.stack([torch.repeat_interleave(torch.arange(4 * k, 4 * k + 4), torch.tensor(c)) for k, c in enumerate(counts)], 1)
+    ids = ids.to(torch.int32).cuda()
+    weights = torch.rand(tokens, 3, generator=gen).cuda()
+    stack = lambda ts: torch.stack([t.view(torch.uint8) for t in ts]).view(torch.float8_e4m3fn).cuda()  # noqa: E731
+    first = [quant_block_fp8(torch.randn(2 * inter, hidden, generator=gen) * (2.0 / hidden**0.5)) for _ in range(12)]
+    second = [quant_block_fp8(torch.randn(hidden, inter, generator=gen) / inter**0.5) for _ in range(12)]
+    pack = (stack([q for q, _ in first]), torch.stack([s for _, s in first]).cuda(),
+            stack([q for q, _ in second]), torch.stack([s for _, s in second]).cuda())
+    layer = FixedEPLayer(cfg, 0, 1, None, None, capacity=tokens, backend="cuda", device="cuda", wait_ns=50_000_000,
+                         gemm_kwargs={"block_m": 64, "n_sms": n_sms})
+    layer.set_weights_fp8(*pack)
+    xs_ = [make_hidden(tokens, cfg, seed, device="cuda") for seed in (3, 4, 5)]
+    for x in xs_ * 3:
+        layer.forward_routed(x, weights, ids)
+    assert layer.check_status()["code"] == 0 and layer.plan[1:3].tolist() == [1, 1]
+
+    offsets, n = layer.offsets.tolist(), tokens * 3
+    assert [b - a for a, b in zip(offsets, offsets[1:])] == [c for slot in counts for c in slot]
+    tp = plan_from_offsets(offsets, 64, x.device)
+    xq, xs = quant_rows_1x128(x)
+    rows = layer.entry_row[:n].clone()
+    act = gate_up_swiglu_fp8(xq, xs, *pack[:2], tp, row_index=rows, limit=cfg.swiglu_limit)
+    aq, a_s = quant_rows_1x128(act.contiguous())
+    f = layer._fp8
+    assert torch.equal(f["aq"][:n], aq.view(torch.uint8)) and torch.equal(f["as"][:n], a_s)
+    assert torch.equal(layer.y[:n], down_proj_fp8(aq, a_s, *pack[2:], tp, row_scale=layer.entry_w[:n].clone()))
+    xf = dequant_rows(xq, xs)[rows.long()]
+    for e, (lo, hi) in enumerate(zip(offsets[:-1], offsets[1:])):
+        gate, up = (xf[lo:hi] @ dequant_block_fp8(pack[0][e], pack[1][e]).t()).chunk(2, dim=-1)
+        ref = torch.nn.functional.silu(gate.clamp(max=cfg.swiglu_limit)) * up.clamp(-cfg.swiglu_limit, cfg.swiglu_limit)
+        # one bf16 rounding of every element (2**-9) on sums whose fp32 error is far below it
+        assert normwise_rel_err(act[lo:hi], ref) < 4 * 2.0**-8

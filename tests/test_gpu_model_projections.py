@@ -57,6 +57,7 @@ def test_position_and_mask_of_captured_steps(n_layers, batch):
             model.x.copy_(torch.randn(batch, 512, generator=gen).bfloat16())
             outs.append(model.step().clone())
             assert int(model.pos) == 17 + step and int((model.mask == 0).sum()) == 18 + step
+        assert model.check_status()["code"] == 0
         runs.append(outs)
         model.close()
     assert all(torch.equal(a, b) for a, b in zip(*runs))
