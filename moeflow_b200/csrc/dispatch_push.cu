@@ -249,9 +249,8 @@ __global__ void __launch_bounds__(32 * kManyWarps) dispatch_push_many_kernel(con
 // second launch, no flags, no cold start of another kernel behind a weight stream that has swept its code and pages out
 // of the caches.  The rows of e4m3 layers are quantised by the CTAs that hold them in registers.  512 threads: one
 // 16-byte chunk of a 4096-wide row each, and eight slot words each in the metadata pass.
-// The layout is there, from the kernel's start and between passes that stream weights: 1 token on 288 experts 9.0 us (13.1
-// with the router's scores in shared memory, the payload in front of the fence and the metadata pass unrolled throughout),
-// 128 tokens 13.4 (19.6).
+// The layout is there, from the kernel's start and between passes that stream weights, after 13.1 us at 128 tokens on 288 experts
+// (19.6 with the router's scores in shared memory, the payload in front of the fence and the metadata pass unrolled throughout).
 //
 // Up to kLocalThreads / 32 token positions one more CTA, the bookkeeper, routes all of them for itself, a warp each, and
 // builds the layout from shared memory: nothing of it goes through L2 (slot words, fence, arrival and the loads behind it took

@@ -74,9 +74,8 @@ __device__ __forceinline__ void clear_counters(const mf_meta_args& a, int n_tile
 // it saves of the stream.  bf16, us per layer, cut / whole: 4 blocks (8 experts) 1 token 22.6 / 20.2, 8 tokens 24.3 / 20.4;
 // 8 blocks (32 experts) 24.5 / 22.4, 24.6 / 22.8; 12 blocks (16 experts) 26.8 / 24.7, 27.9 / 25.8; 14 blocks, 4 tokens 28.2 / 26.9.
 // With one to three units nearly the whole chip is idle, and a cut pays from 12 blocks on: 12 blocks 22.2 / 22.7, 14 blocks
-// 23.4 / 23.6; 8 blocks 22.6 / 21.2, 22.6 / 21.5 and 21.8 / 20.9, 4 blocks 22.1 / 20.2.  (The line is not drawn there for so few
-// units: before the GEMMs' instruction issue got cheaper a cut paid from 8 blocks on, and layers of one to three weight blocks
-// are what the checks of cut units are made of.)
+// 23.4 / 23.6; 8 blocks 22.6 / 21.2, 22.6 / 21.5 and 21.8 / 20.9, 4 blocks 22.1 / 20.2.  (For so few units no line is drawn all
+// the same: before the GEMMs' instruction issue got cheaper a cut paid from 8 blocks on.  At 4 to 8 blocks it costs 1 to 2 us now.)
 constexpr long long kNoSplit = 0x7fffffffffffffffll;
 constexpr int kMinCutBlocks = 16, kMinCutUnits = 4;
 __host__ __device__ __forceinline__ long long split_cost(int log_s, int units, int k_blocks, int k_step, int n_sms, int max_slots,

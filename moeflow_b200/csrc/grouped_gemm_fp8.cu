@@ -69,7 +69,8 @@ struct F8Cfg {
   // 16 or 32 columns take 3 to 5 us, the first one of a launch 7 with its instructions in DRAM) runs while the other
   // promotes the next unit.  With both groups at every unit (and nothing to do for the second) the four accumulators ahead
   // covered 2.7 us of it, and the weight stream stood still for the rest.
-  // Calls, us: 8 tokens on 288 experts 179.7 / 177.7, 250 on 72 (inter 2048) 362 / 357, decode model of 64 246.6 / 242.8.
+  // Calls, us: 8 tokens on 288 experts 179.7 / 177.7, 250 on 72 (inter 2048) 362 / 357, decode model of 64 246.6 / 242.8 (all before
+  // both groups took part in the hand-over of every scale table, which costs up to 0.4 %).
   static constexpr bool kTurns = kGateUp && kGroups == 2;
   static constexpr int kGather = kFourGather ? 128 : 32;  // threads
   static constexpr int kThreads = 128 + 32 * kPromo + (kFourGather ? 128 : 0);

@@ -11,11 +11,11 @@
 //   * the epilogue's quantisation group (128 activations of a token) lies in two threads instead of 128.
 // Promotion works on 16 columns at a time, the next load under way while one is multiplied; its eight warps (a lane
 // quarter and half of the columns each) hold 128 sums and two loads in registers, which is why the other four warps
-// hand registers over to them.  Loads of 32 columns leave too few registers for the rest (both GEMMs spill; the down GEMM does
-// not with 16); single multiply-adds, not pairs: the same rate (128 a clock), and no even register numbers to keep to.
-// Kernels alone, 2000 tokens on 36 experts, us, gate/up and down: 32 columns in pairs 309 /
-// 173, 16 in pairs 320 / 153, 32 single 297 / 161, 16 single 297 / 156.  Of the 297, with parts left out: epilogue 37,
-// multiply-adds 61, the rest (operands through L2, tensor-memory loads) 199.
+// hand registers over to them.  Single multiply-adds, not pairs: the same rate (128 a clock).  Kernels alone, 2000 tokens on 36
+// experts, us, gate/up and down: 32 columns in pairs 309 / 173, 16 in pairs 320 / 153, 32 single 297 / 161, 16 single 297 / 156.
+// Spills explain the down GEMM only (rows by map, 28 bytes stored with 32 in pairs, none with 16 single); the gate/up GEMM
+// (gathered rows) has 4 and 60 and is the faster one with 60, for a reason that was not looked for.  Of the 297, with parts
+// left out: epilogue 37, multiply-adds 61, the rest (operands through L2, tensor-memory loads) 199.
 // 36 experts of 3 x 4096 x 1536, whole layer, against the 64-row kernel's form on 128-row tiles, forwards on three weight sets
 // in turn, with the promotion in its first form (32 columns in pairs): 2000 tokens 917 / 581 us, 1000 tokens 524 / 353, 500 tokens
 // 317 / 222.  What bounds it now: per K block 48 KB through L2 and the promotion, which only half overlaps it.
