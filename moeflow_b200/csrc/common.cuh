@@ -202,13 +202,17 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
 
 // Bounded mbarrier wait.  `abort_flag` is a CTA-shared int: once any role has given up, every other
 // wait in the CTA returns quickly so that the CTA can tear down (free TMEM, exit).
+// kCluster: the arrivals may come from another CTA of the cluster.
+__device__ __forceinline__ bool mbar_try_wait_cluster(uint64_t* bar, uint32_t parity);
+template <bool kCluster = false>
 __device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar, uint32_t parity, volatile int* abort_flag,
                                                   unsigned long long limit_ns) {
-  if (mbar_try_wait(bar, parity)) return true;
+  auto there = [&]() { return kCluster ? mbar_try_wait_cluster(bar, parity) : mbar_try_wait(bar, parity); };
+  if (there()) return true;
   const unsigned long long t0 = global_timer_ns();
   unsigned spins = 0;
   while (true) {
-    if (mbar_try_wait(bar, parity)) return true;
+    if (there()) return true;
     if ((++spins & 255u) == 0u) {
       if (*abort_flag != 0) return false;
       if (global_timer_ns() - t0 > limit_ns) {
@@ -292,7 +296,7 @@ __device__ __forceinline__ void tc_fence_after_sync() {
 // instruction cost its warp about 100 cycles: the operands live in uniform registers, and behind a test of the lane number the
 // compiler has to move each of them there again.  K blocks of 16 KB of e4m3 weights were bound by that (128 tokens on 288
 // experts, down GEMM 273 / 205 us; 8 tokens 77 / 59), and of 32 KB by a little (gate/up 117 / 111 at 8 tokens).
-#define MF_UMMA_BLOCK(KIND)                                                                  \
+#define MF_UMMA_BLOCK(GROUP, KIND)                                                               \
   asm volatile(                                                                              \
       "{\n\t"                                                                                \
       ".reg .pred one, more, first;\n\t"                                                     \
@@ -302,13 +306,13 @@ __device__ __forceinline__ void tc_fence_after_sync() {
       "setp.eq.b32 more, 0, 0;\n\t"                                                          \
       "add.u64 a1, %1, 2;\n\tadd.u64 a2, %1, 4;\n\tadd.u64 a3, %1, 6;\n\t"                   \
       "add.u64 b1, %2, 2;\n\tadd.u64 b2, %2, 4;\n\tadd.u64 b3, %2, 6;\n\t"                   \
-      "@one tcgen05.mma.cta_group::1.kind::" KIND " [%0], %1, %2, %3, first;\n\t"            \
-      "@one tcgen05.mma.cta_group::1.kind::" KIND " [%0], a1, b1, %3, more;\n\t"             \
-      "@one tcgen05.mma.cta_group::1.kind::" KIND " [%0], a2, b2, %3, more;\n\t"             \
-      "@one tcgen05.mma.cta_group::1.kind::" KIND " [%0], a3, b3, %3, more;\n\t"             \
+      "@one tcgen05.mma.cta_group::" GROUP ".kind::" KIND " [%0], %1, %2, %3, first;\n\t"            \
+      "@one tcgen05.mma.cta_group::" GROUP ".kind::" KIND " [%0], a1, b1, %3, more;\n\t"             \
+      "@one tcgen05.mma.cta_group::" GROUP ".kind::" KIND " [%0], a2, b2, %3, more;\n\t"             \
+      "@one tcgen05.mma.cta_group::" GROUP ".kind::" KIND " [%0], a3, b3, %3, more;\n\t"             \
       "}" ::"r"(d), "l"(a), "l"(b), "r"(idesc), "r"(accumulate)                              \
       : "memory")
-#define MF_UMMA_BLOCK_TWO(KIND)                                                              \
+#define MF_UMMA_BLOCK_TWO(GROUP, KIND)                                                           \
   asm volatile(                                                                              \
       "{\n\t"                                                                                \
       ".reg .pred one, more, first;\n\t"                                                     \
@@ -319,27 +323,32 @@ __device__ __forceinline__ void tc_fence_after_sync() {
       "add.u64 a1, %1, 2;\n\tadd.u64 a2, %1, 4;\n\tadd.u64 a3, %1, 6;\n\t"                   \
       "add.u64 b1, %2, 2;\n\tadd.u64 b2, %2, 4;\n\tadd.u64 b3, %2, 6;\n\t"                   \
       "add.u64 c1, %6, 2;\n\tadd.u64 c2, %6, 4;\n\tadd.u64 c3, %6, 6;\n\t"                   \
-      "@one tcgen05.mma.cta_group::1.kind::" KIND " [%0], %1, %2, %3, first;\n\t"            \
-      "@one tcgen05.mma.cta_group::1.kind::" KIND " [%5], %6, %2, %3, first;\n\t"            \
-      "@one tcgen05.mma.cta_group::1.kind::" KIND " [%0], a1, b1, %3, more;\n\t"             \
-      "@one tcgen05.mma.cta_group::1.kind::" KIND " [%5], c1, b1, %3, more;\n\t"             \
-      "@one tcgen05.mma.cta_group::1.kind::" KIND " [%0], a2, b2, %3, more;\n\t"             \
-      "@one tcgen05.mma.cta_group::1.kind::" KIND " [%5], c2, b2, %3, more;\n\t"             \
-      "@one tcgen05.mma.cta_group::1.kind::" KIND " [%0], a3, b3, %3, more;\n\t"             \
-      "@one tcgen05.mma.cta_group::1.kind::" KIND " [%5], c3, b3, %3, more;\n\t"             \
+      "@one tcgen05.mma.cta_group::" GROUP ".kind::" KIND " [%0], %1, %2, %3, first;\n\t"            \
+      "@one tcgen05.mma.cta_group::" GROUP ".kind::" KIND " [%5], %6, %2, %3, first;\n\t"            \
+      "@one tcgen05.mma.cta_group::" GROUP ".kind::" KIND " [%0], a1, b1, %3, more;\n\t"             \
+      "@one tcgen05.mma.cta_group::" GROUP ".kind::" KIND " [%5], c1, b1, %3, more;\n\t"             \
+      "@one tcgen05.mma.cta_group::" GROUP ".kind::" KIND " [%0], a2, b2, %3, more;\n\t"             \
+      "@one tcgen05.mma.cta_group::" GROUP ".kind::" KIND " [%5], c2, b2, %3, more;\n\t"             \
+      "@one tcgen05.mma.cta_group::" GROUP ".kind::" KIND " [%0], a3, b3, %3, more;\n\t"             \
+      "@one tcgen05.mma.cta_group::" GROUP ".kind::" KIND " [%5], c3, b3, %3, more;\n\t"             \
       "}" ::"r"(d), "l"(a), "l"(b), "r"(idesc), "r"(accumulate), "r"(d2), "l"(a2nd)          \
       : "memory")
 // bf16 / f16 (kind::f16) or 8-bit floats (kind::f8f6f4); the types stand in idesc.
-template <bool kF8>
+// kPair: issued by one CTA of a pair for both (cta_group::2, see "CTA pairs" below).
+template <bool kF8, bool kPair = false>
 __device__ __forceinline__ void umma_block(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t accumulate) {
-  if (kF8) MF_UMMA_BLOCK("f8f6f4");
-  else MF_UMMA_BLOCK("f16");
+  if (kPair && kF8) MF_UMMA_BLOCK("2", "f8f6f4");
+  else if (kPair) MF_UMMA_BLOCK("2", "f16");
+  else if (kF8) MF_UMMA_BLOCK("1", "f8f6f4");
+  else MF_UMMA_BLOCK("1", "f16");
 }
-template <bool kF8>
+template <bool kF8, bool kPair = false>
 __device__ __forceinline__ void umma_block(uint32_t d, uint32_t d2, uint64_t a, uint64_t a2nd, uint64_t b, uint32_t idesc,
                                            uint32_t accumulate) {
-  if (kF8) MF_UMMA_BLOCK_TWO("f8f6f4");
-  else MF_UMMA_BLOCK_TWO("f16");
+  if (kPair && kF8) MF_UMMA_BLOCK_TWO("2", "f8f6f4");
+  else if (kPair) MF_UMMA_BLOCK_TWO("2", "f16");
+  else if (kF8) MF_UMMA_BLOCK_TWO("1", "f8f6f4");
+  else MF_UMMA_BLOCK_TWO("1", "f16");
 }
 #undef MF_UMMA_BLOCK
 #undef MF_UMMA_BLOCK_TWO
@@ -377,6 +386,83 @@ __device__ __forceinline__ void tmem_ld_16(uint32_t taddr, uint32_t (&r)[16]) {
       : "memory");
 }
 __device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
+
+// ---------------------------------------------------------------------------------------------
+// Clusters
+// ---------------------------------------------------------------------------------------------
+__device__ __forceinline__ uint32_t cluster_rank() {
+  uint32_t r;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return r;
+}
+__device__ __forceinline__ void cluster_sync_all() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// The same shared-memory offset in CTA `rank` of this cluster.
+__device__ __forceinline__ uint32_t cluster_map(uint32_t smem_addr, uint32_t rank) {
+  uint32_t r;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(smem_addr), "r"(rank));
+  return r;
+}
+
+// ---------------------------------------------------------------------------------------------
+// CTA pairs (cta_group::2): the two CTAs of a cluster share one MMA of M = 256.  Each holds its own 128 rows of A, one half of
+// B's rows and its own 128 accumulator rows over all of B; the instruction is issued by CTA 0, reads both shared memories
+// at the same offsets and writes both tensor memories.  So each CTA fetches half of B, and its shared memory gives half of it.
+// ---------------------------------------------------------------------------------------------
+__device__ __forceinline__ void tmem_alloc_pair(uint32_t* smem_result, uint32_t ncols) {  // the same warp of both CTAs
+  asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(smem_result)), "r"(ncols)
+               : "memory");
+}
+__device__ __forceinline__ void tmem_relinquish_pair() {
+  asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void tmem_dealloc_pair(uint32_t taddr, uint32_t ncols) {
+  asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols) : "memory");
+}
+// umma_commit for the pair: the barrier at this offset in both CTAs gets one arrival.
+__device__ __forceinline__ void umma_commit_pair(uint64_t* bar) {
+  asm volatile(
+      "{\n\t"
+      ".reg .pred one;\n\t"
+      ".reg .b16 both;\n\t"
+      "elect.sync _|one, 0xffffffff;\n\t"
+      "mov.b16 both, 3;\n\t"
+      "@one tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], both;\n\t"
+      "}" ::"r"(smem_u32(bar))
+      : "memory");
+}
+// A box into this CTA's shared memory whose bytes are counted by a barrier of either CTA of the pair (cluster address).
+__device__ __forceinline__ void tma_load_2d_pair(void* smem_dst, const void* tmap, uint32_t bar, int x, int y, uint64_t policy) {
+  asm volatile(
+      "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1, {%3, %4}], [%2], %5;"
+      ::"r"(smem_u32(smem_dst)), "l"(reinterpret_cast<uint64_t>(tmap)), "r"(bar), "r"(x), "r"(y), "l"(policy)
+      : "memory");
+}
+// Arrival on a barrier of either CTA.  kData: what this thread has written is released to the cluster (the waiter takes the
+// acquire form), which costs about a microsecond.  Without: for operands in shared memory, which a proxy fence has handed to the
+// tensor core, and for accumulators.
+template <bool kData = false>
+__device__ __forceinline__ void mbar_arrive_cluster(uint32_t bar) {
+  if (kData) asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
+  else asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
+}
+__device__ __forceinline__ bool mbar_try_wait_cluster(uint64_t* bar, uint32_t parity) {
+  uint32_t ok;
+  asm volatile(
+      "{\n\t"
+      ".reg .pred p;\n\t"
+      "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t"
+      "}"
+      : "=r"(ok)
+      : "r"(smem_u32(bar)), "r"(parity)
+      : "memory");
+  return ok != 0;
+}
+__device__ __forceinline__ void st_cluster_s32(uint32_t addr, int v) {
+  asm volatile("st.shared::cluster.s32 [%0], %1;" ::"r"(addr), "r"(v) : "memory");
+}
 
 // Shared-memory matrix descriptor for a K-major operand tile stored as rows of 128 bytes with the
 // 128-byte swizzle (the layout a TMA box of 64 bf16 x rows with SWIZZLE_128B produces): 8-row groups
@@ -422,19 +508,32 @@ struct alignas(16) U4 {
 extern "C" int mf_pdl_enabled(void);
 
 namespace mf {
+// `cluster`: CTAs of a cluster (1: launched without one).
 template <typename... KArgs, typename... Args>
-inline cudaError_t launch_kernel(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
-                                 bool dependent, Args&&... args) {
+inline cudaError_t launch_cluster(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
+                                  bool dependent, unsigned cluster, Args&&... args) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = grid;
   cfg.blockDim = block;
   cfg.dynamicSmemBytes = smem;
   cfg.stream = stream;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchAttribute attr[2];
   cfg.attrs = attr;
-  cfg.numAttrs = (dependent && mf_pdl_enabled()) ? 1 : 0;
+  if (dependent && mf_pdl_enabled()) {
+    attr[cfg.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[cfg.numAttrs++].val.programmaticStreamSerializationAllowed = 1;
+  }
+  if (cluster > 1) {
+    attr[cfg.numAttrs].id = cudaLaunchAttributeClusterDimension;
+    attr[cfg.numAttrs].val.clusterDim.x = cluster;
+    attr[cfg.numAttrs].val.clusterDim.y = 1;
+    attr[cfg.numAttrs++].val.clusterDim.z = 1;
+  }
   return cudaLaunchKernelEx(&cfg, kern, static_cast<KArgs>(args)...);
+}
+template <typename... KArgs, typename... Args>
+inline cudaError_t launch_kernel(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
+                                 bool dependent, Args&&... args) {
+  return launch_cluster(kern, grid, block, smem, stream, dependent, 1, static_cast<KArgs>(args)...);
 }
 }  // namespace mf

@@ -30,6 +30,14 @@
 //               12-15), or warp 2 alone fetches contiguous rows by TMA
 //   warps 4-7   epilogue: tcgen05.ld -> registers -> activation / scale -> global
 //
+// CTA pairs (kPair: units of two accumulators on 256-row tiles): the two CTAs of a cluster take adjacent weight blocks of one
+// token tile and hold one half of its rows each, as one MMA of M = 256 (cta_group::2, issued by CTA 0).  Per K block of a full
+// tile a CTA then pulls 48 KB through L2 and reads 64 KB of operands out of shared memory for 1024 tensor cycles, instead of 64
+// and 96, and gathers half of the rows.  Both CTAs run every role but the UMMA issuer's: in CTA 1 that warp reports gathered rows
+// (a local barrier, a proxy fence, one arrival at CTA 0; with release.cluster on that arrival a K block took 1.15 us).
+// Single CTAs / pairs, kernels alone in a burst, us: gate/up 72 experts 1000 tokens 341 / 323, 2000 tokens 482 / 446, 36 experts
+// 8192 tokens 1359 / 1243; down 177 / 174, 247 / 239, 708 / 696.
+//
 // Replaces the reference's Triton grouped GEMM, unfused SwiGLU and expert-input gather
 // (moeflow/kernels/grouped_gemm.py:15-80, moeflow/experts.py:10-17, moeflow/kernels/expert_prepare.py:10-38).
 #include <cuda.h>
@@ -63,11 +71,11 @@ constexpr int kMaxAccStages = 2;
 constexpr int kOutStageBytes = 1024;   // 16 token columns x 32 weight rows of 16-bit outputs, per epilogue warp
 constexpr int kMaxDevices = 64;        // devices one process may drive (per-device launch configuration)
 
-template <bool kGateUp, int N_MAX>
+template <bool kGateUp, int N_MAX, bool kPair = false>
 struct GemmCfg {
   static constexpr int kATiles = kGateUp ? 2 : 1;
   static constexpr int kStageA = kATiles * kTileBytesA;
-  static constexpr int kStageB = N_MAX * 128;
+  static constexpr int kStageB = (kPair ? N_MAX / 2 : N_MAX) * 128;
   static constexpr int kStageBytes = kStageA + kStageB;
   // As many stages as fit in 216 KB of the 227 KB a CTA may use (2 KB more go to alignment slack and
   // barriers): the bytes in flight per SM, not the tensor pipe, bound these weight-streaming kernels.
@@ -242,13 +250,15 @@ __device__ __forceinline__ void finish_store(const mf_gemm_args& a, float (&v)[C
   }
 }
 
-template <bool kGateUp, int N_MAX, bool kReturn = false>
+template <bool kGateUp, int N_MAX, bool kReturn = false, bool kPair = false>
 __global__ void __launch_bounds__(kLaunchThreads<kGateUp, N_MAX, kReturn>, 1)
 grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_b,
                     const mf_gemm_args a) {
-  using Cfg = GemmCfg<kGateUp, N_MAX>;
+  static_assert(!kPair || (kGateUp && !kReturn), "pairs: two accumulators, no return warps");
+  using Cfg = GemmCfg<kGateUp, N_MAX, kPair>;
   constexpr int STAGES = Cfg::kStages;
   constexpr int kGroups = kEpiGroups<N_MAX, kReturn>;
+  constexpr int kRowsB = kPair ? N_MAX / 2 : N_MAX;  // token rows of a tile that this CTA holds
   constexpr bool kFourGather = kWideGather<kGateUp, N_MAX, kReturn>;
   constexpr int kGatherThreads = kFourGather ? 128 : 64, kGatherStep = kGatherThreads / 8;
 
@@ -267,8 +277,12 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
   int* ret_desc = reinterpret_cast<int*>(ret_empty + 4 * kRetDepth);  // [4][kRetDepth][4]: n_rows, row_start, mb
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(ret_desc + 4 * kRetDepth * 4);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+  // Pairs have no return queue: CTA 1's mail from CTA 0 lies there, and the barriers of the gathered rows.
+  PairMail* mail = reinterpret_cast<PairMail*>(ret_full);
+  uint64_t* rows_bar = reinterpret_cast<uint64_t*>(mail + 1);  // [STAGES] CTA 1: the rows it gathers are there
   static_assert(sizeof(SegRing) + (2 * STAGES + 2 * kMaxAccStages + 8 * kRetDepth) * 8 + 4 * kRetDepth * 16 + 8 <= 1024,
                 "barriers, segment ring and return queue");
+  static_assert(!kPair || (sizeof(PairMail) + STAGES * 8 <= 8 * kRetDepth * 8 && STAGES + 2 <= kPairMail), "mail");
   uint8_t* out_stage = smem + STAGES * Cfg::kStageBytes + 1024;  // [4 epilogue warps][kOutStageBytes]
   // The fused return path runs on four extra warps (the kernel is then launched with 384 threads).
   constexpr bool with_return = kReturn;  // the down GEMM with four extra warps for the fused return path
@@ -279,6 +293,9 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
   // Token operand by TMA (contiguous rows) instead of the cp.async gather: warp 2 issues one bulk copy per
   // stage, warp 3 has nothing to do.
   const bool b_tma = a.b_tmap != nullptr;
+  // Pairs: CTA 0 issues the MMAs.  Both fill their operands for them; all of it is counted by CTA 0's full barriers.
+  const int rank = kPair ? (int)cluster_rank() : 0;
+  const int cta = kPair ? (int)blockIdx.x / 2 : (int)blockIdx.x, ctas = kPair ? (int)gridDim.x / 2 : (int)gridDim.x;
   // Optional per-CTA time stamps: 0 entry, 1 dependencies met, 2 first weight tile requested, 3 first
   // operand stage complete, 4 first accumulator complete, 5 last epilogue done, 6 exit.
   unsigned long long* trace = a.trace ? a.trace + (size_t)blockIdx.x * 16 : nullptr;
@@ -299,14 +316,17 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
   if (tid == 0) {
     for (int s = 0; s < STAGES; ++s) {
       // weight TMA expect_tx arrive + (one per gather thread | the token TMA expect_tx arrive)
-      mbar_init(&full_bar[s], b_tma ? 2 : 1 + kGatherThreads);
+      // (pairs: both CTAs' bytes in one arrival each; CTA 1 adds one arrival for the rows that it has gathered)
+      mbar_init(&full_bar[s], b_tma ? 2 : (kPair ? 2 : 1) + kGatherThreads);
       mbar_init(&empty_bar[s], 1);                  // tcgen05.commit
+      if (kPair) mbar_init(&rows_bar[s], kGatherThreads);
     }
     for (int s = 0; s < Cfg::kAccStages; ++s) {
       mbar_init(&acc_full[s], 1);   // tcgen05.commit
-      mbar_init(&acc_empty[s], 4 * kGroups);  // one per epilogue warp
+      mbar_init(&acc_empty[s], 4 * kGroups * (kPair ? 2 : 1));  // one per epilogue warp (of both CTAs: CTA 0's barrier)
     }
-    for (int s = 0; s < 4 * kRetDepth; ++s) {
+    if (kPair) mail->init();
+    for (int s = 0; !kPair && s < 4 * kRetDepth; ++s) {
       mbar_init(&ret_full[s], 1);
       mbar_init(&ret_empty[s], 1);
     }
@@ -316,12 +336,23 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
     tma_prefetch_desc(&tmap_w);
     if (b_tma) tma_prefetch_desc(&tmap_b);
   }
+  if (kPair) __syncwarp();
   if (warp == 1) {
-    tmem_alloc(tmem_slot, Cfg::kTmemCols);
-    tmem_relinquish();
+    if (kPair) {
+      tmem_alloc_pair(tmem_slot, Cfg::kTmemCols);
+      tmem_relinquish_pair();
+    } else {
+      tmem_alloc(tmem_slot, Cfg::kTmemCols);
+      tmem_relinquish();
+    }
   }
   tc_fence_before_sync();
-  __syncthreads();
+  if (kPair) {
+    __syncwarp();
+    cluster_sync_all();  // the other CTA's barriers exist, both have their tensor memory
+  } else {
+    __syncthreads();
+  }
   tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_slot;
 
@@ -367,7 +398,8 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
   const long long slot_floats = (long long)Cfg::kATiles * slot_cols * kBlockM;
   const unsigned long long wait_ns = a.wait_ns;
   WorkIter work;
-  work.init(a, N_MAX, n_tiles, cut, blockIdx.x, gridDim.x);
+  work.init(a, N_MAX, n_tiles, cut, cta, ctas);
+  constexpr int kCtas = kPair ? 2 : 1;  // a pair's unit is two units of the plan, next to each other
   {
     // A plan that does not fit the buffers it indexes (a tile count or a cut larger than what the caller
     // sized the scratch for) is refused here, on the device, before anything is stored: every thread of
@@ -375,14 +407,22 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
     bool bad = n_tiles < 0 || !(cut == 0 || cut == 1 || cut == 2 || cut == 4 || cut == 8) ||
                (cut > 1 && a.k_blocks % cut != 0);
     bad = bad || (a.max_tiles > 0 && n_tiles > a.max_tiles);
-    bad = bad || (a.n_counters > 0 && (long long)n_tiles * a.m_blocks * 4 * kGroups > (long long)a.n_counters);
-    bad = bad || (a.partial_floats > 0 && work.slots_needed() * slot_floats > a.partial_floats);
+    bad = bad || (a.n_counters > 0 && (long long)n_tiles * a.m_blocks * kCtas * 4 * kGroups > (long long)a.n_counters);
+    bad = bad || (a.partial_floats > 0 && work.slots_needed() * kCtas * slot_floats > a.partial_floats);
     if (bad) {
       if (tid == 0) report_status(a.status, kBadArgument, 6, blockIdx.x, 0);
       n_tiles = 0;
-      work.init(a, N_MAX, 0, 1, blockIdx.x, gridDim.x);
+      work.init(a, N_MAX, 0, 1, cta, ctas);
     }
   }
+  // MMA columns of a tile: its rows in steps of 16; of 32 for a pair, whose CTAs hold one half of the rows each.
+  auto tile_cols = [&](int n_rows) {
+    const int n = kPair ? (n_rows + 31) & ~31 : (n_rows + 15) & ~15;
+    return n < 16 * kCtas ? 16 * kCtas : n;
+  };
+  // Block (or two adjacent blocks) of a unit that is this CTA's.
+  auto block_of = [&](const Seg& s) { return kPair ? 2 * s.mb + rank : s.mb; };
+  auto slot_ix = [&](const Seg& s, int seg) { return (long long)slot_of(s, seg) * kCtas + rank; };
 
   SegReader reader(ring, abort_flag, wait_ns);
   // Token-operand producers that gather rows by index (gt: 0 .. kGatherThreads - 1).
@@ -394,11 +434,14 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
     bool ok = true;
     Seg sg, nx;
     int ready_tile = -1;
-    int idx[N_MAX / kGatherStep];  // source rows of the segment at hand, fetched during the previous one
+    int idx[kRowsB / kGatherStep];  // source rows of the segment at hand, fetched during the previous one
+    // a pair's CTA 1 gathers the rows behind the first half of the tile's columns
+    auto first_row = [&](const Seg& s_) { return r_in + (kPair ? rank * (tile_cols(s_.n_rows) / 2) : 0); };
     auto row_indices = [&](const Seg& s_) {
+      const int first = first_row(s_);
 #pragma unroll
-      for (int i = 0; i < N_MAX / kGatherStep; ++i) {
-        const int n = r_in + kGatherStep * i;
+      for (int i = 0; i < kRowsB / kGatherStep; ++i) {
+        const int n = first + kGatherStep * i;
         if (n < s_.n_rows) idx[i] = a.b_index ? __ldcg(a.b_index + s_.row_start + n) : s_.row_start + n;
       }
     };
@@ -418,12 +461,12 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
         ready_tile = sg.tt;
       }
       const int n_rows = sg.n_rows;
-      int n_tile = (n_rows + 15) & ~15;
-      if (n_tile < 16) n_tile = 16;
-      const uint8_t* rp[N_MAX / kGatherStep];
+      const int n_tile = tile_cols(n_rows) / kCtas;
+      const int first = first_row(sg);
+      const uint8_t* rp[kRowsB / kGatherStep];
 #pragma unroll
-      for (int i = 0; i < N_MAX / kGatherStep; ++i) {
-        const int n = r_in + kGatherStep * i;
+      for (int i = 0; i < kRowsB / kGatherStep; ++i) {
+        const int n = first + kGatherStep * i;
         rp[i] = n < n_rows ? static_cast<const uint8_t*>(a.b_base) + (long long)idx[i] * a.b_pitch + chunk * 16 : nullptr;
       }
       for (int j = 0; j < sg.nkb; ++j) {
@@ -436,7 +479,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
         }
         const uint32_t b_stage = smem_u32(sB + st.stage * Cfg::kStageB);
 #pragma unroll
-        for (int i = 0; i < N_MAX / kGatherStep; ++i) {
+        for (int i = 0; i < kRowsB / kGatherStep; ++i) {
           const int n = r_in + kGatherStep * i;
           if (n < n_tile) {
             const bool live = rp[i] != nullptr;
@@ -444,7 +487,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
                         live ? 16u : 0u);
           }
         }
-        cp_async_mbar_arrive_noinc(&full_bar[st.stage]);
+        cp_async_mbar_arrive_noinc(kPair && rank == 1 ? &rows_bar[st.stage] : &full_bar[st.stage]);
         st.advance(STAGES);
         // the producer warp publishes the next segment during the third K block of this one
         if (j == (sg.nkb < 4 ? sg.nkb - 1 : 3)) {
@@ -467,7 +510,11 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
       // ------------------------------------------------------------------ weight TMA producer
       PipeState st;
       bool ok = true;
-      SegFeed feed(work, ring, abort_flag, wait_ns);
+      SegFeedOf<kPair> feed(work, ring, abort_flag, wait_ns);
+      if (kPair) {
+        feed.mail = mail;
+        feed.rank = rank;
+      }
       // Tiles of up to 64 rows are decode: an expert usually has one tile, and its weights are then read once per forward.
       // Skewed routing gives a hot expert several that read the same blocks, but they run close together and most blocks are
       // still read once: evict-first / normal, us per layer, 1 token 81 / 96, 128 tokens 1325 / 1347 (bf16, 288 experts), 8
@@ -477,7 +524,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
       Seg sg;
       bool have = feed.first(sg);
       while (ok && have) {
-        const int row0 = sg.e * a.rows_per_expert + sg.mb * (a.two_blocks ? 2 * kBlockM : kBlockM);
+        const int row0 = sg.e * a.rows_per_expert + block_of(sg) * (a.two_blocks ? 2 * kBlockM : kBlockM);
         for (int j = 0; j < sg.nkb; ++j) {
           const int kb = sg.kb0 + j;
           ok = mbar_wait_bounded(&empty_bar[st.stage], st.phase ^ 1u, abort_flag, wait_ns);
@@ -487,11 +534,17 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
             break;
           }
           if (elect_one()) {
-            mbar_arrive_expect_tx(&full_bar[st.stage], Cfg::kStageA);
+            if (!kPair || rank == 0) mbar_arrive_expect_tx(&full_bar[st.stage], Cfg::kStageA * kCtas);
             uint8_t* dst = sA + st.stage * Cfg::kStageA;
             if (trace && trace[2] == 0) trace[2] = global_timer_ns();  // see the note at MF_STAMP_ONCE
-            tma_load_2d(dst, &tmap_w, &full_bar[st.stage], kb * 64, row0, policy);
-            if (kGateUp) tma_load_2d(dst + kTileBytesA, &tmap_w, &full_bar[st.stage], kb * 64, row0 + a.up_row_offset, policy);
+            if (kPair) {
+              const uint32_t bar = cluster_map(smem_u32(&full_bar[st.stage]), 0);
+              tma_load_2d_pair(dst, &tmap_w, bar, kb * 64, row0, policy);
+              tma_load_2d_pair(dst + kTileBytesA, &tmap_w, bar, kb * 64, row0 + a.up_row_offset, policy);
+            } else {
+              tma_load_2d(dst, &tmap_w, &full_bar[st.stage], kb * 64, row0, policy);
+              if (kGateUp) tma_load_2d(dst + kTileBytesA, &tmap_w, &full_bar[st.stage], kb * 64, row0 + a.up_row_offset, policy);
+            }
           }
           __syncwarp();
           st.advance(STAGES);
@@ -500,6 +553,11 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
         if (ok) have = feed.next(sg);
       }
       if (feed.bad_tile && lane == 0) report_status(a.status, kBadArgument, 7, blockIdx.x, 0);
+      // Pairs: the last MMAs' commits arrive in both CTAs; neither leaves before.
+      for (int s = 0; kPair && ok && s < STAGES; ++s) {
+        ok = __all_sync(0xffffffffu, mbar_wait_bounded(&empty_bar[st.stage], st.phase ^ 1u, abort_flag, wait_ns));
+        st.advance(STAGES);
+      }
       if (!ok) {
         // Give copies that are still in flight a moment to land before the CTA goes away.
         const unsigned long long t0 = global_timer_ns();
@@ -511,8 +569,23 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
       bool ok = true;
       Seg sg;
       while (ok && reader.next(sg, ok)) {
-        const uint32_t n_tile = (uint32_t)((sg.n_rows + 15) & ~15);
-        const uint32_t idesc = umma_idesc(1, 1, kBlockM, n_tile < 16 ? 16 : n_tile);
+        if (kPair && rank == 1) {
+          // CTA 1 tells CTA 0 that its gathered rows are there
+          for (int j = 0; !b_tma && j < sg.nkb; ++j) {
+            ok = __all_sync(0xffffffffu, mbar_wait_bounded(&rows_bar[st.stage], st.phase, abort_flag, wait_ns));
+            if (!ok) {
+              if (lane == 0) report_status(a.status, kGemmFullTimeout, 1, blockIdx.x, 0);
+              break;
+            }
+            fence_proxy_async_smem();
+            if (lane == 0) mbar_arrive_cluster(cluster_map(smem_u32(&full_bar[st.stage]), 0));
+            __syncwarp();
+            st.advance(STAGES);
+          }
+          continue;
+        }
+        const uint32_t n_tile = (uint32_t)tile_cols(sg.n_rows);
+        const uint32_t idesc = umma_idesc(1, 1, kBlockM * kCtas, n_tile);
         const bool wide = Cfg::kWide && n_tile > 128;
         PipeState acc2 = acc;  // a wide unit's second stage
         acc2.advance(Cfg::kAccStages);
@@ -538,14 +611,20 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
           if (!b_tma) fence_proxy_async_smem();  // the gathered rows
           const uint64_t a_desc = umma_desc_sw128(smem_u32(sA + st.stage * Cfg::kStageA));
           const uint64_t b_desc = umma_desc_sw128(smem_u32(sB + st.stage * Cfg::kStageB));
-          if (kGateUp) umma_block<false>(d0, d1, a_desc, a_desc + (kTileBytesA >> 4), b_desc, idesc, j > 0 ? 1u : 0u);
+          if (kGateUp) umma_block<false, kPair>(d0, d1, a_desc, a_desc + (kTileBytesA >> 4), b_desc, idesc, j > 0 ? 1u : 0u);
           else umma_block<false>(d0, a_desc, b_desc, idesc, j > 0 ? 1u : 0u);
-          umma_commit(&empty_bar[st.stage]);
+          if (kPair) umma_commit_pair(&empty_bar[st.stage]);
+          else umma_commit(&empty_bar[st.stage]);
           st.advance(STAGES);
         }
         if (!ok) break;
-        umma_commit(&acc_full[acc.stage]);
-        if (wide) umma_commit(&acc_full[acc2.stage]);
+        if (kPair) {
+          umma_commit_pair(&acc_full[acc.stage]);
+          if (wide) umma_commit_pair(&acc_full[acc2.stage]);
+        } else {
+          umma_commit(&acc_full[acc.stage]);
+          if (wide) umma_commit(&acc_full[acc2.stage]);
+        }
         acc.advance(Cfg::kAccStages);
         if (wide) acc.advance(Cfg::kAccStages);
       }
@@ -574,7 +653,9 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
             }
             ready_tile = sg.tt;
           }
-          const int n_box = max(1, (sg.n_rows + box_rows - 1) / box_rows);
+          const int cols = tile_cols(sg.n_rows) / kCtas;  // (pairs: this CTA's half of the tile's columns)
+          const int n_box = kPair ? (cols + box_rows - 1) / box_rows : max(1, (sg.n_rows + box_rows - 1) / box_rows);
+          const int first = sg.row_start + rank * cols;
           for (int j = 0; j < sg.nkb; ++j) {
             const int kb = sg.kb0 + j;
             ok = mbar_wait_bounded(&empty_bar[st.stage], st.phase ^ 1u, abort_flag, wait_ns);
@@ -587,10 +668,14 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
               // as many boxes as hold the tile's rows: rows past the tile (the next expert's entries, or zero fill
               // past the end of the buffer) land in smem rows the MMA does not read or in accumulator columns the
               // epilogue skips
-              mbar_arrive_expect_tx(&full_bar[st.stage], n_box * box_rows * 128);
-              for (int i = 0; i < n_box; ++i)
-                tma_load_2d(sB + st.stage * Cfg::kStageB + i * box_rows * 128, &tmap_b, &full_bar[st.stage], kb * 64,
-                            sg.row_start + i * box_rows);
+              if (!kPair || rank == 0) mbar_arrive_expect_tx(&full_bar[st.stage], n_box * box_rows * 128 * kCtas);
+              for (int i = 0; i < n_box; ++i) {
+                uint8_t* dst = sB + st.stage * Cfg::kStageB + i * box_rows * 128;
+                if (kPair)
+                  tma_load_2d_pair(dst, &tmap_b, cluster_map(smem_u32(&full_bar[st.stage]), 0), kb * 64, first + i * box_rows, l2_evict_normal());
+                else
+                  tma_load_2d(dst, &tmap_b, &full_bar[st.stage], kb * 64, sg.row_start + i * box_rows);
+              }
             }
             __syncwarp();
             st.advance(STAGES);
@@ -635,13 +720,16 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
       rq.advance(kRetDepth);
       return true;
     };
+    auto acc_free = [&](int stage) {
+      if (kPair) mbar_arrive_cluster(cluster_map(smem_u32(&acc_empty[stage]), 0));
+      else mbar_arrive(&acc_empty[stage]);
+    };
     Seg sg;
     while (ok && reader.next(sg, ok)) {
-      const int mb = sg.mb;
+      const int mb = block_of(sg);
       const int n_rows = sg.n_rows;
       const int row_start = sg.row_start;
-      int n_tile = (n_rows + 15) & ~15;
-      if (n_tile < 16) n_tile = 16;
+      const int n_tile = tile_cols(n_rows);
       const bool wide = Cfg::kWide && n_tile > 128;
       PipeState acc2 = acc;
       acc2.advance(Cfg::kAccStages);
@@ -663,7 +751,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
       const int c_half = kGroups == 2 ? ((n_tile / 16 + 1) / 2) * 16 : n_tile;
       const int c_begin = grp * c_half;
       const int c_end = (kGroups == 2 && grp == 0) ? c_half : n_tile;
-      const int counter_ix = (sg.unit * 4 + wq) * kGroups + grp;
+      const int counter_ix = ((sg.unit * kCtas + rank) * 4 + wq) * kGroups + grp;
       if (sg.nseg == 1) {
         // A real loop over 16-column groups (one copy of the code: unrolled over the whole tile it no longer fits
         // the instruction cache, and every group is executed once per unit).  Lane l fetches the routing weight of
@@ -696,8 +784,8 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
         tc_fence_before_sync();
         __syncwarp();
         if (lane == 0) {
-          mbar_arrive(&acc_empty[acc.stage]);
-          if (wide) mbar_arrive(&acc_empty[acc2.stage]);
+          acc_free(acc.stage);
+          if (wide) acc_free(acc2.stage);
         }
         if (a.tile_done != nullptr) {
           __threadfence();  // every lane's stores are visible device-wide before the count
@@ -708,7 +796,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
       } else {
         // The unit is cut along K: park the fp32 partial sums, then the last quarter-warp to arrive adds
         // the segments in K order.
-        float* mine = a.partial + (long long)slot_of(sg, sg.seg) * slot_floats;
+        float* mine = a.partial + slot_ix(sg, sg.seg) * slot_floats;
         for (int c0 = c_begin; c0 < c_end; c0 += 16) {
           uint32_t g[16], up[16];
           tmem_ld_16(taddr + c0, g);
@@ -726,8 +814,8 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
         tc_fence_before_sync();
         __syncwarp();
         if (lane == 0) {
-          mbar_arrive(&acc_empty[acc.stage]);
-          if (wide) mbar_arrive(&acc_empty[acc2.stage]);
+          acc_free(acc.stage);
+          if (wide) acc_free(acc2.stage);
         }
         __threadfence();
         __syncwarp();
@@ -746,7 +834,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
 #pragma unroll
             for (int j = 0; j < kFix; ++j) v[j] = w[j] = 0.f;
             for (int s = 0; s < sg.nseg; ++s) {
-              const float* p = a.partial + (long long)slot_of(sg, s) * slot_floats;
+              const float* p = a.partial + slot_ix(sg, s) * slot_floats;
               float pv[kFix], pw[kFix];
 #pragma unroll
               for (int j = 0; j < kFix; ++j) {
@@ -812,11 +900,13 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
 
   __syncwarp();
   tc_fence_before_sync();
-  __syncthreads();
+  if (kPair) cluster_sync_all();  // neither CTA leaves while the other may still use its memories
+  else __syncthreads();
   if (trace && tid == 0) trace[6] = global_timer_ns();
   if (warp == 1) {
     tc_fence_after_sync();
-    tmem_dealloc(tmem_base, Cfg::kTmemCols);
+    if (kPair) tmem_dealloc_pair(tmem_base, Cfg::kTmemCols);
+    else tmem_dealloc(tmem_base, Cfg::kTmemCols);
   }
 }
 
@@ -841,12 +931,12 @@ static EncodeTiledFn get_encode_fn() {
 
 #undef MF_STAMP_ONCE
 
-template <bool kGateUp, int N_MAX, bool kReturn = false>
+template <bool kGateUp, int N_MAX, bool kReturn = false, bool kPair = false>
 static int launch(const void* tmap, const mf_gemm_args* args, int grid, cudaStream_t stream) {
-  using Cfg = GemmCfg<kGateUp, N_MAX>;
+  using Cfg = GemmCfg<kGateUp, N_MAX, kPair>;
   // The shared-memory attribute belongs to (function, device): set it once per device this process drives.
   static bool configured[kMaxDevices] = {};
-  auto kern = grouped_gemm_kernel<kGateUp, N_MAX, kReturn>;
+  auto kern = grouped_gemm_kernel<kGateUp, N_MAX, kReturn, kPair>;
   int dev = 0;
   cudaError_t de = cudaGetDevice(&dev);
   if (de != cudaSuccess) return (int)de;
@@ -859,7 +949,22 @@ static int launch(const void* tmap, const mf_gemm_args* args, int grid, cudaStre
   memcpy(&tm, tmap, sizeof(tm));
   memcpy(&tb, args->b_tmap ? args->b_tmap : tmap, sizeof(tb));
   const int threads = kLaunchThreads<kGateUp, N_MAX, kReturn>;
-  return (int)launch_kernel(kern, dim3(grid), dim3(threads), Cfg::kSmemBytes, stream, true, tm, tb, *args);
+  mf_gemm_args b = *args;
+  if (kPair) {
+    b.m_blocks /= 2;
+    grid &= ~1;
+  }
+  return (int)launch_cluster(kern, dim3(grid), dim3(threads), Cfg::kSmemBytes, stream, true, kPair ? 2 : 1, tm, tb, b);
+}
+
+// Two accumulators (gate and up, or two weight blocks) on tiles of up to 256 rows: CTA pairs wherever they can be formed, that
+// is, for an even number of units per token tile, two CTAs or more, and token boxes that fit one half of a tile.  They are the
+// faster form for all tiles of this height (whole layer, single / pairs: 72 experts, 85 rows expected 548 / 520, 111 rows 610 / 577
+// us, 265 rows 831 / 781; 36 experts, 882 rows 1350 / 1276, 1820 rows 2901 / 2739).
+static int launch_two_256(const void* tmap, const mf_gemm_args* args, int grid, cudaStream_t stream) {
+  const bool boxes = args->b_tmap == nullptr || (args->b_box_rows > 0 && args->b_box_rows <= 128);  // a half of the rows per CTA
+  if (args->m_blocks % 2 == 0 && grid >= 2 && boxes) return launch<true, 256, false, true>(tmap, args, grid, stream);
+  return launch<true, 256>(tmap, args, grid, stream);
 }
 
 static int check_args(const mf_gemm_args* a, int n_max, int grid) {
@@ -926,7 +1031,7 @@ int mf_gemm_gate_up(const void* tmap, const mf_gemm_args* args, int n_max, int g
   if (n_max == 32) return mf::launch<true, 32>(tmap, args, grid, s);
   if (n_max == 64) return mf::launch<true, 64>(tmap, args, grid, s);
   if (n_max == 128) return mf::launch<true, 128>(tmap, args, grid, s);
-  return mf::launch<true, 256>(tmap, args, grid, s);
+  return mf::launch_two_256(tmap, args, grid, s);
 }
 
 int mf_gemm_down(const void* tmap, const mf_gemm_args* args, int n_max, int grid, mf_stream_t stream) {
@@ -939,7 +1044,7 @@ int mf_gemm_down(const void* tmap, const mf_gemm_args* args, int n_max, int grid
     if (n_max == 32) return mf::launch<true, 32>(tmap, args, grid, s);
     if (n_max == 64) return mf::launch<true, 64>(tmap, args, grid, s);
     if (n_max == 128) return mf::launch<true, 128>(tmap, args, grid, s);
-    return mf::launch<true, 256>(tmap, args, grid, s);
+    return mf::launch_two_256(tmap, args, grid, s);
   }
   if (args->ret_peer != nullptr) {  // owner reduce + return push fused into the epilogue (four extra warps)
     if (n_max == 32) return mf::launch<false, 32, true>(tmap, args, grid, s);

@@ -32,20 +32,6 @@ constexpr int kSkThreads = 192;   // warp 0 TMA, warp 1 UMMA, warps 2-5 tensor m
 constexpr int kSkSmem = kSkStages * kSkStage + 1024 + 256;
 static_assert(kSkN * kSkM * 4 <= kSkStages * kSkStage, "the partial tile is parked in the pipeline stages");
 
-__device__ __forceinline__ uint32_t cluster_rank() {
-  uint32_t r;
-  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-  return r;
-}
-__device__ __forceinline__ void cluster_sync_all() {
-  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-// The same shared-memory offset in CTA `rank` of this cluster.
-__device__ __forceinline__ uint32_t cluster_map(uint32_t smem_addr, uint32_t rank) {
-  uint32_t r;
-  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(smem_addr), "r"(rank));
-  return r;
-}
 __device__ __forceinline__ float ld_cluster_f32(uint32_t addr) {
   float v;
   asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(addr) : "memory");

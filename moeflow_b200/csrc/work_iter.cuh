@@ -175,9 +175,23 @@ struct SegReader {
   }
 };
 
+// A CTA pair works on the same segments: CTA 0 asks the counter and leaves each answer here in CTA 1's shared memory.  An answer
+// is at most one segment ahead of a K block whose stage CTA 1 has filled (CTA 0's producer waits for that stage's MMA, which
+// needs both CTAs' operands), so with up to kPairMail - 2 pipeline stages no answer is overwritten before it is read.
+constexpr int kPairMail = 8;
+struct PairMail {
+  int u[kPairMail];
+  uint64_t bar[kPairMail];
+  __device__ __forceinline__ void init() {
+    for (int i = 0; i < kPairMail; ++i) mbar_init(&bar[i], 1);
+  }
+};
+
 // Producer side (the weight producer warp, the whole warp calls).  The segment behind the current one is prepared in
 // three steps spread over the current one's first K blocks: ask the counter, fetch the tile's words, publish.
-struct SegFeed {
+// kPair: the two CTAs of a pair (rank 0 and 1) publish the same segments, each in its own ring.
+template <bool kPair>
+struct SegFeedOf {
   WorkIter it;
   SegRing* ring;
   volatile int* abort_flag;
@@ -186,8 +200,33 @@ struct SegFeed {
   int i = 0, stage = 0;
   uint32_t phase = 0;
   bool have = false, bad_tile = false, ok = true;
-  __device__ __forceinline__ SegFeed(const WorkIter& w, SegRing* r, volatile int* abort, unsigned long long ns)
+  PairMail* mail = nullptr;
+  int rank = 0, n_mail = 0;
+  __device__ __forceinline__ SegFeedOf(const WorkIter& w, SegRing* r, volatile int* abort, unsigned long long ns)
       : it(w), ring(r), abort_flag(abort), wait_ns(ns) {}
+
+  __device__ __forceinline__ void step() {
+    if (!kPair || rank == 0 || it.a->sched == nullptr) it.step();
+  }
+  __device__ __forceinline__ void stepped() {
+    if (!kPair || it.stream || it.a->sched == nullptr) {
+      it.stepped();
+      return;
+    }
+    const int i_ = n_mail % kPairMail;
+    if (rank == 0) {
+      it.stepped();
+      if (lane_id() == 0) {
+        st_cluster_s32(cluster_map(smem_u32(&mail->u[i_]), 1), it.u);
+        mbar_arrive_cluster<true>(cluster_map(smem_u32(&mail->bar[i_]), 1));
+      }
+      __syncwarp();
+    } else {
+      ok = ok && __all_sync(0xffffffffu, mbar_wait_bounded<true>(&mail->bar[i_], (uint32_t)(n_mail / kPairMail) & 1u, abort_flag, wait_ns));
+      it.u = ok ? *reinterpret_cast<volatile int*>(&mail->u[i_]) : 0x7fffffff;  // (past every unit)
+    }
+    ++n_mail;
+  }
 
   __device__ __forceinline__ void publish() {
     ok = ok && __all_sync(0xffffffffu, mbar_wait_bounded(&ring->empty[i], phase ^ 1u, abort_flag, wait_ns));
@@ -207,13 +246,18 @@ struct SegFeed {
   // One of the three steps; after the third the next segment is in `nx` (have == false: there is none).
   __device__ __forceinline__ void advance() {
     if (stage == 0) {
-      it.step();
+      step();
     } else if (stage == 1) {
-      it.stepped();
+      stepped();
       have = it.locate(nx);
     } else if (stage == 2) {
-      // a plan built for wider tiles than this kernel: such segments are skipped (and reported)
-      while (have && (unsigned)nx.n_rows > (unsigned)it.n_max) {
+      // a plan built for wider tiles than this kernel: such segments are skipped (and reported); by a pair they are worked
+      // through as tiles without rows, since skipping runs ahead of the other CTA
+      if (kPair && have && (unsigned)nx.n_rows > (unsigned)it.n_max) {
+        bad_tile = true;
+        nx.n_rows = 0;
+      }
+      while (!kPair && have && (unsigned)nx.n_rows > (unsigned)it.n_max) {
         bad_tile = true;
         it.step();
         it.stepped();
@@ -235,5 +279,6 @@ struct SegFeed {
     return have && ok;
   }
 };
+using SegFeed = SegFeedOf<false>;
 
 }  // namespace mf

@@ -1,0 +1,74 @@
+"""256-row tiles on CTA pairs against the same layer on one CTA (which takes the single form): the same products in the same
+order, so the same bits, at the edges of a tile's halves, for gathered and boxed rows, odd and even block counts."""
+
+import pytest
+import torch
+
+from moeflow_b200 import MoEConfig
+from moeflow_b200.testing import make_hidden, make_weights
+
+pytestmark = pytest.mark.gpu
+
+
+def _layer(cfg, w13, w2, tokens, n_sms=None, **kw):
+    from moeflow_b200.fixed import FixedEPLayer
+
+    layer = FixedEPLayer(cfg, 0, 1, w13, w2, capacity=tokens, backend="cuda", gemm_kwargs={"block_m": 256, **kw}, wait_ns=200_000_000)
+    if n_sms is not None:
+        layer.n_sms = n_sms  # CTAs of the GEMMs; the plan stays the one for the whole device
+    return layer
+
+
+@pytest.mark.parametrize("hidden,inter", [(512, 256), (768, 128), (1024, 512)])
+@pytest.mark.parametrize("counts", [(1, 16, 17, 31), (32, 33, 127, 128), (129, 0, 255, 256), (257, 500, 3, 64)])
+@pytest.mark.parametrize("kw", [{"permute_rows": False}, {"permute_rows": True}, {"permute_rows": False, "b_tma": False}])
+def test_pairs_equal_single_ctas_bitwise(hidden, inter, counts, kw):
+    cfg = MoEConfig(hidden_size=hidden, moe_intermediate_size=inter, n_routed_experts=4, top_k=1)
+    w13, w2 = make_weights(cfg, 0, device="cuda")
+    t = sum(counts)
+    x = make_hidden(t, cfg, 1, device="cuda")
+    g = torch.Generator().manual_seed(2)
+    ids = torch.repeat_interleave(torch.arange(4), torch.tensor(counts))[torch.randperm(t, generator=g)].int()[:, None].cuda()
+    weights = torch.rand(t, 1, generator=g).cuda() + 0.5
+    outs = []
+    for n_sms in (1, 2, 5, None):  # (an odd number of CTAs leaves one out)
+        layer = _layer(cfg, w13, w2, t, n_sms, **kw)
+        for _ in range(2):
+            outs.append(layer.forward_routed(x, weights, ids).clone())
+            assert layer.check_status()["code"] == 0
+    assert outs[0].abs().sum() > 0
+    assert all(torch.equal(o, outs[0]) for o in outs[1:])
+
+
+@pytest.mark.parametrize("split", [1, 2, 4, 0])
+def test_cut_units_of_pairs(split):
+    """K splits add the same segments in the same order as one CTA does; stream-K cuts elsewhere (fp32 sums)."""
+    from moeflow_b200.ops.grouped_gemm import gate_up_swiglu, plan_from_offsets
+
+    offsets = [0, 200, 205, 461]
+    g = torch.Generator().manual_seed(3)
+    w13 = (torch.randn(3, 1024, 1024, generator=g) / 16).bfloat16().cuda()
+    x = torch.randn(offsets[-1], 1024, generator=g).bfloat16().cuda()
+    got = []
+    for grid in (1, 2, 148):
+        status = torch.zeros(1, dtype=torch.int64, device="cuda")
+        got.append(gate_up_swiglu(x, w13, plan_from_offsets(offsets, 256, x.device), split=split, status=status, wait_ns=200_000_000, grid=grid).clone())
+        assert int(status.item()) == 0
+    for o in got[1:]:
+        # (stream-K: activations rounded to bf16 once, so 2**-8 of one where the sums straddle a rounding point)
+        assert torch.equal(o, got[0]) if split else (o.float() - got[0].float()).norm() < 2.0**-9 * got[0].float().norm()
+
+
+def test_a_tile_that_is_too_tall_is_reported_and_not_stored():
+    from moeflow_b200.ops.grouped_gemm import gate_up_swiglu, plan_from_offsets
+
+    g = torch.Generator().manual_seed(4)
+    w13 = (torch.randn(2, 512, 512, generator=g) / 16).bfloat16().cuda()
+    x = torch.randn(400, 512, generator=g).bfloat16().cuda()
+    tp = plan_from_offsets([0, 100, 400], 256, x.device)
+    tp.tile_n[1] = 300
+    status = torch.zeros(1, dtype=torch.int64, device="cuda")
+    out = gate_up_swiglu(x, w13, tp, status=status, wait_ns=200_000_000)
+    torch.cuda.synchronize()
+    assert int(status.item()) & 0xFF == 7  # bad argument
+    assert out[:100].abs().sum() > 0 and int(out[100:356].count_nonzero()) == 0
