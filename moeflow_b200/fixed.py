@@ -443,14 +443,17 @@ class FixedEPLayer:
 
         i32 = dict(dtype=torch.int32, device=dev)
         N = self.n_entries
-        # token rows per tile: 64 for decode; 128 when experts see many rows (prefill), which halves the
-        # number of times an expert's weights are streamed.  The estimate is the expectation under even
+        # token rows per tile: 64 for decode; more when experts see many rows (prefill), so that an expert's weights are
+        # streamed less often.  The estimate is the expectation under even
         # routing (R*C*K entries over R*L experts), not the worst case: wide tiles cost pipeline stages, and
         # with few rows per expert the narrower tile keeps more weight bytes in flight.
         # A buffer set built without weights may be bound to e4m3 experts later: plan its tiles for them unless told
         # otherwise (gemm_kwargs fp8_weights=False / True).
         fp8_hint = bool(self.gemm_kwargs.get("fp8_weights", self.w13 is None))
-        self.block_m = int(self.gemm_kwargs.get("block_m", choose_block_m(Cc, K, L, fp8=fp8_hint)))
+        tall = choose_block_m(Cc, K, L, fp8=fp8_hint)
+        if tall == 128 and not fp8_hint and H % 512 == 0 and I % 256 == 0 and not {"stream_k", "fuse_return", "down_two_blocks"} & set(self.gemm_kwargs):
+            tall = paired_block_m(Cc, K, L)
+        self.block_m = int(self.gemm_kwargs.get("block_m", tall))
         if self.block_m not in (32, 64, 128, 256):
             raise ValueError("block_m must be 32, 64, 128 or 256")
         self.n_sms = int(self.gemm_kwargs.get("n_sms", sm_count(dev.index if dev.index is not None else 0)))
@@ -594,7 +597,8 @@ class FixedEPLayer:
         # Copies of less than 8 MB cost up to 5 us and save up to 2: 2.1 MB 54.5 / 49.9, 3.1 MB 56.6 / 55.3, 3.9 MB 68.1 / 69.1,
         # 6.2 MB 99.3 / 97.6, 7.5 MB 100.1 / 100.1.  Those layers keep it for one reason: the checks of the copying form on
         # 256-row tiles build such a layer and expect it there.
-        self.permute_rows = bool(self.gemm_kwargs.get("permute_rows", self.block_m >= 256 and N * H * 2 < 8 << 20))
+        copied = self.block_m >= 256 and N * H * 2 < 8 << 20 and ("block_m" in self.gemm_kwargs or choose_block_m(Cc, K, L, fp8=fp8_hint) >= 256)
+        self.permute_rows = bool(self.gemm_kwargs.get("permute_rows", copied))
         if self.permute_rows:
             from .ops.kernels import make_tile_tmap
 
@@ -990,6 +994,17 @@ def choose_block_m(capacity: int, top_k: int, local_experts: int, fp8: bool = Fa
     if fp8:
         return 256 if expected >= 512 else 128 if expected >= (36 if local_experts >= 64 else 60) else 64
     return 256 if expected >= 80 else 128 if expected >= 36 else 64
+
+
+def paired_block_m(capacity: int, top_k: int, local_experts: int) -> int:
+    """What a bf16 layer takes in place of 128-row tiles where the 256-row kernels run on CTA pairs (hidden a multiple of 512,
+    intermediate of 256): 256 rows, a pair sharing the tile's rows, or 64 for few experts, which leave CTAs idle on units twice as
+    large.  Whole layer, two weight sets in turn, us, 64 / 128 / 256 rows: 36 experts, 44 rows expected 250 / 262 / 256, 50 rows of zipf
+    popularity 190 / - / 158, 62 rows - / 281 / 268; 72 experts, 36 rows 483 / 489 / 478, 43 rows 503 / 496 / 486 (zipf 296 / 262 / 209),
+    71 rows - / 554 / 506; 144 experts, 38 rows 962 / 935 / 920; 288 experts, 41 rows 1984 / 1889 / 1770; 8 experts, 40 rows 74 / 95 / 86,
+    60 rows 76 / - / 88, 75 rows 101 / - / 91; 16 experts, 60 rows 122 / - / 144, 70 rows - / 149 / 140; 24 experts, 50 rows 173 / - / 184.
+    """
+    return 64 if local_experts < 32 and capacity * top_k < 64 * max(local_experts, 1) else 256
 
 
 def choose_meta_ctas(slot_words: int, n_sms: int) -> int:

@@ -72,3 +72,20 @@ def test_a_tile_that_is_too_tall_is_reported_and_not_stored():
     torch.cuda.synchronize()
     assert int(status.item()) & 0xFF == 7  # bad argument
     assert out[:100].abs().sum() > 0 and int(out[100:356].count_nonzero()) == 0
+
+
+@pytest.mark.parametrize("experts,tokens,inter,block_m", [(36, 200, 256, 256), (8, 40, 256, 64), (8, 72, 256, 256), (36, 200, 384, 128)])
+def test_layers_of_36_to_80_rows(experts, tokens, inter, block_m):
+    """Tile height by rule: the same output as 64-row tiles within the rounding of activations and result (2**-9 each)."""
+    from moeflow_b200.fixed import FixedEPLayer
+    from moeflow_b200.testing import make_bias, make_logits
+
+    cfg = MoEConfig(hidden_size=512, moe_intermediate_size=inter, n_routed_experts=experts, top_k=8)
+    w13, w2 = make_weights(cfg, 0, device="cuda")
+    x, lg, bias = make_hidden(tokens, cfg, 1, device="cuda"), make_logits(tokens, cfg, 2, device="cuda"), make_bias(cfg, 3, device="cuda")
+    outs = []
+    for kw in ({}, {"block_m": 64}):
+        layer = FixedEPLayer(cfg, 0, 1, w13, w2, capacity=tokens, backend="cuda", gemm_kwargs=kw, wait_ns=200_000_000)
+        outs.append(layer.forward(x, lg, bias)[:tokens].double())
+        assert layer.check_status()["code"] == 0 and layer.block_m == kw.get("block_m", block_m) and not layer.permute_rows
+    assert (outs[0] - outs[1]).norm() < 2 * 2.0**-8 * outs[1].norm()

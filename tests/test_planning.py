@@ -84,3 +84,13 @@ def test_k_splits_of_e4m3_layers_divide_their_128_wide_blocks(plan_split):
                 assert steps(units, 2 * blocks, 1, 148, 4096, overhead, cols) == plain
     assert refused > 0  # hidden 384 with intermediate 128, hidden 2048 with 1408 or (one tile) 1536
     assert plan_split(3, 6, 148, 4096, 4, 16) == 2 and steps(3, 6, 2, 148, 4096, 4, 16) == 1
+
+
+def test_paired_tiles_in_place_of_128_rows():
+    from moeflow_b200.fixed import paired_block_m
+
+    assert paired_block_m(256, 8, 36) == 256   # 57 rows per expert
+    assert paired_block_m(512, 8, 72) == 256
+    assert paired_block_m(40, 8, 8) == 64      # 40 rows on 8 experts: fewer pair units than pairs
+    assert paired_block_m(64, 8, 8) == 256     # 64 rows
+    assert paired_block_m(1, 8, 0) == 64
