@@ -187,17 +187,12 @@ __device__ __forceinline__ void return_finish(const mf_gemm_args& a, int complet
   }
 }
 
-// Last step of the epilogue for C token columns of one weight row: the activation (gate/up), or the routing
-// weight (down), then the stores.  The arithmetic of all C columns comes first and has no branch that depends on
-// the column, so that the C dependency chains (exp, reciprocal) overlap: the epilogue warps are alone on their
-// scheduler and a column-by-column loop ran at one chain's latency (about 300 cycles per column).
-// v: first accumulator (gate, or the only one); w: second accumulator (up; with two_blocks the second weight block).
-// With a staging buffer (`stage`, 1 KB of shared memory owned by the calling warp; C == 16) the 16 x 32 block is transposed through it, and every lane stores 16 bytes (8 weight rows of one
-// token): two store instructions per block instead of sixteen 64-byte ones.
+// Last step of the epilogue for C values of each of one or two accumulators: the activation (gate/up), or the routing weight
+// (down).  v: first accumulator (gate, or the only one); w: second accumulator (up; with two_blocks the second weight block);
+// sc: routing weights.  No branch depends on the column, so that the C dependency chains (exp, reciprocal) overlap: the epilogue
+// warps are alone on their scheduler and a column-by-column loop ran at one chain's latency (about 300 cycles per column).
 template <bool kTwoAcc, int C>
-__device__ __forceinline__ void finish_store(const mf_gemm_args& a, float (&v)[C], float (&w)[C], const float (&sc)[C],
-                                             int n0, int n_rows, int row_start, long long out_col,
-                                             uint8_t* stage = nullptr, int lane = 0) {
+__device__ __forceinline__ void finish(const mf_gemm_args& a, float (&v)[C], float (&w)[C], const float (&sc)[C]) {
   if (kTwoAcc && !a.two_blocks) {
     if (a.round_h) {
 #pragma unroll
@@ -215,30 +210,14 @@ __device__ __forceinline__ void finish_store(const mf_gemm_args& a, float (&v)[C
       if (kTwoAcc) w[j] *= sc[j];
     }
   }
+}
+
+// ... of C token columns of one weight row per lane, and their stores, 2 bytes each.
+template <bool kTwoAcc, int C>
+__device__ __forceinline__ void finish_store(const mf_gemm_args& a, float (&v)[C], float (&w)[C], const float (&sc)[C],
+                                             int n0, int n_rows, int row_start, long long out_col) {
+  finish<kTwoAcc, C>(a, v, w, sc);
   const bool second = kTwoAcc && a.two_blocks;  // the other weight block's outputs, 128 columns further
-  if (C == 16 && stage != nullptr && (a.out_pitch & 7) == 0 &&
-      (reinterpret_cast<uintptr_t>(a.out) & 15) == 0) {  // 16-byte stores need rows that start on 16 bytes
-    __nv_bfloat16* st = reinterpret_cast<__nv_bfloat16*>(stage);
-    __nv_bfloat16* out = static_cast<__nv_bfloat16*>(a.out) + (long long)(row_start + n0) * a.out_pitch + (out_col - lane) +
-                         (lane & 3) * 8;
-    const uint4* src = reinterpret_cast<const uint4*>(stage) + lane;  // token lane / 4 (+ 8), rows 8 (lane & 3) ..
-#pragma unroll
-    for (int pass = 0; pass < (kTwoAcc ? 2 : 1); ++pass) {
-      if (pass == 1 && !second) break;
-      __syncwarp();  // the previous block's reads are done
-#pragma unroll
-      for (int j = 0; j < C; ++j) st[j * 32 + lane] = __float2bfloat16_rn(pass == 0 ? v[j] : w[j]);
-      __syncwarp();
-#pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        const int t = 8 * h + (lane >> 2);
-        const uint4 x = src[32 * h];
-        if (n0 + t < n_rows)
-          *reinterpret_cast<uint4*>(out + (long long)t * a.out_pitch + (pass == 1 ? kBlockM : 0)) = x;
-      }
-    }
-    return;
-  }
   const bool all = n0 + C <= n_rows;
   __nv_bfloat16* p = static_cast<__nv_bfloat16*>(a.out) + (long long)(row_start + n0) * a.out_pitch + out_col;
 #pragma unroll
@@ -247,6 +226,30 @@ __device__ __forceinline__ void finish_store(const mf_gemm_args& a, float (&v)[C
       p[(long long)j * a.out_pitch] = __float2bfloat16_rn(v[j]);
       if (second) p[(long long)j * a.out_pitch + kBlockM] = __float2bfloat16_rn(w[j]);
     }
+  }
+}
+
+// Outputs of 16 token columns x 32 weight rows, in the layout of tmem_ld_16x16 (x[8 h ..]: weight rows 16 h ..), to global memory
+// through 1 KB of shared memory owned by the warp: pairs of tokens are rounded together and stored transposed, a token's 32 values
+// in four chunks of 16 bytes (chunk c of token t at place c ^ (t / 2 & 3): no bank conflicts either way), and every lane then
+// stores 16 bytes of one token.  `p`: the first token's first value of this warp.
+__device__ __forceinline__ void store_16x32(const float (&x)[16], uint8_t* stage, int lane, __nv_bfloat16* p, int pitch, int rows) {
+  const int m = lane >> 3, j = lane & 7;
+  const uint32_t to = smem_u32(stage) + j * 64 + ((m ^ (j >> 1)) << 4);
+  __syncwarp();  // the previous block's reads are done
+#pragma unroll
+  for (int k = 0; k < 2; ++k) {
+    const uint32_t r[4] = {pack_bf16x2(x[4 * k], x[4 * k + 1]), pack_bf16x2(x[4 * k + 2], x[4 * k + 3]),
+                           pack_bf16x2(x[8 + 4 * k], x[8 + 4 * k + 1]), pack_bf16x2(x[8 + 4 * k + 2], x[8 + 4 * k + 3])};
+    stmatrix_x4_trans(to + k * 512, r);
+  }
+  __syncwarp();
+  const int t = lane >> 2, c = lane & 3;
+  const uint8_t* from = stage + t * 64 + ((c ^ (t >> 1)) << 4);
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    const uint4 y = *reinterpret_cast<const uint4*>(from + h * 512);
+    if (t + 8 * h < rows) *reinterpret_cast<uint4*>(p + (long long)(t + 8 * h) * pitch + c * 8) = y;
   }
 }
 
@@ -761,15 +764,46 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
           return (scaled && n < n_rows) ? __ldcg(a.row_scale + row_start + n) : 1.f;
         };
         float s_next = scale_of(c_begin);
+        // 16-byte stores need rows that start on 16 bytes
+        const bool wide_stores = (a.out_pitch & 7) == 0 && (reinterpret_cast<uintptr_t>(a.out) & 15) == 0;
+        uint8_t* stage = out_stage + (warp - 4) * kOutStageBytes;
+        __nv_bfloat16* out = static_cast<__nv_bfloat16*>(a.out) + (long long)row_start * a.out_pitch + (out_col - lane);
 #pragma unroll 1
-        for (int c0 = c_begin; c0 < c_end; c0 += 16) {
+        for (int c0 = c_begin; c0 < c_end && wide_stores; c0 += 16) {
+          uint32_t g[16], up[16];
+          tmem_ld_16x16(taddr + c0, g);
+          tmem_ld_16x16(taddr + (16u << 16) + c0, g + 8);
+          if (kGateUp) {
+            tmem_ld_16x16(tup + c0, up);
+            tmem_ld_16x16(tup + (16u << 16) + c0, up + 8);
+          }
+          const float s_cur = s_next;
+          s_next = scale_of(c0 + 16);
+          tmem_ld_wait();
+          if (warp == 4 && lane == 0) MF_STAMP_ONCE(8);
+          float v[16], w[16], sc[16], s4[4];
+#pragma unroll
+          for (int j = 0; j < 4; ++j) s4[j] = scaled ? __shfl_sync(0xffffffffu, s_cur, 8 * (j >> 1) + 2 * (lane & 3) + (j & 1)) : 1.f;
+#pragma unroll
+          for (int j = 0; j < 16; ++j) {
+            v[j] = __uint_as_float(g[j]);
+            w[j] = kGateUp ? __uint_as_float(up[j]) : 0.f;
+            sc[j] = s4[(j >> 2 & 1) * 2 + (j & 1)];
+          }
+          finish<kGateUp, 16>(a, v, w, sc);
+          __nv_bfloat16* p = out + (long long)c0 * a.out_pitch;
+          store_16x32(v, stage, lane, p, a.out_pitch, n_rows - c0);
+          if (kGateUp && a.two_blocks) store_16x32(w, stage, lane, p + kBlockM, a.out_pitch, n_rows - c0);
+          if (warp == 4 && lane == 0) MF_STAMP_ONCE(9);
+        }
+#pragma unroll 1
+        for (int c0 = c_begin; c0 < c_end && !wide_stores; c0 += 16) {
           uint32_t g[16], up[16];
           tmem_ld_16(taddr + c0, g);
           if (kGateUp) tmem_ld_16(tup + c0, up);
           const float s_cur = s_next;
           s_next = scale_of(c0 + 16);
           tmem_ld_wait();
-          if (warp == 4 && lane == 0) MF_STAMP_ONCE(8);
           float v[16], w[16], sc[16];
 #pragma unroll
           for (int j = 0; j < 16; ++j) {
@@ -777,8 +811,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
             w[j] = kGateUp ? __uint_as_float(up[j]) : 0.f;
             sc[j] = scaled ? __shfl_sync(0xffffffffu, s_cur, j) : 1.f;
           }
-          finish_store<kGateUp, 16>(a, v, w, sc, c0, n_rows, row_start, out_col, out_stage + (warp - 4) * kOutStageBytes, lane);
-          if (warp == 4 && lane == 0) MF_STAMP_ONCE(9);
+          finish_store<kGateUp, 16>(a, v, w, sc, c0, n_rows, row_start, out_col);
         }
         if (warp == 4 && lane == 0) MF_STAMP_ONCE(10);
         tc_fence_before_sync();
