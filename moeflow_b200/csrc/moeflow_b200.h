@@ -302,6 +302,9 @@ typedef struct {
   // reduced row is stored there as well (zeros for rows without a hit) and no arrival is sent: no combine launch follows.
   void* out;
   int rows;                  // > 0: only these first rows of `out` are written
+  // Optional, both or neither, with `out`: [rows of out, H] bf16, 16-byte aligned; out = (add1 + row) + add2, rounded to bf16 each time.
+  const void* add1;
+  const void* add2;
 } mf_reduce_push_args;
 int mf_owner_reduce_push(const mf_reduce_push_args* args, mf_stream_t stream);
 

@@ -40,6 +40,22 @@ __device__ __forceinline__ uint4 pack_bf16x8(const float (&acc)[8]) {
   return o;
 }
 
+// (add1 + r) + add2 for one chunk of row t, rounded to bf16 after either addition.
+__device__ __forceinline__ uint4 add_rows(const mf_reduce_push_args& a, int t, int c, const uint4& r) {
+  const size_t at = (size_t)t * (a.H / 8) + c;
+  const uint4 x = __ldcg(static_cast<const uint4*>(a.add1) + at), s = __ldcg(static_cast<const uint4*>(a.add2) + at);
+  float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+  acc_bf16x8(acc, x);
+  acc_bf16x8(acc, r);
+#pragma unroll
+  for (int i = 0; i < 8; ++i) acc[i] = bf16_round(acc[i]);
+  acc_bf16x8(acc, s);
+  return pack_bf16x8(acc);
+}
+
+// With add1 and add2 (decode model: residual stream and shared expert) the output is their sum with the routed row.  The shared
+// expert's down projection added the three itself before and could only start its last step behind this kernel.
+//
 // kThreads: kRowThreads, or 512 where a row has more 16-byte chunks than that and there are only a few hundred rows: one round
 // trip to L2 behind the down GEMM instead of two.  Layer (36 bf16 experts), 256 / 512 threads: 64 rows 248.2 / 247.5 us, 128 rows
 // 255.2 / 254.0, 256 rows 287 / 272; above, no gain that lasts: 300 rows 287 / 283, 400 rows 322 / 320, 512 rows 368 / 376.
@@ -93,11 +109,12 @@ __global__ void __launch_bounds__(kThreads) owner_reduce_push_kernel(const mf_re
       }
       const uint4 packed = pack_bf16x8(acc);
       dst[c] = packed;
-      if (out != nullptr) out[c] = packed;
+      if (out != nullptr) out[c] = a.add1 != nullptr ? add_rows(a, t, c, packed) : packed;
     }
   } else if (a.out != nullptr && (a.rows <= 0 || t < a.rows)) {
     uint4* out = static_cast<uint4*>(a.out) + (size_t)t * (a.H / 8);
-    for (int c = tid; c < a.H / 8; c += kThreads) out[c] = make_uint4(0u, 0u, 0u, 0u);
+    const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
+    for (int c = tid; c < a.H / 8; c += kThreads) out[c] = a.add1 != nullptr ? add_rows(a, t, c, zero) : zero;
   }
   if (a.out != nullptr) {
     if (trace) trace[2] = global_timer_ns();  // row stored
@@ -202,6 +219,7 @@ extern "C" {
 int mf_owner_reduce_push(const mf_reduce_push_args* a, mf_stream_t stream) {
   if (!a || a->K > 32 || a->H % 8 != 0 || a->R < 1 || a->C < 1) return -1;
   if (a->out != nullptr && a->R != 1) return -2;
+  if ((a->add1 != nullptr) != (a->add2 != nullptr) || (a->add1 != nullptr && a->out == nullptr)) return -3;
   if (a->R * a->C <= 256 && a->H / 8 > mf::kRowThreads)
     return (int)mf::launch_kernel(mf::owner_reduce_push_kernel<512>, dim3(a->R * a->C), dim3(512), 0,
                                   static_cast<cudaStream_t>(stream), true, *a);

@@ -375,6 +375,36 @@ class FixedEPLayer:
             out = self.stage_combine(hit, x.dtype)
         return out[:T]
 
+    @property
+    def adds_to_output(self) -> bool:
+        """Does this layer's last kernel write the output, so that ``forward_add`` is available?"""
+        return self.backend == "cuda" and self.fuse_combine
+
+    def forward_add(self, x, logits, bias, num_valid, first: torch.Tensor, second: torch.Tensor, out: torch.Tensor, join=None) -> torch.Tensor:
+        """``out = (first + forward(x, ...)) + second``, all ``[T, H]``, rounded to bf16 after each addition, by the layer's last
+        kernel (one rank).  ``join`` is called ahead of that kernel's launch, with everything else launched: ``second`` may be
+        the work of another stream that is waited for there."""
+        for t in (first, second, out):
+            if tuple(t.shape) != (x.shape[0], self.H) or t.dtype != torch.bfloat16 or not t.is_cuda or not t.is_contiguous() or t.data_ptr() % 16:
+                raise ValueError("contiguous bf16 rows on the device expected")
+        if not self.adds_to_output:
+            raise ValueError("the output is merged from several ranks")
+        if x.shape[0] > self.C:
+            raise ValueError(f"{x.shape[0]} tokens exceed capacity {self.C}")
+        if x.shape[0] == 0:
+            if join is not None:
+                join()
+            return out
+        _, meta_done = self._cuda_dispatch(x, None, None, num_valid, logits=logits, bias=bias, whole=True)
+        self._cuda_experts("GEMM2", meta_done=meta_done)
+        if join is not None:
+            join()
+        a = type(self._a_reduce_out).from_buffer_copy(self._a_reduce_out)
+        a.out, a.rows, a.add1, a.add2 = out.data_ptr(), x.shape[0], first.data_ptr(), second.data_ptr()
+        self._keep += [first, second, out]
+        self._cuda_reduce(a)
+        return out
+
     def forward(self, x, logits, bias, num_valid: torch.Tensor | None = None, stop_after: str | None = None):
         """Whole layer; ``stop_after`` (one of ``STAGES``) truncates it for prefix-graph stage timing."""
         if stop_after is not None and stop_after not in STAGES:
@@ -902,7 +932,7 @@ class FixedEPLayer:
             _lib.check(lib.mf_gemm_down_fp8(f["tm2"], C.byref(f["a2"]), self.block_m, self.n_sms, s), "fp8 down gemm")
             if stop_after == "GEMM2":
                 return
-            self._cuda_reduce(to_output)
+            self._cuda_reduce(self._a_reduce_out if to_output else self._a_reduce)
             return
         if self.permute_rows:
             _lib.check(self._lib.mf_permute_rows(self._recv_store.data_ptr(), self.pitch * 2, self.entry_row.data_ptr(),
@@ -914,14 +944,14 @@ class FixedEPLayer:
         _lib.check(self._lib.mf_gemm_down(self._tmap2, C.byref(self._a_gemm2), self.block_m, self.n_sms, s), "down gemm")
         if stop_after == "GEMM2" or self.fuse_return:
             return
-        self._cuda_reduce(to_output)
+        self._cuda_reduce(self._a_reduce_out if to_output else self._a_reduce)
 
-    def _cuda_reduce(self, to_output: bool) -> None:
+    def _cuda_reduce(self, a) -> None:
+        """``a``: ``_a_reduce`` (partial rows only), or a block that names an output as well."""
         from .ops import _lib
 
-        a = self._a_reduce_out if to_output else self._a_reduce
         _lib.check(self._lib.mf_owner_reduce_push(C.byref(a), _lib.stream_ptr()), "owner_reduce_push")
-        if to_output and self._node_log is not None:
+        if a.out and self._node_log is not None:
             self._node_log["last"] = (_lib.last_captured_node(), [a])
 
     def _cuda_push_partials(self, partials: torch.Tensor) -> None:

@@ -68,13 +68,14 @@ class SharedExpert:
         self._gate_up = DenseProjection(self.w13, gate_up=True, limit=limit, status=self.status)
         self._down = DenseProjection(self.w2, status=self.status)
 
-    def begin(self, x: torch.Tensor, branch: torch.cuda.Stream) -> None:
+    def begin(self, x: torch.Tensor, branch: torch.cuda.Stream, whole: bool = False) -> torch.Tensor | None:
         """The gate/up half of ``add_to(x, ..., begun=branch)`` on a branch of the graph that is being captured: next to the
         router, the dispatch and the start of the routed experts, which leave most SMs idle, instead of behind the routed
-        experts (12 us of a decode layer)."""
+        experts (12 us of a decode layer).  ``whole``: the down half as well; returns the rows (valid behind the branch)."""
         branch.wait_stream(torch.cuda.current_stream())
         with torch.cuda.stream(branch):
             self._gate_up(x, self.act)
+            return self._down(self.act[: x.shape[0]], self.out) if whole else None
 
     def __call__(self, x: torch.Tensor) -> torch.Tensor:
         if not self.cuda:
@@ -141,12 +142,17 @@ class MoEBlock:
         # only in a graph, where a branch costs the host nothing per step
         capturing = fused and self.branch is not None and self.routed.backend == "cuda" and torch.cuda.is_current_stream_capturing()
         begun = self.branch if capturing else None
+        # one rank: the whole shared expert runs on the branch, and the routed experts' last kernel adds the three up
+        added = begun is not None and self.routed.adds_to_output and x.is_contiguous() and x.data_ptr() % 16 == 0
         if begun is not None:
-            self.shared.begin(h, begun)
+            beside = self.shared.begin(h, begun, whole=added)
         if self.router is not None:
             logits = self.router(h)
         else:
             logits = torch.matmul(h.to(self.gate_w.dtype), self.gate_w.transpose(0, 1)).to(torch.float32)
+        if added:
+            join = lambda: torch.cuda.current_stream().wait_stream(begun)
+            return self.routed.forward_add(h, logits, self.bias, num_valid, x, beside, torch.empty_like(h) if out is None else out, join)
         routed = self.routed.forward(h, logits, self.bias, num_valid)[: x.shape[0]]
         if begun is not None or (fused and routed.dtype == torch.bfloat16):
             return self.shared.add_to(h, x, routed, torch.empty_like(h) if out is None else out, begun)

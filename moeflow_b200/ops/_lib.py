@@ -215,6 +215,8 @@ class ReducePushArgs(C.Structure):
         ("trace", C.c_void_p),
         ("out", C.c_void_p),
         ("rows", C.c_int),
+        ("add1", C.c_void_p),
+        ("add2", C.c_void_p),
     ]
 
 
