@@ -186,6 +186,10 @@ int mf_router_topk(const float* logits, const float* bias, float* weights, int* 
 // mf_rmsnorm).
 int mf_add_rmsnorm(const void* x, const void* add, const void* gamma, void* sum, void* out, int rows, int hidden, float eps,
                    mf_stream_t stream);
+// mf_add_rmsnorm and, from the normalised rows, logits[r, e] = out[r, :] . gate[e, :] (gate [experts, hidden] bf16, fp32 sums).
+// sum and out overlap no input; hidden up to 16384.
+int mf_add_rmsnorm_logits(const void* x, const void* add, const void* gamma, void* sum, void* out, int rows, int hidden, float eps,
+                          const void* gate, int experts, float* logits, int n_sms, mf_stream_t stream);
 // Row *pos of the caches [B, kv_heads, S, head_dim] (bf16) from the keys and values of this step, each [B, kv_heads *
 // head_dim] with rows pitch elements apart; a position outside the cache stores nothing.  head_dim and pitch: multiples of
 // 8; all pointers 16-byte aligned.

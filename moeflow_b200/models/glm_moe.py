@@ -49,6 +49,14 @@ def _rmsnorm(x: torch.Tensor, gamma: torch.Tensor, eps: float) -> torch.Tensor:
     return (xf * torch.rsqrt(xf.pow(2).mean(-1, keepdim=True) + eps) * gamma.to(torch.float32)).to(x.dtype)
 
 
+#: Up to this many router logits per step (sequences x experts) come from the kernel that normalises the rows; it reads the gate matrix
+#: once per sequence, the dense kernel once per 64.  Normalisation and logits in a row of such pairs, cold gates, us, two launches / one:
+#: 36 experts, 1 sequence 6.5 / 4.2, 32 7.8 / 5.2, 64 8.7 / 9.2; 72 experts, 16 7.1 / 4.9, 32 7.8 / 7.9, 64 8.8 / 10.1; 288 experts, 4
+#: 7.3 / 6.1, 16 7.6 / 10.2.  Inside a decode step the second launch costs more: 64 sequences on 36 experts 226.2 / 222.4, on 72
+#: 294.1 / 301.3, 45 on 72 461.6 / 464.9.
+NORM_LOGITS = 2304
+
+
 class SharedExpert:
     """Dense SwiGLU MLP ``w2 . swiglu(w13 . x)`` for up to ``capacity`` rows per call.  ``block_m`` is accepted for older
     call sites and selects nothing."""
@@ -116,6 +124,17 @@ class RouterLogits:
     def __call__(self, h: torch.Tensor) -> torch.Tensor:
         return self._project(h, self.logits)
 
+    def fits_norm(self, rows: int) -> bool:
+        """Is ``after_norm`` the faster form?"""
+        return self.H <= 16384 and 0 < rows <= self.C and rows * self.E <= NORM_LOGITS
+
+    def after_norm(self, x: torch.Tensor, add: torch.Tensor, gamma: torch.Tensor, eps: float) -> tuple[torch.Tensor, torch.Tensor, torch.Tensor]:
+        """``(x + add, h = rmsnorm(x + add), router logits of h)`` in one launch."""
+        from ..ops.kernels import add_rmsnorm_logits
+
+        total, h = add_rmsnorm_logits(x, add, gamma, self.w, self.E, self.logits, eps)
+        return total, h, self.logits[: x.shape[0]]
+
 
 class MoEBlock:
     """Pre-norm MoE block: ``x + routed(norm(x)) + shared(norm(x))``."""
@@ -131,10 +150,14 @@ class MoEBlock:
                  out: torch.Tensor | None = None) -> torch.Tensor:
         """``add``: summand of ``x`` that is still missing (the attention output).  ``out`` (contiguous bf16 ``[T, H]``,
         not ``x``) receives the result."""
+        logits = None
         if add is not None and x.is_cuda and x.dtype == torch.bfloat16:
             from ..ops.kernels import add_rmsnorm
 
-            x, h = add_rmsnorm(x, add, self.norm_w, self.eps)
+            if self.router is not None and x.dim() == 2 and self.router.fits_norm(x.shape[0]):
+                x, h, logits = self.router.after_norm(x, add, self.norm_w, self.eps)
+            else:
+                x, h = add_rmsnorm(x, add, self.norm_w, self.eps)
         else:
             x = x if add is None else x + add
             h = _rmsnorm(x, self.norm_w, self.eps)
@@ -146,7 +169,9 @@ class MoEBlock:
         added = begun is not None and self.routed.adds_to_output and x.is_contiguous() and x.data_ptr() % 16 == 0
         if begun is not None:
             beside = self.shared.begin(h, begun, whole=added)
-        if self.router is not None:
+        if logits is not None:
+            pass
+        elif self.router is not None:
             logits = self.router(h)
         else:
             logits = torch.matmul(h.to(self.gate_w.dtype), self.gate_w.transpose(0, 1)).to(torch.float32)

@@ -277,6 +277,7 @@ def lib() -> C.CDLL:
         "mf_router_topk": [P, P, P, P, I, I, I, I, I, I, I, F, P],
         "mf_rmsnorm": [P, P, P, I, I, F, P],
         "mf_add_rmsnorm": [P, P, P, P, P, I, I, F, P],
+        "mf_add_rmsnorm_logits": [P, P, P, P, P, I, I, F, P, I, P, I, P],
         "mf_kv_append": [P, P, LL, P, P, P, I, I, I, I, P],
         "mf_dispatch_push": [C.POINTER(DispatchArgs), P],
         "mf_dispatch_local": [C.POINTER(DispatchArgs), C.POINTER(MetaArgs), P],

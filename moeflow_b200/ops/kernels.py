@@ -94,6 +94,31 @@ def add_rmsnorm(x: torch.Tensor, add: torch.Tensor, gamma: torch.Tensor, eps: fl
     return total, out
 
 
+def add_rmsnorm_logits(x: torch.Tensor, add: torch.Tensor, gamma: torch.Tensor, gate: torch.Tensor, experts: int, logits: torch.Tensor,
+                       eps: float = 1e-6) -> tuple[torch.Tensor, torch.Tensor]:
+    """``add_rmsnorm`` and the router logits of the normalised rows, ``logits[: rows] = h . gate[: experts]^T`` in fp32, in one
+    launch."""
+    for name, t in (("x", x), ("add", add), ("gamma", gamma), ("gate", gate)):
+        _need_cuda(t, name)
+        if t.dtype != torch.bfloat16:
+            raise ValueError("add_rmsnorm_logits takes bf16 tensors")
+    _need_cuda(logits, "logits")
+    hidden = x.shape[-1]
+    rows = x.numel() // hidden
+    if add.shape != x.shape or gamma.numel() != hidden or gate.dim() != 2 or gate.shape[1] != hidden or gate.shape[0] < experts:
+        raise ValueError("x, add, gamma and gate do not fit each other")
+    if logits.dtype != torch.float32 or logits.dim() != 2 or logits.shape[0] < rows or logits.shape[1] != experts:
+        raise ValueError("logits must be fp32 [rows, experts]")
+    total, out = torch.empty_like(x), torch.empty_like(x)
+    _lib.check(
+        _lib.lib().mf_add_rmsnorm_logits(x.data_ptr(), add.data_ptr(), gamma.data_ptr(), total.data_ptr(), out.data_ptr(), rows, hidden,
+                                         float(eps), gate.data_ptr(), experts, logits.data_ptr(), sm_count(x.device.index or 0),
+                                         _lib.stream_ptr()),
+        "add_rmsnorm_logits",
+    )
+    return total, out
+
+
 def kv_append(k: torch.Tensor, v: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor, pos: torch.Tensor) -> None:
     """Stores ``k`` / ``v`` (``[B, kv * d]``, equal row strides) as row ``pos`` (device int64 scalar) of the contiguous
     bf16 caches ``[B, kv, S, d]``."""

@@ -69,3 +69,34 @@ def test_rows_off_the_16_byte_grid_and_host_tensors_are_refused():
         with pytest.raises(ValueError):
             layer.forward(*args)
     assert not layer.forward(fine, lg, bias.cuda()).any() and layer.check_status()["code"] == 0
+
+
+@pytest.mark.parametrize("rows,hidden,experts", [(1, 8, 1), (3, 264, 7), (4, 4096, 36), (64, 4096, 36), (200, 1024, 17), (5, 16384, 9), (700, 512, 3)])
+def test_add_rmsnorm_logits(rows, hidden, experts):
+    from moeflow_b200.ops.kernels import add_rmsnorm, add_rmsnorm_logits
+
+    g = torch.Generator().manual_seed(rows)
+    x, add = (torch.randn(rows, hidden, generator=g).bfloat16().cuda() for _ in range(2))
+    gamma = torch.rand(hidden, generator=g).bfloat16().cuda() + 0.5
+    gate = torch.randn(experts + 3, hidden, generator=g).bfloat16().cuda()
+    logits = torch.full((rows + 2, experts), 9.0, device="cuda")
+    total, h = add_rmsnorm_logits(x, add, gamma, gate, experts, logits)
+    want_total, want_h = add_rmsnorm(x, add, gamma)
+    assert torch.equal(total, want_total) and torch.equal(h, want_h)
+    exact = h.double() @ gate[:experts].double().t()
+    # each product is exact in fp32; a sum of n of them in any order errs by at most n * 2**-24 of their absolute sum
+    bound = hidden * 2.0**-24 * (h.double().abs() @ gate[:experts].double().abs().t())
+    assert bool(((logits[:rows].double() - exact).abs() <= bound + 1e-30).all()) and bool((logits[rows:] == 9).all())
+
+
+def test_add_rmsnorm_logits_refuses_what_does_not_fit():
+    from moeflow_b200.ops.kernels import add_rmsnorm_logits
+
+    x, gamma = torch.zeros(4, 64, dtype=torch.bfloat16, device="cuda"), torch.ones(64, dtype=torch.bfloat16, device="cuda")
+    gate, logits = torch.zeros(8, 64, dtype=torch.bfloat16, device="cuda"), torch.zeros(4, 8, device="cuda")
+    add_rmsnorm_logits(x, x, gamma, gate, 8, logits)
+    for bad in (lambda: add_rmsnorm_logits(x, x[:3], gamma, gate, 8, logits), lambda: add_rmsnorm_logits(x, x, gamma, gate[:, :32].contiguous(), 8, logits),
+                lambda: add_rmsnorm_logits(x, x, gamma, gate, 9, logits), lambda: add_rmsnorm_logits(x, x, gamma, gate, 8, logits[:3].contiguous()),
+                lambda: add_rmsnorm_logits(x, x, gamma, gate.float(), 8, logits), lambda: add_rmsnorm_logits(x, x, gamma, gate, 8, logits.double())):
+        with pytest.raises(ValueError):
+            bad()
