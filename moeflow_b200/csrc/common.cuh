@@ -223,6 +223,33 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar, uint32_t parity
   }
 }
 
+// The same for a whole warp that waits together.  Every try is a vote, so that the compiler sees one branch for the warp and not a
+// loop that lanes leave one by one.
+__device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, volatile int* abort_flag, unsigned long long limit_ns) {
+  if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
+  unsigned long long t0 = 0;
+  unsigned spins = 0;
+  while (!__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) {
+    if ((++spins & 255u) != 0u) continue;
+    const unsigned long long now = global_timer_ns();
+    if (t0 == 0) t0 = now;
+    const bool over = now - t0 > limit_ns;
+    if (over) *abort_flag = 1;
+    if (__any_sync(0xffffffffu, over || *abort_flag != 0)) return false;
+  }
+  return true;
+}
+// `count` arrivals for the warp (which has met before, __syncwarp); no branch.
+__device__ __forceinline__ void mbar_arrive_warp(uint64_t* bar, uint32_t count = 1) {
+  asm volatile(
+      "{\n\t"
+      ".reg .pred one;\n\t"
+      "elect.sync _|one, 0xffffffff;\n\t"
+      "@one mbarrier.arrive.shared::cta.b64 _, [%0], %1;\n\t"
+      "}" ::"r"(smem_u32(bar)), "r"(count)
+      : "memory");
+}
+
 // ---------------------------------------------------------------------------------------------
 // TMA (tiled bulk tensor copy, global -> this CTA's shared memory, no multicast)
 // ---------------------------------------------------------------------------------------------

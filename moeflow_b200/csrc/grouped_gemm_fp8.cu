@@ -578,9 +578,8 @@ grouped_gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid
         const int nb = kTrip == 2 && j + 1 < sg.nkb ? 2 : 1;
         F8Pipe nxt = tmp;
         nxt.advance(Cfg::kTmpStages);
-        ok = mbar_wait_bounded(&tmp_full[tmp.stage], tmp.phase, abort_flag, wait_ns);
-        if (ok && nb == 2) ok = mbar_wait_bounded(&tmp_full[nxt.stage], nxt.phase, abort_flag, wait_ns);
-        ok = __all_sync(0xffffffffu, ok);
+        ok = mbar_wait_warp(&tmp_full[tmp.stage], tmp.phase, abort_flag, wait_ns);
+        if (ok && nb == 2) ok = mbar_wait_warp(&tmp_full[nxt.stage], nxt.phase, abort_flag, wait_ns);
         if (!ok) {
           if (lane == 0) report_status(a.status, kGemmAccTimeout, 3, blockIdx.x, 0);
           break;
@@ -627,10 +626,8 @@ grouped_gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid
         }
         tc_fence_before_sync();
         __syncwarp();
-        if (lane == 0) {
-          mbar_arrive(&tmp_empty[tmp.stage], share);
-          if (nb == 2) mbar_arrive(&tmp_empty[nxt.stage], share);
-        }
+        mbar_arrive_warp(&tmp_empty[tmp.stage], share);
+        if (nb == 2) mbar_arrive_warp(&tmp_empty[nxt.stage], share);
         tmp.advance(Cfg::kTmpStages);
         if (nb == 2) tmp.advance(Cfg::kTmpStages);
       }

@@ -467,9 +467,8 @@ grouped_gemm_fp8_wide_kernel(const __grid_constant__ CUtensorMap tmap_w, const _
 
       for (int j = 0; j < sg.nkb; ++j) {
         const int sub = j & 3;
-        if (sub == 0) ok = mbar_wait_bounded(&sc_full[sc.stage], sc.phase, abort_flag, wait_ns);
-        if (ok) ok = mbar_wait_bounded(&tmp_full[tmp.stage], tmp.phase, abort_flag, wait_ns);
-        ok = __all_sync(0xffffffffu, ok);
+        if (sub == 0) ok = mbar_wait_warp(&sc_full[sc.stage], sc.phase, abort_flag, wait_ns);
+        if (ok) ok = mbar_wait_warp(&tmp_full[tmp.stage], tmp.phase, abort_flag, wait_ns);
         if (!ok) {
           if (lane == 0) report_status(a.status, kGemmAccTimeout, 3, blockIdx.x, 0);
           break;
@@ -484,7 +483,7 @@ grouped_gemm_fp8_wide_kernel(const __grid_constant__ CUtensorMap tmap_w, const _
           auto release = [&]() {  // everything is in registers
             tc_fence_before_sync();
             __syncwarp();
-            if (lane == 0) mbar_arrive(&tmp_empty[tmp.stage]);
+            mbar_arrive_warp(&tmp_empty[tmp.stage]);
           };
           tmem_ld_16(d, p);
           tmem_ld_wait_16(p);
@@ -514,12 +513,12 @@ grouped_gemm_fp8_wide_kernel(const __grid_constant__ CUtensorMap tmap_w, const _
         } else {
           tc_fence_before_sync();
           __syncwarp();
-          if (lane == 0) mbar_arrive(&tmp_empty[tmp.stage]);
+          mbar_arrive_warp(&tmp_empty[tmp.stage]);
         }
         tmp.advance(kFwTmp);
         if (sub == 3 || j == sg.nkb - 1) {
           __syncwarp();
-          if (lane == 0) mbar_arrive(&sc_free[sc.stage]);
+          mbar_arrive_warp(&sc_free[sc.stage]);
           sc.advance(kFwScaleSlots);
         }
       }
