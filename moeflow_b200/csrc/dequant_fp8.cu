@@ -8,11 +8,11 @@
 // Layout: w8 [rows, K] e4m3, scale [rows / 128, K / 128] fp32 (the checkpoint's weight_scale_inv, experts
 // concatenated along the rows), out [rows, K] bf16.  value = float(e4m3) * scale, rounded once to bf16.
 #include <cuda_bf16.h>
-#include <cuda_fp8.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
 
 #include "common.cuh"
+#include "expand.cuh"
 #include "moeflow_b200.h"
 
 namespace mf {
@@ -25,23 +25,10 @@ constexpr int kDqThreads = 256;
 constexpr int kDqRows = 16;
 constexpr int kDqBatch = 8;
 
-__device__ __forceinline__ uint4 expand_8(uint2 q, float s) {
-  const uint32_t words[2] = {q.x, q.y};
-  uint32_t o[4];
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const __nv_fp8x2_storage_t pair = (__nv_fp8x2_storage_t)((words[i >> 1] >> (16 * (i & 1))) & 0xffffu);
-    const __half2_raw hr = __nv_cvt_fp8x2_to_halfraw2(pair, __NV_E4M3);
-    const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&hr));
-    const __nv_bfloat162 b = __floats2bfloat162_rn(f.x * s, f.y * s);
-    o[i] = *reinterpret_cast<const uint32_t*>(&b);
-  }
-  return make_uint4(o[0], o[1], o[2], o[3]);
-}
-
-__global__ void __launch_bounds__(kDqThreads) dequant_block_fp8_kernel(const uint8_t* w8, const float* scale, __nv_bfloat16* out, int K) {
+__global__ void __launch_bounds__(kDqThreads) dequant_block_fp8_kernel(const uint8_t* w8, const float* scale, __nv_bfloat16* out, int K, int* zero) {
   grid_dep_wait_cta();
   grid_dep_launch();
+  if (zero != nullptr && blockIdx.x == 0 && threadIdx.x == 0) *zero = 0;
   const int cpr = K / 8;                                  // steps of 8 values per row
   const int n = kDqRows * cpr;
   const size_t at = (size_t)blockIdx.x * n;               // rows are contiguous
@@ -72,13 +59,17 @@ __global__ void __launch_bounds__(kDqThreads) dequant_block_fp8_kernel(const uin
 
 // rows % 128 == 0, K % 128 == 0; pointers 16-byte aligned.  Returns 0, a negative code for bad arguments, or the
 // CUDA error of the launch.
-extern "C" int mf_dequant_block_fp8(const void* w8, const float* scale, void* out_bf16, long long rows, int K,
-                                    void* stream) {
+extern "C" int mf_dequant_block_fp8_zero(const void* w8, const float* scale, void* out_bf16, long long rows, int K, int* zero,
+                                         void* stream) {
   if (w8 == nullptr || scale == nullptr || out_bf16 == nullptr) return -1;
   if (rows <= 0 || K <= 0 || rows % 128 != 0 || K % 128 != 0) return -2;
   if ((reinterpret_cast<uintptr_t>(w8) | reinterpret_cast<uintptr_t>(out_bf16)) & 15) return -3;
   if (rows / mf::kDqRows > 0x7fffffffLL) return -2;
   return (int)mf::launch_kernel(mf::dequant_block_fp8_kernel, dim3((unsigned)(rows / mf::kDqRows)), dim3(mf::kDqThreads), 0,
                                 static_cast<cudaStream_t>(stream), true, static_cast<const uint8_t*>(w8), scale,
-                                static_cast<__nv_bfloat16*>(out_bf16), K);
+                                static_cast<__nv_bfloat16*>(out_bf16), K, zero);
+}
+
+extern "C" int mf_dequant_block_fp8(const void* w8, const float* scale, void* out_bf16, long long rows, int K, void* stream) {
+  return mf_dequant_block_fp8_zero(w8, scale, out_bf16, rows, K, nullptr, stream);
 }

@@ -45,6 +45,7 @@
 #include <cstring>
 
 #include "common.cuh"
+#include "expand.cuh"
 #include "moeflow_b200.h"
 #include "work_iter.cuh"
 
@@ -526,6 +527,16 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
       const uint64_t policy = N_MAX <= 64 ? l2_evict_first() : l2_evict_normal();
       Seg sg;
       bool have = feed.first(sg);
+      if (N_MAX >= 256 && have && a.w_wait != nullptr) {
+        // the weights are expanded by the GEMM before this one
+        const bool got = lane != 0 || wait_count_ge_gpu(a.w_wait, a.w_wait_target, wait_ns);
+        ok = __all_sync(0xffffffffu, got);
+        fence_proxy_async_all();  // the copies below, by whichever lane, come after the acquire
+        if (!ok && lane == 0) {
+          *abort_flag = 1;
+          report_status(a.status, kGemmFullTimeout, 9, blockIdx.x, 0);
+        }
+      }
       while (ok && have) {
         const int row0 = sg.e * a.rows_per_expert + block_of(sg) * (a.two_blocks ? 2 * kBlockM : kBlockM);
         for (int j = 0; j < sg.nkb; ++j) {
@@ -691,6 +702,12 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
       }
     } else if (!kFourGather) {
       gather_rows(tid - 64);
+    } else if (a.expand_src != nullptr) {
+      // ------------------------------------------------------------------ the down GEMM's weights, by two warps that have nothing to do
+      const int n = expand_pieces(a, 2 * blockIdx.x + (warp - 2), 2 * gridDim.x, lane);
+      __threadfence();  // every lane's stores are visible device-wide before the count
+      __syncwarp();
+      if (lane == 0 && n > 0) atomicAdd(a.expand_done, n);
     }
   } else if (kFourGather && warp >= 12) {
     if (kFourGather) asm volatile("setmaxnreg.dec.sync.aligned.u32 104;");
@@ -995,6 +1012,13 @@ static int launch(const void* tmap, const mf_gemm_args* args, int grid, cudaStre
 // faster form for all tiles of this height (whole layer, single / pairs: 72 experts, 85 rows expected 548 / 520, 111 rows 610 / 577
 // us, 265 rows 831 / 781; 36 experts, 882 rows 1350 / 1276, 1820 rows 2901 / 2739).
 static int launch_two_256(const void* tmap, const mf_gemm_args* args, int grid, cudaStream_t stream) {
+  if (args->expand_src != nullptr) {
+    const uintptr_t all = reinterpret_cast<uintptr_t>(args->expand_src) | reinterpret_cast<uintptr_t>(args->expand_out);
+    if (args->b_tmap != nullptr || !args->expand_scale || !args->expand_out || !args->expand_done || (all & 15) != 0 || args->expand_rows < 1 ||
+        args->expand_cols < 1 || args->expand_rows % 128 != 0 || args->expand_cols % 128 != 0 ||
+        (long long)args->expand_rows * args->expand_cols / 16 > 0x7fffffffLL - 256)
+      return -12;
+  }
   const bool boxes = args->b_tmap == nullptr || (args->b_box_rows > 0 && args->b_box_rows <= 128);  // a half of the rows per CTA
   if (args->m_blocks % 2 == 0 && grid >= 2 && boxes) return launch<true, 256, false, true>(tmap, args, grid, stream);
   return launch<true, 256>(tmap, args, grid, stream);
@@ -1007,6 +1031,7 @@ static int check_args(const mf_gemm_args* a, int n_max, int grid) {
   if ((a->b_pitch & 15) != 0 || (reinterpret_cast<uintptr_t>(a->b_base) & 15) != 0) return -4;
   if (a->b_box_rows < 0 || (a->b_box_rows > 0 && (a->b_box_rows % 16 != 0 || n_max % a->b_box_rows != 0))) return -8;
   if (a->b_tmap != nullptr && a->b_index != nullptr) return -5;  // TMA token tiles need contiguous rows
+  if (n_max != 256 && (a->expand_src != nullptr || a->w_wait != nullptr)) return -12;
   return 0;
 }
 

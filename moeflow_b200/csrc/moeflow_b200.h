@@ -101,7 +101,19 @@ typedef struct {
   int* sched;
   int b_box_rows;            // bf16 and 128-row e4m3 kernels: rows of a box of b_tmap, 0 = n_max; a divisor of n_max and a multiple of 16.
                              // The e4m3 kernels of 32- and 64-row tiles take boxes of n_max rows and do not look at it
+  // Optional (expand_src != NULL), gate/up GEMM of 256-row tiles that gathers its rows (no b_tmap): beside the GEMM its CTAs expand
+  // another block-scaled e4m3 matrix to bf16 (as mf_dequant_block_fp8; the down GEMM's weights).  expand_done, zero before, counts
+  // finished pieces of MF_EXPAND_PIECE values; the down GEMM of 256-row tiles, given the counter as w_wait, fetches no weights
+  // before it has reached w_wait_target.
+  const void* expand_src;    // [expand_rows, expand_cols] e4m3, 16-byte aligned; both multiples of 128, less than 2^31 values / 16
+  const float* expand_scale; // [expand_rows / 128, expand_cols / 128]
+  void* expand_out;          // [expand_rows, expand_cols] bf16, 16-byte aligned
+  int expand_rows, expand_cols;
+  int* expand_done;
+  const int* w_wait;
+  int w_wait_target;
 } mf_gemm_args;
+#define MF_EXPAND_PIECE 4096
 
 // Encode a 2-D tiled tensor map (K innermost) for a weight matrix [rows, k_elems]; box = 128 bytes x
 // 128 rows with the 128-byte swizzle.  `out_tmap` receives 128 bytes.

@@ -92,7 +92,7 @@ class GraphedMoELayer:
         if fp8 is not None and not fp8["in_meta"]:
             front += 1  # quantiser of the received rows
         if getattr(ly, "_expand", None) is not None:
-            front += 2
+            front += 1 if ly._expand_beside else 2
         if getattr(ly, "permute_rows", False) and fp8 is None:
             front += 1
         tail = 1 if getattr(ly, "fuse_return", False) or getattr(ly, "fuse_combine", False) else 2

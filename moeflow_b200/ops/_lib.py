@@ -84,6 +84,14 @@ class GemmArgs(C.Structure):
         ("q_scale_pitch", C.c_longlong),
         ("sched", C.c_void_p),
         ("b_box_rows", C.c_int),
+        ("expand_src", C.c_void_p),
+        ("expand_scale", C.c_void_p),
+        ("expand_out", C.c_void_p),
+        ("expand_rows", C.c_int),
+        ("expand_cols", C.c_int),
+        ("expand_done", C.c_void_p),
+        ("w_wait", C.c_void_p),
+        ("w_wait_target", C.c_int),
     ]
 
 
@@ -274,6 +282,7 @@ def lib() -> C.CDLL:
         "mf_gemm_down_fp8": [P, C.POINTER(GemmArgs), I, I, P],
         "mf_quant_rows_1x128": [P, LL, P, I, I, P, P, LL, P, P],
         "mf_dequant_block_fp8": [P, P, P, LL, I, P],
+        "mf_dequant_block_fp8_zero": [P, P, P, LL, I, P, P],
         "mf_router_topk": [P, P, P, P, I, I, I, I, I, I, I, F, P],
         "mf_rmsnorm": [P, P, P, I, I, F, P],
         "mf_add_rmsnorm": [P, P, P, P, P, I, I, F, P],

@@ -71,3 +71,31 @@ def test_k_splits_of_the_one_pass_metadata(tokens, experts):
     for word, m, k, per, over in ((1, 2, 8, 256, 4), (2, 4, 4, 128, 8)):
         want = _lib.lib().mf_plan_split(plan[0] * m, k, layer.n_sms, floats // (per * cols), over, cols)
         assert plan[word] == want
+
+
+@pytest.mark.parametrize("hidden,inter,tokens", [(512, 256, 600), (768, 128, 300), (512, 384, 90), (4096, 1536, 600)])
+def test_down_weights_expanded_beside_the_gate_up_gemm(hidden, inter, tokens):
+    """The same bits as with both expansions ahead of the GEMMs; weights that change between forwards are expanded anew."""
+    from moeflow_b200.fixed import FixedEPLayer
+    from moeflow_b200.testing import make_bias, make_logits
+    from moeflow_b200.weights import quant_block_fp8
+
+    cfg = MoEConfig(hidden_size=hidden, moe_intermediate_size=inter, n_routed_experts=4, top_k=2)
+    bias = make_bias(cfg, 1, device="cuda")
+    layers = [FixedEPLayer(cfg, 0, 1, None, None, capacity=tokens, device="cuda", backend="cuda", wait_ns=200_000_000,
+                           gemm_kwargs={"block_m": 256, "permute_rows": False, "expand_beside": beside}) for beside in (True, False)]
+    for seed in range(3):
+        def pack(w):
+            q, s = zip(*(quant_block_fp8(m) for m in w))
+            return torch.stack([t.view(torch.uint8) for t in q]).view(torch.float8_e4m3fn).cuda(), torch.stack(list(s)).cuda()
+
+        w13, w2 = make_weights(cfg, seed, dtype=torch.float32)
+        weights = (*pack(w13), *pack(w2))
+        x, lg = make_hidden(tokens, cfg, 10 + seed, device="cuda"), make_logits(tokens, cfg, 20 + seed, device="cuda")
+        outs = []
+        for layer in layers:
+            layer.set_weights_fp8(*weights)
+            FixedEPLayer._expand_scratch[(layer.device.index, layer.L, layer.I, layer.H)]["w2"].fill_(float("nan"))
+            outs.append(layer.forward(x, lg, bias)[:tokens].clone())
+            assert layer.check_status()["code"] == 0
+        assert bool(torch.isfinite(outs[0].float()).all()) and outs[0].abs().sum() > 0 and torch.equal(*outs)
