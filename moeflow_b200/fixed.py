@@ -640,10 +640,13 @@ class FixedEPLayer:
             g1.b_base, g1.b_pitch, g1.b_index = self._xg.data_ptr(), H * 2, None
             g1.b_tmap = C.addressof(self._tmap_xg)
         # Expanded e4m3 layers: the gate/up GEMM's idle warps expand the down weights, where it gathers its rows (with token boxes
-        # these warps are busy) and the down GEMM is of its kind.  Layer, expanded ahead of / beside the GEMM, us: 36 experts, 8192
-        # tokens 2651 / 2618, 5000 tokens (inter 2048) 2321 / 2273, 2304 tokens 1060 / 1059; 72 experts, 4700 tokens 2136 / 2122.
-        self._expand_beside = (self.block_m == 256 and not self.permute_rows and self.down_two_blocks and L * H * I // 16 < 2**31 - 256
-                               and bool(self.gemm_kwargs.get("expand_beside", True)))
+        # these warps are busy) and the down GEMM is of its kind.  From 768 expected rows per expert on: two warps need as long as a
+        # gate/up GEMM of about 500.  Layer, expanded ahead of / beside the GEMM, two runs, us: 36 experts, 1820 rows 2651 / 2618 and
+        # 2620 / 2589, 1111 rows (inter 2048) 2321 / 2273 and 2278 / 2249, 512 rows 1060 / 1059 and 1038 / 1045; 8 experts, 2000 rows
+        # 664 / 658 and 663 / 641; 72 experts, 522 rows 2136 / 2122 and 2097 / 2096.  (The gate/up weights as well, each expert's waited
+        # for by the copies that need it: 1820 rows 2594, 512 rows 1326.)
+        beside = bool(self.gemm_kwargs.get("expand_beside", Cc * K >= 768 * L))
+        self._expand_beside = self.block_m == 256 and not self.permute_rows and self.down_two_blocks and L * H * I // 16 < 2**31 - 256 and beside
         self._expand_done = torch.zeros(1, **i32)
         # Owner reduce + return push can run inside the down GEMM (gemm_kwargs fuse_return=True: four extra
         # warps reduce a row as soon as its last slot is written and store it into the source rank's
