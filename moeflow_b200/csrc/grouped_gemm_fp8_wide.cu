@@ -14,11 +14,13 @@
 // hand registers over to them.  Single multiply-adds, not pairs: the same rate (128 a clock).  Kernels alone, 2000 tokens on 36
 // experts, us, gate/up and down: 32 columns in pairs 309 / 173, 16 in pairs 320 / 153, 32 single 297 / 161, 16 single 297 / 156.
 // Spills explain the down GEMM only (rows by map, 28 bytes stored with 32 in pairs, none with 16 single); the gate/up GEMM
-// (gathered rows) has 4 and 60 and is the faster one with 60, for a reason that was not looked for.  Of the 297, with parts
-// left out: epilogue 37, multiply-adds 61, the rest (operands through L2, tensor-memory loads) 199.
+// (gathered rows) has 4 and 60 and is the faster one with 60, for a reason that was not looked for.  With waits and arrivals
+// that do not branch per lane (mbar_wait_warp): 291 / 157.
 // 36 experts of 3 x 4096 x 1536, whole layer, against the 64-row kernel's form on 128-row tiles, forwards on three weight sets
 // in turn, with the promotion in its first form (32 columns in pairs): 2000 tokens 917 / 581 us, 1000 tokens 524 / 353, 500 tokens
-// 317 / 222.  What bounds it now: per K block 48 KB through L2 and the promotion, which only half overlaps it.
+// 317 / 222.  What bounds it now: a promotion warp's own instructions per K block (loads, waits, multiply-adds), not the 48 KB that a
+// block brings through L2: CTA pairs, which fetch 32, took 324 / 179 for the same bits.  Also slower: sixteen promotion warps 426 /
+// 172, the columns in halves on accumulators of their own 349 / 329, the next block's loads under this one's sums 320.
 //
 // Warps: 0 weight TMA and segment hand-out, 1 UMMA, 2 token TMA (b_tmap: contiguous rows in boxes), 3 activation and weight
 // scales (four K blocks at a time, up to 16 ahead) and finished token tiles, 4-11 promotion and epilogue, 12-15 gather

@@ -1021,7 +1021,8 @@ class _CudaLayout:
 
 def choose_block_m(capacity: int, top_k: int, local_experts: int, fp8: bool = False) -> int:
     """Token rows per GEMM tile from the expected rows per expert under even routing (``R * C * K`` entries over
-    ``R * L`` experts): 64 for decode, 128 from 36 expected rows, 256 from 80.
+    ``R * L`` experts): 64 for decode, 128 from 36 expected rows, 256 from 80.  (Layers whose 256-row kernels run on CTA pairs
+    take ``paired_block_m`` where this says 128.)
 
     Measured on 72 local experts (whole layer, two weight sets in turn, us, narrower / wider tile): 28 rows 446 / 463, 43 rows
     498 / 475, 57 rows 545 / 521, 85 rows 683 / 557 (64 / 128); 85 rows 585 / 548, 114 rows 676 / 613, 171 rows 873 / 763
