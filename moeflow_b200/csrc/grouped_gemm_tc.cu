@@ -395,8 +395,6 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
     }
   }
   // ---- the plan: tile count and the K cut, checked against what the caller's buffers can hold -----------
-  FirstTile first_tile;
-  first_tile.ask(a, cta, warp == 0);
   int n_tiles = __ldcg(a.plan + MF_PLAN_N_TILES);
   const int cut = __ldcg(a.plan + a.split_word);  // 0 = stream-K, else the K split
   int slot_cols = __ldcg(a.plan + MF_PLAN_SLOT_COLS);
@@ -528,7 +526,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
       // 116 / 129, 250 on 72 e4m3 (inter 2048) 223 / 230.
       const uint64_t policy = N_MAX <= 64 ? l2_evict_first() : l2_evict_normal();
       Seg sg;
-      bool have = feed.first(sg, first_tile);
+      bool have = feed.first(sg);
       if (N_MAX >= 256 && have && a.w_wait != nullptr) {
         // the weights are expanded by the GEMM before this one
         const bool got = lane != 0 || wait_count_ge_gpu(a.w_wait, a.w_wait_target, wait_ns);

@@ -73,13 +73,6 @@ struct WorkIter {
 
   // The segment at the cursor, its tile words still in flight (nothing here waits for the three loads).
   __device__ __forceinline__ bool locate(Seg& s) {
-    if (!place(s)) return false;
-    s.e = __ldcg(a->tile_e + s.tt);
-    s.row_start = __ldcg(a->tile_s + s.tt);
-    s.n_rows = __ldcg(a->tile_n + s.tt);
-    return true;
-  }
-  __device__ __forceinline__ bool place(Seg& s) {  // ... without them
     if (stream) {
       if (w >= w1) return false;
       s.unit = (int)(w / KB);
@@ -105,6 +98,9 @@ struct WorkIter {
     }
     s.tt = s.unit / m_blocks;
     s.mb = s.unit - s.tt * m_blocks;
+    s.e = __ldcg(a->tile_e + s.tt);
+    s.row_start = __ldcg(a->tile_s + s.tt);
+    s.n_rows = __ldcg(a->tile_n + s.tt);
     return true;
   }
   // Moves the cursor of a K split (stream-K moves in locate).  The counter's answer may still be in flight on return.
@@ -176,22 +172,6 @@ struct SegReader {
       phase ^= 1u;
     }
     return s.unit >= 0;
-  }
-};
-
-// A CTA's first segment is known from its number and the K split, of which there are four: lane k of the producer warp asks for the
-// tile words of split 2^k together with the plan, one trip to L2 ahead of the first rows.  (bf16 kernels: 1 token on 288 experts
-// 67.5 / 66.7 us, others the same.  In the e4m3 kernels 100 zipf tokens on 36 experts took 89.9 / 90.7, so they do without.)
-struct FirstTile {
-  int e = 0, s = 0, n = 0;
-  bool there = false;
-  __device__ __forceinline__ void ask(const mf_gemm_args& a, int cta, bool producer) {
-    there = a.max_tiles > 0;
-    if (!producer || !there || lane_id() >= 4) return;
-    const int tt = min((cta >> lane_id()) / a.m_blocks, a.max_tiles - 1);
-    e = __ldcg(a.tile_e + tt);
-    s = __ldcg(a.tile_s + tt);
-    n = __ldcg(a.tile_n + tt);
   }
 };
 
@@ -289,19 +269,6 @@ struct SegFeedOf {
   }
   __device__ __forceinline__ bool first(Seg& s) {
     have = it.locate(nx);
-    stage = 2;
-    return next(s);
-  }
-  __device__ __forceinline__ bool first(Seg& s, const FirstTile& t) {
-    if (t.there && !it.stream) {
-      const int k = 31 - __clz(it.split);
-      have = it.place(nx);
-      nx.e = __shfl_sync(0xffffffffu, t.e, k);
-      nx.row_start = __shfl_sync(0xffffffffu, t.s, k);
-      nx.n_rows = __shfl_sync(0xffffffffu, t.n, k);
-    } else {
-      have = it.locate(nx);
-    }
     stage = 2;
     return next(s);
   }
