@@ -527,6 +527,13 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
       const uint64_t policy = N_MAX <= 64 ? l2_evict_first() : l2_evict_normal();
       Seg sg;
       bool have = feed.first(sg);
+      if (N_MAX >= 256 && !have && a.w_wait != nullptr && blockIdx.x == 0) {
+        // A grid without segments (a rank that received no rows, a refused plan) waits for no token tile and no counter, but the
+        // GEMM before it expands all the same: what follows may set the counter back and write to the weights' scratch, and has
+        // an edge from this grid's end only.
+        if (lane == 0) grid_dep_wait();
+        __syncwarp();
+      }
       if (N_MAX >= 256 && have && a.w_wait != nullptr) {
         // the weights are expanded by the GEMM before this one
         const bool got = lane != 0 || wait_count_ge_gpu(a.w_wait, a.w_wait_target, wait_ns);

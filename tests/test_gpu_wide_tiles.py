@@ -99,3 +99,49 @@ def test_down_weights_expanded_beside_the_gate_up_gemm(hidden, inter, tokens):
             outs.append(layer.forward(x, lg, bias)[:tokens].clone())
             assert layer.check_status()["code"] == 0
         assert bool(torch.isfinite(outs[0].float()).all()) and outs[0].abs().sum() > 0 and torch.equal(*outs)
+
+
+def test_an_empty_forward_ends_behind_the_expansion_beside_it():
+    """No token tile: the down GEMM waits for no tile and no weights, but the call is over only when its gate/up GEMM has expanded
+    everything, since the next layer on these buffers sets the counter back and writes to the same scratch."""
+    from moeflow_b200.fixed import FixedEPLayer
+    from moeflow_b200.testing import make_bias, make_logits
+
+    cfg = MoEConfig(hidden_size=4096, moe_intermediate_size=1536, n_routed_experts=8, top_k=2)
+    layer = FixedEPLayer(cfg, 0, 1, None, None, capacity=300, device="cuda", backend="cuda", wait_ns=200_000_000,
+                         gemm_kwargs={"block_m": 256, "permute_rows": False, "expand_beside": True})
+
+    def pack(seed):
+        g = torch.Generator(device="cuda").manual_seed(seed)
+        q = [(torch.randn(*s, generator=g, device="cuda")).to(torch.float8_e4m3fn) for s in ((8, 3072, 4096), (8, 4096, 1536))]
+        s = [torch.rand(*s, generator=g, device="cuda") * 0.02 + 0.001 for s in ((8, 24, 32), (8, 32, 12))]
+        return layer.make_fp8_pack(q[0], s[0], q[1], s[1])
+
+    packs = [pack(seed) for seed in (1, 2, 3)]
+    x, lg, bias = make_hidden(300, cfg, 4, device="cuda"), make_logits(300, cfg, 5, device="cuda"), make_bias(cfg, 6, device="cuda")
+    none, done, outs = torch.zeros((), dtype=torch.int32, device="cuda"), [], []
+
+    def calls():
+        done.clear(), outs.clear()
+        for i, p in enumerate(packs):
+            layer.bind_weights_fp8(p)
+            empty = layer.forward(x, lg, bias, none)
+            done.append(layer._expand_done.clone())
+            outs.append(empty.clone())
+            layer.bind_weights_fp8(packs[(i + 1) % 3])
+            outs.append(layer.forward(x, lg, bias).clone())
+
+    calls()
+    want = [o.clone() for o in outs]
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        calls()
+    for _ in range(5):
+        graph.replay()
+        torch.cuda.synchronize()
+        assert [int(d) for d in done] == [packs[0]["w2"].numel() // 4096] * 3
+        for got, right in zip(outs, want):
+            assert torch.equal(got, right)
+        assert not outs[0].any() and bool(outs[1].any())
+    assert layer.check_status()["code"] == 0
