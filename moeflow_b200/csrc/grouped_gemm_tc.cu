@@ -538,6 +538,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
         // the weights are expanded by the GEMM before this one
         const bool got = lane != 0 || wait_count_ge_gpu(a.w_wait, a.w_wait_target, wait_ns);
         ok = __all_sync(0xffffffffu, got);
+        __syncwarp();             // lane 0's acquire comes before what the other lanes do (the vote orders no memory)
         fence_proxy_async_all();  // the copies below, by whichever lane, come after the acquire
         if (!ok && lane == 0) {
           *abort_flag = 1;
