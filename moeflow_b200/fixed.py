@@ -480,14 +480,19 @@ class FixedEPLayer:
         # A buffer set built without weights may be bound to e4m3 experts later: plan its tiles for them unless told
         # otherwise (gemm_kwargs fp8_weights=False / True).
         fp8_hint = bool(self.gemm_kwargs.get("fp8_weights", self.w13 is None))
-        tall = choose_block_m(Cc, K, L, fp8=fp8_hint)
+        tall = fp8_tall = choose_block_m(Cc, K, L, fp8=fp8_hint)
         if tall == 128 and not fp8_hint and H % 512 == 0 and I % 256 == 0 and not {"stream_k", "fuse_return", "down_two_blocks"} & set(self.gemm_kwargs):
             tall = paired_block_m(Cc, K, L)
-        self.block_m = int(self.gemm_kwargs.get("block_m", tall))
-        if self.block_m not in (32, 64, 128, 256):
+        if "block_m" in self.gemm_kwargs:
+            tall = fp8_tall = int(self.gemm_kwargs["block_m"])
+        if tall not in (32, 64, 128, 256):
             raise ValueError("block_m must be 32, 64, 128 or 256")
+        # `paired_block_m` is a rule of the bf16 kernels: with e4m3 weights bound, such a layer's tiles have the 128 rows that it
+        # would have without the rule.  Its buffers hold the plans of both heights; block_m is the one of the weights bound now.
+        self.block_m, self._bf16_block_m, self._fp8_block_m = tall, tall, fp8_tall
+        low, high = min(tall, fp8_tall), max(tall, fp8_tall)
         self.n_sms = int(self.gemm_kwargs.get("n_sms", sm_count(dev.index if dev.index is not None else 0)))
-        self.max_tiles = N // self.block_m + min(L, N)  # every tile holds an entry, and full ones hold block_m
+        self.max_tiles = N // low + min(L, N)  # every tile holds an entry, and full ones hold block_m
         self.out = torch.zeros(Cc, H, dtype=torch.bfloat16, device=dev)
         self.hit = torch.zeros(Cc, R, dtype=torch.uint8, device=dev)
         self._route_w = torch.zeros(Cc, K, dtype=torch.float32, device=dev)
@@ -505,7 +510,7 @@ class FixedEPLayer:
         self.tile_s = torch.zeros(self.max_tiles, **i32)
         self.tile_n = torch.zeros(self.max_tiles, **i32)
         self.plan = torch.zeros(_lib.PLAN_WORDS, **i32)
-        self.act = torch.zeros(max(N, self.block_m), I, dtype=torch.bfloat16, device=dev)  # >= one TMA box of rows
+        self.act = torch.zeros(max(N, high), I, dtype=torch.bfloat16, device=dev)  # >= one TMA box of rows
         self.y = torch.zeros(N, H, dtype=torch.bfloat16, device=dev)
         mb1, mb2 = I // 128, H // 128
         # arrival counters of cut units: one per (unit, 32-row quarter) and, in the fp8 kernels with 128-column
@@ -519,7 +524,7 @@ class FixedEPLayer:
         # split-K scratch: a byte budget; the metadata kernel sizes the partial slots for the widest token tile
         # (each GEMM gets its own half: the down GEMM may run while gate/up units are still being fixed up)
         partial_floats = int(self.gemm_kwargs.get("split_scratch_mb", 64)) * (1 << 20) // 4 // 2
-        self.max_split_slots = partial_floats // (2 * self.block_m * 128)
+        self.max_split_slots = self._split_slots(partial_floats)
         self._partial = torch.zeros(2 * partial_floats, dtype=torch.float32, device=dev)
         self._keep: list = []  # ctypes objects and temporaries that must outlive launches
 
@@ -646,7 +651,7 @@ class FixedEPLayer:
         # 664 / 658 and 663 / 641; 72 experts, 522 rows 2136 / 2122 and 2097 / 2096.  (The gate/up weights as well, each expert's waited
         # for by the copies that need it: 1820 rows 2594, 512 rows 1326.)
         beside = bool(self.gemm_kwargs.get("expand_beside", Cc * K >= 768 * L))
-        self._expand_beside = self.block_m == 256 and not self.permute_rows and self.down_two_blocks and L * H * I // 16 < 2**31 - 256 and beside
+        self._expand_beside = self._fp8_block_m == 256 and not self.permute_rows and self.down_two_blocks and L * H * I // 16 < 2**31 - 256 and beside
         self._expand_done = torch.zeros(1, **i32)
         # Owner reduce + return push can run inside the down GEMM (gemm_kwargs fuse_return=True: four extra
         # warps reduce a row as soon as its last slot is written and store it into the source rank's
@@ -742,7 +747,7 @@ class FixedEPLayer:
             raise ValueError("fp8 path supports K <= 4096")
         pack = {"w13": w13_q.contiguous(), "w2": w2_q.contiguous(), "s13": w13_s.to(torch.float32).contiguous(),
                 "s2": w2_s.to(torch.float32).contiguous()}
-        if self.block_m > 128:
+        if self._fp8_block_m > 128:
             # Long-prefill layers (256-row token tiles): the block-scaled kernels take tiles of up to 128 rows, so every
             # forward expands the bound experts into a bf16 scratch (shared by all layers of this shape on the device) and
             # runs the bf16 kernels on it; the activations are not quantised.
@@ -785,11 +790,11 @@ class FixedEPLayer:
         f = {}
         f["xq"] = torch.zeros(rows, H, dtype=torch.uint8, device=dev)
         f["xs"] = torch.zeros(rows, H // 128, dtype=torch.float32, device=dev)
-        f["aq"] = torch.zeros(max(N, self.block_m), I, dtype=torch.uint8, device=dev)  # >= one TMA box of rows
-        f["as"] = torch.zeros(max(N, self.block_m), I // 128, dtype=torch.float32, device=dev)
+        f["aq"] = torch.zeros(max(N, self._fp8_block_m), I, dtype=torch.uint8, device=dev)  # >= one TMA box of rows
+        f["as"] = torch.zeros(max(N, self._fp8_block_m), I // 128, dtype=torch.float32, device=dev)
         g1, g2 = self._a_gemm1, self._a_gemm2
         common = dict(tile_e=g1.tile_e, tile_s=g1.tile_s, tile_n=g1.tile_n, plan=g1.plan, partial=g1.partial,
-                      max_split_slots=g1.max_split_slots, limit=g1.limit, round_h=0, status=g1.status, wait_ns=g1.wait_ns,
+                      max_split_slots=self.max_split_slots, limit=g1.limit, round_h=0, status=g1.status, wait_ns=g1.wait_ns,
                       partial_floats=g1.partial_floats, max_tiles=g1.max_tiles)
         f["a1"] = _lib.GemmArgs(b_base=f["xq"].data_ptr(), b_pitch=H, b_index=self.entry_row.data_ptr(),
                                 split_word=_lib.PLAN_SPLIT1, m_blocks=I // 128, k_blocks=H // 128, rows_per_expert=2 * I,
@@ -808,14 +813,14 @@ class FixedEPLayer:
         if bool(self.gemm_kwargs.get("b_tma", True)):
             from .ops.kernels import make_tile_tmap
 
-            box = min(self.block_m, 64)  # as in the bf16 layers
+            box = min(self._fp8_block_m, 64)  # as in the bf16 layers
             f["tm_aq"] = make_tile_tmap(f["aq"], box)  # the down GEMM reads its e4m3 token tiles by TMA
             f["a2"].b_tmap, f["a2"].b_box_rows = C.addressof(f["tm_aq"]), box
         a1.sched, f["a2"].sched = g1.sched, g2.sched
         if self.tile_handover:  # one count per promotion warp of the gate/up kernel and weight block
             a1.tile_done = self._tile_done.data_ptr()
             f["a2"].tile_wait = self._tile_done.data_ptr()
-            f["a2"].tile_wait_target = (4 if self.block_m <= 32 else 8) * (I // 128)
+            f["a2"].tile_wait_target = (4 if self._fp8_block_m <= 32 else 8) * (I // 128)
         # up to 8192 slot words the metadata launch quantises the received rows as well
         f["in_meta"] = self.meta_ctas == 1 and rows * self.K <= 8192
         self._fp8_shared = f
@@ -836,6 +841,7 @@ class FixedEPLayer:
             self.w13, self.w2, self._tmap13, self._tmap2 = e["w13"], e["w2"], e["tm13"], e["tm2"]
             return
         self._expand = None
+        self._set_block_m(self._fp8_block_m)
         f = self._fp8_buffers()
         f["a1"].w_scale, f["a2"].w_scale = pack["s13"].data_ptr(), pack["s2"].data_ptr()
         f["tm13"], f["tm2"], f["pack"] = pack["tm13"], pack["tm2"], pack
@@ -868,7 +874,17 @@ class FixedEPLayer:
         self._bind_bf16()
         self.w13, self.w2, self._tmap13, self._tmap2 = w13_local, w2_local, tmap13, tmap2
 
+    def _split_slots(self, partial_floats: int) -> int:
+        """Partial tiles of the present height that one GEMM's half of the split-K scratch holds."""
+        return partial_floats // (2 * self.block_m * 128)
+
+    def _set_block_m(self, block_m: int) -> None:
+        """Token rows per tile of the forwards from now on."""
+        self.block_m = self._a_meta.block_m = block_m
+        self.max_split_slots = self._a_meta.max_split_slots = self._split_slots(self._a_meta.partial_floats)
+
     def _bind_bf16(self) -> None:
+        self._set_block_m(self._bf16_block_m)
         self._fp8 = self._expand = None
         self._a_gemm1.expand_src = self._a_gemm2.w_wait = None
         self._a_meta.xq = self._a_meta.xs = None
