@@ -482,7 +482,7 @@ class FixedEPLayer:
         fp8_hint = bool(self.gemm_kwargs.get("fp8_weights", self.w13 is None))
         tall = fp8_tall = choose_block_m(Cc, K, L, fp8=fp8_hint)
         if tall == 128 and not fp8_hint and H % 512 == 0 and I % 256 == 0 and not {"stream_k", "fuse_return", "down_two_blocks"} & set(self.gemm_kwargs):
-            tall = paired_block_m(Cc, K, L)
+            tall = paired_block_m(Cc, K, L, H, I)
         if "block_m" in self.gemm_kwargs:
             tall = fp8_tall = int(self.gemm_kwargs["block_m"])
         if tall not in (32, 64, 128, 256):
@@ -1037,7 +1037,7 @@ class _CudaLayout:
 
 def choose_block_m(capacity: int, top_k: int, local_experts: int, fp8: bool = False) -> int:
     """Token rows per GEMM tile from the expected rows per expert under even routing (``R * C * K`` entries over
-    ``R * L`` experts): 64 for decode, 128 from 36 expected rows, 256 from 80.  (Layers whose 256-row kernels run on CTA pairs
+    ``R * L`` experts): 64 for decode, 128 from 36 expected rows, 256 from 80.  (bf16 layers whose 256-row kernels run on CTA pairs
     take ``paired_block_m`` where this says 128.)
 
     Measured on 72 local experts (whole layer, two weight sets in turn, us, narrower / wider tile): 28 rows 446 / 463, 43 rows
@@ -1060,15 +1060,35 @@ def choose_block_m(capacity: int, top_k: int, local_experts: int, fp8: bool = Fa
     return 256 if expected >= 80 else 128 if expected >= 36 else 64
 
 
-def paired_block_m(capacity: int, top_k: int, local_experts: int) -> int:
+def paired_block_m(capacity: int, top_k: int, local_experts: int, hidden: int = 4096, inter: int = 1536) -> int:
     """What a bf16 layer takes in place of 128-row tiles where the 256-row kernels run on CTA pairs (hidden a multiple of 512,
-    intermediate of 256): 256 rows, a pair sharing the tile's rows, or 64 for few experts, which leave CTAs idle on units twice as
-    large.  Whole layer, two weight sets in turn, us, 64 / 128 / 256 rows: 36 experts, 44 rows expected 250 / 262 / 256, 50 rows of zipf
-    popularity 190 / - / 158, 62 rows - / 281 / 268; 72 experts, 36 rows 483 / 489 / 478, 43 rows 503 / 496 / 486 (zipf 296 / 262 / 209),
-    71 rows - / 554 / 506; 144 experts, 38 rows 962 / 935 / 920; 288 experts, 41 rows 1984 / 1889 / 1770; 8 experts, 40 rows 74 / 95 / 86,
-    60 rows 76 / - / 88, 75 rows 101 / - / 91; 16 experts, 60 rows 122 / - / 144, 70 rows - / 149 / 140; 24 experts, 50 rows 173 / - / 184.
+    intermediate of 256).  A pair shares the tile's rows, so its units are twice as large, and what that costs depends on how many
+    there are.  Whole layer, two weight sets in turn, graph, us, 64 / 128 / 256 rows:
+
+    64 rows for fewer than 32 experts and 64 rows per expert; never above 128 rows by more than 5 %: 4096 x 1536, 8 experts, 40 rows
+    72 / 87 / 83, 16 experts 120 / 129 / 129; 2048 x 1536, 8 experts 48 / 58 / 67; 512 x 1024 40 / 42 / 47; 512 x 256 26 / 29 / 27; 5120 x
+    1536, 11 experts 102 / 111 / 118; 4096 x 1280, 29 experts, zipf popularity 149 / 142 / 141; 7168 x 1280, 30 experts 291 / 291 / 292.
+
+    256 rows from 2e8 weights of one projection on (1.2 GB of experts): many rounds of units, uneven ends cost little, and the pairs'
+    smaller traffic counts; 1 % slower at worst: 4096 x 1536, 36 experts, 40 rows 238 / 250 / 252, 60 rows 281 / 266 / 265, 75 rows 310 / 279 /
+    275, 50 rows of zipf popularity 206 / 205 / 195; 72 experts, 40 rows 475 / 470 / 474, 75 rows 619 / 549 / 506, zipf 353 / 312 / 227; 128
+    experts, 75 rows 1061 / 980 / 858; 2048 x 768, 128 experts, 38 rows 235 / 234 / 238, 75 rows 296 / 282 / 262; 3072 x 1024, 72 experts
+    287 / 277 / 281; 512 x 2048, 192 experts 250 / 264 / 251; 7168 x 2048, 36 experts, 40 rows 523 / 528 / 524, 75 rows 719 / 626 / 570.
+
+    256 rows, too, where all units are under way at once, up to 48 pairs in the gate/up GEMM and at least as many in the down GEMM: 512 x
+    256, 36 experts, 40 rows 36 / 39 / 33, 75 rows 44 / 48 / 44 (zipf 35 / 39 / 42); 1024 x 512, 16 experts, 75 rows 41 / 44 / 41; 4096 x 1536,
+    8 experts, 75 rows 97 / 90 / 86.  With fewer units in the down GEMM its CTAs stand idle: 512 x 1024, 16 experts 42 / 40 / 52;
+    2048 x 1536, 8 experts 57 / 62 / 72.
+
+    128 rows between: one to three rounds of units, the last one of twice the length: 1024 x 512, 48 experts, 75 rows 69 / 78 / 82; 512 x 1024,
+    32 experts 55 / 62 / 65, 55 experts, zipf 55 / 59 / 72; 2048 x 768, 48 experts, 40 rows 97 / 106 / 110; 4096 x 512, 32 experts, 60 rows
+    112 / 105 / 110.  (64 rows would be faster on many of these layers, and 256 on some of skewed popularity.)
     """
-    return 64 if local_experts < 32 and capacity * top_k < 64 * max(local_experts, 1) else 256
+    if local_experts < 32 and capacity * top_k < 64 * max(local_experts, 1):
+        return 64
+    if local_experts * hidden * inter >= 200_000_000:
+        return 256
+    return 256 if local_experts <= 36 and local_experts * inter <= 48 * 256 and hidden >= 2 * inter else 128
 
 
 def choose_meta_ctas(slot_words: int, n_sms: int) -> int:

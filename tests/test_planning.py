@@ -94,3 +94,17 @@ def test_paired_tiles_in_place_of_128_rows():
     assert paired_block_m(40, 8, 8) == 64      # 40 rows on 8 experts: fewer pair units than pairs
     assert paired_block_m(64, 8, 8) == 256     # 64 rows
     assert paired_block_m(1, 8, 0) == 64
+
+
+def test_paired_tiles_by_the_layer_s_size():
+    from moeflow_b200.fixed import paired_block_m
+
+    assert paired_block_m(200, 8, 36, 512, 256) == 256 and paired_block_m(72, 8, 8, 512, 256) == 256  # all units under way at once
+    assert paired_block_m(150, 8, 16, 512, 1024) == 128   # a down GEMM of few units
+    assert paired_block_m(75, 8, 8, 2048, 1536) == 128
+    assert paired_block_m(450, 8, 48, 1024, 512) == 128   # one to three rounds of units
+    assert paired_block_m(300, 8, 32, 512, 1024) == 128
+    assert paired_block_m(180, 8, 32, 4096, 512) == 128
+    assert paired_block_m(40, 8, 8, 512, 1024) == 64
+    assert paired_block_m(240, 8, 32, 4096, 1536) == 256  # 2e8 weights per projection
+    assert paired_block_m(540, 8, 72, 7168, 2048) == 256
