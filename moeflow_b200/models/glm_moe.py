@@ -165,8 +165,10 @@ class MoEBlock:
         # only in a graph, where a branch costs the host nothing per step
         capturing = fused and self.branch is not None and self.routed.backend == "cuda" and torch.cuda.is_current_stream_capturing()
         begun = self.branch if capturing else None
-        # one rank: the whole shared expert runs on the branch, and the routed experts' last kernel adds the three up
-        added = begun is not None and self.routed.adds_to_output and x.is_contiguous() and x.data_ptr() % 16 == 0
+        # one rank: the whole shared expert runs on the branch, and the routed experts' last kernel adds the three up, in rows of 16-byte
+        # chunks; any other `out` is left to the shared expert's down projection
+        wide = lambda t: t.shape == h.shape and t.dtype == h.dtype and t.device == h.device and t.is_contiguous() and t.data_ptr() % 16 == 0
+        added = begun is not None and self.routed.adds_to_output and wide(x) and (out is None or wide(out))
         if begun is not None:
             beside = self.shared.begin(h, begun, whole=added)
         if logits is not None:
