@@ -49,12 +49,21 @@ def _rmsnorm(x: torch.Tensor, gamma: torch.Tensor, eps: float) -> torch.Tensor:
     return (xf * torch.rsqrt(xf.pow(2).mean(-1, keepdim=True) + eps) * gamma.to(torch.float32)).to(x.dtype)
 
 
-#: Up to this many router logits per step (sequences x experts) come from the kernel that normalises the rows; it reads the gate matrix
-#: once per sequence, the dense kernel once per 64.  Normalisation and logits in a row of such pairs, cold gates, us, two launches / one:
-#: 36 experts, 1 sequence 6.5 / 4.2, 32 7.8 / 5.2, 64 8.7 / 9.2; 72 experts, 16 7.1 / 4.9, 32 7.8 / 7.9, 64 8.8 / 10.1; 288 experts, 4
-#: 7.3 / 6.1, 16 7.6 / 10.2.  Inside a decode step the second launch costs more: 64 sequences on 36 experts 226.2 / 222.4, on 72
-#: 294.1 / 301.3, 45 on 72 461.6 / 464.9.
+#: Up to this many router logits per step (sequences x experts) of rows of up to 4096 values come from the kernel that normalises the
+#: rows, and of longer rows accordingly fewer: it reads the gate matrix once per sequence, the dense kernel once per 64.  Normalisation and
+#: logits in a row of such pairs, cold gates, us, two launches / one: 36 experts, 1 sequence 6.5 / 4.2, 32 7.8 / 5.2, 64 8.7 / 9.2; 72
+#: experts, 16 7.1 / 4.9, 32 7.8 / 7.9, 64 8.8 / 10.1; 288 experts, 4 7.3 / 6.1, 16 7.6 / 10.2.  Inside a decode step the second launch
+#: costs more.  One layer of hidden 4096, 36 experts of 1536, e4m3: 4 sequences 150.3 / 144.6, 16 178.9 / 170.8, 40 208.8 / 203.9, 64 229.0 /
+#: 222.5; bf16: 2 158.8 / 151.1, 64 319.2 / 312.3; 72 experts: 8 e4m3 204.2 / 197.0, 40 bf16 488.4 / 481.5, 64 508.1 / 507.6; but 1 sequence
+#: 117.0 / 118.3, and 288 experts of 512, 16 sequences 234 to 240 / 241 to 246.  At hidden 8192, 36 experts of 1536: 24 sequences 489.8 / 488.4, 64
+#: 509.2 / 513.5 (two layers' mean).
 NORM_LOGITS = 2304
+#: Below this hidden size a block with a shared expert keeps the two launches: its first half starts behind the normalisation, and the
+#: dense kernel then runs beside it.  Hidden 2048, two layers' mean, two launches / one: intermediate 1536, 36 experts, 8 sequences 144.5 /
+#: 147.1, 24 162.4 / 164.3, 40 174.5 / 177.6, 64 179.4 / 181.5; 1024, 72 experts, 32 183.3 / 189.4, 36 experts, 24 130.3 / 133.0; 512, 72
+#: experts, 32 129.5 / 131.7 (8 sequences on 36 88.4 / 86.2); hidden 1024 within noise.  Without a shared expert (hidden 4096) one launch is
+#: faster at all of these sizes: intermediate 512, 36 experts, 64 sequences 159.7 / 154.2; 1536, 72 experts, 32 428.1 / 421.3.
+NORM_LOGITS_SHARED_HIDDEN = 4096
 
 
 class SharedExpert:
@@ -124,9 +133,11 @@ class RouterLogits:
     def __call__(self, h: torch.Tensor) -> torch.Tensor:
         return self._project(h, self.logits)
 
-    def fits_norm(self, rows: int) -> bool:
-        """Is ``after_norm`` the faster form?"""
-        return self.H <= 16384 and 0 < rows <= self.C and rows * self.E <= NORM_LOGITS
+    def fits_norm(self, rows: int, shared: bool = False) -> bool:
+        """Is ``after_norm`` the faster form?  ``shared``: in a block with a shared expert."""
+        if not 0 < rows <= self.C or self.H > 16384 or (shared and self.H < NORM_LOGITS_SHARED_HIDDEN):
+            return False
+        return rows * self.E * max(self.H, 4096) <= NORM_LOGITS * 4096
 
     def after_norm(self, x: torch.Tensor, add: torch.Tensor, gamma: torch.Tensor, eps: float) -> tuple[torch.Tensor, torch.Tensor, torch.Tensor]:
         """``(x + add, h = rmsnorm(x + add), router logits of h)`` in one launch."""
@@ -154,7 +165,7 @@ class MoEBlock:
         if add is not None and x.is_cuda and x.dtype == torch.bfloat16:
             from ..ops.kernels import add_rmsnorm
 
-            if self.router is not None and x.dim() == 2 and self.router.fits_norm(x.shape[0]):
+            if self.router is not None and x.dim() == 2 and self.router.fits_norm(x.shape[0], self.shared is not None):
                 x, h, logits = self.router.after_norm(x, add, self.norm_w, self.eps)
             else:
                 x, h = add_rmsnorm(x, add, self.norm_w, self.eps)

@@ -108,3 +108,19 @@ def test_paired_tiles_by_the_layer_s_size():
     assert paired_block_m(40, 8, 8, 512, 1024) == 64
     assert paired_block_m(240, 8, 32, 4096, 1536) == 256  # 2e8 weights per projection
     assert paired_block_m(540, 8, 72, 7168, 2048) == 256
+
+
+def test_where_the_router_s_logits_come_with_the_normalisation():
+    from moeflow_b200.models.glm_moe import RouterLogits
+
+    def fits(hidden, experts, rows, shared, capacity=1 << 20):
+        router = object.__new__(RouterLogits)
+        router.H, router.E, router.C = hidden, experts, capacity
+        return router.fits_norm(rows, shared)
+
+    for shared in (False, True):
+        assert fits(4096, 36, 64, shared) and not fits(4096, 36, 65, shared) and not fits(4096, 72, 33, shared)
+        assert fits(8192, 36, 32, shared) and not fits(8192, 36, 33, shared) and fits(16384, 36, 16, shared)
+        assert not fits(16448, 1, 1, shared) and not fits(4096, 36, 0, shared) and not fits(4096, 36, 9, shared, capacity=8)
+    # shorter rows: the limit of hidden 4096, and two launches next to a shared expert
+    assert fits(512, 36, 64, False) and not fits(512, 36, 65, False) and not fits(4032, 1, 1, True)
