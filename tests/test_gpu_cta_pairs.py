@@ -89,3 +89,83 @@ def test_layers_of_36_to_80_rows(experts, tokens, inter, block_m):
         outs.append(layer.forward(x, lg, bias)[:tokens].double())
         assert layer.check_status()["code"] == 0 and layer.block_m == kw.get("block_m", block_m) and not layer.permute_rows
     assert (outs[0] - outs[1]).norm() < 2 * 2.0**-8 * outs[1].norm()
+
+
+def test_units_of_pairs_cut_in_eight():
+    """The largest K split, segments of two K blocks: both GEMMs, against one CTA."""
+    from moeflow_b200.ops.grouped_gemm import down_proj, gate_up_swiglu, plan_from_offsets
+
+    offsets = [0, 31, 287, 288]
+    g = torch.Generator().manual_seed(8)
+    w = (torch.randn(3, 1024, 1024, generator=g) / 16).bfloat16().cuda()
+    x = torch.randn(offsets[-1], 1024, generator=g).bfloat16().cuda()
+    scale = torch.rand(offsets[-1], generator=g).cuda() + 0.5
+    for call in (lambda tp, **kw: gate_up_swiglu(x, w, tp, **kw),
+                 lambda tp, **kw: down_proj(x, w, tp, row_scale=scale, b_tma=False, two_blocks=True, **kw)):
+        got = []
+        for grid in (1, 2, 148):
+            status = torch.zeros(1, dtype=torch.int64, device="cuda")
+            got.append(call(plan_from_offsets(offsets, 256, x.device), split=8, status=status, wait_ns=200_000_000, grid=grid).clone())
+            assert int(status.item()) == 0
+        assert got[0].abs().sum() > 0 and all(torch.equal(o, got[0]) for o in got[1:])
+
+
+@pytest.mark.parametrize("hidden,inter", [(4096, 256), (4096, 1536), (512, 2048)])
+def test_long_k_loops_on_pairs_equal_single_ctas_bitwise(hidden, inter):
+    counts = (256, 131, 0, 17)
+    cfg = MoEConfig(hidden_size=hidden, moe_intermediate_size=inter, n_routed_experts=4, top_k=1)
+    w13, w2 = make_weights(cfg, 0, device="cuda")
+    t = sum(counts)
+    x = make_hidden(t, cfg, 1, device="cuda")
+    g = torch.Generator().manual_seed(2)
+    ids = torch.repeat_interleave(torch.arange(4), torch.tensor(counts))[torch.randperm(t, generator=g)].int()[:, None].cuda()
+    weights = torch.rand(t, 1, generator=g).cuda() + 0.5
+    outs = []
+    for n_sms in (1, 7, None):
+        layer = _layer(cfg, w13, w2, t, n_sms, permute_rows=False)
+        outs.append(layer.forward_routed(x, weights, ids).clone())
+        assert layer.check_status()["code"] == 0
+    assert outs[0].abs().sum() > 0 and all(torch.equal(o, outs[0]) for o in outs[1:])
+
+
+@pytest.mark.parametrize("block_m", [32, 64, 128, 256])
+@pytest.mark.parametrize("two_blocks", [False, True])
+def test_infinities_and_nan_stay_where_they_belong(block_m, two_blocks):
+    """Through the epilogue's transposition: a token's row and a weight row's column, nothing else."""
+    from moeflow_b200.ops.grouped_gemm import down_proj, gate_up_swiglu, plan_from_offsets
+
+    offsets, inter, hidden = [0, 40, 40, 300], 128, 512
+    g = torch.Generator().manual_seed(block_m)
+    act = torch.randn(offsets[-1], inter, generator=g).bfloat16().cuda()
+    w2 = torch.randn(3, hidden, inter, generator=g).bfloat16().cuda()
+    tp = plan_from_offsets(offsets, block_m, act.device)
+    clean = down_proj(act, w2, tp, two_blocks=two_blocks, b_tma=False).clone()
+    bad_rows = {3: float("inf"), 39: float("nan"), 40: float("-inf"), 201: float("inf"), 299: float("nan")}
+    bad_cols = {0: (5, float("inf")), 2: (hidden - 3, float("nan"))}  # expert: (weight row, value)
+    act_bad, w_bad = act.clone(), w2.clone()
+    for row, value in bad_rows.items():
+        act_bad[row, row % inter] = value
+    for e, (row, value) in bad_cols.items():
+        w_bad[e, row, 7] = value
+    y = down_proj(act_bad, w_bad, tp, two_blocks=two_blocks, b_tma=False)
+    want, hit = clean.float(), torch.zeros_like(clean, dtype=torch.bool)
+    for e, (lo, hi) in enumerate(zip(offsets, offsets[1:])):
+        for row in [r for r in bad_rows if lo <= r < hi]:
+            hit[row] = True
+            want[row] = (act_bad[row].float() * w_bad[e].float()).sum(1)  # one value that is not finite decides every sum
+        if e in bad_cols and hi > lo:
+            col = bad_cols[e][0]
+            hit[lo:hi, col] = True
+            want[lo:hi, col] = (act_bad[lo:hi].float() * w_bad[e, col].float()).sum(1)
+    assert torch.equal(y[~hit], clean[~hit])
+    assert torch.equal(torch.isnan(y[hit]), torch.isnan(want[hit])) and not torch.isfinite(want[hit]).any()
+    inf = torch.isinf(want[hit])
+    assert torch.equal(y[hit][inf].float(), want[hit][inf])
+    # gate/up: the other rows keep their bits (what a row with such values becomes is up to the clamp)
+    w13 = torch.randn(3, 2 * inter, hidden, generator=g).bfloat16().cuda()
+    x = torch.randn(offsets[-1], hidden, generator=g).bfloat16().cuda()
+    plain = gate_up_swiglu(x, w13, tp).clone()
+    for row, value in bad_rows.items():
+        x[row, row] = value
+    rows = [r for r in range(offsets[-1]) if r not in bad_rows]
+    assert torch.equal(gate_up_swiglu(x, w13, tp)[rows], plain[rows])

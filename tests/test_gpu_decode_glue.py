@@ -100,3 +100,20 @@ def test_add_rmsnorm_logits_refuses_what_does_not_fit():
                 lambda: add_rmsnorm_logits(x, x, gamma, gate.float(), 8, logits), lambda: add_rmsnorm_logits(x, x, gamma, gate, 8, logits.double())):
         with pytest.raises(ValueError):
             bad()
+
+
+def test_add_rmsnorm_logits_of_rows_that_are_not_finite():
+    """They stay in their own row, and a gate row's in its own column."""
+    from moeflow_b200.ops.kernels import add_rmsnorm, add_rmsnorm_logits
+
+    g = torch.Generator().manual_seed(1)
+    x, add = (torch.randn(9, 1024, generator=g).bfloat16().cuda() for _ in range(2))
+    gamma, gate = torch.rand(1024, generator=g).bfloat16().cuda() + 0.5, torch.randn(36, 1024, generator=g).bfloat16().cuda()
+    clean, logits = torch.empty(9, 36, device="cuda"), torch.empty(9, 36, device="cuda")
+    add_rmsnorm_logits(x, add, gamma, gate, 36, clean)
+    x[2, 5], add[4, 1023], x[7, 0], add[7, 0], gate[35, 8] = float("inf"), float("nan"), float("inf"), float("-inf"), float("nan")
+    total, h = add_rmsnorm_logits(x, add, gamma, gate, 36, logits)
+    for got, want in zip((total, h), add_rmsnorm(x, add, gamma)):
+        torch.testing.assert_close(got, want, rtol=0, atol=0, equal_nan=True)
+    rows = [0, 1, 3, 5, 6, 8]
+    assert torch.equal(logits[rows, :35], clean[rows, :35]) and bool(logits[:, 35].isnan().all()) and bool(logits[[2, 4, 7]].isnan().all())
