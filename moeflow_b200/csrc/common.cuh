@@ -323,7 +323,7 @@ __device__ __forceinline__ void tc_fence_after_sync() {
 // instruction cost its warp about 100 cycles: the operands live in uniform registers, and behind a test of the lane number the
 // compiler has to move each of them there again.  K blocks of 16 KB of e4m3 weights were bound by that (128 tokens on 288
 // experts, down GEMM 273 / 205 us; 8 tokens 77 / 59), and of 32 KB by a little (gate/up 117 / 111 at 8 tokens).
-#define MF_UMMA_BLOCK(GROUP, KIND)                                                               \
+#define MF_UMMA_BLOCK(KIND)                                                                  \
   asm volatile(                                                                              \
       "{\n\t"                                                                                \
       ".reg .pred one, more, first;\n\t"                                                     \
@@ -333,10 +333,10 @@ __device__ __forceinline__ void tc_fence_after_sync() {
       "setp.eq.b32 more, 0, 0;\n\t"                                                          \
       "add.u64 a1, %1, 2;\n\tadd.u64 a2, %1, 4;\n\tadd.u64 a3, %1, 6;\n\t"                   \
       "add.u64 b1, %2, 2;\n\tadd.u64 b2, %2, 4;\n\tadd.u64 b3, %2, 6;\n\t"                   \
-      "@one tcgen05.mma.cta_group::" GROUP ".kind::" KIND " [%0], %1, %2, %3, first;\n\t"            \
-      "@one tcgen05.mma.cta_group::" GROUP ".kind::" KIND " [%0], a1, b1, %3, more;\n\t"             \
-      "@one tcgen05.mma.cta_group::" GROUP ".kind::" KIND " [%0], a2, b2, %3, more;\n\t"             \
-      "@one tcgen05.mma.cta_group::" GROUP ".kind::" KIND " [%0], a3, b3, %3, more;\n\t"             \
+      "@one tcgen05.mma.cta_group::1.kind::" KIND " [%0], %1, %2, %3, first;\n\t"            \
+      "@one tcgen05.mma.cta_group::1.kind::" KIND " [%0], a1, b1, %3, more;\n\t"             \
+      "@one tcgen05.mma.cta_group::1.kind::" KIND " [%0], a2, b2, %3, more;\n\t"             \
+      "@one tcgen05.mma.cta_group::1.kind::" KIND " [%0], a3, b3, %3, more;\n\t"             \
       "}" ::"r"(d), "l"(a), "l"(b), "r"(idesc), "r"(accumulate)                              \
       : "memory")
 #define MF_UMMA_BLOCK_TWO(GROUP, KIND)                                                           \
@@ -361,19 +361,17 @@ __device__ __forceinline__ void tc_fence_after_sync() {
       "}" ::"r"(d), "l"(a), "l"(b), "r"(idesc), "r"(accumulate), "r"(d2), "l"(a2nd)          \
       : "memory")
 // bf16 / f16 (kind::f16) or 8-bit floats (kind::f8f6f4); the types stand in idesc.
-// kPair: issued by one CTA of a pair for both (cta_group::2, see "CTA pairs" below).
-template <bool kF8, bool kPair = false>
+// kPair: issued by one CTA of a pair for both (cta_group::2, see "CTA pairs" below); two accumulators of 16-bit types only.
+template <bool kF8>
 __device__ __forceinline__ void umma_block(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t accumulate) {
-  if (kPair && kF8) MF_UMMA_BLOCK("2", "f8f6f4");
-  else if (kPair) MF_UMMA_BLOCK("2", "f16");
-  else if (kF8) MF_UMMA_BLOCK("1", "f8f6f4");
-  else MF_UMMA_BLOCK("1", "f16");
+  if (kF8) MF_UMMA_BLOCK("f8f6f4");
+  else MF_UMMA_BLOCK("f16");
 }
 template <bool kF8, bool kPair = false>
 __device__ __forceinline__ void umma_block(uint32_t d, uint32_t d2, uint64_t a, uint64_t a2nd, uint64_t b, uint32_t idesc,
                                            uint32_t accumulate) {
-  if (kPair && kF8) MF_UMMA_BLOCK_TWO("2", "f8f6f4");
-  else if (kPair) MF_UMMA_BLOCK_TWO("2", "f16");
+  static_assert(!(kF8 && kPair), "no kernel of 8-bit operands runs on pairs");
+  if (kPair) MF_UMMA_BLOCK_TWO("2", "f16");
   else if (kF8) MF_UMMA_BLOCK_TWO("1", "f8f6f4");
   else MF_UMMA_BLOCK_TWO("1", "f16");
 }
