@@ -159,8 +159,8 @@ __global__ void __launch_bounds__(kDispatchThreads) dispatch_push_kernel(const m
 // Kernel at 8192 tokens 74 / 53 us, at 2000 21 / 14, at 700 18.5 / 10.3, at 512 10.4 / 8.4.  Below, 256 to 511 tokens, it is
 // 10.4 / 8.3 as well, but the layer takes the same (185 / 181, 206 / 206, 235 / 238 us with 36 e4m3 experts), and one rank
 // uses the local dispatch there (top-8: up to 512 tokens).
-// The whole row is in flight while its token is routed (with half of it, the other half's loads came behind the routing), and one
-// rank fences nothing: kernel at 1000 tokens 13.0 / 8.8 us, at 8192 56 / 38; 600 tokens on 36 e4m3 experts 264.6 / 260.5, 520 on
+// A row's first 4096 values are in flight while its token is routed (with 2048, the others' loads came behind the routing), and one
+// rank fences nothing.  At hidden 4096: kernel at 1000 tokens 13.0 / 8.8 us, at 8192 56 / 38; 600 tokens on 36 e4m3 experts 264.6 / 260.5, 520 on
 // 72 bf16 ones 246.4 / 242.9, calls at the power cap as before.
 constexpr int kManyWarps = 4;
 
@@ -175,7 +175,7 @@ __global__ void __launch_bounds__(32 * kManyWarps) dispatch_push_many_kernel(con
   if (t < a.C) {
     const bool has_token = t < a.T;
     const bool live = has_token && (a.num_valid == nullptr || t < *a.num_valid);
-    // the row is under way while the token is routed
+    // the first kAhead * 256 values of the row are under way while the token is routed, any others are loaded behind it
     const int chunks = a.H / 8;  // 16-byte chunks
     constexpr int kAhead = 16;
     const uint4* xr = reinterpret_cast<const uint4*>(static_cast<const __nv_bfloat16*>(a.x) + (size_t)t * a.H);

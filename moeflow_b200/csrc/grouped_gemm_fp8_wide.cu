@@ -13,9 +13,9 @@
 // quarter and half of the columns each) hold 128 sums and two loads in registers, which is why the other four warps
 // hand registers over to them.  Single multiply-adds, not pairs: the same rate (128 a clock).  Kernels alone, 2000 tokens on 36
 // experts, us, gate/up and down: 32 columns in pairs 309 / 173, 16 in pairs 320 / 153, 32 single 297 / 161, 16 single 297 / 156.
-// Spills explain the down GEMM only (rows by map, 28 bytes stored with 32 in pairs, none with 16 single); the gate/up GEMM
-// (gathered rows) has 4 and 60 and is the faster one with 60, for a reason that was not looked for.  With waits and arrivals
-// that do not branch per lane (mbar_wait_warp): 291 / 157.
+// With waits and arrivals that do not branch per lane (mbar_wait_warp): 291 / 157; the call of 2000 tokens, together with a faster
+// dispatch, 595 / 589 in four alternating runs.  Registers spilled (bytes stored / loaded, before and with these waits): down by map 0 / 0 and 8 / 16, down gathered
+// 28 / 44 and 72 / 84, gate/up by map 8 / 16 and 92 / 92, gate/up gathered 60 / 64 and 28 / 60.  The times do not follow the spills.
 // 36 experts of 3 x 4096 x 1536, whole layer, against the 64-row kernel's form on 128-row tiles, forwards on three weight sets
 // in turn, with the promotion in its first form (32 columns in pairs): 2000 tokens 917 / 581 us, 1000 tokens 524 / 353, 500 tokens
 // 317 / 222.  What bounds it now: a promotion warp's own instructions per K block (loads, waits, multiply-adds), not the 48 KB that a

@@ -24,10 +24,11 @@
 // 32-row quarter) adds the segments in K order, so the result does not depend on arrival order.
 //
 // Warp roles (256 threads, one CTA per SM, persistent):
-//   warp 0      TMA producer for the weight tiles (lane 0 issues); hands the segments out to the other roles
-//   warp 1      UMMA issuer (lane 0 issues); owns the tensor-memory allocation
-//   warps 2-3   token-operand producers: gather rows by index with cp.async into the swizzled tile (256-row tiles: warps
-//               12-15), or warp 2 alone fetches contiguous rows by TMA
+//   warp 0      TMA producer for the weight tiles (an elected lane issues); hands the segments out to the other roles
+//   warp 1      UMMA issuer (an elected lane issues); owns the tensor-memory allocation
+//   warps 2-3   token-operand producers: gather rows by index with cp.async into the swizzled tile, or warp 2 alone fetches
+//               contiguous rows by TMA.  256-row tiles of two accumulators gather with warps 12-15; these two then have
+//               nothing to do but, where asked for, to expand the down GEMM's e4m3 weights (expand_src)
 //   warps 4-7   epilogue: tcgen05.ld -> registers -> activation / scale -> global
 //
 // CTA pairs (kPair: units of two accumulators on 256-row tiles): the two CTAs of a cluster take adjacent weight blocks of one
@@ -84,8 +85,8 @@ struct GemmCfg {
   static constexpr int kAccCols = kATiles * N_MAX;
   // Two accumulator stages: the epilogue of unit i overlaps the main loop of unit i + 1.  With two accumulators of 256
   // columns a wide unit (more than 128 token columns) needs all 512 tensor-memory columns and takes both stages; a narrow
-  // one takes one, its accumulators 128 columns apart.  Tiles are narrow more often than not where 256-row tiles begin (80
-  // expected rows per expert).
+  // one takes one, its accumulators 128 columns apart.  Tiles are narrow more often than not where 256-row tiles begin (36
+  // expected rows per expert on CTA pairs, else 80).
   static constexpr int kAccStages = 2;
   static constexpr bool kWide = kAccStages * kAccCols > 512;
   static constexpr int kStageCols = kWide ? 256 : kAccCols;

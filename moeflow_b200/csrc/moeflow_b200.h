@@ -105,7 +105,7 @@ typedef struct {
   // another block-scaled e4m3 matrix to bf16 (as mf_dequant_block_fp8; the down GEMM's weights).  expand_done, zero before, counts
   // finished pieces of MF_EXPAND_PIECE values; the down GEMM of 256-row tiles, given the counter as w_wait, fetches no weights
   // before it has reached w_wait_target.
-  const void* expand_src;    // [expand_rows, expand_cols] e4m3, 16-byte aligned; both multiples of 128, less than 2^31 values / 16
+  const void* expand_src;    // [expand_rows, expand_cols] e4m3, 16-byte aligned; both multiples of 128, rows * cols / 16 < 2^31 - 256
   const float* expand_scale; // [expand_rows / 128, expand_cols / 128]
   void* expand_out;          // [expand_rows, expand_cols] bf16, 16-byte aligned
   int expand_rows, expand_cols;

@@ -631,7 +631,8 @@ class FixedEPLayer:
         # 2000 tokens 826 / 806 (72 experts), 700 tokens 340 / 330, 8192 tokens (e4m3, expanded) 2838 / 2700 (36 experts).
         # Copies of less than 8 MB cost up to 5 us and save up to 2: 2.1 MB 54.5 / 49.9, 3.1 MB 56.6 / 55.3, 3.9 MB 68.1 / 69.1,
         # 6.2 MB 99.3 / 97.6, 7.5 MB 100.1 / 100.1.  Those layers keep it for one reason: the checks of the copying form on
-        # 256-row tiles build such a layer and expect it there.
+        # 256-row tiles build such a layer and expect it there, by `choose_block_m` or with a height of 256 asked for.  Tiles that
+        # are 256 rows high by `paired_block_m` only never had it and gather.
         copied = self.block_m >= 256 and N * H * 2 < 8 << 20 and ("block_m" in self.gemm_kwargs or choose_block_m(Cc, K, L, fp8=fp8_hint) >= 256)
         self.permute_rows = bool(self.gemm_kwargs.get("permute_rows", copied))
         if self.permute_rows:
@@ -1077,7 +1078,8 @@ def paired_block_m(capacity: int, top_k: int, local_experts: int, hidden: int = 
 
     256 rows, too, where all units are under way at once, up to 48 pairs in the gate/up GEMM and at least as many in the down GEMM: 512 x
     256, 36 experts, 40 rows 36 / 39 / 33, 75 rows 44 / 48 / 44 (zipf 35 / 39 / 42); 1024 x 512, 16 experts, 75 rows 41 / 44 / 41; 4096 x 1536,
-    8 experts, 75 rows 97 / 90 / 86.  With fewer units in the down GEMM its CTAs stand idle: 512 x 1024, 16 experts 42 / 40 / 52;
+    8 experts, 75 rows 97 / 90 / 86.  From 19 experts on zipf popularity loses up to 8 % there (4096 x 256, 24 experts 69 / 87 / 94) where
+    even popularity gains up to 15.  With fewer units in the down GEMM its CTAs stand idle: 512 x 1024, 16 experts 42 / 40 / 52;
     2048 x 1536, 8 experts 57 / 62 / 72.
 
     128 rows between: one to three rounds of units, the last one of twice the length: 1024 x 512, 48 experts, 75 rows 69 / 78 / 82; 512 x 1024,
